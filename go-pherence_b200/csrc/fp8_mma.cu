@@ -352,9 +352,11 @@ fp8_mma_kernel(const __grid_constant__ Fp8Args a) {
         for (int j = 0; j < i; ++j, wk.next(a))
           bulk_load_1d(smem_u32(ring + (size_t)j * kStage) + TT * kABytes, b_src(wk), kBBytes, full0 + 8 * j);
       }
-      for (; wk.live(a) && ok; ++i, wk.next(a)) {
-        const int slot = i % S, round = i / S;
-        if (round > 0) ok = mbar_wait(empty0 + 8 * slot, (round - 1) & 1, a.status, 501);
+      RingCursor rc;
+      for (int j = 0; j < i; ++j) rc.next(S);
+      for (; wk.live(a) && ok; ++i, wk.next(a), rc.next(S)) {
+        const int slot = rc.s;
+        if (i >= S) ok = mbar_wait(empty0 + 8 * slot, rc.ph ^ 1u, a.status, 501);
         if (!ok) break;
         const uint32_t dst = smem_u32(ring + (size_t)slot * kStage);
         const int nt = tiles_of(wk);
@@ -371,16 +373,16 @@ fp8_mma_kernel(const __grid_constant__ Fp8Args a) {
     const uint64_t adesc_hi = ((uint64_t)(2048u >> 4) << 16) | ((uint64_t)(128u >> 4) << 32) | (1ull << 46);
     // B: halves (N / 8) * 128 B apart, row groups 128 B apart
     const uint64_t bdesc_hi = ((uint64_t)(((N / 8) * 128u) >> 4) << 16) | ((uint64_t)(128u >> 4) << 32) | (1ull << 46);
-    int i = 0;
+    RingCursor rc;
     for (int it = 0; wk.live(a) && ok; ++it) {
       const int b = it % ND;
       if (it >= ND) ok = mbar_wait(dfree0 + 8 * b, ((it - ND) / ND) & 1, a.status, 502);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       bool first = true;
-      for (;; ++i) {
-        const int slot = i % S;
-        ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * slot, (i / S) & 1, a.status, 503));
+      for (;; rc.next(S)) {
+        const int slot = rc.s;
+        ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * slot, rc.ph, a.status, 503));
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const bool last = wk.last_stage();
@@ -405,7 +407,7 @@ fp8_mma_kernel(const __grid_constant__ Fp8Args a) {
         first = false;
         wk.next(a);
         if (last) {
-          ++i;
+          rc.next(S);
           break;
         }
       }

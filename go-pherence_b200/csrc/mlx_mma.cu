@@ -513,9 +513,11 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
         for (int j = 0; j < i; ++j, sw.next(a))
           bulk_load_1d(smem_u32(ring + (size_t)j * kStage) + C * kStageBytes, bsrc(sw), sw.nc() * kBTileBytes, full0 + 8 * j);
       }
-      for (; sw.live(a) && ok; ++i, sw.next(a)) {
-        int slot = i % S, round = i / S;
-        if (round > 0) ok = mbar_wait(empty0 + 8 * slot, (round - 1) & 1, a.status, 1);
+      RingCursor rc;
+      for (int j = 0; j < i; ++j) rc.next(S);
+      for (; sw.live(a) && ok; ++i, sw.next(a), rc.next(S)) {
+        const int slot = rc.s;
+        if (i >= S) ok = mbar_wait(empty0 + 8 * slot, rc.ph ^ 1u, a.status, 1);
         else if (i == kFirstStages) ok = mbar_wait(full0, 0, a.status, 11);  // the first stage is in: the rest of the ring may follow
         if (!ok) break;
         uint32_t dst = smem_u32(ring + (size_t)slot * kStage);
@@ -539,9 +541,10 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
       const uint64_t desc_hi = ((uint64_t)(kLBO >> 4) << 16) | ((uint64_t)(kSBO >> 4) << 32) | (1ull << 46);
       // Every role sees every stage in order, so no barrier phase is ever skipped (a parity wait
       // can only tell the current phase from the one before it).
-      for (int i = 0; sw.live(a) && ok; ++i) {
-        const int ba = i % NA, b = i % ND, slot = i % S;
-        ok = mbar_wait(full0 + 8 * slot, (i / S) & 1, a.status, 8);
+      RingCursor rc;
+      for (int i = 0; sw.live(a) && ok; ++i, rc.next(S)) {
+        const int ba = i % NA, b = i % ND, slot = rc.s;
+        ok = mbar_wait(full0 + 8 * slot, rc.ph, a.status, 8);
         if (ok && F::kConv) ok = mbar_wait(aready0 + 8 * ba, (i / NA) & 1, a.status, 2);
         if (ok && i >= ND) ok = mbar_wait(dfree0 + 8 * b, ((i - ND) / ND) & 1, a.status, 5);
         ok = __all_sync(0xffffffffu, ok);
@@ -590,9 +593,10 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
     const int q4 = warp & 3, grp = warp >> 2;
     const int r = q4 * 32 + lane;
     const uint32_t lane_base = (uint32_t)(q4 * 32) << 16;
-    for (int i = 0; sw.live(a) && ok; ++i, sw.next(a)) {
-      const int ba = i % NA, slot = i % S;
-      ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * slot, (i / S) & 1, a.status, 4));
+    RingCursor rc;
+    for (int i = 0; sw.live(a) && ok; ++i, sw.next(a), rc.next(S)) {
+      const int ba = i % NA, slot = rc.s;
+      ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * slot, rc.ph, a.status, 4));
       if (ok && i >= NA) ok = __all_sync(0xffffffffu, mbar_wait(afree0 + 8 * ba, ((i - NA) / NA) & 1, a.status, 3));
       if (!ok) break;
       if ((i & 1) != grp) continue;
@@ -660,8 +664,9 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
     constexpr int kSub = kHB * N <= 64 ? kHB : 64 / N;      // blocks per pass (at most 64 columns in registers)
     constexpr bool kNarrow = kSub * N == 8;                 // a pass of one 8-column block: one 8-column load
     constexpr int NLD = kNarrow ? 1 : kSub * N / 16;        // 16-column loads per pass
-    for (int i = 0; sw.live(a) && ok; ++i) {
-      int b = i % ND, slot = i % S;
+    RingCursor rc;
+    for (int i = 0; sw.live(a) && ok; ++i, rc.next(S)) {
+      const int b = i % ND, slot = rc.s;
       if (G && sw.entry != cur_entry) {
         // a new entry: its tables, row count and result rows.  Every epilogue thread passed the barrier
         // that ends the item before, so nobody still reads the old tables.
@@ -674,7 +679,7 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
         for (int m = 0; m < (G ? MB : 1); ++m) orow[m] = a.gdirect ? __ldg(&ge->item[m]) : cur_entry * MB + m;
         asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
       }
-      ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * slot, (i / S) & 1, a.status, 6));
+      ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * slot, rc.ph, a.status, 6));
       uint4 mvs[C];
       uint32_t q6d = 0;  // Q6_K: the super-block's f16 d (the 16 int8 scales are in mvs)
       const int nc = sw.nc();
