@@ -11,6 +11,7 @@
 #include <string.h>
 
 #include "stream_gemv.cuh"
+#include "qgemm.cuh"
 #include "tc_gemm.cuh"
 
 namespace goph {
@@ -97,6 +98,16 @@ __global__ void fp8_fill_scale_kernel(float* __restrict__ dst, const float* __re
 
 static bool valid_fp8(const goph_fp8_linear* w) {
   return w && w->magic == kMagicFP8 && (w->weight || w->tiled) && w->scale && w->in_dim > 0 && w->out_dim > 0;
+}
+
+// The several-row tensor-core product (qgemm.cu) reads both layouts (rows of whole 16-byte units).
+static bool qgemm_takes(const goph_fp8_linear* w, const void* x, int batch) {
+  return batch > options().gemm_rows && w->in_dim % 16 == 0 && w->in_dim <= 65536 && (uintptr_t)x % 16 == 0;
+}
+
+static int fp8_qgemm(const goph_fp8_linear* w, float* out, const void* x, bool x_bf16, int batch, cudaStream_t stream) {
+  const QWeight q{Q_FP8, w->tiled != nullptr, w->tiled ? w->tiled : w->weight, nullptr, w->scale, w->bias, w->device, w->out_dim, w->in_dim};
+  return qgemm(q, out, x, x_bf16, batch, stream);
 }
 
 }  // namespace goph
@@ -230,6 +241,7 @@ GOPH_API int goph_fp8_gemm(float* out_dev, uint64_t out_len, const float* x_dev,
   cudaStream_t s = (cudaStream_t)stream;
   // Tensor-core layout: every batch size goes to the kernel that feeds the e4m3 bytes to the MMA as
   // they lie (fp8_mma.cu); the row-major layout is served by the CUDA-core kernels below.
+  if (qgemm_takes(w, x_dev, batch)) return fp8_qgemm(w, out_dev, x_dev, false, batch, s);
   if (w->tiled) return tc_gemm_fp8(w, out_dev, x_dev, false, batch, s);
   if (!w->tiled && w->in_dim % 16 != 0) {
     note_launch();
@@ -269,6 +281,7 @@ GOPH_API int goph_fp8_gemm_bf16(float* out_dev, uint64_t out_len, const uint16_t
                 "goph_fp8_gemm_bf16 needs a linear in the tensor-core layout (in_dim a multiple of 256, no NaN codes, "
                 "uploaded with fp8_layout 0 or 2)");
   if (int rc = use_device(w->device)) return rc;
+  if (qgemm_takes(w, x_bf16_dev, batch)) return fp8_qgemm(w, out_dev, x_bf16_dev, true, batch, (cudaStream_t)stream);
   return tc_gemm_fp8(w, out_dev, x_bf16_dev, true, batch, (cudaStream_t)stream);
 }
 

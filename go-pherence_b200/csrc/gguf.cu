@@ -22,6 +22,7 @@
 #include <string.h>
 
 #include "mlx_mma.cuh"
+#include "qgemm.cuh"
 #include "stream_gemv.cuh"
 #include "gguf_fmt.cuh"
 
@@ -353,6 +354,17 @@ static bool valid_gguf(const goph_gguf_matrix* m) {
                                    ((m->qtype == GOPH_GGUF_Q8_0 || m->qtype == GOPH_GGUF_Q6_K) && m->d16))));
 }
 
+// The several-row tensor-core product (qgemm.cu) reads both layouts.
+static bool qgemm_takes(const goph_gguf_matrix* m, const void* x, int batch) {
+  return batch > options().gemm_rows && m->in_dim <= 65536 && (uintptr_t)x % 16 == 0;
+}
+
+static int gguf_qgemm(const goph_gguf_matrix* m, float* out, const float* x, int batch, cudaStream_t stream) {
+  const int fmt = m->qtype == GOPH_GGUF_Q4_K ? Q_Q4K : m->qtype == GOPH_GGUF_Q5_K ? Q_Q5K : m->qtype == GOPH_GGUF_Q6_K ? Q_Q6K : Q_Q80;
+  const QWeight q{fmt, m->tiled != nullptr, m->tiled ? m->tiled : m->data, m->d16, nullptr, nullptr, m->device, m->out_dim, m->in_dim};
+  return qgemm(q, out, x, false, batch, stream);
+}
+
 static long gguf_row_bytes(int qtype, int in_dim) {
   if (qtype == GOPH_GGUF_Q8_0) return in_dim % 32 ? -1 : (long)in_dim / 32 * 34;
   if (qtype == GOPH_GGUF_Q4_K) return in_dim % 256 ? -1 : (long)in_dim / 256 * 144;
@@ -511,6 +523,7 @@ GOPH_API int goph_gguf_project(float* out_dev, uint64_t out_len, const float* x_
     return fail(GOPH_E_INVALID, "buffers x=%llu/%llu out=%llu/%llu", (unsigned long long)x_len,
                 (unsigned long long)need_x, (unsigned long long)out_len, (unsigned long long)need_o);
   if (int rc = use_device(m->device)) return rc;
+  if (qgemm_takes(m, x_dev, batch)) return gguf_qgemm(m, out_dev, x_dev, batch, (cudaStream_t)stream);
   if (m->tiled) return gguf_mma_launch(m, out_dev, x_dev, batch, options().mlx_digits, (cudaStream_t)stream);
   StreamArgs a;
   memset(&a, 0, sizeof a);
@@ -548,7 +561,7 @@ GOPH_API int goph_gguf_project_pair(float* out_a_dev, uint64_t out_a_len, float*
   if (!valid_gguf(a) || !valid_gguf(b)) return fail(GOPH_E_INVALID, "invalid GGUF matrix handle");
   if (a->device != b->device || a->in_dim != b->in_dim)
     return fail(GOPH_E_INVALID, "pair projection: matrices differ in device or inDim (%d vs %d)", a->in_dim, b->in_dim);
-  if (a->tiled && b->tiled && a->qtype == b->qtype) {
+  if (a->tiled && b->tiled && a->qtype == b->qtype && !qgemm_takes(a, x_dev, batch)) {
     // both on the tensor-core path: validated like a single projection, x prepared once
     if (batch <= 0) return fail(GOPH_E_INVALID, "batch=%d", batch);
     uint64_t need_x, need_a, need_b;

@@ -63,6 +63,7 @@ struct Options {
   int gguf_layout = 0; // as mlx_layout, for Q4_K / Q8_0 matrices
   int fp8_layout = 0;  // as mlx_layout, for FP8 linears
   int fp8_convert = 0; // 1: bf16 batches above 32 rows of a tensor-core FP8 linear go through the kernel that turns e4m3 into bf16
+  int gemm_rows = 8;   // activation rows above which a product runs in the several-row tensor-core kernel
   int mlx_rows = 0, gguf_rows = 0, fp8_rows = 0;
   int mlx_ctas_per_sm = 0;  // tuning aid: cap on resident CTAs per SM of the MLX streaming kernel and of product lists (0 = by shape)
 };
@@ -101,6 +102,8 @@ struct goph_mlx_weight {
   int device;
   int in_dim, out_dim, group_size, groups;
   int sb_bf16;          // 1: sb is __nv_bfloat162 {scale,bias}; 0: float2 {scale,bias}
+  int foldable;         // every scale is zero or of magnitude 2^-27 .. 7.875: scale * (nibble - 8) * 2^10 is an f16
+                        // exactly (8 + 3 significant bits), which lets qgemm.cu scale the weights as it converts them
   uint32_t* qweight;    // [out_dim][in_dim/8]
   void* sb;             // [out_dim][groups]
   uint8_t* tiled;       // tiled layout or nullptr

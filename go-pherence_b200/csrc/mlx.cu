@@ -30,6 +30,7 @@
 
 #include "goph_internal.cuh"
 #include "mlx_mma.cuh"
+#include "qgemm.cuh"
 #include "tc_gemm.cuh"
 
 namespace goph {
@@ -732,10 +733,13 @@ __global__ void mlx_dequant_tiled_kernel(const unsigned char* __restrict__ tiled
 
 // Upload helpers: decide whether every scale/bias is a bf16 value, then interleave.
 __global__ void mlx_sb_probe_kernel(const float* __restrict__ s, const float* __restrict__ b, size_t n,
-                                    int* __restrict__ not_bf16) {
+                                    int* __restrict__ flags) {
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  if ((__float_as_uint(s[i]) & 0xFFFFu) | (__float_as_uint(b[i]) & 0xFFFFu)) *not_bf16 = 1;
+  if ((__float_as_uint(s[i]) & 0xFFFFu) | (__float_as_uint(b[i]) & 0xFFFFu)) atomicOr(flags, 1);
+  // scale * (nibble - 8) * 2^10 is an f16 exactly (see goph_mlx_weight::foldable)
+  const float m = fabsf(s[i]);
+  if (!(m == 0.f || (m >= 7.4505806e-9f && m <= 7.875f))) atomicOr(flags, 2);
 }
 
 __global__ void mlx_sb_pack_kernel(const float* __restrict__ s, const float* __restrict__ b, size_t n,
@@ -892,23 +896,34 @@ static int launch_generic(const goph_mlx_weight* w, float* out, const float* x, 
   return GOPH_OK;
 }
 
+// The several-row tensor-core product (qgemm.cu) reads both layouts of 64-element groups with bf16 tables.
+static bool qgemm_takes(const goph_mlx_weight* w, const void* x) {
+  return w->group_size == 64 && w->sb_bf16 && w->in_dim <= 65536 && (w->tiled || (uintptr_t)x % 16 == 0);
+}
+
+static int mlx_qgemm(const goph_mlx_weight* w, float* out, const void* x, bool x_bf16, int batch, cudaStream_t stream) {
+  const QWeight q{w->foldable ? Q_MLX4F : Q_MLX4, w->tiled != nullptr, w->tiled ? (const void*)w->tiled : w->qweight, w->sb, nullptr, nullptr, w->device, w->out_dim, w->in_dim};
+  return qgemm(q, out, x, x_bf16, batch, stream);
+}
+
 // Products for n weights sharing x [batch,in]; outs[i] is [batch,out_i].
 static int mlx_products(int n, float* const* outs, const goph_mlx_weight* const* ws, const float* x, int batch,
                         cudaStream_t stream) {
   const goph_mlx_weight* w0 = ws[0];
-  bool any_tiled = false;
-  for (int i = 0; i < n; ++i) any_tiled = any_tiled || ws[i]->tiled;
-  if (any_tiled) {
+  bool any_tiled = false, any_rows = false;
+  for (int i = 0; i < n; ++i) {
+    any_tiled = any_tiled || ws[i]->tiled;
+    any_rows = any_rows || (batch > options().gemm_rows && qgemm_takes(ws[i], x));
+  }
+  if (any_tiled || any_rows) {
     // tiled weights run on the tensor cores; row-major ones in the same call take their own path
     bool prepared = false;  // weights of one call share x: its digits are prepared once
     for (int i = 0; i < n; ++i) {
       const goph_mlx_weight* one = ws[i];
       float* o = outs[i];
       int rc;
-      if (one->tiled && batch > 8) {
-        // more rows than one pass of the integer kernel takes: bf16 operands, weights streamed once
-        // per 16 rows (general f32 activations are split into three exact bf16 pieces)
-        rc = tc_gemm_mlx(one, o, x, false, batch, stream);
+      if (batch > options().gemm_rows && qgemm_takes(one, x)) {
+        rc = mlx_qgemm(one, o, x, false, batch, stream);
       } else if (one->tiled) {
         rc = mlx_mma_launch(one, o, x, batch, options().mlx_digits, stream, prepared);
         prepared = true;
@@ -1204,9 +1219,10 @@ static int mlx_upload_common(int device, const uint32_t* weight, const float* sc
   UP(cudaMemset(flag, 0, sizeof(int)));
   unsigned blocks = (unsigned)((want_s + 255) / 256);
   mlx_sb_probe_kernel<<<blocks, 256>>>(ds, db, want_s, flag);
-  int not_bf16 = 0;
-  UP(cudaMemcpy(&not_bf16, flag, sizeof(int), cudaMemcpyDeviceToHost));
-  h->sb_bf16 = not_bf16 ? 0 : 1;
+  int flags = 0;
+  UP(cudaMemcpy(&flags, flag, sizeof(int), cudaMemcpyDeviceToHost));
+  h->sb_bf16 = flags & 1 ? 0 : 1;
+  h->foldable = flags & 2 ? 0 : 1;
   UP(cudaMalloc(&h->sb, want_s * (h->sb_bf16 ? 4 : 8)));
   mlx_sb_pack_kernel<<<blocks, 256>>>(ds, db, want_s, h->sb, h->sb_bf16);
   UP(cudaGetLastError());
@@ -1288,7 +1304,7 @@ GOPH_API int goph_kernel_status(int device, int* out_status) {
   if (!out_status) return fail(GOPH_E_INVALID, "goph_kernel_status: nil result pointer");
   if (int rc = use_device(device)) return rc;
   *out_status = mlx_mma_status(device);
-  if (*out_status == 0) *out_status = tc_gemm_status(device);
+  if (*out_status == 0) *out_status = qgemm_status(device);
   if (*out_status == 0) *out_status = fp8_mma_status(device);
   if (*out_status == 0) *out_status = gguf_work_status(device);
   if (*out_status == 0) *out_status = moe_status(device);
@@ -1301,7 +1317,7 @@ GOPH_API int goph_kernel_status_clear(int device) {
   if (int rc = use_device(device)) return rc;
   GOPH_CUDA(cudaDeviceSynchronize());
   mlx_mma_status_clear(device);
-  tc_gemm_status_clear(device);
+  qgemm_status_clear(device);
   fp8_mma_status_clear(device);
   gguf_work_status_clear(device);
   moe_status_clear(device);
@@ -1383,7 +1399,7 @@ GOPH_API int goph_mlx_gemm_bf16(float* out_dev, uint64_t out_len, const uint16_t
                 "goph_mlx_gemm_bf16 needs a weight in the tiled layout (group size 64, in_dim a multiple of 256, "
                 "uploaded with mlx_layout 0 or 2); this one is row-major");
   if (int rc = use_device(w->device)) return rc;
-  return tc_gemm_mlx(w, out_dev, x_bf16_dev, true, batch, (cudaStream_t)stream);
+  return mlx_qgemm(w, out_dev, x_bf16_dev, true, batch, (cudaStream_t)stream);
 }
 
 GOPH_API int goph_mlx_gemv(float* out_dev, uint64_t out_len, const float* x_dev, uint64_t x_len,

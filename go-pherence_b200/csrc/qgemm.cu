@@ -1,0 +1,1341 @@
+// Quantised weights times several activation rows on the 5th-generation tensor cores: f16 operands,
+// f32 accumulators in TMEM, one kernel for every weight format and both device layouts.
+//
+// Stands behind nvidia.GemmMLX (backends/nvidia/runtime/mlx.go:395-431), GPUGGUFMatrix.
+// ProjectBatchToBuffer (runtime/gguf_matrix.go:121-135) and GemmFP8E4M3Buffer (runtime/fp8.go:271-320)
+// for prefill chunks and verifier batches.
+//
+// Arithmetic
+//   * A operand (weights, the 128 rows of a tile), written to TMEM as f16 by converter warps, exact:
+//       MLX4F  scale * (nibble - 8) * 2^10, at most 11 significant bits: weights whose scales allow it
+//              (goph_mlx_weight::foldable; every checkpoint seen does), so thousands of elements accumulate in
+//              one block of columns and nothing is scaled on the way out.
+//       MLX4   the others: nibble n as the f16 subnormal n * 2^-24 (the masked nibble IS the bit pattern; the
+//              nibbles at bits 4..7 of a half read as 16 n and meet activations scaled by 1/16), a block of
+//              columns per 64 elements.
+//       Q4_K   the nibble as a subnormal times the sub-block's 6-bit scale: sc * n has at most 10 bits (Q5_K:
+//       Q5_K   11, the most an f16 holds), so a block of columns lasts a super-block.
+//       Q6_K   q - 32, a block per 16 elements (an 8-bit scale times 6 bits does not fit).
+//       Q8_0   the signed byte, a block per 32 elements.
+//       FP8    e4m3 -> f16 (exact, NaN codes stay NaN), a block of 4096 elements.
+//   * B operand (activations): every row is scaled by a power of two so that its largest magnitude
+//     lies in [2^14, 2^15), and written as the sum of up to three f16 values, each the rounding of
+//     what the ones before it left over.  Three hold an f32 exactly down to 2^-39 of the row's largest
+//     element (f32 sums do not see below that); a bf16 needs one.  All pieces accumulate into the
+//     same columns.  The preparation kernel notes per row and 256 elements how many pieces are not
+//     zero: f32 buffers that hold bf16 values cost one pass of the tensor cores, not three.
+//   * The affine term (biases or minima times the groups' sums of x) is one or two more K16 steps per
+//     chunk in bf16: A the biases, B the sums in three bf16 pieces (exact).
+//   * Epilogue: tcgen05.ld per block, times the block's scale, running sums in registers, f32.
+//
+// What bounds it: the hand-overs between the roles (a wait that succeeds at once costs a warp about a
+// hundred cycles), the conversion, and in front of it all the preparation launch.  An MMA of M128 x N x
+// K16 takes N/2 cycles with A in TMEM (measured down to N = 16; with A in shared memory 32 + N/4 below
+// N = 128), so 256 elements of a tile and 64 columns take 512 cycles per piece.  The B tiles cross from
+// the L2 once per row tile, which at 64 columns is more than an SM gets: with TT = 2 the two tiles of an
+// item share each B tile.
+//
+// Work: items (group of TT row tiles, block of up to 64 or 128 activation rows).  The items of the last,
+// partial wave are cut along K over the CTAs of a thread-block cluster, whose sums meet in shared memory,
+// added in split order.
+//
+// A CTA, one per SM, 28 warps: W loader (tiled layouts: a bulk copy per 256 elements and tile, stored
+// contiguously; row-major and streaming layouts: 16-byte cp.async into the same image, rows and elements
+// past the matrix zero-filled), B loader (a slot per half chunk, all of its pieces), 2 MMA warps, 16
+// converter and 8 epilogue warps, half of them in either of two pipes (see the kernel).
+// Every wait is bounded (~2 s); a waiter that gives up records a code (800+) and the CTA winds down.
+//
+// Measured (B200, a call among others, us; before: integer products of 4 or 8 rows, or the bf16 kernel's
+// passes of 16 f32 or 64 bf16 rows):
+//   Q8_0 4096x4096 x19 44.5 -> 18.1; Q4_K 14336x4096 x64 381 -> 39.8; MLX4 6144x4096 x100 f32 129 -> 31.8;
+//   MLX4 8192x8192 x64 bf16 33.2 -> 32.3; FP8 28672x8192 x256 bf16 226 -> 112
+#include <string.h>
+
+#include <mutex>
+
+#include "qgemm.cuh"
+#include "tc_common.cuh"
+
+namespace goph {
+
+using namespace tc;
+
+namespace {
+
+// Tuning build only (-DGOPH_TUNING): one CTA records clock64 at the hand-over points.
+#ifdef GOPH_TUNING
+__device__ long long g_qg_trace[8][64];
+#define TP(...) __VA_ARGS__
+#define MARK(ev, i) \
+  if (blockIdx.x == gridDim.x / 2 && lane == 0 && (i) < 64) g_qg_trace[ev][i] = clock64()
+#else
+#define TP(...)
+#define MARK(ev, i)
+#endif
+
+constexpr int kTileRows = 128;
+constexpr int kChunkK = 256;
+constexpr int kConvWarps = 16, kEpiWarps = 8, kEpiThreads = kEpiWarps * 32;  // in both pipes
+constexpr int kWarpMMA = kConvWarps + kEpiWarps, kWarpB = kWarpMMA + 2, kWarpW = kWarpB + 1;  // two MMA warps
+constexpr int kThreads = (kWarpW + 1) * 32;
+// Registers: the block is launched with 72 a thread (896 threads: 64512); the epilogue, which keeps a
+// row's sums of 64 columns, takes what the others give up: 256 * 128 + 512 * 48 + 128 * 56 = 64512.
+constexpr int kEpiRegs = 128, kConvRegs = 48, kMiscRegs = 56;
+constexpr int kMaxSplits = 8;
+
+// What a format's slot of the weight ring looks like: [weights][row metadata].
+template <int F, bool TILED>
+struct QF {
+  // packed nibbles in the row image (16-byte unit u of row r at r * 128 + ((u ^ (r & 7)) << 4)), else a
+  // byte per weight as [16-byte unit][row]
+  static constexpr bool kMLX = F == Q_MLX4 || F == Q_MLX4F;
+  static constexpr bool kNibble = kMLX || F == Q_Q4K || (!TILED && (F == Q_Q5K || F == Q_Q6K));
+  static constexpr int kHigh = kNibble && F == Q_Q5K ? 4096 : kNibble && F == Q_Q6K ? 8192 : 0;  // bits above the nibble, [16-byte unit][row]
+  static constexpr int kHighOff = kTileRows * 128;
+  static constexpr int kWBytes = (kNibble ? kTileRows * 128 : kTileRows * 256) + kHigh;
+  static constexpr int kMeta = F == Q_FP8 ? 0 : F == Q_Q6K || (F == Q_Q80 && !TILED) ? 32 : 16;  // metadata bytes of a row
+  static constexpr int kAux = F == Q_MLX4 ? 1 : F == Q_Q4K || F == Q_Q5K || F == Q_MLX4F ? 2 : 0;  // K16 steps of the affine term per chunk
+  static constexpr bool kLong = F == Q_FP8 || F == Q_MLX4F;  // accumulator blocks of many chunks: nothing is scaled in between
+  static constexpr bool kChunk = F == Q_Q4K || F == Q_Q5K;    // a block per pipe and chunk
+  static constexpr int kBlk = F == Q_MLX4 ? 64 : F == Q_Q80 ? 32 : F == Q_Q6K ? 16 : 128;  // elements of a block, for the others
+  static constexpr int kSlot = kWBytes + kTileRows * kMeta;
+  static constexpr float kUnit = F == Q_MLX4 ? 16777216.f : F == Q_MLX4F ? 1.f / 1024.f : F == Q_Q4K || F == Q_Q5K ? 16384.f : 1.f;  // A holds the weights (the nibbles, the scale times the nibble) / kUnit
+  // order of the elements inside a K16 step: 0 natural; 1 the nibble order (0 4 1 5 2 6 3 7 of each
+  // packed word); 2 the same with the odd elements' activations scaled by 1/16
+  static constexpr int kOrder = F == Q_MLX4 ? 2 : kNibble ? 1 : 0;
+  // sums of x of the affine term: 1 four of 64 elements, 2 eight of 32, 3 four of 64 and eight times the same
+  static constexpr int kSums = F == Q_MLX4 ? 1 : kChunk ? 2 : F == Q_MLX4F ? 3 : 0;
+};
+
+struct QArgs {
+  const unsigned char* w;
+  const void* aux;
+  const unsigned char* xb;     // B tiles [row block][chunk * 2 + half][piece][K step 8][K half 2][n/8][8][16 B]
+  const unsigned char* xaux;   // [row block][chunk][K16 step][K half 2][n/8][8][16 B]: sums of x in three bf16 pieces (scaled like x, / kUnit)
+  const float* xinv;           // [batch] 2^-s of each activation row
+  const unsigned char* flags;  // [row block][chunk][64] pieces in use, or nullptr: one piece
+  const float* scale;
+  const float* bias;
+  float* out;
+  int* status;
+  size_t xb_stride;            // bytes of a row block in xb
+  int out_dim, in_dim, batch;
+  int ntiles, nchunks, nblocks;
+  int nfull, ntail, splits;    // whole items (a multiple of the grid), then at most one per cluster, cut along K
+  int wslots, bslots, bslot, comb, pmax;  // depths of the rings, bytes of a B slot and of comb, pieces per half chunk in xb
+};
+
+struct Walk {
+  int k, tail, id, group, nb, split, c, c1, rot;
+  bool live;
+  __device__ __forceinline__ void open(const QArgs& a) {
+    int j = k * (int)gridDim.x + (int)blockIdx.x;
+    live = true;
+    tail = -1;
+    split = 0;
+    if (j < a.nfull) {
+      id = j;
+      c = 0;
+      c1 = a.nchunks;
+    } else {
+      // the CTAs of a cluster share the item (one each where nothing is cut), and it is their last
+      j = (k - a.nfull / (int)gridDim.x) * (int)gridDim.x + (int)blockIdx.x;
+      tail = j / a.splits;
+      split = j - tail * a.splits;
+      if (tail >= a.ntail) {
+        live = false;
+        return;
+      }
+      id = a.nfull + tail;
+      c = split * a.nchunks / a.splits;
+      c1 = (split + 1) * a.nchunks / a.splits;
+    }
+    group = id / a.nblocks;
+    nb = id - group * a.nblocks;
+    rot = (group * 5) % (c1 - c);
+  }
+  // The chunk to work on at step i of [c, c1): CTAs walk their K ranges in step, and starting every
+  // group of tiles at a chunk of its own keeps them from all asking the L2 for the same activation
+  // tile at the same moment.  (The sums are taken in this order; it is fixed per group.)
+  __device__ __forceinline__ int chunk(int i) const { return i + rot < c1 ? i + rot : i + rot - (c1 - c); }
+  __device__ __forceinline__ explicit Walk(const QArgs& a) : k(0) { open(a); }
+  __device__ __forceinline__ void next_item(const QArgs& a) {
+    ++k;
+    open(a);
+  }
+};
+
+template <int NB>
+__device__ __forceinline__ int block_cols(const QArgs& a, int nb) {
+  const int left = a.batch - nb * NB;
+  return left >= NB ? NB : (left + 15) & ~15;
+}
+
+// ---- activation preparation -------------------------------------------------------------------
+
+__device__ __forceinline__ uint32_t f16_bits(float v) { return (uint32_t)__half_as_ushort(__float2half_rn(v)); }
+
+// One CTA per activation row: its largest magnitude, then eight consecutive elements per thread and
+// step, one 16-byte core-matrix row per piece; a warp covers one 256-element chunk per step.
+template <int ORDER, int SUMS, bool XBF16>
+__global__ void __launch_bounds__(512)
+qg_prep_x_kernel(const void* __restrict__ xv, unsigned char* __restrict__ xb, unsigned char* __restrict__ xaux, float* __restrict__ xinv,
+                 unsigned char* __restrict__ flags, int batch, int in_dim, int nchunks, int NB, size_t xb_stride, float unit_inv) {
+  constexpr int P = XBF16 ? 1 : 3;
+  __shared__ float red[16];
+  const int m = blockIdx.x, tid = threadIdx.x, lane = tid & 31, nthr = blockDim.x;
+  const int nb = m / NB, j = m - nb * NB;
+  pdl_launch_dependents();
+  pdl_wait();  // x may be the output of the kernel in front; the tiles may still be read by it
+  auto load8 = [&](int k, float (&v)[8]) {
+    if (k >= in_dim) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = 0.f;
+    } else if (XBF16) {
+      const uint4 q = *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(xv) + (size_t)m * in_dim + k);
+      const uint32_t ws[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        v[2 * e] = __uint_as_float(ws[e] << 16);
+        v[2 * e + 1] = __uint_as_float(ws[e] & 0xFFFF0000u);
+      }
+    } else {
+      const float4* p = reinterpret_cast<const float4*>(static_cast<const float*>(xv) + (size_t)m * in_dim + k);
+      const float4 c = p[0], d = p[1];
+      v[0] = c.x; v[1] = c.y; v[2] = c.z; v[3] = c.w;
+      v[4] = d.x; v[5] = d.y; v[6] = d.z; v[7] = d.w;
+    }
+  };
+  float mx = 0.f;
+  for (int k = tid * 8; k < in_dim; k += nthr * 8) {
+    float v[8];
+    load8(k, v);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) mx = fmaxf(mx, fabsf(v[e]));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if (lane == 0) red[tid >> 5] = mx;
+  __syncthreads();
+  mx = red[0];
+  for (int i = 1; i < nthr / 32; ++i) mx = fmaxf(mx, red[i]);
+  // x * 2^s: the largest element lands in [2^14, 2^15)
+  int E = (int)((__float_as_uint(mx) >> 23) & 0xFFu) - 127;
+  if (mx == 0.f || E > 127) E = 14;  // an all-zero row, or inf / NaN in x (whose products are not finite anyway)
+  if (E < -112) E = -112;            // keeps 2^s a normal float
+  const float s = __uint_as_float((uint32_t)(14 - E + 127) << 23);
+  if (tid == 0) xinv[m] = __uint_as_float((uint32_t)(E - 14 + 127) << 23);
+  int n = batch - nb * NB;
+  n = n >= NB ? NB : (n + 15) & ~15;
+  for (int k = tid * 8; k < nchunks * kChunkK; k += nthr * 8) {
+    float v[8];
+    load8(k, v);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] *= s;
+    const int c = k >> 8, half = (k >> 7) & 1, step = (k >> 4) & 7, kh = (k >> 3) & 1;
+    if (SUMS != 0) {
+      // sums of x per scale group, as three bf16 pieces (exact): slots [piece][sum] of the affine term's
+      // K16 steps (four sums: 4 + 4 | 4 and zeros; eight: 8 | 8, then 8 | zeros)
+      constexpr int kG = SUMS == 1 ? 4 : 8, kPer = SUMS == 2 ? 4 : 8, kSteps = SUMS == 1 ? 1 : 2;
+      float t = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+      t += __shfl_xor_sync(0xffffffffu, t, 1);
+      t += __shfl_xor_sync(0xffffffffu, t, 2);
+      if (SUMS != 2) t += __shfl_xor_sync(0xffffffffu, t, 4);
+      t *= unit_inv;
+      uint32_t piece[3];
+#pragma unroll
+      for (int p = 0; p < 3; ++p) {
+        piece[p] = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(t));
+        t -= __uint_as_float(piece[p] << 16);
+      }
+      // lane l gathers slot l (of 16 or 32): sum l % kG, piece l / kG
+      const int src = (SUMS == 3 ? lane % 4 : lane % kG) * kPer;
+      const uint32_t g0 = __shfl_sync(0xffffffffu, piece[0], src), g1 = __shfl_sync(0xffffffffu, piece[1], src),
+                     g2 = __shfl_sync(0xffffffffu, piece[2], src);
+      const int pc = lane / kG;
+      uint32_t mine = pc == 0 ? g0 : pc == 1 ? g1 : pc == 2 ? g2 : 0u;
+      if (SUMS == 3 && (lane & 4)) mine = __float_as_uint(__uint_as_float(mine << 16) * 8.f) >> 16;  // exact
+      if (lane < 16 * kSteps)
+        *reinterpret_cast<unsigned short*>(xaux + ((size_t)nb * nchunks + c) * (kSteps * 32) * NB + (lane >> 4) * (n * 32) + ((lane >> 3) & 1) * (n * 16) +
+                                           (j >> 3) * 128 + (j & 7) * 16 + (lane & 7) * 2) = (unsigned short)mine;
+    }
+    if (ORDER == 2) {
+#pragma unroll
+      for (int e = 1; e < 8; e += 2) v[e] *= 0.0625f;
+    }
+    unsigned char* dst = xb + (size_t)nb * xb_stride + (size_t)(c * 2 + half) * P * n * 256 + step * (n * 32) + kh * (n * 16) + (j >> 3) * 128 + (j & 7) * 16;
+    int used = 1;
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      uint32_t h[8], any = 0;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        h[e] = f16_bits(v[e]);
+        any |= h[e] & 0x7FFFu;
+        v[e] -= __half2float(__ushort_as_half((unsigned short)h[e]));  // exact
+      }
+      uint32_t q[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) q[ORDER == 0 ? e : 2 * (e & 3) + (e >> 2)] = h[e];
+      *reinterpret_cast<uint4*>(dst + (size_t)p * n * 256) =
+          make_uint4(q[0] | (q[1] << 16), q[2] | (q[3] << 16), q[4] | (q[5] << 16), q[6] | (q[7] << 16));
+      if (P > 1 && p > 0 && __any_sync(0xffffffffu, any != 0)) used = p + 1;
+    }
+    if (P > 1 && lane == 0) flags[((size_t)nb * nchunks + c) * 64 + j] = (unsigned char)used;
+  }
+}
+
+// ---- the product kernel: pieces ------------------------------------------------------------------
+
+__device__ __forceinline__ uint32_t mul2(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+__device__ __forceinline__ uint32_t sub2(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+__device__ __forceinline__ uint32_t fma2h(uint32_t a, uint32_t b, uint32_t c) {
+  uint32_t d;
+  asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, int bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
+
+template <int N>
+__device__ __forceinline__ void reg_dec() {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
+}
+template <int N>
+__device__ __forceinline__ void reg_inc() {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+}
+
+// The row-major and streaming layouts: one chunk of one tile into a slot, by a warp (lt).
+template <int F>
+__device__ __forceinline__ void load_rows(const QArgs& a, uint32_t slot, int tile, int c, int lt) {
+  typedef QF<F, false> T;
+  const int row0 = tile * kTileRows;
+  const uint32_t meta = slot + T::kWBytes;
+  if (T::kMLX) {
+    const int G = a.in_dim / 64;
+    for (int i = lt; i < 1024; i += 32) {
+      const int r = i >> 3, u = i & 7;
+      const bool ok = row0 + r < a.out_dim && c * 256 + u * 32 < a.in_dim;
+      cp_async16(slot + r * 128 + ((u ^ (r & 7)) << 4), ok ? a.w + (size_t)(row0 + r) * (a.in_dim / 2) + c * 128 + u * 16 : a.w, ok);
+    }
+    for (int i = lt; i < 512; i += 32) {
+      const int r = i >> 2, g = i & 3;
+      const bool ok = row0 + r < a.out_dim && c * 4 + g < G;
+      const uint32_t* sb = static_cast<const uint32_t*>(a.aux);
+      cp_async4(meta + r * 16 + g * 4, ok ? sb + (size_t)(row0 + r) * G + c * 4 + g : sb, ok ? 4 : 0);
+    }
+  } else if (F == Q_Q4K) {
+    for (int i = lt; i < 128 * 9; i += 32) {
+      const int r = i / 9, u = i - r * 9;
+      const bool ok = row0 + r < a.out_dim;
+      const unsigned char* src = a.w + ((size_t)(ok ? row0 + r : 0) * a.nchunks + c) * 144;
+      if (u < 8) cp_async16(slot + r * 128 + ((u ^ (r & 7)) << 4), src + 16 + 16 * u, ok);
+      else cp_async16(meta + r * 16, src, ok);
+    }
+  } else if (F == Q_Q5K) {
+    for (int i = lt; i < 128 * 11; i += 32) {
+      const int r = i / 11, u = i - r * 11;
+      const bool ok = row0 + r < a.out_dim;
+      const unsigned char* src = a.w + ((size_t)(ok ? row0 + r : 0) * a.nchunks + c) * 176;
+      if (u < 8) cp_async16(slot + r * 128 + ((u ^ (r & 7)) << 4), src + 16 + 16 * u, ok);
+      else if (u == 8) cp_async16(meta + r * 16, src, ok);
+      else cp_async16(slot + T::kHighOff + (u - 9) * 2048 + r * 16, src + 144 + 16 * (u - 9), ok);
+    }
+  } else if (F == Q_Q6K) {
+    const size_t n = (size_t)a.out_dim * a.in_dim;
+    const unsigned char* hi = static_cast<const unsigned char*>(a.aux);
+    const unsigned char* sc = hi + n / 4;
+    const unsigned char* dd = sc + n / 16;
+    for (int i = lt; i < 128 * 14; i += 32) {
+      const int r = i / 14, u = i - r * 14;
+      const bool ok = row0 + r < a.out_dim;
+      const size_t row = ok ? row0 + r : 0;
+      if (u < 8) cp_async16(slot + r * 128 + ((u ^ (r & 7)) << 4), a.w + row * (a.in_dim / 2) + c * 128 + 16 * u, ok);
+      else if (u < 12) cp_async16(slot + T::kHighOff + (u - 8) * 2048 + r * 16, hi + row * (a.in_dim / 4) + c * 64 + 16 * (u - 8), ok);
+      else if (u == 12) cp_async16(meta + r * 32, sc + row * (a.in_dim / 16) + c * 16, ok);
+      else {  // the f16 d, in its aligned pair (the last one of an odd count stands alone)
+        const size_t h = row * a.nchunks + c, word = h >> 1, total = (size_t)a.out_dim * a.nchunks;
+        cp_async4(meta + r * 32 + 16, dd + word * 4, !ok ? 0 : 2 * word + 1 < total ? 4 : 2);
+      }
+    }
+  } else {  // a byte per weight
+    for (int i = lt; i < 2048; i += 32) {
+      const int r = i >> 4, U = i & 15;
+      const bool ok = row0 + r < a.out_dim && c * 256 + U * 16 < a.in_dim;
+      cp_async16(slot + U * 2048 + r * 16, ok ? a.w + (size_t)(row0 + r) * a.in_dim + c * 256 + U * 16 : a.w, ok);
+    }
+    if (F == Q_Q80) {  // the row's f16 scales from the aligned pair that holds the first one
+      const int nb = a.in_dim / 32;
+      const size_t total = (size_t)a.out_dim * nb;
+      for (int i = lt; i < 128 * 5; i += 32) {
+        const int r = i / 5, k = i - r * 5;
+        const size_t word = (((size_t)(row0 + r) * nb + c * 8) >> 1) + k;
+        const bool ok = row0 + r < a.out_dim && 2 * word < total;
+        const unsigned char* d = static_cast<const unsigned char*>(a.aux);
+        cp_async4(meta + r * 32 + k * 4, ok ? d + word * 4 : d, !ok ? 0 : 2 * word + 1 < total ? 4 : 2);
+      }
+    }
+  }
+}
+
+// Field of sub-block s (0..7, a constant after unrolling) of a K-quant header: scale | minimum << 6.
+__device__ __forceinline__ uint32_t kq_field(const uint4& h, int s) {
+  const int bit = 12 * s, wi = bit >> 5, sh = bit & 31;
+  const uint32_t lo = wi == 0 ? h.y : wi == 1 ? h.z : h.w;
+  const uint32_t hi = wi == 0 ? h.z : wi == 1 ? h.w : 0u;
+  return __funnelshift_r(lo, hi, sh) & 0xFFFu;
+}
+// The 6-bit scale as a pair of f16: times 2^10 (exact, at most 64512).
+__device__ __forceinline__ uint32_t kq_scale2(uint32_t field) {
+  const uint32_t v = field & 63u;
+  return mul2(sub2((v | (v << 16)) | 0x64006400u, 0x64006400u), 0x64006400u);
+}
+
+// 64 elements (quarter kq of half hh of the chunk) of row r: f16 values into the A buffer's columns at `abuf`.
+template <int F, bool TILED>
+__device__ __forceinline__ void convert_unit(const unsigned char* st, int r, int hh, int kq, uint32_t abuf) {
+  typedef QF<F, TILED> T;
+  uint4 head = make_uint4(0, 0, 0, 0);
+  if (F == Q_Q4K || F == Q_Q5K) head = *reinterpret_cast<const uint4*>(st + T::kWBytes + r * 16);
+  const int u0 = 4 * hh + 2 * kq;  // the first of two 32-element sub-blocks
+  uint32_t fs = 0;                 // MLX4F: the group's scale times 2^10, as a pair of f16 (exact)
+  if (F == Q_MLX4F) {
+    const uint32_t m = *reinterpret_cast<const uint32_t*>(st + T::kWBytes + r * 16 + (2 * hh + kq) * 4);
+    fs = f16_bits(__uint_as_float(m << 16) * 1024.f);
+    fs |= fs << 16;
+  }
+  if (T::kNibble) {
+    uint4 qv[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) qv[u] = *reinterpret_cast<const uint4*>(st + r * 128 + (((u0 + u) ^ (r & 7)) << 4));
+    uint2 hb = make_uint2(0, 0);       // Q5_K: fifth bits, a word per 32 elements
+    uint4 hv = make_uint4(0, 0, 0, 0);  // Q6_K: two bits per element, two words per 32
+    if (F == Q_Q5K) hb = *reinterpret_cast<const uint2*>(st + T::kHighOff + hh * 2048 + r * 16 + kq * 8);
+    if (F == Q_Q6K) hv = *reinterpret_cast<const uint4*>(st + T::kHighOff + (2 * hh + kq) * 2048 + r * 16);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const uint32_t ws[4] = {qv[u].x, qv[u].y, qv[u].z, qv[u].w};
+      uint32_t m0 = 0, m1 = 0;  // Q4_K, Q5_K: the sub-block's scale for nibbles read as n and as 16 n
+      if (F == Q_Q4K || F == Q_Q5K) {
+        m0 = kq_scale2(kq_field(head, u0 + u));
+        m1 = mul2(m0, 0x2C002C00u);  // / 16
+      }
+#pragma unroll
+      for (int s2 = 0; s2 < 2; ++s2) {
+        uint32_t regs[8];
+#pragma unroll
+        for (int wi = 0; wi < 2; ++wi) {
+          const uint32_t w = ws[2 * s2 + wi], w8 = w >> 8;
+          uint32_t e[4] = {w & 0x000F000Fu, w & 0x00F000F0u, w8 & 0x000F000Fu, w8 & 0x00F000F0u};
+          if (F == Q_MLX4F) {
+            // (n - 8) times the scale: 4 + 8 bits less one, exact
+            e[0] = mul2(sub2(e[0] | 0x64006400u, 0x64086408u), fs);               // 1024 + n
+            e[1] = mul2(fma2h(e[1] | 0x64006400u, 0x2C002C00u, 0xD480D480u), fs);  // (1024 + 16 n) / 16 - 72
+            e[2] = mul2(sub2(e[2] | 0x64006400u, 0x64086408u), fs);
+            e[3] = mul2(fma2h(e[3] | 0x64006400u, 0x2C002C00u, 0xD480D480u), fs);
+          } else if (F == Q_Q4K) {
+            e[0] = mul2(e[0], m0);
+            e[1] = mul2(e[1], m1);
+            e[2] = mul2(e[2], m0);
+            e[3] = mul2(e[3], m1);
+          } else if (F == Q_Q5K) {
+            // fifth bits of the word's eight elements, those of 0..3 in the low half and of 4..7 in the high half
+            const uint32_t b8 = ((u == 0 ? hb.x : hb.y) >> (8 * (2 * s2 + wi))) & 0xFFu, t = (b8 & 0xFu) | ((b8 >> 4) << 16);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const uint32_t n = (k & 1) ? e[k] >> 4 : e[k];
+              e[k] = mul2(n | (((t >> k) & 0x00010001u) << 4), m0);
+            }
+          } else if (F == Q_Q6K) {
+            // two bits of the word's eight elements: 0..3 in the low half, 4..7 in the high half
+            const uint32_t hw = u == 0 ? (s2 == 0 ? hv.x : hv.y) : (s2 == 0 ? hv.z : hv.w);
+            const uint32_t h16 = (hw >> (16 * wi)) & 0xFFFFu, t = (h16 & 0xFFu) | ((h16 >> 8) << 16);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const uint32_t n = (k & 1) ? e[k] >> 4 : e[k];
+              e[k] = sub2(n | (((t >> (2 * k)) & 0x00030003u) << 4) | 0x64006400u, 0x64206420u);  // (1024 + q) - 1056
+            }
+          }
+#pragma unroll
+          for (int k = 0; k < 4; ++k) regs[4 * wi + k] = e[k];
+        }
+        tmem_st8(abuf + (2 * u + s2) * 8, regs);
+      }
+    }
+  } else {
+    uint4 qv[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) qv[u] = *reinterpret_cast<const uint4*>(st + (8 * hh + 4 * kq + u) * 2048 + r * 16);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const uint32_t ws[4] = {qv[u].x, qv[u].y, qv[u].z, qv[u].w};
+      uint32_t m0 = 0;
+      if (F == Q_Q5K) m0 = kq_scale2(kq_field(head, u0 + (u >> 1)));
+      uint32_t regs[8];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        uint32_t w = ws[k];
+        if (F == Q_FP8) {
+          asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(regs[2 * k]) : "h"((unsigned short)(w & 0xFFFFu)));
+          asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(regs[2 * k + 1]) : "h"((unsigned short)(w >> 16)));
+        } else if (F == Q_Q5K) {
+          regs[2 * k] = mul2(__byte_perm(w, 0u, 0x4140), m0);
+          regs[2 * k + 1] = mul2(__byte_perm(w, 0u, 0x4342), m0);
+        } else {
+          if (TILED) w ^= 0x80808080u;  // signed bytes; the streaming layout keeps q + 128
+          regs[2 * k] = sub2(__byte_perm(w, 0x64646464u, 0x4140), 0x64806480u);  // (1024 + 128 + q) - 1152
+          regs[2 * k + 1] = sub2(__byte_perm(w, 0x64646464u, 0x4342), 0x64806480u);
+        }
+      }
+      tmem_st8(abuf + u * 8, regs);
+    }
+  }
+}
+
+// The affine term's A operand of row r: the chunk's biases (MLX4: four, twice; MLX4F: four biases and the
+// four scales that meet the 8 taken from every nibble) or minima (K-quants: eight) as eight bf16, in both
+// K halves of a K16 step.
+template <int F, bool TILED>
+__device__ __forceinline__ void convert_aux(const unsigned char* st, int r, unsigned char* dst) {
+  const uint4 h = *reinterpret_cast<const uint4*>(st + QF<F, TILED>::kWBytes + r * 16);
+  uint4 v;
+  if (F == Q_MLX4) {
+    v.x = v.z = __byte_perm(h.x, h.y, 0x7632);
+    v.y = v.w = __byte_perm(h.z, h.w, 0x7632);
+  } else if (F == Q_MLX4F) {
+    v.x = __byte_perm(h.x, h.y, 0x7632);
+    v.y = __byte_perm(h.z, h.w, 0x7632);
+    v.z = __byte_perm(h.x, h.y, 0x5410);
+    v.w = __byte_perm(h.z, h.w, 0x5410);
+  } else {
+    uint32_t b[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {  // small integers are exact in bf16
+      const uint32_t lo = __float_as_uint((float)(kq_field(h, 2 * k) >> 6)), hi = __float_as_uint((float)(kq_field(h, 2 * k + 1) >> 6));
+      b[k] = (lo >> 16) | (hi & 0xFFFF0000u);
+    }
+    v = make_uint4(b[0], b[1], b[2], b[3]);
+  }
+  unsigned char* d = dst + (r >> 3) * 128 + (r & 7) * 16;
+  *reinterpret_cast<uint4*>(d) = v;
+  *reinterpret_cast<uint4*>(d + 2048) = v;
+}
+// D[tmem] (+)= A[smem descriptor] * B[smem descriptor], 16-bit floats, f32 accumulate.
+__device__ __forceinline__ void umma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
+      : "memory");
+}
+
+// ---- the product kernel ----------------------------------------------------------------------------
+// TT: row tiles of an item; NB: activation rows of an item (columns of an accumulator block).
+// The work runs in two pipes, each with its converters, MMA warp, accumulators and epilogue warps: a
+// pipe takes one of the two tiles (TT = 2), or one half of every chunk (TT = 1; their sums meet in
+// shared memory when the item ends).  One issuing warp alone could not keep up: a wait that succeeds at
+// once still costs it over a hundred cycles, and an MMA forty.
+template <int F, bool TILED, int TT, int NB>
+__global__ void __launch_bounds__(kThreads, 1)
+qg_kernel(const __grid_constant__ QArgs a) {
+  typedef QF<F, TILED> T;
+  static_assert(NB == 64 || (NB == 128 && F == Q_FP8 && TT == 2), "wide blocks only where a block is read once per item");
+  constexpr bool kLong = T::kLong, kChunk = T::kChunk;
+  constexpr bool kItemBlock = kLong && NB == 128; // one per item, read straight to the result
+  // The tensor core's f32 sums drift towards zero with their length (0.6e-6 of the largest output at 8192
+  // elements): a block is closed and added in registers every 4096, an item of one block is kept to 8192
+  constexpr int kSeg = kItemBlock ? 1 << 20 : 16;
+  constexpr int DT = 128 / NB;                    // accumulator blocks of a pipe
+  constexpr int kPer = kLong || kChunk ? 1 : 128 / T::kBlk; // blocks (or the part of one) in a unit
+  constexpr int KS = 8 / kPer;                    // K16 steps of it
+  constexpr int UPC = TT == 2 ? 2 : 1;            // units a pipe takes of a chunk
+  constexpr int UB = kLong ? kSeg * UPC : kChunk ? UPC : 1;  // units of a block
+  constexpr int kAuxBytes = T::kAux ? 4 * 4096 : 0;  // the affine term's A operand, [pipe][2]
+  constexpr uint32_t kCols = 512;
+
+  extern __shared__ unsigned char smem_dyn[];
+  unsigned char* wring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
+  const int SW = a.wslots, SB = a.bslots;
+  unsigned char* bring = wring + (size_t)SW * T::kSlot;
+  unsigned char* aux = bring + (size_t)SB * a.bslot;
+  float* comb = reinterpret_cast<float*>(aux + kAuxBytes);  // TT = 1: [column][128] sums of pipe 1
+  uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(comb) + (TT == 1 ? a.comb : 0));
+  const uint32_t wfull = smem_u32(bars), wempty = wfull + 8 * SW, bfull = wempty + 8 * SW, bempty = bfull + 8 * SB;
+  const uint32_t aready = bempty + 8 * SB, afree = aready + 32, dfull = afree + 32, dfree = dfull + 32;  // [pipe][2] each
+  volatile int* pieces = reinterpret_cast<volatile int*>(bars + 2 * SW + 2 * SB + 16);  // [SB] pieces in the slot
+  uint32_t* tmem_holder = const_cast<uint32_t*>(reinterpret_cast<volatile uint32_t*>(pieces + SB));
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) {
+    for (int s = 0; s < SW; ++s) {
+      mbar_init(wfull + 8 * s, TILED ? 1 : 32);
+      mbar_init(wempty + 8 * s, (TT == 2 ? 1 : 2) * (8 + (kLong ? 0 : 4)));
+    }
+    for (int s = 0; s < SB; ++s) {
+      mbar_init(bfull + 8 * s, 1);
+      mbar_init(bempty + 8 * s, TT);
+    }
+    for (int s = 0; s < 4; ++s) {
+      mbar_init(aready + 8 * s, 8);
+      mbar_init(afree + 8 * s, 1);
+      mbar_init(dfull + 8 * s, 1);
+      mbar_init(dfree + 8 * s, 4);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == kWarpMMA) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_holder)), "r"(kCols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  pdl_launch_dependents();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_holder;  // A: columns [pipe][2][64], then D: [pipe][DT][NB]
+  bool ok = true;
+  Walk wk(a);
+  // is the affine term of the item's i-th chunk this pipe's, and with which unit of the chunk
+  auto aux_here = [&](int w, int i, int u) { return T::kAux != 0 && (TT == 2 ? u == 1 : (i & 1) == w); };
+
+  if (warp == kWarpW) {
+    // ------------------------------------------------------------------ weights
+    reg_dec<kMiscRegs>();
+    if (!TILED || lane == 0) {
+      auto slot_at = [&](int s) { return smem_u32(wring) + s * T::kSlot; };
+      auto tile_of = [&](int t) {  // the last group of an odd tile count repeats its tile (nothing of the copy is stored)
+        const int tile = wk.group * TT + t;
+        return tile < a.ntiles ? tile : a.ntiles - 1;
+      };
+      RingCursor cur;
+      int i = 0;
+      for (; wk.live && ok; wk.next_item(a)) {
+        for (int ci = wk.c; ci < wk.c1 && ok; ++ci) {
+          const int c = wk.chunk(ci);
+#pragma unroll 1
+          for (int t = 0; t < TT; ++t, ++i, cur.next(SW)) {
+            const int s = cur.s;
+            // The weights do not depend on the kernel in front.  Only the first two stages are asked for at
+            // once, the rest of the ring when the first is in (a grid that asked for all its rings at once
+            // would see every first stage land last).
+            if (i == 2) ok = mbar_wait(wfull, 0, a.status, 801);
+            if (ok && i >= SW) ok = mbar_wait(wempty + 8 * s, cur.ph ^ 1u, a.status, 802);
+            if (!ok) break;
+            if (lane == 0) { MARK(0, i); }
+            if (TILED) {
+              mbar_expect_tx(wfull + 8 * s, T::kSlot);
+              bulk_load_1d(slot_at(s), a.w + ((size_t)tile_of(t) * a.nchunks + c) * T::kSlot, T::kSlot, wfull + 8 * s);
+            } else {
+              load_rows<F>(a, slot_at(s), tile_of(t), c, lane);
+              cp_async_arrive(wfull + 8 * s);
+            }
+          }
+        }
+      }
+    }
+    if (!TILED) asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+  } else if (warp == kWarpB) {
+    // ------------------------------------------------------------------ prepared activations
+    reg_dec<kMiscRegs>();
+    pdl_wait();
+    RingCursor bc;
+    bool wrapped = false;
+    auto used_of = [&](const Walk& w, int c) -> uint32_t {  // most pieces any of the block's rows has in this chunk
+      if (!a.flags) return 1u;
+      const unsigned char* f = a.flags + ((size_t)w.nb * a.nchunks + c) * 64;
+      const int col = w.nb * NB + 2 * lane;
+      uint32_t v = 1;
+      if (col < a.batch) v = max(v, (uint32_t)__ldcg(f + 2 * lane));
+      if (col + 1 < a.batch) v = max(v, (uint32_t)__ldcg(f + 2 * lane + 1));
+      return v;
+    };
+    for (; wk.live && ok; wk.next_item(a)) {
+      const int n = block_cols<NB>(a, wk.nb);
+      const uint32_t bytes = n * 256;  // of a piece
+      const unsigned char* src = a.xb + (size_t)wk.nb * a.xb_stride;
+      const unsigned char* asrc = a.xaux + (size_t)wk.nb * a.nchunks * (T::kAux * 32 * NB);
+      uint32_t nxt = used_of(wk, wk.chunk(wk.c));
+      for (int ci = wk.c; ci < wk.c1 && ok; ++ci) {
+        const int c = wk.chunk(ci);
+        const uint32_t cur = nxt;
+        if (ci + 1 < wk.c1) nxt = used_of(wk, wk.chunk(ci + 1));
+        const int P = (int)__reduce_max_sync(0xffffffffu, cur);
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {
+          const int s = bc.s;
+          if (wrapped) ok = __all_sync(0xffffffffu, mbar_wait(bempty + 8 * s, bc.ph ^ 1u, a.status, 803));
+          if (!ok) break;
+          if (lane == 0) {
+            const bool ax = TT == 2 ? aux_here(0, 0, h) : aux_here(h, ci - wk.c, 0);
+            const uint32_t dst = smem_u32(bring) + s * a.bslot, axb = T::kAux * n * 32;
+            pieces[s] = P;
+            mbar_expect_tx(bfull + 8 * s, P * bytes + (ax ? axb : 0));
+            bulk_load_1d(dst, src + (size_t)(2 * c + h) * a.pmax * bytes, P * bytes, bfull + 8 * s);
+            if (ax) bulk_load_1d(dst + a.pmax * bytes, asrc + (size_t)c * (T::kAux * 32 * NB), axb, bfull + 8 * s);
+          }
+          __syncwarp();
+          bc.next(SB);
+          wrapped = wrapped || bc.s == 0;
+        }
+      }
+    }
+  } else if (warp >= kWarpMMA) {
+    // ------------------------------------------------------------------ MMA, a warp per pipe
+    reg_dec<kMiscRegs>();
+    const int w = warp - kWarpMMA;
+    RingCursor bc, ac, dc;  // B slots, A buffers (2), accumulator blocks (DT)
+    int used = 0;           // accumulator blocks opened so far, up to DT
+    if (TT == 1 && w == 1) bc.next(SB);
+    // (the masks: in a cluster launch a shared-memory address carries the CTA's rank above the 18 bits that descriptors hold)
+    const uint32_t bring_u = (smem_u32(bring) >> 4) & 0x3FFF, ar = aready + 16 * w, af = afree + 16 * w, df = dfull + 16 * w, de = dfree + 16 * w;
+    const uint32_t colA = tmem + w * 128, colD = tmem + 256 + w * (DT * NB);
+    TP(int mk = 0;)
+    // the next accumulator block is free (the epilogue has read what it held)
+    auto open_block = [&] {
+      if (used < DT) {
+        ++used;
+        return true;
+      }
+      const bool r = __all_sync(0xffffffffu, mbar_wait(de + 8 * dc.s, dc.ph ^ 1u, a.status, 807));
+      tc_fence_after();
+      return r;
+    };
+    for (; wk.live && ok; wk.next_item(a)) {
+      const int n = block_cols<NB>(a, wk.nb);
+      // instruction descriptor: D f32, A f16, B f16, both K-major, N = n, M = 128; the affine term's: A, B bf16
+      const uint32_t idesc = (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((128u >> 4) << 24), idesc_aux = idesc | (1u << 7) | (1u << 10);
+      const uint64_t desc_hi = ((uint64_t)((uint32_t)n) << 16) | ((uint64_t)(128u >> 4) << 32) | (1ull << 46);  // halves n * 16 B apart, row groups 128 B
+      const int units = (wk.c1 - wk.c) * UPC;
+      for (int i = 0; i < units; ++i) {
+        ok = mbar_wait(bfull + 8 * bc.s, bc.ph, a.status, 804) && mbar_wait(ar + 8 * ac.s, ac.ph, a.status, 806);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+        if (w == 0) { MARK(3, mk); }
+        const int P = pieces[bc.s];
+        const uint32_t blo = bring_u + ((bc.s * a.bslot) >> 4), acol = colA + ac.s * 64;
+        const bool opens = UB == 1 || i % UB == 0, closes = UB == 1 || i + 1 == units || (i + 1) % UB == 0;
+        const bool ax = aux_here(w, i / UPC, i % UPC);
+        const uint64_t adesc = ((uint64_t)(2048u >> 4) << 16) | ((uint64_t)(128u >> 4) << 32) | (1ull << 46) | (uint64_t)((smem_u32(aux + (w * 2 + ac.s) * 4096) >> 4) & 0x3FFF);
+#pragma unroll
+        for (int b = 0; b < kPer; ++b) {
+          if (opens) {
+            ok = open_block();
+            if (!ok) break;
+          }
+          if (elect_one()) {
+            const uint32_t dcol = colD + dc.s * NB;
+#pragma unroll
+            for (int p = 0; p < 3; ++p) {
+              if (p < P) {
+#pragma unroll
+                for (int k = 0; k < KS; ++k)
+                  umma_bf16_ts(dcol, acol + (b * KS + k) * 8, desc_hi | (uint64_t)(blo + (p * 8 + b * KS + k) * (n * 2)), idesc, !(opens && p == 0 && k == 0));
+              }
+            }
+            if (kLong && T::kAux != 0 && ax) {  // the affine term joins the open block
+#pragma unroll
+              for (int k = 0; k < T::kAux; ++k) umma_f16_ss(dcol, adesc, desc_hi | (uint64_t)(blo + a.pmax * (n * 16) + k * (n * 2)), idesc_aux, 1);
+            }
+            if (closes) umma_commit(df + 8 * dc.s);
+          }
+          __syncwarp();
+          if (closes) dc.next(DT);
+        }
+        if (!ok) break;
+        if (!kLong && T::kAux != 0 && ax) {
+          ok = open_block();
+          if (!ok) break;
+          if (elect_one()) {
+#pragma unroll
+            for (int k = 0; k < T::kAux; ++k)
+              umma_f16_ss(colD + dc.s * NB, adesc, desc_hi | (uint64_t)(blo + a.pmax * (n * 16) + k * (n * 2)), idesc_aux, k != 0);
+            umma_commit(df + 8 * dc.s);
+          }
+          __syncwarp();
+          dc.next(DT);
+        }
+        if (elect_one()) {
+          umma_commit(af + 8 * ac.s);
+          umma_commit(bempty + 8 * bc.s);
+        }
+        __syncwarp();
+        if (w == 0) { MARK(4, mk); }
+        TP(++mk;)
+        ac.next(2);
+        bc.next(SB);
+        if (TT == 1) bc.next(SB);
+      }
+    }
+  } else if (warp < kConvWarps) {
+    // ------------------------------------------------------------------ converters, eight warps per pipe: (row, half a unit)
+    reg_dec<kConvRegs>();
+    const int w = warp >> 3, kq = (warp >> 2) & 1, q4 = warp & 3, r = q4 * 32 + lane;
+    RingCursor wc, ac;
+    int filled = 0;
+    if (TT == 2 && w == 1) wc.next(SW);
+    const uint32_t abase = tmem + ((uint32_t)(q4 * 32) << 16) + w * 128 + kq * 32, ar = aready + 16 * w, af = afree + 16 * w;
+    TP(int mk = 0;)
+    for (; wk.live && ok; wk.next_item(a)) {
+      for (int ci = wk.c; ci < wk.c1 && ok; ++ci) {
+        ok = __all_sync(0xffffffffu, mbar_wait(wfull + 8 * wc.s, wc.ph, a.status, 808));
+        if (!ok) break;
+        const unsigned char* st = wring + wc.s * T::kSlot;
+#pragma unroll 1
+        for (int h = 0; h < UPC; ++h) {
+          if (filled == 2) ok = __all_sync(0xffffffffu, mbar_wait(af + 8 * ac.s, ac.ph ^ 1u, a.status, 809));
+          else ++filled;
+          if (!ok) break;
+          tc_fence_after();
+          if (warp == 0) { MARK(1, mk); }
+          if (T::kAux != 0 && kq == 1 && aux_here(w, ci - wk.c, h)) {
+            convert_aux<F, TILED>(st, r, aux + (w * 2 + ac.s) * 4096);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the MMA reads it through the async proxy
+          }
+          convert_unit<F, TILED>(st, r, TT == 2 ? h : w, kq, abase + ac.s * 64);
+          tmem_wait_st();
+          tc_fence_before();
+          warp_arrive(ar + 8 * ac.s, lane);
+          if (warp == 0) { MARK(2, mk); }
+          TP(++mk;)
+          ac.next(2);
+        }
+        if (ok) warp_arrive(wempty + 8 * wc.s, lane);
+        wc.next(SW);
+        if (TT == 2) wc.next(SW);
+      }
+    }
+  } else {
+    // ------------------------------------------------------------------ epilogue, four warps per pipe: a row's NB columns per thread
+    reg_inc<kEpiRegs>();
+    const int e = warp - kConvWarps, q4 = warp & 3, w = e >> 2;
+    const int r = q4 * 32 + lane, t = TT == 2 ? w : 0;
+    const uint32_t dbase = tmem + 256 + ((uint32_t)(q4 * 32) << 16) + w * (DT * NB), df = dfull + 16 * w, de = dfree + 16 * w;
+    RingCursor wc, dc;
+    if (TT == 2 && w == 1) wc.next(SW);
+    TP(int mk = 0;)
+    float2 acc[kItemBlock ? 1 : NB / 2];
+    pdl_wait();  // the activations' scales come from the preparation kernel in front
+    for (; wk.live; wk.next_item(a)) {
+      const int n = block_cols<NB>(a, wk.nb);
+      const int row = (wk.group * TT + t) * kTileRows + r;
+      float rs = 1.f, rb = 0.f;
+      if (F == Q_FP8 && row < a.out_dim) {
+        rs = __ldg(a.scale + row);
+        if (a.bias) rb = __ldg(a.bias + row);
+      }
+      auto store = [&](int j, float v) {  // activation row j of the block
+        const int m = wk.nb * NB + j;
+        if (m < a.batch && row < a.out_dim) {
+          v = (v * T::kUnit) * __ldg(a.xinv + m);
+          a.out[(size_t)m * a.out_dim + row] = F == Q_FP8 ? fmaf(v, rs, rb) : v;
+        }
+      };
+      if (kItemBlock) {
+        if (ok) ok = __all_sync(0xffffffffu, mbar_wait(df + 8 * dc.s, dc.ph, a.status, 810));
+        if (ok) {
+          tc_fence_after();
+#pragma unroll 1
+          for (int j0 = 0; j0 < n; j0 += 16) {
+            uint32_t d[16];
+            tmem_ld16(dbase + dc.s * NB + j0, d);
+            tmem_wait_ld(d);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              if (a.splits > 1 && wk.tail >= 0) break;
+              store(j0 + j, __uint_as_float(d[j]));
+            }
+          }
+          tc_fence_before();
+          warp_arrive(de + 8 * dc.s, lane);
+        }
+        dc.next(DT);
+      } else {
+#pragma unroll
+        for (int j = 0; j < NB / 2; ++j) acc[j] = make_float2(0.f, 0.f);
+        // one accumulator block: read, released, added times sc
+        auto take = [&](float sc) {
+          ok = __all_sync(0xffffffffu, mbar_wait(df + 8 * dc.s, dc.ph, a.status, 812));
+          if (!ok) return;
+          tc_fence_after();
+          if (e == 0) { MARK(5, mk); }
+          const float2 sc2 = make_float2(sc, sc);
+#pragma unroll
+          for (int j0 = 0; j0 < NB; j0 += 32) {
+            if (j0 < n) {
+              uint32_t d[2][16];
+              tmem_ld16(dbase + dc.s * NB + j0, d[0]);
+              tmem_ld16(dbase + dc.s * NB + j0 + 16, d[1]);
+              tmem_wait_ld(d[0]);
+              tmem_wait_ld(d[1]);
+              if (j0 + 32 >= n) {
+                tc_fence_before();
+                warp_arrive(de + 8 * dc.s, lane);
+              }
+#pragma unroll
+              for (int j = 0; j < 16; ++j)
+                fma2(acc[j0 / 2 + j], sc2, make_float2(__uint_as_float(d[j / 8][(2 * j) & 15]), __uint_as_float(d[j / 8][(2 * j + 1) & 15])));
+            }
+          }
+          dc.next(DT);
+          if (e == 0) { MARK(6, mk); }
+          TP(++mk;)
+        };
+        const int chunks = wk.c1 - wk.c;
+        if (kLong) {
+          for (int ci = 0; ci < chunks && ok; ci += kSeg) take(1.f);
+        } else {
+          for (int ci = 0; ci < chunks && ok; ++ci) {
+            ok = __all_sync(0xffffffffu, mbar_wait(wfull + 8 * wc.s, wc.ph, a.status, 811));
+            if (!ok) break;
+            const unsigned char* mrow = wring + wc.s * T::kSlot + T::kWBytes + r * T::kMeta;
+            uint4 mv = *reinterpret_cast<const uint4*>(mrow);
+            uint32_t m4 = 0;  // Q6_K: d; streaming Q8_0: the fifth pair of scales
+            if (F == Q_Q6K || (F == Q_Q80 && !TILED)) m4 = *reinterpret_cast<const uint32_t*>(mrow + 16);
+            // the metadata is in registers (the reduction consumes it): the slot is free for the next load
+            if (__reduce_or_sync(0xffffffffu, mv.x | mv.y | mv.z | mv.w | m4 | 1u) && lane == 0) mbar_arrive(wempty + 8 * wc.s);
+            wc.next(SW);
+            if (TT == 2) wc.next(SW);
+            const int c = wk.chunk(wk.c + ci);
+            if (F == Q_Q6K && !TILED) m4 >>= 16 * (int)(((size_t)row * a.nchunks + c) & 1);
+            if (F == Q_Q80 && !TILED) {
+              if (((size_t)row * (a.in_dim / 32)) & 1) {  // the row's scales start in the middle of a pair
+                mv = make_uint4(__funnelshift_r(mv.x, mv.y, 16), __funnelshift_r(mv.y, mv.z, 16), __funnelshift_r(mv.z, mv.w, 16),
+                                __funnelshift_r(mv.w, m4, 16));
+              }
+            }
+            auto word = [&](int k) { return k == 0 ? mv.x : k == 1 ? mv.y : k == 2 ? mv.z : mv.w; };
+#pragma unroll 1
+            for (int u = kChunk ? UPC - 1 : 0; u < UPC && ok; ++u) {
+              const int b0 = (TT == 2 ? u : w) * kPer;  // the unit's first block in the chunk
+#pragma unroll 1
+              for (int k = 0; k < kPer && ok; ++k) {
+                const int b = b0 + k;
+                float sc;
+                if (F == Q_MLX4) {
+                  sc = __uint_as_float(word(b) << 16);
+                } else if (F == Q_Q80) {
+                  sc = __half2float(__ushort_as_half((unsigned short)(word(b >> 1) >> (16 * (b & 1)))));
+                  if (!TILED && c * 8 + b >= a.in_dim / 32) sc = 0.f;  // past the row: no scale of its own
+                } else if (F == Q_Q6K) {
+                  const float q = (float)(signed char)((word(b >> 2) >> (8 * (b & 3))) & 0xFFu);
+                  sc = __fmul_rn(__half2float(__ushort_as_half((unsigned short)(m4 & 0xFFFFu))), q);  // d * scale, rounded as dequantRowQ6K does
+                } else {
+                  sc = __half2float(__ushort_as_half((unsigned short)(mv.x & 0xFFFFu)));
+                }
+                take(sc);
+              }
+              // the affine term: biases times sums of x, or minus dmin times (minima times sums of x)
+              if (T::kAux != 0 && ok && aux_here(w, ci, u))
+                take(F == Q_MLX4 ? 1.f : -__half2float(__ushort_as_half((unsigned short)(mv.x >> 16))));
+            }
+          }
+        }
+      }
+      // ---- the item is complete (every epilogue warp comes through here, waits given up or not) ----
+      if (a.splits > 1 && wk.tail >= 0) break;  // the CTA's last item, shared with the cluster: below
+      if constexpr (!kItemBlock) {
+        if (TT == 1) {  // the pipes' sums: pipe 1 hands its own over through shared memory
+          if (w == 1) {
+#pragma unroll
+            for (int j = 0; j < NB; ++j)
+              if (j < n) comb[j * kTileRows + r] = (j & 1) ? acc[j / 2].y : acc[j / 2].x;
+          }
+          asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
+        }
+        if (ok && (TT == 2 || w == 0)) {
+#pragma unroll
+          for (int j = 0; j < NB; ++j)
+            if (j < n) store(j, ((j & 1) ? acc[j / 2].y : acc[j / 2].x) + (TT == 1 ? comb[j * kTileRows + r] : 0.f));
+        }
+        if (TT == 1) asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
+      }
+    }
+    if (a.splits > 1) {
+      // The K splits of the last item are the CTAs of this cluster (rank == split).  Nothing is in flight in
+      // the rings any more, here or (after the first meeting) in the peers: each thread hands its sums to
+      // the CTAs that finish the columns, a share of them each, which add in split order and store.
+      cluster_sync_all();
+      const int n = block_cols<NB>(a, wk.nb), S = a.splits, share = (n + S - 1) / S;
+      constexpr int kSrc = TT == 1 ? 2 : 1;  // sources per split
+      if (wk.live) {
+        const uint32_t at = smem_u32(wring) + (uint32_t)(((wk.split * kSrc + (TT == 1 ? w : 0)) * TT + t) * share * kTileRows + r) * 4;
+        if constexpr (kItemBlock) {
+          // (the block is still in TMEM: nothing has been opened after it)
+          RingCursor last = dc;
+          const uint32_t d0 = dbase + (DT == 1 ? 0 : (last.s ^ 1) * NB);
+          tc_fence_after();
+          int owner = 0, left = share;
+          uint32_t dst = cluster_map(at, 0);
+#pragma unroll 1
+          for (int j0 = 0; j0 < n; j0 += 16) {
+            uint32_t d[16];
+            tmem_ld16(d0 + j0, d);
+            tmem_wait_ld(d);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              cluster_store_f32(dst, __uint_as_float(d[j]));
+              dst += kTileRows * 4;
+              if (--left == 0 && ++owner < S) {
+                left = share;
+                dst = cluster_map(at, owner);
+              }
+            }
+          }
+        } else {
+          int owner = 0, left = share;
+          uint32_t dst = cluster_map(at, 0);
+#pragma unroll
+          for (int j = 0; j < NB; ++j) {
+            if (j < n) {
+              cluster_store_f32(dst, (j & 1) ? acc[j / 2].y : acc[j / 2].x);
+              dst += kTileRows * 4;
+              if (--left == 0 && ++owner < S) {
+                left = share;
+                dst = cluster_map(at, owner);
+              }
+            }
+          }
+        }
+      }
+      cluster_sync_all();
+      if (wk.live && ok) {
+        const int row = (wk.group * TT + t) * kTileRows + r, c0 = wk.split * share;
+        const float rs = F == Q_FP8 && row < a.out_dim ? __ldg(a.scale + row) : 1.f, rb = F == Q_FP8 && a.bias && row < a.out_dim ? __ldg(a.bias + row) : 0.f;
+        const float* in = reinterpret_cast<const float*>(wring) + (size_t)t * share * kTileRows + r;
+        for (int j = TT == 1 ? w : 0; j < share; j += TT == 1 ? 2 : 1) {
+          const int m = wk.nb * NB + c0 + j;
+          if (c0 + j >= n || m >= a.batch || row >= a.out_dim) break;
+          float v = 0.f;
+          for (int s2 = 0; s2 < S * kSrc; ++s2) v += in[(size_t)(s2 * TT * share + j) * kTileRows];
+          v = (v * T::kUnit) * __ldg(a.xinv + m);
+          a.out[(size_t)m * a.out_dim + row] = F == Q_FP8 ? fmaf(v, rs, rb) : v;
+        }
+      }
+    }
+  }
+  if (a.splits > 1 && (warp < kConvWarps || warp >= kWarpMMA)) {  // the other roles meet the cluster too
+    __syncwarp();
+    cluster_sync_all();
+    cluster_sync_all();
+  }
+  // ---- wind down: everyone meets, outstanding copies are drained, TMEM is returned ----
+  tc_fence_before();
+  __syncthreads();
+  if (warp == kWarpB && lane == 0 && *reinterpret_cast<volatile int*>(a.status) != 0) {
+    // a waiter gave up: bulk copies may still be in flight; give every slot a bounded chance to land
+    for (int s = 0; s < SW + SB; ++s) {
+      const uint32_t bar = s < SW ? wfull + 8 * s : bfull + 8 * (s - SW);
+      long long t0 = clock64();
+      while (!mbar_try_wait(bar, 0) && !mbar_try_wait(bar, 1) && clock64() - t0 < kTimeoutCycles / 8) {
+      }
+    }
+  }
+  __syncthreads();
+  if (warp == kWarpMMA) {
+    __syncwarp();
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
+  }
+}
+
+// ---- host side ---------------------------------------------------------------------------------------
+
+constexpr int kMaxIn = 65536;
+constexpr int kMaxRows = 256;                       // activation rows of one launch
+constexpr size_t kXbBytes = (size_t)64 << 20;       // prepared activations
+constexpr size_t kXauxBytes = (size_t)(kMaxRows / 64) * (kMaxIn / kChunkK) * 64 * 64;
+constexpr size_t kFlagBytes = (size_t)(kMaxRows / 64) * (kMaxIn / kChunkK) * 64;
+constexpr size_t kSmemBudget2 = 227 * 1024;         // all that a CTA may have
+
+struct QBufs {
+  unsigned char* xb = nullptr;
+  unsigned char* xaux = nullptr;
+  float* xinv = nullptr;
+  unsigned char* flags = nullptr;
+  int* status = nullptr;
+};
+
+// Allocated on a device's first product of this kind; published only when complete.
+QBufs* q_bufs(int device, bool allocate = true) {
+  static QBufs bufs[kMaxDevices];
+  static bool ready[kMaxDevices] = {};
+  static std::mutex mu;
+  if (device < 0 || device >= kMaxDevices) return nullptr;
+  std::lock_guard<std::mutex> lock(mu);
+  if (ready[device]) return &bufs[device];
+  if (!allocate) return nullptr;
+  QBufs b;
+  bool ok = cudaMalloc(&b.xb, kXbBytes) == cudaSuccess && cudaMalloc(&b.xaux, kXauxBytes) == cudaSuccess &&
+            cudaMalloc(&b.xinv, kMaxRows * 4) == cudaSuccess && cudaMalloc(&b.flags, kFlagBytes) == cudaSuccess &&
+            cudaMalloc(&b.status, 256) == cudaSuccess;
+  ok = ok && cudaMemset(b.status, 0, 256) == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess;
+  if (!ok) {
+    cudaGetLastError();
+    cudaFree(b.xb);
+    cudaFree(b.xaux);
+    cudaFree(b.xinv);
+    cudaFree(b.flags);
+    cudaFree(b.status);
+    return nullptr;
+  }
+  bufs[device] = b;
+  ready[device] = true;
+  return &bufs[device];
+}
+
+// Clusters of `size` CTAs that the device holds at once (every CTA takes a whole SM, so this is a
+// property of how the SMs are grouped); asked once per device and size.
+int cluster_room(int device, int size) {
+  static std::mutex mu;
+  static int room[kMaxDevices][kMaxSplits + 1];
+  static bool known[kMaxDevices][kMaxSplits + 1] = {};
+  if (size == 1) return device_state(device).sm_count;
+  std::lock_guard<std::mutex> lock(mu);
+  if (!known[device][size]) {
+    auto kern = qg_kernel<Q_MLX4, true, 1, 64>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget2);
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = size;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof cfg);
+    cfg.gridDim = dim3(size * 16);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = kSmemBudget2;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    room[device][size] = n;
+    known[device][size] = true;
+  }
+  return room[device][size];
+}
+
+// How a launch is cut up: row tiles per item, whole items (a multiple of the grid), the items after
+// them and the CTAs that share each of these.
+struct Plan {
+  int TT, grid, nfull, ntail, splits;
+};
+
+// The plan with the smallest estimate, in cycles of the busiest SM.  A chunk of an item takes the
+// largest of the tensor pipe's time (half a cycle per column and K16 step), the converters' (300
+// cycles a tile) and what the L2 can hand to one SM (45 bytes a cycle); sharing the last items costs two
+// meetings of the cluster and the exchange.  max_chunks: longest K range of an item.
+bool choose_plan(int device, int ntiles, int nchunks, int nblocks, int n, int pieces, int wbytes, int NB, int max_chunks, Plan* best) {
+  double best_cost = -1;
+  for (int TT = NB == 128 ? 2 : 1; TT <= 2; ++TT) {
+    if (TT == 2 && ntiles < 2) break;
+    const int items = (ntiles + TT - 1) / TT * nblocks;
+    const double mma = TT * 8.0 * pieces * n, conv = 300.0 * TT, mem = (TT * (double)wbytes + pieces * n * 512.0) / 45;
+    const double chunk = mma > conv ? (mma > mem ? mma : mem) : (conv > mem ? conv : mem);
+    for (int S = 1; S <= kMaxSplits && S <= nchunks; ++S) {
+      if (S > 1 && !options().mlx_cluster) break;
+      const int clusters = cluster_room(device, S);
+      if (clusters < 1) continue;
+      const int grid = clusters * S;
+      const int nfull = items / grid * grid, ntail = items - nfull;
+      if (ntail > clusters || (S > 1 && ntail == 0)) continue;  // the shared items are the last thing a cluster does
+      if ((nfull && nchunks > max_chunks) || (ntail && (nchunks + S - 1) / S > max_chunks)) continue;
+      const double cost = (nfull / grid * (nchunks * chunk + 1500.0)) + (ntail ? (nchunks + S - 1) / S * chunk + 1500.0 : 0) + (S > 1 ? 1500.0 + TT * n * 8.0 : 0);
+      if (best_cost < 0 || cost < best_cost) {
+        best_cost = cost;
+        *best = Plan{TT, nfull ? grid : ntail * S, nfull, ntail, S};
+      }
+    }
+  }
+  return best_cost >= 0;
+}
+
+template <int F, bool TILED, int TT, int NB>
+int launch_product(QArgs& a, const Plan& p, int n, int device, cudaStream_t stream) {
+  typedef QF<F, TILED> T;
+  // B slots hold every piece of half a chunk and the affine term's sums: two at least, more where they are
+  // small; the weight ring gets the rest
+  a.bslot = n * 256 * a.pmax + T::kAux * n * 32;
+  a.comb = TT == 1 ? n * kTileRows * 4 : 0;
+  a.bslots = (int)((size_t)(NB == 128 ? 96 : 104) * 1024 / a.bslot);
+  if (a.bslots > 6) a.bslots = 6;
+  // A pipe must see every round of the slots that it waits for (a parity wait cannot tell a round from the
+  // one two before it): where the pipes take turns, their slots stay apart by an even depth.
+  if (TT == 1) a.bslots &= ~1;
+  const size_t fixed = 1024 + 1024 + (size_t)a.bslots * a.bslot + a.comb + (T::kAux ? 4 * 4096 : 0);
+  a.wslots = (int)((kSmemBudget2 - fixed) / T::kSlot);
+  if (a.wslots > 10) a.wslots = 10;
+  if (TT == 2) a.wslots &= ~1;
+  if (a.wslots < 2 || a.bslots < 2) return fail(GOPH_E_UNSUPPORTED, "several-row products: no room for the rings");
+  size_t smem = fixed + (size_t)a.wslots * T::kSlot;
+  if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM (the kernel owns all of TMEM)
+  auto kern = qg_kernel<F, TILED, TT, NB>;
+  static bool sized[kMaxDevices] = {};
+  if (!sized[device]) {
+    GOPH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget2));
+    sized[device] = true;
+  }
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = options().pdl ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = p.splits;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof cfg);
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = p.splits > 1 ? 2 : 1;
+  cfg.gridDim = dim3(p.grid);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  note_launch();
+  GOPH_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
+  return GOPH_OK;
+}
+
+template <int F, bool TILED, bool XBF16>
+int run_rows(const QWeight& w, float* out, const void* x, int batch, cudaStream_t stream) {
+  typedef QF<F, TILED> T;
+  QBufs* bufs = q_bufs(w.device);
+  if (!bufs) return fail(GOPH_E_NOMEM, "cannot allocate the several-row products' device scratch");
+  constexpr int pmax = XBF16 ? 1 : 3;
+  const int nchunks = (w.in_dim + kChunkK - 1) / kChunkK;
+  const size_t xstride = (size_t)w.in_dim * (XBF16 ? 2 : 4);
+  for (int b0 = 0; b0 < batch;) {
+    // wide column blocks halve the weight traffic where one is read out once per item
+    int NB = F == Q_FP8 && TILED && XBF16 && batch - b0 > 64 ? 128 : 64;
+    Plan p;
+    if (NB == 128) {
+      const int rows = batch - b0 < kMaxRows ? batch - b0 : kMaxRows;
+      if (!choose_plan(w.device, (w.out_dim + kTileRows - 1) / kTileRows, nchunks, (rows + 127) / 128, rows < 128 ? (rows + 15) & ~15 : 128, 1, T::kSlot, NB, 32, &p))
+        NB = 64;
+    }
+    const size_t block_bytes = (size_t)NB * nchunks * kChunkK * 2 * pmax;
+    int cap = (int)(kXbBytes / block_bytes) * NB;
+    if (cap > kMaxRows) cap = kMaxRows;
+    const int rows = batch - b0 < cap ? batch - b0 : cap;
+    QArgs a;
+    memset(&a, 0, sizeof a);
+    a.w = static_cast<const unsigned char*>(w.w);
+    a.aux = w.aux;
+    a.xb = bufs->xb;
+    a.xaux = bufs->xaux;
+    a.xinv = bufs->xinv;
+    a.flags = XBF16 ? nullptr : bufs->flags;
+    a.scale = w.scale;
+    a.bias = w.bias;
+    a.out = out + (size_t)b0 * w.out_dim;
+    a.status = bufs->status;
+    a.xb_stride = block_bytes;
+    a.out_dim = w.out_dim;
+    a.in_dim = w.in_dim;
+    a.batch = rows;
+    a.ntiles = (w.out_dim + kTileRows - 1) / kTileRows;
+    a.nchunks = nchunks;
+    a.nblocks = (rows + NB - 1) / NB;
+    a.pmax = pmax;
+    const int n = rows >= NB ? NB : (rows + 15) & ~15;  // columns of the first (widest) block
+    if (!choose_plan(w.device, a.ntiles, nchunks, a.nblocks, n, T::kMLX ? 1 : pmax, T::kSlot, NB, NB == 128 ? 32 : 1 << 20, &p))
+      return fail(GOPH_E_UNSUPPORTED, "several-row products: the device holds no CTA of this kernel");
+    a.nfull = p.nfull;
+    a.ntail = p.ntail;
+    a.splits = p.splits;
+
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = options().pdl ? 1 : 0;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof cfg);
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cfg.gridDim = dim3(rows);
+    const int want = nchunks * 32;  // a warp per chunk
+    cfg.blockDim = dim3(want < 512 ? want : 512);
+    note_launch();
+    GOPH_CUDA(cudaLaunchKernelEx(&cfg, qg_prep_x_kernel<T::kOrder, T::kSums, XBF16>,
+                                 static_cast<const void*>(static_cast<const unsigned char*>(x) + (size_t)b0 * xstride), bufs->xb,
+                                 bufs->xaux, bufs->xinv, bufs->flags, rows, w.in_dim, nchunks, NB, a.xb_stride, 1.f / T::kUnit));
+    int rc;
+    if constexpr (F == Q_FP8 && TILED && XBF16) {
+      if (NB == 128) rc = launch_product<F, TILED, 2, 128>(a, p, n, w.device, stream);
+      else rc = p.TT == 2 ? launch_product<F, TILED, 2, 64>(a, p, n, w.device, stream) : launch_product<F, TILED, 1, 64>(a, p, n, w.device, stream);
+    } else {
+      rc = p.TT == 2 ? launch_product<F, TILED, 2, 64>(a, p, n, w.device, stream) : launch_product<F, TILED, 1, 64>(a, p, n, w.device, stream);
+    }
+    if (rc) return rc;
+    b0 += rows;
+  }
+  return GOPH_OK;
+}
+
+template <int F>
+int run_fmt(const QWeight& w, float* out, const void* x, bool x_bf16, int batch, cudaStream_t stream) {
+  if constexpr (F == Q_MLX4 || F == Q_MLX4F || F == Q_FP8) {
+    if (x_bf16)
+      return w.tiled ? run_rows<F, true, true>(w, out, x, batch, stream) : fail(GOPH_E_UNSUPPORTED, "bf16 activations need the tiled layout");
+  } else if (x_bf16) {
+    return fail(GOPH_E_UNSUPPORTED, "bf16 activations: MLX 4-bit and FP8 only");
+  }
+  return w.tiled ? run_rows<F, true, false>(w, out, x, batch, stream) : run_rows<F, false, false>(w, out, x, batch, stream);
+}
+
+}  // namespace
+
+int qgemm(const QWeight& w, float* out, const void* x, bool x_bf16, int batch, cudaStream_t stream) {
+  if (w.in_dim > kMaxIn) return fail(GOPH_E_UNSUPPORTED, "several-row products: in_dim=%d is above %d", w.in_dim, kMaxIn);
+  if ((uintptr_t)x % 16) return fail(GOPH_E_INVALID, "x must be 16-byte aligned");
+  switch (w.fmt) {
+    case Q_MLX4: return run_fmt<Q_MLX4>(w, out, x, x_bf16, batch, stream);
+    case Q_MLX4F: return run_fmt<Q_MLX4F>(w, out, x, x_bf16, batch, stream);
+    case Q_Q4K: return run_fmt<Q_Q4K>(w, out, x, x_bf16, batch, stream);
+    case Q_Q5K: return run_fmt<Q_Q5K>(w, out, x, x_bf16, batch, stream);
+    case Q_Q6K: return run_fmt<Q_Q6K>(w, out, x, x_bf16, batch, stream);
+    case Q_Q80: return run_fmt<Q_Q80>(w, out, x, x_bf16, batch, stream);
+    case Q_FP8: return run_fmt<Q_FP8>(w, out, x, x_bf16, batch, stream);
+  }
+  return fail(GOPH_E_INVALID, "unknown weight format %d", w.fmt);
+}
+
+int qgemm_status(int device) {
+  QBufs* b = q_bufs(device, false);
+  if (!b) return 0;
+  int v = -1;
+  cudaMemcpy(&v, b->status, sizeof v, cudaMemcpyDeviceToHost);
+  return v;
+}
+
+void qgemm_status_clear(int device) {
+  QBufs* b = q_bufs(device, false);
+  if (b) cudaMemset(b->status, 0, sizeof(int));
+}
+
+}  // namespace goph
+
+#ifdef GOPH_TUNING
+GOPH_API int goph_tuning_probe_q(long long* out512) {
+  return cudaMemcpyFromSymbol(out512, goph::g_qg_trace, 8 * 64 * sizeof(long long)) == cudaSuccess ? 0 : -1;
+}
+#endif

@@ -1,0 +1,32 @@
+// Quantised weights times several activation rows (prefill chunks, verifier batches) on the tensor
+// cores, for every weight format and both device layouts; implemented in qgemm.cu.
+#pragma once
+
+#include "goph_internal.cuh"
+
+namespace goph {
+
+// Q_MLX4F: MLX 4-bit weights whose scales are zero or of magnitude 2^-27 to 7.875 (goph_mlx_weight::foldable)
+enum QFormat { Q_MLX4 = 0, Q_Q4K = 1, Q_Q5K = 2, Q_Q6K = 3, Q_Q80 = 4, Q_FP8 = 5, Q_MLX4F = 6 };
+
+// A weight matrix as the kernel sees it.  tiled: `w` is the format's tiled layout; else `w` and `aux`
+// are the row-major / streaming layout's buffers (MLX: words and the bf16 {scale,bias} table; Q4_K,
+// Q5_K: blocks; Q6_K: low nibbles, and the highs, scales and d one plane after another; Q8_0: biased
+// bytes and f16 scales; FP8: bytes).
+struct QWeight {
+  int fmt;
+  bool tiled;
+  const void* w;
+  const void* aux;
+  const float* scale;  // FP8: [out_dim]
+  const float* bias;   // FP8: [out_dim] or nullptr
+  int device, out_dim, in_dim;
+};
+
+// out [batch][out_dim] = x [batch][in_dim] . W^T, x f32 or bf16 bit patterns, 16-byte aligned.
+int qgemm(const QWeight& w, float* out, const void* x, bool x_bf16, int batch, cudaStream_t stream);
+
+int qgemm_status(int device);
+void qgemm_status_clear(int device);
+
+}  // namespace goph

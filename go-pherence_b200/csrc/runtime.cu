@@ -170,6 +170,8 @@ GOPH_API int goph_set_option(const char* name, int value) {
     o.moe_rows = value;
   } else if (!strcmp(name, "mlx_cluster")) {
     o.mlx_cluster = value ? 1 : 0;
+  } else if (!strcmp(name, "gemm_rows")) {
+    o.gemm_rows = value;
   } else if (!strcmp(name, "fp8_convert")) {
     o.fp8_convert = value ? 1 : 0;
   } else if (!strcmp(name, "mlx_chunks")) {
