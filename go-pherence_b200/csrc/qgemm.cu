@@ -173,17 +173,20 @@ __device__ __forceinline__ int block_cols(const QArgs& a, int nb) {
 
 // ---- activation preparation -------------------------------------------------------------------
 
+constexpr int kPrepThreads = 256;
+
 __device__ __forceinline__ uint32_t f16_bits(float v) { return (uint32_t)__half_as_ushort(__float2half_rn(v)); }
 
-// One CTA per activation row: its largest magnitude, then eight consecutive elements per thread and
-// step, one 16-byte core-matrix row per piece; a warp covers one 256-element chunk per step.
+// Grid (activation row, slice of its chunks): the row's largest magnitude, which every CTA of a row finds
+// for itself (the row comes from the L2, four loads in flight per thread), then eight consecutive elements
+// per thread and step, one 16-byte core-matrix row per piece; a warp covers one 256-element chunk per step.
 template <int ORDER, int SUMS, bool XBF16>
-__global__ void __launch_bounds__(512)
+__global__ void __launch_bounds__(kPrepThreads)
 qg_prep_x_kernel(const void* __restrict__ xv, unsigned char* __restrict__ xb, unsigned char* __restrict__ xaux, float* __restrict__ xinv,
                  unsigned char* __restrict__ flags, int batch, int in_dim, int nchunks, int NB, size_t xb_stride, float unit_inv) {
   constexpr int P = XBF16 ? 1 : 3;
-  __shared__ float red[16];
-  const int m = blockIdx.x, tid = threadIdx.x, lane = tid & 31, nthr = blockDim.x;
+  __shared__ float red[kPrepThreads / 32];
+  const int m = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
   const int nb = m / NB, j = m - nb * NB;
   pdl_launch_dependents();
   pdl_wait();  // x may be the output of the kernel in front; the tiles may still be read by it
@@ -207,27 +210,33 @@ qg_prep_x_kernel(const void* __restrict__ xv, unsigned char* __restrict__ xb, un
     }
   };
   float mx = 0.f;
-  for (int k = tid * 8; k < in_dim; k += nthr * 8) {
-    float v[8];
-    load8(k, v);
+  for (int k = tid * 8; k < in_dim; k += 4 * kPrepThreads * 8) {
+    float v[4][8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) mx = fmaxf(mx, fabsf(v[e]));
+    for (int i = 0; i < 4; ++i) load8(k + i * kPrepThreads * 8, v[i]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) mx = fmaxf(mx, fabsf(v[i][e]));
+    }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   if (lane == 0) red[tid >> 5] = mx;
   __syncthreads();
   mx = red[0];
-  for (int i = 1; i < nthr / 32; ++i) mx = fmaxf(mx, red[i]);
+#pragma unroll
+  for (int i = 1; i < kPrepThreads / 32; ++i) mx = fmaxf(mx, red[i]);
   // x * 2^s: the largest element lands in [2^14, 2^15)
   int E = (int)((__float_as_uint(mx) >> 23) & 0xFFu) - 127;
   if (mx == 0.f || E > 127) E = 14;  // an all-zero row, or inf / NaN in x (whose products are not finite anyway)
   if (E < -112) E = -112;            // keeps 2^s a normal float
   const float s = __uint_as_float((uint32_t)(14 - E + 127) << 23);
-  if (tid == 0) xinv[m] = __uint_as_float((uint32_t)(E - 14 + 127) << 23);
+  if (tid == 0 && blockIdx.y == 0) xinv[m] = __uint_as_float((uint32_t)(E - 14 + 127) << 23);
   int n = batch - nb * NB;
   n = n >= NB ? NB : (n + 15) & ~15;
-  for (int k = tid * 8; k < nchunks * kChunkK; k += nthr * 8) {
+  const int k_end = (int)((blockIdx.y + 1) * nchunks / gridDim.y) * kChunkK;
+  for (int k = (int)(blockIdx.y * nchunks / gridDim.y) * kChunkK + tid * 8; k < k_end; k += kPrepThreads * 8) {
     float v[8];
     load8(k, v);
 #pragma unroll
@@ -604,7 +613,6 @@ qg_kernel(const __grid_constant__ QArgs a) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_holder)), "r"(kCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  pdl_launch_dependents();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -655,6 +663,7 @@ qg_kernel(const __grid_constant__ QArgs a) {
     // ------------------------------------------------------------------ prepared activations
     reg_dec<kMiscRegs>();
     pdl_wait();
+    MARK(7, 0);
     RingCursor bc;
     bool wrapped = false;
     auto used_of = [&](const Walk& w, int c) -> uint32_t {  // most pieces any of the block's rows has in this chunk
@@ -832,6 +841,27 @@ qg_kernel(const __grid_constant__ QArgs a) {
     if (TT == 2 && w == 1) wc.next(SW);
     TP(int mk = 0;)
     float2 acc[kItemBlock ? 1 : NB / 2];
+    // TT = 1: the pipes' sums meet through shared memory; afterwards a pipe holds every other group of four columns
+    auto combine = [&](int n) {
+      if constexpr (TT == 1 && !kItemBlock) {
+        float4* cb = reinterpret_cast<float4*>(comb) + r;
+#pragma unroll
+        for (int g = 0; g < NB / 4; ++g)
+          if (4 * g < n && (g & 1) != w) cb[g * kTileRows] = make_float4(acc[2 * g].x, acc[2 * g].y, acc[2 * g + 1].x, acc[2 * g + 1].y);
+        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
+#pragma unroll
+        for (int g = 0; g < NB / 4; ++g) {
+          if (4 * g < n && (g & 1) == w) {
+            const float4 o = cb[g * kTileRows];
+            acc[2 * g].x += o.x;
+            acc[2 * g].y += o.y;
+            acc[2 * g + 1].x += o.z;
+            acc[2 * g + 1].y += o.w;
+          }
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
+      }
+    };
     pdl_wait();  // the activations' scales come from the preparation kernel in front
     for (; wk.live; wk.next_item(a)) {
       const int n = block_cols<NB>(a, wk.nb);
@@ -952,81 +982,87 @@ qg_kernel(const __grid_constant__ QArgs a) {
       // ---- the item is complete (every epilogue warp comes through here, waits given up or not) ----
       if (a.splits > 1 && wk.tail >= 0) break;  // the CTA's last item, shared with the cluster: below
       if constexpr (!kItemBlock) {
-        if (TT == 1) {  // the pipes' sums: pipe 1 hands its own over through shared memory
-          if (w == 1) {
+        combine(n);
+        if (ok) {
 #pragma unroll
-            for (int j = 0; j < NB; ++j)
-              if (j < n) comb[j * kTileRows + r] = (j & 1) ? acc[j / 2].y : acc[j / 2].x;
+          for (int g = 0; g < NB / 4; ++g) {
+            if (4 * g < n && (TT == 2 || (g & 1) == w)) {
+              store(4 * g, acc[2 * g].x);
+              store(4 * g + 1, acc[2 * g].y);
+              store(4 * g + 2, acc[2 * g + 1].x);
+              store(4 * g + 3, acc[2 * g + 1].y);
+            }
           }
-          asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
         }
-        if (ok && (TT == 2 || w == 0)) {
-#pragma unroll
-          for (int j = 0; j < NB; ++j)
-            if (j < n) store(j, ((j & 1) ? acc[j / 2].y : acc[j / 2].x) + (TT == 1 ? comb[j * kTileRows + r] : 0.f));
-        }
-        if (TT == 1) asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
       }
     }
     if (a.splits > 1) {
-      // The K splits of the last item are the CTAs of this cluster (rank == split).  Nothing is in flight in
-      // the rings any more, here or (after the first meeting) in the peers: each thread hands its sums to
-      // the CTAs that finish the columns, a share of them each, which add in split order and store.
+      // The K splits of the last item are the CTAs of this cluster (rank == split).  Each thread hands its
+      // sums, four columns a store, to the CTAs that finish the columns, a share of them each, which add in
+      // split order and store.  (A float a store took 14 us for 64 columns of two tiles: a remote store costs
+      // by the instruction.)  They land in the rings, in which nothing is in flight any more: here, and after
+      // the first meeting in the peers.
+      const int n = block_cols<NB>(a, wk.nb), S = a.splits, sg = ((n + S - 1) / S + 3) / 4;  // sg: groups of four columns of a share
+      if constexpr (!kItemBlock) {
+        if (wk.live) combine(n);
+      }
       cluster_sync_all();
-      const int n = block_cols<NB>(a, wk.nb), S = a.splits, share = (n + S - 1) / S;
-      constexpr int kSrc = TT == 1 ? 2 : 1;  // sources per split
       if (wk.live) {
-        const uint32_t at = smem_u32(wring) + (uint32_t)(((wk.split * kSrc + (TT == 1 ? w : 0)) * TT + t) * share * kTileRows + r) * 4;
+        const uint32_t at = smem_u32(wring) + (uint32_t)((wk.split * TT + t) * sg * kTileRows + r) * 16;
+        int owner = 0, left = sg;
+        uint32_t dst = cluster_map(at, 0);
+        auto send = [&](bool mine, float x, float y, float z, float v) {
+          if (mine)
+            asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "f"(x), "f"(y), "f"(z), "f"(v) : "memory");
+          dst += kTileRows * 16;
+          if (--left == 0 && ++owner < S) {
+            left = sg;
+            dst = cluster_map(at, owner);
+          }
+        };
         if constexpr (kItemBlock) {
           // (the block is still in TMEM: nothing has been opened after it)
-          RingCursor last = dc;
-          const uint32_t d0 = dbase + (DT == 1 ? 0 : (last.s ^ 1) * NB);
+          const uint32_t d0 = dbase + (DT == 1 ? 0 : (dc.s ^ 1) * NB);
           tc_fence_after();
-          int owner = 0, left = share;
-          uint32_t dst = cluster_map(at, 0);
 #pragma unroll 1
           for (int j0 = 0; j0 < n; j0 += 16) {
             uint32_t d[16];
             tmem_ld16(d0 + j0, d);
             tmem_wait_ld(d);
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              cluster_store_f32(dst, __uint_as_float(d[j]));
-              dst += kTileRows * 4;
-              if (--left == 0 && ++owner < S) {
-                left = share;
-                dst = cluster_map(at, owner);
-              }
-            }
+            for (int j = 0; j < 16; j += 4)
+              send(true, __uint_as_float(d[j]), __uint_as_float(d[j + 1]), __uint_as_float(d[j + 2]), __uint_as_float(d[j + 3]));
           }
         } else {
-          int owner = 0, left = share;
-          uint32_t dst = cluster_map(at, 0);
 #pragma unroll
-          for (int j = 0; j < NB; ++j) {
-            if (j < n) {
-              cluster_store_f32(dst, (j & 1) ? acc[j / 2].y : acc[j / 2].x);
-              dst += kTileRows * 4;
-              if (--left == 0 && ++owner < S) {
-                left = share;
-                dst = cluster_map(at, owner);
-              }
-            }
-          }
+          for (int g = 0; g < NB / 4; ++g)
+            if (4 * g < n) send(TT == 2 || (g & 1) == w, acc[2 * g].x, acc[2 * g].y, acc[2 * g + 1].x, acc[2 * g + 1].y);
         }
       }
       cluster_sync_all();
       if (wk.live && ok) {
-        const int row = (wk.group * TT + t) * kTileRows + r, c0 = wk.split * share;
+        const int row = (wk.group * TT + t) * kTileRows + r, m0 = wk.nb * NB, c0 = wk.split * sg * 4;
         const float rs = F == Q_FP8 && row < a.out_dim ? __ldg(a.scale + row) : 1.f, rb = F == Q_FP8 && a.bias && row < a.out_dim ? __ldg(a.bias + row) : 0.f;
-        const float* in = reinterpret_cast<const float*>(wring) + (size_t)t * share * kTileRows + r;
-        for (int j = TT == 1 ? w : 0; j < share; j += TT == 1 ? 2 : 1) {
-          const int m = wk.nb * NB + c0 + j;
-          if (c0 + j >= n || m >= a.batch || row >= a.out_dim) break;
-          float v = 0.f;
-          for (int s2 = 0; s2 < S * kSrc; ++s2) v += in[(size_t)(s2 * TT * share + j) * kTileRows];
-          v = (v * T::kUnit) * __ldg(a.xinv + m);
-          a.out[(size_t)m * a.out_dim + row] = F == Q_FP8 ? fmaf(v, rs, rb) : v;
+        const float4* in = reinterpret_cast<const float4*>(wring) + (size_t)t * sg * kTileRows + r;
+#pragma unroll 2
+        for (int g = TT == 1 ? w : 0; g < sg; g += TT == 1 ? 2 : 1) {
+          if (c0 + 4 * g >= n) break;
+          float v[4] = {0.f, 0.f, 0.f, 0.f};
+          for (int s2 = 0; s2 < S; ++s2) {
+            const float4 q = in[(size_t)(s2 * TT * sg + g) * kTileRows];
+            v[0] += q.x;
+            v[1] += q.y;
+            v[2] += q.z;
+            v[3] += q.w;
+          }
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int m = m0 + c0 + 4 * g + k;
+            if (m < a.batch && row < a.out_dim) {
+              const float y = (v[k] * T::kUnit) * __ldg(a.xinv + m);
+              a.out[(size_t)m * a.out_dim + row] = F == Q_FP8 ? fmaf(y, rs, rb) : y;
+            }
+          }
         }
       }
     }
@@ -1036,6 +1072,10 @@ qg_kernel(const __grid_constant__ QArgs a) {
     cluster_sync_all();
     cluster_sync_all();
   }
+  // (the next kernel's CTAs are asked for now and not at the start: the preparation kernel of a following
+  // product would crowd onto the few SMs this one leaves free and do all its work there)
+  if (warp == kConvWarps) { MARK(7, 1); }
+  pdl_launch_dependents();
   // ---- wind down: everyone meets, outstanding copies are drained, TMEM is returned ----
   tc_fence_before();
   __syncthreads();
@@ -1271,9 +1311,11 @@ int run_rows(const QWeight& w, float* out, const void* x, int batch, cudaStream_
     cfg.stream = stream;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    cfg.gridDim = dim3(rows);
-    const int want = nchunks * 32;  // a warp per chunk
-    cfg.blockDim = dim3(want < 512 ? want : 512);
+    // two CTAs per SM where the row has the chunks for it (a warp takes one)
+    int slices = 2 * device_state(w.device).sm_count / rows;
+    if (slices > (nchunks + 7) / 8) slices = (nchunks + 7) / 8;
+    cfg.gridDim = dim3(rows, slices < 1 ? 1 : slices);
+    cfg.blockDim = dim3(kPrepThreads);
     note_launch();
     GOPH_CUDA(cudaLaunchKernelEx(&cfg, qg_prep_x_kernel<T::kOrder, T::kSums, XBF16>,
                                  static_cast<const void*>(static_cast<const unsigned char*>(x) + (size_t)b0 * xstride), bufs->xb,
