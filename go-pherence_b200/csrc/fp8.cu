@@ -12,7 +12,7 @@
 
 #include "stream_gemv.cuh"
 #include "qgemm.cuh"
-#include "tc_gemm.cuh"
+#include "fp8_mma.cuh"
 
 namespace goph {
 
@@ -101,8 +101,9 @@ static bool valid_fp8(const goph_fp8_linear* w) {
 }
 
 // The several-row tensor-core product (qgemm.cu) reads both layouts (rows of whole 16-byte units).
-static bool qgemm_takes(const goph_fp8_linear* w, const void* x, int batch) {
-  return batch > options().gemm_rows && w->in_dim % 16 == 0 && w->in_dim <= 65536 && (uintptr_t)x % 16 == 0;
+static bool qgemm_takes(const goph_fp8_linear* w, const void* x, bool x_bf16, int batch) {
+  return w->in_dim % 16 == 0 && w->in_dim <= 65536 && (uintptr_t)x % 16 == 0 &&
+         qgemm_wants(Q_FP8, w->tiled != nullptr, x_bf16, w->out_dim, w->in_dim, batch);
 }
 
 static int fp8_qgemm(const goph_fp8_linear* w, float* out, const void* x, bool x_bf16, int batch, cudaStream_t stream) {
@@ -239,9 +240,9 @@ GOPH_API int goph_fp8_gemm(float* out_dev, uint64_t out_len, const float* x_dev,
                 (unsigned long long)need_x, (unsigned long long)out_len, (unsigned long long)need_o);
   if (int rc = use_device(w->device)) return rc;
   cudaStream_t s = (cudaStream_t)stream;
-  // Tensor-core layout: every batch size goes to the kernel that feeds the e4m3 bytes to the MMA as
-  // they lie (fp8_mma.cu); the row-major layout is served by the CUDA-core kernels below.
-  if (qgemm_takes(w, x_dev, batch)) return fp8_qgemm(w, out_dev, x_dev, false, batch, s);
+  // Several rows: qgemm.cu.  Few rows: in the tensor-core layout the kernel that feeds the e4m3 bytes to the
+  // MMA as they lie (fp8_mma.cu), in the row-major layout the CUDA-core kernels below.
+  if (qgemm_takes(w, x_dev, false, batch)) return fp8_qgemm(w, out_dev, x_dev, false, batch, s);
   if (w->tiled) return tc_gemm_fp8(w, out_dev, x_dev, false, batch, s);
   if (!w->tiled && w->in_dim % 16 != 0) {
     note_launch();
@@ -281,7 +282,7 @@ GOPH_API int goph_fp8_gemm_bf16(float* out_dev, uint64_t out_len, const uint16_t
                 "goph_fp8_gemm_bf16 needs a linear in the tensor-core layout (in_dim a multiple of 256, no NaN codes, "
                 "uploaded with fp8_layout 0 or 2)");
   if (int rc = use_device(w->device)) return rc;
-  if (qgemm_takes(w, x_bf16_dev, batch)) return fp8_qgemm(w, out_dev, x_bf16_dev, true, batch, (cudaStream_t)stream);
+  if (qgemm_takes(w, x_bf16_dev, true, batch)) return fp8_qgemm(w, out_dev, x_bf16_dev, true, batch, (cudaStream_t)stream);
   return tc_gemm_fp8(w, out_dev, x_bf16_dev, true, batch, (cudaStream_t)stream);
 }
 

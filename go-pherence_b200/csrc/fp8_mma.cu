@@ -1,6 +1,6 @@
 // FP8 E4M3 linears on the 5th-generation tensor cores with nothing converted on the way:
 // tcgen05.mma kind::f8f6f4, both operands read from shared memory through descriptors, f32
-// accumulators in TMEM.  One kernel for every batch size of a linear in the tensor-core layout.
+// accumulators in TMEM.  For few activation rows of a linear in the tensor-core layout (qgemm.cu has the others).
 //
 // Stands behind nvidia.GemvFP8E4M3Buffer / GemmFP8E4M3Buffer (backends/nvidia/runtime/fp8.go:158-222,
 // :271-320; kernel text backends/nvidia/ptx/fp8/fp8.go:154-309, which decodes every weight on the
@@ -45,7 +45,7 @@
 
 #include "goph_internal.cuh"
 #include "tc_common.cuh"
-#include "tc_gemm.cuh"
+#include "fp8_mma.cuh"
 
 namespace goph {
 
@@ -271,9 +271,6 @@ __device__ __forceinline__ void umma_f8_ss(uint32_t d_tmem, uint64_t a_desc, uin
 // KS: K bytes of a pipeline stage, 256 (a whole block) or 128 (half a block, for wide B tiles).  The
 // MMA warp spends some 70 cycles per instruction and 300 per stage on waits and commits, so the
 // longer stage is what lets a single SM keep up with its share of the HBM rate.
-// TT: row tiles per item (1 or 2).  With a wide B tile (64 activation rows in two pieces are 128 B
-// rows: 16 KiB of activations per 16 KiB of weights, re-read from the L2 for every row tile) two row
-// tiles share each B tile: half the L2 traffic and twice the MMAs per wait and commit.
 template <int N, int P, int MP, int KS, int TT>
 __global__ void __launch_bounds__(kThreads, 1)
 fp8_mma_kernel(const __grid_constant__ Fp8Args a) {
@@ -604,6 +601,26 @@ Fp8Bufs* fp8_bufs(int device, bool allocate = true) {
   return &bufs[device];
 }
 
+// K splits per tile: the split whose busiest CTA spends the least time (items are dealt to the
+// CTAs round-robin), in units of one stage; fix_cost is what writing and re-reading one item's
+// partial sums costs in those units.
+static int choose_splits(int ntiles, int nchunks, int sms, int max_items, float fix_cost) {
+  int best = 1;
+  float best_cost = -1.f;
+  for (int s = 1; s <= 8 && s <= nchunks; ++s) {
+    const long items = (long)ntiles * s;
+    if (items > max_items && s > 1) break;
+    const int grid = items < sms ? (int)items : sms;
+    const long per_cta = (items + grid - 1) / grid;
+    const float cost = per_cta * ((nchunks + s - 1) / s + (s > 1 ? fix_cost : 0.f));
+    if (best_cost < 0.f || cost < best_cost) {
+      best_cost = cost;
+      best = s;
+    }
+  }
+  return best;
+}
+
 template <int N, int P, int MP, bool XBF16, int TT = 1>
 int launch_pass(const goph_fp8_linear* w, float* out, const void* x, int nb, Fp8Bufs* bufs, cudaStream_t stream) {
   constexpr int KS = (N <= 64 && TT == 1) ? 256 : 128;
@@ -629,7 +646,7 @@ int launch_pass(const goph_fp8_linear* w, float* out, const void* x, int nb, Fp8
   if (a.ntiles > (int)kMaxCounters) max_items = 0;
   const int ngroups = (a.ntiles + TT - 1) / TT;  // items are groups of TT row tiles x K splits
   a.splits = options().mlx_splits > 0 ? (options().mlx_splits < a.nks ? options().mlx_splits : a.nks)
-                                      : tc_choose_splits(ngroups, a.nks, st.sm_count, max_items / TT, 2.f + TT * MP / 16.f);
+                                      : choose_splits(ngroups, a.nks, st.sm_count, max_items / TT, 2.f + TT * MP / 16.f);
   while (a.splits > 1 && (long)a.ntiles * a.splits > max_items) --a.splits;
   a.items = ngroups * a.splits;
   const int grid = a.items < st.sm_count ? a.items : st.sm_count;
@@ -731,8 +748,7 @@ __global__ void fp8_dequant_tiled_kernel(const unsigned char* __restrict__ tiled
 
 }  // namespace
 
-// Passes of up to 32 activation rows.  f32 activations: six pieces (an f32 exactly); bf16 activations:
-// two pieces.
+// f32 activations: six pieces (an f32 exactly), up to 4 rows; bf16 activations: two pieces, up to 16 rows.
 int tc_gemm_fp8(const goph_fp8_linear* w, float* out, const void* x, bool x_bf16, int batch, cudaStream_t stream) {
   if (!w->tiled) return fail(GOPH_E_UNSUPPORTED, "FP8 linear is not in the tensor-core layout");
   if (w->in_dim % kChunkK != 0 || w->in_dim > kMaxIn)
@@ -747,19 +763,12 @@ int tc_gemm_fp8(const goph_fp8_linear* w, float* out, const void* x, bool x_bf16
     float* op = out + (size_t)b0 * w->out_dim;
     int rc, nb;
     if (x_bf16) {
-      // two pieces hold a bf16 value; from 17 rows two row tiles share each B tile
-      if (options().fp8_convert && left > 32) return tc_gemm_fp8_converted(w, op, xp, true, left, stream);
-      if (left <= 8) rc = launch_pass<16, 2, 8, true>(w, op, xp, nb = left, bufs, stream);
-      else if (left <= 16) rc = launch_pass<32, 2, 16, true>(w, op, xp, nb = left, bufs, stream);
-      else if (left <= 32) rc = launch_pass<64, 2, 32, true, 2>(w, op, xp, nb = left, bufs, stream);
-      else rc = launch_pass<128, 2, 64, true, 2>(w, op, xp, nb = left < 64 ? left : 64, bufs, stream);
+      if (left <= 8) rc = launch_pass<16, 2, 8, true>(w, op, xp, nb = left, bufs, stream);  // two pieces hold a bf16 value
+      else rc = launch_pass<32, 2, 16, true>(w, op, xp, nb = left < 16 ? left : 16, bufs, stream);
     } else {
       // six pieces hold an f32 exactly
       if (left <= 2) rc = launch_pass<16, 6, 2, false>(w, op, xp, nb = left, bufs, stream);
-      else if (left <= 4) rc = launch_pass<32, 6, 4, false>(w, op, xp, nb = left, bufs, stream);
-      else if (left <= 8) rc = launch_pass<48, 6, 8, false>(w, op, xp, nb = left, bufs, stream);
-      else if (left <= 16) rc = launch_pass<96, 6, 16, false>(w, op, xp, nb = left, bufs, stream);
-      else rc = launch_pass<192, 6, 32, false>(w, op, xp, nb = left < 32 ? left : 32, bufs, stream);
+      else rc = launch_pass<32, 6, 4, false>(w, op, xp, nb = left < 4 ? left : 4, bufs, stream);
     }
     if (rc) return rc;
     b0 += nb;

@@ -354,14 +354,17 @@ static bool valid_gguf(const goph_gguf_matrix* m) {
                                    ((m->qtype == GOPH_GGUF_Q8_0 || m->qtype == GOPH_GGUF_Q6_K) && m->d16))));
 }
 
+static int q_format(int qtype) {
+  return qtype == GOPH_GGUF_Q4_K ? Q_Q4K : qtype == GOPH_GGUF_Q5_K ? Q_Q5K : qtype == GOPH_GGUF_Q6_K ? Q_Q6K : Q_Q80;
+}
+
 // The several-row tensor-core product (qgemm.cu) reads both layouts.
 static bool qgemm_takes(const goph_gguf_matrix* m, const void* x, int batch) {
-  return batch > options().gemm_rows && m->in_dim <= 65536 && (uintptr_t)x % 16 == 0;
+  return m->in_dim <= 65536 && (uintptr_t)x % 16 == 0 && qgemm_wants(q_format(m->qtype), m->tiled != nullptr, false, m->out_dim, m->in_dim, batch);
 }
 
 static int gguf_qgemm(const goph_gguf_matrix* m, float* out, const float* x, int batch, cudaStream_t stream) {
-  const int fmt = m->qtype == GOPH_GGUF_Q4_K ? Q_Q4K : m->qtype == GOPH_GGUF_Q5_K ? Q_Q5K : m->qtype == GOPH_GGUF_Q6_K ? Q_Q6K : Q_Q80;
-  const QWeight q{fmt, m->tiled != nullptr, m->tiled ? m->tiled : m->data, m->d16, nullptr, nullptr, m->device, m->out_dim, m->in_dim};
+  const QWeight q{q_format(m->qtype), m->tiled != nullptr, m->tiled ? m->tiled : m->data, m->d16, nullptr, nullptr, m->device, m->out_dim, m->in_dim};
   return qgemm(q, out, x, false, batch, stream);
 }
 

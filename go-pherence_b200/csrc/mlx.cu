@@ -31,7 +31,7 @@
 #include "goph_internal.cuh"
 #include "mlx_mma.cuh"
 #include "qgemm.cuh"
-#include "tc_gemm.cuh"
+#include "fp8_mma.cuh"
 
 namespace goph {
 
@@ -897,8 +897,9 @@ static int launch_generic(const goph_mlx_weight* w, float* out, const float* x, 
 }
 
 // The several-row tensor-core product (qgemm.cu) reads both layouts of 64-element groups with bf16 tables.
-static bool qgemm_takes(const goph_mlx_weight* w, const void* x) {
-  return w->group_size == 64 && w->sb_bf16 && w->in_dim <= 65536 && (w->tiled || (uintptr_t)x % 16 == 0);
+static bool qgemm_takes(const goph_mlx_weight* w, const void* x, int batch) {
+  return w->group_size == 64 && w->sb_bf16 && w->in_dim <= 65536 && (uintptr_t)x % 16 == 0 &&
+         qgemm_wants(Q_MLX4, w->tiled != nullptr, false, w->out_dim, w->in_dim, batch);
 }
 
 static int mlx_qgemm(const goph_mlx_weight* w, float* out, const void* x, bool x_bf16, int batch, cudaStream_t stream) {
@@ -913,7 +914,7 @@ static int mlx_products(int n, float* const* outs, const goph_mlx_weight* const*
   bool any_tiled = false, any_rows = false;
   for (int i = 0; i < n; ++i) {
     any_tiled = any_tiled || ws[i]->tiled;
-    any_rows = any_rows || (batch > options().gemm_rows && qgemm_takes(ws[i], x));
+    any_rows = any_rows || qgemm_takes(ws[i], x, batch);
   }
   if (any_tiled || any_rows) {
     // tiled weights run on the tensor cores; row-major ones in the same call take their own path
@@ -922,7 +923,7 @@ static int mlx_products(int n, float* const* outs, const goph_mlx_weight* const*
       const goph_mlx_weight* one = ws[i];
       float* o = outs[i];
       int rc;
-      if (batch > options().gemm_rows && qgemm_takes(one, x)) {
+      if (qgemm_takes(one, x, batch)) {
         rc = mlx_qgemm(one, o, x, false, batch, stream);
       } else if (one->tiled) {
         rc = mlx_mma_launch(one, o, x, batch, options().mlx_digits, stream, prepared);

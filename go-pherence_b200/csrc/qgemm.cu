@@ -122,6 +122,7 @@ struct QArgs {
   int out_dim, in_dim, batch;
   int ntiles, nchunks, nblocks;
   int nfull, ntail, splits;    // whole items (a multiple of the grid), then at most one per cluster, cut along K
+  int dcol;                    // columns an accumulator block takes: 16, 32, 64 or 128
   int wslots, bslots, bslot, comb, pmax;  // depths of the rings, bytes of a B slot and of comb, pieces per half chunk in xb
 };
 
@@ -545,6 +546,16 @@ __device__ __forceinline__ void convert_aux(const unsigned char* st, int r, unsi
   *reinterpret_cast<uint4*>(d) = v;
   *reinterpret_cast<uint4*>(d + 2048) = v;
 }
+// D[tmem] (+)= A[tmem] * B[smem descriptor: low and high word], 16-bit floats, f32 accumulate.
+__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "mov.b64 b, {%2, %3};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 // D[tmem] (+)= A[smem descriptor] * B[smem descriptor], 16-bit floats, f32 accumulate.
 __device__ __forceinline__ void umma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -571,39 +582,43 @@ qg_kernel(const __grid_constant__ QArgs a) {
   // The tensor core's f32 sums drift towards zero with their length (0.6e-6 of the largest output at 8192
   // elements): a block is closed and added in registers every 4096, an item of one block is kept to 8192
   constexpr int kSeg = kItemBlock ? 1 << 20 : 16;
-  constexpr int DT = 128 / NB;                    // accumulator blocks of a pipe
+  constexpr int kAB = kLong && NB == 64 ? 3 : 2;  // A units (128 elements, 64 TMEM columns) of a pipe
+  constexpr int kDC = 256 - kAB * 64;             // accumulator columns of a pipe: DT blocks of a.dcol
   constexpr int kPer = kLong || kChunk ? 1 : 128 / T::kBlk; // blocks (or the part of one) in a unit
   constexpr int KS = 8 / kPer;                    // K16 steps of it
   constexpr int UPC = TT == 2 ? 2 : 1;            // units a pipe takes of a chunk
   constexpr int UB = kLong ? kSeg * UPC : kChunk ? UPC : 1;  // units of a block
-  constexpr int kAuxBytes = T::kAux ? 4 * 4096 : 0;  // the affine term's A operand, [pipe][2]
+  constexpr int kAuxBytes = T::kAux ? 2 * kAB * 4096 : 0;  // the affine term's A operand, one beside each A unit
   constexpr uint32_t kCols = 512;
 
   extern __shared__ unsigned char smem_dyn[];
   unsigned char* wring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
-  const int SW = a.wslots, SB = a.bslots;
+  const int SW = a.wslots, SB = a.bslots, DT = kDC / a.dcol;
   unsigned char* bring = wring + (size_t)SW * T::kSlot;
   unsigned char* aux = bring + (size_t)SB * a.bslot;
   float* comb = reinterpret_cast<float*>(aux + kAuxBytes);  // TT = 1: [column][128] sums of pipe 1
   uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(comb) + (TT == 1 ? a.comb : 0));
   const uint32_t wfull = smem_u32(bars), wempty = wfull + 8 * SW, bfull = wempty + 8 * SW, bempty = bfull + 8 * SB;
-  const uint32_t aready = bempty + 8 * SB, afree = aready + 32, dfull = afree + 32, dfree = dfull + 32;  // [pipe][2] each
-  volatile int* pieces = reinterpret_cast<volatile int*>(bars + 2 * SW + 2 * SB + 16);  // [SB] pieces in the slot
+  const uint32_t aready = bempty + 8 * SB, afree = aready + 64, dfull = afree + 64, dfree = dfull + 128;  // [pipe][4], [pipe][8]
+  volatile int* pieces = reinterpret_cast<volatile int*>(bars + 2 * SW + 2 * SB + 48);  // [SB] pieces in the slot
   uint32_t* tmem_holder = const_cast<uint32_t*>(reinterpret_cast<volatile uint32_t*>(pieces + SB));
+  float* xinv = reinterpret_cast<float*>(tmem_holder + 1);  // [kMaxRows]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
     for (int s = 0; s < SW; ++s) {
       mbar_init(wfull + 8 * s, TILED ? 1 : 32);
-      mbar_init(wempty + 8 * s, (TT == 2 ? 1 : 2) * (8 + (kLong ? 0 : 4)));
+      mbar_init(wempty + 8 * s, TT == 2 ? 8 + (kLong ? 0 : 4) : 2 * (4 + (kLong ? 0 : 4)));
     }
     for (int s = 0; s < SB; ++s) {
       mbar_init(bfull + 8 * s, 1);
       mbar_init(bempty + 8 * s, TT);
     }
-    for (int s = 0; s < 4; ++s) {
-      mbar_init(aready + 8 * s, 8);
+    for (int s = 0; s < 8; ++s) {
+      mbar_init(aready + 8 * s, 4);
       mbar_init(afree + 8 * s, 1);
+    }
+    for (int s = 0; s < 16; ++s) {
       mbar_init(dfull + 8 * s, 1);
       mbar_init(dfree + 8 * s, 4);
     }
@@ -616,7 +631,7 @@ qg_kernel(const __grid_constant__ QArgs a) {
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_holder;  // A: columns [pipe][2][64], then D: [pipe][DT][NB]
+  const uint32_t tmem = *tmem_holder;  // A: columns [pipe][kAB][64], then D: [pipe][DT][a.dcol]
   bool ok = true;
   Walk wk(a);
   // is the affine term of the item's i-th chunk this pipe's, and with which unit of the chunk
@@ -709,12 +724,12 @@ qg_kernel(const __grid_constant__ QArgs a) {
     // ------------------------------------------------------------------ MMA, a warp per pipe
     reg_dec<kMiscRegs>();
     const int w = warp - kWarpMMA;
-    RingCursor bc, ac, dc;  // B slots, A buffers (2), accumulator blocks (DT)
+    RingCursor bc, ac, dc;  // B slots, A buffers (kAB), accumulator blocks (DT)
     int used = 0;           // accumulator blocks opened so far, up to DT
     if (TT == 1 && w == 1) bc.next(SB);
     // (the masks: in a cluster launch a shared-memory address carries the CTA's rank above the 18 bits that descriptors hold)
-    const uint32_t bring_u = (smem_u32(bring) >> 4) & 0x3FFF, ar = aready + 16 * w, af = afree + 16 * w, df = dfull + 16 * w, de = dfree + 16 * w;
-    const uint32_t colA = tmem + w * 128, colD = tmem + 256 + w * (DT * NB);
+    const uint32_t bring_u = (smem_u32(bring) >> 4) & 0x3FFF, ar = aready + 32 * w, af = afree + 32 * w, df = dfull + 64 * w, de = dfree + 64 * w;
+    const uint32_t colA = tmem + w * (kAB * 64), colD = tmem + 2 * kAB * 64 + w * kDC;
     TP(int mk = 0;)
     // the next accumulator block is free (the epilogue has read what it held)
     auto open_block = [&] {
@@ -730,7 +745,8 @@ qg_kernel(const __grid_constant__ QArgs a) {
       const int n = block_cols<NB>(a, wk.nb);
       // instruction descriptor: D f32, A f16, B f16, both K-major, N = n, M = 128; the affine term's: A, B bf16
       const uint32_t idesc = (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((128u >> 4) << 24), idesc_aux = idesc | (1u << 7) | (1u << 10);
-      const uint64_t desc_hi = ((uint64_t)((uint32_t)n) << 16) | ((uint64_t)(128u >> 4) << 32) | (1ull << 46);  // halves n * 16 B apart, row groups 128 B
+      // B descriptors: halves n * 16 B apart, row groups 128 B; address and the first stride in the low word
+      const uint32_t dlo = bring_u | ((uint32_t)n << 16), bhi = (128u >> 4) | (1u << 14), n2 = n * 2;
       const int units = (wk.c1 - wk.c) * UPC;
       for (int i = 0; i < units; ++i) {
         ok = mbar_wait(bfull + 8 * bc.s, bc.ph, a.status, 804) && mbar_wait(ar + 8 * ac.s, ac.ph, a.status, 806);
@@ -739,10 +755,10 @@ qg_kernel(const __grid_constant__ QArgs a) {
         tc_fence_after();
         if (w == 0) { MARK(3, mk); }
         const int P = pieces[bc.s];
-        const uint32_t blo = bring_u + ((bc.s * a.bslot) >> 4), acol = colA + ac.s * 64;
+        const uint32_t blo = dlo + ((bc.s * a.bslot) >> 4), acol = colA + ac.s * 64;
         const bool opens = UB == 1 || i % UB == 0, closes = UB == 1 || i + 1 == units || (i + 1) % UB == 0;
         const bool ax = aux_here(w, i / UPC, i % UPC);
-        const uint64_t adesc = ((uint64_t)(2048u >> 4) << 16) | ((uint64_t)(128u >> 4) << 32) | (1ull << 46) | (uint64_t)((smem_u32(aux + (w * 2 + ac.s) * 4096) >> 4) & 0x3FFF);
+        const uint64_t adesc = ((uint64_t)(2048u >> 4) << 16) | ((uint64_t)(128u >> 4) << 32) | (1ull << 46) | (uint64_t)((smem_u32(aux + (w * kAB + ac.s) * 4096) >> 4) & 0x3FFF);
 #pragma unroll
         for (int b = 0; b < kPer; ++b) {
           if (opens) {
@@ -750,18 +766,18 @@ qg_kernel(const __grid_constant__ QArgs a) {
             if (!ok) break;
           }
           if (elect_one()) {
-            const uint32_t dcol = colD + dc.s * NB;
+            const uint32_t dcol = colD + dc.s * a.dcol;
 #pragma unroll
             for (int p = 0; p < 3; ++p) {
               if (p < P) {
 #pragma unroll
                 for (int k = 0; k < KS; ++k)
-                  umma_bf16_ts(dcol, acol + (b * KS + k) * 8, desc_hi | (uint64_t)(blo + (p * 8 + b * KS + k) * (n * 2)), idesc, !(opens && p == 0 && k == 0));
+                  umma_f16_ts(dcol, acol + (b * KS + k) * 8, blo + (p * 8 + b * KS + k) * n2, bhi, idesc, !(opens && p == 0 && k == 0));
               }
             }
             if (kLong && T::kAux != 0 && ax) {  // the affine term joins the open block
 #pragma unroll
-              for (int k = 0; k < T::kAux; ++k) umma_f16_ss(dcol, adesc, desc_hi | (uint64_t)(blo + a.pmax * (n * 16) + k * (n * 2)), idesc_aux, 1);
+              for (int k = 0; k < T::kAux; ++k) umma_f16_ss(dcol, adesc, ((uint64_t)bhi << 32) | (blo + a.pmax * (n * 16) + k * n2), idesc_aux, 1);
             }
             if (closes) umma_commit(df + 8 * dc.s);
           }
@@ -775,7 +791,7 @@ qg_kernel(const __grid_constant__ QArgs a) {
           if (elect_one()) {
 #pragma unroll
             for (int k = 0; k < T::kAux; ++k)
-              umma_f16_ss(colD + dc.s * NB, adesc, desc_hi | (uint64_t)(blo + a.pmax * (n * 16) + k * (n * 2)), idesc_aux, k != 0);
+              umma_f16_ss(colD + dc.s * a.dcol, adesc, ((uint64_t)bhi << 32) | (blo + a.pmax * (n * 16) + k * n2), idesc_aux, k != 0);
             umma_commit(df + 8 * dc.s);
           }
           __syncwarp();
@@ -788,45 +804,51 @@ qg_kernel(const __grid_constant__ QArgs a) {
         __syncwarp();
         if (w == 0) { MARK(4, mk); }
         TP(++mk;)
-        ac.next(2);
+        ac.next(kAB);
         bc.next(SB);
         if (TT == 1) bc.next(SB);
       }
     }
   } else if (warp < kConvWarps) {
-    // ------------------------------------------------------------------ converters, eight warps per pipe: (row, half a unit)
+    // ------------------------------------------------------------------ converters, two groups of four warps per pipe
+    // The groups take turns at the pipe's units, thread = row: while one waits, stores and hands over (some
+    // 500 cycles of a unit), the other converts.
     reg_dec<kConvRegs>();
-    const int w = warp >> 3, kq = (warp >> 2) & 1, q4 = warp & 3, r = q4 * 32 + lane;
+    const int w = warp >> 3, grp = (warp >> 2) & 1, q4 = warp & 3, r = q4 * 32 + lane;
     RingCursor wc, ac;
-    int filled = 0;
+    bool used = false;  // this A buffer has been filled before
+    int cc = 0;         // chunks so far
     if (TT == 2 && w == 1) wc.next(SW);
-    const uint32_t abase = tmem + ((uint32_t)(q4 * 32) << 16) + w * 128 + kq * 32, ar = aready + 16 * w, af = afree + 16 * w;
+    if (grp == 1) ac.next(kAB);
+    const uint32_t abase = tmem + ((uint32_t)(q4 * 32) << 16) + w * (kAB * 64), ar = aready + 32 * w, af = afree + 32 * w;
     TP(int mk = 0;)
     for (; wk.live && ok; wk.next_item(a)) {
-      for (int ci = wk.c; ci < wk.c1 && ok; ++ci) {
-        ok = __all_sync(0xffffffffu, mbar_wait(wfull + 8 * wc.s, wc.ph, a.status, 808));
-        if (!ok) break;
-        const unsigned char* st = wring + wc.s * T::kSlot;
-#pragma unroll 1
-        for (int h = 0; h < UPC; ++h) {
-          if (filled == 2) ok = __all_sync(0xffffffffu, mbar_wait(af + 8 * ac.s, ac.ph ^ 1u, a.status, 809));
-          else ++filled;
+      for (int ci = wk.c; ci < wk.c1 && ok; ++ci, ++cc) {
+        if (TT == 2 || (cc & 1) == grp) {
+          ok = __all_sync(0xffffffffu, mbar_wait(wfull + 8 * wc.s, wc.ph, a.status, 808));
+          if (ok && used) ok = __all_sync(0xffffffffu, mbar_wait(af + 8 * ac.s, ac.ph ^ 1u, a.status, 809));
           if (!ok) break;
           tc_fence_after();
           if (warp == 0) { MARK(1, mk); }
-          if (T::kAux != 0 && kq == 1 && aux_here(w, ci - wk.c, h)) {
-            convert_aux<F, TILED>(st, r, aux + (w * 2 + ac.s) * 4096);
+          const unsigned char* st = wring + wc.s * T::kSlot;
+          if (aux_here(w, ci - wk.c, grp)) {
+            convert_aux<F, TILED>(st, r, aux + (w * kAB + ac.s) * 4096);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the MMA reads it through the async proxy
           }
-          convert_unit<F, TILED>(st, r, TT == 2 ? h : w, kq, abase + ac.s * 64);
+          convert_unit<F, TILED>(st, r, TT == 2 ? grp : w, 0, abase + ac.s * 64);
+          convert_unit<F, TILED>(st, r, TT == 2 ? grp : w, 1, abase + ac.s * 64 + 32);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(wempty + 8 * wc.s);
           tmem_wait_st();
           tc_fence_before();
           warp_arrive(ar + 8 * ac.s, lane);
           if (warp == 0) { MARK(2, mk); }
           TP(++mk;)
-          ac.next(2);
+          ac.next(kAB);
+          used = used || ac.ph != 0;
+          ac.next(kAB);
+          used = used || ac.ph != 0;
         }
-        if (ok) warp_arrive(wempty + 8 * wc.s, lane);
         wc.next(SW);
         if (TT == 2) wc.next(SW);
       }
@@ -836,7 +858,7 @@ qg_kernel(const __grid_constant__ QArgs a) {
     reg_inc<kEpiRegs>();
     const int e = warp - kConvWarps, q4 = warp & 3, w = e >> 2;
     const int r = q4 * 32 + lane, t = TT == 2 ? w : 0;
-    const uint32_t dbase = tmem + 256 + ((uint32_t)(q4 * 32) << 16) + w * (DT * NB), df = dfull + 16 * w, de = dfree + 16 * w;
+    const uint32_t dbase = tmem + 2 * kAB * 64 + ((uint32_t)(q4 * 32) << 16) + w * kDC, df = dfull + 64 * w, de = dfree + 64 * w;
     RingCursor wc, dc;
     if (TT == 2 && w == 1) wc.next(SW);
     TP(int mk = 0;)
@@ -863,6 +885,8 @@ qg_kernel(const __grid_constant__ QArgs a) {
       }
     };
     pdl_wait();  // the activations' scales come from the preparation kernel in front
+    if (tid - kConvWarps * 32 < a.batch) xinv[tid - kConvWarps * 32] = __ldg(a.xinv + tid - kConvWarps * 32);
+    asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
     for (; wk.live; wk.next_item(a)) {
       const int n = block_cols<NB>(a, wk.nb);
       const int row = (wk.group * TT + t) * kTileRows + r;
@@ -874,7 +898,7 @@ qg_kernel(const __grid_constant__ QArgs a) {
       auto store = [&](int j, float v) {  // activation row j of the block
         const int m = wk.nb * NB + j;
         if (m < a.batch && row < a.out_dim) {
-          v = (v * T::kUnit) * __ldg(a.xinv + m);
+          v = (v * T::kUnit) * xinv[m];
           a.out[(size_t)m * a.out_dim + row] = F == Q_FP8 ? fmaf(v, rs, rb) : v;
         }
       };
@@ -885,7 +909,7 @@ qg_kernel(const __grid_constant__ QArgs a) {
 #pragma unroll 1
           for (int j0 = 0; j0 < n; j0 += 16) {
             uint32_t d[16];
-            tmem_ld16(dbase + dc.s * NB + j0, d);
+            tmem_ld16(dbase + dc.s * a.dcol + j0, d);
             tmem_wait_ld(d);
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
@@ -911,10 +935,15 @@ qg_kernel(const __grid_constant__ QArgs a) {
           for (int j0 = 0; j0 < NB; j0 += 32) {
             if (j0 < n) {
               uint32_t d[2][16];
-              tmem_ld16(dbase + dc.s * NB + j0, d[0]);
-              tmem_ld16(dbase + dc.s * NB + j0 + 16, d[1]);
+              tmem_ld16(dbase + dc.s * a.dcol + j0, d[0]);
+              if (j0 + 16 < n) {  // (a block may have 16 columns, and the last one ends where the allocation does)
+                tmem_ld16(dbase + dc.s * a.dcol + j0 + 16, d[1]);
+                tmem_wait_ld(d[1]);
+              } else {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) d[1][j] = 0;
+              }
               tmem_wait_ld(d[0]);
-              tmem_wait_ld(d[1]);
               if (j0 + 32 >= n) {
                 tc_fence_before();
                 warp_arrive(de + 8 * dc.s, lane);
@@ -1002,6 +1031,7 @@ qg_kernel(const __grid_constant__ QArgs a) {
       // split order and store.  (A float a store took 14 us for 64 columns of two tiles: a remote store costs
       // by the instruction.)  They land in the rings, in which nothing is in flight any more: here, and after
       // the first meeting in the peers.
+      __syncwarp();
       const int n = block_cols<NB>(a, wk.nb), S = a.splits, sg = ((n + S - 1) / S + 3) / 4;  // sg: groups of four columns of a share
       if constexpr (!kItemBlock) {
         if (wk.live) combine(n);
@@ -1022,7 +1052,7 @@ qg_kernel(const __grid_constant__ QArgs a) {
         };
         if constexpr (kItemBlock) {
           // (the block is still in TMEM: nothing has been opened after it)
-          const uint32_t d0 = dbase + (DT == 1 ? 0 : (dc.s ^ 1) * NB);
+          const uint32_t d0 = dbase;
           tc_fence_after();
 #pragma unroll 1
           for (int j0 = 0; j0 < n; j0 += 16) {
@@ -1059,7 +1089,7 @@ qg_kernel(const __grid_constant__ QArgs a) {
           for (int k = 0; k < 4; ++k) {
             const int m = m0 + c0 + 4 * g + k;
             if (m < a.batch && row < a.out_dim) {
-              const float y = (v[k] * T::kUnit) * __ldg(a.xinv + m);
+              const float y = (v[k] * T::kUnit) * xinv[m];
               a.out[(size_t)m * a.out_dim + row] = F == Q_FP8 ? fmaf(y, rs, rb) : y;
             }
           }
@@ -1218,14 +1248,15 @@ int launch_product(QArgs& a, const Plan& p, int n, int device, cudaStream_t stre
   a.bslot = n * 256 * a.pmax + T::kAux * n * 32;
   a.comb = TT == 1 ? n * kTileRows * 4 : 0;
   a.bslots = (int)((size_t)(NB == 128 ? 96 : 104) * 1024 / a.bslot);
-  if (a.bslots > 6) a.bslots = 6;
+  if (a.bslots > 4) a.bslots = 4;  // (six: FP8 8192x28672 x5 53.2 us, four 49.4, two 54.7: small B slots leave the room to the weights)
   // A pipe must see every round of the slots that it waits for (a parity wait cannot tell a round from the
   // one two before it): where the pipes take turns, their slots stay apart by an even depth.
   if (TT == 1) a.bslots &= ~1;
-  const size_t fixed = 1024 + 1024 + (size_t)a.bslots * a.bslot + a.comb + (T::kAux ? 4 * 4096 : 0);
+  a.dcol = n <= 16 ? 16 : n <= 32 ? 32 : NB;
+  const size_t fixed = 1024 + 2048 + (size_t)a.bslots * a.bslot + a.comb + (T::kAux ? (T::kLong && NB == 64 ? 6 : 4) * 4096 : 0);
   a.wslots = (int)((kSmemBudget2 - fixed) / T::kSlot);
   if (a.wslots > 10) a.wslots = 10;
-  if (TT == 2) a.wslots &= ~1;
+  a.wslots &= ~1;  // (the same for the tiles of an item, or the converter groups of a pipe)
   if (a.wslots < 2 || a.bslots < 2) return fail(GOPH_E_UNSUPPORTED, "several-row products: no room for the rings");
   size_t smem = fixed + (size_t)a.wslots * T::kSlot;
   if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM (the kernel owns all of TMEM)
@@ -1345,6 +1376,27 @@ int run_fmt(const QWeight& w, float* out, const void* x, bool x_bf16, int batch,
 }
 
 }  // namespace
+
+// The lines lie where the two times met at 1024x1024 (us at 8 rows: 6-8 for the few-row kernels, 10 here, most
+// of it two launches), 1536x4096, 4096x4096, 14336x4096, 4096x14336 and 8192x8192.  Tiled layouts: the GEMV
+// kernels take 8 rows a launch (Q4_K, Q5_K, Q6_K: 4), so a second launch, or the wider accumulator blocks of 5 to 8
+// rows, decide; Q6_K and Q8_0 have a block per 16 or 32 elements here too and gain later.  Other layouts: the
+// CUDA-core kernels' time grows with the rows, above 4 Mi weights from the fourth.
+bool qgemm_wants(int fmt, bool tiled, bool x_bf16, int out_dim, int in_dim, int batch) {
+  if (x_bf16) return fmt != Q_FP8 || batch > 16;  // (FP8 14336x4096: 16 rows 16.7 against 18.2, 24 rows 22.7 against 21.2)
+  if (tiled) {
+    switch (fmt) {
+      case Q_Q4K: return batch > 3;                       // 4 rows: 24.1 against 23.4 (14336x4096)
+      case Q_MLX4: case Q_MLX4F: case Q_Q5K: return batch > 4;  // 5 rows, MLX4: 24.6 against 21.0
+      case Q_Q6K: return batch > 12;                      // 16 rows: 93 against 70
+      case Q_FP8: return batch > 4;                       // 5 rows: 20.3 against 20.6; 8192x28672 58.5 against 53.2
+      default: return batch > 8;                          // Q8_0 9 rows: 42.9 against 42.3
+    }
+  }
+  const bool large = (long)out_dim * in_dim >= (4l << 20);
+  if (fmt == Q_Q6K) return batch > (large ? 8 : 16);
+  return batch > (large ? (fmt == Q_Q5K || fmt == Q_MLX4 || fmt == Q_MLX4F ? 4 : 3) : 8);
+}
 
 int qgemm(const QWeight& w, float* out, const void* x, bool x_bf16, int batch, cudaStream_t stream) {
   if (w.in_dim > kMaxIn) return fail(GOPH_E_UNSUPPORTED, "several-row products: in_dim=%d is above %d", w.in_dim, kMaxIn);

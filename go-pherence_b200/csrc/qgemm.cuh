@@ -23,6 +23,10 @@ struct QWeight {
   int device, out_dim, in_dim;
 };
 
+// Whether `batch` activation rows of such a weight go to this kernel; the others are the business of the kernels
+// for few rows (integer tensor-core GEMV, CUDA-core streaming, FP8 pieces).
+bool qgemm_wants(int fmt, bool tiled, bool x_bf16, int out_dim, int in_dim, int batch);
+
 // out [batch][out_dim] = x [batch][in_dim] . W^T, x f32 or bf16 bit patterns, 16-byte aligned.
 int qgemm(const QWeight& w, float* out, const void* x, bool x_bf16, int batch, cudaStream_t stream);
 

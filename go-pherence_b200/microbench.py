@@ -32,8 +32,7 @@ def run(fmt, out_dim, in_dim, batch=1, launches=200, copies=0, opts=(), warmup=1
     rt.init(0)
     tune = dict((k, v) for k, v in opts if k.startswith("tune_"))
     opts = [(k, v) for k, v in opts if not k.startswith("tune_")]
-    if tune:  # tuning build only: parts of the kernels left out / chunk rotation off
-        rt.lib().goph_tuning_set(int(tune.get("tune_dbg", 0)), int(tune.get("tune_rotate", 1)))
+    if tune:  # tuning build only: parts of the kernels left out
         rt.lib().goph_tuning_set_gemv(int(tune.get("tune_gemv", 0)))
     for k, v in opts:
         rt.SetOption(k, v)
@@ -117,10 +116,10 @@ def run(fmt, out_dim, in_dim, batch=1, launches=200, copies=0, opts=(), warmup=1
     res = {"format": fmt, "out": out_dim, "in": in_dim, "batch": batch, "x": "bf16" if xbf16 else "f32", "tflops": round(tflops, 1), "opts": dict(opts), "copies": copies, "chain": bool(chain),
            "us_per_launch": round(us, 3), "GBps": round(gbs, 1), "frac_of_hbm_peak": round(gbs / peak, 4),
            "bytes": nbytes}
-    if hasattr(rt.lib(), "goph_tuning_probe"):  # tuning build: clock64 timeline of one CTA's last launch
+    if hasattr(rt.lib(), "goph_tuning_probe_gemv") and fmt != "fp8" and batch <= 2:  # tuning build: clock64 timeline of one CTA's last GEMV launch
         import ctypes
         buf = (ctypes.c_longlong * 512)()
-        (rt.lib().goph_tuning_probe if batch > 8 or fmt == "fp8" else rt.lib().goph_tuning_probe_gemv)(buf)
+        rt.lib().goph_tuning_probe_gemv(buf)
         t0 = buf[7 * 64]
         names = ["loads_issued", "mma_sees_stage", "mma_issued", "conv_starts", "conv_done", "epi_sees_unit0", "epi_done"]
         res["trace"] = {"end": buf[7 * 64 + 1] - t0, "pdl_wait_done": buf[7 * 64 + 2] - t0}
