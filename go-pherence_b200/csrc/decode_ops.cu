@@ -106,10 +106,14 @@ qk_norm_rope_append_kernel(float* __restrict__ q, const float* __restrict__ k, c
                            const float* __restrict__ qw, const float* __restrict__ kw,
                            const float* __restrict__ table, const int* __restrict__ pos_dev,
                            float* __restrict__ kcache, float* __restrict__ vcache, int heads, int kv_heads,
-                           int head_dim, float eps, int max_seq) {
+                           int head_dim, float eps, int max_seq, int row_stride) {
   __shared__ float sh[8];
   pdl_begin();
-  const int pos = *pos_dev, half = head_dim / 2, i = threadIdx.x;
+  // blockIdx.y: the row of a prompt chunk, row_stride floats behind the one before, at the next position
+  const int pos = *pos_dev + (int)blockIdx.y, half = head_dim / 2, i = threadIdx.x;
+  q += (size_t)blockIdx.y * row_stride;
+  k += (size_t)blockIdx.y * row_stride;
+  v += (size_t)blockIdx.y * row_stride;
   if (pos < 0 || pos >= max_seq) {
     if (i == 0) atomicCAS(&g_decode_status, 0, 401);
     return;
@@ -191,6 +195,7 @@ struct AttnArgs {
   const int* pos_dev;
   int heads, kv_heads, head_dim;
   int max_seq;           // rows of the caches and of the RoPE table
+  int q_stride, out_stride;  // floats from one row of a prompt chunk to the next (blockIdx.z, at the next position)
   float scale, eps;
   float* scratch;
   unsigned int* counters;
@@ -204,7 +209,9 @@ attn_decode_kernel(const __grid_constant__ AttnArgs a) {
   __shared__ float part[W][EPL * 32];
   __shared__ int s_last;
   pdl_begin();
-  const int pos = *a.pos_dev, seq = pos + 1;
+  const int pos = *a.pos_dev + (int)blockIdx.z, seq = pos + 1;
+  const float* q_row = a.q + (size_t)blockIdx.z * a.q_stride;
+  float* out_row = a.out + (size_t)blockIdx.z * a.out_stride;
   if (pos < 0 || pos >= a.max_seq) {
     if (threadIdx.x == 0) atomicCAS(&g_decode_status, 0, 402);
     return;
@@ -223,7 +230,7 @@ attn_decode_kernel(const __grid_constant__ AttnArgs a) {
   const int nloc = my_blocks * B;  // local indices (some past seq in the last block)
   float qr[EPL];
 #pragma unroll
-  for (int e = 0; e < EPL; ++e) qr[e] = a.q[(size_t)head * head_dim + lane + 32 * e];
+  for (int e = 0; e < EPL; ++e) qr[e] = q_row[(size_t)head * head_dim + lane + 32 * e];
   if (FUSED) norm_rope_head<EPL>(qr, a.q_norm, a.table + (size_t)pos * head_dim, head_dim, a.eps, lane);
   float acc[EPL];
 #pragma unroll
@@ -305,7 +312,7 @@ attn_decode_kernel(const __grid_constant__ AttnArgs a) {
       float r = 0.f;
 #pragma unroll
       for (int w = 0; w < W; ++w) r += part[w][d];
-      a.out[(size_t)head * head_dim + d] = __fmul_rn(r, inv);
+      out_row[(size_t)head * head_dim + d] = __fmul_rn(r, inv);
     }
     return;
   }
@@ -350,16 +357,20 @@ attn_decode_kernel(const __grid_constant__ AttnArgs a) {
   for (int d = threadIdx.x; d < head_dim; d += blockDim.x) {
     float r = 0.f;
     for (int s2 = 0; s2 < splits; ++s2) r = fmaf(__ldcg(base + s2 * stride + 2 + d), fac[s2], r);
-    a.out[(size_t)head * head_dim + d] = __fmul_rn(r, inv);
+    out_row[(size_t)head * head_dim + d] = __fmul_rn(r, inv);
   }
   if (threadIdx.x == 0) a.counters[head] = 0;
 }
 
 // out[i] = silu(gate[i]) * up[i]; gate and up are the two halves of one fused projection output.
-__global__ void silu_mul_kernel(float* __restrict__ out, const float* __restrict__ gate, const float* __restrict__ up, int n) {
+// blockIdx.y: the row, in_stride floats behind the one before (n in out).
+__global__ void silu_mul_kernel(float* __restrict__ out, const float* __restrict__ gate, const float* __restrict__ up, int n, int in_stride) {
   pdl_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
+  gate += (size_t)blockIdx.y * in_stride;
+  up += (size_t)blockIdx.y * in_stride;
+  out += (size_t)blockIdx.y * n;
   const float g = gate[i];
   out[i] = __fmul_rn(__fdiv_rn(g, __fadd_rn(1.f, expf(-g))), up[i]);  // expf: see attn_decode_kernel
 }
@@ -435,7 +446,8 @@ __global__ void embed_mlx_kernel(float* __restrict__ out, const uint32_t* __rest
                                  const unsigned char* __restrict__ tiled, const int* __restrict__ tok_dev, int in_dim,
                                  int group_size, int sb_bf16) {
   pdl_begin();
-  const int row = *tok_dev;
+  const int row = tok_dev[blockIdx.y];  // blockIdx.y: the token of a prompt chunk
+  out += (size_t)blockIdx.y * in_dim;
   const int word = blockIdx.x * blockDim.x + threadIdx.x;  // packed word index within the row
   if (word >= in_dim / 8) return;
   const int col = word * 8, groups = in_dim / group_size, g = col / group_size;
@@ -508,7 +520,16 @@ GOPH_API int goph_qk_norm_rope_append(int device, float* q_dev, const float* k_d
                                       const float* q_norm_dev, const float* k_norm_dev, const float* rope_table_dev,
                                       const int* pos_dev, float* kcache_dev, float* vcache_dev, int max_seq, int heads,
                                       int kv_heads, int head_dim, float eps, void* stream) {
+  return goph_qk_norm_rope_append_rows(device, q_dev, k_dev, v_dev, 0, 1, q_norm_dev, k_norm_dev, rope_table_dev, pos_dev, kcache_dev,
+                                       vcache_dev, max_seq, heads, kv_heads, head_dim, eps, stream);
+}
+
+GOPH_API int goph_qk_norm_rope_append_rows(int device, float* q_dev, const float* k_dev, const float* v_dev, int row_stride, int rows,
+                                           const float* q_norm_dev, const float* k_norm_dev, const float* rope_table_dev,
+                                           const int* pos_dev, float* kcache_dev, float* vcache_dev, int max_seq, int heads,
+                                           int kv_heads, int head_dim, float eps, void* stream) {
   clear_error();
+  if (rows <= 0 || rows > 65535 || row_stride < 0) return fail(GOPH_E_INVALID, "goph_qk_norm_rope_append: rows=%d stride=%d", rows, row_stride);
   if (max_seq <= 0) return fail(GOPH_E_INVALID, "max_seq=%d", max_seq);
   if (!q_dev || !k_dev || !v_dev || !rope_table_dev || !pos_dev || !kcache_dev || !vcache_dev)
     return fail(GOPH_E_INVALID, "goph_qk_norm_rope_append: nil buffer");
@@ -517,11 +538,11 @@ GOPH_API int goph_qk_norm_rope_append(int device, float* q_dev, const float* k_d
                 kv_heads, head_dim);
   if ((q_norm_dev == nullptr) != (k_norm_dev == nullptr)) return fail(GOPH_E_INVALID, "QNorm without KNorm");
   if (int rc = use_device(device)) return rc;
-  return op_launch(qk_norm_rope_append_kernel, dim3(heads + kv_heads), head_dim / 2, 0, stream, q_dev, k_dev, v_dev, q_norm_dev,
-                   k_norm_dev, rope_table_dev, pos_dev, kcache_dev, vcache_dev, heads, kv_heads, head_dim, eps, max_seq);
+  return op_launch(qk_norm_rope_append_kernel, dim3(heads + kv_heads, rows), head_dim / 2, 0, stream, q_dev, k_dev, v_dev, q_norm_dev,
+                   k_norm_dev, rope_table_dev, pos_dev, kcache_dev, vcache_dev, heads, kv_heads, head_dim, eps, max_seq, row_stride);
 }
 
-static int attn_launch(int device, AttnArgs& a, int max_seq, bool fused, void* stream) {
+static int attn_launch(int device, AttnArgs& a, int max_seq, bool fused, void* stream, int rows = 1) {
   if (a.heads <= 0 || a.kv_heads <= 0 || a.heads % a.kv_heads || a.head_dim < 64 || a.head_dim > 256 || a.head_dim % 64)
     return fail(GOPH_E_UNSUPPORTED, "attention dims heads=%d kv_heads=%d head_dim=%d (head_dim 64, 128 or 256)", a.heads,
                 a.kv_heads, a.head_dim);
@@ -563,8 +584,8 @@ static int attn_launch(int device, AttnArgs& a, int max_seq, bool fused, void* s
   const int per_cta = small ? 16 : 256;
   int splits = (max_seq + per_cta - 1) / per_cta;
   if (splits > kAttnMaxSplits) splits = kAttnMaxSplits;
-  if (splits < 1) splits = 1;
-  const dim3 grid(a.heads, splits);
+  if (splits < 1 || rows > 1) splits = 1;  // (the rows of a prompt chunk fill the machine without)
+  const dim3 grid(a.heads, splits, rows);
 #define GOPH_ATTN(EPL)                                                                                          \
   return small ? (fused ? op_launch(attn_decode_kernel<EPL, true, 4>, grid, 4 * 32, 0, stream, a)               \
                         : op_launch(attn_decode_kernel<EPL, false, 4>, grid, 4 * 32, 0, stream, a))             \
@@ -579,7 +600,15 @@ static int attn_launch(int device, AttnArgs& a, int max_seq, bool fused, void* s
 GOPH_API int goph_attn_decode(int device, float* out_dev, const float* q_dev, const float* kcache_dev,
                               const float* vcache_dev, const int* pos_dev, int max_seq, int heads, int kv_heads,
                               int head_dim, float scale, void* stream) {
+  return goph_attn_rows(device, out_dev, 0, q_dev, 0, 1, kcache_dev, vcache_dev, pos_dev, max_seq, heads, kv_heads, head_dim, scale, stream);
+}
+
+GOPH_API int goph_attn_rows(int device, float* out_dev, int out_stride, const float* q_dev, int q_stride, int rows,
+                            const float* kcache_dev, const float* vcache_dev, const int* pos_dev, int max_seq, int heads,
+                            int kv_heads, int head_dim, float scale, void* stream) {
   clear_error();
+  if (rows <= 0 || rows > 65535 || out_stride < 0 || q_stride < 0)
+    return fail(GOPH_E_INVALID, "goph_attn_rows: rows=%d strides=%d, %d", rows, out_stride, q_stride);
   if (!out_dev || !q_dev || !kcache_dev || !vcache_dev || !pos_dev) return fail(GOPH_E_INVALID, "goph_attn_decode: nil buffer");
   AttnArgs a;
   memset(&a, 0, sizeof a);
@@ -592,7 +621,9 @@ GOPH_API int goph_attn_decode(int device, float* out_dev, const float* q_dev, co
   a.kv_heads = kv_heads;
   a.head_dim = head_dim;
   a.scale = scale;
-  return attn_launch(device, a, max_seq, false, stream);
+  a.q_stride = q_stride;
+  a.out_stride = out_stride;
+  return attn_launch(device, a, max_seq, false, stream, rows);
 }
 
 GOPH_API int goph_attn_decode_fused(int device, float* out_dev, const float* q_dev, const float* k_dev, const float* v_dev,
@@ -624,10 +655,16 @@ GOPH_API int goph_attn_decode_fused(int device, float* out_dev, const float* q_d
 }
 
 GOPH_API int goph_silu_mul(int device, float* out_dev, const float* gate_dev, const float* up_dev, int n, void* stream) {
+  return goph_silu_mul_rows(device, out_dev, gate_dev, up_dev, n, 0, 1, stream);
+}
+
+GOPH_API int goph_silu_mul_rows(int device, float* out_dev, const float* gate_dev, const float* up_dev, int n, int in_stride, int rows,
+                                void* stream) {
   clear_error();
-  if (!out_dev || !gate_dev || !up_dev || n <= 0) return fail(GOPH_E_INVALID, "goph_silu_mul: n=%d", n);
+  if (!out_dev || !gate_dev || !up_dev || n <= 0 || rows <= 0 || rows > 65535 || in_stride < 0)
+    return fail(GOPH_E_INVALID, "goph_silu_mul: n=%d rows=%d stride=%d", n, rows, in_stride);
   if (int rc = use_device(device)) return rc;
-  return op_launch(silu_mul_kernel, dim3((n + 255) / 256), 256, 0, stream, out_dev, gate_dev, up_dev, n);
+  return op_launch(silu_mul_kernel, dim3((n + 255) / 256, rows), 256, 0, stream, out_dev, gate_dev, up_dev, n, in_stride);
 }
 
 GOPH_API int goph_argmax_advance(int device, const float* logits_dev, int n, int* tok_dev, int* pos_dev, int* history_dev,
@@ -671,11 +708,16 @@ GOPH_API int goph_argmax_advance(int device, const float* logits_dev, int n, int
 }
 
 GOPH_API int goph_mlx_embed(float* out_dev, uint64_t out_len, const goph_mlx_weight* w, const int* tok_dev, void* stream) {
+  return goph_mlx_embed_rows(out_dev, out_len, w, tok_dev, 1, stream);
+}
+
+GOPH_API int goph_mlx_embed_rows(float* out_dev, uint64_t out_len, const goph_mlx_weight* w, const int* tok_dev, int rows, void* stream) {
   clear_error();
   if (!w || w->magic != kMagicMLX) return fail(GOPH_E_INVALID, "invalid MLX weight handle");
-  if (!out_dev || out_len < (uint64_t)w->in_dim || !tok_dev) return fail(GOPH_E_INVALID, "goph_mlx_embed: buffers");
+  if (rows <= 0 || rows > 65535) return fail(GOPH_E_INVALID, "goph_mlx_embed: rows=%d", rows);
+  if (!out_dev || out_len < (uint64_t)w->in_dim * rows || !tok_dev) return fail(GOPH_E_INVALID, "goph_mlx_embed: buffers");
   if (int rc = use_device(w->device)) return rc;
   const int words = w->in_dim / 8;
-  return op_launch(embed_mlx_kernel, dim3((words + 127) / 128), 128, 0, stream, out_dev, (const uint32_t*)w->qweight,
+  return op_launch(embed_mlx_kernel, dim3((words + 127) / 128, rows), 128, 0, stream, out_dev, (const uint32_t*)w->qweight,
                    (const void*)w->sb, (const unsigned char*)w->tiled, tok_dev, w->in_dim, w->group_size, w->sb_bf16);
 }

@@ -9,12 +9,16 @@ product lists (goph_mlx_program_create_pre) — everything between two attention
 gate|up, SiLU * up, down, add + norm, the next layer's q|k|v) as one cooperative launch: two launches
 per layer.
 The position, the current token, the prompt and the produced tokens live in device memory, so the
-whole step is captured once as a CUDA graph and replayed per token — prompt tokens included (they
-are fed one by one, as the reference's sequential loop does).  torch is used for stream capture only.
+whole step is captured once as a CUDA graph and replayed per token.  A prompt goes through the layers in
+chunks (every projection once per chunk instead of once per token, and no logits: nobody asks for
+those of a prompt token) up to its last token, which the step takes; when the logits of every position
+are wanted, it is fed token by token, as the reference's sequential loop does.  torch is used for stream capture only.
 """
 import math
 
 import numpy as np
+
+PREFILL_ROWS = 128   # prompt tokens that go through the layers together
 
 
 class MLXDecoder:
@@ -61,6 +65,7 @@ class MLXDecoder:
         self.forced = rt.wrap(self.ints.Ptr + 8 + 4 * c.max_seq, 4 * c.max_seq)
         self.scale = 1.0 / math.sqrt(c.head_dim)
         self.graph = None
+        self.chunk = None   # buffers of prefill(), made for the first prompt
         self.launches_per_step = 0
         self.lists = self._build_lists() if (self.fused and lists) else None
 
@@ -163,10 +168,51 @@ class MLXDecoder:
         rt.ArgmaxAdvance(self.logits, c.vocab, self.tok, self.pos, self.history, self.forced, c.max_seq, stream)
         self.launches_per_step = n + 3 + (1 if self.lm.OutDim * self.lm.InDim >= (8 << 20) else 0)
 
-    def reset(self, prompt):
+    def prefill(self, prompt, stream=None):
+        """The keys and values of every prompt token but the last into the caches, and the decoder set up
+        for a step with the last one.  The last layer ends with its keys and values."""
+        rt, c = self.rt, self.cfg
+        n = len(prompt) - 1
+        self.reset(prompt, n)
+        rows = min(n, PREFILL_ROWS)
+        if self.chunk is None or self.chunk["rows"] < rows:
+            if self.chunk is not None:
+                rt.Sync()
+                for b in self.chunk["bufs"]:
+                    b.Free()
+            bufs = [rt.Malloc(rows * d) for d in (c.hidden, c.hidden, self.qd + 2 * self.kvd, self.qd, c.hidden, 2 * c.inter, c.inter)]
+            starts = rt.from_numpy(np.arange(0, c.max_seq, PREFILL_ROWS, dtype=np.int32))
+            self.chunk = {"rows": rows, "bufs": bufs + [starts], "starts": starts}
+        hidden, normed, qkv, attn, proj, gu, act = self.chunk["bufs"][:7]
+        width = self.qd + 2 * self.kvd
+        q, k, v = self._sub(qkv, 0, self.qd), self._sub(qkv, self.qd, self.kvd), self._sub(qkv, self.qd + self.kvd, self.kvd)
+        gate, up = self._sub(gu, 0, c.inter), self._sub(gu, c.inter, c.inter)
+        for s0 in range(0, n, PREFILL_ROWS):
+            m = min(PREFILL_ROWS, n - s0)
+            pos = rt.wrap(self.chunk["starts"].Ptr + 4 * (s0 // PREFILL_ROWS), 4)
+            rt.EmbedMLXRows(hidden, self.lm, rt.wrap(self.forced.Ptr + 4 * s0, 4 * m), m, stream)
+            prev = None
+            for e in self.L:
+                rt.AddRMSNorm(hidden if prev is not None else None, normed, hidden, prev, e["input_norm"], c.hidden, m, c.eps, stream)
+                rt.GemmMLX(qkv, normed, e["qkv"], m, stream)
+                rt.QKNormRoPEAppendRows(q, k, v, width, m, e["q_norm"], e["k_norm"], self.table, pos, e["kc"], e["vc"], c.max_seq,
+                                        c.heads, c.kv_heads, c.head_dim, c.eps, stream)
+                if e is self.L[-1]:
+                    break
+                rt.AttnRows(attn, self.qd, q, width, m, e["kc"], e["vc"], pos, c.max_seq, c.heads, c.kv_heads, c.head_dim, self.scale,
+                            stream)
+                rt.GemmMLX(proj, attn, e["o"], m, stream)
+                rt.AddRMSNorm(hidden, normed, hidden, proj, e["post_norm"], c.hidden, m, c.eps, stream)
+                rt.GemmMLX(gu, normed, e["gate_up"], m, stream)
+                rt.SiLUMulRows(act, gate, up, c.inter, 2 * c.inter, m, stream)
+                rt.GemmMLX(proj, act, e["down"], m, stream)
+                prev = proj
+
+    def reset(self, prompt, start=0):
+        """The next step takes prompt[start] at position `start`."""
         c = self.cfg
         ints = np.full(2 + 2 * c.max_seq, -1, dtype=np.int32)
-        ints[0], ints[1] = prompt[0], 0
+        ints[0], ints[1] = prompt[start], start
         ints[2:2 + len(prompt)] = prompt                       # history
         ints[2 + c.max_seq:2 + c.max_seq + len(prompt)] = prompt   # forced
         self.ints.UploadBytes(ints.view(np.uint8))
@@ -193,8 +239,13 @@ class MLXDecoder:
         if use_graph and self.graph is None:
             self.reset(prompt)
             self.capture()
-        self.reset(prompt)
-        for i in range(total - 1):
+        # from four prompt tokens a chunk (some 350 launches) takes less time than the steps it saves (some 150 each)
+        first = len(prompt) - 1 if len(prompt) > 3 and logits_all is None else 0
+        if first:
+            self.prefill(prompt)
+        else:
+            self.reset(prompt)
+        for i in range(first, total - 1):
             if use_graph:
                 self.graph.replay()
             else:

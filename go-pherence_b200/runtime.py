@@ -38,7 +38,7 @@ EXPORTS = [
     "goph_fp8_gemm_host",
     "goph_moe_create", "goph_moe_set_router", "goph_moe_set_expert", "goph_moe_free", "goph_moe_forward",
     "goph_moe_forward_logits", "goph_moe_last_routing",
-    "goph_add_rmsnorm", "goph_qk_norm_rope_append", "goph_attn_decode", "goph_attn_decode_fused", "goph_silu_mul", "goph_argmax_advance", "goph_mlx_embed", "goph_mlx_gemv_pre",
+    "goph_add_rmsnorm", "goph_qk_norm_rope_append", "goph_attn_decode", "goph_attn_decode_fused", "goph_silu_mul", "goph_argmax_advance", "goph_mlx_embed", "goph_qk_norm_rope_append_rows", "goph_attn_rows", "goph_silu_mul_rows", "goph_mlx_embed_rows", "goph_mlx_gemv_pre",
     "goph_shard_rows", "goph_gather_create", "goph_gather_export", "goph_gather_open_peer", "goph_gather_attach_local",
     "goph_gather_free", "goph_gather_status", "goph_gather_shard_buffer", "goph_gather_all",
     "goph_mlx_gemm_allgather", "goph_gguf_project_allgather", "goph_fp8_gemm_allgather", "goph_moe_forward_sharded",
@@ -826,6 +826,28 @@ def QKNormRoPEAppend(q, k, v, qNorm, kNorm, ropeTable, pos, kCache, vCache, maxS
 def AttnDecode(out, q, kCache, vCache, pos, maxSeq, heads, kvHeads, headDim, scale, stream=None):
     _check(lib().goph_attn_decode(_device, _ptr(out), _ptr(q), _ptr(kCache), _ptr(vCache), _ptr(pos), int(maxSeq), int(heads),
                                   int(kvHeads), int(headDim), C.c_float(scale), _stream_ptr(stream)))
+
+
+def QKNormRoPEAppendRows(q, k, v, rowStride, rows, qNorm, kNorm, ropeTable, pos, kCache, vCache, maxSeq, heads, kvHeads, headDim,
+                         eps=1e-6, stream=None):
+    """QKNormRoPEAppend for the tokens of a prompt chunk at consecutive positions."""
+    _check(lib().goph_qk_norm_rope_append_rows(_device, _ptr(q), _ptr(k), _ptr(v), int(rowStride), int(rows), _ptr(qNorm), _ptr(kNorm),
+                                               _ptr(ropeTable), _ptr(pos), _ptr(kCache), _ptr(vCache), int(maxSeq), int(heads),
+                                               int(kvHeads), int(headDim), C.c_float(eps), _stream_ptr(stream)))
+
+
+def AttnRows(out, outStride, q, qStride, rows, kCache, vCache, pos, maxSeq, heads, kvHeads, headDim, scale, stream=None):
+    """AttnDecode for the tokens of a prompt chunk, each over the positions up to its own."""
+    _check(lib().goph_attn_rows(_device, _ptr(out), int(outStride), _ptr(q), int(qStride), int(rows), _ptr(kCache), _ptr(vCache),
+                                _ptr(pos), int(maxSeq), int(heads), int(kvHeads), int(headDim), C.c_float(scale), _stream_ptr(stream)))
+
+
+def SiLUMulRows(out, gate, up, n, inStride, rows, stream=None):
+    _check(lib().goph_silu_mul_rows(_device, _ptr(out), _ptr(gate), _ptr(up), int(n), int(inStride), int(rows), _stream_ptr(stream)))
+
+
+def EmbedMLXRows(out, w, toks, rows, stream=None):
+    _check(lib().goph_mlx_embed_rows(_ptr(out), C.c_uint64(out.n), _mlx_handle(w), _ptr(toks), int(rows), _stream_ptr(stream)))
 
 
 def SiLUMul(out, gate, up, n, stream=None):

@@ -414,10 +414,21 @@ int goph_qk_norm_rope_append(int device, float* q_dev, const float* k_dev, const
                              const float* q_norm_dev, const float* k_norm_dev, const float* rope_table_dev,
                              const int* pos_dev, float* kcache_dev, float* vcache_dev, int max_seq, int heads,
                              int kv_heads, int head_dim, float eps, void* stream);
+/* The same for the `rows` tokens of a prompt chunk at positions *pos_dev, *pos_dev + 1, ..: q, k and v of a row
+ * stand row_stride floats behind those of the row before. */
+int goph_qk_norm_rope_append_rows(int device, float* q_dev, const float* k_dev, const float* v_dev, int row_stride, int rows,
+                                  const float* q_norm_dev, const float* k_norm_dev, const float* rope_table_dev,
+                                  const int* pos_dev, float* kcache_dev, float* vcache_dev, int max_seq, int heads,
+                                  int kv_heads, int head_dim, float eps, void* stream);
 /* simd.GQAAttentionScaleInto over positions 0..*pos_dev (backends/simd/runtime/attention.go:82-113). */
 int goph_attn_decode(int device, float* out_dev, const float* q_dev, const float* kcache_dev,
                      const float* vcache_dev, const int* pos_dev, int max_seq, int heads, int kv_heads,
                      int head_dim, float scale, void* stream);
+/* The same for the `rows` tokens of a prompt chunk, row r over positions 0..*pos_dev + r of the caches (in which
+ * goph_qk_norm_rope_append_rows has put the chunk). */
+int goph_attn_rows(int device, float* out_dev, int out_stride, const float* q_dev, int q_stride, int rows,
+                   const float* kcache_dev, const float* vcache_dev, const int* pos_dev, int max_seq, int heads,
+                   int kv_heads, int head_dim, float scale, void* stream);
 /* goph_qk_norm_rope_append and goph_attn_decode in one launch: q_dev, k_dev, v_dev are the raw
  * projection outputs of the current position; the new k and v are also written into their cache rows. */
 int goph_attn_decode_fused(int device, float* out_dev, const float* q_dev, const float* k_dev, const float* v_dev,
@@ -426,6 +437,9 @@ int goph_attn_decode_fused(int device, float* out_dev, const float* q_dev, const
                            int kv_heads, int head_dim, float scale, float eps, void* stream);
 /* simd.VecSiLUMul (backends/simd/kernels/activation.go:15-24). */
 int goph_silu_mul(int device, float* out_dev, const float* gate_dev, const float* up_dev, int n, void* stream);
+/* Row by row: gate and up of a row in_stride floats behind those of the row before, results n floats. */
+int goph_silu_mul_rows(int device, float* out_dev, const float* gate_dev, const float* up_dev, int n, int in_stride, int rows,
+                       void* stream);
 /* ArgmaxLogits (model/inference_helpers.go:248-261: the first maximum) and the bookkeeping of the
  * greedy loop: *tok_dev = the winner (or forced_dev[*pos_dev + 1] when that is >= 0: prompt tokens),
  * history_dev[*pos_dev + 1] = it, *pos_dev += 1. */
@@ -441,6 +455,8 @@ int goph_mlx_gemv_pre(float* out_dev, uint64_t out_len, const goph_mlx_weight* w
                       const float* b_dev, const float* norm_w_dev, float* hidden_out_dev, float eps, void* stream);
 /* LlamaModel.TokenEmbeddingInto for a tied MLX LM head: dequantised row *tok_dev (model/inference_helpers.go:20-44). */
 int goph_mlx_embed(float* out_dev, uint64_t out_len, const goph_mlx_weight* w, const int* tok_dev, void* stream);
+/* The rows of the tokens tok_dev[0..rows). */
+int goph_mlx_embed_rows(float* out_dev, uint64_t out_len, const goph_mlx_weight* w, const int* tok_dev, int rows, void* stream);
 
 /* ---- row-sharded products across the GPUs of one box ----------------------------------------
  * The reference is single-GPU.  A projection [out x in] is split by rows: rank r of `world` uploads

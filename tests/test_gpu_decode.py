@@ -355,3 +355,25 @@ def test_product_lists_change_nothing(gpu, pkg):
     assert with_lists.launches_per_step < without.launches_per_step
     assert all(p.Status() == 0 for p in with_lists.lists)
     assert with_lists.generate(prompt, 12, use_graph=False) == a
+
+
+@pytest.mark.parametrize("prompt_len", [4, 5, 17, 129, 131])
+def test_prompt_in_chunks(gpu, pkg, prompt_len):
+    """The prompt through the layers in chunks against the same prompt token by token (logits of every
+    position asked for): chunk edges (128 tokens), products on both sides of the several-row kernel's
+    line.  The same f32 operations up to the products' summation order: LOGIT_TOL."""
+    cfg = od.DecodeConfig(hidden=512, layers=3, heads=8, kv_heads=4, head_dim=64, inter=1024, vocab=4096, max_seq=160, qk_norm=True)
+    layers_gpu, _, lm, final_norm = build_model(pkg, cfg, "chunks", centred=True)
+    table = od.rope_table(cfg.max_seq, cfg.head_dim, cfg.theta)
+    prompt = [int(t) for t in pkg.synth.rng("prompt", "chunks").integers(0, cfg.vocab, prompt_len)]
+    dec = pkg.decode.MLXDecoder(gpu, cfg, layers_gpu, lm, final_norm, table)
+    every, last = [], []
+    want = dec.generate(prompt, 4, logits_all=every)
+    got = dec.generate(prompt, 4, logits_at=last)
+    assert gpu.KernelStatus() == 0
+    ref = every[prompt_len - 1]
+    assert np.max(np.abs(last[0] - ref)) <= LOGIT_TOL * np.max(np.abs(ref))
+    top = np.sort(ref)[-2:]
+    assert got[:prompt_len + 1] == want[:prompt_len + 1] or top[1] - top[0] <= 2 * LOGIT_TOL * np.max(np.abs(ref))
+    with pytest.raises(gpu.GophError):
+        gpu.AttnRows(dec.attn, 1, dec.qkv, 1, 0, dec.L[0]["kc"], dec.L[0]["vc"], dec.pos, cfg.max_seq, 8, 4, 64, 1.0)
