@@ -581,6 +581,205 @@ mlx_gemv_kernel(const __grid_constant__ MlxArgs a) {
                                      [] { asm volatile("griddepcontrol.wait;" ::: "memory"); });
 }
 
+// The product of one activation row and a matrix that fits the machine at once (every row-major matrix
+// of the automatic layout, under 8 Mi weights): a warp owns R rows' next 1024 elements and nothing else, so
+// that little is left to do once x exists.  The S warps of a row group stand side by side in a CTA
+// (8 / S groups each).  In front of the wait for the producer of x: the weights' loads, the nibbles of the
+// first rows turned into floats, the norm weights' loads.  Behind it: x into shared memory (one pass), eight
+// LDS.128 and the FMAs; the slices' {scale, dot, bias, sum x} go through shared memory to the first warp of
+// the row group, which runs the same chain of FMAs as mlx_gemv_body's loop: the same bits.
+// Latency is the bound.  Four such products in a dependent chain (1024 .. 6144 rows of 1024 .. 3072): the
+// looping kernel spent 1.7 to 3.8 us of each 4.3 us behind the wait, on few warps working through several
+// tiles one after the other; this one takes 2.6 us a product.
+constexpr int kRowMaxSlices = 8;
+
+template <int R, int MODE, bool SB_BF16, int PRE>
+__global__ void __launch_bounds__(kThreads, R == 1 ? 3 : 2)
+mlx_gemv_row_kernel(const __grid_constant__ MlxArgs a, int S, int groups_per_cta) {
+  constexpr int P = R < 2 ? R : 2;  // rows unpacked ahead
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float4* xs = reinterpret_cast<float4*>(smem_raw);                                   // [S][8 slots][32 units]
+  float4* part = reinterpret_cast<float4*>(smem_raw + (size_t)S * 8 * 32 * 16);       // [warp][R][32]
+  __shared__ float red[kWarps];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  typedef typename std::conditional<SB_BF16, uint32_t, float2>::type SbT;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int grp = warp / S, slice = warp - grp * S;
+  const int task = (int)blockIdx.x * groups_per_cta + grp;
+  const bool live = grp < groups_per_cta && task < a.tasks;
+  uint4 w[R];
+  SbT sb[R];
+  float f[P][32];
+  float* out = nullptr;
+  int row0 = 0, rows = 0;
+  if (live) {
+    int seg = 0;
+#pragma unroll
+    for (int s = 1; s < kMaxSeg; ++s)
+      if (s < a.nseg && task >= a.seg[s].task0) seg = s;
+    const MlxSeg& sg = a.seg[seg];
+    row0 = (task - sg.task0) * R;
+    rows = sg.rows;
+    out = sg.out;
+    int unit = slice * 32 + lane;
+    if (unit >= a.units) unit = a.units - 1;  // x is zero there; any finite weight will do
+    const int grpi = unit >> a.ug_shift;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int row = row0 + r < rows ? row0 + r : rows - 1;
+      w[r] = ld_stream(sg.w + (size_t)row * a.units + unit);
+      sb[r] = __ldg(reinterpret_cast<const SbT*>(sg.sb) + (size_t)row * a.groups + grpi);
+    }
+  }
+  // this thread's part of x: float4 number tid + 256 i (slot tid % 8 of unit (tid + 256 i) / 8)
+  constexpr int kV = 4;  // of them at a time
+  const int slot = tid & 7, u0 = tid >> 3;
+  float4 nw[kV];
+  if (PRE == 1) {
+#pragma unroll
+    for (int i = 0; i < kV; ++i)
+      if (i < S && i * 32 + u0 < a.units) nw[i] = __ldg(reinterpret_cast<const float4*>(a.pre_w) + i * 256 + tid);
+  }
+  if (live) {
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint32_t word = k == 0 ? w[p].x : k == 1 ? w[p].y : k == 2 ? w[p].z : w[p].w;
+        float t[8];
+        Unpack<MODE>::run(word, t);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[p][8 * k + e] = t[e];
+      }
+    }
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (PRE == 1) {
+    // v = x (+ b), hidden = v, inv = 1 / sqrt(mean(v^2) + eps), staged x = (v inv) w; S <= kV
+    float4 v[kV], b[kV];
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < kV; ++i) {
+      const bool in = i < S && i * 32 + u0 < a.units;
+      v[i] = in ? *(reinterpret_cast<const float4*>(a.x) + i * 256 + tid) : zero;
+      b[i] = in && a.pre_b ? *(reinterpret_cast<const float4*>(a.pre_b) + i * 256 + tid) : zero;
+    }
+#pragma unroll
+    for (int i = 0; i < kV; ++i) {
+      if (i < S && i * 32 + u0 < a.units) {
+        if (a.pre_b) v[i] = make_float4(__fadd_rn(v[i].x, b[i].x), __fadd_rn(v[i].y, b[i].y), __fadd_rn(v[i].z, b[i].z), __fadd_rn(v[i].w, b[i].w));
+        if (a.pre_hidden && blockIdx.x == 0) *(reinterpret_cast<float4*>(a.pre_hidden) + i * 256 + tid) = v[i];
+        ss = fmaf(v[i].x, v[i].x, fmaf(v[i].y, v[i].y, fmaf(v[i].z, v[i].z, fmaf(v[i].w, v[i].w, ss))));
+      }
+    }
+    ss = warp_sum(ss);
+    if (lane == 0) red[warp] = ss;
+    __syncthreads();
+    float t = 0.f;
+#pragma unroll
+    for (int k = 0; k < kWarps; ++k) t += red[k];
+    const float inv = __fdiv_rn(1.f, __fsqrt_rn(__fadd_rn(__fdiv_rn(t, (float)a.in_dim), a.pre_eps)));
+#pragma unroll
+    for (int i = 0; i < kV; ++i) {
+      if (i < S) {
+        if (i * 32 + u0 < a.units)
+          v[i] = make_float4(__fmul_rn(__fmul_rn(v[i].x, inv), nw[i].x), __fmul_rn(__fmul_rn(v[i].y, inv), nw[i].y),
+                             __fmul_rn(__fmul_rn(v[i].z, inv), nw[i].z), __fmul_rn(__fmul_rn(v[i].w, inv), nw[i].w));
+        xs[(i * 8 + slot) * 32 + u0] = v[i];
+      }
+    }
+  } else {
+    for (int i0 = 0; i0 < S; i0 += kV) {
+      float4 v[kV], b[kV];
+#pragma unroll
+      for (int i = 0; i < kV; ++i) {
+        const int unit = (i0 + i) * 32 + u0;
+        const bool in = i0 + i < S && unit < a.units;
+        const float* p = a.x + (size_t)unit * 32 + slot * 4;
+        v[i] = !in ? zero : a.x_aligned ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
+        if (PRE == 2) b[i] = in ? *(reinterpret_cast<const float4*>(a.pre_b) + (i0 + i) * 256 + tid) : zero;
+      }
+#pragma unroll
+      for (int i = 0; i < kV; ++i) {
+        if (i0 + i >= S) break;
+        if (PRE == 2) {  // silu(x) * b; single-precision exp (2 ulp), see mlx_stage_x_pre
+          v[i].x = __fmul_rn(__fdiv_rn(v[i].x, __fadd_rn(1.f, expf(-v[i].x))), b[i].x);
+          v[i].y = __fmul_rn(__fdiv_rn(v[i].y, __fadd_rn(1.f, expf(-v[i].y))), b[i].y);
+          v[i].z = __fmul_rn(__fdiv_rn(v[i].z, __fadd_rn(1.f, expf(-v[i].z))), b[i].z);
+          v[i].w = __fmul_rn(__fdiv_rn(v[i].w, __fadd_rn(1.f, expf(-v[i].w))), b[i].w);
+        }
+        xs[((i0 + i) * 8 + slot) * 32 + u0] = v[i];
+      }
+    }
+  }
+  __syncthreads();
+  float dot[R], cy = 0.f;
+  if (live) {
+    float2 F[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) F[r] = make_float2(0.f, 0.f);
+    float se = 0.f, so = 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float4 xa = xs[(slice * 8 + 2 * k) * 32 + lane], xb = xs[(slice * 8 + 2 * k + 1) * 32 + lane];
+      se += xa.x + xa.z;
+      so += xa.y + xa.w;
+      se += xb.x + xb.z;
+      so += xb.y + xb.w;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        float t[8];
+        if (r < P) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) t[e] = f[r < P ? r : 0][8 * k + e];
+        } else {
+          const uint32_t word = k == 0 ? w[r].x : k == 1 ? w[r].y : k == 2 ? w[r].z : w[r].w;
+          Unpack<MODE>::run(word, t);
+        }
+        fma2(F[r], make_float2(t[0], t[1]), make_float2(xa.x, xa.y));
+        fma2(F[r], make_float2(t[2], t[3]), make_float2(xa.z, xa.w));
+        fma2(F[r], make_float2(t[4], t[5]), make_float2(xb.x, xb.y));
+        fma2(F[r], make_float2(t[6], t[7]), make_float2(xb.z, xb.w));
+      }
+    }
+    const float2 c = mlx_unit_consts<MODE>(se, so);
+    cy = c.y;
+#pragma unroll
+    for (int r = 0; r < R; ++r) dot[r] = (F[r].x + F[r].y) - c.x;
+  }
+  float sc[R], bi[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    if constexpr (SB_BF16) {
+      sc[r] = __uint_as_float(sb[r] << 16);
+      bi[r] = __uint_as_float(sb[r] & 0xFFFF0000u);
+    } else {
+      sc[r] = sb[r].x;
+      bi[r] = sb[r].y;
+    }
+  }
+  if (S > 1) {
+    if (live && slice > 0) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) part[(warp * R + r) * 32 + lane] = make_float4(sc[r], dot[r], bi[r], cy);
+    }
+    __syncthreads();
+  }
+  if (!live || slice > 0) return;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    float acc = fmaf(bi[r], cy, fmaf(sc[r], dot[r], 0.f));
+    for (int s = 1; s < S; ++s) {
+      const float4 q = part[((warp + s) * R + r) * 32 + lane];
+      acc = fmaf(q.x, q.y, acc);
+      acc = fmaf(q.z, q.w, acc);
+    }
+    acc = warp_sum(acc);
+    if (lane == 0 && row0 + r < rows) out[row0 + r] = acc;
+  }
+}
+
 // A list of products in one cooperative launch: every CTA works through the list, and a barrier
 // over the whole grid stands between consecutive products (product k+1 may read what product k
 // wrote).  Each CTA issues its first weight loads of product k+1 before it waits at the barrier,
@@ -802,6 +1001,36 @@ struct MlxPre {
   float eps = 0.f;
 };
 
+typedef void (*MlxRowKernel)(const MlxArgs, int, int);
+
+template <int R>
+static MlxRowKernel pick_row_kernel(int pre, bool bf16) {
+  if (pre == 1) return bf16 ? (MlxRowKernel)mlx_gemv_row_kernel<R, UNPACK_EXACT, true, 1> : (MlxRowKernel)mlx_gemv_row_kernel<R, UNPACK_EXACT, false, 1>;
+  if (pre == 2) return bf16 ? (MlxRowKernel)mlx_gemv_row_kernel<R, UNPACK_EXACT, true, 2> : (MlxRowKernel)mlx_gemv_row_kernel<R, UNPACK_EXACT, false, 2>;
+  return bf16 ? (MlxRowKernel)mlx_gemv_row_kernel<R, UNPACK_EXACT, true, 0> : (MlxRowKernel)mlx_gemv_row_kernel<R, UNPACK_EXACT, false, 0>;
+}
+
+static int launch_row(const MlxArgs& a, int R, int S, int groups, int grid, bool bf16, cudaStream_t stream) {
+  MlxRowKernel k = R == 1 ? pick_row_kernel<1>(a.pre_op, bf16) : R == 2 ? pick_row_kernel<2>(a.pre_op, bf16) : pick_row_kernel<4>(a.pre_op, bf16);
+  const size_t smem = (size_t)S * 8 * 32 * 16 + (S > 1 ? (size_t)kWarps * R * 32 * 16 : 0);
+  if (smem > 48 * 1024)  // (a driver call per launch otherwise: the usual sizes need none)
+    GOPH_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = options().pdl ? 1 : 0;
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof cfg);
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  note_launch();
+  GOPH_CUDA(cudaLaunchKernelEx(&cfg, k, a, S, groups));
+  return GOPH_OK;
+}
+
 static int launch_stream(const goph_mlx_weight* const* ws, float* const* outs, int n, const float* x,
                          int batch, cudaStream_t stream, const MlxPre* pre = nullptr) {
   const goph_mlx_weight* w0 = ws[0];
@@ -830,6 +1059,26 @@ static int launch_stream(const goph_mlx_weight* const* ws, float* const* outs, i
   int M = batch <= 1 ? 1 : batch <= 2 ? 2 : batch <= 4 ? 4 : 8;
   long total_rows = 0;
   for (int i = 0; i < n; ++i) total_rows += ws[i]->out_dim;
+  if (batch == 1 && a.iters <= (a.pre_op == 1 ? 4 : kRowMaxSlices) && options().mlx_unpack == UNPACK_EXACT && options().mlx_rows == 0 &&
+      options().mlx_ctas_per_sm == 0) {
+    // All of it at once?  The fewest rows per warp whose CTAs are resident together (three per SM with one
+    // row, else two); more rows than that run in the looping kernel.
+    const int S = a.iters, groups = kWarps / S;
+    for (int R = 1; R <= 4; R *= 2) {
+      int tasks = 0;
+      for (int i = 0; i < n; ++i) {
+        a.seg[i].w = reinterpret_cast<const uint4*>(ws[i]->qweight);
+        a.seg[i].sb = ws[i]->sb;
+        a.seg[i].out = outs[i];
+        a.seg[i].rows = ws[i]->out_dim;
+        a.seg[i].task0 = tasks;
+        tasks += (ws[i]->out_dim + R - 1) / R;
+      }
+      a.tasks = tasks;
+      const int grid = (tasks + groups - 1) / groups;
+      if (grid <= st.sm_count * (R == 1 ? 3 : 2)) return launch_row(a, R, S, groups, grid, w0->sb_bf16 != 0, stream);
+    }
+  }
   // Rows per warp.  Batches: as many as keep every SM's 16 resident warps busy for two rounds.
   // Batch 1 is latency-bound (every CTA stages the whole x, and a launch costs by the CTA): two rows per
   // warp from 512 rows on.  Measured on the Qwen3-0.6B decode step (145 dependent launches per token,
