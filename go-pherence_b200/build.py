@@ -7,6 +7,7 @@ library has no toolkit dependency at run time beyond the driver.
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -16,6 +17,7 @@ CSRC = os.path.join(HERE, "csrc")
 TUNING = os.environ.get("GOPH_TUNING") == "1"
 OBJ = os.path.join(HERE, "build_tuning" if TUNING else "build")
 LIB = os.path.join(HERE, "libgoph_b200_tuning.so" if TUNING else "libgoph_b200.so")
+PYCALL = os.path.join(HERE, "goph_pycall.so")  # the caller of the C ABI that runtime.py uses
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
@@ -55,7 +57,18 @@ def _compile(src, verbose):
     return obj, True
 
 
+def _build_pycall(force):
+    src = os.path.join(CSRC, "pycall.c")
+    if not force and os.path.exists(PYCALL) and os.path.getmtime(PYCALL) >= os.path.getmtime(src):
+        return
+    cmd = [os.environ.get("CC", "gcc"), "-O2", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"], src, "-o", PYCALL]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("gcc failed for pycall.c:\n%s\n%s" % (r.stdout, r.stderr))
+
+
 def build(force=False, verbose=False):
+    _build_pycall(force)
     os.makedirs(OBJ, exist_ok=True)
     if force:
         for f in os.listdir(OBJ):

@@ -9,7 +9,9 @@ Importing this module never touches the GPU; the first call that needs the libra
 it and fails loudly if it has not been built.
 """
 import ctypes as C
+import importlib.util
 import os
+import struct
 
 import numpy as np
 
@@ -45,6 +47,33 @@ EXPORTS = [
 ]
 
 
+# The entry points that a program calls per step go through goph_pycall (csrc/pycall.c), which takes numbers, None
+# and handles as they are: ctypes makes an object per argument, 1.1 to 2.8 us a call, as much as a small product's
+# launch itself.  p: address or handle, n: element or byte count, i: int, f: float.
+_HOT = {
+    "goph_memset": "ipin",
+    "goph_mlx_gemv": "pnpnpp", "goph_mlx_gemm": "pnpnpip", "goph_mlx_gemm_bf16": "pnpnpip", "goph_mlx_gemm_multi": "ipppnip",
+    "goph_mlx_gemv_pre": "pnpippppfp", "goph_mlx_embed": "pnppp", "goph_mlx_embed_rows": "pnppip",
+    "goph_gguf_project": "pnpnipp", "goph_fp8_gemm": "pnpnipp", "goph_fp8_gemm_bf16": "pnpnipp",
+    "goph_gguf_gate_up_gelu_by_work": "pnpnpiiipp", "goph_gguf_scatter_by_work": "pnpnpppiipp",
+    "goph_moe_forward": "ppnpnip",
+    "goph_add_rmsnorm": "ipppppiifp", "goph_silu_mul": "ipppip", "goph_silu_mul_rows": "ipppiiip",
+    "goph_qk_norm_rope_append": "ippppppppp" + "iiiifp", "goph_attn_decode": "ipppppiiiifp", "goph_argmax_advance": "ipippppip",
+    "goph_qk_norm_rope_append_rows": "ipppiippppppiiiifp", "goph_attn_rows": "ipipiipppiiiifp",
+    "goph_attn_decode_fused": "ipppppppppp" + "iiiiffp",
+}
+
+
+def _pycall():
+    path = os.path.join(_HERE, "goph_pycall.so")
+    if not os.path.exists(path):
+        raise GophError(-1, "goph_pycall.so is not built (run __graft_entry__.build())")
+    spec = importlib.util.spec_from_file_location("goph_pycall", path)
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    return mod
+
+
 class GophError(RuntimeError):
     def __init__(self, code, text):
         super().__init__("goph error %d: %s" % (code, text))
@@ -68,6 +97,9 @@ def lib():
         for name in ("goph_mlx_resident_bytes", "goph_gguf_resident_bytes", "goph_fp8_resident_bytes", "goph_gptq_resident_bytes"):
             getattr(L, name).restype = C.c_uint64
             getattr(L, name).argtypes = [C.c_void_p]
+        call = _pycall()
+        for name, sig in _HOT.items():
+            setattr(L, name, call.Function(C.cast(getattr(L, name), C.c_void_p).value, sig))
         _lib = L
     return _lib
 
@@ -83,7 +115,7 @@ def _vp(a):
 
 def _stream_ptr(stream):
     if stream is None:
-        return C.c_void_p(0)
+        return None
     if hasattr(stream, "cuda_stream"):
         return C.c_void_p(stream.cuda_stream)
     return C.c_void_p(int(stream))
@@ -209,7 +241,7 @@ class GPUMLXWeight:
     """nvidia.GPUMLXWeight (runtime/mlx.go:21-32)."""
 
     def __init__(self, handle, in_dim, out_dim, gs):
-        self._h = handle
+        self._h, self._addr = handle, handle.value or 0
         self.InDim, self.OutDim, self.GroupSz, self.Groups = in_dim, out_dim, gs, in_dim // gs
 
     def ResidentBytes(self):
@@ -218,7 +250,7 @@ class GPUMLXWeight:
     def Free(self):
         if self._h:
             _check(lib().goph_mlx_free(self._h))
-            self._h = None
+            self._h, self._addr = None, 0
 
 
 def UploadMLXWeight(weight, scales, biases, inDim, outDim, groupSize, wantNative=False):
@@ -239,6 +271,12 @@ def UploadMLXWeightNative(weight, scales, biases, inDim, outDim, groupSize):
     return UploadMLXWeight(weight, scales, biases, inDim, outDim, groupSize, True)
 
 
+def _mlx_addr(w):
+    if not isinstance(w, GPUMLXWeight) or not w._addr:
+        raise GophError(1, "nil or freed GPUMLXWeight")
+    return w._addr
+
+
 def _mlx_handle(w):
     if not isinstance(w, GPUMLXWeight) or not w._h:
         raise GophError(1, "nil or freed GPUMLXWeight")
@@ -254,8 +292,9 @@ def GemvMLX(out, x, w, stream=None):
     """nvidia.GemvMLX (runtime/mlx.go:287)."""
     if out is None or x is None:
         raise GophError(1, "nil buffer")
-    _check(lib().goph_mlx_gemv(C.c_void_p(out.Ptr), C.c_uint64(out.n), C.c_void_p(x.Ptr), C.c_uint64(x.n),
-                               _mlx_handle(w), _stream_ptr(stream)))
+    rc = (_lib or lib()).goph_mlx_gemv(out.Ptr, out.Size >> 2, x.Ptr, x.Size >> 2, _mlx_addr(w), _stream_ptr(stream))
+    if rc:
+        _check(rc)
 
 
 def GemvMLXNoAlloc(out, x, w, stream=None):
@@ -290,8 +329,9 @@ def GemmMLX(out, input, w, B, stream=None):
     """nvidia.GemmMLX (runtime/mlx.go:395)."""
     if out is None or input is None:
         raise GophError(1, "nil buffer")
-    _check(lib().goph_mlx_gemm(C.c_void_p(out.Ptr), C.c_uint64(out.n), C.c_void_p(input.Ptr),
-                               C.c_uint64(input.n), _mlx_handle(w), int(B), _stream_ptr(stream)))
+    rc = (_lib or lib()).goph_mlx_gemm(out.Ptr, out.Size >> 2, input.Ptr, input.Size >> 2, _mlx_addr(w), int(B), _stream_ptr(stream))
+    if rc:
+        _check(rc)
 
 
 def to_bf16_bits(a):
@@ -305,18 +345,24 @@ def GemmMLXBF16(out, input, w, B, stream=None):
     B * inDim bf16 bit patterns (2 bytes each)."""
     if out is None or input is None:
         raise GophError(1, "nil buffer")
-    _check(lib().goph_mlx_gemm_bf16(C.c_void_p(out.Ptr), C.c_uint64(out.n), C.c_void_p(input.Ptr),
-                                    C.c_uint64(input.Size // 2), _mlx_handle(w), int(B), _stream_ptr(stream)))
+    rc = (_lib or lib()).goph_mlx_gemm_bf16(out.Ptr, out.Size >> 2, input.Ptr, input.Size >> 1, _mlx_addr(w), int(B), _stream_ptr(stream))
+    if rc:
+        _check(rc)
+
+
+_ADDRESSES = {n: struct.Struct("%dP" % n).pack for n in range(1, 17)}
 
 
 def GemmMLXMulti(outs, x, weights, B=1, stream=None):
     """mlx.Gemv2To generalised (backends/mlx/gemv.go:32-60): several weights, one x, one launch."""
     n = len(weights)
-    if n != len(outs) or n == 0:
+    if n != len(outs) or n == 0 or n > 16:
         raise GophError(1, "outs/weights length mismatch")
-    op = (C.c_void_p * n)(*[o.Ptr for o in outs])
-    wp = (C.c_void_p * n)(*[_mlx_handle(w) for w in weights])
-    _check(lib().goph_mlx_gemm_multi(n, op, wp, C.c_void_p(x.Ptr), C.c_uint64(x.n), int(B), _stream_ptr(stream)))
+    op = _ADDRESSES[n](*[o.Ptr or 0 for o in outs])  # arrays of addresses; the call copies them
+    wp = _ADDRESSES[n](*[_mlx_addr(w) for w in weights])
+    rc = (_lib or lib()).goph_mlx_gemm_multi(n, op, wp, x.Ptr, x.Size >> 2, int(B), _stream_ptr(stream))
+    if rc:
+        _check(rc)
 
 
 def GemmMLXHost(x, w, B=1):
@@ -333,19 +379,20 @@ class GPUGGUFMatrix:
     GPUQ8_0Matrix (runtime/q4k.go:39-47, q8.go:20-25)."""
 
     def __init__(self, handle, qtype, in_dim, out_dim):
-        self._h, self.QType, self.InDim, self.OutDim = handle, qtype, in_dim, out_dim
+        self._h, self._addr, self.QType, self.InDim, self.OutDim = handle, handle.value or 0, qtype, in_dim, out_dim
 
     def ResidentBytes(self):
         return lib().goph_gguf_resident_bytes(self._h) if self._h else 0
 
     def ProjectBatchToBuffer(self, out, x, batch, stream=None):
         """GPUGGUFMatrix.ProjectBatchToBuffer (runtime/gguf_matrix.go:121-135)."""
-        if not self._h:
+        if not self._addr:
             raise GophError(1, "nil or freed GPUGGUFMatrix")
         if out is None or x is None:
             raise GophError(1, "nil buffer")
-        _check(lib().goph_gguf_project(C.c_void_p(out.Ptr), C.c_uint64(out.n), C.c_void_p(x.Ptr),
-                                       C.c_uint64(x.n), int(batch), self._h, _stream_ptr(stream)))
+        rc = (_lib or lib()).goph_gguf_project(out.Ptr, out.Size >> 2, x.Ptr, x.Size >> 2, int(batch), self._addr, _stream_ptr(stream))
+        if rc:
+            _check(rc)
 
     def Dequant(self, out, stream=None):
         if not self._h:
@@ -355,7 +402,7 @@ class GPUGGUFMatrix:
     def Free(self):
         if self._h:
             _check(lib().goph_gguf_free(self._h))
-            self._h = None
+            self._h, self._addr = None, 0
 
 
 def ProjectQ4PairToBuffers(outA, outB, x, batch, a, b, stream=None):
@@ -446,8 +493,7 @@ def GateUpGELUQ4KBatchToBuffer(out, x, batch, intermediate, m, stream=None):
 
 def GateUpGELUQ4KByWorkToBuffer(out, x, workExperts, workLen, intermediate, activeExperts, m, stream=None):
     """nvidia.GateUpGELUQ4KByWorkToBuffer (runtime/q4k.go:322-336); workExperts: device buffer of uint32."""
-    _check(lib().goph_gguf_gate_up_gelu_by_work(C.c_void_p(out.Ptr), C.c_uint64(out.n), C.c_void_p(x.Ptr), C.c_uint64(x.n),
-                                                C.c_void_p(workExperts.Ptr), int(workLen), int(intermediate),
+    _check(lib().goph_gguf_gate_up_gelu_by_work(out.Ptr, out.Size >> 2, x.Ptr, x.Size >> 2, workExperts.Ptr, int(workLen), int(intermediate),
                                                 int(activeExperts), m._h, _stream_ptr(stream)))
 
 
@@ -459,8 +505,7 @@ def GemvQ8_0BatchScatter(dst, x, pos, weight, batch, m, stream=None):
 
 def GemvQ8_0ScatterByWork(dst, x, workActive, workPos, workWeight, workLen, activeExperts, m, stream=None):
     """nvidia.GemvQ8_0ScatterByWork (runtime/q8.go:193-207)."""
-    _check(lib().goph_gguf_scatter_by_work(C.c_void_p(dst.Ptr), C.c_uint64(dst.n), C.c_void_p(x.Ptr), C.c_uint64(x.n),
-                                           C.c_void_p(workActive.Ptr), C.c_void_p(workPos.Ptr), C.c_void_p(workWeight.Ptr),
+    _check(lib().goph_gguf_scatter_by_work(dst.Ptr, dst.Size >> 2, x.Ptr, x.Size >> 2, workActive.Ptr, workPos.Ptr, workWeight.Ptr,
                                            int(workLen), int(activeExperts), m._h, _stream_ptr(stream)))
 
 
@@ -588,7 +633,7 @@ class GPUFP8E4M3Linear:
     """nvidia.GPUFP8E4M3Linear (runtime/fp8.go:35-44)."""
 
     def __init__(self, handle, out_dim, in_dim):
-        self._h, self.OutDim, self.InDim = handle, out_dim, in_dim
+        self._h, self._addr, self.OutDim, self.InDim = handle, handle.value or 0, out_dim, in_dim
 
     def ResidentBytes(self):
         return lib().goph_fp8_resident_bytes(self._h) if self._h else 0
@@ -596,7 +641,7 @@ class GPUFP8E4M3Linear:
     def Free(self):
         if self._h:
             _check(lib().goph_fp8_free(self._h))
-            self._h = None
+            self._h, self._addr = None, 0
 
 
 def UploadFP8E4M3Linear(weight, scale, bias, outDim, inDim):
@@ -613,6 +658,12 @@ def UploadFP8E4M3Linear(weight, scale, bias, outDim, inDim):
     return GPUFP8E4M3Linear(h, int(outDim), int(inDim))
 
 
+def _fp8_addr(w):
+    if not isinstance(w, GPUFP8E4M3Linear) or not w._addr:
+        raise GophError(1, "nil or freed GPUFP8E4M3Linear")
+    return w._addr
+
+
 def _fp8_handle(w):
     if not isinstance(w, GPUFP8E4M3Linear) or not w._h:
         raise GophError(1, "nil or freed GPUFP8E4M3Linear")
@@ -623,8 +674,9 @@ def GemmFP8E4M3Buffer(out, x, batch, w, stream=None):
     """nvidia.GemmFP8E4M3Buffer (runtime/fp8.go:271)."""
     if out is None or x is None:
         raise GophError(1, "nil buffer")
-    _check(lib().goph_fp8_gemm(C.c_void_p(out.Ptr), C.c_uint64(out.n), C.c_void_p(x.Ptr), C.c_uint64(x.n),
-                               int(batch), _fp8_handle(w), _stream_ptr(stream)))
+    rc = (_lib or lib()).goph_fp8_gemm(out.Ptr, out.Size >> 2, x.Ptr, x.Size >> 2, int(batch), _fp8_addr(w), _stream_ptr(stream))
+    if rc:
+        _check(rc)
 
 
 def GemmFP8E4M3BF16Buffer(out, x, batch, w, stream=None):
@@ -632,8 +684,9 @@ def GemmFP8E4M3BF16Buffer(out, x, batch, w, stream=None):
     of batch * inDim bf16 bit patterns."""
     if out is None or x is None:
         raise GophError(1, "nil buffer")
-    _check(lib().goph_fp8_gemm_bf16(C.c_void_p(out.Ptr), C.c_uint64(out.n), C.c_void_p(x.Ptr), C.c_uint64(x.Size // 2),
-                                    int(batch), _fp8_handle(w), _stream_ptr(stream)))
+    rc = (_lib or lib()).goph_fp8_gemm_bf16(out.Ptr, out.Size >> 2, x.Ptr, x.Size >> 1, int(batch), _fp8_addr(w), _stream_ptr(stream))
+    if rc:
+        _check(rc)
 
 
 def GemvFP8E4M3Buffer(out, x, w, stream=None):
@@ -693,8 +746,9 @@ class GPUMoELayer:
 
     def Forward(self, out, x, tokens=1, stream=None):
         """moeForwardGPU for `tokens` rows of x (model/moe_gpu.go:49)."""
-        _check(lib().goph_moe_forward(self._handle(), C.c_void_p(out.Ptr), C.c_uint64(out.n), C.c_void_p(x.Ptr),
-                                      C.c_uint64(x.n), int(tokens), _stream_ptr(stream)))
+        rc = (_lib or lib()).goph_moe_forward(self._handle(), out.Ptr, out.Size >> 2, x.Ptr, x.Size >> 2, int(tokens), _stream_ptr(stream))
+        if rc:
+            _check(rc)
 
     def ForwardLogits(self, out, x, logits, tokens=1, stream=None):
         """The selected-expert projection with router logits supplied by the caller."""
@@ -808,24 +862,24 @@ class Gather:
 
 # ------------------------------------------------------------------------------ decode-step operations
 def _ptr(b):
-    return C.c_void_p(b.Ptr if b is not None else 0)
+    return b.Ptr if b is not None else None
 
 
 def AddRMSNorm(hidden, normed, a, b, weight, n, rows=1, eps=1e-6, stream=None):
     """hidden = a (+ b); normed = RMSNorm(hidden) * weight (simd.RMSNorm after the residual add)."""
     _check(lib().goph_add_rmsnorm(_device, _ptr(hidden), _ptr(normed), _ptr(a), _ptr(b), _ptr(weight), int(n), int(rows),
-                                  C.c_float(eps), _stream_ptr(stream)))
+                                  eps, _stream_ptr(stream)))
 
 
 def QKNormRoPEAppend(q, k, v, qNorm, kNorm, ropeTable, pos, kCache, vCache, maxSeq, heads, kvHeads, headDim, eps=1e-6, stream=None):
     _check(lib().goph_qk_norm_rope_append(_device, _ptr(q), _ptr(k), _ptr(v), _ptr(qNorm), _ptr(kNorm), _ptr(ropeTable),
                                           _ptr(pos), _ptr(kCache), _ptr(vCache), int(maxSeq), int(heads), int(kvHeads), int(headDim),
-                                          C.c_float(eps), _stream_ptr(stream)))
+                                          eps, _stream_ptr(stream)))
 
 
 def AttnDecode(out, q, kCache, vCache, pos, maxSeq, heads, kvHeads, headDim, scale, stream=None):
     _check(lib().goph_attn_decode(_device, _ptr(out), _ptr(q), _ptr(kCache), _ptr(vCache), _ptr(pos), int(maxSeq), int(heads),
-                                  int(kvHeads), int(headDim), C.c_float(scale), _stream_ptr(stream)))
+                                  int(kvHeads), int(headDim), scale, _stream_ptr(stream)))
 
 
 def QKNormRoPEAppendRows(q, k, v, rowStride, rows, qNorm, kNorm, ropeTable, pos, kCache, vCache, maxSeq, heads, kvHeads, headDim,
@@ -833,13 +887,13 @@ def QKNormRoPEAppendRows(q, k, v, rowStride, rows, qNorm, kNorm, ropeTable, pos,
     """QKNormRoPEAppend for the tokens of a prompt chunk at consecutive positions."""
     _check(lib().goph_qk_norm_rope_append_rows(_device, _ptr(q), _ptr(k), _ptr(v), int(rowStride), int(rows), _ptr(qNorm), _ptr(kNorm),
                                                _ptr(ropeTable), _ptr(pos), _ptr(kCache), _ptr(vCache), int(maxSeq), int(heads),
-                                               int(kvHeads), int(headDim), C.c_float(eps), _stream_ptr(stream)))
+                                               int(kvHeads), int(headDim), eps, _stream_ptr(stream)))
 
 
 def AttnRows(out, outStride, q, qStride, rows, kCache, vCache, pos, maxSeq, heads, kvHeads, headDim, scale, stream=None):
     """AttnDecode for the tokens of a prompt chunk, each over the positions up to its own."""
     _check(lib().goph_attn_rows(_device, _ptr(out), int(outStride), _ptr(q), int(qStride), int(rows), _ptr(kCache), _ptr(vCache),
-                                _ptr(pos), int(maxSeq), int(heads), int(kvHeads), int(headDim), C.c_float(scale), _stream_ptr(stream)))
+                                _ptr(pos), int(maxSeq), int(heads), int(kvHeads), int(headDim), scale, _stream_ptr(stream)))
 
 
 def SiLUMulRows(out, gate, up, n, inStride, rows, stream=None):
@@ -847,7 +901,7 @@ def SiLUMulRows(out, gate, up, n, inStride, rows, stream=None):
 
 
 def EmbedMLXRows(out, w, toks, rows, stream=None):
-    _check(lib().goph_mlx_embed_rows(_ptr(out), C.c_uint64(out.n), _mlx_handle(w), _ptr(toks), int(rows), _stream_ptr(stream)))
+    _check(lib().goph_mlx_embed_rows(_ptr(out), out.Size >> 2, _mlx_addr(w), _ptr(toks), int(rows), _stream_ptr(stream)))
 
 
 def SiLUMul(out, gate, up, n, stream=None):
@@ -860,13 +914,13 @@ def ArgmaxAdvance(logits, n, tok, pos, history, forced, historyCap, stream=None)
 
 
 def EmbedMLX(out, w, tok, stream=None):
-    _check(lib().goph_mlx_embed(_ptr(out), C.c_uint64(out.n), _mlx_handle(w), _ptr(tok), _stream_ptr(stream)))
+    _check(lib().goph_mlx_embed(_ptr(out), out.Size >> 2, _mlx_addr(w), _ptr(tok), _stream_ptr(stream)))
 
 
 def GemvMLXPre(out, w, preOp, x, b, normW, hiddenOut, eps=1e-6, stream=None):
     """out = W . f(x): preOp 1 = RMSNorm(x (+ b)) * normW with hiddenOut = x (+ b); preOp 2 = silu(x) * b."""
-    _check(lib().goph_mlx_gemv_pre(_ptr(out), C.c_uint64(out.n), _mlx_handle(w), int(preOp), _ptr(x), _ptr(b), _ptr(normW),
-                                   _ptr(hiddenOut), C.c_float(eps), _stream_ptr(stream)))
+    _check(lib().goph_mlx_gemv_pre(_ptr(out), out.Size >> 2, _mlx_addr(w), int(preOp), _ptr(x), _ptr(b), _ptr(normW),
+                                   _ptr(hiddenOut), eps, _stream_ptr(stream)))
 
 
 def AttnDecodeFused(out, q, k, v, qNorm, kNorm, ropeTable, pos, kCache, vCache, maxSeq, heads, kvHeads, headDim, scale,
@@ -874,4 +928,4 @@ def AttnDecodeFused(out, q, k, v, qNorm, kNorm, ropeTable, pos, kCache, vCache, 
     """QKNormRoPEAppend + AttnDecode in one launch (q, k, v: raw projection outputs of the current position)."""
     _check(lib().goph_attn_decode_fused(_device, _ptr(out), _ptr(q), _ptr(k), _ptr(v), _ptr(qNorm), _ptr(kNorm), _ptr(ropeTable),
                                         _ptr(pos), _ptr(kCache), _ptr(vCache), int(maxSeq), int(heads), int(kvHeads),
-                                        int(headDim), C.c_float(scale), C.c_float(eps), _stream_ptr(stream)))
+                                        int(headDim), scale, eps, _stream_ptr(stream)))
