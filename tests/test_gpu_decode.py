@@ -86,6 +86,42 @@ def test_qk_norm_rope_append_and_attention(gpu, pkg, heads, kv_heads, head_dim, 
             t.Free()
 
 
+@pytest.mark.parametrize("max_seq,positions", [(1, (0,)), (32, (0, 7, 31)), (33, (31, 32)), (64, (32, 63)), (129, (63, 64, 127, 128)),
+                                               (256, (0, 95, 224, 255)), (257, (255, 256))])
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(4, 2, 64), (6, 2, 128), (3, 3, 256)])
+def test_fused_attention_of_a_short_cache(gpu, pkg, heads, kv_heads, head_dim, max_seq, positions):
+    """The edges of a warp's, a CTA's and a cluster's positions; rows past the position hold NaN.  Tolerances as above."""
+    g = pkg.synth.rng("short", max_seq, head_dim)
+    kvd = kv_heads * head_dim
+    table = od.rope_table(max_seq, head_dim, 1e6)
+    T = gpu.from_numpy(table.reshape(-1))
+    qn, kn = (1 + 0.1 * g.standard_normal((2, head_dim))).astype(F)
+    QN, KN = gpu.from_numpy(qn), gpu.from_numpy(kn)
+    scale = 1.0 / np.sqrt(head_dim)
+    for pos in positions:
+        ref_k, ref_v = g.standard_normal((2, max_seq, kvd), dtype=F)
+        ref_k[pos:], ref_v[pos:] = np.nan, np.nan
+        kc, vc = gpu.from_numpy(ref_k.reshape(-1)), gpu.from_numpy(ref_v.reshape(-1))
+        q, k, v = g.standard_normal(heads * head_dim, dtype=F), g.standard_normal(kvd, dtype=F), g.standard_normal(kvd, dtype=F)
+        Q, K, V, P = gpu.from_numpy(q), gpu.from_numpy(k), gpu.from_numpy(v), gpu.from_numpy(np.array([pos], dtype=np.int32))
+        out = gpu.Malloc(heads * head_dim)
+        gpu.AttnDecodeFused(out, Q, K, V, QN, KN, T, P, kc, vc, max_seq, heads, kv_heads, head_dim, scale, 1e-6)
+        gpu.Sync()
+        rq = np.concatenate([od.rmsnorm(q[h * head_dim:(h + 1) * head_dim], qn, 1e-6) for h in range(heads)]).astype(F)
+        rk = np.concatenate([od.rmsnorm(k[h * head_dim:(h + 1) * head_dim], kn, 1e-6) for h in range(kv_heads)]).astype(F)
+        od.apply_rope(rq, table, pos, heads, head_dim)
+        od.apply_rope(rk, table, pos, kv_heads, head_dim)
+        ref_k[pos], ref_v[pos] = rk, v
+        assert np.allclose(kc.Download().reshape(max_seq, kvd)[pos], rk, rtol=1e-5, atol=1e-6)
+        assert np.array_equal(vc.Download().reshape(max_seq, kvd)[pos], v)
+        want = od.attention(rq, ref_k, ref_v, pos + 1, heads, kv_heads, head_dim, scale)
+        assert np.allclose(out.Download(), want, rtol=1e-4, atol=2e-5)
+        for b in (kc, vc, Q, K, V, P, out):
+            b.Free()
+    for b in (T, QN, KN):
+        b.Free()
+
+
 @pytest.mark.parametrize("fused", [False, True])
 @pytest.mark.parametrize("bad_pos", [16, -1, 1 << 20])
 def test_position_outside_the_cache_is_refused(gpu, pkg, fused, bad_pos):
