@@ -82,6 +82,7 @@ constexpr int kThreads = (kWarpW + 1) * 32;
 // row's sums of 64 columns, takes what the others give up: 256 * 128 + 512 * 48 + 128 * 56 = 64512.
 constexpr int kEpiRegs = 128, kConvRegs = 48, kMiscRegs = 56;
 constexpr int kMaxSplits = 8;
+constexpr int kMaxRows = 256;                       // activation rows of one launch
 
 // What a format's slot of the weight ring looks like: [weights][row metadata].
 template <int F, bool TILED>
@@ -603,6 +604,7 @@ qg_kernel(const __grid_constant__ QArgs a) {
   volatile int* pieces = reinterpret_cast<volatile int*>(bars + 2 * SW + 2 * SB + 48);  // [SB] pieces in the slot
   uint32_t* tmem_holder = const_cast<uint32_t*>(reinterpret_cast<volatile uint32_t*>(pieces + SB));
   float* xinv = reinterpret_cast<float*>(tmem_holder + 1);  // [kMaxRows]
+  volatile int* shared_item = reinterpret_cast<volatile int*>(xinv + kMaxRows);  // the cluster's item: group (or -1), block, split
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
@@ -1026,81 +1028,88 @@ qg_kernel(const __grid_constant__ QArgs a) {
       }
     }
     if (a.splits > 1) {
-      // The K splits of the last item are the CTAs of this cluster (rank == split).  Each thread hands its
-      // sums, four columns a store, to the CTAs that finish the columns, a share of them each, which add in
-      // split order and store.  (A float a store took 14 us for 64 columns of two tiles: a remote store costs
-      // by the instruction.)  They land in the rings, in which nothing is in flight any more: here, and after
-      // the first meeting in the peers.
-      __syncwarp();
-      const int n = block_cols<NB>(a, wk.nb), S = a.splits, sg = ((n + S - 1) / S + 3) / 4;  // sg: groups of four columns of a share
-      if constexpr (!kItemBlock) {
-        if (wk.live) combine(n);
+      // the sums of the item that the cluster shares go to the CTA's own rings, which are idle once both
+      // pipes' blocks have been read: [pipe][group of four columns][row]
+      asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
+      if (tid == kConvWarps * 32) {
+        shared_item[0] = wk.live ? wk.group : -1;
+        shared_item[1] = wk.nb;
+        shared_item[2] = wk.split;
       }
-      cluster_sync_all();
+      float4* ring = reinterpret_cast<float4*>(wring) + (size_t)w * (NB / 4) * kTileRows + r;
       if (wk.live) {
-        const uint32_t at = smem_u32(wring) + (uint32_t)((wk.split * TT + t) * sg * kTileRows + r) * 16;
-        int owner = 0, left = sg;
-        uint32_t dst = cluster_map(at, 0);
-        auto send = [&](bool mine, float x, float y, float z, float v) {
-          if (mine)
-            asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "f"(x), "f"(y), "f"(z), "f"(v) : "memory");
-          dst += kTileRows * 16;
-          if (--left == 0 && ++owner < S) {
-            left = sg;
-            dst = cluster_map(at, owner);
-          }
-        };
         if constexpr (kItemBlock) {
           // (the block is still in TMEM: nothing has been opened after it)
-          const uint32_t d0 = dbase;
           tc_fence_after();
 #pragma unroll 1
-          for (int j0 = 0; j0 < n; j0 += 16) {
+          for (int j0 = 0; j0 < block_cols<NB>(a, wk.nb); j0 += 16) {
             uint32_t d[16];
-            tmem_ld16(d0 + j0, d);
+            tmem_ld16(dbase + j0, d);
             tmem_wait_ld(d);
 #pragma unroll
             for (int j = 0; j < 16; j += 4)
-              send(true, __uint_as_float(d[j]), __uint_as_float(d[j + 1]), __uint_as_float(d[j + 2]), __uint_as_float(d[j + 3]));
+              ring[(j0 + j) / 4 * kTileRows] = make_float4(__uint_as_float(d[j]), __uint_as_float(d[j + 1]), __uint_as_float(d[j + 2]), __uint_as_float(d[j + 3]));
           }
         } else {
 #pragma unroll
-          for (int g = 0; g < NB / 4; ++g)
-            if (4 * g < n) send(TT == 2 || (g & 1) == w, acc[2 * g].x, acc[2 * g].y, acc[2 * g + 1].x, acc[2 * g + 1].y);
+          for (int g = 0; g < NB / 4; ++g) ring[g * kTileRows] = make_float4(acc[2 * g].x, acc[2 * g].y, acc[2 * g + 1].x, acc[2 * g + 1].y);
         }
       }
-      cluster_sync_all();
-      if (wk.live && ok) {
-        const int row = (wk.group * TT + t) * kTileRows + r, m0 = wk.nb * NB, c0 = wk.split * sg * 4;
-        const float rs = F == Q_FP8 && row < a.out_dim ? __ldg(a.scale + row) : 1.f, rb = F == Q_FP8 && a.bias && row < a.out_dim ? __ldg(a.bias + row) : 0.f;
-        const float4* in = reinterpret_cast<const float4*>(wring) + (size_t)t * sg * kTileRows + r;
-#pragma unroll 2
-        for (int g = TT == 1 ? w : 0; g < sg; g += TT == 1 ? 2 : 1) {
-          if (c0 + 4 * g >= n) break;
-          float v[4] = {0.f, 0.f, 0.f, 0.f};
-          for (int s2 = 0; s2 < S; ++s2) {
-            const float4 q = in[(size_t)(s2 * TT * sg + g) * kTileRows];
-            v[0] += q.x;
-            v[1] += q.y;
-            v[2] += q.z;
-            v[3] += q.w;
-          }
+      if (e == 0) { MARK(7, 2); }
+    }
+  }
+  if (a.splits > 1) {
+    // The K splits of the last item are the CTAs of this cluster (rank == split), and each finishes a share of
+    // the columns with all of its warps: the others' sums, four columns a load, added in split order (TT = 1:
+    // two a split, one from each pipe), and stored.  Everything here runs once, so what it costs is fetching
+    // its instructions: short loops, hardly unrolled.  (B200, us a call, with
+    // sums pushed to their owners and eight warps at the end: Q4_K 14336x4096 x64 33.8 -> 31.6, MLX4 6144x4096
+    // x100 24.8 -> 22.7, bf16 8192x8192 x64 25.6 -> 24.4.)
+    __syncwarp();
+    cluster_sync_all();
+    const int group = shared_item[0], nb = shared_item[1];
+    if (warp == 0) { MARK(7, 3); }
+    if (group >= 0 && warp < kWarpMMA) {
+      constexpr int kPipes = 3 - TT;  // parts of a split's sum
+      const int n = block_cols<NB>(a, nb), S = a.splits, sg = ((n + S - 1) / S + 3) / 4, r = tid & (kTileRows - 1);
+      const int g0 = shared_item[2] * sg, ng = (g0 + sg < n / 4 ? g0 + sg : n / 4) - g0;
+#pragma unroll 1
+      for (int u = warp >> 2; u < ng * TT; u += kWarpMMA / 4) {
+        const int t = TT == 2 && u >= ng ? 1 : 0, g = g0 + u - t * ng, row = (group * TT + t) * kTileRows + r;
+        const uint32_t at = smem_u32(wring) + (uint32_t)((t * (NB / 4) + g) * kTileRows + r) * 16;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+        for (int s0 = 0; s0 < S; s0 += 2 * TT) {
+          float4 q[4];
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
-            const int m = m0 + c0 + 4 * g + k;
-            if (m < a.batch && row < a.out_dim) {
-              const float y = (v[k] * T::kUnit) * xinv[m];
-              a.out[(size_t)m * a.out_dim + row] = F == Q_FP8 ? fmaf(y, rs, rb) : y;
-            }
+            const int s2 = s0 + k / kPipes;
+            q[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (s2 < S)
+              asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(q[k].x), "=f"(q[k].y), "=f"(q[k].z), "=f"(q[k].w)
+                           : "r"(cluster_map(at + (k % kPipes) * (NB * kTileRows * 4), s2)) : "memory");
+          }
+#pragma unroll
+          for (int k = 0; k < 4; ++k) v = make_float4(v.x + q[k].x, v.y + q[k].y, v.z + q[k].z, v.w + q[k].w);
+        }
+        if (row >= a.out_dim) continue;
+        const float rs = F == Q_FP8 ? __ldg(a.scale + row) : 1.f, rb = F == Q_FP8 && a.bias ? __ldg(a.bias + row) : 0.f;
+        const int m = nb * NB + 4 * g;
+        float* o = a.out + (size_t)m * a.out_dim + row;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (m + j < a.batch) {
+            const float y = ((j == 0 ? v.x : j == 1 ? v.y : j == 2 ? v.z : v.w) * T::kUnit) * xinv[m + j];
+            o[(size_t)j * a.out_dim] = F == Q_FP8 ? fmaf(y, rs, rb) : y;
           }
         }
       }
     }
-  }
-  if (a.splits > 1 && (warp < kConvWarps || warp >= kWarpMMA)) {  // the other roles meet the cluster too
     __syncwarp();
-    cluster_sync_all();
-    cluster_sync_all();
+    if (warp == 0) { MARK(7, 5); }
+    // nobody leaves while its sums are being read (they are in registers and added by now: nothing to publish)
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+    if (warp == 0) { MARK(7, 6); }
   }
   // (the next kernel's CTAs are asked for now and not at the start: the preparation kernel of a following
   // product would crowd onto the few SMs this one leaves free and do all its work there)
@@ -1129,7 +1138,6 @@ qg_kernel(const __grid_constant__ QArgs a) {
 // ---- host side ---------------------------------------------------------------------------------------
 
 constexpr int kMaxIn = 65536;
-constexpr int kMaxRows = 256;                       // activation rows of one launch
 constexpr size_t kXbBytes = (size_t)64 << 20;       // prepared activations
 constexpr size_t kXauxBytes = (size_t)(kMaxRows / 64) * (kMaxIn / kChunkK) * 64 * 64;
 constexpr size_t kFlagBytes = (size_t)(kMaxRows / 64) * (kMaxIn / kChunkK) * 64;
