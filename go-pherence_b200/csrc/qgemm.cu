@@ -607,35 +607,54 @@ qg_kernel(const __grid_constant__ QArgs a) {
   volatile int* shared_item = reinterpret_cast<volatile int*>(xinv + kMaxRows);  // the cluster's item: group (or -1), block, split
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid == 0) {
-    for (int s = 0; s < SW; ++s) {
-      mbar_init(wfull + 8 * s, TILED ? 1 : 32);
-      mbar_init(wempty + 8 * s, TT == 2 ? 8 + (kLong ? 0 : 4) : 2 * (4 + (kLong ? 0 : 4)));
+  Walk wk(a);
+  auto load_weights = [&](int s, int t, int c) {  // the W loader: chunk c of the item's tile t into slot s
+    int tile = wk.group * TT + t;
+    if (tile >= a.ntiles) tile = a.ntiles - 1;  // the last group of an odd tile count repeats its tile (nothing of the copy is stored)
+    const uint32_t slot = smem_u32(wring) + s * T::kSlot;
+    if (!TILED) {
+      load_rows<F>(a, slot, tile, c, lane);
+      cp_async_arrive(wfull + 8 * s);
+    } else if (lane == 0) {
+      mbar_expect_tx(wfull + 8 * s, T::kSlot);
+      bulk_load_1d(slot, a.w + ((size_t)tile * a.nchunks + c) * T::kSlot, T::kSlot, wfull + 8 * s);
     }
-    for (int s = 0; s < SB; ++s) {
-      mbar_init(bfull + 8 * s, 1);
-      mbar_init(bempty + 8 * s, TT);
-    }
-    for (int s = 0; s < 8; ++s) {
-      mbar_init(aready + 8 * s, 4);
-      mbar_init(afree + 8 * s, 1);
-    }
-    for (int s = 0; s < 16; ++s) {
-      mbar_init(dfull + 8 * s, 1);
-      mbar_init(dfree + 8 * s, 4);
+  };
+  // The set-up, spread over four warps (by one thread it took 1.7 us with what follows it): the first two
+  // weight stages, which do not depend on the kernel in front, are asked for before anything else.
+  const int early = !wk.live ? 0 : TT == 2 || wk.c + 1 < wk.c1 ? 2 : 1;
+  if (warp == kWarpW) {
+    if (lane < SW) {
+      mbar_init(wfull + 8 * lane, TILED ? 1 : 32);
+      mbar_init(wempty + 8 * lane, TT == 2 ? 8 + (kLong ? 0 : 4) : 2 * (4 + (kLong ? 0 : 4)));
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == kWarpMMA) {
+    __syncwarp();
+    for (int i = 0; i < early; ++i) load_weights(i, TT == 2 ? i : 0, wk.chunk(TT == 2 ? wk.c : wk.c + i));
+  } else if (warp == kWarpB) {
+    if (lane < SB) {
+      mbar_init(bfull + 8 * lane, 1);
+      mbar_init(bempty + 8 * lane, TT);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  } else if (warp == kWarpMMA) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_holder)), "r"(kCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  } else if (warp == kWarpMMA + 1) {
+    if (lane < 8) {
+      mbar_init(aready + 8 * lane, 4);
+      mbar_init(afree + 8 * lane, 1);
+    } else if (lane < 24) {
+      mbar_init(dfull + 8 * (lane - 8), 1);
+      mbar_init(dfree + 8 * (lane - 8), 4);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_holder;  // A: columns [pipe][kAB][64], then D: [pipe][DT][a.dcol]
   bool ok = true;
-  Walk wk(a);
   // is the affine term of the item's i-th chunk this pipe's, and with which unit of the chunk
   auto aux_here = [&](int w, int i, int u) { return T::kAux != 0 && (TT == 2 ? u == 1 : (i & 1) == w); };
 
@@ -643,11 +662,6 @@ qg_kernel(const __grid_constant__ QArgs a) {
     // ------------------------------------------------------------------ weights
     reg_dec<kMiscRegs>();
     if (!TILED || lane == 0) {
-      auto slot_at = [&](int s) { return smem_u32(wring) + s * T::kSlot; };
-      auto tile_of = [&](int t) {  // the last group of an odd tile count repeats its tile (nothing of the copy is stored)
-        const int tile = wk.group * TT + t;
-        return tile < a.ntiles ? tile : a.ntiles - 1;
-      };
       RingCursor cur;
       int i = 0;
       for (; wk.live && ok; wk.next_item(a)) {
@@ -655,21 +669,14 @@ qg_kernel(const __grid_constant__ QArgs a) {
           const int c = wk.chunk(ci);
 #pragma unroll 1
           for (int t = 0; t < TT; ++t, ++i, cur.next(SW)) {
-            const int s = cur.s;
-            // The weights do not depend on the kernel in front.  Only the first two stages are asked for at
-            // once, the rest of the ring when the first is in (a grid that asked for all its rings at once
-            // would see every first stage land last).
-            if (i == 2) ok = mbar_wait(wfull, 0, a.status, 801);
-            if (ok && i >= SW) ok = mbar_wait(wempty + 8 * s, cur.ph ^ 1u, a.status, 802);
+            // The first two stages have been asked for, the rest of the ring follows when the first is in (a
+            // grid that asked for all its rings at once would see every first stage land last).
+            if (i < early) continue;
+            if (i == early) ok = mbar_wait(wfull, 0, a.status, 801);
+            if (ok && i >= SW) ok = mbar_wait(wempty + 8 * cur.s, cur.ph ^ 1u, a.status, 802);
             if (!ok) break;
             if (lane == 0) { MARK(0, i); }
-            if (TILED) {
-              mbar_expect_tx(wfull + 8 * s, T::kSlot);
-              bulk_load_1d(slot_at(s), a.w + ((size_t)tile_of(t) * a.nchunks + c) * T::kSlot, T::kSlot, wfull + 8 * s);
-            } else {
-              load_rows<F>(a, slot_at(s), tile_of(t), c, lane);
-              cp_async_arrive(wfull + 8 * s);
-            }
+            load_weights(cur.s, t, c);
           }
         }
       }
@@ -692,14 +699,24 @@ qg_kernel(const __grid_constant__ QArgs a) {
       if (col + 1 < a.batch) v = max(v, (uint32_t)__ldcg(f + 2 * lane + 1));
       return v;
     };
+    auto load_half = [&](int s, int ci, int h, int P) {  // half chunk h of the item's step ci, P pieces; returns the bytes
+      const int n = block_cols<NB>(a, wk.nb), c = wk.chunk(ci);
+      const uint32_t bytes = n * 256, axb = T::kAux * n * 32, dst = smem_u32(bring) + s * a.bslot;  // bytes: of a piece
+      bulk_load_1d(dst, a.xb + (size_t)wk.nb * a.xb_stride + (size_t)(2 * c + h) * a.pmax * bytes, P * bytes, bfull + 8 * s);
+      const bool ax = TT == 2 ? aux_here(0, 0, h) : aux_here(h, ci - wk.c, 0);
+      if (ax) bulk_load_1d(dst + a.pmax * bytes, a.xaux + ((size_t)wk.nb * a.nchunks + c) * (T::kAux * 32 * NB), axb, bfull + 8 * s);
+      return P * bytes + (ax ? axb : 0);
+    };
+    // the first two half chunks come whole, so that they need not wait for the flags
+    uint32_t first0 = 0, first1 = 0;
+    if (wk.live && lane == 0) {
+      first0 = load_half(0, wk.c, 0, a.pmax);
+      first1 = load_half(1, wk.c, 1, a.pmax);
+    }
+    bool first = true;
     for (; wk.live && ok; wk.next_item(a)) {
-      const int n = block_cols<NB>(a, wk.nb);
-      const uint32_t bytes = n * 256;  // of a piece
-      const unsigned char* src = a.xb + (size_t)wk.nb * a.xb_stride;
-      const unsigned char* asrc = a.xaux + (size_t)wk.nb * a.nchunks * (T::kAux * 32 * NB);
       uint32_t nxt = used_of(wk, wk.chunk(wk.c));
       for (int ci = wk.c; ci < wk.c1 && ok; ++ci) {
-        const int c = wk.chunk(ci);
         const uint32_t cur = nxt;
         if (ci + 1 < wk.c1) nxt = used_of(wk, wk.chunk(ci + 1));
         const int P = (int)__reduce_max_sync(0xffffffffu, cur);
@@ -709,17 +726,15 @@ qg_kernel(const __grid_constant__ QArgs a) {
           if (wrapped) ok = __all_sync(0xffffffffu, mbar_wait(bempty + 8 * s, bc.ph ^ 1u, a.status, 803));
           if (!ok) break;
           if (lane == 0) {
-            const bool ax = TT == 2 ? aux_here(0, 0, h) : aux_here(h, ci - wk.c, 0);
-            const uint32_t dst = smem_u32(bring) + s * a.bslot, axb = T::kAux * n * 32;
             pieces[s] = P;
-            mbar_expect_tx(bfull + 8 * s, P * bytes + (ax ? axb : 0));
-            bulk_load_1d(dst, src + (size_t)(2 * c + h) * a.pmax * bytes, P * bytes, bfull + 8 * s);
-            if (ax) bulk_load_1d(dst + a.pmax * bytes, asrc + (size_t)c * (T::kAux * 32 * NB), axb, bfull + 8 * s);
+            const uint32_t bytes = first ? (h ? first1 : first0) : load_half(s, ci, h, P);
+            mbar_expect_tx(bfull + 8 * s, bytes);
           }
           __syncwarp();
           bc.next(SB);
           wrapped = wrapped || bc.s == 0;
         }
+        first = false;
       }
     }
   } else if (warp >= kWarpMMA) {
