@@ -425,7 +425,7 @@ __device__ __forceinline__ void mlx_gemv_body(const MlxArgs& a, unsigned char* s
 template <int MODE, bool SB_BF16, class Wait>
 __device__ __forceinline__ void mlx_list_body(const MlxArgs& a, unsigned char* smem_raw, int cta, int nctas, Wait wait) {
   float4* xs = reinterpret_cast<float4*>(smem_raw);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // (uniform, for the compiler)
   const int task_stride = nctas * kWarps, iters = a.iters, units = a.units;
   typedef typename std::conditional<SB_BF16, uint32_t, float2>::type SbT;
   constexpr int D = 4, P = 2;
@@ -603,7 +603,7 @@ mlx_gemv_row_kernel(const __grid_constant__ MlxArgs a, int S, int groups_per_cta
   __shared__ float red[kWarps];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   typedef typename std::conditional<SB_BF16, uint32_t, float2>::type SbT;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (uniform, for the compiler)
   const int grp = warp / S, slice = warp - grp * S;
   const int task = (int)blockIdx.x * groups_per_cta + grp;
   const bool live = grp < groups_per_cta && task < a.tasks;

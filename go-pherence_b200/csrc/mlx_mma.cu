@@ -420,7 +420,10 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
   static_assert((EP - 1) * MB <= 8, "room for the parts' sums");
   float* recv = pair + 8 * kTileRows;  // [splits-1][MB][128]: partial sums from the cluster's other CTAs (first CTA only)
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // (the shuffle tells the compiler that a warp's number is the same in all of its lanes: what follows from it is
+  // kept in uniform registers, from where the MMAs take their operands.  MLX4 28672x4096 17.6 us without, 16.7
+  // with, Q4_K 4096x14336 12.7 and 12.0)
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + S);
   const uint32_t aready0 = smem_u32(bars + 2 * S), afree0 = aready0 + 8 * NA;
   const uint32_t mdone0 = afree0 + 8 * NA, dfree0 = mdone0 + 8 * ND;  // mdone: a stage's accumulators are complete

@@ -132,7 +132,7 @@ __device__ __forceinline__ void moe_router_block(const uint4* __restrict__ w, co
   const int units = hidden / 32, iters = (units + 31) / 32;
   float4* xs = reinterpret_cast<float4*>(smem_raw);
   float2* xc = reinterpret_cast<float2*>(smem_raw + (size_t)iters * 256 * 16);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // (uniform, for the compiler)
   const int e0 = (eblock * kMoeWarps + warp) * 2, e1 = min(e0 + 1, num_experts - 1);
   const size_t sb_row = (size_t)groups * (SB_BF16 ? 4 : 8);
   // the weights do not depend on the kernel in front: first units in flight before the wait
@@ -535,7 +535,7 @@ __device__ __forceinline__ void moe_expert_pass(const MoeWork& wk, const int* __
                                                 int out_rows, int top_k, int ug_shift, int groups, float4* xs, float2* xc,
                                                 unsigned char* ring, int bx, int nbx) {
   // bx of nbx: this CTA's place among the CTAs that share the expert's rows
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // (uniform, for the compiler)
   const int units = in_dim / 32, iters = (units + 31) / 32;
   const size_t sb_row = (size_t)groups * (SB_BF16 ? 4 : 8);
   const int tasks = PHASE == 0 ? out_rows : (out_rows + 1) / 2;

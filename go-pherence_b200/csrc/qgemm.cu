@@ -606,7 +606,10 @@ qg_kernel(const __grid_constant__ QArgs a) {
   float* xinv = reinterpret_cast<float*>(tmem_holder + 1);  // [kMaxRows]
   volatile int* shared_item = reinterpret_cast<volatile int*>(xinv + kMaxRows);  // the cluster's item: group (or -1), block, split
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // (the shuffle tells the compiler that a warp's number is the same in all of its lanes: what follows from it is
+  // kept in uniform registers, from where the MMAs take their operands.  Q8_0 4096x4096 x19 16.5 us without, 15.1
+  // with, Q4_K 14336x4096 x64 30.8 and 29.4)
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   Walk wk(a);
   auto load_weights = [&](int s, int t, int c) {  // the W loader: chunk c of the item's tile t into slot s
     int tile = wk.group * TT + t;
