@@ -1,0 +1,99 @@
+"""GPU parity at the edges of the several-row products (f16 tensor-core tiles of 128 rows, 64 or 128 columns
+and 256 elements, cut along K over clusters) and of the one-pass row-major GEMV, against the oracle's dequantised
+weights in double precision, through the C ABI."""
+import numpy as np
+import pytest
+
+from gpu_util import F, out_with_canary, read_and_check_canary
+from oracle import binding as orc
+
+pytestmark = pytest.mark.gpu
+
+GGUF = {"q8_0": (orc.Q8_0, "q8_0_matrix"), "q4_k": (orc.Q4_K, "q4k_matrix"), "q5_k": (orc.Q5_K, "q5k_matrix"), "q6_k": (orc.Q6_K, "q6k_matrix")}
+
+
+def make(gpu, pkg, fmt, tiled, out_dim, in_dim):
+    """(device weight, run(out, x, rows), dequantised weight, bias or None)"""
+    layout = "fp8_layout" if fmt == "fp8" else "mlx_layout" if fmt.startswith("mlx") else "gguf_layout"
+    gpu.SetOption(layout, 2 if tiled else 1)
+    try:
+        if fmt.startswith("mlx"):
+            w, s, b = pkg.synth.mlx_weight(("rows", fmt), out_dim, in_dim)
+            if fmt == "mlx_wide":  # scales too far apart for f16: the groups are scaled after the tensor cores
+                s[::7] *= F(2.0 ** -24)
+                b[::7] *= F(2.0 ** -24)
+            h = gpu.UploadMLXWeight(w, s, b, in_dim, out_dim, 64, True)
+            return h, lambda o, x, n: gpu.GemmMLX(o, x, h, n), orc.mlx_dequant(w, s, b, out_dim, in_dim, 64), None
+        if fmt == "fp8":
+            w, s, b = pkg.synth.fp8_linear("rows", out_dim, in_dim, bias=True)
+            w[(out_dim - 1) * in_dim + 7] = 0x7F  # a NaN code: its output element only
+            h = gpu.UploadFP8E4M3Linear(w, s, b, out_dim, in_dim)
+            return h, lambda o, x, n: gpu.GemmFP8E4M3Buffer(o, x, n, h), orc.fp8_dequant(w, s, out_dim, in_dim), b
+        qtype, gen = GGUF[fmt]
+        raw = getattr(pkg.synth, gen)("rows", out_dim, in_dim)
+        h = gpu.UploadGGUFMatrix(qtype, raw, in_dim, out_dim)
+        return h, lambda o, x, n: h.ProjectBatchToBuffer(o, x, n), orc.gguf_dequant(raw, qtype, in_dim, out_dim), None
+    finally:
+        gpu.SetOption(layout, 0)
+
+
+# out_dim: one tile, a row more, five tiles (odd: the last group of two repeats one); in_dim: one chunk, ragged chunks
+# (MLX, Q8_0, FP8), enough chunks for K splits.  rows: either side of the column steps 16, 32, 64 and of the blocks.
+@pytest.mark.parametrize("tiled", [True, False])
+@pytest.mark.parametrize("fmt,shapes", [
+    ("mlx", ((128, 256), (129, 320), (640, 2112))), ("mlx_wide", ((129, 320), (640, 2112))), ("fp8", ((128, 256), (129, 272), (640, 2064))),
+    ("q8_0", ((128, 256), (129, 288), (640, 2080))), ("q4_k", ((128, 256), (129, 512), (640, 2816))),
+    ("q5_k", ((128, 256), (129, 512), (640, 2816))), ("q6_k", ((128, 256), (129, 512), (640, 2816)))])
+def test_several_rows(gpu, pkg, fmt, shapes, tiled):
+    """The tensor cores truncate a sum at every K16 step and piece (2^-23 of it, three pieces); an affine format's terms
+    reach four times the dequantised ones."""
+    for out_dim, in_dim in shapes:
+        h, run, W, bias = make(gpu, pkg, fmt, tiled, out_dim, in_dim)
+        W = np.asarray(W, dtype=np.float64).reshape(out_dim, in_dim)
+        for rows in (5, 9, 16, 17, 32, 33, 64, 65, 129):
+            x = pkg.synth.activations(("rows", rows, in_dim), rows * in_dim, bf16=rows in (16, 65)).reshape(rows, in_dim)
+            x[rows // 2] *= F(2.0 ** 40)  # every row has its own scale
+            if rows > 9:
+                x[3] = 0
+            xo, out = gpu.from_numpy(np.ascontiguousarray(x).reshape(-1)), out_with_canary(gpu, rows * out_dim)
+            run(out, xo, rows)
+            gpu.Sync()
+            got = read_and_check_canary(out, rows * out_dim).reshape(rows, out_dim).astype(np.float64)
+            want, size = x.astype(np.float64) @ W.T, np.abs(x.astype(np.float64)) @ np.abs(W).T
+            if bias is not None:
+                want, size = want + bias, size + np.abs(bias)
+            nan = np.isnan(want)
+            assert np.array_equal(np.isnan(got), nan), (rows, out_dim, in_dim)
+            err = np.abs(got - want)[~nan] - 4 * (3 * in_dim / 16 + 64) * 2.0 ** -23 * size[~nan]
+            assert np.max(err) <= 0, (rows, out_dim, in_dim, np.max(err))
+            xo.Free(); out.Free()
+        h.Free()
+    assert gpu.KernelStatus() == 0
+
+
+@pytest.mark.parametrize("in_dim", [32, 64, 1024, 1056, 3072, 4096, 5120, 8192])   # one to eight slices, ragged ones
+@pytest.mark.parametrize("out_dims", [(1,), (443,), (449,), (885, 3), (1185, 7, 1), (4097,)])  # rows per warp: one, two, four; several weights
+def test_row_gemv_has_the_looping_kernels_bits(gpu, pkg, in_dim, out_dims):
+    hs, want = [], []
+    x = gpu.from_numpy(pkg.synth.activations(("rowg", in_dim), in_dim, bf16=False))
+    outs = [out_with_canary(gpu, o) for o in out_dims]
+    gpu.SetOption("mlx_layout", 1)
+    try:
+        for i, o in enumerate(out_dims):
+            w, s, b = pkg.synth.mlx_weight(("rowg", i), o, in_dim, 32)
+            hs.append(gpu.UploadMLXWeight(w, s, b, in_dim, o, 32, True))
+            want.append(orc.mlx_gemv(pkg.synth.activations(("rowg", in_dim), in_dim, bf16=False), w, s, b, o, in_dim, 32, nthreads=8))
+        got = []
+        for rows in (0, 1):   # 1: the kernel that walks its rows
+            gpu.SetOption("mlx_rows", rows)
+            gpu.GemmMLXMulti(outs, x, hs, 1)
+            gpu.Sync()
+            got.append([read_and_check_canary(b, o).copy() for b, o in zip(outs, out_dims)])
+    finally:
+        gpu.SetOption("mlx_rows", 0)
+        gpu.SetOption("mlx_layout", 0)
+    for a, b, w in zip(got[0], got[1], want):
+        assert np.array_equal(a, b)
+        assert pkg.synth.rel_err(a, w) <= 2e-3
+    for t in hs + outs + [x]:
+        t.Free()
