@@ -79,14 +79,14 @@ struct Fp8Args {
   float* scratch;           // split-K partial sums [tile][split][MP][128]
   unsigned int* counters;   // per-tile arrival counters, zero between launches
   int out_dim, in_dim, batch;
-  int ntiles, nks, splits, items, stages;  // nks: stages along K (in_dim / KS); items = row-tile groups x splits
-  // 1: the K splits of a group are the CTAs of a thread-block cluster (every CTA has one item) and
+  int ntiles, nks, splits, items, stages;  // nks: stages along K (in_dim / 256); items = row tiles x splits
+  // 1: the K splits of a tile are the CTAs of a thread-block cluster (every CTA has one item) and
   // their partial sums go through the first CTA's shared memory instead of device scratch
   int cluster;
 };
 
 struct ItemWalk {
-  int w, tile, split, k, k1;  // tile: the item's group of TT consecutive row tiles
+  int w, tile, split, k, k1;
   __device__ __forceinline__ void open(const Fp8Args& a) {
     tile = w / a.splits;
     split = w - tile * a.splits;
@@ -268,22 +268,20 @@ __device__ __forceinline__ void umma_f8_ss(uint32_t d_tmem, uint64_t a_desc, uin
 }
 
 // ---- the product kernel -----------------------------------------------------------------------
-// KS: K bytes of a pipeline stage, 256 (a whole block) or 128 (half a block, for wide B tiles).  The
-// MMA warp spends some 70 cycles per instruction and 300 per stage on waits and commits, so the
-// longer stage is what lets a single SM keep up with its share of the HBM rate.
-template <int N, int P, int MP, int KS, int TT>
+// A pipeline stage is a whole block of 256 elements: the MMA warp spends some 70 cycles per instruction and
+// 300 per stage on waits and commits, so a stage's length is what lets a single SM keep up with its share of
+// the HBM rate.
+template <int N, int P, int MP>
 __global__ void __launch_bounds__(kThreads, 1)
 fp8_mma_kernel(const __grid_constant__ Fp8Args a) {
-  static_assert(KS == 128 || KS == 256, "a stage is a block or half a block");
-  static_assert(TT == 1 || (TT == 2 && 4 * N <= 512), "two accumulator buffers of TT x N columns");
-  constexpr int kABytes = kTileRows * KS;
+  constexpr int kABytes = kTileRows * kChunkK;
   static_assert(N % 16 == 0 && N >= 16 && N <= 256 && P * MP <= N, "B rows: P pieces of MP activation rows (the rows past P * MP are unused)");
   constexpr int HM = MP / 2;           // rows of one epilogue warp
   constexpr int G = HM >= 16 ? 16 : HM;  // rows per register group
   static_assert(MP >= 2 && MP % 2 == 0 && HM % G == 0, "rows split over two epilogue warps in groups");
-  constexpr int kBBytes = N * KS;
-  constexpr int kStage = TT * kABytes + kBBytes;  // [TT weight tiles][B tile]
-  constexpr int ND = 2;                // accumulator buffers of TT x N columns
+  constexpr int kBBytes = N * kChunkK;
+  constexpr int kStage = kABytes + kBBytes;  // [weight tile][B tile]
+  constexpr int ND = 2;                // accumulator buffers of N columns
   constexpr float kPieceScale[3] = {1.f, 1.f / 256.f, 1.f / 65536.f};  // pieces 2p and 2p+1 were written 2^(8p) up
   constexpr uint32_t kCols = 512;
   extern __shared__ unsigned char smem_dyn[];
@@ -292,7 +290,7 @@ fp8_mma_kernel(const __grid_constant__ Fp8Args a) {
   uint64_t* bars = reinterpret_cast<uint64_t*>(ring + (size_t)S * kStage);
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 2 * S + 2 * ND + 1);
   volatile int* last_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
-  float* recv = reinterpret_cast<float*>(tmem_holder + 4);  // cluster launches: [split - 1][tile of the group][row m][128]
+  float* recv = reinterpret_cast<float*>(tmem_holder + 4);  // cluster launches: [split - 1][row m][128]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * S, dfull0 = empty0 + 8 * S, dfree0 = dfull0 + 8 * ND;
   const uint32_t clbar = dfree0 + 8 * ND;  // cluster launches: the other CTAs' partial sums have arrived (one arrival per epilogue warp)
@@ -321,33 +319,23 @@ fp8_mma_kernel(const __grid_constant__ Fp8Args a) {
   const uint32_t tmem_base = *tmem_holder;
   bool ok = true;
   ItemWalk wk(a);
-  const int nchunks = a.in_dim / kChunkK;
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
     if (lane == 0) {
-      auto a_src = [&](const ItemWalk& q, int t) {
-        const size_t tile = (size_t)q.tile * TT + t;
-        return KS == 256 ? a.w + (tile * nchunks + q.k) * kBlockBytes : a.w + (tile * nchunks + (q.k >> 1)) * kBlockBytes + (q.k & 1) * kABytes;
-      };
-      // row tiles of the item that exist (the last group of an odd tile count has one)
-      auto tiles_of = [&](const ItemWalk& q) { return q.tile * TT + TT <= a.ntiles ? TT : a.ntiles - q.tile * TT; };
-      auto b_src = [&](const ItemWalk& q) {
-        return KS == 256 ? a.xb + (size_t)q.k * (N * kChunkK) : a.xb + (size_t)(q.k >> 1) * (N * kChunkK) + (q.k & 1) * kBBytes;
-      };
+      auto a_src = [&](const ItemWalk& q) { return a.w + ((size_t)q.tile * a.nks + q.k) * kABytes; };
+      auto b_src = [&](const ItemWalk& q) { return a.xb + (size_t)q.k * kBBytes; };
       int i = 0;
       {
         // the weights do not depend on the kernel in front: the first stages' copies go out at once
         ItemWalk q = wk;
         for (; i < S && i < 2 && q.live(a); ++i, q.next(a)) {
-          const int nt = tiles_of(q);
-          mbar_expect_tx(full0 + 8 * i, nt * kABytes + kBBytes);
-          for (int t = 0; t < nt; ++t)
-            bulk_load_1d(smem_u32(ring + (size_t)i * kStage) + t * kABytes, a_src(q, t), kABytes, full0 + 8 * i);
+          mbar_expect_tx(full0 + 8 * i, kStage);
+          bulk_load_1d(smem_u32(ring + (size_t)i * kStage), a_src(q), kABytes, full0 + 8 * i);
         }
         pdl_wait();
         for (int j = 0; j < i; ++j, wk.next(a))
-          bulk_load_1d(smem_u32(ring + (size_t)j * kStage) + TT * kABytes, b_src(wk), kBBytes, full0 + 8 * j);
+          bulk_load_1d(smem_u32(ring + (size_t)j * kStage) + kABytes, b_src(wk), kBBytes, full0 + 8 * j);
       }
       RingCursor rc;
       for (int j = 0; j < i; ++j) rc.next(S);
@@ -356,10 +344,9 @@ fp8_mma_kernel(const __grid_constant__ Fp8Args a) {
         if (i >= S) ok = mbar_wait(empty0 + 8 * slot, rc.ph ^ 1u, a.status, 501);
         if (!ok) break;
         const uint32_t dst = smem_u32(ring + (size_t)slot * kStage);
-        const int nt = tiles_of(wk);
-        mbar_expect_tx(full0 + 8 * slot, nt * kABytes + kBBytes);
-        for (int t = 0; t < nt; ++t) bulk_load_1d(dst + t * kABytes, a_src(wk, t), kABytes, full0 + 8 * slot);
-        bulk_load_1d(dst + TT * kABytes, b_src(wk), kBBytes, full0 + 8 * slot);
+        mbar_expect_tx(full0 + 8 * slot, kStage);
+        bulk_load_1d(dst, a_src(wk), kABytes, full0 + 8 * slot);
+        bulk_load_1d(dst + kABytes, b_src(wk), kBBytes, full0 + 8 * slot);
       }
     }
   } else if (warp == 1) {
@@ -383,19 +370,13 @@ fp8_mma_kernel(const __grid_constant__ Fp8Args a) {
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const bool last = wk.last_stage();
-        const int nt = wk.tile * TT + TT <= a.ntiles ? TT : a.ntiles - wk.tile * TT;
         if (elect_one()) {
-          const uint32_t abase = smem_u32(ring + (size_t)slot * kStage), bbase = abase + TT * kABytes;
+          const uint32_t abase = smem_u32(ring + (size_t)slot * kStage), bbase = abase + kABytes;
 #pragma unroll
-          for (int t = 0; t < TT; ++t) {
-            if (t < nt) {
-#pragma unroll
-              for (int st = 0; st < KS / 32; ++st) {
-                const uint64_t adesc = adesc_hi | (uint64_t)(((abase + t * kABytes + st * 4096) >> 4) & 0x3FFF);
-                const uint64_t bdesc = bdesc_hi | (uint64_t)(((bbase + st * (N * 32)) >> 4) & 0x3FFF);
-                umma_f8_ss(tmem_base + b * (TT * N) + t * N, adesc, bdesc, idesc, (first && st == 0) ? 0u : 1u);
-              }
-            }
+          for (int st = 0; st < kChunkK / 32; ++st) {
+            const uint64_t adesc = adesc_hi | (uint64_t)(((abase + st * 4096) >> 4) & 0x3FFF);
+            const uint64_t bdesc = bdesc_hi | (uint64_t)(((bbase + st * (N * 32)) >> 4) & 0x3FFF);
+            umma_f8_ss(tmem_base + b * N, adesc, bdesc, idesc, (first && st == 0) ? 0u : 1u);
           }
           umma_commit(empty0 + 8 * slot);
           if (last) umma_commit(dfull0 + 8 * b);
@@ -417,127 +398,97 @@ fp8_mma_kernel(const __grid_constant__ Fp8Args a) {
     const uint32_t lane_base = (uint32_t)(q4 * 32) << 16;
     pdl_wait();  // the row scales of x come from the preparation kernel in front
     for (int it = 0; wk.live(a) && ok; ++it) {
-      const int b = it % ND, group = wk.tile, split = wk.split;
-      const int nt = group * TT + TT <= a.ntiles ? TT : a.ntiles - group * TT;
+      const int b = it % ND, tile = wk.tile, split = wk.split, row = tile * kTileRows + r;
       // this role takes no part in the stages: on to the item's end
       wk.k = wk.k1 - 1;
       wk.next(a);
       // the rows' scales and biases are asked for before the wait, not behind it
-      float scs[TT], bis[TT];
-#pragma unroll
-      for (int t = 0; t < TT; ++t) {
-        const int row = (group * TT + t) * kTileRows + r;
-        scs[t] = (t < nt && row < a.out_dim) ? __ldg(a.scale + row) : 0.f;
-        bis[t] = (t < nt && a.bias && row < a.out_dim) ? __ldg(a.bias + row) : 0.f;
-      }
+      const float sc = row < a.out_dim ? __ldg(a.scale + row) : 0.f, bi = a.bias && row < a.out_dim ? __ldg(a.bias + row) : 0.f;
       float xi[HM];  // 2^-e of this warp's activation rows
 #pragma unroll
       for (int j = 0; j < HM; ++j) xi[j] = __ldg(a.xinv + hf * HM + j);
       ok = __all_sync(0xffffffffu, mbar_wait(dfull0 + 8 * b, (it / ND) & 1, a.status, 504));
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      float dot[TT][HM];
+      float dot[HM];
 #pragma unroll
-      for (int t = 0; t < TT; ++t) {
+      for (int g = 0; g < HM / G; ++g) {
+        float part[G];
 #pragma unroll
-        for (int g = 0; g < HM / G; ++g) {
-          float part[G];
+        for (int j = 0; j < G; ++j) part[j] = 0.f;
 #pragma unroll
-          for (int j = 0; j < G; ++j) part[j] = 0.f;
-          if (t < nt) {
+        for (int p = P - 1; p >= 0; --p) {  // the smallest pieces first
+          uint32_t v[G];
+          tmem_ld_cols<G>(tmem_base + lane_base + b * N + p * MP + hf * HM + g * G, v);
+          tmem_ld_cols_wait<G>(v);
 #pragma unroll
-            for (int p = P - 1; p >= 0; --p) {  // the smallest pieces first
-              uint32_t v[G];
-              tmem_ld_cols<G>(tmem_base + lane_base + b * (TT * N) + t * N + p * MP + hf * HM + g * G, v);
-              tmem_ld_cols_wait<G>(v);
-#pragma unroll
-              for (int j = 0; j < G; ++j) part[j] = fmaf(__uint_as_float(v[j]), kPieceScale[p >> 1], part[j]);
-            }
-          }
-#pragma unroll
-          for (int j = 0; j < G; ++j) dot[t][g * G + j] = part[j];
+          for (int j = 0; j < G; ++j) part[j] = fmaf(__uint_as_float(v[j]), kPieceScale[p >> 1], part[j]);
         }
+#pragma unroll
+        for (int j = 0; j < G; ++j) dot[g * G + j] = part[j];
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(dfree0 + 8 * b);
       if (a.cluster) {
-        // The K splits of this group are the CTAs of this cluster (rank == split), one item each.
+        // The K splits of this tile are the CTAs of this cluster (rank == split), one item each.
         // Ranks above 0 put their sums into rank 0's shared memory and arrive on its barrier (one
         // releasing arrival per warp); rank 0 waits, adds in split order — the order of the scratch
         // path, so the same bits — and stores.
         if (split != 0) {
 #pragma unroll
-          for (int t = 0; t < TT; ++t) {
-            if (t < nt) {
-#pragma unroll
-              for (int j = 0; j < HM; ++j)
-                cluster_store_f32(cluster_map(smem_u32(recv + ((size_t)((split - 1) * TT + t) * MP + hf * HM + j) * kTileRows + r), 0), dot[t][j]);
-            }
-          }
+          for (int j = 0; j < HM; ++j)
+            cluster_store_f32(cluster_map(smem_u32(recv + ((size_t)(split - 1) * MP + hf * HM + j) * kTileRows + r), 0), dot[j]);
           __syncwarp();
           if (lane == 0) cluster_arrive_release(cluster_map(clbar, 0));
         } else {
           ok = __all_sync(0xffffffffu, mbar_wait_cluster(clbar, 0, a.status, 505));
           if (ok) {
 #pragma unroll
-            for (int t = 0; t < TT; ++t) {
-              if (t < nt) {
-                const int row = (group * TT + t) * kTileRows + r;
-#pragma unroll
-                for (int j = 0; j < HM; ++j) {
-                  const int m = hf * HM + j;
-                  float sum = dot[t][j];
-                  for (int s2 = 1; s2 < a.splits; ++s2) sum += recv[((size_t)((s2 - 1) * TT + t) * MP + m) * kTileRows + r];
-                  if (m < a.batch && row < a.out_dim) a.out[(size_t)m * a.out_dim + row] = fmaf(sum * xi[j], scs[t], bis[t]);
-                }
-              }
+            for (int j = 0; j < HM; ++j) {
+              const int m = hf * HM + j;
+              float sum = dot[j];
+              for (int s2 = 1; s2 < a.splits; ++s2) sum += recv[((size_t)(s2 - 1) * MP + m) * kTileRows + r];
+              if (m < a.batch && row < a.out_dim) a.out[(size_t)m * a.out_dim + row] = fmaf(sum * xi[j], sc, bi);
             }
           }
         }
         continue;
       }
+      if (a.splits == 1) {
 #pragma unroll
-      for (int t = 0; t < TT; ++t) {
-        if (t >= nt) break;
-        const int tile = group * TT + t;
-        const int row = tile * kTileRows + r;
-        const float sc = scs[t], bi = bis[t];
-        if (a.splits == 1) {
+        for (int j = 0; j < HM; ++j) {
+          const int m = hf * HM + j;
+          if (m < a.batch && row < a.out_dim) a.out[(size_t)m * a.out_dim + row] = fmaf(dot[j] * xi[j], sc, bi);
+        }
+      } else {
+        // Partial sums of this K range go to scratch; the CTA that arrives last at the tile adds the
+        // partials in split order (so the result does not depend on arrival order) and stores.
+        float* part = a.scratch + ((size_t)tile * a.splits + split) * (MP * kTileRows);
+#pragma unroll
+        for (int j = 0; j < HM; ++j) part[(hf * HM + j) * kTileRows + r] = dot[j];
+        __threadfence();
+        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
+        if (et == 0) *last_flag = (atomicAdd(a.counters + tile, 1u) == (unsigned)a.splits - 1) ? 1 : 0;
+        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
+        if (*last_flag) {
+          __threadfence();
+          const float* base = a.scratch + (size_t)tile * a.splits * (MP * kTileRows);
+          float sum[HM];
+#pragma unroll
+          for (int j = 0; j < HM; ++j) sum[j] = 0.f;
+          for (int s2 = 0; s2 < a.splits; ++s2) {  // a split's HM loads are independent: all in flight together
+#pragma unroll
+            for (int j = 0; j < HM; ++j) sum[j] += __ldcg(base + (size_t)s2 * (MP * kTileRows) + (hf * HM + j) * kTileRows + r);
+          }
 #pragma unroll
           for (int j = 0; j < HM; ++j) {
             const int m = hf * HM + j;
-            if (m < a.batch && row < a.out_dim) a.out[(size_t)m * a.out_dim + row] = fmaf(dot[t][j] * xi[j], sc, bi);
+            if (m < a.batch && row < a.out_dim) a.out[(size_t)m * a.out_dim + row] = fmaf(sum[j] * xi[j], sc, bi);
           }
-        } else {
-          // Partial sums of this K range go to scratch; the CTA that arrives last at the tile adds the
-          // partials in split order (so the result does not depend on arrival order) and stores.
-          float* part = a.scratch + ((size_t)tile * a.splits + split) * (MP * kTileRows);
-#pragma unroll
-          for (int j = 0; j < HM; ++j) part[(hf * HM + j) * kTileRows + r] = dot[t][j];
-          __threadfence();
-          asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
-          if (et == 0) *last_flag = (atomicAdd(a.counters + tile, 1u) == (unsigned)a.splits - 1) ? 1 : 0;
-          asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
-          if (*last_flag) {
-            __threadfence();
-            const float* base = a.scratch + (size_t)tile * a.splits * (MP * kTileRows);
-            float sum[HM];
-#pragma unroll
-            for (int j = 0; j < HM; ++j) sum[j] = 0.f;
-            for (int s2 = 0; s2 < a.splits; ++s2) {  // a split's HM loads are independent: all in flight together
-#pragma unroll
-              for (int j = 0; j < HM; ++j) sum[j] += __ldcg(base + (size_t)s2 * (MP * kTileRows) + (hf * HM + j) * kTileRows + r);
-            }
-#pragma unroll
-            for (int j = 0; j < HM; ++j) {
-              const int m = hf * HM + j;
-              if (m < a.batch && row < a.out_dim) a.out[(size_t)m * a.out_dim + row] = fmaf(sum[j] * xi[j], sc, bi);
-            }
-            if (et == 0) a.counters[tile] = 0;
-          }
-          asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
+          if (et == 0) a.counters[tile] = 0;
         }
+        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
       }
     }
   }
@@ -621,10 +572,9 @@ static int choose_splits(int ntiles, int nchunks, int sms, int max_items, float 
   return best;
 }
 
-template <int N, int P, int MP, bool XBF16, int TT = 1>
+template <int N, int P, int MP, bool XBF16>
 int launch_pass(const goph_fp8_linear* w, float* out, const void* x, int nb, Fp8Bufs* bufs, cudaStream_t stream) {
-  constexpr int KS = (N <= 64 && TT == 1) ? 256 : 128;
-  constexpr int kStage = TT * kTileRows * KS + N * KS;
+  constexpr int kStage = (kTileRows + N) * kChunkK;
   DeviceState& st = device_state(w->device);
   Fp8Args a;
   memset(&a, 0, sizeof a);
@@ -641,18 +591,17 @@ int launch_pass(const goph_fp8_linear* w, float* out, const void* x, int nb, Fp8
   a.in_dim = w->in_dim;
   a.batch = nb;
   a.ntiles = (w->out_dim + kTileRows - 1) / kTileRows;
-  a.nks = w->in_dim / KS;
+  a.nks = w->in_dim / kChunkK;
   int max_items = (int)(kScratchFloats / ((size_t)MP * kTileRows));
   if (a.ntiles > (int)kMaxCounters) max_items = 0;
-  const int ngroups = (a.ntiles + TT - 1) / TT;  // items are groups of TT row tiles x K splits
   a.splits = options().mlx_splits > 0 ? (options().mlx_splits < a.nks ? options().mlx_splits : a.nks)
-                                      : choose_splits(ngroups, a.nks, st.sm_count, max_items / TT, 2.f + TT * MP / 16.f);
+                                      : choose_splits(a.ntiles, a.nks, st.sm_count, max_items, 2.f + MP / 16.f);
   while (a.splits > 1 && (long)a.ntiles * a.splits > max_items) --a.splits;
-  a.items = ngroups * a.splits;
+  a.items = a.ntiles * a.splits;
   const int grid = a.items < st.sm_count ? a.items : st.sm_count;
-  // K splits that all run at once, one item per CTA, whose partial sums fit the receive area: a cluster per group
+  // K splits that all run at once, one item per CTA, whose partial sums fit the receive area: a cluster per tile
   const bool want_cluster = options().mlx_cluster && a.splits > 1 && a.splits <= 8 && a.items == grid &&
-                            (size_t)(a.splits - 1) * TT * MP * kTileRows * 4 <= (size_t)kRecvBytes;
+                            (size_t)(a.splits - 1) * MP * kTileRows * 4 <= (size_t)kRecvBytes;
   const size_t extra = 2048 + (want_cluster ? kRecvBytes : 0);
   int stages = (int)((kSmemBudget - extra) / kStage);
   if (stages > kMaxStages) stages = kMaxStages;
@@ -672,7 +621,7 @@ int launch_pass(const goph_fp8_linear* w, float* out, const void* x, int nb, Fp8
   cfg.blockDim = dim3(256);
   note_launch();
   GOPH_CUDA(cudaLaunchKernelEx(&cfg, fp8_prep_x_kernel<P, XBF16>, x, bufs->xb, bufs->xinv, nb, w->in_dim, N, MP));
-  auto kern = fp8_mma_kernel<N, P, MP, KS, TT>;
+  auto kern = fp8_mma_kernel<N, P, MP>;
   GOPH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(kThreads);
