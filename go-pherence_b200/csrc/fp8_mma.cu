@@ -24,14 +24,14 @@
 //
 // Device layout of the weights (built at upload): blocks of 128 rows x 256 bytes ordered
 // [row tile][K chunk]; inside a block the K-major 8 x 16-byte core matrices the MMA reads:
-// [K step of 32 (8)][K half of 16 (2)][row group (16)][row (8)][16 B].  A block, or half a block (128
-// rows x 128 bytes of K) where the B tile is wide, is one pipeline stage and one contiguous bulk copy.
+// [K step of 32 (8)][K half of 16 (2)][row group (16)][row (8)][16 B].  A block is one
+// pipeline stage and one contiguous bulk copy.
 //
 // Pipeline of one CTA (10 warps, one persistent CTA per SM, walking (tile, K split) items):
-//   producer warp   per stage one bulk copy of the weights and one of the B tile into a ring guarded by full/empty mbarriers; the weight copies of the first two
-//                   stages are issued before the kernel in front (the activation preparation) ends.
+//   producer warp   per stage one bulk copy of the weights and one of the B tile into a ring guarded by
+//                   full/empty mbarriers; the weight copies of the first two stages are issued before the kernel in front (the activation preparation) ends.
 //   MMA warp        waits as a warp, one elected lane issues the stage's M128 x N x K32 instructions
-//                   (eight, or four) and commits to the stage's barrier and, after an item's last stage, to the
+//                   (eight) and commits to the stage's barrier and, after an item's last stage, to the
 //                   accumulator's.  Two accumulator buffers: the next item's MMAs run while the
 //                   epilogue reads the last one.
 //   8 epilogue warps  two per TMEM lane quarter, each with half of the activation rows: tcgen05.ld,

@@ -6,6 +6,12 @@
 // memory as f32 in the order [batch][it][slot][lane] (conflict-free LDS.128), with one
 // float2 of per-unit constants beside it when the format needs them (offset removal and
 // the affine term).  The next step's weights are in flight while the current step computes.
+// The first step's weights are asked for before the kernel in front has ended (programmatic dependent launch; the
+// kernel itself lets the next one start when it ends: asked for earlier, the next one's CTAs crowd onto a few SMs,
+// Q8_0 1536x4096 12.4 us a call instead of 5.8).  Small matrices come here, so a call's own cost bounds most of
+// them: two driver queries per launch, x read in 16-byte pieces 128 bytes apart.  Without these and with the early start
+// (B200, us a call): Q4_K 2048x2048 6.2 -> 4.2, Q6_K 2048x2048 x2 8.2 -> 4.6, Q8_0 1536x4096 8.3 -> 5.8, Q5_K 1024x2816
+// x8 16.4 -> 10.7, Q8_0 4096x1536 x3 10.3 -> 8.7.
 //
 // A format policy F provides:
 //   kSlots                 float4 of x per unit (unit elements / 4)
@@ -16,6 +22,10 @@
 //   dot(Row, xs, c, acc)   acc[m] += contribution of this unit, for m < M
 //   finish(a,row,v)        per-row epilogue (row scale, bias)
 #pragma once
+
+#include <string.h>
+
+#include <mutex>
 
 #include "goph_internal.cuh"
 
@@ -51,7 +61,7 @@ stream_gemv_kernel(const __grid_constant__ StreamArgs a) {
   float4* xs = reinterpret_cast<float4*>(smem_raw);
   float2* xc = reinterpret_cast<float2*>(smem_raw + (size_t)M * a.iters * S * 32 * 16);
 
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // (uniform, for the compiler)
   const int iters = a.iters;
   const int tasks = (a.rows + R - 1) / R;
   const int task_stride = gridDim.x * kGWarps;
@@ -71,22 +81,31 @@ stream_gemv_kernel(const __grid_constant__ StreamArgs a) {
   const bool has_work = task < tasks;
   if (has_work) load_tile(task, 0, cur);
 
-  // ---- stage x ----
+  // ---- stage x (which the kernel in front may write): coalesced reads, kV of them in flight ----
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   {
-    const int per_m = iters * S * 32, total = M * per_m;
-    for (int idx = threadIdx.x; idx < total; idx += kGThreads) {
-      int m = idx / per_m, rem = idx - m * per_m;
-      int i = rem / (S * 32), slot = (rem >> 5) % S, l = rem & 31;
-      int unit = i * 32 + l;
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (m < a.batch && unit < a.units) {
-        const float* p = a.x + (size_t)m * a.in_dim + (size_t)unit * (S * 4) + slot * 4;
-        if (a.x_aligned)
-          v = __ldg(reinterpret_cast<const float4*>(p));
-        else
-          v = make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+    constexpr int kV = 4;
+    const int per_m = iters * S * 32;  // float4s of a row, as float4 q of the row: slot q % S of unit q / S
+#pragma unroll 1
+    for (int m = 0; m < M; ++m) {
+#pragma unroll 1
+      for (int q0 = threadIdx.x; q0 < per_m; q0 += kV * kGThreads) {
+        float4 v[kV];
+#pragma unroll
+        for (int k = 0; k < kV; ++k) {
+          const int q = q0 + k * kGThreads, unit = q / S;
+          v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (m < a.batch && unit < a.units) {
+            const float* p = a.x + (size_t)m * a.in_dim + (size_t)q * 4;
+            v[k] = a.x_aligned ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < kV; ++k) {
+          const int q = q0 + k * kGThreads, unit = q / S;
+          if (q < per_m) xs[(size_t)m * per_m + ((unit >> 5) * S + q % S) * 32 + (unit & 31)] = v[k];
+        }
       }
-      xs[idx] = v;
     }
     __syncthreads();
     if (F::kHasConsts) {
@@ -171,6 +190,37 @@ static StreamKernel stream_pick(int R, int M) {
   }
 }
 
+// CTAs of kernel <F, R, M> an SM holds with `smem` bytes each.  The shared-memory limit of a kernel and the answer for
+// the last size asked for are kept: the two driver calls cost more than the launch.
+template <class F>
+static int stream_occupancy(StreamKernel k, int R, int M, size_t smem, int device) {
+  struct Known {
+    size_t limit, smem;
+    int per_sm;
+  };
+  static std::mutex mu;
+  static Known known[kMaxDevices][3][4] = {};
+  std::lock_guard<std::mutex> lock(mu);
+  Known& e = known[device][R >> 1][M == 1 ? 0 : M == 2 ? 1 : M == 4 ? 2 : 3];
+  if (e.limit < smem) {
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    e.limit = smem;
+  }
+  if (e.smem != smem) {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kGThreads, smem) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    e.smem = smem;
+    e.per_sm = n;
+  }
+  return e.per_sm;
+}
+
 // Runs x [batch,in] through the streaming kernel in batch tiles that fit shared memory.
 // Returns GOPH_E_UNSUPPORTED when even one activation row does not fit.
 template <class F>
@@ -198,16 +248,24 @@ static int stream_launch(StreamArgs a, int device, int batch, cudaStream_t strea
     a.x_aligned = ((uintptr_t)a.x % 16) == 0;
     StreamKernel k = stream_pick<F>(R, M);
     size_t smem = stream_smem_bytes<F>(M, a.iters);
-    GOPH_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int per_sm = 0;
-    GOPH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kGThreads, smem));
+    const int per_sm = stream_occupancy<F>(k, R, M, smem, device);
     if (per_sm < 1) return fail(GOPH_E_UNSUPPORTED, "streaming kernel does not fit (smem %zu)", smem);
     int tasks = (a.rows + R - 1) / R;
     int grid = (tasks + kGWarps - 1) / kGWarps;
     if (grid > st.sm_count * per_sm) grid = st.sm_count * per_sm;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = options().pdl ? 1 : 0;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof cfg);
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kGThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
     note_launch();
-    k<<<grid, kGThreads, smem, stream>>>(a);
-    GOPH_CUDA(cudaGetLastError());
+    GOPH_CUDA(cudaLaunchKernelEx(&cfg, k, a));
   }
   return GOPH_OK;
 }
