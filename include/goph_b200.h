@@ -182,9 +182,9 @@ int goph_mlx_dequant(const goph_mlx_weight* w, float* out_dev, uint64_t out_len,
 int goph_mlx_gemv(float* out_dev, uint64_t out_len, const float* x_dev, uint64_t x_len,
                   const goph_mlx_weight* w, void* stream);
 /* nvidia.GemmMLX (runtime/mlx.go:395-431): x [batch,in] → out [batch,out].  Tiled weights: up to
- * 8 rows run on the integer tensor-core kernel; more rows on the bf16 tensor-core kernel, which
- * streams the weights once per 16 rows (every f32 activation is split into three bf16 pieces
- * that add up to it exactly, so the result is as exact as the 8-row path's). */
+ * 4 rows run on the integer tensor-core kernel; more rows on the f16 tensor-core kernel, which
+ * streams the weights once per 64 rows (every f32 activation is split into up to three f16 pieces
+ * that add up to it, so the result is as exact as the few-row path's). */
 int goph_mlx_gemm(float* out_dev, uint64_t out_len, const float* x_dev, uint64_t x_len,
                   const goph_mlx_weight* w, int batch, void* stream);
 /* nvidia.GemmMLX (runtime/mlx.go:395-431) for activations held as bf16 (prefill chunks and verifier
@@ -351,7 +351,7 @@ int goph_fp8_dequant(const goph_fp8_linear* w, float* out_dev, uint64_t out_len,
 int goph_fp8_gemm(float* out_dev, uint64_t out_len, const float* x_dev, uint64_t x_len, int batch,
                   const goph_fp8_linear* w, void* stream);
 /* nvidia.GemmFP8E4M3Buffer (runtime/fp8.go:271-320) for activations held as bf16: x_bf16_dev is
- * [batch,in] bf16 bit patterns, 16-byte aligned; the weights are streamed once per 64 rows.
+ * [batch,in] bf16 bit patterns, 16-byte aligned; the weights are streamed once per 64 or 128 rows.
  * Linears in the tensor-core layout only (GOPH_E_UNSUPPORTED otherwise). */
 int goph_fp8_gemm_bf16(float* out_dev, uint64_t out_len, const uint16_t* x_bf16_dev, uint64_t x_len, int batch,
                        const goph_fp8_linear* w, void* stream);
