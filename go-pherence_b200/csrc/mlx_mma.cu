@@ -437,7 +437,7 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
       mbar_init(empty0 + 8 * s, (F::kConv ? kConvWarps / 2 : 0) + kEpiWarps + 1);
     }
     for (int b = 0; b < NA; ++b) {
-      mbar_init(aready0 + 8 * b, kConvWarps / 2);
+      mbar_init(aready0 + 8 * b, kConvWarps);
       mbar_init(afree0 + 8 * b, 1);
     }
     for (int b = 0; b < ND; ++b) {
@@ -452,7 +452,7 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  pdl_launch_dependents();
+  if (!G) pdl_launch_dependents();  // (grouped: the small kernels behind it gain nothing; the 8-token MoE layer 62.3 us with it, 61.3 without)
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -590,9 +590,9 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
     // Two groups of four warps convert alternate stages (thread = row r of the tile), so two stages
     // are in conversion at any time: a stage's conversion is a fixed latency of well over a
     // thousand cycles whatever its size, and what counts is how many run side by side.  Both groups
-    // follow every stage's barriers in order, also those of the stages they do not convert, so no
-    // barrier phase is ever skipped (a parity wait can only tell the current phase from the one
-    // before it).
+    // follow every stage's barriers in order, also those of the stages they do not convert, and both
+    // arrive for every stage, so no barrier phase is ever skipped (a parity wait can only tell the
+    // current phase from the one before it).
     const int q4 = warp & 3, grp = warp >> 2;
     const int r = q4 * 32 + lane;
     const uint32_t lane_base = (uint32_t)(q4 * 32) << 16;
@@ -602,7 +602,14 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
       ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * slot, rc.ph, a.status, 4));
       if (ok && i >= NA) ok = __all_sync(0xffffffffu, mbar_wait(afree0 + 8 * ba, ((i - NA) / NA) & 1, a.status, 3));
       if (!ok) break;
-      if ((i & 1) != grp) continue;
+      if ((i & 1) != grp) {
+        // The other group's stage: this one has seen its barriers and says so.  Without this the MMA could be
+        // done with the stage before a warp held up here has looked (an instruction fetch of the first launch is
+        // enough), which would then wait for a round that is two further on.
+        __syncwarp();
+        if (lane == 0) mbar_arrive(aready0 + 8 * ba);
+        continue;
+      }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       TP(if (tr && q4 == 0 && lane == 0 && i < 64) g_mma_trace[3][i] = clock64();)
       const unsigned char* st = ring + (size_t)slot * kStage;
