@@ -380,7 +380,6 @@ attn_step_kernel(const __grid_constant__ AttnArgs a) {
   __shared__ float s_m[W], s_l[W];
   __shared__ __align__(16) float all[kStepCtas][D];
   __shared__ float2 all_ml[kStepCtas];
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // (the first CTA's shared memory exists)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rank = blockIdx.x, head = blockIdx.y, per = a.heads / a.kv_heads, kvh = head / per;
@@ -393,6 +392,7 @@ attn_step_kernel(const __grid_constant__ AttnArgs a) {
     kn[e] = norm ? __ldg(a.k_norm + lane + 32 * e) : 1.f;
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // (earlier, a third kernel's CTAs would come in)
   const int pos = *a.pos_dev;
   float q[EPL], nk[EPL], nv[EPL], k[T][EPL], v[T][EPL];
 #pragma unroll

@@ -135,8 +135,8 @@ fp8_prep_x_kernel(const void* __restrict__ xv, unsigned char* __restrict__ xb, f
                   int N, int MP) {
   __shared__ float red[8];
   const int m = blockIdx.x, tid = threadIdx.x;
-  pdl_launch_dependents();
   pdl_wait();  // x may be the output of the kernel in front; the tiles may still be read by it
+  pdl_launch_dependents();  // (in front of the wait: 8192x8192 21.3 us a call, here 20.6)
   const bool real = m < batch;
   float mx = 0.f;
   if (real) {
