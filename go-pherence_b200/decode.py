@@ -170,7 +170,8 @@ class MLXDecoder:
 
     def prefill(self, prompt, stream=None):
         """The keys and values of every prompt token but the last into the caches, and the decoder set up
-        for a step with the last one.  The last layer ends with its keys and values."""
+        for a step with the last one, which has to run on the same stream (or behind it).  The last layer ends
+        with its keys and values."""
         rt, c = self.rt, self.cfg
         n = len(prompt) - 1
         self.reset(prompt, n)
@@ -216,6 +217,7 @@ class MLXDecoder:
         ints[2:2 + len(prompt)] = prompt                       # history
         ints[2 + c.max_seq:2 + c.max_seq + len(prompt)] = prompt   # forced
         self.ints.UploadBytes(ints.view(np.uint8))
+        self.rt.Sync()   # (a copy from pageable memory may still be under way when the call returns; a side stream would not wait for it)
 
     def capture(self):
         import torch
@@ -227,6 +229,12 @@ class MLXDecoder:
         with torch.cuda.graph(self.graph, stream=s):
             self.step(torch.cuda.current_stream())
         return self.graph
+
+    @staticmethod
+    def _graph_stream():
+        """The stream that a graph's replay goes to."""
+        import torch
+        return torch.cuda.current_stream()
 
     def generate(self, prompt, max_new, use_graph=True, logits_at=None, logits_all=None):
         """Returns prompt + max_new greedy tokens.  logits_at: optional list that receives the logits
@@ -242,7 +250,9 @@ class MLXDecoder:
         # from four prompt tokens a chunk (some 350 launches) takes less time than the steps it saves (some 150 each)
         first = len(prompt) - 1 if len(prompt) > 3 and logits_all is None else 0
         if first:
-            self.prefill(prompt)
+            # on the steps' stream: torch's side streams are not ordered with the default stream, and the first
+            # step reads the caches that the prompt's chunks write
+            self.prefill(prompt, self._graph_stream() if use_graph else None)
         else:
             self.reset(prompt)
         for i in range(first, total - 1):

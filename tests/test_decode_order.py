@@ -1,0 +1,79 @@
+"""MLXDecoder.generate enqueues the prompt's chunks and the steps on one stream, checked on a stand-in runtime that
+notes the stream of every call (no GPU), and through the C ABI inside a side stream."""
+import types
+
+import numpy as np
+import pytest
+
+from oracle import decode as od
+
+F = np.float32
+
+
+class _Buffer:
+    Ptr = 4096
+
+    def Free(self):
+        pass
+
+    def UploadBytes(self, data):
+        pass
+
+    def Download(self, n=0, dtype=F):
+        return np.zeros(n, dtype=dtype)
+
+
+class _Runtime:
+    """Buffers and weights are stand-ins; any other call is a launch, whose stream (the last argument) is noted."""
+
+    def __init__(self):
+        self.launches = []
+
+    def __getattr__(self, name):
+        if name in ("Malloc", "MallocBytes", "from_numpy", "wrap"):
+            return lambda *a, **k: _Buffer()
+        if name == "UploadMLXWeight":
+            return lambda w, s, b, in_dim, out_dim, *a: types.SimpleNamespace(InDim=in_dim, OutDim=out_dim)
+        if name == "Sync":
+            return lambda: None
+        return lambda *a, **k: self.launches.append((name, k.get("stream", a[-1])))
+
+
+def _config(**more):
+    return types.SimpleNamespace(**{**dict(hidden=64, layers=2, heads=2, kv_heads=1, head_dim=64, inter=64, vocab=96, eps=1e-6, theta=1e6,
+                                           qk_norm=True, max_seq=300), **more})
+
+
+@pytest.mark.parametrize("use_graph", [True, False])
+@pytest.mark.parametrize("prompt", [1, 3, 4, 200])   # by steps, by steps, one chunk, two chunks
+def test_prompt_and_steps_share_a_stream(pkg, monkeypatch, prompt, use_graph):
+    rt, c, side = _Runtime(), _config(), object()
+    part = (np.zeros((1, 1)),) * 3
+    layers = [dict({n: part for n in ("q", "k", "v", "o", "gate", "up", "down")}, input_norm=[0.0], post_norm=[0.0], q_norm=[0.0], k_norm=[0.0])] * c.layers
+    dec = pkg.decode.MLXDecoder(rt, c, layers, part, [0.0], np.zeros(2))
+    monkeypatch.setattr("torch.cuda.current_stream", lambda *a: side)
+    dec.graph = types.SimpleNamespace(replay=lambda: rt.launches.append(("replay", side)))   # torch replays on the current stream
+    dec.generate(list(range(prompt)), 2, use_graph=use_graph)
+    assert len(rt.launches) >= 2
+    assert {s for _, s in rt.launches} == {side if use_graph else None}
+
+
+@pytest.mark.gpu
+def test_generate_inside_a_side_stream(gpu, pkg):
+    """The same tokens and logits as on the default stream, again and again on streams of their own."""
+    import torch
+    c = _config(hidden=512, layers=8, heads=8, kv_heads=4, inter=1024, vocab=4096, max_seq=192)
+    g = pkg.synth.rng("side")
+    shapes = {"q": (512, 512), "k": (256, 512), "v": (256, 512), "o": (512, 512), "gate": (1024, 512), "up": (1024, 512), "down": (512, 1024)}
+    layers = [dict({n: pkg.synth.mlx_weight(("side", l, n), o, i) for n, (o, i) in shapes.items()}, input_norm=np.ones(512, F),
+                   post_norm=np.ones(512, F), q_norm=np.ones(64, F), k_norm=np.ones(64, F)) for l in range(c.layers)]
+    dec = pkg.decode.MLXDecoder(gpu, c, layers, pkg.synth.mlx_weight("side lm", 4096, 512), np.ones(512, F), od.rope_table(192, 64, 1e6))
+    prompt = g.integers(0, 4096, 130).tolist()
+    want_logits = []
+    want = dec.generate(prompt, 6, logits_at=want_logits)
+    for _ in range(5):
+        logits = []
+        with torch.cuda.stream(torch.cuda.Stream()):
+            assert dec.generate(prompt, 6, logits_at=logits) == want
+        assert np.array_equal(np.stack(logits), np.stack(want_logits))
+    assert gpu.KernelStatus() == 0
