@@ -101,9 +101,9 @@ static bool valid_fp8(const goph_fp8_linear* w) {
 }
 
 // The several-row tensor-core product (qgemm.cu) reads both layouts (rows of whole 16-byte units).
-static bool qgemm_takes(const goph_fp8_linear* w, const void* x, bool x_bf16, int batch) {
+static bool qgemm_takes(const goph_fp8_linear* w, const void* x, bool x_bf16, int batch, cudaStream_t stream) {
   return w->in_dim % 16 == 0 && w->in_dim <= 65536 && (uintptr_t)x % 16 == 0 &&
-         qgemm_wants(Q_FP8, w->tiled != nullptr, x_bf16, w->out_dim, w->in_dim, batch);
+         qgemm_wants(Q_FP8, w->tiled != nullptr, x_bf16, w->out_dim, w->in_dim, batch) && (w->tiled || qgemm_scratch(w->device, stream));
 }
 
 static int fp8_qgemm(const goph_fp8_linear* w, float* out, const void* x, bool x_bf16, int batch, cudaStream_t stream) {
@@ -190,6 +190,7 @@ GOPH_API int goph_fp8_upload(int device, const uint8_t* weight, uint64_t weight_
       h->bytes = (uint64_t)((out_dim + 127) / 128) * 128 * in_dim + (uint64_t)out_dim * 4 * (bias ? 2 : 1);
     }
   }
+  qgemm_weights(device, 1);
   *out = h;
   return bail(GOPH_OK);
 }
@@ -203,6 +204,7 @@ GOPH_API int goph_fp8_free(goph_fp8_linear* w) {
   cudaFree(w->tiled);
   cudaFree(w->scale);
   cudaFree(w->bias);
+  qgemm_weights(w->device, -1);
   w->magic = 0;
   delete w;
   return GOPH_OK;
@@ -242,7 +244,7 @@ GOPH_API int goph_fp8_gemm(float* out_dev, uint64_t out_len, const float* x_dev,
   cudaStream_t s = (cudaStream_t)stream;
   // Several rows: qgemm.cu.  Few rows: in the tensor-core layout the kernel that feeds the e4m3 bytes to the
   // MMA as they lie (fp8_mma.cu), in the row-major layout the CUDA-core kernels below.
-  if (qgemm_takes(w, x_dev, false, batch)) return fp8_qgemm(w, out_dev, x_dev, false, batch, s);
+  if (qgemm_takes(w, x_dev, false, batch, s)) return fp8_qgemm(w, out_dev, x_dev, false, batch, s);
   if (w->tiled) return tc_gemm_fp8(w, out_dev, x_dev, false, batch, s);
   if (!w->tiled && w->in_dim % 16 != 0) {
     note_launch();
@@ -282,7 +284,7 @@ GOPH_API int goph_fp8_gemm_bf16(float* out_dev, uint64_t out_len, const uint16_t
                 "goph_fp8_gemm_bf16 needs a linear in the tensor-core layout (in_dim a multiple of 256, no NaN codes, "
                 "uploaded with fp8_layout 0 or 2)");
   if (int rc = use_device(w->device)) return rc;
-  if (qgemm_takes(w, x_bf16_dev, true, batch)) return fp8_qgemm(w, out_dev, x_bf16_dev, true, batch, (cudaStream_t)stream);
+  if (qgemm_takes(w, x_bf16_dev, true, batch, (cudaStream_t)stream)) return fp8_qgemm(w, out_dev, x_bf16_dev, true, batch, (cudaStream_t)stream);
   return tc_gemm_fp8(w, out_dev, x_bf16_dev, true, batch, (cudaStream_t)stream);
 }
 

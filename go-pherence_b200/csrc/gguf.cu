@@ -359,8 +359,9 @@ static int q_format(int qtype) {
 }
 
 // The several-row tensor-core product (qgemm.cu) reads both layouts.
-static bool qgemm_takes(const goph_gguf_matrix* m, const void* x, int batch) {
-  return m->in_dim <= 65536 && (uintptr_t)x % 16 == 0 && qgemm_wants(q_format(m->qtype), m->tiled != nullptr, false, m->out_dim, m->in_dim, batch);
+static bool qgemm_takes(const goph_gguf_matrix* m, const void* x, int batch, cudaStream_t stream) {
+  return m->in_dim <= 65536 && (uintptr_t)x % 16 == 0 && qgemm_wants(q_format(m->qtype), m->tiled != nullptr, false, m->out_dim, m->in_dim, batch) &&
+         (m->tiled || qgemm_scratch(m->device, stream));
 }
 
 static int gguf_qgemm(const goph_gguf_matrix* m, float* out, const float* x, int batch, cudaStream_t stream) {
@@ -464,6 +465,7 @@ GOPH_API int goph_gguf_upload(int device, int qtype, const uint8_t* raw, uint64_
     h->data = nullptr;
     h->d16 = nullptr;
   }
+  qgemm_weights(device, 1);
   *out = h;
   return bail(GOPH_OK);
 }
@@ -476,6 +478,7 @@ GOPH_API int goph_gguf_free(goph_gguf_matrix* m) {
   cudaFree(m->data);
   cudaFree(m->d16);
   cudaFree(m->tiled);
+  qgemm_weights(m->device, -1);
   m->magic = 0;
   delete m;
   return GOPH_OK;
@@ -526,7 +529,7 @@ GOPH_API int goph_gguf_project(float* out_dev, uint64_t out_len, const float* x_
     return fail(GOPH_E_INVALID, "buffers x=%llu/%llu out=%llu/%llu", (unsigned long long)x_len,
                 (unsigned long long)need_x, (unsigned long long)out_len, (unsigned long long)need_o);
   if (int rc = use_device(m->device)) return rc;
-  if (qgemm_takes(m, x_dev, batch)) return gguf_qgemm(m, out_dev, x_dev, batch, (cudaStream_t)stream);
+  if (qgemm_takes(m, x_dev, batch, (cudaStream_t)stream)) return gguf_qgemm(m, out_dev, x_dev, batch, (cudaStream_t)stream);
   if (m->tiled) return gguf_mma_launch(m, out_dev, x_dev, batch, options().mlx_digits, (cudaStream_t)stream);
   StreamArgs a;
   memset(&a, 0, sizeof a);
@@ -564,7 +567,7 @@ GOPH_API int goph_gguf_project_pair(float* out_a_dev, uint64_t out_a_len, float*
   if (!valid_gguf(a) || !valid_gguf(b)) return fail(GOPH_E_INVALID, "invalid GGUF matrix handle");
   if (a->device != b->device || a->in_dim != b->in_dim)
     return fail(GOPH_E_INVALID, "pair projection: matrices differ in device or inDim (%d vs %d)", a->in_dim, b->in_dim);
-  if (a->tiled && b->tiled && a->qtype == b->qtype && !qgemm_takes(a, x_dev, batch)) {
+  if (a->tiled && b->tiled && a->qtype == b->qtype && !qgemm_takes(a, x_dev, batch, (cudaStream_t)stream)) {
     // both on the tensor-core path: validated like a single projection, x prepared once
     if (batch <= 0) return fail(GOPH_E_INVALID, "batch=%d", batch);
     uint64_t need_x, need_a, need_b;

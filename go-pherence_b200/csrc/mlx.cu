@@ -1149,9 +1149,9 @@ static int launch_generic(const goph_mlx_weight* w, float* out, const float* x, 
 }
 
 // The several-row tensor-core product (qgemm.cu) reads both layouts of 64-element groups with bf16 tables.
-static bool qgemm_takes(const goph_mlx_weight* w, const void* x, int batch) {
+static bool qgemm_takes(const goph_mlx_weight* w, const void* x, int batch, cudaStream_t stream) {
   return w->group_size == 64 && w->sb_bf16 && w->in_dim <= 65536 && (uintptr_t)x % 16 == 0 &&
-         qgemm_wants(Q_MLX4, w->tiled != nullptr, false, w->out_dim, w->in_dim, batch);
+         qgemm_wants(Q_MLX4, w->tiled != nullptr, false, w->out_dim, w->in_dim, batch) && (w->tiled || qgemm_scratch(w->device, stream));
 }
 
 static int mlx_qgemm(const goph_mlx_weight* w, float* out, const void* x, bool x_bf16, int batch, cudaStream_t stream) {
@@ -1166,7 +1166,7 @@ static int mlx_products(int n, float* const* outs, const goph_mlx_weight* const*
   bool any_tiled = false, any_rows = false;
   for (int i = 0; i < n; ++i) {
     any_tiled = any_tiled || ws[i]->tiled;
-    any_rows = any_rows || qgemm_takes(ws[i], x, batch);
+    any_rows = any_rows || qgemm_takes(ws[i], x, batch, stream);
   }
   if (any_tiled || any_rows) {
     // tiled weights run on the tensor cores; row-major ones in the same call take their own path
@@ -1175,7 +1175,7 @@ static int mlx_products(int n, float* const* outs, const goph_mlx_weight* const*
       const goph_mlx_weight* one = ws[i];
       float* o = outs[i];
       int rc;
-      if (qgemm_takes(one, x, batch)) {
+      if (qgemm_takes(one, x, batch, stream)) {
         rc = mlx_qgemm(one, o, x, false, batch, stream);
       } else if (one->tiled) {
         rc = mlx_mma_launch(one, o, x, batch, options().mlx_digits, stream, prepared);
@@ -1492,6 +1492,7 @@ static int mlx_upload_common(int device, const uint32_t* weight, const float* sc
     h->qweight = nullptr;
     h->sb = nullptr;
   }
+  qgemm_weights(device, 1);
   *out = h;
   return cleanup(GOPH_OK);
 }
@@ -1547,6 +1548,7 @@ GOPH_API int goph_mlx_free(goph_mlx_weight* w) {
   cudaFree(w->qweight);
   cudaFree(w->sb);
   cudaFree(w->tiled);
+  qgemm_weights(w->device, -1);
   w->magic = 0;
   delete w;
   return GOPH_OK;

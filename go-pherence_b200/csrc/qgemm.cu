@@ -1161,14 +1161,35 @@ constexpr size_t kXauxBytes = (size_t)(kMaxRows / 64) * (kMaxIn / kChunkK) * 64 
 constexpr size_t kFlagBytes = (size_t)(kMaxRows / 64) * (kMaxIn / kChunkK) * 64;
 constexpr size_t kSmemBudget2 = 227 * 1024;         // all that a CTA may have
 
+// The preparation and the product of a call meet in scratch; `enqueue` is held from the one launch to the other, so
+// that calls of several threads on one stream do not come between them.
 struct QBufs {
   unsigned char* xb = nullptr;
   unsigned char* xaux = nullptr;
   float* xinv = nullptr;
   unsigned char* flags = nullptr;
   int* status = nullptr;
+  size_t xb_bytes = 0;
+  std::mutex enqueue;
 };
 
+bool carve(QBufs* b, size_t xb_bytes) {
+  const size_t total = xb_bytes + kXauxBytes + kMaxRows * 4 + kFlagBytes + 256;
+  unsigned char* p = nullptr;
+  if (cudaMalloc(&p, total) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  b->xb = p;
+  b->xb_bytes = xb_bytes;
+  b->xaux = b->xb + xb_bytes;
+  b->xinv = reinterpret_cast<float*>(b->xaux + kXauxBytes);
+  b->flags = reinterpret_cast<unsigned char*>(b->xinv + kMaxRows);
+  b->status = reinterpret_cast<int*>(b->flags + kFlagBytes);
+  return true;
+}
+
+// The tiled layouts' area, one per device (goph_b200.h asks callers for an order between such calls).
 // Allocated on a device's first product of this kind; published only when complete.
 QBufs* q_bufs(int device, bool allocate = true) {
   static QBufs bufs[kMaxDevices];
@@ -1177,24 +1198,67 @@ QBufs* q_bufs(int device, bool allocate = true) {
   if (device < 0 || device >= kMaxDevices) return nullptr;
   std::lock_guard<std::mutex> lock(mu);
   if (ready[device]) return &bufs[device];
-  if (!allocate) return nullptr;
-  QBufs b;
-  bool ok = cudaMalloc(&b.xb, kXbBytes) == cudaSuccess && cudaMalloc(&b.xaux, kXauxBytes) == cudaSuccess &&
-            cudaMalloc(&b.xinv, kMaxRows * 4) == cudaSuccess && cudaMalloc(&b.flags, kFlagBytes) == cudaSuccess &&
-            cudaMalloc(&b.status, 256) == cudaSuccess;
-  ok = ok && cudaMemset(b.status, 0, 256) == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess;
-  if (!ok) {
+  if (!allocate || !carve(&bufs[device], kXbBytes)) return nullptr;
+  if (cudaMemset(bufs[device].status, 0, 256) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
     cudaGetLastError();
-    cudaFree(b.xb);
-    cudaFree(b.xaux);
-    cudaFree(b.xinv);
-    cudaFree(b.flags);
-    cudaFree(b.status);
+    cudaFree(bufs[device].xb);
     return nullptr;
   }
-  bufs[device] = b;
   ready[device] = true;
   return &bufs[device];
+}
+
+// The other layouts' areas.  The kernels for few rows that also serve these layouts need no scratch, so callers may
+// use them on streams without an order between them, from several threads and under capture: every stream has
+// an area of its own (found by the stream's id, which no later stream gets again).  Where none is to be had -- under
+// capture, since a graph may be replayed beside anything; on the streams after the first kStreamAreas of a device;
+// without memory -- the call goes to the kernels for few rows.  Areas go back with the device's last weight.
+constexpr int kStreamAreas = 8;
+constexpr size_t kStreamXbBytes = (size_t)64 * kMaxIn * 6;  // one block of rows of the widest matrix (24 MB)
+
+struct StreamAreas {
+  std::mutex mu;
+  int weights = 0;  // handles of the device
+  int n = 0;
+  int lost_status = 0;  // of areas given back
+  unsigned long long id[kStreamAreas];
+  QBufs bufs[kStreamAreas];
+};
+
+StreamAreas& stream_areas(int device) {
+  static StreamAreas areas[kMaxDevices];
+  return areas[device];
+}
+
+QBufs* q_stream_bufs(int device, cudaStream_t stream) {
+  cudaStreamCaptureStatus capture;
+  unsigned long long id;
+  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone || cudaStreamGetId(stream, &id) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  StreamAreas& s = stream_areas(device);
+  std::lock_guard<std::mutex> lock(s.mu);
+  for (int i = 0; i < s.n; ++i)
+    if (s.id[i] == id) return &s.bufs[i];
+  if (s.n == kStreamAreas) return nullptr;
+  // (another thread may be capturing a stream of its own, which an allocation must not disturb)
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  QBufs& b = s.bufs[s.n];
+  bool ok = carve(&b, kStreamXbBytes);
+  if (ok && cudaMemsetAsync(b.status, 0, 256, stream) != cudaSuccess) {
+    cudaGetLastError();
+    cudaFree(b.xb);
+    ok = false;
+  }
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (!ok) return nullptr;
+  s.id[s.n++] = id;
+  return &b;
 }
 
 // Clusters of `size` CTAs that the device holds at once (every CTA takes a whole SM, so this is a
@@ -1315,8 +1379,9 @@ int launch_product(QArgs& a, const Plan& p, int n, int device, cudaStream_t stre
 template <int F, bool TILED, bool XBF16>
 int run_rows(const QWeight& w, float* out, const void* x, int batch, cudaStream_t stream) {
   typedef QF<F, TILED> T;
-  QBufs* bufs = q_bufs(w.device);
+  QBufs* bufs = TILED ? q_bufs(w.device) : q_stream_bufs(w.device, stream);
   if (!bufs) return fail(GOPH_E_NOMEM, "cannot allocate the several-row products' device scratch");
+  std::lock_guard<std::mutex> enqueue(bufs->enqueue);
   constexpr int pmax = XBF16 ? 1 : 3;
   const int nchunks = (w.in_dim + kChunkK - 1) / kChunkK;
   const size_t xstride = (size_t)w.in_dim * (XBF16 ? 2 : 4);
@@ -1330,7 +1395,7 @@ int run_rows(const QWeight& w, float* out, const void* x, int batch, cudaStream_
         NB = 64;
     }
     const size_t block_bytes = (size_t)NB * nchunks * kChunkK * 2 * pmax;
-    int cap = (int)(kXbBytes / block_bytes) * NB;
+    int cap = (int)(bufs->xb_bytes / block_bytes) * NB;
     if (cap > kMaxRows) cap = kMaxRows;
     const int rows = batch - b0 < cap ? batch - b0 : cap;
     QArgs a;
@@ -1439,17 +1504,44 @@ int qgemm(const QWeight& w, float* out, const void* x, bool x_bf16, int batch, c
   return fail(GOPH_E_INVALID, "unknown weight format %d", w.fmt);
 }
 
+bool qgemm_scratch(int device, cudaStream_t stream) { return q_stream_bufs(device, stream) != nullptr; }
+
+void qgemm_weights(int device, int change) {
+  StreamAreas& s = stream_areas(device);
+  std::lock_guard<std::mutex> lock(s.mu);
+  s.weights += change;
+  if (s.weights > 0) return;
+  for (; s.n > 0; --s.n) {  // (reading the status word and freeing both wait for the device)
+    QBufs& b = s.bufs[s.n - 1];
+    int v = 0;
+    if (cudaMemcpy(&v, b.status, sizeof v, cudaMemcpyDeviceToHost) == cudaSuccess && s.lost_status == 0) s.lost_status = v;
+    cudaFree(b.xb);
+  }
+  cudaGetLastError();
+}
+
 int qgemm_status(int device) {
-  QBufs* b = q_bufs(device, false);
-  if (!b) return 0;
-  int v = -1;
-  cudaMemcpy(&v, b->status, sizeof v, cudaMemcpyDeviceToHost);
+  int v = 0;
+  if (QBufs* b = q_bufs(device, false)) {
+    v = -1;
+    cudaMemcpy(&v, b->status, sizeof v, cudaMemcpyDeviceToHost);
+  }
+  StreamAreas& s = stream_areas(device);
+  std::lock_guard<std::mutex> lock(s.mu);
+  if (v == 0) v = s.lost_status;
+  for (int i = 0; i < s.n && v == 0; ++i) {
+    v = -1;
+    cudaMemcpy(&v, s.bufs[i].status, sizeof v, cudaMemcpyDeviceToHost);
+  }
   return v;
 }
 
 void qgemm_status_clear(int device) {
-  QBufs* b = q_bufs(device, false);
-  if (b) cudaMemset(b->status, 0, sizeof(int));
+  if (QBufs* b = q_bufs(device, false)) cudaMemset(b->status, 0, sizeof(int));
+  StreamAreas& s = stream_areas(device);
+  std::lock_guard<std::mutex> lock(s.mu);
+  s.lost_status = 0;
+  for (int i = 0; i < s.n; ++i) cudaMemset(s.bufs[i].status, 0, sizeof(int));
 }
 
 }  // namespace goph

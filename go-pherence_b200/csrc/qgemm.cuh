@@ -27,6 +27,13 @@ struct QWeight {
 // for few rows (integer tensor-core GEMV, CUDA-core streaming, FP8 pieces).
 bool qgemm_wants(int fmt, bool tiled, bool x_bf16, int out_dim, int in_dim, int batch);
 
+// Layouts other than the tiled ones: whether a call on this stream has scratch (see q_stream_bufs); if not, it is the
+// business of the kernels for few rows, which need none.
+bool qgemm_scratch(int device, cudaStream_t stream);
+
+// A weight handle of any format was made (+1) or is being freed (-1).
+void qgemm_weights(int device, int change);
+
 // out [batch][out_dim] = x [batch][in_dim] . W^T, x f32 or bf16 bit patterns, 16-byte aligned.
 int qgemm(const QWeight& w, float* out, const void* x, bool x_bf16, int batch, cudaStream_t stream);
 

@@ -26,6 +26,10 @@
  *     on one device whose kernels could overlap on the GPU — different streams with no ordering
  *     between them — must be ordered by the caller (one stream, or events), whatever handles
  *     they use.  The reference launches everything on one stream, which satisfies this.
+ *     Products of weights in the other layouts need no such order and may be captured at any time:
+ *     those of several rows keep an area per stream (28 MB, for up to eight streams of a device,
+ *     until its last weight is freed) and use the kernels that need none where they have no area
+ *     (under capture, on further streams, without memory), whose sums are grouped differently.
  *   - Matrices are row-major; x is [batch, in_dim], out is [batch, out_dim], both f32.
  */
 #ifndef GOPH_B200_H

@@ -97,3 +97,87 @@ def test_row_gemv_has_the_looping_kernels_bits(gpu, pkg, in_dim, out_dims):
         assert pkg.synth.rel_err(a, w) <= 2e-3
     for t in hs + outs + [x]:
         t.Free()
+
+
+def _scaled_inputs(gpu, pkg, key, n, rows, in_dim):
+    """n inputs whose sizes lie far apart (a product that mixes two up is off by orders of magnitude), on the host and the device."""
+    xs = [pkg.synth.activations((key, i), rows * in_dim, bf16=False).reshape(rows, in_dim) * F(2.0 ** (7 * (i % 8) - 24)) for i in range(n)]
+    return xs, [gpu.from_numpy(x.reshape(-1)) for x in xs]
+
+
+def _check(got, x, W, bias):
+    """Against double precision, relative to the largest output of the activation row (f32 sums: see test_several_rows)."""
+    want = x.astype(np.float64) @ W.T + (0 if bias is None else bias)
+    ok = ~np.isnan(want)
+    assert np.max((np.abs(got - want) / np.nanmax(np.abs(want), axis=1, keepdims=True))[ok]) <= 2e-5
+    assert np.isnan(got[~ok]).all()
+
+
+@pytest.mark.parametrize("fmt", ["mlx", "q8_0", "q6_k", "fp8"])
+def test_row_major_products_need_no_order(gpu, pkg, fmt):
+    """Streams without an order between them (more of them than keep an area of scratch), then two threads on one stream."""
+    import threading
+    import torch
+    out_dim, in_dim, rows, n = 640, 2048, 24, 12
+    h, run, W, bias = make(gpu, pkg, fmt, False, out_dim, in_dim)
+    W = np.asarray(W, dtype=np.float64).reshape(out_dim, in_dim)
+    xs, xd = _scaled_inputs(gpu, pkg, ("order", fmt), n, rows, in_dim)
+    outs = [out_with_canary(gpu, rows * out_dim) for _ in range(n)]
+    call = {"mlx": lambda i, s: gpu.GemmMLX(outs[i], xd[i], h, rows, s), "fp8": lambda i, s: gpu.GemmFP8E4M3Buffer(outs[i], xd[i], rows, h, s)}.get(
+        fmt, lambda i, s: h.ProjectBatchToBuffer(outs[i], xd[i], rows, s))
+    streams = [torch.cuda.Stream() for _ in range(n)]
+    for _ in range(8):
+        for i in range(n):
+            call(i, streams[i])
+    gpu.Sync()
+    for i in range(n):
+        _check(read_and_check_canary(outs[i], rows * out_dim).reshape(rows, out_dim), xs[i], W, bias)
+        outs[i].Zero()
+
+    def work(i):
+        for _ in range(200):
+            call(i, None)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in (1, 6)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    gpu.Sync()
+    for i in (1, 6):
+        _check(outs[i].Download()[:rows * out_dim].reshape(rows, out_dim), xs[i], W, bias)
+    for t in [h] + xd + outs:
+        t.Free()
+    assert gpu.KernelStatus() == 0
+
+
+@pytest.mark.parametrize("fmt", ["mlx", "q8_0", "fp8"])
+def test_row_major_products_under_capture(gpu, pkg, fmt):
+    """The first call of all on a stream may be under capture (nothing is allocated), and two graphs may run beside each other."""
+    import torch
+    out_dim, in_dim, rows = 640, 2048, 24
+    h, run, W, bias = make(gpu, pkg, fmt, False, out_dim, in_dim)
+    W = np.asarray(W, dtype=np.float64).reshape(out_dim, in_dim)
+    xs, xd = _scaled_inputs(gpu, pkg, ("capture", fmt), 2, rows, in_dim)
+    outs = [out_with_canary(gpu, rows * out_dim) for _ in range(2)]
+    graphs, streams = [], [torch.cuda.Stream() for _ in range(2)]
+    capture = torch.cuda.Stream()
+    for i in range(2):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=capture):
+            if fmt == "mlx":
+                gpu.GemmMLX(outs[i], xd[i], h, rows, capture)
+            elif fmt == "fp8":
+                gpu.GemmFP8E4M3Buffer(outs[i], xd[i], rows, h, capture)
+            else:
+                h.ProjectBatchToBuffer(outs[i], xd[i], rows, capture)
+        graphs.append(g)
+    for _ in range(8):
+        for g, s in zip(graphs, streams):
+            with torch.cuda.stream(s):
+                g.replay()
+    gpu.Sync()
+    for i in range(2):
+        _check(read_and_check_canary(outs[i], rows * out_dim).reshape(rows, out_dim), xs[i], W, bias)
+    for t in [h] + xd + outs:
+        t.Free()
