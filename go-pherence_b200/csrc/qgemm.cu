@@ -49,6 +49,7 @@
 // passes of 16 f32 or 64 bf16 rows):
 //   Q8_0 4096x4096 x19 44.5 -> 15.1; Q4_K 14336x4096 x64 381 -> 29.3; MLX4 6144x4096 x100 f32 129 -> 20.7;
 //   MLX4 8192x8192 x64 bf16 33.2 -> 21.9; FP8 28672x8192 x256 bf16 226 -> 103
+#include <math_constants.h>
 #include <string.h>
 
 #include <mutex>
@@ -231,7 +232,10 @@ qg_prep_x_kernel(const void* __restrict__ xv, unsigned char* __restrict__ xb, un
   for (int i = 1; i < kPrepThreads / 32; ++i) mx = fmaxf(mx, red[i]);
   // x * 2^s: the largest element lands in [2^14, 2^15)
   int E = (int)((__float_as_uint(mx) >> 23) & 0xFFu) - 127;
-  if (mx == 0.f || E > 127) E = 14;  // an all-zero row, or inf / NaN in x (whose products are not finite anyway)
+  // A row with an infinity: its outputs are infinite with the sign of the weight there (NaN for a zero weight or
+  // two opposite ones) whatever the finite elements are, which only must not overflow an f16 themselves.
+  const bool infinite = E > 127;
+  if (mx == 0.f || infinite) E = 14;
   if (E < -112) E = -112;            // keeps 2^s a normal float
   const float s = __uint_as_float((uint32_t)(14 - E + 127) << 23);
   if (tid == 0 && blockIdx.y == 0) xinv[m] = __uint_as_float((uint32_t)(E - 14 + 127) << 23);
@@ -243,6 +247,11 @@ qg_prep_x_kernel(const void* __restrict__ xv, unsigned char* __restrict__ xb, un
     load8(k, v);
 #pragma unroll
     for (int e = 0; e < 8; ++e) v[e] *= s;
+    if (infinite) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        if (fabsf(v[e]) < CUDART_INF_F) v[e] = fminf(fmaxf(v[e], -65504.f), 65504.f);
+    }
     const int c = k >> 8, half = (k >> 7) & 1, step = (k >> 4) & 7, kh = (k >> 3) & 1;
     if (SUMS != 0) {
       // sums of x per scale group, as three bf16 pieces (exact): slots [piece][sum] of the affine term's
@@ -284,6 +293,7 @@ qg_prep_x_kernel(const void* __restrict__ xv, unsigned char* __restrict__ xb, un
         h[e] = f16_bits(v[e]);
         any |= h[e] & 0x7FFFu;
         v[e] -= __half2float(__ushort_as_half((unsigned short)h[e]));  // exact
+        if (infinite && (h[e] & 0x7FFFu) == 0x7C00u) v[e] = 0.f;       // (and not inf - inf)
       }
       uint32_t q[8];
 #pragma unroll

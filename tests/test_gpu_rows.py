@@ -181,3 +181,28 @@ def test_row_major_products_under_capture(gpu, pkg, fmt):
         _check(read_and_check_canary(outs[i], rows * out_dim).reshape(rows, out_dim), xs[i], W, bias)
     for t in [h] + xd + outs:
         t.Free()
+
+
+@pytest.mark.parametrize("tiled", [True, False])
+@pytest.mark.parametrize("fmt", ["q6_k", "fp8", "q8_0"])
+def test_an_infinite_activation(gpu, pkg, fmt, tiled):
+    """Formats without a minimum or bias: +-inf by the weight's sign, NaN where two infinities meet or the weight is
+    zero, as the dequantised weights give; large finite elements of the same row change nothing; other rows are not touched."""
+    out_dim, in_dim, rows = 256, 1024, 24
+    h, run, W, bias = make(gpu, pkg, fmt, tiled, out_dim, in_dim)
+    W = np.asarray(W, dtype=np.float64).reshape(out_dim, in_dim)
+    x = pkg.synth.activations(("inf", fmt), rows * in_dim, bf16=False).reshape(rows, in_dim)
+    x[0, 100] = np.inf
+    x[1, 700], x[1, 701] = -np.inf, F(1e30)
+    x[2, 5], x[2, 900] = np.inf, np.inf
+    x[3, 64] = np.nan
+    xo, out = gpu.from_numpy(x.reshape(-1)), out_with_canary(gpu, rows * out_dim)
+    run(out, xo, rows)
+    gpu.Sync()
+    got = read_and_check_canary(out, rows * out_dim).reshape(rows, out_dim)
+    with np.errstate(invalid="ignore"):
+        want = (x.astype(np.float64)[:4, None, :] * W[None]).sum(-1)
+    assert np.array_equal(got[:4], want.astype(F), equal_nan=True)
+    _check(got[4:], x[4:], W, bias)
+    for t in (h, xo, out):
+        t.Free()
