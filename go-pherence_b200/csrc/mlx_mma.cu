@@ -383,6 +383,7 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
   TP(const long long t_entry = clock64();)
   typedef StageWalkT<G> StageWalk;
   constexpr int EP = epi_parts<N, FMT>();
+  constexpr bool kSpills = !Fmt<FMT>::kConv && MB == 8;  // a byte per weight, eight rows: the epilogue is short of registers
   constexpr int kEpiWarps = 4 * EP, kEpiThreads = kEpiWarps * 32;
   constexpr int kWarpTMA = kConvWarps + kEpiWarps, kWarpMMA = kWarpTMA + 1;
   constexpr int kThreads = mma_threads<N, FMT>();
@@ -422,8 +423,9 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
 
   // (the shuffle tells the compiler that a warp's number is the same in all of its lanes: what follows from it is
   // kept in uniform registers, from where the MMAs take their operands.  MLX4 28672x4096 17.6 us without, 16.7
-  // with, Q4_K 4096x14336 12.7 and 12.0)
-  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  // with, Q4_K 4096x14336 12.7 and 12.0.  kSpills: there the cursor and the uniform numbers only cost spills,
+  // Q8_0 14336x4096 x5 32.3 us with and 28.2 without, 4096x14336 x6 37.1 and 32.8)
+  const int tid = threadIdx.x, warp = kSpills ? tid >> 5 : __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + S);
   const uint32_t aready0 = smem_u32(bars + 2 * S), afree0 = aready0 + 8 * NA;
   const uint32_t mdone0 = afree0 + 8 * NA, dfree0 = mdone0 + 8 * ND;  // mdone: a stage's accumulators are complete
@@ -676,7 +678,7 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
     constexpr int NLD = kNarrow ? 1 : kSub * N / 16;        // 16-column loads per pass
     RingCursor rc;
     for (int i = 0; sw.live(a) && ok; ++i, rc.next(S)) {
-      const int b = i % ND, slot = rc.s;
+      const int b = i % ND, slot = kSpills ? i % S : rc.s;
       if (G && sw.entry != cur_entry) {
         // a new entry: its tables, row count and result rows.  Every epilogue thread passed the barrier
         // that ends the item before, so nobody still reads the old tables.
@@ -689,7 +691,7 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
         for (int m = 0; m < (G ? MB : 1); ++m) orow[m] = a.gdirect ? __ldg(&ge->item[m]) : cur_entry * MB + m;
         asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
       }
-      ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * slot, rc.ph, a.status, 6));
+      ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * slot, kSpills ? (i / S) & 1 : rc.ph, a.status, 6));
       uint4 mvs[C];
       uint32_t q6d = 0;  // Q6_K: the super-block's f16 d (the 16 int8 scales are in mvs)
       const int nc = sw.nc();
