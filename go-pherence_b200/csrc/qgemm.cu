@@ -1314,9 +1314,12 @@ struct Plan {
 // The plan with the smallest estimate, in cycles of the busiest SM.  A chunk of an item takes the
 // largest of the tensor pipe's time (half a cycle per column and K16 step), the converters' (300
 // cycles a tile) and what the L2 can hand to one SM (45 bytes a cycle); sharing the last items costs two
-// meetings of the cluster and the exchange.  max_chunks: longest K range of an item.
+// meetings of the cluster and the exchange.  max_chunks: longest K range of an item.  The option mlx_splits asks
+// for a number of CTAs per shared item, as far as there is a plan with that many.
 bool choose_plan(int device, int ntiles, int nchunks, int nblocks, int n, int pieces, int wbytes, int NB, int max_chunks, Plan* best) {
   double best_cost = -1;
+  int want = options().mlx_splits < kMaxSplits ? options().mlx_splits : kMaxSplits;
+  if (want > nchunks) want = nchunks;
   for (int TT = NB == 128 ? 2 : 1; TT <= 2; ++TT) {
     if (TT == 2 && ntiles < 2) break;
     const int items = (ntiles + TT - 1) / TT * nblocks;
@@ -1330,7 +1333,8 @@ bool choose_plan(int device, int ntiles, int nchunks, int nblocks, int n, int pi
       const int nfull = items / grid * grid, ntail = items - nfull;
       if (ntail > clusters || (S > 1 && ntail == 0)) continue;  // the shared items are the last thing a cluster does
       if ((nfull && nchunks > max_chunks) || (ntail && (nchunks + S - 1) / S > max_chunks)) continue;
-      const double cost = (nfull / grid * (nchunks * chunk + 1500.0)) + (ntail ? (nchunks + S - 1) / S * chunk + 1500.0 : 0) + (S > 1 ? 1500.0 + TT * n * 8.0 : 0);
+      const double cost = (nfull / grid * (nchunks * chunk + 1500.0)) + (ntail ? (nchunks + S - 1) / S * chunk + 1500.0 : 0) + (S > 1 ? 1500.0 + TT * n * 8.0 : 0) +
+                          (want && S != want ? 1e12 : 0);
       if (best_cost < 0 || cost < best_cost) {
         best_cost = cost;
         *best = Plan{TT, nfull ? grid : ntail * S, nfull, ntail, S};

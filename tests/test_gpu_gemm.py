@@ -165,9 +165,10 @@ def test_fp8_small_shapes(gpu, pkg, out_dim, in_dim, all_codes, batch, xkind):
 
 @pytest.mark.parametrize("xkind", ["f32", "bf16"])
 @pytest.mark.parametrize("splits", [1, 2, 3, 7])
-def test_fp8_k_splits(gpu, pkg, splits, xkind):
-    # the K range of a tile shared by several CTAs (partial sums through device scratch, added in split order)
-    out_dim, in_dim, batch = 700, 4096, 5
+@pytest.mark.parametrize("batch", [5, 4])   # f32: the several-row kernel (sums through the cluster), the few-row one
+def test_fp8_k_splits(gpu, pkg, batch, splits, xkind):
+    # the K range of a tile shared by several CTAs (partial sums through device scratch or a cluster, added in split order)
+    out_dim, in_dim = 700, 4096
     w = _fp8_bytes(("ks", out_dim, in_dim), out_dim, in_dim)
     _, scale, bias = pkg.synth.fp8_linear(("ks", out_dim), out_dim, 16, bias=True)
     gpu.SetOption("fp8_layout", 2)

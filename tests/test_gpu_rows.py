@@ -26,7 +26,8 @@ def make(gpu, pkg, fmt, tiled, out_dim, in_dim):
             return h, lambda o, x, n: gpu.GemmMLX(o, x, h, n), orc.mlx_dequant(w, s, b, out_dim, in_dim, 64), None
         if fmt == "fp8":
             w, s, b = pkg.synth.fp8_linear("rows", out_dim, in_dim, bias=True)
-            w[(out_dim - 1) * in_dim + 7] = 0x7F  # a NaN code: its output element only
+            if not tiled:  # (a matrix with a NaN code keeps the row-major layout)
+                w[(out_dim - 1) * in_dim + 7] = 0x7F  # its output element only
             h = gpu.UploadFP8E4M3Linear(w, s, b, out_dim, in_dim)
             return h, lambda o, x, n: gpu.GemmFP8E4M3Buffer(o, x, n, h), orc.fp8_dequant(w, s, out_dim, in_dim), b
         qtype, gen = GGUF[fmt]
@@ -206,3 +207,34 @@ def test_an_infinite_activation(gpu, pkg, fmt, tiled):
     _check(got[4:], x[4:], W, bias)
     for t in (h, xo, out):
         t.Free()
+
+
+# one tile per item, two, and the 128-column blocks that are read straight from the tensor memory, the last one ragged
+@pytest.mark.parametrize("fmt,rows", [("mlx", 20), ("mlx_wide", 20), ("q4_k", 20), ("q6_k", 20), ("q8_0", 20), ("fp8", 20), ("q4_k", 64), ("fp8", 64),
+                                      ("fp8_bf16", 129), ("fp8_bf16", 256)])
+def test_several_rows_k_splits(gpu, pkg, fmt, rows):
+    """Every number of CTAs that can share an item; each groups the sums in its own way."""
+    out_dim, in_dim = 640, 2560
+    h, run, W, bias = make(gpu, pkg, fmt.split("_bf")[0], True, out_dim, in_dim)
+    W = np.asarray(W, dtype=np.float64).reshape(out_dim, in_dim)
+    x = pkg.synth.activations(("splits", rows), rows * in_dim, bf16=fmt == "fp8_bf16").reshape(rows, in_dim)
+    if fmt == "fp8_bf16":
+        xo = gpu.from_numpy(gpu.to_bf16_bits(x.reshape(-1)))
+        run = lambda o, xd, n: gpu.GemmFP8E4M3BF16Buffer(o, xd, n, h)
+    else:
+        xo = gpu.from_numpy(x.reshape(-1))
+    out, bits = out_with_canary(gpu, rows * out_dim), set()
+    try:
+        for splits in range(1, 9):
+            gpu.SetOption("mlx_splits", splits)
+            run(out, xo, rows)
+            gpu.Sync()
+            got = read_and_check_canary(out, rows * out_dim).reshape(rows, out_dim)
+            _check(got, x, W, bias)
+            bits.add(got.tobytes())
+    finally:
+        gpu.SetOption("mlx_splits", 0)
+    assert len(bits) > 4
+    for t in (h, xo, out):
+        t.Free()
+    assert gpu.KernelStatus() == 0
