@@ -486,7 +486,7 @@ attn_step_kernel(const __grid_constant__ AttnArgs a) {
 #pragma unroll
     for (int j = 0; j < T; ++j) {
       if (rank * kStepTile + warp + j * W > pos) continue;  // (a row that was never written may hold anything)
-      const float p = expf(sc[j] - m);
+      const float p = sc[j] == -CUDART_INF_F ? 0.f : expf(sc[j] - m);  // (all four may be: m is not the head's maximum)
       l += p;
 #pragma unroll
       for (int e = 0; e < EPL; ++e) acc[e] = fmaf(p, v[j][e], acc[e]);
@@ -532,7 +532,7 @@ attn_step_kernel(const __grid_constant__ AttnArgs a) {
 #pragma unroll
   for (int c = 0; c < kStepCtas; ++c) {
     if (c >= ctas) continue;
-    const float f = expf(all_ml[c].x - top);
+    const float f = all_ml[c].x == -CUDART_INF_F ? 0.f : expf(all_ml[c].x - top);
     den = fmaf(all_ml[c].y, f, den);
     num = fmaf(all[c][tid], f, num);
   }
@@ -772,6 +772,7 @@ static int attn_launch(int device, AttnArgs& a, int max_seq, bool fused, void* s
   if (splits > kAttnMaxSplits) splits = kAttnMaxSplits;
   if (splits < 1 || rows > 1) splits = 1;  // (the rows of a prompt chunk fill the machine without)
   const dim3 grid(a.heads, splits, rows);
+  static_assert(kStepTile * kStepCtas == 16 * kAttnMaxSplits, "below, a fused call is never small");
   if (fused && max_seq <= kStepTile * kStepCtas) {
     int ctas = 1;
     while (ctas * kStepTile < max_seq) ctas *= 2;

@@ -413,3 +413,32 @@ def test_prompt_in_chunks(gpu, pkg, prompt_len):
     assert got[:prompt_len + 1] == want[:prompt_len + 1] or top[1] - top[0] <= 2 * LOGIT_TOL * np.max(np.abs(ref))
     with pytest.raises(gpu.GophError):
         gpu.AttnRows(dec.attn, 1, dec.qkv, 1, 0, dec.L[0]["kc"], dec.L[0]["vc"], dec.pos, cfg.max_seq, 8, 4, 64, 1.0)
+
+
+@pytest.mark.parametrize("hidden_rows", [lambda pos: [t for t in range(pos) if t % 8 == 3],    # a warp's four positions
+                                         lambda pos: list(range(32, min(64, pos)))])           # a CTA's
+@pytest.mark.parametrize("max_seq,pos", [(64, 63), (256, 130), (1024, 130)])
+def test_fused_attention_of_minus_infinity(gpu, pkg, max_seq, pos, hidden_rows):
+    """Keys whose scores are minus infinity take no part in the softmax, also where a part of the cache has no others."""
+    heads, kv_heads, head_dim = 4, 2, 64
+    g = pkg.synth.rng("minf", max_seq)
+    kvd, table, scale = kv_heads * head_dim, od.rope_table(max_seq, head_dim, 1e6), 0.125
+    ref_k, ref_v = g.standard_normal((2, max_seq, kvd), dtype=F)
+    q, k, v = (g.standard_normal(n, dtype=F) for n in (heads * head_dim, kvd, kvd))
+    rq, rk = q.copy(), k.copy()
+    od.apply_rope(rq, table, pos, heads, head_dim)
+    od.apply_rope(rk, table, pos, kv_heads, head_dim)
+    for h in range(kv_heads):   # two query heads per key head: an element where both have the sign that gives minus infinity
+        d = [i for i in range(head_dim) if rq[2 * h * head_dim + i] * rq[(2 * h + 1) * head_dim + i] > 0][0]
+        ref_k[np.ix_(hidden_rows(pos), [h * head_dim + d])] = -np.sign(rq[2 * h * head_dim + d]) * F(np.inf)
+    kc, vc, T = gpu.from_numpy(ref_k.reshape(-1)), gpu.from_numpy(ref_v.reshape(-1)), gpu.from_numpy(table.reshape(-1))
+    Q, K, V, P = gpu.from_numpy(q), gpu.from_numpy(k), gpu.from_numpy(v), gpu.from_numpy(np.array([pos], dtype=np.int32))
+    out = gpu.Malloc(heads * head_dim)
+    gpu.AttnDecodeFused(out, Q, K, V, None, None, T, P, kc, vc, max_seq, heads, kv_heads, head_dim, scale, 1e-6)
+    gpu.Sync()
+    keep = [t for t in range(pos + 1) if t not in hidden_rows(pos)]
+    ref_k[pos], ref_v[pos] = rk, v
+    want = od.attention(rq, ref_k[keep], ref_v[keep], len(keep), heads, kv_heads, head_dim, scale)
+    assert np.allclose(out.Download(), want, rtol=1e-4, atol=2e-5)
+    for b in (kc, vc, T, Q, K, V, P, out):
+        b.Free()
