@@ -238,3 +238,19 @@ def test_several_rows_k_splits(gpu, pkg, fmt, rows):
     for t in (h, xo, out):
         t.Free()
     assert gpu.KernelStatus() == 0
+
+
+@pytest.mark.parametrize("tiled", [True, False])
+@pytest.mark.parametrize("rows", [2, 24])
+def test_pair_projection_refuses_before_it_launches(gpu, pkg, rows, tiled):
+    """A second output that is too short is refused before the first one is written."""
+    out_dim, in_dim = 256, 512
+    h, run, W, bias = make(gpu, pkg, "q4_k", tiled, out_dim, in_dim)
+    x = gpu.from_numpy(pkg.synth.activations("pairv", rows * in_dim, bf16=False))
+    a, b = out_with_canary(gpu, rows * out_dim), gpu.Malloc(rows * out_dim - 1)
+    with pytest.raises(gpu.GophError):
+        gpu.ProjectQ4PairToBuffers(a, b, x, rows, h, h)
+    gpu.Sync()
+    assert np.all(a.Download() == F(123.0))
+    for t in (h, x, a, b):
+        t.Free()
