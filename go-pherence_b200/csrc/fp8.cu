@@ -108,7 +108,7 @@ static bool qgemm_takes(const goph_fp8_linear* w, const void* x, bool x_bf16, in
 
 static int fp8_qgemm(const goph_fp8_linear* w, float* out, const void* x, bool x_bf16, int batch, cudaStream_t stream) {
   const QWeight q{Q_FP8, w->tiled != nullptr, w->tiled ? w->tiled : w->weight, nullptr, w->scale, w->bias, w->device, w->out_dim, w->in_dim};
-  return qgemm(q, out, x, x_bf16, batch, stream);
+  return qgemm(1, &q, &out, x, x_bf16, batch, stream);
 }
 
 }  // namespace goph

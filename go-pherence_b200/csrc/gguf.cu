@@ -364,9 +364,8 @@ static bool qgemm_takes(const goph_gguf_matrix* m, const void* x, int batch, cud
          (m->tiled || qgemm_scratch(m->device, stream));
 }
 
-static int gguf_qgemm(const goph_gguf_matrix* m, float* out, const float* x, int batch, cudaStream_t stream) {
-  const QWeight q{q_format(m->qtype), m->tiled != nullptr, m->tiled ? m->tiled : m->data, m->d16, nullptr, nullptr, m->device, m->out_dim, m->in_dim};
-  return qgemm(q, out, x, false, batch, stream);
+static QWeight q_weight(const goph_gguf_matrix* m) {
+  return QWeight{q_format(m->qtype), m->tiled != nullptr, m->tiled ? m->tiled : m->data, m->d16, nullptr, nullptr, m->device, m->out_dim, m->in_dim};
 }
 
 static long gguf_row_bytes(int qtype, int in_dim) {
@@ -529,7 +528,10 @@ GOPH_API int goph_gguf_project(float* out_dev, uint64_t out_len, const float* x_
     return fail(GOPH_E_INVALID, "buffers x=%llu/%llu out=%llu/%llu", (unsigned long long)x_len,
                 (unsigned long long)need_x, (unsigned long long)out_len, (unsigned long long)need_o);
   if (int rc = use_device(m->device)) return rc;
-  if (qgemm_takes(m, x_dev, batch, (cudaStream_t)stream)) return gguf_qgemm(m, out_dev, x_dev, batch, (cudaStream_t)stream);
+  if (qgemm_takes(m, x_dev, batch, (cudaStream_t)stream)) {
+    const QWeight q = q_weight(m);
+    return qgemm(1, &q, &out_dev, x_dev, false, batch, (cudaStream_t)stream);
+  }
   if (m->tiled) return gguf_mma_launch(m, out_dev, x_dev, batch, options().mlx_digits, (cudaStream_t)stream);
   StreamArgs a;
   memset(&a, 0, sizeof a);
@@ -578,7 +580,13 @@ GOPH_API int goph_gguf_project_pair(float* out_a_dev, uint64_t out_a_len, float*
                 (unsigned long long)need_x, (unsigned long long)out_a_len, (unsigned long long)need_a,
                 (unsigned long long)out_b_len, (unsigned long long)need_b);
   if (int rc = use_device(a->device)) return rc;
-  if (a->tiled && b->tiled && a->qtype == b->qtype && !qgemm_takes(a, x_dev, batch, (cudaStream_t)stream)) {  // x prepared once
+  const bool rows_a = qgemm_takes(a, x_dev, batch, (cudaStream_t)stream), rows_b = qgemm_takes(b, x_dev, batch, (cudaStream_t)stream);
+  if (rows_a && rows_b) {  // x prepared once
+    const QWeight q[2] = {q_weight(a), q_weight(b)};
+    float* const outs[2] = {out_a_dev, out_b_dev};
+    return qgemm(2, q, outs, x_dev, false, batch, (cudaStream_t)stream);
+  }
+  if (a->tiled && b->tiled && a->qtype == b->qtype && !rows_a) {  // here too
     if (int rc = gguf_mma_launch(a, out_a_dev, x_dev, batch, options().mlx_digits, (cudaStream_t)stream, false)) return rc;
     return gguf_mma_launch(b, out_b_dev, x_dev, batch, options().mlx_digits, (cudaStream_t)stream, true);
   }

@@ -1154,39 +1154,14 @@ static bool qgemm_takes(const goph_mlx_weight* w, const void* x, int batch, cuda
          qgemm_wants(Q_MLX4, w->tiled != nullptr, false, w->out_dim, w->in_dim, batch) && (w->tiled || qgemm_scratch(w->device, stream));
 }
 
-static int mlx_qgemm(const goph_mlx_weight* w, float* out, const void* x, bool x_bf16, int batch, cudaStream_t stream) {
-  const QWeight q{w->foldable ? Q_MLX4F : Q_MLX4, w->tiled != nullptr, w->tiled ? (const void*)w->tiled : w->qweight, w->sb, nullptr, nullptr, w->device, w->out_dim, w->in_dim};
-  return qgemm(q, out, x, x_bf16, batch, stream);
+static QWeight q_weight(const goph_mlx_weight* w) {
+  return QWeight{w->foldable ? Q_MLX4F : Q_MLX4, w->tiled != nullptr, w->tiled ? (const void*)w->tiled : w->qweight, w->sb, nullptr, nullptr, w->device, w->out_dim, w->in_dim};
 }
 
-// Products for n weights sharing x [batch,in]; outs[i] is [batch,out_i].
-static int mlx_products(int n, float* const* outs, const goph_mlx_weight* const* ws, const float* x, int batch,
-                        cudaStream_t stream) {
+// Row-major weights sharing x on the CUDA cores.
+static int mlx_row_products(int n, float* const* outs, const goph_mlx_weight* const* ws, const float* x, int batch,
+                            cudaStream_t stream) {
   const goph_mlx_weight* w0 = ws[0];
-  bool any_tiled = false, any_rows = false;
-  for (int i = 0; i < n; ++i) {
-    any_tiled = any_tiled || ws[i]->tiled;
-    any_rows = any_rows || qgemm_takes(ws[i], x, batch, stream);
-  }
-  if (any_tiled || any_rows) {
-    // tiled weights run on the tensor cores; row-major ones in the same call take their own path
-    bool prepared = false;  // weights of one call share x: its digits are prepared once
-    for (int i = 0; i < n; ++i) {
-      const goph_mlx_weight* one = ws[i];
-      float* o = outs[i];
-      int rc;
-      if (qgemm_takes(one, x, batch, stream)) {
-        rc = mlx_qgemm(one, o, x, false, batch, stream);
-      } else if (one->tiled) {
-        rc = mlx_mma_launch(one, o, x, batch, options().mlx_digits, stream, prepared);
-        prepared = true;
-      } else {
-        rc = mlx_products(1, &o, &one, x, batch, stream);
-      }
-      if (rc) return rc;
-    }
-    return GOPH_OK;
-  }
   bool uniform = true;
   for (int i = 0; i < n; ++i)
     uniform = uniform && fast_path_ok(ws[i]) && ws[i]->sb_bf16 == w0->sb_bf16;
@@ -1194,7 +1169,7 @@ static int mlx_products(int n, float* const* outs, const goph_mlx_weight* const*
     for (int i = 0; i < n; ++i) {
       const goph_mlx_weight* one = ws[i];
       float* o = outs[i];
-      int rc = fast_path_ok(one) ? mlx_products(1, &o, &one, x, batch, stream)
+      int rc = fast_path_ok(one) ? mlx_row_products(1, &o, &one, x, batch, stream)
                                  : launch_generic(one, o, x, batch, stream);
       if (rc) return rc;
     }
@@ -1216,6 +1191,33 @@ static int mlx_products(int n, float* const* outs, const goph_mlx_weight* const*
     if (int rc = launch_stream(ws, sub, n, x + (size_t)b0 * w0->in_dim, nb, stream)) return rc;
   }
   return GOPH_OK;
+}
+
+// Products for n weights sharing x [batch,in]; outs[i] is [batch,out_i].
+static int mlx_products(int n, float* const* outs, const goph_mlx_weight* const* ws, const float* x, int batch,
+                        cudaStream_t stream) {
+  // Weights of one call share x, which is prepared once for those of a kind: several rows on the tensor cores, few rows
+  // on the tensor cores (tiled weights), and the other row-major ones, which are launched together.
+  QWeight several[kMaxSeg];
+  float *several_out[kMaxSeg], *rest_out[kMaxSeg];
+  const goph_mlx_weight* rest[kMaxSeg];
+  int ns = 0, nr = 0;
+  bool prepared = false;
+  for (int i = 0; i < n; ++i) {
+    if (qgemm_takes(ws[i], x, batch, stream)) {
+      several[ns] = q_weight(ws[i]);
+      several_out[ns++] = outs[i];
+    } else if (ws[i]->tiled) {
+      if (int rc = mlx_mma_launch(ws[i], outs[i], x, batch, options().mlx_digits, stream, prepared)) return rc;
+      prepared = true;
+    } else {
+      rest[nr] = ws[i];
+      rest_out[nr++] = outs[i];
+    }
+  }
+  if (ns)
+    if (int rc = qgemm(ns, several, several_out, x, false, batch, stream)) return rc;
+  return nr ? mlx_row_products(nr, rest_out, rest, x, batch, stream) : GOPH_OK;
 }
 
 typedef void (*MlxProgramKernel)(const MlxArgs*, int, unsigned*, unsigned*, int*);
@@ -1654,7 +1656,8 @@ GOPH_API int goph_mlx_gemm_bf16(float* out_dev, uint64_t out_len, const uint16_t
                 "goph_mlx_gemm_bf16 needs a weight in the tiled layout (group size 64, in_dim a multiple of 256, "
                 "uploaded with mlx_layout 0 or 2); this one is row-major");
   if (int rc = use_device(w->device)) return rc;
-  return mlx_qgemm(w, out_dev, x_bf16_dev, true, batch, (cudaStream_t)stream);
+  const QWeight q = q_weight(w);
+  return qgemm(1, &q, &out_dev, x_bf16_dev, true, batch, (cudaStream_t)stream);
 }
 
 GOPH_API int goph_mlx_gemv(float* out_dev, uint64_t out_len, const float* x_dev, uint64_t x_len,

@@ -1390,12 +1390,16 @@ int launch_product(QArgs& a, const Plan& p, int n, int device, cudaStream_t stre
   return GOPH_OK;
 }
 
+// What an area of scratch holds of the call's x, so that weights of one call share its preparation.
+struct Prepared {
+  bool valid = false;
+  int order, sums, nb;
+  float unit;
+};
+
 template <int F, bool TILED, bool XBF16>
-int run_rows(const QWeight& w, float* out, const void* x, int batch, cudaStream_t stream) {
+int run_rows(const QWeight& w, float* out, const void* x, int batch, QBufs* bufs, Prepared* prep, cudaStream_t stream) {
   typedef QF<F, TILED> T;
-  QBufs* bufs = TILED ? q_bufs(w.device) : q_stream_bufs(w.device, stream);
-  if (!bufs) return fail(GOPH_E_NOMEM, "cannot allocate the several-row products' device scratch");
-  std::lock_guard<std::mutex> enqueue(bufs->enqueue);
   constexpr int pmax = XBF16 ? 1 : 3;
   const int nchunks = (w.in_dim + kChunkK - 1) / kChunkK;
   const size_t xstride = (size_t)w.in_dim * (XBF16 ? 2 : 4);
@@ -1452,10 +1456,17 @@ int run_rows(const QWeight& w, float* out, const void* x, int batch, cudaStream_
     if (slices > (nchunks + 7) / 8) slices = (nchunks + 7) / 8;
     cfg.gridDim = dim3(rows, slices < 1 ? 1 : slices);
     cfg.blockDim = dim3(kPrepThreads);
-    note_launch();
-    GOPH_CUDA(cudaLaunchKernelEx(&cfg, qg_prep_x_kernel<T::kOrder, T::kSums, XBF16>,
-                                 static_cast<const void*>(static_cast<const unsigned char*>(x) + (size_t)b0 * xstride), bufs->xb,
-                                 bufs->xaux, bufs->xinv, bufs->flags, rows, w.in_dim, nchunks, NB, a.xb_stride, 1.f / T::kUnit));
+    if (!(prep->valid && rows == batch && prep->order == T::kOrder && prep->sums == T::kSums && prep->nb == NB && prep->unit == T::kUnit)) {
+      note_launch();
+      GOPH_CUDA(cudaLaunchKernelEx(&cfg, qg_prep_x_kernel<T::kOrder, T::kSums, XBF16>,
+                                   static_cast<const void*>(static_cast<const unsigned char*>(x) + (size_t)b0 * xstride), bufs->xb,
+                                   bufs->xaux, bufs->xinv, bufs->flags, rows, w.in_dim, nchunks, NB, a.xb_stride, 1.f / T::kUnit));
+      prep->valid = rows == batch;
+      prep->order = T::kOrder;
+      prep->sums = T::kSums;
+      prep->nb = NB;
+      prep->unit = T::kUnit;
+    }
     int rc;
     if constexpr (F == Q_FP8 && TILED && XBF16) {
       if (NB == 128) rc = launch_product<F, TILED, 2, 128>(a, p, n, w.device, stream);
@@ -1470,14 +1481,27 @@ int run_rows(const QWeight& w, float* out, const void* x, int batch, cudaStream_
 }
 
 template <int F>
-int run_fmt(const QWeight& w, float* out, const void* x, bool x_bf16, int batch, cudaStream_t stream) {
+int run_fmt(const QWeight& w, float* out, const void* x, bool x_bf16, int batch, QBufs* bufs, Prepared* prep, cudaStream_t stream) {
   if constexpr (F == Q_MLX4 || F == Q_MLX4F || F == Q_FP8) {
     if (x_bf16)
-      return w.tiled ? run_rows<F, true, true>(w, out, x, batch, stream) : fail(GOPH_E_UNSUPPORTED, "bf16 activations need the tiled layout");
+      return w.tiled ? run_rows<F, true, true>(w, out, x, batch, bufs, prep, stream) : fail(GOPH_E_UNSUPPORTED, "bf16 activations need the tiled layout");
   } else if (x_bf16) {
     return fail(GOPH_E_UNSUPPORTED, "bf16 activations: MLX 4-bit and FP8 only");
   }
-  return w.tiled ? run_rows<F, true, false>(w, out, x, batch, stream) : run_rows<F, false, false>(w, out, x, batch, stream);
+  return w.tiled ? run_rows<F, true, false>(w, out, x, batch, bufs, prep, stream) : run_rows<F, false, false>(w, out, x, batch, bufs, prep, stream);
+}
+
+int run_one(const QWeight& w, float* out, const void* x, bool x_bf16, int batch, QBufs* bufs, Prepared* prep, cudaStream_t stream) {
+  switch (w.fmt) {
+    case Q_MLX4: return run_fmt<Q_MLX4>(w, out, x, x_bf16, batch, bufs, prep, stream);
+    case Q_MLX4F: return run_fmt<Q_MLX4F>(w, out, x, x_bf16, batch, bufs, prep, stream);
+    case Q_Q4K: return run_fmt<Q_Q4K>(w, out, x, x_bf16, batch, bufs, prep, stream);
+    case Q_Q5K: return run_fmt<Q_Q5K>(w, out, x, x_bf16, batch, bufs, prep, stream);
+    case Q_Q6K: return run_fmt<Q_Q6K>(w, out, x, x_bf16, batch, bufs, prep, stream);
+    case Q_Q80: return run_fmt<Q_Q80>(w, out, x, x_bf16, batch, bufs, prep, stream);
+    case Q_FP8: return run_fmt<Q_FP8>(w, out, x, x_bf16, batch, bufs, prep, stream);
+  }
+  return fail(GOPH_E_INVALID, "unknown weight format %d", w.fmt);
 }
 
 }  // namespace
@@ -1503,19 +1527,25 @@ bool qgemm_wants(int fmt, bool tiled, bool x_bf16, int out_dim, int in_dim, int 
   return batch > (large ? (fmt == Q_Q5K || fmt == Q_MLX4 || fmt == Q_MLX4F ? 4 : 3) : 8);
 }
 
-int qgemm(const QWeight& w, float* out, const void* x, bool x_bf16, int batch, cudaStream_t stream) {
-  if (w.in_dim > kMaxIn) return fail(GOPH_E_UNSUPPORTED, "several-row products: in_dim=%d is above %d", w.in_dim, kMaxIn);
+int qgemm(int n, const QWeight* w, float* const* out, const void* x, bool x_bf16, int batch, cudaStream_t stream) {
   if ((uintptr_t)x % 16) return fail(GOPH_E_INVALID, "x must be 16-byte aligned");
-  switch (w.fmt) {
-    case Q_MLX4: return run_fmt<Q_MLX4>(w, out, x, x_bf16, batch, stream);
-    case Q_MLX4F: return run_fmt<Q_MLX4F>(w, out, x, x_bf16, batch, stream);
-    case Q_Q4K: return run_fmt<Q_Q4K>(w, out, x, x_bf16, batch, stream);
-    case Q_Q5K: return run_fmt<Q_Q5K>(w, out, x, x_bf16, batch, stream);
-    case Q_Q6K: return run_fmt<Q_Q6K>(w, out, x, x_bf16, batch, stream);
-    case Q_Q80: return run_fmt<Q_Q80>(w, out, x, x_bf16, batch, stream);
-    case Q_FP8: return run_fmt<Q_FP8>(w, out, x, x_bf16, batch, stream);
+  bool any[2] = {};
+  for (int i = 0; i < n; ++i) {
+    if (w[i].in_dim > kMaxIn) return fail(GOPH_E_UNSUPPORTED, "several-row products: in_dim=%d is above %d", w[i].in_dim, kMaxIn);
+    any[w[i].tiled] = true;
   }
-  return fail(GOPH_E_INVALID, "unknown weight format %d", w.fmt);
+  // the device's area for tiled weights, the stream's for the others; both are held to the call's last launch
+  QBufs* bufs[2] = {any[0] ? q_stream_bufs(w[0].device, stream) : nullptr, any[1] ? q_bufs(w[0].device) : nullptr};
+  std::unique_lock<std::mutex> held[2];
+  Prepared prep[2];
+  for (int t = 0; t < 2; ++t) {
+    if (!any[t]) continue;
+    if (!bufs[t]) return fail(GOPH_E_NOMEM, "cannot allocate the several-row products' device scratch");
+    held[t] = std::unique_lock<std::mutex>(bufs[t]->enqueue);
+  }
+  for (int i = 0; i < n; ++i)
+    if (int rc = run_one(w[i], out[i], x, x_bf16, batch, bufs[w[i].tiled], &prep[w[i].tiled], stream)) return rc;
+  return GOPH_OK;
 }
 
 bool qgemm_scratch(int device, cudaStream_t stream) { return q_stream_bufs(device, stream) != nullptr; }

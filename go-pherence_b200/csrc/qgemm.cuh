@@ -34,8 +34,9 @@ bool qgemm_scratch(int device, cudaStream_t stream);
 // A weight handle of any format was made (+1) or is being freed (-1).
 void qgemm_weights(int device, int change);
 
-// out [batch][out_dim] = x [batch][in_dim] . W^T, x f32 or bf16 bit patterns, 16-byte aligned.
-int qgemm(const QWeight& w, float* out, const void* x, bool x_bf16, int batch, cudaStream_t stream);
+// out[i] [batch][out_dim] = x [batch][in_dim] . W[i]^T for n weights of one device and in_dim, x f32 or bf16 bit
+// patterns, 16-byte aligned, prepared once for weights of the same format and kind of layout.
+int qgemm(int n, const QWeight* w, float* const* out, const void* x, bool x_bf16, int batch, cudaStream_t stream);
 
 int qgemm_status(int device);
 void qgemm_status_clear(int device);

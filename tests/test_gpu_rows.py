@@ -254,3 +254,35 @@ def test_pair_projection_refuses_before_it_launches(gpu, pkg, rows, tiled):
     assert np.all(a.Download() == F(123.0))
     for t in (h, x, a, b):
         t.Free()
+
+
+def test_weights_of_one_call_share_the_preparation(gpu, pkg):
+    """The bits of separate calls, with a launch per weight and one per kind of preparation: MLX weights of both kinds of
+    scales, in both layouts, in an order that mixes them."""
+    in_dim, rows = 1024, 40
+    kinds = [("mlx", True), ("mlx_wide", True), ("mlx", False), ("mlx", True), ("mlx_wide", False), ("mlx", False)]
+    hs = [make(gpu, pkg, fmt, tiled, 4096 + 128 * i, in_dim)[0] for i, (fmt, tiled) in enumerate(kinds)]
+    x = gpu.from_numpy(pkg.synth.activations("share", rows * in_dim, bf16=False))
+    outs = [[out_with_canary(gpu, rows * h.OutDim) for h in hs] for _ in range(2)]
+    for h, o in zip(hs, outs[0]):
+        gpu.GemmMLX(o, x, h, rows)
+    for pick, kinds_prepared in (([0, 3], 1), ([2, 5], 1), ([0, 1, 3], 3), ([0, 3, 1], 2), ([0, 2, 3, 5], 2), ([0, 1, 2, 3, 4, 5], 6)):
+        before = gpu.LaunchCount()
+        gpu.GemmMLXMulti([outs[1][i] for i in pick], x, [hs[i] for i in pick], rows)
+        assert gpu.LaunchCount() - before == len(pick) + kinds_prepared, pick
+        gpu.Sync()
+        for i in pick:
+            n = rows * hs[i].OutDim
+            assert np.array_equal(read_and_check_canary(outs[0][i], n), read_and_check_canary(outs[1][i], n))
+            outs[1][i].Upload(np.full(n + 64, 123.0, dtype=F))
+    a, b = (make(gpu, pkg, "q4_k", True, o, in_dim)[0] for o in (640, 384))
+    oa, ob = ([out_with_canary(gpu, rows * h.OutDim) for _ in range(2)] for h in (a, b))
+    a.ProjectBatchToBuffer(oa[0], x, rows)
+    b.ProjectBatchToBuffer(ob[0], x, rows)
+    before = gpu.LaunchCount()
+    gpu.ProjectQ4PairToBuffers(oa[1], ob[1], x, rows, a, b)
+    assert gpu.LaunchCount() - before == 3
+    gpu.Sync()
+    assert np.array_equal(oa[0].Download(), oa[1].Download()) and np.array_equal(ob[0].Download(), ob[1].Download())
+    for t in hs + outs[0] + outs[1] + [a, b, x] + oa + ob:
+        t.Free()
