@@ -1149,9 +1149,8 @@ static int launch_generic(const goph_mlx_weight* w, float* out, const float* x, 
 }
 
 // The several-row tensor-core product (qgemm.cu) reads both layouts of 64-element groups with bf16 tables.
-static bool qgemm_takes(const goph_mlx_weight* w, const void* x, int batch, cudaStream_t stream) {
-  return w->group_size == 64 && w->sb_bf16 && w->in_dim <= 65536 && (uintptr_t)x % 16 == 0 &&
-         qgemm_wants(Q_MLX4, w->tiled != nullptr, false, w->out_dim, w->in_dim, batch) && (w->tiled || qgemm_scratch(w->device, stream));
+static bool qgemm_reads(const goph_mlx_weight* w, const void* x) {
+  return w->group_size == 64 && w->sb_bf16 && w->in_dim <= 65536 && (uintptr_t)x % 16 == 0;
 }
 
 static QWeight q_weight(const goph_mlx_weight* w) {
@@ -1196,15 +1195,28 @@ static int mlx_row_products(int n, float* const* outs, const goph_mlx_weight* co
 // Products for n weights sharing x [batch,in]; outs[i] is [batch,out_i].
 static int mlx_products(int n, float* const* outs, const goph_mlx_weight* const* ws, const float* x, int batch,
                         cudaStream_t stream) {
-  // Weights of one call share x, which is prepared once for those of a kind: several rows on the tensor cores, few rows
-  // on the tensor cores (tiled weights), and the other row-major ones, which are launched together.
+  bool any_tiled = false, rows_wanted = false;  // rows_wanted: the row-major weights go to the several-row product
+  for (int i = 0; i < n; ++i) any_tiled = any_tiled || ws[i]->tiled;
+  if (batch > 1) {
+    int weights = 0;
+    long out_dims = 0;
+    for (int i = 0; i < n; ++i) {
+      if (ws[i]->tiled || !qgemm_reads(ws[i], x)) continue;
+      ++weights;
+      out_dims += ws[i]->out_dim;
+    }
+    rows_wanted = weights && qgemm_wants(Q_MLX4, false, false, out_dims, ws[0]->in_dim, batch, weights) && qgemm_scratch(ws[0]->device, stream);
+  }
+  if (!any_tiled && !rows_wanted) return mlx_row_products(n, outs, ws, x, batch, stream);
+  // x is prepared once for the weights of a kind: several rows on the tensor cores, few rows on the tensor cores
+  // (tiled weights), and the other row-major ones, which are launched together.
   QWeight several[kMaxSeg];
   float *several_out[kMaxSeg], *rest_out[kMaxSeg];
   const goph_mlx_weight* rest[kMaxSeg];
   int ns = 0, nr = 0;
   bool prepared = false;
   for (int i = 0; i < n; ++i) {
-    if (qgemm_takes(ws[i], x, batch, stream)) {
+    if (qgemm_reads(ws[i], x) && (ws[i]->tiled ? qgemm_wants(Q_MLX4, true, false, ws[i]->out_dim, ws[i]->in_dim, batch) : rows_wanted)) {
       several[ns] = q_weight(ws[i]);
       several_out[ns++] = outs[i];
     } else if (ws[i]->tiled) {

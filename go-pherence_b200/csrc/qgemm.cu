@@ -49,7 +49,6 @@
 // passes of 16 f32 or 64 bf16 rows):
 //   Q8_0 4096x4096 x19 44.5 -> 15.1; Q4_K 14336x4096 x64 381 -> 29.3; MLX4 6144x4096 x100 f32 129 -> 20.7;
 //   MLX4 8192x8192 x64 bf16 33.2 -> 21.9; FP8 28672x8192 x256 bf16 226 -> 103
-#include <math_constants.h>
 #include <string.h>
 
 #include <mutex>
@@ -232,10 +231,10 @@ qg_prep_x_kernel(const void* __restrict__ xv, unsigned char* __restrict__ xb, un
   for (int i = 1; i < kPrepThreads / 32; ++i) mx = fmaxf(mx, red[i]);
   // x * 2^s: the largest element lands in [2^14, 2^15)
   int E = (int)((__float_as_uint(mx) >> 23) & 0xFFu) - 127;
-  // A row with an infinity: its outputs are infinite with the sign of the weight there (NaN for a zero weight or
-  // two opposite ones) whatever the finite elements are, which only must not overflow an f16 themselves.
-  const bool infinite = E > 127;
-  if (mx == 0.f || infinite) E = 14;
+  // A row with an infinity: its outputs are infinite with the sign of the weight there (NaN for a zero weight or two
+  // opposite ones) whatever the finite elements are, which only must not overflow an f16 themselves.
+  if (mx == 0.f) E = 14;
+  if (E > 127) E = 127;
   if (E < -112) E = -112;            // keeps 2^s a normal float
   const float s = __uint_as_float((uint32_t)(14 - E + 127) << 23);
   if (tid == 0 && blockIdx.y == 0) xinv[m] = __uint_as_float((uint32_t)(E - 14 + 127) << 23);
@@ -247,11 +246,6 @@ qg_prep_x_kernel(const void* __restrict__ xv, unsigned char* __restrict__ xb, un
     load8(k, v);
 #pragma unroll
     for (int e = 0; e < 8; ++e) v[e] *= s;
-    if (infinite) {
-#pragma unroll
-      for (int e = 0; e < 8; ++e)
-        if (fabsf(v[e]) < CUDART_INF_F) v[e] = fminf(fmaxf(v[e], -65504.f), 65504.f);
-    }
     const int c = k >> 8, half = (k >> 7) & 1, step = (k >> 4) & 7, kh = (k >> 3) & 1;
     if (SUMS != 0) {
       // sums of x per scale group, as three bf16 pieces (exact): slots [piece][sum] of the affine term's
@@ -293,7 +287,7 @@ qg_prep_x_kernel(const void* __restrict__ xv, unsigned char* __restrict__ xb, un
         h[e] = f16_bits(v[e]);
         any |= h[e] & 0x7FFFu;
         v[e] -= __half2float(__ushort_as_half((unsigned short)h[e]));  // exact
-        if (infinite && (h[e] & 0x7FFFu) == 0x7C00u) v[e] = 0.f;       // (and not inf - inf)
+        if ((h[e] & 0x7FFFu) >= 0x7C00u) v[e] = 0.f;                   // (and not inf - inf)
       }
       uint32_t q[8];
 #pragma unroll
@@ -1506,25 +1500,46 @@ int run_one(const QWeight& w, float* out, const void* x, bool x_bf16, int batch,
 
 }  // namespace
 
-// The lines lie where the two times met at 1024x1024 (us at 8 rows: 6-8 for the few-row kernels, 10 here, most
-// of it two launches), 1536x4096, 4096x4096, 14336x4096, 4096x14336 and 8192x8192.  Tiled layouts: the GEMV
-// kernels take 8 rows a launch (Q4_K, Q5_K, Q6_K: 4), so a second launch, or the wider accumulator blocks of 5 to 8
-// rows, decide; Q6_K and Q8_0 have a block per 16 or 32 elements here too and gain later.  Other layouts: the
-// CUDA-core kernels' time grows with the rows, above 4 Mi weights from the fourth.
-bool qgemm_wants(int fmt, bool tiled, bool x_bf16, int out_dim, int in_dim, int batch) {
-  if (x_bf16) return fmt != Q_FP8 || batch > 16;  // (FP8 14336x4096: 16 rows 16.7 against 18.2, 24 rows 22.7 against 21.2)
+// The lines lie where this kernel's time and the few-row kernels' met (B200, us a call: few-row / this).
+// Tiled layouts: the GEMV kernels take 8 rows a launch (Q4_K, Q5_K: 4), so a second launch, or the wider accumulator
+// blocks of 5 to 8 rows, decide.  Q6_K and Q8_0, with a block per 16 or 32 elements here too, gain later on large matrices.
+// Other layouts: the CUDA-core kernels' time grows with the rows and the weights, this one's hardly, but two launches
+// and the start cost it 8 to 10 us (Q5_K 12, Q6_K 20, converted from the streaming layout).  A weight of `weights` that
+// share x costs a launch of its own here, while the MLX streaming kernel takes all of them in one; out_dim is their sum.
+bool qgemm_wants(int fmt, bool tiled, bool x_bf16, long out_dim, int in_dim, int batch, int weights) {
+  if (x_bf16) return fmt != Q_FP8 || batch > 16;  // FP8 14336x4096: 16 rows 16.7 / 18.2, 24 rows 22.7 / 21.2
+  const long size = out_dim * in_dim, Mi = 1l << 20;
   if (tiled) {
     switch (fmt) {
-      case Q_Q4K: return batch > 3;                       // 4 rows: 24.1 against 23.4 (14336x4096)
-      case Q_MLX4: case Q_MLX4F: case Q_Q5K: return batch > 4;  // 5 rows, MLX4: 24.6 against 21.0
-      case Q_Q6K: return batch > 12;                      // 16 rows: 93 against 70
-      case Q_FP8: return batch > 4;                       // 5 rows: 20.3 against 20.6; 8192x28672 58.5 against 53.2
-      default: return batch > 8;                          // Q8_0 9 rows: 42.9 against 42.3
-    }
+      case Q_Q4K: return batch > 3;                             // 14336x4096 4 rows 21.5 / 21.4, 4096x4096 12.4 / 11.7
+      case Q_MLX4: case Q_MLX4F: case Q_Q5K: return batch > 4;  // MLX 4096x4096 4 rows 10.5 / 11.0, 5 rows 16.2 / 10.9; Q5_K 14336x4096 19.8 / 21.5, 48 / 21.5
+      case Q_FP8: return batch > 4;                             // 4096x14336 4 rows 17.4 / 19.7, 5 rows 34.1 / 19.8
+      default: return batch > (size <= 16 * Mi ? 4 : 8);        // Q6_K 4096x4096 4 rows 12.9 / 17.8, 5 rows 19.5 / 17.7; 14336x4096 8 rows 46.4 / 53.4,
+    }                                                           // 9 rows 58.7 / 53.3; Q8_0 4096x4096 15.8 / 13.4 at 5, 14336x4096 28.5 / 33.6 at 8, 39.7 / 33.6 at 9
   }
-  const bool large = (long)out_dim * in_dim >= (4l << 20);
-  if (fmt == Q_Q6K) return batch > (large ? 8 : 16);
-  return batch > (large ? (fmt == Q_Q5K || fmt == Q_MLX4 || fmt == Q_MLX4F ? 4 : 3) : 8);
+  if (weights > 1) {  // (MLX) by their mean size: 2048, 1024 and 1024 rows of 1024 at 16 rows 21.6 / 23.8, at 20 28.4 / 25.2;
+    const long mean = size / weights;  // 2048, 512, 512 of 2048 at 10 22.1 / 27.6, at 14 30.8 / 27.6; twice 2048x2048 at 8 18.4 / 21.3, at 9 22.0 / 21.3;
+    return batch > (mean < Mi ? 24 : mean < 2 * Mi ? 16 : mean < 3 * Mi ? 10 : mean < 5 * Mi ? 8 : 4);  // twice 2000x4096 at 4 18.3 / 23.7, at 5 30.3 / 23.8
+  }
+  // Above 8 Mi weights this layout is the exception (widths that no tile takes, NaN codes, the layout options).
+  // in_dim above 8192: four rows of x no longer fit the CUDA-core kernels' shared memory, which then read the weights again.
+  const bool small = size < 4 * Mi, long_rows = size >= 6 * Mi && in_dim >= 4096, wide_x = in_dim > 8192;
+  switch (fmt) {
+    case Q_Q6K:  // 1024x1024 24 rows 16.0 / 20.5; 3072x1024 16 rows 19.5 / 20.3, 20 rows 25.0 / 20.9; 2048x2048 16 rows 23.4 / 34.4; 1536x4096 12 rows 29.7 / 34.5,
+                 // 14 rows 36.1 / 34.5; 14336x4096 24 rows 160 / 208; 4096x14336 8 rows 165 / 179, 9 rows 200 / 179
+      return batch > (size < 2 * Mi ? 24 : wide_x && size >= 8 * Mi ? 8 : size > 16 * Mi ? 24 : long_rows ? 12 : 16);
+    case Q_Q5K:  // 512x2048 10 rows 11.7 / 12.8, 12 rows 13.1 / 12.8; 2048x2048 8 rows 13.0 / 16.5, 9 rows 17.1 / 16.5; 1536x4096 4 rows 12.9 / 18.5, 5 rows 20.3 / 18.6
+      return batch > (size < 2 * Mi ? 10 : long_rows || size >= 8 * Mi ? 4 : 8);
+    case Q_Q4K: case Q_MLX4: case Q_MLX4F:  // MLX 1024x1024 8 rows 5.6 / 8.5, 9 rows 9.5 / 8.4; 2048x2048 4 rows 7.8 / 11.0, 5 rows 12.8 / 10.9; 1536x4096 2 rows 8.0 / 11.2,
+                                            // 3 rows 12.8 / 11.2; 8192x2112 2 rows 13.9 / 15.4, 3 rows 22.1 / 15.3; 28672x4160 4 rows 59.5 / 66.7, 5 rows 104 / 67
+      return batch > (small ? 8 : (long_rows || (size >= 8 * Mi && in_dim > 1024)) && size <= 64 * Mi ? 2 : 4);
+    case Q_FP8:  // 1024x2048 8 rows 7.0 / 9.1, 9 rows 9.2 / 9.1; 7000x1024 4 rows 8.3 / 10.7, 5 rows 12.8 / 10.6; 4096x4160 4 rows 19.7 / 17.9; 28672x4160 4 rows 54.6 / 63.7;
+                 // 512x14336 2 rows 17.1 / 19.3, 3 rows 32.2 / 19.3; 8192x8256 2 rows 35.9 / 37.4, 3 rows 67.6 / 37.3
+      return batch > (small ? 8 : wide_x ? 2 : size >= 16 * Mi && size < 48 * Mi ? 3 : 4);
+    default:     // Q8_0 2048x2048 8 rows 11.5 / 14.1, 9 rows 15.0 / 14.1; 1536x4096 4 rows 11.0 / 14.4, 5 rows 19.2 / 14.4; 28672x1088 4 rows 23.2 / 34.5, 5 rows 42.7 / 34.6;
+                 // 8192x8256 2 rows 39.8 / 61.0, 3 rows 68.6 / 61.0; 512x14336 2 rows 15.3 / 27.4, 3 rows 27.8 / 27.4
+      return batch > (small ? 8 : wide_x ? 2 : long_rows || size >= 8 * Mi ? 4 : 8);
+  }
 }
 
 int qgemm(int n, const QWeight* w, float* const* out, const void* x, bool x_bf16, int batch, cudaStream_t stream) {

@@ -24,8 +24,9 @@ struct QWeight {
 };
 
 // Whether `batch` activation rows of such a weight go to this kernel; the others are the business of the kernels
-// for few rows (integer tensor-core GEMV, CUDA-core streaming, FP8 pieces).
-bool qgemm_wants(int fmt, bool tiled, bool x_bf16, int out_dim, int in_dim, int batch);
+// for few rows (integer tensor-core GEMV, CUDA-core streaming, FP8 pieces).  `weights` of one call that share x and could
+// share a launch there count together, out_dim being the sum of theirs.
+bool qgemm_wants(int fmt, bool tiled, bool x_bf16, long out_dim, int in_dim, int batch, int weights = 1);
 
 // Layouts other than the tiled ones: whether a call on this stream has scratch (see q_stream_bufs); if not, it is the
 // business of the kernels for few rows, which need none.
