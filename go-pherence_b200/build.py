@@ -5,6 +5,7 @@ objects are linked into one shared library with the CUDA runtime linked statical
 library has no toolkit dependency at run time beyond the driver.
 """
 import os
+import platform
 import subprocess
 import sys
 import sysconfig
@@ -17,7 +18,8 @@ CSRC = os.path.join(HERE, "csrc")
 TUNING = os.environ.get("GOPH_TUNING") == "1"
 OBJ = os.path.join(HERE, "build_tuning" if TUNING else "build")
 LIB = os.path.join(HERE, "libgoph_b200_tuning.so" if TUNING else "libgoph_b200.so")
-PYCALL = os.path.join(HERE, "goph_pycall.so")  # the caller of the C ABI that runtime.py uses
+# the caller of the C ABI that runtime.py uses, for this Python (the suffix names its version and machine)
+PYCALL = os.path.join(HERE, "goph_pycall" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
@@ -57,8 +59,16 @@ def _compile(src, verbose):
     return obj, True
 
 
+def _pycall_wanted():
+    """runtime.py does without the module (through ctypes, slower) where it cannot be: another machine, no Python headers."""
+    return platform.machine() in ("x86_64", "AMD64") and os.name == "posix" and os.path.exists(
+        os.path.join(sysconfig.get_paths()["include"], "Python.h"))
+
+
 def _build_pycall(force):
     src = os.path.join(CSRC, "pycall.c")
+    if not _pycall_wanted():
+        return
     if not force and os.path.exists(PYCALL) and os.path.getmtime(PYCALL) >= os.path.getmtime(src):
         return
     cmd = [os.environ.get("CC", "gcc"), "-O2", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"], src, "-o", PYCALL]

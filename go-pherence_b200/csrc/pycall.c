@@ -4,6 +4,9 @@
  * Signature letters: p address (number, None, bytes, or an object with a number as .value), n / i numbers, f float.
  * System V x86-64: integer words go to the integer registers and the stack in their order, floats to the vector
  * registers in theirs, so one call with all words and two floats serves every signature. */
+#if !defined(__x86_64__) || defined(__ILP32__) || defined(_WIN32)
+#error "written for the System V x86-64 calling convention; the package does without this module elsewhere"
+#endif
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <stddef.h>

@@ -12,6 +12,7 @@ import ctypes as C
 import importlib.util
 import os
 import struct
+import sysconfig
 
 import numpy as np
 
@@ -64,10 +65,14 @@ _HOT = {
 }
 
 
+_CTYPES = {"p": C.c_void_p, "n": C.c_uint64, "i": C.c_int, "f": C.c_float}
+
+
 def _pycall():
-    path = os.path.join(_HERE, "goph_pycall.so")
+    """The module, or None where the build made none for this Python: its calls then go through ctypes."""
+    path = os.path.join(_HERE, "goph_pycall" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
     if not os.path.exists(path):
-        raise GophError(-1, "goph_pycall.so is not built (run __graft_entry__.build())")
+        return None
     spec = importlib.util.spec_from_file_location("goph_pycall", path)
     mod = importlib.util.module_from_spec(spec)
     spec.loader.exec_module(mod)
@@ -99,7 +104,10 @@ def lib():
             getattr(L, name).argtypes = [C.c_void_p]
         call = _pycall()
         for name, sig in _HOT.items():
-            setattr(L, name, call.Function(C.cast(getattr(L, name), C.c_void_p).value, sig))
+            if call is not None:
+                setattr(L, name, call.Function(C.cast(getattr(L, name), C.c_void_p).value, sig))
+            else:
+                getattr(L, name).argtypes = [_CTYPES[k] for k in sig]
         _lib = L
     return _lib
 
