@@ -892,12 +892,15 @@ qg_kernel(const __grid_constant__ QArgs a) {
       if constexpr (TT == 1 && !kItemBlock) {
         float4* cb = reinterpret_cast<float4*>(comb) + r;
 #pragma unroll
-        for (int g = 0; g < NB / 4; ++g)
-          if (4 * g < n && (g & 1) != w) cb[g * kTileRows] = make_float4(acc[2 * g].x, acc[2 * g].y, acc[2 * g + 1].x, acc[2 * g + 1].y);
+        for (int g = 0; g < NB / 4; ++g) {
+          if (4 * g >= n) break;  // (out of the unrolled loop: a step over each group costs an instruction fetch)
+          if ((g & 1) != w) cb[g * kTileRows] = make_float4(acc[2 * g].x, acc[2 * g].y, acc[2 * g + 1].x, acc[2 * g + 1].y);
+        }
         asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
 #pragma unroll
         for (int g = 0; g < NB / 4; ++g) {
-          if (4 * g < n && (g & 1) == w) {
+          if (4 * g >= n) break;
+          if ((g & 1) == w) {
             const float4 o = cb[g * kTileRows];
             acc[2 * g].x += o.x;
             acc[2 * g].y += o.y;
@@ -1039,7 +1042,8 @@ qg_kernel(const __grid_constant__ QArgs a) {
         if (ok) {
 #pragma unroll
           for (int g = 0; g < NB / 4; ++g) {
-            if (4 * g < n && (TT == 2 || (g & 1) == w)) {
+            if (4 * g >= n) break;
+            if (TT == 2 || (g & 1) == w) {
               store(4 * g, acc[2 * g].x);
               store(4 * g + 1, acc[2 * g].y);
               store(4 * g + 2, acc[2 * g + 1].x);
@@ -1074,7 +1078,10 @@ qg_kernel(const __grid_constant__ QArgs a) {
           }
         } else {
 #pragma unroll
-          for (int g = 0; g < NB / 4; ++g) ring[g * kTileRows] = make_float4(acc[2 * g].x, acc[2 * g].y, acc[2 * g + 1].x, acc[2 * g + 1].y);
+          for (int g = 0; g < NB / 4; ++g) {
+            if (4 * g >= block_cols<NB>(a, wk.nb)) break;
+            ring[g * kTileRows] = make_float4(acc[2 * g].x, acc[2 * g].y, acc[2 * g + 1].x, acc[2 * g + 1].y);
+          }
         }
       }
       if (e == 0) { MARK(7, 2); }
