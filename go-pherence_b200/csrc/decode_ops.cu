@@ -483,10 +483,13 @@ attn_step_kernel(const __grid_constant__ AttnArgs a) {
     }
 #pragma unroll
     for (int e = 0; e < EPL; ++e) acc[e] = 0.f;
+    // (all four scores may be minus infinity though the head's maximum is not; asked once here and not for each, which
+    // cost 80 ns a launch)
+    const float m0 = m == -CUDART_INF_F ? 0.f : m;
 #pragma unroll
     for (int j = 0; j < T; ++j) {
       if (rank * kStepTile + warp + j * W > pos) continue;  // (a row that was never written may hold anything)
-      const float p = sc[j] == -CUDART_INF_F ? 0.f : expf(sc[j] - m);  // (all four may be: m is not the head's maximum)
+      const float p = expf(sc[j] - m0);
       l += p;
 #pragma unroll
       for (int e = 0; e < EPL; ++e) acc[e] = fmaf(p, v[j][e], acc[e]);
@@ -532,7 +535,7 @@ attn_step_kernel(const __grid_constant__ AttnArgs a) {
 #pragma unroll
   for (int c = 0; c < kStepCtas; ++c) {
     if (c >= ctas) continue;
-    const float f = all_ml[c].x == -CUDART_INF_F ? 0.f : expf(all_ml[c].x - top);
+    const float f = expf(all_ml[c].x - top);
     den = fmaf(all_ml[c].y, f, den);
     num = fmaf(all[c][tid], f, num);
   }
