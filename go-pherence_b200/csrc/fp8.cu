@@ -101,14 +101,16 @@ static bool valid_fp8(const goph_fp8_linear* w) {
 }
 
 // The several-row tensor-core product (qgemm.cu) reads both layouts (rows of whole 16-byte units).
-static bool qgemm_takes(const goph_fp8_linear* w, const void* x, bool x_bf16, int batch, cudaStream_t stream) {
+// rows: its scratch in the row-major layout.
+static bool qgemm_takes(const goph_fp8_linear* w, const void* x, bool x_bf16, int batch, cudaStream_t stream, QBufs** rows) {
+  *rows = nullptr;
   return w->in_dim % 16 == 0 && w->in_dim <= 65536 && (uintptr_t)x % 16 == 0 &&
-         qgemm_wants(Q_FP8, w->tiled != nullptr, x_bf16, w->out_dim, w->in_dim, batch) && (w->tiled || qgemm_scratch(w->device, stream));
+         qgemm_wants(Q_FP8, w->tiled != nullptr, x_bf16, w->out_dim, w->in_dim, batch) && (w->tiled || (*rows = qgemm_scratch(w->device, stream)));
 }
 
-static int fp8_qgemm(const goph_fp8_linear* w, float* out, const void* x, bool x_bf16, int batch, cudaStream_t stream) {
+static int fp8_qgemm(const goph_fp8_linear* w, float* out, const void* x, bool x_bf16, int batch, QBufs* rows, cudaStream_t stream) {
   const QWeight q{Q_FP8, w->tiled != nullptr, w->tiled ? w->tiled : w->weight, nullptr, w->scale, w->bias, w->device, w->out_dim, w->in_dim};
-  return qgemm(1, &q, &out, x, x_bf16, batch, stream);
+  return qgemm(1, &q, &out, x, x_bf16, batch, rows, stream);
 }
 
 }  // namespace goph
@@ -244,7 +246,8 @@ GOPH_API int goph_fp8_gemm(float* out_dev, uint64_t out_len, const float* x_dev,
   cudaStream_t s = (cudaStream_t)stream;
   // Several rows: qgemm.cu.  Few rows: in the tensor-core layout the kernel that feeds the e4m3 bytes to the
   // MMA as they lie (fp8_mma.cu), in the row-major layout the CUDA-core kernels below.
-  if (qgemm_takes(w, x_dev, false, batch, s)) return fp8_qgemm(w, out_dev, x_dev, false, batch, s);
+  QBufs* rows;
+  if (qgemm_takes(w, x_dev, false, batch, s, &rows)) return fp8_qgemm(w, out_dev, x_dev, false, batch, rows, s);
   if (w->tiled) return tc_gemm_fp8(w, out_dev, x_dev, false, batch, s);
   if (!w->tiled && w->in_dim % 16 != 0) {
     note_launch();
@@ -284,7 +287,8 @@ GOPH_API int goph_fp8_gemm_bf16(float* out_dev, uint64_t out_len, const uint16_t
                 "goph_fp8_gemm_bf16 needs a linear in the tensor-core layout (in_dim a multiple of 256, no NaN codes, "
                 "uploaded with fp8_layout 0 or 2)");
   if (int rc = use_device(w->device)) return rc;
-  if (qgemm_takes(w, x_bf16_dev, true, batch, (cudaStream_t)stream)) return fp8_qgemm(w, out_dev, x_bf16_dev, true, batch, (cudaStream_t)stream);
+  QBufs* rows;
+  if (qgemm_takes(w, x_bf16_dev, true, batch, (cudaStream_t)stream, &rows)) return fp8_qgemm(w, out_dev, x_bf16_dev, true, batch, rows, (cudaStream_t)stream);
   return tc_gemm_fp8(w, out_dev, x_bf16_dev, true, batch, (cudaStream_t)stream);
 }
 

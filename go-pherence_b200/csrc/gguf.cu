@@ -359,9 +359,10 @@ static int q_format(int qtype) {
 }
 
 // The several-row tensor-core product (qgemm.cu) reads both layouts.
-static bool qgemm_takes(const goph_gguf_matrix* m, const void* x, int batch, cudaStream_t stream) {
+// rows: its scratch in the streaming layout.
+static bool qgemm_takes(const goph_gguf_matrix* m, const void* x, int batch, cudaStream_t stream, QBufs** rows) {
   return m->in_dim <= 65536 && (uintptr_t)x % 16 == 0 && qgemm_wants(q_format(m->qtype), m->tiled != nullptr, false, m->out_dim, m->in_dim, batch) &&
-         (m->tiled || qgemm_scratch(m->device, stream));
+         (m->tiled || (*rows = qgemm_scratch(m->device, stream)));
 }
 
 static QWeight q_weight(const goph_gguf_matrix* m) {
@@ -528,9 +529,10 @@ GOPH_API int goph_gguf_project(float* out_dev, uint64_t out_len, const float* x_
     return fail(GOPH_E_INVALID, "buffers x=%llu/%llu out=%llu/%llu", (unsigned long long)x_len,
                 (unsigned long long)need_x, (unsigned long long)out_len, (unsigned long long)need_o);
   if (int rc = use_device(m->device)) return rc;
-  if (qgemm_takes(m, x_dev, batch, (cudaStream_t)stream)) {
+  QBufs* rows = nullptr;
+  if (qgemm_takes(m, x_dev, batch, (cudaStream_t)stream, &rows)) {
     const QWeight q = q_weight(m);
-    return qgemm(1, &q, &out_dev, x_dev, false, batch, (cudaStream_t)stream);
+    return qgemm(1, &q, &out_dev, x_dev, false, batch, rows, (cudaStream_t)stream);
   }
   if (m->tiled) return gguf_mma_launch(m, out_dev, x_dev, batch, options().mlx_digits, (cudaStream_t)stream);
   StreamArgs a;
@@ -580,11 +582,12 @@ GOPH_API int goph_gguf_project_pair(float* out_a_dev, uint64_t out_a_len, float*
                 (unsigned long long)need_x, (unsigned long long)out_a_len, (unsigned long long)need_a,
                 (unsigned long long)out_b_len, (unsigned long long)need_b);
   if (int rc = use_device(a->device)) return rc;
-  const bool rows_a = qgemm_takes(a, x_dev, batch, (cudaStream_t)stream), rows_b = qgemm_takes(b, x_dev, batch, (cudaStream_t)stream);
+  QBufs* rows = nullptr;
+  const bool rows_a = qgemm_takes(a, x_dev, batch, (cudaStream_t)stream, &rows), rows_b = qgemm_takes(b, x_dev, batch, (cudaStream_t)stream, &rows);
   if (rows_a && rows_b) {  // x prepared once
     const QWeight q[2] = {q_weight(a), q_weight(b)};
     float* const outs[2] = {out_a_dev, out_b_dev};
-    return qgemm(2, q, outs, x_dev, false, batch, (cudaStream_t)stream);
+    return qgemm(2, q, outs, x_dev, false, batch, rows, (cudaStream_t)stream);
   }
   if (a->tiled && b->tiled && a->qtype == b->qtype && !rows_a) {  // here too
     if (int rc = gguf_mma_launch(a, out_a_dev, x_dev, batch, options().mlx_digits, (cudaStream_t)stream, false)) return rc;

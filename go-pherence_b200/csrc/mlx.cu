@@ -1195,7 +1195,8 @@ static int mlx_row_products(int n, float* const* outs, const goph_mlx_weight* co
 // Products for n weights sharing x [batch,in]; outs[i] is [batch,out_i].
 static int mlx_products(int n, float* const* outs, const goph_mlx_weight* const* ws, const float* x, int batch,
                         cudaStream_t stream) {
-  bool any_tiled = false, rows_wanted = false;  // rows_wanted: the row-major weights go to the several-row product
+  bool any_tiled = false;
+  QBufs* rows = nullptr;  // the scratch of row-major weights that go to the several-row product
   for (int i = 0; i < n; ++i) any_tiled = any_tiled || ws[i]->tiled;
   if (batch > 1) {
     int weights = 0;
@@ -1205,9 +1206,9 @@ static int mlx_products(int n, float* const* outs, const goph_mlx_weight* const*
       ++weights;
       out_dims += ws[i]->out_dim;
     }
-    rows_wanted = weights && qgemm_wants(Q_MLX4, false, false, out_dims, ws[0]->in_dim, batch, weights) && qgemm_scratch(ws[0]->device, stream);
+    if (weights && qgemm_wants(Q_MLX4, false, false, out_dims, ws[0]->in_dim, batch, weights)) rows = qgemm_scratch(ws[0]->device, stream);
   }
-  if (!any_tiled && !rows_wanted) return mlx_row_products(n, outs, ws, x, batch, stream);
+  if (!any_tiled && !rows) return mlx_row_products(n, outs, ws, x, batch, stream);
   // x is prepared once for the weights of a kind: several rows on the tensor cores, few rows on the tensor cores
   // (tiled weights), and the other row-major ones, which are launched together.
   QWeight several[kMaxSeg];
@@ -1216,7 +1217,7 @@ static int mlx_products(int n, float* const* outs, const goph_mlx_weight* const*
   int ns = 0, nr = 0;
   bool prepared = false;
   for (int i = 0; i < n; ++i) {
-    if (qgemm_reads(ws[i], x) && (ws[i]->tiled ? qgemm_wants(Q_MLX4, true, false, ws[i]->out_dim, ws[i]->in_dim, batch) : rows_wanted)) {
+    if (qgemm_reads(ws[i], x) && (ws[i]->tiled ? qgemm_wants(Q_MLX4, true, false, ws[i]->out_dim, ws[i]->in_dim, batch) : rows != nullptr)) {
       several[ns] = q_weight(ws[i]);
       several_out[ns++] = outs[i];
     } else if (ws[i]->tiled) {
@@ -1228,7 +1229,7 @@ static int mlx_products(int n, float* const* outs, const goph_mlx_weight* const*
     }
   }
   if (ns)
-    if (int rc = qgemm(ns, several, several_out, x, false, batch, stream)) return rc;
+    if (int rc = qgemm(ns, several, several_out, x, false, batch, rows, stream)) return rc;
   return nr ? mlx_row_products(nr, rest_out, rest, x, batch, stream) : GOPH_OK;
 }
 
@@ -1669,7 +1670,7 @@ GOPH_API int goph_mlx_gemm_bf16(float* out_dev, uint64_t out_len, const uint16_t
                 "uploaded with mlx_layout 0 or 2); this one is row-major");
   if (int rc = use_device(w->device)) return rc;
   const QWeight q = q_weight(w);
-  return qgemm(1, &q, &out_dev, x_bf16_dev, true, batch, (cudaStream_t)stream);
+  return qgemm(1, &q, &out_dev, x_bf16_dev, true, batch, nullptr, (cudaStream_t)stream);
 }
 
 GOPH_API int goph_mlx_gemv(float* out_dev, uint64_t out_len, const float* x_dev, uint64_t x_len,

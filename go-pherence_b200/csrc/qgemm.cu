@@ -17,11 +17,12 @@
 //       Q5_K   11, the most an f16 holds), so a block of columns lasts a super-block.
 //       Q6_K   q - 32, a block per 16 elements (an 8-bit scale times 6 bits does not fit).
 //       Q8_0   the signed byte, a block per 32 elements.
-//       FP8    e4m3 -> f16 (exact, NaN codes stay NaN), a block of 4096 elements.
+//       FP8    e4m3 -> f16 (exact, NaN codes stay NaN), a block of 4096 elements (128 columns: of an item, at most 8192).
 //   * B operand (activations): every row is scaled by a power of two so that its largest magnitude
 //     lies in [2^14, 2^15), and written as the sum of up to three f16 values, each the rounding of
 //     what the ones before it left over.  Three hold an f32 exactly down to 2^-39 of the row's largest
-//     element (f32 sums do not see below that); a bf16 needs one.  All pieces accumulate into the
+//     element (f32 sums do not see below that, unless the weights at the larger elements are zero); a bf16 needs
+//     one.  A row with an infinity is scaled by 2^-113.  All pieces accumulate into the
 //     same columns.  The preparation kernel notes per row and 256 elements how many pieces are not
 //     zero: f32 buffers that hold bf16 values cost one pass of the tensor cores, not three.
 //   * The affine term (biases or minima times the groups' sums of x) is one or two more K16 steps per
@@ -60,6 +61,18 @@ namespace goph {
 
 using namespace tc;
 
+// The preparation and the product of a call meet in scratch; `enqueue` is held from the one launch to the other, so
+// that calls of several threads on one stream do not come between them.
+struct QBufs {
+  unsigned char* xb = nullptr;
+  unsigned char* xaux = nullptr;
+  float* xinv = nullptr;
+  unsigned char* flags = nullptr;
+  int* status = nullptr;
+  size_t xb_bytes = 0;
+  std::mutex enqueue;
+};
+
 namespace {
 
 // Tuning build only (-DGOPH_TUNING): one CTA records clock64 at the hand-over points.
@@ -80,6 +93,8 @@ constexpr int kWarpMMA = kConvWarps + kEpiWarps, kWarpB = kWarpMMA + 2, kWarpW =
 constexpr int kThreads = (kWarpW + 1) * 32;
 // Registers: the block is launched with 72 a thread (896 threads: 64512); the epilogue, which keeps a
 // row's sums of 64 columns, takes what the others give up: 256 * 128 + 512 * 48 + 128 * 56 = 64512.
+// The compiler allots 72 to every role all the same and spills up to 160 bytes a thread in the epilogue's (frames of
+// 8 to 40 bytes, the forms with two tiles most).
 constexpr int kEpiRegs = 128, kConvRegs = 48, kMiscRegs = 56;
 constexpr int kMaxSplits = 8;
 constexpr int kMaxRows = 256;                       // activation rows of one launch
@@ -1042,8 +1057,10 @@ qg_kernel(const __grid_constant__ QArgs a) {
         if (ok) {
 #pragma unroll
           for (int g = 0; g < NB / 4; ++g) {
-            if (4 * g >= n) break;
-            if (TT == 2 || (g & 1) == w) {
+            // (with two tiles the way out costs Q5_K and Q6_K registers in the main loop: Q6_K 6144x24832 x91 392 us
+            // against 386, where Q8_0 14336x4096 x200 takes 148 with it and 157 without)
+            if ((TT == 1 || (F != Q_Q5K && F != Q_Q6K)) && 4 * g >= n) break;
+            if (4 * g < n && (TT == 2 || (g & 1) == w)) {
               store(4 * g, acc[2 * g].x);
               store(4 * g + 1, acc[2 * g].y);
               store(4 * g + 2, acc[2 * g + 1].x);
@@ -1172,18 +1189,6 @@ constexpr size_t kXauxBytes = (size_t)(kMaxRows / 64) * (kMaxIn / kChunkK) * 64 
 constexpr size_t kFlagBytes = (size_t)(kMaxRows / 64) * (kMaxIn / kChunkK) * 64;
 constexpr size_t kSmemBudget2 = 227 * 1024;         // all that a CTA may have
 
-// The preparation and the product of a call meet in scratch; `enqueue` is held from the one launch to the other, so
-// that calls of several threads on one stream do not come between them.
-struct QBufs {
-  unsigned char* xb = nullptr;
-  unsigned char* xaux = nullptr;
-  float* xinv = nullptr;
-  unsigned char* flags = nullptr;
-  int* status = nullptr;
-  size_t xb_bytes = 0;
-  std::mutex enqueue;
-};
-
 bool carve(QBufs* b, size_t xb_bytes) {
   const size_t total = xb_bytes + kXauxBytes + kMaxRows * 4 + kFlagBytes + 256;
   unsigned char* p = nullptr;
@@ -1239,37 +1244,6 @@ struct StreamAreas {
 StreamAreas& stream_areas(int device) {
   static StreamAreas areas[kMaxDevices];
   return areas[device];
-}
-
-QBufs* q_stream_bufs(int device, cudaStream_t stream) {
-  cudaStreamCaptureStatus capture;
-  unsigned long long id;
-  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone || cudaStreamGetId(stream, &id) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  StreamAreas& s = stream_areas(device);
-  std::lock_guard<std::mutex> lock(s.mu);
-  for (int i = 0; i < s.n; ++i)
-    if (s.id[i] == id) return &s.bufs[i];
-  if (s.n == kStreamAreas) return nullptr;
-  // (another thread may be capturing a stream of its own, which an allocation must not disturb)
-  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-  if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  QBufs& b = s.bufs[s.n];
-  bool ok = carve(&b, kStreamXbBytes);
-  if (ok && cudaMemsetAsync(b.status, 0, 256, stream) != cudaSuccess) {
-    cudaGetLastError();
-    cudaFree(b.xb);
-    ok = false;
-  }
-  cudaThreadExchangeStreamCaptureMode(&mode);
-  if (!ok) return nullptr;
-  s.id[s.n++] = id;
-  return &b;
 }
 
 // Clusters of `size` CTAs that the device holds at once (every CTA takes a whole SM, so this is a
@@ -1549,7 +1523,7 @@ bool qgemm_wants(int fmt, bool tiled, bool x_bf16, long out_dim, int in_dim, int
   }
 }
 
-int qgemm(int n, const QWeight* w, float* const* out, const void* x, bool x_bf16, int batch, cudaStream_t stream) {
+int qgemm(int n, const QWeight* w, float* const* out, const void* x, bool x_bf16, int batch, QBufs* rows, cudaStream_t stream) {
   if ((uintptr_t)x % 16) return fail(GOPH_E_INVALID, "x must be 16-byte aligned");
   bool any[2] = {};
   for (int i = 0; i < n; ++i) {
@@ -1557,7 +1531,7 @@ int qgemm(int n, const QWeight* w, float* const* out, const void* x, bool x_bf16
     any[w[i].tiled] = true;
   }
   // the device's area for tiled weights, the stream's for the others; both are held to the call's last launch
-  QBufs* bufs[2] = {any[0] ? q_stream_bufs(w[0].device, stream) : nullptr, any[1] ? q_bufs(w[0].device) : nullptr};
+  QBufs* bufs[2] = {any[0] ? rows : nullptr, any[1] ? q_bufs(w[0].device) : nullptr};
   std::unique_lock<std::mutex> held[2];
   Prepared prep[2];
   for (int t = 0; t < 2; ++t) {
@@ -1570,7 +1544,38 @@ int qgemm(int n, const QWeight* w, float* const* out, const void* x, bool x_bf16
   return GOPH_OK;
 }
 
-bool qgemm_scratch(int device, cudaStream_t stream) { return q_stream_bufs(device, stream) != nullptr; }
+QBufs* qgemm_scratch(int device, cudaStream_t stream) {
+  unsigned long long id = ~0ull;  // the legacy default stream, which is never captured: no questions (0.5 us a call)
+  if (stream != nullptr && stream != cudaStreamLegacy) {
+    cudaStreamCaptureStatus capture;
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone || cudaStreamGetId(stream, &id) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+  }
+  StreamAreas& s = stream_areas(device);
+  std::lock_guard<std::mutex> lock(s.mu);
+  for (int i = 0; i < s.n; ++i)
+    if (s.id[i] == id) return &s.bufs[i];
+  if (s.n == kStreamAreas) return nullptr;
+  // (another thread may be capturing a stream of its own, which an allocation must not disturb)
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  QBufs& b = s.bufs[s.n];
+  bool ok = carve(&b, kStreamXbBytes);
+  if (ok && cudaMemsetAsync(b.status, 0, 256, stream) != cudaSuccess) {
+    cudaGetLastError();
+    cudaFree(b.xb);
+    ok = false;
+  }
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (!ok) return nullptr;
+  s.id[s.n++] = id;
+  return &b;
+}
 
 void qgemm_weights(int device, int change) {
   StreamAreas& s = stream_areas(device);

@@ -28,16 +28,18 @@ struct QWeight {
 // share a launch there count together, out_dim being the sum of theirs.
 bool qgemm_wants(int fmt, bool tiled, bool x_bf16, long out_dim, int in_dim, int batch, int weights = 1);
 
-// Layouts other than the tiled ones: whether a call on this stream has scratch (see q_stream_bufs); if not, it is the
-// business of the kernels for few rows, which need none.
-bool qgemm_scratch(int device, cudaStream_t stream);
+// Layouts other than the tiled ones: the scratch of a call on this stream (see the definition), which qgemm wants; if
+// there is none, the call is the business of the kernels for few rows, which need none.
+struct QBufs;
+QBufs* qgemm_scratch(int device, cudaStream_t stream);
 
 // A weight handle of any format was made (+1) or is being freed (-1).
 void qgemm_weights(int device, int change);
 
 // out[i] [batch][out_dim] = x [batch][in_dim] . W[i]^T for n weights of one device and in_dim, x f32 or bf16 bit
-// patterns, 16-byte aligned, prepared once for weights of the same format and kind of layout.
-int qgemm(int n, const QWeight* w, float* const* out, const void* x, bool x_bf16, int batch, cudaStream_t stream);
+// patterns, 16-byte aligned, prepared once for weights of the same format and kind of layout.  rows: qgemm_scratch's
+// answer where a weight is not tiled.
+int qgemm(int n, const QWeight* w, float* const* out, const void* x, bool x_bf16, int batch, QBufs* rows, cudaStream_t stream);
 
 int qgemm_status(int device);
 void qgemm_status_clear(int device);

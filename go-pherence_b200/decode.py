@@ -232,9 +232,10 @@ class MLXDecoder:
 
     @staticmethod
     def _graph_stream():
-        """The stream that a graph's replay goes to."""
+        """The stream that a graph's replay goes to (None: the default stream, as the library's calls name it)."""
         import torch
-        return torch.cuda.current_stream()
+        s = torch.cuda.current_stream()
+        return s if s.cuda_stream else None
 
     def generate(self, prompt, max_new, use_graph=True, logits_at=None, logits_all=None):
         """Returns prompt + max_new greedy tokens.  logits_at: optional list that receives the logits

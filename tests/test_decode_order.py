@@ -44,18 +44,20 @@ def _config(**more):
                                            qk_norm=True, max_seq=300), **more})
 
 
+@pytest.mark.parametrize("stream", [4096, 0])   # a side stream, the default one
 @pytest.mark.parametrize("use_graph", [True, False])
 @pytest.mark.parametrize("prompt", [1, 3, 4, 200])   # by steps, by steps, one chunk, two chunks
-def test_prompt_and_steps_share_a_stream(pkg, monkeypatch, prompt, use_graph):
-    rt, c, side = _Runtime(), _config(), object()
+def test_prompt_and_steps_share_a_stream(pkg, monkeypatch, prompt, use_graph, stream):
+    rt, c, side = _Runtime(), _config(), types.SimpleNamespace(cuda_stream=stream)
     part = (np.zeros((1, 1)),) * 3
     layers = [dict({n: part for n in ("q", "k", "v", "o", "gate", "up", "down")}, input_norm=[0.0], post_norm=[0.0], q_norm=[0.0], k_norm=[0.0])] * c.layers
     dec = pkg.decode.MLXDecoder(rt, c, layers, part, [0.0], np.zeros(2))
     monkeypatch.setattr("torch.cuda.current_stream", lambda *a: side)
-    dec.graph = types.SimpleNamespace(replay=lambda: rt.launches.append(("replay", side)))   # torch replays on the current stream
+    dec.graph = types.SimpleNamespace(replay=lambda: rt.launches.append(("replay", side if stream else None)))   # torch replays on the current stream
     dec.generate(list(range(prompt)), 2, use_graph=use_graph)
     assert len(rt.launches) >= 2
-    assert {s for _, s in rt.launches} == {side if use_graph else None}
+    want = side if use_graph and stream else None
+    assert all(s is want for _, s in rt.launches)
 
 
 @pytest.mark.gpu
