@@ -49,7 +49,7 @@
 // Measured (B200, a call among others, us; before: integer products of 4 or 8 rows, or the bf16 kernel's
 // passes of 16 f32 or 64 bf16 rows):
 //   Q8_0 4096x4096 x19 44.5 -> 15.1; Q4_K 14336x4096 x64 381 -> 29.3; MLX4 6144x4096 x100 f32 129 -> 20.7;
-//   MLX4 8192x8192 x64 bf16 33.2 -> 21.9; FP8 28672x8192 x256 bf16 226 -> 103
+//   MLX4 8192x8192 x64 bf16 33.2 -> 21.8; FP8 28672x8192 x256 bf16 226 -> 103 to 123 by the box
 #include <string.h>
 
 #include <mutex>

@@ -91,18 +91,21 @@ int goph_sm_count(int device);
  *                 prologue and weight prefetch overlap the tail of the kernel in front; 0 plain launches
  *   "mlx_layout"  device layout chosen by goph_mlx_upload.  The tiled layout feeds the tensor-core
  *                 (tcgen05) kernel and needs group size 64, in_dim a multiple of 256 and bf16-valued
- *                 scales and biases; the row-major layout feeds the CUDA-core kernels.  0 (default):
- *                 tiled for matrices of 8 Mi weights or more, row-major below; 1: always row-major;
- *                 2: tiled whenever the shape allows
+ *                 scales and biases; the row-major layout feeds the CUDA-core kernels, and with several
+ *                 rows (from 3 to 25, by size) the tensor-core kernel of several rows as well.
+ *                 0 (default): tiled for matrices of 8 Mi weights or more, row-major below; 1: always
+ *                 row-major; 2: tiled whenever the shape allows
  *   "gguf_layout" the same choice for goph_gguf_upload (Q4_K, Q5_K, Q6_K, Q8_0; in_dim a multiple of 256;
  *                 Q5_K and Q6_K take 1.06 / 1.13 bytes per weight in the tensor-core layout):
  *                 0 (default) tensor-core layout from 8 Mi weights, 1 always the streaming layout,
- *                 2 tensor-core layout whenever the shape allows.  "mlx_digits" and "mlx_splits"
- *                 apply to these products as well
+ *                 2 tensor-core layout whenever the shape allows.  "mlx_digits" (few rows) and
+ *                 "mlx_splits" apply to these products as well
  *   "fp8_layout"  the same choice for goph_fp8_upload (in_dim a multiple of 256, no NaN codes in the
- *                 weight): the tensor-core layout serves every batch size on the tensor cores (the
- *                 e4m3 bytes go to the MMA as they lie; f32 activations as six e4m3 pieces, exact,
- *                 bf16 activations as two); the row-major layout is served by the CUDA-core kernels
+ *                 weight).  In the tensor-core layout up to 4 f32 or 16 bf16 rows run with the e4m3
+ *                 bytes read by the MMA as they lie (f32 activations as six e4m3 pieces, exact, bf16
+ *                 activations as two); the row-major layout is served by the CUDA-core kernels.
+ *                 More rows of either layout run on the kernel of several rows, the bytes turned into
+ *                 f16 (exact), f32 activations as up to three f16 pieces, bf16 ones as one
  *   "fp8_convert" accepted, without effect (it chose between two kernels for larger bf16 batches)
  *   "mlx_digits"  signed base-128 digits each activation is written in on the tensor-core path,
  *                 relative to the largest magnitude of its 64-element group: 4 (default, 27 bits)
@@ -113,10 +116,12 @@ int goph_sm_count(int device);
  *   "mlx_chunks"  256-element chunks per pipeline stage of the tensor-core GEMV: 0 (default) two for
  *                 the nibble formats where tensor memory has the columns (up to 4 activation rows
  *                 for MLX 4-bit, 2 for Q4_K), 1 always one
- *   "mlx_splits"  CTAs that share the K range of one 128-row tile (0 = chosen by shape)
+ *   "mlx_splits"  CTAs that share the K range of one 128-row tile (0 = chosen by shape); with several
+ *                 rows of an item of the last wave, up to 8, where the device holds that many clusters
  *   "mlx_cluster" 1 (default): K splits that all run at once are launched as thread-block clusters and
  *                 add their partial sums through shared memory; 0: always through device scratch
- *                 and an atomic counter.  Same bits either way
+ *                 and an atomic counter, the same bits.  The kernel of several rows knows clusters
+ *                 only: with 0 it cuts no K range, and its sums are grouped differently
  *   "moe_fused"   1 (default): an MoE call of one token on row-major experts runs as ONE cooperative
  *                 launch (router, routing, gate|up, down and the weighted sum as phases between
  *                 grid-wide barriers), and with more tokens the router rows and the routing share a
