@@ -104,12 +104,12 @@ static bool valid_fp8(const goph_fp8_linear* w) {
 // rows: its scratch in the row-major layout.
 static bool qgemm_takes(const goph_fp8_linear* w, const void* x, bool x_bf16, int batch, cudaStream_t stream, QBufs** rows) {
   *rows = nullptr;
-  return w->in_dim % 16 == 0 && w->in_dim <= 65536 && (uintptr_t)x % 16 == 0 &&
+  return w->in_dim <= 65536 && (w->tiled || w->qmaps.ok) && (uintptr_t)x % 16 == 0 &&
          qgemm_wants(Q_FP8, w->tiled != nullptr, x_bf16, w->out_dim, w->in_dim, batch) && (w->tiled || (*rows = qgemm_scratch(w->device, stream)));
 }
 
 static int fp8_qgemm(const goph_fp8_linear* w, float* out, const void* x, bool x_bf16, int batch, QBufs* rows, cudaStream_t stream) {
-  const QWeight q{Q_FP8, w->tiled != nullptr, w->tiled ? w->tiled : w->weight, nullptr, w->scale, w->bias, w->device, w->out_dim, w->in_dim};
+  const QWeight q{Q_FP8, w->tiled != nullptr, w->tiled ? w->tiled : w->weight, nullptr, w->scale, w->bias, w->device, w->out_dim, w->in_dim, &w->qmaps};
   return qgemm(1, &q, &out, x, x_bf16, batch, rows, stream);
 }
 
@@ -192,6 +192,7 @@ GOPH_API int goph_fp8_upload(int device, const uint8_t* weight, uint64_t weight_
       h->bytes = (uint64_t)((out_dim + 127) / 128) * 128 * in_dim + (uint64_t)out_dim * 4 * (bias ? 2 : 1);
     }
   }
+  if (!h->tiled) qgemm_maps(Q_FP8, h->weight, nullptr, out_dim, in_dim, &h->qmaps);
   qgemm_weights(device, 1);
   *out = h;
   return bail(GOPH_OK);

@@ -361,12 +361,12 @@ static int q_format(int qtype) {
 // The several-row tensor-core product (qgemm.cu) reads both layouts.
 // rows: its scratch in the streaming layout.
 static bool qgemm_takes(const goph_gguf_matrix* m, const void* x, int batch, cudaStream_t stream, QBufs** rows) {
-  return m->in_dim <= 65536 && (uintptr_t)x % 16 == 0 && qgemm_wants(q_format(m->qtype), m->tiled != nullptr, false, m->out_dim, m->in_dim, batch) &&
+  return m->in_dim <= 65536 && (m->tiled || m->qmaps.ok) && (uintptr_t)x % 16 == 0 && qgemm_wants(q_format(m->qtype), m->tiled != nullptr, false, m->out_dim, m->in_dim, batch) &&
          (m->tiled || (*rows = qgemm_scratch(m->device, stream)));
 }
 
 static QWeight q_weight(const goph_gguf_matrix* m) {
-  return QWeight{q_format(m->qtype), m->tiled != nullptr, m->tiled ? m->tiled : m->data, m->d16, nullptr, nullptr, m->device, m->out_dim, m->in_dim};
+  return QWeight{q_format(m->qtype), m->tiled != nullptr, m->tiled ? m->tiled : m->data, m->d16, nullptr, nullptr, m->device, m->out_dim, m->in_dim, &m->qmaps};
 }
 
 static long gguf_row_bytes(int qtype, int in_dim) {
@@ -464,6 +464,8 @@ GOPH_API int goph_gguf_upload(int device, int qtype, const uint8_t* raw, uint64_
     cudaFree(h->d16);
     h->data = nullptr;
     h->d16 = nullptr;
+  } else {
+    qgemm_maps(q_format(qtype), h->data, h->d16, out_dim, in_dim, &h->qmaps);
   }
   qgemm_weights(device, 1);
   *out = h;

@@ -1,6 +1,7 @@
 // Internal declarations shared by the translation units of libgoph_b200.so.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -85,6 +86,12 @@ void gguf_work_status_clear(int device);
 // Largest dynamic shared-memory request the GEMV kernels make.
 constexpr int kSmemBudget = 200 * 1024;
 
+// Tensor maps of a row-major or streaming layout, as the several-row product reads it (qgemm.cuh).
+struct QMaps {
+  CUtensorMap map[3];
+  bool ok;
+};
+
 }  // namespace goph
 
 // MLX weight resident on one GPU, in one of two layouts:
@@ -106,6 +113,7 @@ struct goph_mlx_weight {
   void* sb;             // [out_dim][groups]
   uint8_t* tiled;       // tiled layout or nullptr
   uint64_t bytes;
+  goph::QMaps qmaps;    // row-major
 };
 
 // GGUF matrix resident on one GPU, re-laid out at upload (same byte count as the file):
@@ -121,6 +129,7 @@ struct goph_gguf_matrix {
   uint16_t* d16;   // Q8_0: f16 scales; Q6_K: two-bit highs, int8 scales and f16 d, one plane after another
   uint8_t* tiled;  // tensor-core layout (data and d16 are then null): one stage per 128 rows x 256 elements
   uint64_t bytes;
+  goph::QMaps qmaps;  // streaming layout
 };
 
 // FP8 E4M3 linear resident on one GPU: bytes as uploaded, per-row f32 scale (a per-tensor
@@ -137,6 +146,7 @@ struct goph_fp8_linear {
   float* scale;       // [out_dim]
   float* bias;        // [out_dim] or nullptr
   uint64_t bytes;
+  goph::QMaps qmaps;  // row-major
 };
 
 namespace goph {

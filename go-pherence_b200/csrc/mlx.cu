@@ -1150,11 +1150,11 @@ static int launch_generic(const goph_mlx_weight* w, float* out, const float* x, 
 
 // The several-row tensor-core product (qgemm.cu) reads both layouts of 64-element groups with bf16 tables.
 static bool qgemm_reads(const goph_mlx_weight* w, const void* x) {
-  return w->group_size == 64 && w->sb_bf16 && w->in_dim <= 65536 && (uintptr_t)x % 16 == 0;
+  return w->group_size == 64 && w->sb_bf16 && w->in_dim <= 65536 && (w->tiled || w->qmaps.ok) && (uintptr_t)x % 16 == 0;
 }
 
 static QWeight q_weight(const goph_mlx_weight* w) {
-  return QWeight{w->foldable ? Q_MLX4F : Q_MLX4, w->tiled != nullptr, w->tiled ? (const void*)w->tiled : w->qweight, w->sb, nullptr, nullptr, w->device, w->out_dim, w->in_dim};
+  return QWeight{w->foldable ? Q_MLX4F : Q_MLX4, w->tiled != nullptr, w->tiled ? (const void*)w->tiled : w->qweight, w->sb, nullptr, nullptr, w->device, w->out_dim, w->in_dim, &w->qmaps};
 }
 
 // Row-major weights sharing x on the CUDA cores.
@@ -1506,6 +1506,8 @@ static int mlx_upload_common(int device, const uint32_t* weight, const float* sc
     cudaFree(h->sb);
     h->qweight = nullptr;
     h->sb = nullptr;
+  } else if (gs == 64 && h->sb_bf16) {
+    qgemm_maps(Q_MLX4, h->qweight, h->sb, out_dim, in_dim, &h->qmaps);
   }
   qgemm_weights(device, 1);
   *out = h;

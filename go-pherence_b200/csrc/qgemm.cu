@@ -41,8 +41,8 @@
 // added in split order.
 //
 // A CTA, one per SM, 28 warps: W loader (tiled layouts: a bulk copy per 256 elements and tile, stored
-// contiguously; row-major and streaming layouts: 16-byte cp.async into the same image, rows and elements
-// past the matrix zero-filled), B loader (a slot per half chunk, all of its pieces), 2 MMA warps, 16
+// contiguously; row-major and streaming layouts: tiled TMA copies into the same image, rows and elements
+// past the matrix zero-filled, see load_rows), B loader (a slot per half chunk, all of its pieces), 2 MMA warps, 16
 // converter and 8 epilogue warps, half of them in either of two pipes (see the kernel).
 // Every wait is bounded (~2 s); a waiter that gives up records a code (800+) and the CTA winds down.
 //
@@ -103,7 +103,8 @@ constexpr int kMaxRows = 256;                       // activation rows of one la
 template <int F, bool TILED>
 struct QF {
   // packed nibbles in the row image (16-byte unit u of row r at r * 128 + ((u ^ (r & 7)) << 4)), else a
-  // byte per weight as [16-byte unit][row]
+  // byte per weight as [16-byte unit][row] (tiled) or as two row images of 128 elements
+  // (metadata beside them: kMeta bytes a row; Q6_K of the streaming layout: 16 of scales a row, then 4 with d a row)
   static constexpr bool kMLX = F == Q_MLX4 || F == Q_MLX4F;
   static constexpr bool kNibble = kMLX || F == Q_Q4K || (!TILED && (F == Q_Q5K || F == Q_Q6K));
   static constexpr int kHigh = kNibble && F == Q_Q5K ? 4096 : kNibble && F == Q_Q6K ? 8192 : 0;  // bits above the nibble, [16-byte unit][row]
@@ -124,6 +125,7 @@ struct QF {
 };
 
 struct QArgs {
+  CUtensorMap map[3];          // row-major and streaming layouts: what load_rows asks for
   const unsigned char* w;
   const void* aux;
   const unsigned char* xb;     // B tiles [row block][chunk * 2 + half][piece][K step 8][K half 2][n/8][8][16 B]
@@ -139,6 +141,7 @@ struct QArgs {
   int ntiles, nchunks, nblocks;
   int nfull, ntail, splits;    // whole items (a multiple of the grid), then at most one per cluster, cut along K
   int dcol;                    // columns an accumulator block takes: 16, 32, 64 or 128
+  int meta_tma;                // row-major MLX: the table's rows are whole 16-byte units
   int wslots, bslots, bslot, comb, pmax;  // depths of the rings, bytes of a B slot and of comb, pieces per half chunk in xb
 };
 
@@ -332,9 +335,6 @@ __device__ __forceinline__ uint32_t fma2h(uint32_t a, uint32_t b, uint32_t c) {
   asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
   return d;
 }
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
-}
 __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, int bytes) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
@@ -351,74 +351,81 @@ __device__ __forceinline__ void reg_inc() {
   asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
 }
 
-// The row-major and streaming layouts: one chunk of one tile into a slot, by a warp (lt).
+// Box of a two-dimensional tensor map at byte x of row y.
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map), "r"(x), "r"(y),
+               "r"(bar)
+               : "memory");
+}
+
+// The row-major and streaming layouts: one chunk of one tile into a slot, by a warp.  Weights come as boxes of 128 rows x
+// 128 bytes, whose 128-byte swizzle is the row image's (16-byte unit u of row r at r * 128 + ((u ^ (r & 7)) << 4)), what
+// stands between or beside them as boxes of 128 rows x 16 bytes; every x is a multiple of 16.  Only the f16 scales of
+// Q6_K and Q8_0 and an MLX table whose rows are no whole 16-byte units come by cp.async.  (One warp's cp.async of
+// everything, 44 to 72 a chunk with their addresses, set the pace: B200, us a call, Q5_K 489x9728 x93 39.6 -> 22.7, Q8_0
+// 11376x1504 x42 28.5 -> 23.3, Q6_K 1024x1792 x29 21.4 -> 11.2, FP8 2816x3136 x5 12.3 -> 9.4, MLX4 5722x1280 x99 16.1 -> 12.8.)
 template <int F>
-__device__ __forceinline__ void load_rows(const QArgs& a, uint32_t slot, int tile, int c, int lt) {
+__device__ __forceinline__ bool rows_cp(const QArgs& a) {  // whether a chunk has a part for cp.async
+  return F == Q_Q6K || F == Q_Q80 || (QF<F, false>::kMLX && !a.meta_tma);
+}
+template <int F>
+__device__ __forceinline__ void load_rows(const QArgs& a, uint32_t slot, uint32_t bar, int tile, int c, int lane) {
   typedef QF<F, false> T;
   const int row0 = tile * kTileRows;
   const uint32_t meta = slot + T::kWBytes;
+  if (lane == 0) {
+    constexpr uint32_t kBytes = T::kWBytes + (F == Q_Q80 || F == Q_FP8 || T::kMLX ? 0 : 2048);
+    mbar_expect_tx(bar, kBytes + (T::kMLX && a.meta_tma ? 2048 : 0));
+    if (T::kMLX) {
+      tma_load_2d(slot, &a.map[0], c * 128, row0, bar);
+      if (a.meta_tma) tma_load_2d(meta, &a.map[1], c * 16, row0, bar);
+    } else if (F == Q_Q4K || F == Q_Q5K) {  // super-blocks {16-byte header, nibbles, Q5_K: fifth bits}
+      const int x = c * (F == Q_Q4K ? 144 : 176);
+      tma_load_2d(slot, &a.map[0], x + 16, row0, bar);
+      tma_load_2d(meta, &a.map[1], x, row0, bar);
+      if (F == Q_Q5K) {
+        tma_load_2d(slot + T::kHighOff, &a.map[1], x + 144, row0, bar);
+        tma_load_2d(slot + T::kHighOff + 2048, &a.map[1], x + 160, row0, bar);
+      }
+    } else if (F == Q_Q6K) {  // planes: low nibbles, highs, scales
+      tma_load_2d(slot, &a.map[0], c * 128, row0, bar);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) tma_load_2d(slot + T::kHighOff + u * 2048, &a.map[1], c * 64 + 16 * u, row0, bar);
+      tma_load_2d(meta, &a.map[2], c * 16, row0, bar);
+    } else {  // a byte per weight
+      tma_load_2d(slot, &a.map[0], c * 256, row0, bar);
+      tma_load_2d(slot + 16384, &a.map[0], c * 256 + 128, row0, bar);
+    }
+  }
+  __syncwarp();
   if (T::kMLX) {
-    const int G = a.in_dim / 64;
-    for (int i = lt; i < 1024; i += 32) {
-      const int r = i >> 3, u = i & 7;
-      const bool ok = row0 + r < a.out_dim && c * 256 + u * 32 < a.in_dim;
-      cp_async16(slot + r * 128 + ((u ^ (r & 7)) << 4), ok ? a.w + (size_t)(row0 + r) * (a.in_dim / 2) + c * 128 + u * 16 : a.w, ok);
-    }
-    for (int i = lt; i < 512; i += 32) {
-      const int r = i >> 2, g = i & 3;
-      const bool ok = row0 + r < a.out_dim && c * 4 + g < G;
+    if (!a.meta_tma) {
+      const int G = a.in_dim / 64;
       const uint32_t* sb = static_cast<const uint32_t*>(a.aux);
-      cp_async4(meta + r * 16 + g * 4, ok ? sb + (size_t)(row0 + r) * G + c * 4 + g : sb, ok ? 4 : 0);
-    }
-  } else if (F == Q_Q4K) {
-    for (int i = lt; i < 128 * 9; i += 32) {
-      const int r = i / 9, u = i - r * 9;
-      const bool ok = row0 + r < a.out_dim;
-      const unsigned char* src = a.w + ((size_t)(ok ? row0 + r : 0) * a.nchunks + c) * 144;
-      if (u < 8) cp_async16(slot + r * 128 + ((u ^ (r & 7)) << 4), src + 16 + 16 * u, ok);
-      else cp_async16(meta + r * 16, src, ok);
-    }
-  } else if (F == Q_Q5K) {
-    for (int i = lt; i < 128 * 11; i += 32) {
-      const int r = i / 11, u = i - r * 11;
-      const bool ok = row0 + r < a.out_dim;
-      const unsigned char* src = a.w + ((size_t)(ok ? row0 + r : 0) * a.nchunks + c) * 176;
-      if (u < 8) cp_async16(slot + r * 128 + ((u ^ (r & 7)) << 4), src + 16 + 16 * u, ok);
-      else if (u == 8) cp_async16(meta + r * 16, src, ok);
-      else cp_async16(slot + T::kHighOff + (u - 9) * 2048 + r * 16, src + 144 + 16 * (u - 9), ok);
-    }
-  } else if (F == Q_Q6K) {
-    const size_t n = (size_t)a.out_dim * a.in_dim;
-    const unsigned char* hi = static_cast<const unsigned char*>(a.aux);
-    const unsigned char* sc = hi + n / 4;
-    const unsigned char* dd = sc + n / 16;
-    for (int i = lt; i < 128 * 14; i += 32) {
-      const int r = i / 14, u = i - r * 14;
-      const bool ok = row0 + r < a.out_dim;
-      const size_t row = ok ? row0 + r : 0;
-      if (u < 8) cp_async16(slot + r * 128 + ((u ^ (r & 7)) << 4), a.w + row * (a.in_dim / 2) + c * 128 + 16 * u, ok);
-      else if (u < 12) cp_async16(slot + T::kHighOff + (u - 8) * 2048 + r * 16, hi + row * (a.in_dim / 4) + c * 64 + 16 * (u - 8), ok);
-      else if (u == 12) cp_async16(meta + r * 32, sc + row * (a.in_dim / 16) + c * 16, ok);
-      else {  // the f16 d, in its aligned pair (the last one of an odd count stands alone)
-        const size_t h = row * a.nchunks + c, word = h >> 1, total = (size_t)a.out_dim * a.nchunks;
-        cp_async4(meta + r * 32 + 16, dd + word * 4, !ok ? 0 : 2 * word + 1 < total ? 4 : 2);
+      for (int i = lane; i < 512; i += 32) {
+        const int r = i >> 2, g = i & 3;
+        const bool ok = row0 + r < a.out_dim && c * 4 + g < G;
+        cp_async4(meta + r * 16 + g * 4, ok ? sb + (size_t)(row0 + r) * G + c * 4 + g : sb, ok ? 4 : 0);
       }
     }
-  } else {  // a byte per weight
-    for (int i = lt; i < 2048; i += 32) {
-      const int r = i >> 4, U = i & 15;
-      const bool ok = row0 + r < a.out_dim && c * 256 + U * 16 < a.in_dim;
-      cp_async16(slot + U * 2048 + r * 16, ok ? a.w + (size_t)(row0 + r) * a.in_dim + c * 256 + U * 16 : a.w, ok);
+  } else if (F == Q_Q6K) {  // the f16 d, in its aligned pair (the last one of an odd count stands alone)
+    const unsigned char* dd = static_cast<const unsigned char*>(a.aux) + (size_t)a.out_dim * a.in_dim / 4 + (size_t)a.out_dim * a.in_dim / 16;
+    const size_t total = (size_t)a.out_dim * a.nchunks;
+    for (int r = lane; r < 128; r += 32) {
+      const bool ok = row0 + r < a.out_dim;
+      const size_t word = ((size_t)(ok ? row0 + r : 0) * a.nchunks + c) >> 1;
+      cp_async4(meta + 2048 + r * 4, dd + word * 4, !ok ? 0 : 2 * word + 1 < total ? 4 : 2);
     }
-    if (F == Q_Q80) {  // the row's f16 scales from the aligned pair that holds the first one
-      const int nb = a.in_dim / 32;
-      const size_t total = (size_t)a.out_dim * nb;
-      for (int i = lt; i < 128 * 5; i += 32) {
-        const int r = i / 5, k = i - r * 5;
-        const size_t word = (((size_t)(row0 + r) * nb + c * 8) >> 1) + k;
-        const bool ok = row0 + r < a.out_dim && 2 * word < total;
-        const unsigned char* d = static_cast<const unsigned char*>(a.aux);
-        cp_async4(meta + r * 32 + k * 4, ok ? d + word * 4 : d, !ok ? 0 : 2 * word + 1 < total ? 4 : 2);
+  } else if (F == Q_Q80) {  // the row's f16 scales from the aligned pair that holds the first one
+    const int nb = a.in_dim / 32;
+    const size_t total = (size_t)a.out_dim * nb;
+    const unsigned char* d = static_cast<const unsigned char*>(a.aux);
+    for (int r = lane; r < 128; r += 32) {
+      const size_t word = ((size_t)(row0 + r) * nb + c * 8) >> 1;
+#pragma unroll
+      for (int k = 0; k < 5; ++k) {
+        const bool ok = row0 + r < a.out_dim && 2 * (word + k) < total;
+        cp_async4(meta + r * 32 + k * 4, ok ? d + (word + k) * 4 : d, !ok ? 0 : 2 * (word + k) + 1 < total ? 4 : 2);
       }
     }
   }
@@ -511,7 +518,8 @@ __device__ __forceinline__ void convert_unit(const unsigned char* st, int r, int
   } else {
     uint4 qv[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) qv[u] = *reinterpret_cast<const uint4*>(st + (8 * hh + 4 * kq + u) * 2048 + r * 16);
+    for (int u = 0; u < 4; ++u)
+      qv[u] = *reinterpret_cast<const uint4*>(TILED ? st + (8 * hh + 4 * kq + u) * 2048 + r * 16 : st + hh * 16384 + r * 128 + (((4 * kq + u) ^ (r & 7)) << 4));
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const uint32_t ws[4] = {qv[u].x, qv[u].y, qv[u].z, qv[u].w};
@@ -635,8 +643,8 @@ qg_kernel(const __grid_constant__ QArgs a) {
     if (tile >= a.ntiles) tile = a.ntiles - 1;  // the last group of an odd tile count repeats its tile (nothing of the copy is stored)
     const uint32_t slot = smem_u32(wring) + s * T::kSlot;
     if (!TILED) {
-      load_rows<F>(a, slot, tile, c, lane);
-      cp_async_arrive(wfull + 8 * s);
+      load_rows<F>(a, slot, wfull + 8 * s, tile, c, lane);
+      if (rows_cp<F>(a)) cp_async_arrive(wfull + 8 * s);
     } else if (lane == 0) {
       mbar_expect_tx(wfull + 8 * s, T::kSlot);
       bulk_load_1d(slot, a.w + ((size_t)tile * a.nchunks + c) * T::kSlot, T::kSlot, wfull + 8 * s);
@@ -647,7 +655,7 @@ qg_kernel(const __grid_constant__ QArgs a) {
   const int early = !wk.live ? 0 : TT == 2 || wk.c + 1 < wk.c1 ? 2 : 1;
   if (warp == kWarpW) {
     if (lane < SW) {
-      mbar_init(wfull + 8 * lane, TILED ? 1 : 32);
+      mbar_init(wfull + 8 * lane, !TILED && rows_cp<F>(a) ? 33 : 1);
       mbar_init(wempty + 8 * lane, TT == 2 ? 8 + (kLong ? 0 : 4) : 2 * (4 + (kLong ? 0 : 4)));
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -1006,10 +1014,10 @@ qg_kernel(const __grid_constant__ QArgs a) {
           for (int ci = 0; ci < chunks && ok; ++ci) {
             ok = __all_sync(0xffffffffu, mbar_wait(wfull + 8 * wc.s, wc.ph, a.status, 811));
             if (!ok) break;
-            const unsigned char* mrow = wring + wc.s * T::kSlot + T::kWBytes + r * T::kMeta;
+            const unsigned char* mrow = wring + wc.s * T::kSlot + T::kWBytes + r * (F == Q_Q6K && !TILED ? 16 : T::kMeta);
             uint4 mv = *reinterpret_cast<const uint4*>(mrow);
             uint32_t m4 = 0;  // Q6_K: d; streaming Q8_0: the fifth pair of scales
-            if (F == Q_Q6K || (F == Q_Q80 && !TILED)) m4 = *reinterpret_cast<const uint32_t*>(mrow + 16);
+            if (F == Q_Q6K || (F == Q_Q80 && !TILED)) m4 = *reinterpret_cast<const uint32_t*>(F == Q_Q6K && !TILED ? mrow + 2048 - r * 12 : mrow + 16);
             // the metadata is in registers (the reduction consumes it): the slot is free for the next load
             if (__reduce_or_sync(0xffffffffu, mv.x | mv.y | mv.z | mv.w | m4 | 1u) && lane == 0) mbar_arrive(wempty + 8 * wc.s);
             wc.next(SW);
@@ -1393,6 +1401,10 @@ int run_rows(const QWeight& w, float* out, const void* x, int batch, QBufs* bufs
     const int rows = batch - b0 < cap ? batch - b0 : cap;
     QArgs a;
     memset(&a, 0, sizeof a);
+    if (!TILED) {
+      memcpy(a.map, w.maps->map, sizeof a.map);
+      a.meta_tma = w.in_dim % kChunkK == 0;
+    }
     a.w = static_cast<const unsigned char*>(w.w);
     a.aux = w.aux;
     a.xb = bufs->xb;
@@ -1484,9 +1496,13 @@ int run_one(const QWeight& w, float* out, const void* x, bool x_bf16, int batch,
 // The lines lie where this kernel's time and the few-row kernels' met (B200, us a call: few-row / this).
 // Tiled layouts: the GEMV kernels take 8 rows a launch (Q4_K, Q5_K: 4), so a second launch, or the wider accumulator
 // blocks of 5 to 8 rows, decide.  Q6_K and Q8_0, with a block per 16 or 32 elements here too, gain later on large matrices.
-// Other layouts: the CUDA-core kernels' time grows with the rows and the weights, this one's hardly, but two launches
-// and the start cost it 8 to 10 us (Q5_K 12, Q6_K 20, converted from the streaming layout).  A weight of `weights` that
-// share x costs a launch of its own here, while the MLX streaming kernel takes all of them in one; out_dim is their sum.
+// Other layouts: the CUDA-core kernels' time grows with the rows and the weights (four rows a pass, eight in two), this
+// one's hardly, but two launches and the start cost it 7 to 9 us (Q6_K, a block per 16 elements, 9 to 19).  For Q8_0 and for
+// MLX rows of up to 2048 elements the lines are where the times meet.  Elsewhere this kernel's f32 sums in tensor memory are
+// a little coarser than those of the CUDA cores (against 64 bits, 4096 elements a row: Q4_K 4.6e-7 / 2.9e-7, Q5_K 4.5e-7 /
+// 2.9e-7, Q6_K 1.3e-7 / 1.0e-7, MLX4 1.4e-6 / 4.8e-7, FP8 1.5e-6 / 1.0e-7; but Q8_0 1.7e-7 / 4.4e-7, MLX4 at 2048 4.7e-7 /
+// 5.0e-7), and the lines stay above the rows from which it is the faster one.  A weight of `weights` that share x
+// costs a launch of its own here, while the MLX streaming kernel takes all of them in one; out_dim is their sum.
 bool qgemm_wants(int fmt, bool tiled, bool x_bf16, long out_dim, int in_dim, int batch, int weights) {
   if (x_bf16) return fmt != Q_FP8 || batch > 16;  // FP8 14336x4096: 16 rows 16.7 / 18.2, 24 rows 22.7 / 21.2
   const long size = out_dim * in_dim, Mi = 1l << 20;
@@ -1498,29 +1514,77 @@ bool qgemm_wants(int fmt, bool tiled, bool x_bf16, long out_dim, int in_dim, int
       default: return batch > (size <= 16 * Mi ? 4 : 8);        // Q6_K 4096x4096 4 rows 12.9 / 17.8, 5 rows 19.5 / 17.7; 14336x4096 8 rows 46.4 / 53.4,
     }                                                           // 9 rows 58.7 / 53.3; Q8_0 4096x4096 15.8 / 13.4 at 5, 14336x4096 28.5 / 33.6 at 8, 39.7 / 33.6 at 9
   }
-  if (weights > 1) {  // (MLX) by their mean size: 2048, 1024 and 1024 rows of 1024 at 16 rows 21.6 / 23.8, at 20 28.4 / 25.2;
-    const long mean = size / weights;  // 2048, 512, 512 of 2048 at 10 22.1 / 27.6, at 14 30.8 / 27.6; twice 2048x2048 at 8 18.4 / 21.3, at 9 22.0 / 21.3;
-    return batch > (mean < Mi ? 24 : mean < 2 * Mi ? 16 : mean < 3 * Mi ? 10 : mean < 5 * Mi ? 8 : 4);  // twice 2000x4096 at 4 18.3 / 23.7, at 5 30.3 / 23.8
+  if (weights > 1) {  // (MLX) by their mean size: 2048, 1024 and 1024 rows of 1024 at 16 rows 21.4 / 20.2, at 20 28.2 / 22.3;
+    const long mean = size / weights;  // 2048, 512, 512 of 2048 at 9 21.6 / 22.6, at 12 24.9 / 22.7; twice 2048x2048 at 8 18.1 / 16.4;
+    return batch > (mean < Mi ? 24 : mean < 2 * Mi ? 16 : mean < 3 * Mi ? 10 : mean < 5 * Mi ? 8 : 4);  // twice 2000x4096 at 4 18.1 / 19.1, at 5 30.2 / 19.1
   }
   // Above 8 Mi weights this layout is the exception (widths that no tile takes, NaN codes, the layout options).
   // in_dim above 8192: four rows of x no longer fit the CUDA-core kernels' shared memory, which then read the weights again.
   const bool small = size < 4 * Mi, long_rows = size >= 6 * Mi && in_dim >= 4096, wide_x = in_dim > 8192;
   switch (fmt) {
-    case Q_Q6K:  // 1024x1024 24 rows 16.0 / 20.5; 3072x1024 16 rows 19.5 / 20.3, 20 rows 25.0 / 20.9; 2048x2048 16 rows 23.4 / 34.4; 1536x4096 12 rows 29.7 / 34.5,
-                 // 14 rows 36.1 / 34.5; 14336x4096 24 rows 160 / 208; 4096x14336 8 rows 165 / 179, 9 rows 200 / 179
+    case Q_Q6K:  // 1024x1024 16 rows 10.7 / 9.3; 3072x1024 4 rows 5.6 / 9.6, 9 rows 12.7 / 9.6; 2048x2048 8 rows 11.7 / 13.8, 9 rows 15.3 / 13.8; 1536x4096
+                 // 4 rows 11.5 / 13.5, 5 rows 17.8 / 13.5; 28672x4096 8 rows 97 / 107, 9 rows 148 / 107; 8192x8192 4 rows 57 / 57
       return batch > (size < 2 * Mi ? 24 : wide_x && size >= 8 * Mi ? 8 : size > 16 * Mi ? 24 : long_rows ? 12 : 16);
-    case Q_Q5K:  // 512x2048 10 rows 11.7 / 12.8, 12 rows 13.1 / 12.8; 2048x2048 8 rows 13.0 / 16.5, 9 rows 17.1 / 16.5; 1536x4096 4 rows 12.9 / 18.5, 5 rows 20.3 / 18.6
+    case Q_Q5K:  // 512x2048 8 rows 8.1 / 8.3, 9 rows 11.0 / 8.3; 2048x2048 4 rows 7.4 / 9.3, 5 rows 12.7 / 9.3; 1536x4096 2 rows 8.6 / 9.7, 3 rows 12.6 / 9.7
       return batch > (size < 2 * Mi ? 10 : long_rows || size >= 8 * Mi ? 4 : 8);
-    case Q_Q4K: case Q_MLX4: case Q_MLX4F:  // MLX 1024x1024 8 rows 5.6 / 8.5, 9 rows 9.5 / 8.4; 2048x2048 4 rows 7.8 / 11.0, 5 rows 12.8 / 10.9; 1536x4096 2 rows 8.0 / 11.2,
-                                            // 3 rows 12.8 / 11.2; 8192x2112 2 rows 13.9 / 15.4, 3 rows 22.1 / 15.3; 28672x4160 4 rows 59.5 / 66.7, 5 rows 104 / 67
+    case Q_Q80:  // 1024x1024 9 rows 7.8 / 8.2, 10 rows 8.2 / 8.2; 512x2048 8 rows 7.8 / 8.9, 9 rows 10.6 / 8.9; 2048x2048 4 rows 6.5 / 10.7, 5 rows 11.0 / 10.7;
+                 // 1536x4096 10.8 / 11.5, 19.1 / 11.4; 1024x7168 12.2 / 14.8, 19.3 / 14.8; 512x14336 2 rows 15.2 / 20.8, 3 rows 28.0 / 20.7;
+                 // 4096x4160 13.7 / 18.4, 18.7 / 18.4; 8192x8256 39.7 / 40.2, 66.1 / 40.2; 28672x4160 4 rows 68.7 / 68.5, 5 rows 134 / 68.5
+      return batch > (size < 2 * Mi ? 8 : size < 8 * Mi && !wide_x ? 4 : 2);
+    case Q_Q4K: case Q_MLX4: case Q_MLX4F:
+      // MLX 1024x1024 8 rows 5.4 / 7.2, 9 rows 9.5 / 7.2; 3072x1024 4 rows 6.0 / 7.5, 5 rows 9.3 / 7.5; 7000x1024 8.5 / 8.9, 13.6 / 8.9; 28672x1088 2 rows
+      // 20.6 / 14.2
+      if (fmt != Q_Q4K && in_dim <= 2048) return batch > (size < 2 * Mi ? 8 : size < 12 * Mi ? 4 : 1);
+      // MLX 1536x4096 2 rows 7.7 / 9.1, 3 rows 12.6 / 9.1; 8192x2112 13.6 / 11.7, 22.0 / 11.7; Q4_K 1536x4096 7.7 / 9.4, 12.2 / 9.4
       return batch > (small ? 8 : (long_rows || (size >= 8 * Mi && in_dim > 1024)) && size <= 64 * Mi ? 2 : 4);
-    case Q_FP8:  // 1024x2048 8 rows 7.0 / 9.1, 9 rows 9.2 / 9.1; 7000x1024 4 rows 8.3 / 10.7, 5 rows 12.8 / 10.6; 4096x4160 4 rows 19.7 / 17.9; 28672x4160 4 rows 54.6 / 63.7;
-                 // 512x14336 2 rows 17.1 / 19.3, 3 rows 32.2 / 19.3; 8192x8256 2 rows 35.9 / 37.4, 3 rows 67.6 / 37.3
+    default:     // FP8 1024x1024 8 rows 5.3 / 7.0, 9 rows 7.1 / 7.0; 2048x2048 4 rows 5.7 / 8.2, 5 rows 9.4 / 8.1; 4096x4160 2 rows 11.4 / 10.1; 512x14336
+                 // 2 rows 12.7 / 13.4, 3 rows 22.7 / 13.4; 8192x8256 2 rows 36.2 / 15.8
       return batch > (small ? 8 : wide_x ? 2 : size >= 16 * Mi && size < 48 * Mi ? 3 : 4);
-    default:     // Q8_0 2048x2048 8 rows 11.5 / 14.1, 9 rows 15.0 / 14.1; 1536x4096 4 rows 11.0 / 14.4, 5 rows 19.2 / 14.4; 28672x1088 4 rows 23.2 / 34.5, 5 rows 42.7 / 34.6;
-                 // 8192x8256 2 rows 39.8 / 61.0, 3 rows 68.6 / 61.0; 512x14336 2 rows 15.3 / 27.4, 3 rows 27.8 / 27.4
-      return batch > (small ? 8 : wide_x ? 2 : long_rows || size >= 8 * Mi ? 4 : 8);
   }
+}
+
+// Tensor map of `rows` rows of `bytes` bytes, `pitch` apart: boxes of 128 rows and `box` bytes, zeros past the edges.
+static bool encode_map(CUtensorMap* map, const void* base, uint64_t bytes, uint64_t rows, uint64_t pitch, int box) {
+  typedef CUresult (*Encode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
+                             CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static const Encode encode = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &found) != cudaSuccess || found != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return reinterpret_cast<Encode>(f);
+  }();
+  if (!encode) return false;
+  const cuuint64_t dims[2] = {bytes, rows}, pitches[1] = {pitch};
+  const cuuint32_t boxes[2] = {(cuuint32_t)box, kTileRows}, steps[2] = {1, 1};
+  return encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, pitches, boxes, steps, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                box == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+void qgemm_maps(int fmt, const void* w, const void* aux, int out_dim, int in_dim, QMaps* maps) {
+  const uint64_t rows = out_dim, in = in_dim, chunks = in / 256, n = rows * in;
+  const unsigned char* hi = static_cast<const unsigned char*>(aux);
+  bool ok = true;
+  memset(maps, 0, sizeof *maps);
+  switch (fmt) {
+    case Q_MLX4: case Q_MLX4F:
+      ok = encode_map(&maps->map[0], w, in / 2, rows, in / 2, 128) && (in % 256 != 0 || encode_map(&maps->map[1], aux, in / 16, rows, in / 16, 16));
+      break;
+    case Q_Q4K: case Q_Q5K: {
+      const uint64_t row = chunks * (fmt == Q_Q4K ? 144 : 176);
+      ok = encode_map(&maps->map[0], w, row, rows, row, 128) && encode_map(&maps->map[1], w, row, rows, row, 16);
+      break;
+    }
+    case Q_Q6K:
+      ok = encode_map(&maps->map[0], w, in / 2, rows, in / 2, 128) && encode_map(&maps->map[1], hi, in / 4, rows, in / 4, 16) &&
+           encode_map(&maps->map[2], hi + n / 4, in / 16, rows, in / 16, 16);
+      break;
+    default:
+      ok = in % 16 == 0 && encode_map(&maps->map[0], w, in, rows, in, 128);
+  }
+  maps->ok = ok;
 }
 
 int qgemm(int n, const QWeight* w, float* const* out, const void* x, bool x_bf16, int batch, QBufs* rows, cudaStream_t stream) {

@@ -9,7 +9,7 @@ namespace goph {
 // Q_MLX4F: MLX 4-bit weights whose scales are zero or of magnitude 2^-27 to 7.875 (goph_mlx_weight::foldable)
 enum QFormat { Q_MLX4 = 0, Q_Q4K = 1, Q_Q5K = 2, Q_Q6K = 3, Q_Q80 = 4, Q_FP8 = 5, Q_MLX4F = 6 };
 
-// A weight matrix as the kernel sees it.  tiled: `w` is the format's tiled layout; else `w` and `aux`
+// A weight matrix as the kernel sees it.  maps: of the other layouts, made at upload.  tiled: `w` is the format's tiled layout; else `w` and `aux`
 // are the row-major / streaming layout's buffers (MLX: words and the bf16 {scale,bias} table; Q4_K,
 // Q5_K: blocks; Q6_K: low nibbles, and the highs, scales and d one plane after another; Q8_0: biased
 // bytes and f16 scales; FP8: bytes).
@@ -21,7 +21,12 @@ struct QWeight {
   const float* scale;  // FP8: [out_dim]
   const float* bias;   // FP8: [out_dim] or nullptr
   int device, out_dim, in_dim;
+  const QMaps* maps;
 };
+
+// The tensor maps of a weight in its row-major or streaming layout (w and aux as in QWeight).  maps->ok is false where there
+// are none (no such driver call, rows that are no whole 16-byte units): such a weight is not for this kernel.
+void qgemm_maps(int fmt, const void* w, const void* aux, int out_dim, int in_dim, QMaps* maps);
 
 // Whether `batch` activation rows of such a weight go to this kernel; the others are the business of the kernels
 // for few rows (integer tensor-core GEMV, CUDA-core streaming, FP8 pieces).  `weights` of one call that share x and could

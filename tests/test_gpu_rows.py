@@ -69,6 +69,31 @@ def test_several_rows(gpu, pkg, fmt, shapes, tiled):
     assert gpu.KernelStatus() == 0
 
 
+# Row-major and streaming layouts: matrices smaller than the boxes their tiles are copied in (128 rows x 128 bytes), an MLX
+# table of whole 16-byte rows and one of others, Q6_K's d and Q8_0's scales in odd counts.
+@pytest.mark.parametrize("fmt,shapes", [
+    ("mlx", ((1, 64), (127, 192), (3, 256), (130, 512))), ("mlx_wide", ((1, 64), (127, 192))), ("fp8", ((1, 16), (100, 144), (130, 272))),
+    ("q8_0", ((1, 32), (77, 160), (129, 96))), ("q4_k", ((1, 256), (127, 768))), ("q5_k", ((1, 256), (127, 768))), ("q6_k", ((1, 256), (3, 768), (127, 768)))])
+def test_tiles_smaller_than_a_box(gpu, pkg, fmt, shapes):
+    """Bound, against the sum of the terms' magnitudes (a matrix of one row has no largest output to go by): 3 * 768 / 16 additions
+    cut off at 2^-23, an affine format's terms twice the size of the products.  A lost element would be some 1 / 768."""
+    for out_dim, in_dim in shapes:
+        h, run, W, bias = make(gpu, pkg, fmt, False, out_dim, in_dim)
+        W = np.asarray(W, dtype=np.float64).reshape(out_dim, in_dim)
+        for rows in (25, 70):
+            x = pkg.synth.activations(("box", rows, in_dim), rows * in_dim, bf16=False).reshape(rows, in_dim)
+            xo, out = gpu.from_numpy(x.reshape(-1)), out_with_canary(gpu, rows * out_dim)
+            run(out, xo, rows)
+            gpu.Sync()
+            got, x = read_and_check_canary(out, rows * out_dim).reshape(rows, out_dim).astype(np.float64), x.astype(np.float64)
+            want, size = x @ W.T + (0 if bias is None else bias), np.abs(x) @ np.abs(W).T + (0 if bias is None else np.abs(bias))
+            ok = ~np.isnan(want)
+            assert np.array_equal(ok, ~np.isnan(got)) and np.all(np.abs(got - want)[ok] <= 144 * 2.0 ** -22 * size[ok])
+            xo.Free(); out.Free()
+        h.Free()
+    assert gpu.KernelStatus() == 0
+
+
 @pytest.mark.parametrize("in_dim", [32, 64, 1024, 1056, 3072, 4096, 5120, 8192])   # one to eight slices, ragged ones
 @pytest.mark.parametrize("out_dims", [(1,), (443,), (449,), (885, 3), (1185, 7, 1), (4097,)])  # rows per warp: one, two, four; several weights
 def test_row_gemv_has_the_looping_kernels_bits(gpu, pkg, in_dim, out_dims):
