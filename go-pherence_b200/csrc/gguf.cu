@@ -592,8 +592,9 @@ GOPH_API int goph_gguf_project_pair(float* out_a_dev, uint64_t out_a_len, float*
     return qgemm(2, q, outs, x_dev, false, batch, rows, (cudaStream_t)stream);
   }
   if (a->tiled && b->tiled && a->qtype == b->qtype && !rows_a) {  // here too
-    if (int rc = gguf_mma_launch(a, out_a_dev, x_dev, batch, options().mlx_digits, (cudaStream_t)stream, false)) return rc;
-    return gguf_mma_launch(b, out_b_dev, x_dev, batch, options().mlx_digits, (cudaStream_t)stream, true);
+    bool prepared = false;
+    if (int rc = gguf_mma_launch(a, out_a_dev, x_dev, batch, options().mlx_digits, (cudaStream_t)stream, &prepared)) return rc;
+    return gguf_mma_launch(b, out_b_dev, x_dev, batch, options().mlx_digits, (cudaStream_t)stream, &prepared);
   }
   if (int rc = goph_gguf_project(out_a_dev, out_a_len, x_dev, x_len, batch, a, stream)) return rc;
   return goph_gguf_project(out_b_dev, out_b_len, x_dev, x_len, batch, b, stream);

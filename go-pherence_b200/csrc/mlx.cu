@@ -1221,8 +1221,7 @@ static int mlx_products(int n, float* const* outs, const goph_mlx_weight* const*
       several[ns] = q_weight(ws[i]);
       several_out[ns++] = outs[i];
     } else if (ws[i]->tiled) {
-      if (int rc = mlx_mma_launch(ws[i], outs[i], x, batch, options().mlx_digits, stream, prepared)) return rc;
-      prepared = true;
+      if (int rc = mlx_mma_launch(ws[i], outs[i], x, batch, options().mlx_digits, stream, &prepared)) return rc;
     } else {
       rest[nr] = ws[i];
       rest_out[nr++] = outs[i];

@@ -1152,7 +1152,7 @@ static int cluster_room(int device, int size) {
 }
 
 template <int N, int DIGITS, int MB, int FMT, bool FUSED, int C>
-static int launch_impl(const TiledDesc& w, const MmaArgs& a0, cudaStream_t stream, bool prep, int stages, int splits) {
+static int launch_impl(const TiledDesc& w, const MmaArgs& a0, cudaStream_t stream, bool* prepared, int stages, int splits) {
   MmaArgs a = a0;
   a.dbg = g_mma_dbg;
   DeviceState& st = device_state(w.device);
@@ -1170,13 +1170,14 @@ static int launch_impl(const TiledDesc& w, const MmaArgs& a0, cudaStream_t strea
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (!FUSED && prep) {
+  if (!FUSED && !*prepared) {
     // activations -> digits, sums and scales, once per launch
     cfg.gridDim = dim3(a.batch * (a.in_dim / 64));
     cfg.blockDim = dim3(64);
     note_launch();
     GOPH_CUDA(cudaLaunchKernelEx(&cfg, mlx_prep_x_kernel<DIGITS, FMT != FMT_MLX4, !Fmt<FMT>::kConv, FMT == FMT_Q6K>, a.x,
                                  const_cast<unsigned char*>(a.xb), const_cast<float*>(a.xtab), a.batch, a.in_dim, N));
+    *prepared = true;
   }
   auto kern = mlx_mma_kernel<N, DIGITS, MB, FMT, FUSED, C>;
   GOPH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1237,7 +1238,7 @@ constexpr int stage_chunks() {
 }
 
 template <int N, int DIGITS, int MB, int FMT, int C>
-static int launch_with_chunks(const TiledDesc& w, const MmaArgs& a, cudaStream_t stream, bool prep) {
+static int launch_with_chunks(const TiledDesc& w, const MmaArgs& a, cudaStream_t stream, bool* prepared) {
   const int sms = device_state(w.device).sm_count;
   const int splits = choose_splits<MB>(a, sms, w.device);
   const int cmax = (a.nchunks + splits - 1) / splits;
@@ -1251,28 +1252,28 @@ static int launch_with_chunks(const TiledDesc& w, const MmaArgs& a, cudaStream_t
     size_t fixed = MmaSmem<N, FMT, true, C>::bytes(0, a.batch, a.in_dim, cmax);
     int stages = fixed < kMmaSmemBudget ? (int)((kMmaSmemBudget - fixed) / MmaSmem<N, FMT, true, C>::kStage) : 0;
     if (stages > kMaxStages) stages = kMaxStages;
-    if (stages >= 3) return launch_impl<N, DIGITS, MB, FMT, N == 8, C>(w, a, stream, prep, stages, splits);
+    if (stages >= 3) return launch_impl<N, DIGITS, MB, FMT, N == 8, C>(w, a, stream, prepared, stages, splits);
   }
   size_t fixed = MmaSmem<N, FMT, false, C>::bytes(0, a.batch, a.in_dim);
   int stages = fixed < kMmaSmemBudget ? (int)((kMmaSmemBudget - fixed) / MmaSmem<N, FMT, false, C>::kStage) : 0;
   if (stages > kMaxStages) stages = kMaxStages;
   if (stages < 3) {
-    if (C > 1) return launch_with_chunks<N, DIGITS, MB, FMT, 1>(w, a, stream, prep);
+    if (C > 1) return launch_with_chunks<N, DIGITS, MB, FMT, 1>(w, a, stream, prepared);
     return fail(GOPH_E_UNSUPPORTED, "tensor-core path: activations of %d x %d leave no room for the ring", a.batch, a.in_dim);
   }
-  return launch_impl<N, DIGITS, MB, FMT, false, C>(w, a, stream, prep, stages, splits);
+  return launch_impl<N, DIGITS, MB, FMT, false, C>(w, a, stream, prepared, stages, splits);
 }
 
 template <int N, int DIGITS, int MB, int FMT>
-static int launch_one(const TiledDesc& w, const MmaArgs& a, cudaStream_t stream, bool prep) {
+static int launch_one(const TiledDesc& w, const MmaArgs& a, cudaStream_t stream, bool* prepared) {
   constexpr int C = stage_chunks<N, FMT>();
-  if (C > 1 && options().mlx_chunks != 1) return launch_with_chunks<N, DIGITS, MB, FMT, C>(w, a, stream, prep);
-  return launch_with_chunks<N, DIGITS, MB, FMT, 1>(w, a, stream, prep);
+  if (C > 1 && options().mlx_chunks != 1) return launch_with_chunks<N, DIGITS, MB, FMT, C>(w, a, stream, prepared);
+  return launch_with_chunks<N, DIGITS, MB, FMT, 1>(w, a, stream, prepared);
 }
 
 template <int FMT>
 static int tiled_launch(const TiledDesc& w, float* out, const float* x, int batch, int digits, cudaStream_t stream,
-                        bool x_prepared) {
+                        bool* x_prepared) {
   MmaDeviceBufs* bufs = device_bufs(w.device);
   if (!bufs) return fail(GOPH_E_NOMEM, "cannot allocate the tensor-core path's device scratch");
   MmaArgs a;
@@ -1295,7 +1296,8 @@ static int tiled_launch(const TiledDesc& w, float* out, const float* x, int batc
     a.x = x + (size_t)b0 * w.in_dim;
     a.out = out + (size_t)b0 * w.out_dim;
     a.batch = nb;
-    const bool prep = !(x_prepared && batch <= cap);
+    bool own = false;  // (rows of a later launch of this call do not have the scratch's activations)
+    bool* prep = x_prepared && batch <= cap ? x_prepared : &own;
     int rc;
     if (digits == 3) {
       if (kQ4K && nb == 1) rc = launch_one<8, 3, 1, FMT>(w, a, stream, prep);
@@ -1317,7 +1319,7 @@ static int tiled_launch(const TiledDesc& w, float* out, const float* x, int batc
 }
 
 int mlx_mma_launch(const goph_mlx_weight* w, float* out, const float* x, int batch, int digits, cudaStream_t stream,
-                   bool x_prepared) {
+                   bool* x_prepared) {
   if (!w->tiled) return fail(GOPH_E_UNSUPPORTED, "weight is not in the tiled layout");
   TiledDesc d{w->tiled, w->device, w->out_dim, w->in_dim};
   return tiled_launch<FMT_MLX4>(d, out, x, batch, digits, stream, x_prepared);
@@ -1715,7 +1717,7 @@ int gguf_mma_make_tiled(goph_gguf_matrix* m) {
 }
 
 int gguf_mma_launch(const goph_gguf_matrix* m, float* out, const float* x, int batch, int digits, cudaStream_t stream,
-                    bool x_prepared) {
+                    bool* x_prepared) {
   if (!m->tiled) return fail(GOPH_E_UNSUPPORTED, "matrix is not in the tiled layout");
   TiledDesc d{m->tiled, m->device, m->out_dim, m->in_dim};
   if (m->qtype == GOPH_GGUF_Q4_K) return tiled_launch<FMT_Q4K>(d, out, x, batch, digits, stream, x_prepared);

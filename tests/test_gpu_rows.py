@@ -314,6 +314,28 @@ def test_weights_of_one_call_share_the_preparation(gpu, pkg):
         t.Free()
 
 
+# A call of several tiled weights and few rows: short K ranges prepare x inside the product's launch and leave nothing in the
+# scratch that a weight with longer ones, in the same call, could use.
+@pytest.mark.parametrize("rows", [1, 2, 3, 4])
+@pytest.mark.parametrize("order", [(0, 1), (1, 0), (0, 1, 0)])
+def test_few_rows_of_weights_that_prepare_x_in_different_places(gpu, pkg, rows, order):
+    shapes, in_dim = (1024, 19200), 4096
+    hs = [make(gpu, pkg, "mlx", True, o, in_dim)[0] for o in shapes]
+    junk = gpu.from_numpy(pkg.synth.activations("places junk", rows * in_dim, bf16=False))
+    x = gpu.from_numpy(pkg.synth.activations("places", rows * in_dim, bf16=False))
+    outs = [[out_with_canary(gpu, rows * shapes[i]) for i in order] for _ in range(2)]
+    for i, o in zip(order, outs[0]):
+        gpu.GemmMLX(o, x, hs[i], rows)
+    gpu.GemmMLX(outs[1][-1], junk, hs[1], rows) if order[-1] == 1 else gpu.GemmMLX(out_with_canary(gpu, rows * shapes[1]), junk, hs[1], rows)
+    gpu.GemmMLXMulti(outs[1], x, [hs[i] for i in order], rows)
+    gpu.Sync()
+    for i, a, b in zip(order, *outs):
+        n = rows * shapes[i]
+        assert np.array_equal(read_and_check_canary(a, n).view(np.uint32), read_and_check_canary(b, n).view(np.uint32))
+    for t in hs + [x, junk] + outs[0] + outs[1]:
+        t.Free()
+
+
 @pytest.mark.parametrize("tiled", [True, False])
 @pytest.mark.parametrize("fmt", ["fp8", "q8_0"])
 def test_every_bit_of_x_arrives(gpu, pkg, fmt, tiled):
