@@ -53,6 +53,7 @@
 #include <string.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "qgemm.cuh"
 #include "tc_common.cuh"
@@ -125,7 +126,6 @@ struct QF {
 };
 
 struct QArgs {
-  CUtensorMap map[3];          // row-major and streaming layouts: what load_rows asks for
   const unsigned char* w;
   const void* aux;
   const unsigned char* xb;     // B tiles [row block][chunk * 2 + half][piece][K step 8][K half 2][n/8][8][16 B]
@@ -141,9 +141,18 @@ struct QArgs {
   int ntiles, nchunks, nblocks;
   int nfull, ntail, splits;    // whole items (a multiple of the grid), then at most one per cluster, cut along K
   int dcol;                    // columns an accumulator block takes: 16, 32, 64 or 128
-  int meta_tma;                // row-major MLX: the table's rows are whole 16-byte units
   int wslots, bslots, bslot, comb, pmax;  // depths of the rings, bytes of a B slot and of comb, pieces per half chunk in xb
 };
+
+// The row-major and streaming layouts' second argument: what load_rows asks for.  (Inside QArgs it also cost the tiled
+// layouts' kernels registers: Q6_K 21504x1536 x256 129 us without, 136 with.)
+struct QRowMaps {
+  CUtensorMap map[3];
+  int meta_tma;  // MLX: the table's rows are whole 16-byte units
+};
+struct QNoMaps {};
+template <bool TILED>
+using QMapArgs = std::conditional_t<TILED, QNoMaps, QRowMaps>;
 
 struct Walk {
   int k, tail, id, group, nb, split, c, c1, rot;
@@ -365,41 +374,41 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
 // everything, 44 to 72 a chunk with their addresses, set the pace: B200, us a call, Q5_K 489x9728 x93 39.6 -> 22.7, Q8_0
 // 11376x1504 x42 28.5 -> 23.3, Q6_K 1024x1792 x29 21.4 -> 11.2, FP8 2816x3136 x5 12.3 -> 9.4, MLX4 5722x1280 x99 16.1 -> 12.8.)
 template <int F>
-__device__ __forceinline__ bool rows_cp(const QArgs& a) {  // whether a chunk has a part for cp.async
-  return F == Q_Q6K || F == Q_Q80 || (QF<F, false>::kMLX && !a.meta_tma);
+__device__ __forceinline__ bool rows_cp(const QRowMaps& t) {  // whether a chunk has a part for cp.async
+  return F == Q_Q6K || F == Q_Q80 || (QF<F, false>::kMLX && !t.meta_tma);
 }
 template <int F>
-__device__ __forceinline__ void load_rows(const QArgs& a, uint32_t slot, uint32_t bar, int tile, int c, int lane) {
+__device__ __forceinline__ void load_rows(const QArgs& a, const QRowMaps& t, uint32_t slot, uint32_t bar, int tile, int c, int lane) {
   typedef QF<F, false> T;
   const int row0 = tile * kTileRows;
   const uint32_t meta = slot + T::kWBytes;
   if (lane == 0) {
     constexpr uint32_t kBytes = T::kWBytes + (F == Q_Q80 || F == Q_FP8 || T::kMLX ? 0 : 2048);
-    mbar_expect_tx(bar, kBytes + (T::kMLX && a.meta_tma ? 2048 : 0));
+    mbar_expect_tx(bar, kBytes + (T::kMLX && t.meta_tma ? 2048 : 0));
     if (T::kMLX) {
-      tma_load_2d(slot, &a.map[0], c * 128, row0, bar);
-      if (a.meta_tma) tma_load_2d(meta, &a.map[1], c * 16, row0, bar);
+      tma_load_2d(slot, &t.map[0], c * 128, row0, bar);
+      if (t.meta_tma) tma_load_2d(meta, &t.map[1], c * 16, row0, bar);
     } else if (F == Q_Q4K || F == Q_Q5K) {  // super-blocks {16-byte header, nibbles, Q5_K: fifth bits}
       const int x = c * (F == Q_Q4K ? 144 : 176);
-      tma_load_2d(slot, &a.map[0], x + 16, row0, bar);
-      tma_load_2d(meta, &a.map[1], x, row0, bar);
+      tma_load_2d(slot, &t.map[0], x + 16, row0, bar);
+      tma_load_2d(meta, &t.map[1], x, row0, bar);
       if (F == Q_Q5K) {
-        tma_load_2d(slot + T::kHighOff, &a.map[1], x + 144, row0, bar);
-        tma_load_2d(slot + T::kHighOff + 2048, &a.map[1], x + 160, row0, bar);
+        tma_load_2d(slot + T::kHighOff, &t.map[1], x + 144, row0, bar);
+        tma_load_2d(slot + T::kHighOff + 2048, &t.map[1], x + 160, row0, bar);
       }
     } else if (F == Q_Q6K) {  // planes: low nibbles, highs, scales
-      tma_load_2d(slot, &a.map[0], c * 128, row0, bar);
+      tma_load_2d(slot, &t.map[0], c * 128, row0, bar);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) tma_load_2d(slot + T::kHighOff + u * 2048, &a.map[1], c * 64 + 16 * u, row0, bar);
-      tma_load_2d(meta, &a.map[2], c * 16, row0, bar);
+      for (int u = 0; u < 4; ++u) tma_load_2d(slot + T::kHighOff + u * 2048, &t.map[1], c * 64 + 16 * u, row0, bar);
+      tma_load_2d(meta, &t.map[2], c * 16, row0, bar);
     } else {  // a byte per weight
-      tma_load_2d(slot, &a.map[0], c * 256, row0, bar);
-      tma_load_2d(slot + 16384, &a.map[0], c * 256 + 128, row0, bar);
+      tma_load_2d(slot, &t.map[0], c * 256, row0, bar);
+      tma_load_2d(slot + 16384, &t.map[0], c * 256 + 128, row0, bar);
     }
   }
   __syncwarp();
   if (T::kMLX) {
-    if (!a.meta_tma) {
+    if (!t.meta_tma) {
       const int G = a.in_dim / 64;
       const uint32_t* sb = static_cast<const uint32_t*>(a.aux);
       for (int i = lane; i < 512; i += 32) {
@@ -602,7 +611,7 @@ __device__ __forceinline__ void umma_f16_ss(uint32_t d_tmem, uint64_t a_desc, ui
 // once still costs it over a hundred cycles, and an MMA forty.
 template <int F, bool TILED, int TT, int NB>
 __global__ void __launch_bounds__(kThreads, 1)
-qg_kernel(const __grid_constant__ QArgs a) {
+qg_kernel(const __grid_constant__ QArgs a, const __grid_constant__ QMapArgs<TILED> maps) {
   typedef QF<F, TILED> T;
   static_assert(NB == 64 || (NB == 128 && F == Q_FP8 && TT == 2), "wide blocks only where a block is read once per item");
   constexpr bool kLong = T::kLong, kChunk = T::kChunk;
@@ -642,9 +651,9 @@ qg_kernel(const __grid_constant__ QArgs a) {
     int tile = wk.group * TT + t;
     if (tile >= a.ntiles) tile = a.ntiles - 1;  // the last group of an odd tile count repeats its tile (nothing of the copy is stored)
     const uint32_t slot = smem_u32(wring) + s * T::kSlot;
-    if (!TILED) {
-      load_rows<F>(a, slot, wfull + 8 * s, tile, c, lane);
-      if (rows_cp<F>(a)) cp_async_arrive(wfull + 8 * s);
+    if constexpr (!TILED) {
+      load_rows<F>(a, maps, slot, wfull + 8 * s, tile, c, lane);
+      if (rows_cp<F>(maps)) cp_async_arrive(wfull + 8 * s);
     } else if (lane == 0) {
       mbar_expect_tx(wfull + 8 * s, T::kSlot);
       bulk_load_1d(slot, a.w + ((size_t)tile * a.nchunks + c) * T::kSlot, T::kSlot, wfull + 8 * s);
@@ -655,7 +664,9 @@ qg_kernel(const __grid_constant__ QArgs a) {
   const int early = !wk.live ? 0 : TT == 2 || wk.c + 1 < wk.c1 ? 2 : 1;
   if (warp == kWarpW) {
     if (lane < SW) {
-      mbar_init(wfull + 8 * lane, !TILED && rows_cp<F>(a) ? 33 : 1);
+      int arrivals = 1;
+      if constexpr (!TILED) arrivals += rows_cp<F>(maps) ? 32 : 0;
+      mbar_init(wfull + 8 * lane, arrivals);
       mbar_init(wempty + 8 * lane, TT == 2 ? 8 + (kLong ? 0 : 4) : 2 * (4 + (kLong ? 0 : 4)));
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -1328,7 +1339,7 @@ bool choose_plan(int device, int ntiles, int nchunks, int nblocks, int n, int pi
 }
 
 template <int F, bool TILED, int TT, int NB>
-int launch_product(QArgs& a, const Plan& p, int n, int device, cudaStream_t stream) {
+int launch_product(QArgs& a, const QMapArgs<TILED>& maps, const Plan& p, int n, int device, cudaStream_t stream) {
   typedef QF<F, TILED> T;
   // B slots hold every piece of half a chunk and the affine term's sums: two at least, more where they are
   // small; the weight ring gets the rest
@@ -1369,7 +1380,7 @@ int launch_product(QArgs& a, const Plan& p, int n, int device, cudaStream_t stre
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = smem;
   note_launch();
-  GOPH_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
+  GOPH_CUDA(cudaLaunchKernelEx(&cfg, kern, a, maps));
   return GOPH_OK;
 }
 
@@ -1401,9 +1412,10 @@ int run_rows(const QWeight& w, float* out, const void* x, int batch, QBufs* bufs
     const int rows = batch - b0 < cap ? batch - b0 : cap;
     QArgs a;
     memset(&a, 0, sizeof a);
-    if (!TILED) {
-      memcpy(a.map, w.maps->map, sizeof a.map);
-      a.meta_tma = w.in_dim % kChunkK == 0;
+    QMapArgs<TILED> maps;
+    if constexpr (!TILED) {
+      memcpy(maps.map, w.maps->map, sizeof maps.map);
+      maps.meta_tma = w.in_dim % kChunkK == 0;
     }
     a.w = static_cast<const unsigned char*>(w.w);
     a.aux = w.aux;
@@ -1456,10 +1468,10 @@ int run_rows(const QWeight& w, float* out, const void* x, int batch, QBufs* bufs
     }
     int rc;
     if constexpr (F == Q_FP8 && TILED && XBF16) {
-      if (NB == 128) rc = launch_product<F, TILED, 2, 128>(a, p, n, w.device, stream);
-      else rc = p.TT == 2 ? launch_product<F, TILED, 2, 64>(a, p, n, w.device, stream) : launch_product<F, TILED, 1, 64>(a, p, n, w.device, stream);
+      if (NB == 128) rc = launch_product<F, TILED, 2, 128>(a, maps, p, n, w.device, stream);
+      else rc = p.TT == 2 ? launch_product<F, TILED, 2, 64>(a, maps, p, n, w.device, stream) : launch_product<F, TILED, 1, 64>(a, maps, p, n, w.device, stream);
     } else {
-      rc = p.TT == 2 ? launch_product<F, TILED, 2, 64>(a, p, n, w.device, stream) : launch_product<F, TILED, 1, 64>(a, p, n, w.device, stream);
+      rc = p.TT == 2 ? launch_product<F, TILED, 2, 64>(a, maps, p, n, w.device, stream) : launch_product<F, TILED, 1, 64>(a, maps, p, n, w.device, stream);
     }
     if (rc) return rc;
     b0 += rows;
