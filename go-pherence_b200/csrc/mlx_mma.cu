@@ -241,136 +241,134 @@ struct StageWalkT {
 };
 
 // ---- activation preparation -----------------------------------------------------------------
-// One block of 64 threads per (activation row, 64-element group): group sum, power-of-two scale,
-// and the base-128 digits of every element written where the tensor core expects them:
-// chunk (256 K) -> K-step (32) -> half (16 bytes) -> 8-row core matrix -> row -> byte.
-// G32: sums and scales per 32 elements (one warp each) instead of per 64.  NATURAL: the B bytes of
-// a K step in element order (for A operands that lie in memory in element order) instead of the
-// order the nibble converters produce.
-template <int DIGITS, bool G32 = false, bool NATURAL = false, bool PAIRH = false>
-__global__ void __launch_bounds__(64)
-mlx_prep_x_kernel(const float* __restrict__ x, unsigned char* __restrict__ xb, float* __restrict__ xtab, int batch,
-                  int in_dim, int N) {
+// A warp turns the 256 elements of one chunk of activation row m, eight consecutive ones per lane (SPLIT 4: a block of
+// four warps, four lanes to the same eight elements, each of which writes one digit), into group sums, power-of-two scales and the base-128 digits of every element, written where the tensor core expects them:
+// chunk (256 K) -> K-step (32) -> half (16 bytes) -> 8-row core matrix -> row -> byte.  The lane's eight digits of a place
+// are eight consecutive bytes of one B row.  The digits come from one sum: q + 64 (1 + 128 + 128^2) has d_j + 64 in
+// its j-th seven bits (the top digit has what is left), and a byte pattern d + 64 of seven bits becomes the signed byte.
+// sums, scales: the row's tables at the chunk.  tile: the chunk's B tile of N rows.
+// G32: sums and scales per 32 elements instead of per 64.  NATURAL: the B bytes of a K step in element order (for A operands
+// that lie in memory in element order) instead of the order the nibble converters produce (of a packed word: 0 2 4 6, 1 3 5 7).
+// (An element per thread, ten shuffles and four byte stores each, took four times the instructions: the preparation of
+// 4096 elements by the product's own CTAs cost more than a launch in front, see launch_with_chunks.)
+template <int DIGITS, bool G32, bool NATURAL, bool PAIRH, int SPLIT = 1>
+__device__ __forceinline__ void prep_chunk(const float (&v)[8], int lane, unsigned char* tile, int N, int m, float* sums, float* scales) {
   constexpr int QBITS = DIGITS == 4 ? 26 : 19;  // |q| <= 2^QBITS keeps the top digit within a signed byte
-  constexpr bool PAIRED = G32 && !NATURAL;      // Q4_K: see Fmt::kPaired
-  const int groups = in_dim / 64;
-  const int m = blockIdx.x / groups, g = blockIdx.x - m * groups;
-  const int t = threadIdx.x;
-  pdl_launch_dependents();
-  pdl_wait();  // x may be the output of the kernel in front
-  const float v = x[(size_t)m * in_dim + g * 64 + t];
-  float s = v, mx = fabsf(v);
+  constexpr bool PAIRED = G32 && !NATURAL;      // Q4_K: see Fmt::kHalves
+  constexpr int kLanes = G32 ? 4 : 8;           // of a group
+  float s = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+  float mx = fmaxf(fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))),
+                   fmaxf(fmaxf(fabsf(v[4]), fabsf(v[5])), fmaxf(fabsf(v[6]), fabsf(v[7]))));
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
+  for (int o = SPLIT; o < kLanes * SPLIT; o <<= 1) {
     s += __shfl_xor_sync(0xffffffffu, s, o);
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  }
-  if (!G32) {
-    __shared__ float sh[4];
-    if ((t & 31) == 0) {
-      sh[t >> 5] = s;
-      sh[2 + (t >> 5)] = mx;
-    }
-    __syncthreads();
-    s = sh[0] + sh[1];
-    mx = fmaxf(sh[2], sh[3]);
   }
   int e = (int)((__float_as_uint(mx) >> 23) & 0xFF);  // mx < 2^(e-126)
   if (e < QBITS + 2) e = QBITS + 2;
   if (e > 254) e = 254;  // inf/nan inputs: results are undefined, not a hang
-  if (G32) {
-    if ((t & 31) == 0) {
-      const int g32 = 2 * g + (t >> 5), n32 = 2 * groups;
-      xtab[m * n32 + g32] = s;
-      xtab[(batch + m) * n32 + g32] = __uint_as_float((uint32_t)(e - 126 - QBITS + 127) << 23);
-    }
-  } else if (t == 0) {
-    xtab[m * groups + g] = s;
-    xtab[(batch + m) * groups + g] = __uint_as_float((uint32_t)(e - 126 - QBITS + 127) << 23);  // 2^(E-QBITS)
+  const int sub = lane % SPLIT;
+  lane /= SPLIT;
+  if (sub == 0 && lane % kLanes == 0) {
+    sums[lane / kLanes] = s;
+    scales[lane / kLanes] = __uint_as_float((uint32_t)(e - 126 - QBITS + 127) << 23);  // 2^(E-QBITS)
   }
   const float fi = __uint_as_float((uint32_t)(QBITS - (e - 126) + 127) << 23);
-  int q = __float2int_rn(v * fi);
-  // position of element k inside its chunk's B tile
-  const int k = (g & 3) * 64 + t;          // element within the 256-element chunk
-  const int step = k >> 5, w = (k & 31) >> 3, j = k & 7;
-  const int pos = NATURAL ? (k & 31) : 8 * w + 4 * (j & 1) + (j >> 1);  // byte along K inside the step (order of the A bytes)
-  const size_t base = (size_t)(g >> 2) * (N * 256) + step * (N * 32) + (pos >> 4) * ((N / 8) * 128) + (pos & 15);
-  const int db = N / 2;
+  int q[8];
 #pragma unroll
-  for (int d = 0; d < DIGITS; ++d) {
-    int dig = d == DIGITS - 1 ? q : ((q + 64) & 127) - 64;
-    q = (q - dig) >> 7;
+  for (int i = 0; i < 8; ++i) q[i] = __float2int_rn(v[i] * fi) + (DIGITS == 4 ? 64 * (1 + 128 + 16384) : 64 * (1 + 128));
+  auto digit = [&](int d) {
+    uint32_t p[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      auto at = [&](int i) { return (uint32_t)(q[NATURAL ? 4 * h + i : 2 * i + h] >> (7 * d)); };
+      p[h] = __byte_perm(__byte_perm(at(0), at(1), 0x0040), __byte_perm(at(2), at(3), 0x0040), 0x5410);
+      if (d < DIGITS - 1) {
+        p[h] = (p[h] & 0x7F7F7F7Fu) ^ 0x40404040u;
+        p[h] |= (p[h] & 0x40404040u) << 1;
+      }
+    }
+    return make_uint2(p[0], p[1]);
+  };
+  const int step = lane >> 2, w = lane & 3;  // the lane's eight positions are 8 w .. 8 w + 7 of the K step
+  unsigned char* dst = tile + step * (N * 32) + (w >> 1) * ((N / 8) * 128) + 8 * (w & 1);
+  const bool second = PAIRH ? w >= 2 : (step & 1) != 0;  // halves: Q6_K by the half of the step, Q4_K by the step
+  auto put = [&](int d, uint2 t) {
     int n = m * DIGITS + d;
     if (PAIRED || PAIRH) {  // the other scale group's half of the rows holds zeros at this K position
-      const bool second = PAIRH ? (pos & 16) != 0 : (step & 1) != 0;  // Q6_K: by the half of the step; Q4_K: by the step
-      const int other = n + (second ? 0 : db);
-      n += second ? db : 0;
-      xb[base + (other >> 3) * 128 + (other & 7) * 16] = 0;
+      const int other = n + (second ? 0 : N / 2);
+      n += second ? N / 2 : 0;
+      *reinterpret_cast<uint2*>(dst + (other >> 3) * 128 + (other & 7) * 16) = make_uint2(0, 0);
     }
-    xb[base + (n >> 3) * 128 + (n & 7) * 16] = (unsigned char)(dig & 0xFF);
+    *reinterpret_cast<uint2*>(dst + (n >> 3) * 128 + (n & 7) * 16) = t;
+  };
+  if (SPLIT == 4) {
+    if (sub < DIGITS) put(sub, digit(sub));
+    return;
+  }
+  uint2 dig[DIGITS];
+#pragma unroll
+  for (int d = 0; d < DIGITS; ++d) dig[d] = digit(d);
+#pragma unroll
+  for (int i = 0; i < DIGITS; ++i) {
+    if (DIGITS == 4) {  // (lanes take turns at the places: their addresses are multiples of 128 bytes apart)
+      const int d = (i + step) & 3;
+      put(d, d == 0 ? dig[0] : d == 1 ? dig[1] : d == 2 ? dig[2] : dig[DIGITS - 1]);
+    } else {
+      put(i, dig[i]);
+    }
+  }
+}
+__device__ __forceinline__ void load_eight(const float* p, float (&v)[8]) {
+  if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+    const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+  } else {  // callers may hand in x at any float
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = p[i];
   }
 }
 
-// The same preparation done by a CTA of the product kernel for itself (all warps, before the
-// pipeline starts): digits into the resident B tiles in shared memory, sums and scales into the
-// tables the epilogue reads.  A warp takes one 64-element group at a time, lane l the elements l
-// and l + 32; the arithmetic and its order are those of mlx_prep_x_kernel.
+// The launch in front of the product: a block per (activation row, chunk).  (A warp per chunk, a fourth of the threads:
+// 0.3 to 0.5 us slower.)
+template <int DIGITS, bool G32 = false, bool NATURAL = false, bool PAIRH = false>
+__global__ void __launch_bounds__(128)
+mlx_prep_x_kernel(const float* __restrict__ x, unsigned char* __restrict__ xb, float* __restrict__ xtab, int batch,
+                  int in_dim, int N) {
+  constexpr int kPer = G32 ? 8 : 4;  // table entries of a chunk
+  const int nchunks = in_dim / kChunkK, ntab = nchunks * kPer;
+  const int m = blockIdx.x / nchunks, c = blockIdx.x - m * nchunks, lane = threadIdx.x;
+  pdl_launch_dependents();
+  pdl_wait();  // x may be the output of the kernel in front
+  float v[8];
+  load_eight(x + (size_t)m * in_dim + c * kChunkK + lane / 4 * 8, v);
+  prep_chunk<DIGITS, G32, NATURAL, PAIRH, 4>(v, lane, xb + (size_t)c * (N * 256), N, m, xtab + m * ntab + c * kPer, xtab + (batch + m) * ntab + c * kPer);
+}
+
+// The same done by a CTA of the product kernel for itself (all warps but the producer's, before they take up their roles):
+// digits into the resident B tiles in shared memory, sums and scales into the tables the epilogue reads.
 template <int DIGITS, bool G32, bool NATURAL, int N, bool PAIRH = false>
 __device__ __forceinline__ void prep_x_in_cta(const float* __restrict__ x, int batch, int in_dim, unsigned char* bres,
                                               float* xsum, float* xfs, int warp, int lane, int nwarps, int cbegin, int cend) {
-  constexpr int QBITS = DIGITS == 4 ? 26 : 19;
-  constexpr bool PAIRED = G32 && !NATURAL;
-  constexpr int db = N / 2;
-  const int groups = in_dim / 64;
-  const int ntab = G32 ? 2 * groups : groups;
-  const int gbegin = 4 * cbegin, gcount = 4 * (cend - cbegin);  // the 64-element groups of chunks [cbegin, cend)
-  for (int gi = warp; gi < batch * gcount; gi += nwarps) {
-    const int m = gi / gcount, g = gbegin + (gi - m * gcount);
-    const float* xp = x + (size_t)m * in_dim + g * 64;
-    float v[2] = {xp[lane], xp[32 + lane]};
-    float s[2] = {v[0], v[1]}, mx[2] = {fabsf(v[0]), fabsf(v[1])};
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        s[h] += __shfl_xor_sync(0xffffffffu, s[h], o);
-        mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], o));
-      }
+  constexpr int kPer = G32 ? 8 : 4;
+  const int ntab = in_dim / kChunkK * kPer, n = cend - cbegin;
+  if (batch * n * 4 <= nwarps) {  // short ranges: four warps to a chunk
+    const int i = warp >> 2, l = (warp & 3) * 32 + lane;
+    if (i < batch * n) {
+      const int m = i / n, c = cbegin + (i - m * n), ti = m * ntab + c * kPer;
+      float v[8];
+      load_eight(x + (size_t)m * in_dim + c * kChunkK + l / 4 * 8, v);
+      prep_chunk<DIGITS, G32, NATURAL, PAIRH, 4>(v, l, bres + (size_t)(c - cbegin) * (N * 256), N, m, xsum + ti, xfs + ti);
     }
-    if (!G32) {
-      s[0] = s[1] = s[0] + s[1];
-      mx[0] = mx[1] = fmaxf(mx[0], mx[1]);
-    }
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      int e = (int)((__float_as_uint(mx[h]) >> 23) & 0xFF);
-      if (e < QBITS + 2) e = QBITS + 2;
-      if (e > 254) e = 254;
-      if (lane == 0 && (G32 || h == 0)) {
-        const int ti = m * ntab + (G32 ? 2 * g + h : g);
-        xsum[ti] = s[h];
-        xfs[ti] = __uint_as_float((uint32_t)(e - 126 - QBITS + 127) << 23);
-      }
-      const float fi = __uint_as_float((uint32_t)(QBITS - (e - 126) + 127) << 23);
-      int q = __float2int_rn(v[h] * fi);
-      const int k = (g & 3) * 64 + h * 32 + lane;  // element within the 256-element chunk
-      const int step = k >> 5, w = (k & 31) >> 3, j = k & 7;
-      const int pos = NATURAL ? (k & 31) : 8 * w + 4 * (j & 1) + (j >> 1);
-      unsigned char* base = bres + (size_t)((g >> 2) - cbegin) * (N * 256) + step * (N * 32) + (pos >> 4) * ((N / 8) * 128) + (pos & 15);
-#pragma unroll
-      for (int d = 0; d < DIGITS; ++d) {
-        int dig = d == DIGITS - 1 ? q : ((q + 64) & 127) - 64;
-        q = (q - dig) >> 7;
-        int n = m * DIGITS + d;
-        if (PAIRED || PAIRH) {
-          const bool second = PAIRH ? (pos & 16) != 0 : (step & 1) != 0;
-          const int other = n + (second ? 0 : db);
-          n += second ? db : 0;
-          base[(other >> 3) * 128 + (other & 7) * 16] = 0;
-        }
-        base[(n >> 3) * 128 + (n & 7) * 16] = (unsigned char)(dig & 0xFF);
-      }
-    }
+    return;
+  }
+#pragma unroll 1
+  for (int i = warp; i < batch * n; i += nwarps) {
+    const int m = i / n, c = cbegin + (i - m * n), ti = m * ntab + c * kPer;
+    float v[8];
+    load_eight(x + (size_t)m * in_dim + c * kChunkK + lane * 8, v);
+    prep_chunk<DIGITS, G32, NATURAL, PAIRH>(v, lane, bres + (size_t)(c - cbegin) * (N * 256), N, m, xsum + ti, xfs + ti);
   }
 }
 
@@ -480,23 +478,17 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
   TP(const bool tr = blockIdx.x == gridDim.x / 2 && (!(a.dbg & 8) || a.gmats == 2); if (tr && tid == 0) { g_mma_trace[7][0] = clock64(); g_mma_trace[7][3] = t_entry; })
   const int cbase = sw.live(a) ? sw.c : 0;  // first chunk of this CTA's K range
 
-  if (FUSED) {
-    // The weights do not depend on the kernel in front: the producer fills the ring, then every
-    // warp helps to turn the activations into digits, sums and scales.
-    if (warp == kWarpTMA && lane == 0) {
-      StageWalk sw0 = sw;
-      for (int i = 0; i < S && i < kFirstStages && sw0.live(a); ++i, sw0.next(a)) {
-        mbar_expect_tx(full0 + 8 * i, sw0.nc() * kStageBytes);
-        bulk_load_1d(smem_u32(ring + (size_t)i * kStage), wsrc(sw0), sw0.nc() * kStageBytes, full0 + 8 * i);
-      }
-    }
+  if (FUSED && warp != kWarpTMA) {
+    // The producer is off to its ring (the weights do not depend on the kernel in front); the other warps turn the
+    // activations into digits, sums and scales.
+    static_assert(kWarpMMA == kWarpTMA + 1 && kWarpMMA == kThreads / 32 - 1, "the MMA warp is the last, behind the producer");
     pdl_wait();
     // every item of this CTA covers the same K range (the grid is a multiple of the K splits)
     if (sw.live(a))
-      prep_x_in_cta<DIGITS, FMT != FMT_MLX4, !F::kConv, N, FMT == FMT_Q6K>(a.x, a.batch, a.in_dim, bres, xsum, xfs, warp, lane, kThreads / 32,
-                                                                 sw.c, sw.c1);
+      prep_x_in_cta<DIGITS, FMT != FMT_MLX4, !F::kConv, N, FMT == FMT_Q6K>(a.x, a.batch, a.in_dim, bres, xsum, xfs, warp == kWarpMMA ? kWarpTMA : warp, lane,
+                                                                           kThreads / 32 - 1, sw.c, sw.c1);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the MMA reads the digits through the async proxy
-    __syncthreads();
+    asm volatile("bar.sync 2, %0;" ::"n"(kThreads - 32) : "memory");
   }
 
   if (warp == kWarpTMA) {
@@ -505,15 +497,15 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
       // The weights do not depend on the kernel in front: fill the ring with them first, then
       // wait for the activation digits and add the B tiles of those stages.
       int i = 0;
+      StageWalk sw0 = sw;
+      for (; i < S && i < kFirstStages && sw0.live(a); ++i, sw0.next(a)) {
+        uint32_t dst = smem_u32(ring + (size_t)i * kStage);
+        mbar_expect_tx(full0 + 8 * i, sw0.nc() * kStageLoad);
+        bulk_load_1d(dst, wsrc(sw0), sw0.nc() * kStageBytes, full0 + 8 * i);
+      }
       if (FUSED) {
-        for (; i < S && i < kFirstStages && sw.live(a); ++i) sw.next(a);  // asked for before the activations were prepared
+        sw = sw0;
       } else {
-        StageWalk sw0 = sw;
-        for (; i < S && i < kFirstStages && sw0.live(a); ++i, sw0.next(a)) {
-          uint32_t dst = smem_u32(ring + (size_t)i * kStage);
-          mbar_expect_tx(full0 + 8 * i, sw0.nc() * kStageLoad);
-          bulk_load_1d(dst, wsrc(sw0), sw0.nc() * kStageBytes, full0 + 8 * i);
-        }
         pdl_wait();
         for (int j = 0; j < i; ++j, sw.next(a))
           bulk_load_1d(smem_u32(ring + (size_t)j * kStage) + C * kStageBytes, bsrc(sw), sw.nc() * kBTileBytes, full0 + 8 * j);
@@ -1172,8 +1164,8 @@ static int launch_impl(const TiledDesc& w, const MmaArgs& a0, cudaStream_t strea
   cfg.numAttrs = 1;
   if (!FUSED && !*prepared) {
     // activations -> digits, sums and scales, once per launch
-    cfg.gridDim = dim3(a.batch * (a.in_dim / 64));
-    cfg.blockDim = dim3(64);
+    cfg.gridDim = dim3(a.batch * a.nchunks);
+    cfg.blockDim = dim3(128);
     note_launch();
     GOPH_CUDA(cudaLaunchKernelEx(&cfg, mlx_prep_x_kernel<DIGITS, FMT != FMT_MLX4, !Fmt<FMT>::kConv, FMT == FMT_Q6K>, a.x,
                                  const_cast<unsigned char*>(a.xb), const_cast<float*>(a.xtab), a.batch, a.in_dim, N));
@@ -1242,17 +1234,18 @@ static int launch_with_chunks(const TiledDesc& w, const MmaArgs& a, cudaStream_t
   const int sms = device_state(w.device).sm_count;
   const int splits = choose_splits<MB>(a, sms, w.device);
   const int cmax = (a.nchunks + splits - 1) / splits;
-  // Narrow launches (one or two activation rows) whose items are short (at most four chunks: the
-  // matrices that are split over K to fill the SMs) make the digits of their own K range inside
-  // the product kernel: one launch instead of two (measured 7.3 against 7.6 us for 4096 x 4096 in
-  // a dependent chain).  Longer items are served better by the separate kernel, whose small
-  // blocks prepare the vector once for all CTAs (14336 x 4096: 14.1 against 15.2 us).
-  // Option mlx_fuse = 0 always keeps the separate preparation kernel.
-  if (N == 8 && options().mlx_fuse && splits <= sms && cmax <= 4) {
+  // Narrow launches (one or two activation rows) make the digits of their own K range inside the product kernel, one launch
+  // instead of two, as long as the B tiles that stay resident leave the ring its stages: four do for one row, two rows
+  // want five (B200, us a call, launch in front / own digits, one row: MLX4 4096x14336 11.7 / 10.3, 28672x4096 17.1 / 14.9,
+  // Q4_K 4096x14336 12.8 / 11.8, Q8_0 14336x4096 13.8 / 12.5, with four stages Q4_K 28672x7168 30.4 / 30.3, Q6_K 28672x8192
+  // 47.2 / 46.0; two rows with four stages: MLX4 28672x8192 31.1 / 33.8).  Launches of 16 columns (three or four rows, two
+  // of Q4_K and Q6_K) do it where every warp has one chunk of one row at most (four rows, Q8_0 4096x4096 11.1 / 10.3,
+  // 28672x1024 11.7 / 10.0; with two each Q5_K 6144x4096 13.8 / 14.5).  Option mlx_fuse = 0 always keeps the launch.
+  if (N <= 16 && options().mlx_fuse && splits <= sms && (N == 8 || a.batch * cmax < mma_threads<N, FMT>() / 32)) {
     size_t fixed = MmaSmem<N, FMT, true, C>::bytes(0, a.batch, a.in_dim, cmax);
     int stages = fixed < kMmaSmemBudget ? (int)((kMmaSmemBudget - fixed) / MmaSmem<N, FMT, true, C>::kStage) : 0;
     if (stages > kMaxStages) stages = kMaxStages;
-    if (stages >= 3) return launch_impl<N, DIGITS, MB, FMT, N == 8, C>(w, a, stream, prepared, stages, splits);
+    if (stages >= (MB == 1 ? 4 : 5)) return launch_impl<N, DIGITS, MB, FMT, N <= 16, C>(w, a, stream, prepared, stages, splits);
   }
   size_t fixed = MmaSmem<N, FMT, false, C>::bytes(0, a.batch, a.in_dim);
   int stages = fixed < kMmaSmemBudget ? (int)((kMmaSmemBudget - fixed) / MmaSmem<N, FMT, false, C>::kStage) : 0;
@@ -1328,7 +1321,7 @@ int mlx_mma_launch(const goph_mlx_weight* w, float* out, const float* x, int bat
 // ---- grouped launches (mixture-of-experts) -----------------------------------------------------
 
 // The activations of every (entry, row) as the tensor core wants them: block = one row of one entry,
-// a warp takes 64-element groups; arithmetic and layout are mlx_prep_x_kernel's.  PHASE 0: the row is
+// a warp takes chunks; arithmetic and layout are mlx_prep_x_kernel's.  PHASE 0: the row is
 // the item's token in src[tokens][in_dim]; PHASE 1: silu(g) * u of the gate and up results
 // src[entry * MB + m][2][in_dim] (kernels.SiLU then the multiply, backends/simd/kernels/activation.go:15-24;
 // single-precision exp as in the CUDA-core expert kernels).
@@ -1337,7 +1330,6 @@ __global__ void __launch_bounds__(256)
 moe_mma_prep_kernel(const MmaGroupEntry* __restrict__ work, const int* __restrict__ count, int max_entries,
                     const float* __restrict__ src, int in_dim, int top_k, unsigned char* __restrict__ xb, size_t xb_stride,
                     float* __restrict__ xtab, int tab_stride) {
-  constexpr int DIGITS = 4, QBITS = 26;
   pdl_launch_dependents();
   pdl_wait();
   const int entry = blockIdx.x / MB, m = blockIdx.x - entry * MB;
@@ -1350,50 +1342,17 @@ moe_mma_prep_kernel(const MmaGroupEntry* __restrict__ work, const int* __restric
   const float* row = PHASE == 0 ? src + (size_t)(ge->item[m] / top_k) * in_dim : src + (size_t)(entry * MB + m) * 2 * in_dim;
   unsigned char* bdst = xb + (size_t)entry * xb_stride;
   float* tab = xtab + (size_t)entry * tab_stride;
-  for (int g = warp; g < groups; g += 8) {
-    float v[2];
+  for (int c = warp; c < in_dim / kChunkK; c += 8) {
+    const int k = c * kChunkK + lane * 8;
+    float v[8];
+    load_eight(row + k, v);
+    if (PHASE == 1) {
+      float u[8];
+      load_eight(row + in_dim + k, u);
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int k = g * 64 + h * 32 + lane;
-      if (PHASE == 0) {
-        v[h] = row[k];
-      } else {
-        const float gv = row[k], uv = row[in_dim + k];
-        v[h] = __fmul_rn(__fdiv_rn(gv, __fadd_rn(1.0f, expf(-gv))), uv);
-      }
+      for (int i = 0; i < 8; ++i) v[i] = __fmul_rn(__fdiv_rn(v[i], __fadd_rn(1.0f, expf(-v[i]))), u[i]);
     }
-    // the order of mlx_prep_x_kernel: each half's butterfly, then the halves
-    float s0 = v[0], s1 = v[1], mx = fmaxf(fabsf(v[0]), fabsf(v[1]));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-      s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    }
-    const float s = s0 + s1;
-    int e = (int)((__float_as_uint(mx) >> 23) & 0xFF);
-    if (e < QBITS + 2) e = QBITS + 2;
-    if (e > 254) e = 254;
-    if (lane == 0) {
-      tab[m * groups + g] = s;
-      tab[(MB + m) * groups + g] = __uint_as_float((uint32_t)(e - 126 - QBITS + 127) << 23);
-    }
-    const float fi = __uint_as_float((uint32_t)(QBITS - (e - 126) + 127) << 23);
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      int q = __float2int_rn(v[h] * fi);
-      const int k = (g & 3) * 64 + h * 32 + lane;
-      const int step = k >> 5, w = (k & 31) >> 3, j = k & 7;
-      const int pos = 8 * w + 4 * (j & 1) + (j >> 1);
-      unsigned char* base = bdst + (size_t)(g >> 2) * (N * 256) + step * (N * 32) + (pos >> 4) * ((N / 8) * 128) + (pos & 15);
-#pragma unroll
-      for (int d = 0; d < DIGITS; ++d) {
-        const int dig = d == DIGITS - 1 ? q : ((q + 64) & 127) - 64;
-        q = (q - dig) >> 7;
-        const int n = m * DIGITS + d;
-        base[(n >> 3) * 128 + (n & 7) * 16] = (unsigned char)(dig & 0xFF);
-      }
-    }
+    prep_chunk<4, false, false, false>(v, lane, bdst + (size_t)c * (N * 256), N, m, tab + m * groups + 4 * c, tab + (MB + m) * groups + 4 * c);
   }
 }
 
@@ -1828,8 +1787,8 @@ static int launch_noalloc(const goph_mlx_weight* w, float* out, const float* x, 
   cfg.stream = stream;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  cfg.gridDim = dim3(a.in_dim / 64);
-  cfg.blockDim = dim3(64);
+  cfg.gridDim = dim3(a.nchunks);
+  cfg.blockDim = dim3(128);
   note_launch();
   GOPH_CUDA(cudaLaunchKernelEx(&cfg, mlx_prep_x_kernel<DIGITS>, a.x, const_cast<unsigned char*>(a.xb),
                                const_cast<float*>(a.xtab), 1, a.in_dim, N));

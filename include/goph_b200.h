@@ -110,8 +110,9 @@ int goph_sm_count(int device);
  *   "mlx_digits"  signed base-128 digits each activation is written in on the tensor-core path,
  *                 relative to the largest magnitude of its 64-element group: 4 (default, 27 bits)
  *                 or 3 (20 bits; enough for bf16-valued activations)
- *   "mlx_fuse"    1 (default): tensor-core launches of one or two activation rows make the activation
- *                 digits of their own K range inside the product kernel (one launch per product);
+ *   "mlx_fuse"    1 (default): tensor-core launches of one or two activation rows, and of three or four
+ *                 over short K ranges, make the activation digits of their own K range inside the
+ *                 product kernel (one launch per product);
  *                 0: a separate preparation kernel in front of every product
  *   "mlx_chunks"  256-element chunks per pipeline stage of the tensor-core GEMV: 0 (default) two for
  *                 the nibble formats where tensor memory has the columns (up to 4 activation rows

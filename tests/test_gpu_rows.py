@@ -314,6 +314,35 @@ def test_weights_of_one_call_share_the_preparation(gpu, pkg):
         t.Free()
 
 
+# The digits made inside the product's launch and in a launch in front have the same bits: one, two and (short K ranges)
+# four rows, a chunk per four warps, per warp, and more chunks than warps; x at an address that is no multiple of 16.
+@pytest.mark.parametrize("fmt", ["mlx", "q4_k", "q5_k", "q6_k", "q8_0"])
+@pytest.mark.parametrize("out_dim,in_dim", [(19072, 256), (19072, 1024), (19000, 4352), (200, 6144), (19000, 5120)])
+def test_own_digits_and_a_launch_in_front_agree(gpu, pkg, fmt, out_dim, in_dim):
+    h, run, _, _ = make(gpu, pkg, fmt, True, out_dim, in_dim)
+    for rows in (1, 2, 3, 4):
+        x = pkg.synth.activations(("own", rows, in_dim), rows * in_dim, bf16=False)
+        aligned, buf = gpu.from_numpy(x), gpu.from_numpy(np.concatenate([[F(0)], x]).astype(F))
+        odd = gpu.wrap(buf.Ptr + 4, 4 * rows * in_dim)
+        got = []
+        for fuse, xo in ((1, aligned), (0, aligned), (1, odd), (0, odd)):
+            gpu.SetOption("mlx_fuse", fuse)
+            out = out_with_canary(gpu, rows * out_dim)
+            try:
+                run(out, xo, rows)
+            finally:
+                gpu.SetOption("mlx_fuse", 1)
+            gpu.Sync()
+            got.append(read_and_check_canary(out, rows * out_dim).view(np.uint32))
+            out.Free()
+        # (an x that is not aligned keeps Q4_K from the several-row product that takes its four rows otherwise)
+        assert np.array_equal(got[0], got[1]) and np.array_equal(got[2], got[3])
+        assert np.array_equal(got[0], got[2]) or (fmt, rows) == ("q4_k", 4)
+        aligned.Free(); buf.Free()
+    h.Free()
+    assert gpu.KernelStatus() == 0
+
+
 # A call of several tiled weights and few rows: short K ranges prepare x inside the product's launch and leave nothing in the
 # scratch that a weight with longer ones, in the same call, could use.
 @pytest.mark.parametrize("rows", [1, 2, 3, 4])
