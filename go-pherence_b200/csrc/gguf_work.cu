@@ -6,8 +6,10 @@
 //     (nvidia.GemvQ8_0BatchScatter / GemvQ8_0ScatterByWork, backends/nvidia/runtime/q8.go:193-222;
 //     kernel text backends/nvidia/ptx/q8/q8_scatter*.go).
 // Both for Q4_K and Q8_0 matrices in either device layout (the reference has the first for Q4_K and
-// the second for Q8_0 only).  CUDA-core kernels: one warp per (output row, work item), a lane takes
-// 32-element units of the row; the weights of an item's expert are read once per item.  The indices
+// the second for Q8_0 only).  Matrices in the tensor-core layouts and lists of 8 to 512 items: grouped launches of the
+// integer tensor-core GEMV (mlx_mma.cu) with the stream's scratch; the others, and calls under capture, which have no
+// scratch: CUDA-core kernels, passes over an expert's rows for up to four of its items, or one warp per (output row, work item),
+// a lane taking 32-element units of the row.  The indices
 // of a work list live in device memory, so the kernels check them: an expert index outside the
 // matrix or a destination outside dst is skipped and recorded in the status word (601 / 602).
 #include <string.h>
@@ -16,6 +18,8 @@
 
 #include "goph_internal.cuh"
 #include "gguf_fmt.cuh"
+#include "mlx_mma.cuh"
+#include "qgemm.cuh"
 
 namespace goph {
 namespace {
@@ -107,13 +111,6 @@ __device__ __forceinline__ float row_dot(const WorkView& v, int row, const float
   float acc = 0.f;
   for (int unit = lane; unit < v.in_dim / 32; unit += 32) acc += unit_dot(v, row, unit, x);
   return warp_sum(acc);
-}
-
-// GELU in the tanh form of the reference kernel: 0.5 g (1 + tanh(0.79788456 (g + 0.044715 g^3)))
-__device__ __forceinline__ float gelu_tanh(float g) {
-  const float u = 0.7978845608f * fmaf(0.044715f, g * g * g, g);
-  const float t = 2.f / (1.f + __expf(-2.f * u)) - 1.f;
-  return 0.5f * g * (1.f + t);
 }
 
 // grid (row blocks, items); a warp per (intermediate row i, item w)
@@ -365,9 +362,38 @@ static void (*pick_work_kernel(bool by_item))(const StreamArgs, const WorkArgs) 
   return by_item ? stream_work_kernel<F, MODE, true> : stream_work_kernel<F, MODE, false>;
 }
 
+// Tensor-core layouts: grouped launches on the tensor cores (mlx_mma.cu), with the stream's scratch; false = not taken (no
+// scratch: under capture, on streams beyond the first eight of a device).
+template <int MODE>
+bool launch_grouped_work(const goph_gguf_matrix* m, const float* x, const WorkArgs& wa, cudaStream_t stream, int* rc) {
+  if (!m->tiled || wa.work_len > kMaxWorkList) return false;
+  QBufs* bufs = qgemm_scratch(m->device, stream);
+  if (!bufs) return false;
+  MmaWorkLaunch g;
+  memset(&g, 0, sizeof g);
+  g.x = x;
+  g.experts = wa.experts;
+  g.pos = wa.pos;
+  g.weight = wa.weight;
+  g.out = wa.out;
+  g.dst_len = wa.dst_len;
+  g.status = wa.status;
+  g.items = wa.work_len;
+  g.active = wa.active_experts;
+  g.mats = MODE == 0 ? 2 : 1;
+  g.rows = MODE == 0 ? wa.inter : wa.expert_rows;
+  g.in_dim = m->in_dim;
+  bool taken = false;
+  const QScratch area = qgemm_scratch_area(bufs);
+  std::lock_guard<std::mutex> held(*area.enqueue);  // (threads on one stream do not come between the two launches)
+  *rc = gguf_mma_launch_work(m, g, area.bytes, area.size, stream, &taken);
+  return taken || *rc != GOPH_OK;
+}
+
 template <int MODE>
 bool launch_stream_work(const goph_gguf_matrix* m, const float* x, const WorkArgs& wa, cudaStream_t stream, int* rc) {
   if (wa.work_len > kMaxWorkItems || m->in_dim % 256) return false;
+  if (launch_grouped_work<MODE>(m, x, wa, stream, rc)) return true;
   StreamArgs a;
   memset(&a, 0, sizeof a);
   const bool q4 = m->qtype == GOPH_GGUF_Q4_K, tiled = m->tiled != nullptr;

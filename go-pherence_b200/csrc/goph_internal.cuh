@@ -168,6 +168,13 @@ __device__ __forceinline__ uint4 ld_stream(const uint4* p) {
   return v;
 }
 
+// GELU in the tanh form of the reference kernel: 0.5 g (1 + tanh(0.79788456 (g + 0.044715 g^3)))
+__device__ __forceinline__ float gelu_tanh(float g) {
+  const float u = 0.7978845608f * fmaf(0.044715f, g * g * g, g);
+  const float t = 2.f / (1.f + __expf(-2.f * u)) - 1.f;
+  return 0.5f * g * (1.f + t);
+}
+
 __device__ __forceinline__ float bf16_bits_to_f32(uint32_t b16) { return __uint_as_float(b16 << 16); }
 
 // Two packed f32 FMAs in one instruction (sm_100 fma.rn.f32x2): acc += a*b lane-wise.

@@ -197,7 +197,7 @@ struct MmaSmem {
 // Walks the (tile, chunk) stages of this CTA's work items in the order every role uses.
 // G (grouped launches): the CTA takes one contiguous range of the live items, so that it stays with
 // one entry's activations for several tiles; item w = (entry, matrix, tile of the matrix).
-template <bool G>
+template <bool G, bool WORK = false>
 struct StageWalkT {
   int w, tile, split, c, c1;
   int cps;  // chunks per stage
@@ -209,6 +209,10 @@ struct StageWalkT {
       const int rem = w - entry * per;
       mat = rem / a.gtpe;
       tile = rem - mat * a.gtpe;
+      if (WORK && a.gdirect == 2) {  // gate and up of a tile one behind the other
+        mat = rem & 1;
+        tile = rem >> 1;
+      }
       split = 0;
       c = 0;
       c1 = a.nchunks;
@@ -222,8 +226,9 @@ struct StageWalkT {
   __device__ __forceinline__ StageWalkT(const MmaArgs& a, int chunks_per_stage = 1, int live_items = 0)
       : w(blockIdx.x), cps(chunks_per_stage) {
     if (G) {
-      w = (int)((long long)blockIdx.x * live_items / gridDim.x);
-      wend = (int)((long long)(blockIdx.x + 1) * live_items / gridDim.x);
+      const int each = WORK && a.gdirect == 2 ? 2 : 1;  // (whole pairs)
+      w = (int)((long long)blockIdx.x * (live_items / each) / gridDim.x) * each;
+      wend = (int)((long long)(blockIdx.x + 1) * (live_items / each) / gridDim.x) * each;
     }
     if (live(a)) open(a);
   }
@@ -377,9 +382,10 @@ __device__ __forceinline__ void prep_x_in_cta(const float* __restrict__ x, int b
 template <int N, int DIGITS, int MB, int FMT = FMT_MLX4, bool FUSED = false, int C = 1, bool G = false>
 __global__ void __launch_bounds__((mma_threads<N, FMT>()), 1)
 mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
-  static_assert(!G || (!FUSED && FMT == FMT_MLX4), "grouped launches: MLX 4-bit, activations prepared in front");
+  static_assert(!G || !FUSED, "grouped launches: activations prepared in front");
+  constexpr bool kWork = G && FMT != FMT_MLX4;  // a work list's entries (MmaWorkEntry)
   TP(const long long t_entry = clock64();)
-  typedef StageWalkT<G> StageWalk;
+  typedef StageWalkT<G, kWork> StageWalk;
   constexpr int EP = epi_parts<N, FMT>();
   constexpr bool kSpills = !Fmt<FMT>::kConv && MB == 8;  // a byte per weight, eight rows: the epilogue is short of registers
   constexpr int kEpiWarps = 4 * EP, kEpiThreads = kEpiWarps * 32;
@@ -468,10 +474,13 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
     gitems = n * a.gtpe * a.gmats;
   }
   StageWalk sw(a, C, gitems);
+  auto entry_at = [&](int e) -> const MmaGroupEntry* {
+    return kWork ? &reinterpret_cast<const MmaWorkEntry*>(a.gwork)[e].g : a.gwork + e;
+  };
   // where a stage's weights and prepared activations lie
   auto wsrc = [&](const StageWalk& s) {
     const unsigned char* base = a.w;
-    if (G) base = reinterpret_cast<const unsigned char*>(__ldg(reinterpret_cast<const unsigned long long*>(&a.gwork[s.entry].w[a.gfirst + s.mat])));
+    if (G) base = reinterpret_cast<const unsigned char*>(__ldg(reinterpret_cast<const unsigned long long*>(&entry_at(s.entry)->w[a.gfirst + s.mat])));
     return base + ((size_t)s.tile * a.nchunks + s.c) * kStageBytes;
   };
   auto bsrc = [&](const StageWalk& s) { return a.xb + (G ? (size_t)s.entry * a.gxb : 0) + (size_t)s.c * kBTileBytes; };
@@ -664,6 +673,7 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
     int nb = a.batch;    // activation rows in use (G: of the current entry)
     int cur_entry = -1;  // G: the entry whose tables are in shared memory
     int orow[G ? MB : 1];  // G: result row of each activation row
+    float gate[kWork ? MB : 1];  // work lists: the gate's sums while up is computed
     constexpr int kHB = kBlocks / EP;                       // blocks of this part
     constexpr int kSub = kHB * N <= 64 ? kHB : 64 / N;      // blocks per pass (at most 64 columns in registers)
     constexpr bool kNarrow = kSub * N == 8;                 // a pass of one 8-column block: one 8-column load
@@ -677,10 +687,10 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
         cur_entry = sw.entry;
         const float* tab = a.xtab + (size_t)cur_entry * a.gtab;
         for (int j = et; j < 2 * a.batch * groups; j += kEpiThreads) xsum[j] = __ldcg(tab + j);
-        const MmaGroupEntry* ge = a.gwork + cur_entry;
+        const MmaGroupEntry* ge = entry_at(cur_entry);
         nb = __ldg(&ge->count);
 #pragma unroll
-        for (int m = 0; m < (G ? MB : 1); ++m) orow[m] = a.gdirect ? __ldg(&ge->item[m]) : cur_entry * MB + m;
+        for (int m = 0; m < (G ? MB : 1); ++m) orow[m] = kWork || a.gdirect ? __ldg(&ge->item[m]) : cur_entry * MB + m;
         asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
       }
       ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * slot, kSpills ? (i / S) & 1 : rc.ph, a.status, 6));
@@ -894,7 +904,18 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
         if (half == 0) {
 #pragma unroll
           for (int m = 0; m < MB; ++m) {
-            if (m < nb) a.out[(size_t)orow[G ? m : 0] * a.out_dim + gmat * (a.gtpe * kTileRows) + row] = acc[m];
+            if constexpr (kWork) {
+              if (a.gdirect == 2) {
+                if (gmat == 0) gate[m] = acc[m];
+                else if (m < nb) a.out[(size_t)orow[m] * a.out_dim + row] = gelu_tanh(gate[m]) * acc[m];
+              } else if (m < nb) {
+                const MmaWorkEntry* we = reinterpret_cast<const MmaWorkEntry*>(a.gwork) + cur_entry;
+                float* dst = reinterpret_cast<float*>(__ldg(reinterpret_cast<const unsigned long long*>(&we->dst[m])));
+                if (row < __ldg(&we->room[m])) atomicAdd(dst + row, acc[m] * __ldg(&we->weight[m]));  // items may share a destination row
+              }
+            } else {
+              if (m < nb) a.out[(size_t)orow[G ? m : 0] * a.out_dim + gmat * (a.gtpe * kTileRows) + row] = acc[m];
+            }
             acc[m] = 0.f;
           }
         }
@@ -1702,6 +1723,172 @@ int gguf_mma_dequant(const goph_gguf_matrix* m, float* out, cudaStream_t stream)
   }
   GOPH_CUDA(cudaGetLastError());
   return GOPH_OK;
+}
+
+// ---- grouped launches over a work list (GGUF experts stacked in one matrix) -------------------------------
+
+// Measured with the products behind it (B200, 128 experts of 2048/768, Q4_K gate|up and Q8_0 down, us a call, CUDA-core kernels
+// in front): 16 items 24.8 -> 17.5 and 21.9 -> 11.6, 64 items 76.5 -> 38.6 and 71 -> 20.4, 256 items 248 -> 82.7 and 257 -> 49.6.
+// Bound by the weights of the distinct experts, whose tiles come once per entry, and the end of every item (900 cycles).
+// A CTA per item of the list: the list is cut into entries of up to MB items of one expert, numbered by their first
+// items, and the item's activations become digits, sums and scales of its entry.  Every CTA finds its own place in the
+// list (up to kMaxWorkList words); the first also counts the entries.
+template <int FMT, int MB>
+__global__ void __launch_bounds__(256)
+work_prep_kernel(const __grid_constant__ MmaWorkLaunch g, MmaWorkEntry* __restrict__ work, int* __restrict__ count, unsigned char* __restrict__ xb, size_t gxb,
+                 float* __restrict__ xtab, int gtab, unsigned long long stage_bytes) {
+  typedef Fmt<FMT> F;
+  constexpr int N = 4 * MB * (F::kHalves ? 2 : 1);
+  __shared__ __align__(16) int ex[kMaxWorkList], rank[kMaxWorkList];
+  __shared__ int s_leader;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, w = blockIdx.x;
+  pdl_launch_dependents();
+  pdl_wait();
+  for (int t = tid; t < kMaxWorkList; t += 256) {
+    uint32_t e = 0xFFFFFFFFu;
+    if (t < g.items) e = g.experts ? __ldg(g.experts + t) : 0u;
+    ex[t] = e < (uint32_t)g.active ? (int)e : -1;
+  }
+  __syncthreads();
+  for (int t = tid; t < g.items; t += 256) {  // an item's place among its expert's
+    int r = 0;
+    const int e = ex[t];
+    for (int u = 0; u < t; u += 4) {
+      const int4 q = *reinterpret_cast<const int4*>(ex + u);
+      r += (q.x == e) + (u + 1 < t && q.y == e) + (u + 2 < t && q.z == e) + (u + 3 < t && q.w == e);
+    }
+    rank[t] = e < 0 ? -1 : r;
+  }
+  __syncthreads();
+  const int e = ex[w], first = e < 0 ? 0 : rank[w] / MB * MB;
+  int leaders = 0, id = 0, mine = 0;
+  for (int t0 = 0; t0 < g.items; t0 += 256) {
+    const int t = t0 + tid;
+    const bool in = t < g.items && ex[t] >= 0, same = in && ex[t] == e && rank[t] >= first && rank[t] < first + MB;
+    if (same && rank[t] == first) s_leader = t;
+    leaders += __syncthreads_count(in && rank[t] % MB == 0);
+    mine += __syncthreads_count(same);
+  }
+  if (w == 0 && tid == 0) *count = leaders;
+  if (e < 0) {
+    if (tid == 0) atomicCAS(g.status, 0, 601);
+    return;
+  }
+  const int leader = s_leader, m = rank[w] - first;
+  for (int t0 = 0; t0 < leader; t0 += 256) {
+    const int t = t0 + tid;
+    id += __syncthreads_count(t < leader && ex[t] >= 0 && rank[t] % MB == 0);
+  }
+  MmaWorkEntry* we = work + id;
+  if (tid == 0) {
+    if (m == 0) {
+      for (int k = 0; k < 2; ++k) we->g.w[k] = g.tiled + ((size_t)e * g.mats + k) * (g.rows / kTileRows) * (g.in_dim / kChunkK) * stage_bytes;
+      we->g.count = mine;
+      we->g.expert = e;
+    }
+    we->g.item[m] = w;
+    if (g.pos) {
+      const unsigned long long at = (unsigned long long)__ldg(g.pos + w) * (unsigned long long)g.rows, left = at < g.dst_len ? g.dst_len - at : 0;
+      if (left < (unsigned long long)g.rows) atomicCAS(g.status, 0, 602);
+      we->dst[m] = g.out + (left ? at : 0);
+      we->room[m] = left < (unsigned long long)g.rows ? (int)left : g.rows;
+      we->weight[m] = __ldg(g.weight + w);
+    }
+  }
+  constexpr int kPer = kChunkK / F::kGroup;
+  const int ntab = g.in_dim / F::kGroup;
+  float* tab = xtab + (size_t)id * gtab;
+#pragma unroll 1
+  for (int c = warp; c < g.in_dim / kChunkK; c += 8) {
+    float v[8];
+    load_eight(g.x + (size_t)w * g.in_dim + c * kChunkK + lane * 8, v);
+    prep_chunk<4, true, !F::kConv, FMT == FMT_Q6K>(v, lane, xb + (size_t)id * gxb + (size_t)c * (N * 256), N, m, tab + m * ntab + c * kPer,
+                                                   tab + (MB + m) * ntab + c * kPer);
+  }
+}
+
+template <int FMT, int MB>
+static int launch_work(int device, const MmaWorkLaunch& g, unsigned char* scratch, size_t bytes, cudaStream_t stream, bool* taken) {
+  constexpr int N = 4 * MB * (Fmt<FMT>::kHalves ? 2 : 1), C = stage_chunks<N, FMT>();
+  MmaDeviceBufs* bufs = device_bufs(device);
+  if (!bufs) return GOPH_OK;  // the kernels without scratch
+  MmaArgs a;
+  memset(&a, 0, sizeof a);
+  a.status = bufs->status;
+  a.out = g.out;
+  a.out_dim = g.rows;
+  a.in_dim = g.in_dim;
+  a.batch = MB;
+  a.ntiles = a.gtpe = g.rows / kTileRows;
+  a.nchunks = g.in_dim / kChunkK;
+  a.splits = 1;
+  a.gmats = g.mats;
+  a.gdirect = g.pos ? 3 : 2;
+  a.gtab = 2 * MB * (g.in_dim / Fmt<FMT>::kGroup);
+  a.gxb = (size_t)a.nchunks * N * 256;
+  // scratch: the entries, their number, tables, B tiles.  At most so many entries: every expert may have one that is not full
+  const int most_entries = (int)(((long long)g.items + (long long)(g.active < g.items ? g.active : g.items) * (MB - 1)) / MB);
+  a.gmax = most_entries < g.items ? most_entries : g.items;
+  const size_t entries = (size_t)a.gmax * sizeof(MmaWorkEntry) + 256, tabs = ((size_t)a.gmax * a.gtab * 4 + 255) & ~(size_t)255;
+  size_t fixed = MmaSmem<N, FMT, false, C>::bytes(0, MB, g.in_dim);
+  int stages = fixed < kMmaSmemBudget ? (int)((kMmaSmemBudget - fixed) / MmaSmem<N, FMT, false, C>::kStage) : 0;
+  if (stages > kMaxStages) stages = kMaxStages;
+  a.items = a.gmax * g.mats * a.ntiles;
+  if (stages < 3) return GOPH_OK;
+  MmaWorkEntry* work = reinterpret_cast<MmaWorkEntry*>(scratch);
+  int* count = reinterpret_cast<int*>(scratch + entries - 256);
+  float* xtab = reinterpret_cast<float*>(scratch + ((entries + 255) & ~(size_t)255));
+  unsigned char* xb = reinterpret_cast<unsigned char*>(xtab) + tabs;
+  if ((size_t)(xb - scratch) + (size_t)a.gmax * a.gxb > bytes) return GOPH_OK;
+  a.gwork = reinterpret_cast<const MmaGroupEntry*>(work);
+  a.gcount = count;
+  a.xb = xb;
+  a.xtab = xtab;
+  a.stages = stages;
+  size_t smem = MmaSmem<N, FMT, false, C>::bytes(stages, MB, g.in_dim);
+  if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM
+  auto kern = mlx_mma_kernel<N, 4, MB, FMT, false, C, true>;
+  GOPH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = options().pdl ? 1 : 0;
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof cfg);
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cfg.gridDim = dim3(g.items);
+  cfg.blockDim = dim3(256);
+  *taken = true;
+  note_launch();
+  GOPH_CUDA(cudaLaunchKernelEx(&cfg, work_prep_kernel<FMT, MB>, g, work, count, xb, a.gxb, xtab, a.gtab, (unsigned long long)Fmt<FMT>::kStageBytes));
+  const int sms = device_state(device).sm_count, most = a.items / (g.pos ? 1 : 2);
+  cfg.gridDim = dim3(most < sms ? most : sms);
+  cfg.blockDim = dim3(mma_threads<N, FMT>());
+  cfg.dynamicSmemBytes = smem;
+  note_launch();
+  GOPH_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
+  return GOPH_OK;
+}
+
+int gguf_mma_launch_work(const goph_gguf_matrix* m, const MmaWorkLaunch& g0, unsigned char* scratch, size_t bytes, cudaStream_t stream, bool* taken) {
+  *taken = false;
+  if (!m->tiled || (m->qtype != GOPH_GGUF_Q4_K && m->qtype != GOPH_GGUF_Q8_0) || g0.items > kMaxWorkList || g0.rows % kTileRows || g0.in_dim % kChunkK ||
+      g0.in_dim > 16384)
+    return GOPH_OK;
+  MmaWorkLaunch g = g0;
+  g.tiled = m->tiled;
+  // A short list leaves most SMs idle at a tile (with gate and up: a pair of tiles) a CTA, or is over before the two launches
+  // are, and the CUDA-core kernels, a warp to a row, are as fast: us, those / these, gate|up Q4_K 2 items of 1024x2048 8.4 / 16.9,
+  // 6 of 512x1280 12.4 / 14.0, 8 of 768x1024 12.6 / 12.5, of 768x1536 16.9 / 14.8; down Q8_0 2 items of 2048x1024 6.3 / 9.4, 6 of
+  // 1280x512 8.4 / 8.6, 8 of 1024x768 10.4 / 8.9.
+  const long tiles = (long)g.items * (g.rows / kTileRows), size = (long)g.items * g.rows * g.in_dim;
+  if (tiles < (g.pos ? 64 : 48) || size < (g.pos ? 6l : 8l) << 20) return GOPH_OK;
+  // Entries of two items; of four for Q8_0 where experts have three and more on average.  (Q4_K with four takes accumulator blocks of
+  // 32 columns and one chunk a stage: 1.2 us an entry against 0.55.)
+  const bool wide = g.items >= 3 * g.active;
+  if (m->qtype == GOPH_GGUF_Q4_K) return launch_work<FMT_Q4K, 2>(m->device, g, scratch, bytes, stream, taken);
+  return wide ? launch_work<FMT_Q80, 4>(m->device, g, scratch, bytes, stream, taken) : launch_work<FMT_Q80, 2>(m->device, g, scratch, bytes, stream, taken);
 }
 
 // ---- GEMV without any allocation ---------------------------------------------------------------

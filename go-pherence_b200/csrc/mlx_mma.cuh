@@ -61,6 +61,30 @@ struct MmaGroupLaunch {
 // Two launches: the entries' activations as digits, sums and scales; then the products.
 int mlx_mma_launch_grouped(int device, const MmaGroupLaunch& g, cudaStream_t stream);
 
+// ---- grouped launches over a work list: GGUF experts stacked in one tiled matrix -------------------------
+constexpr int kMaxWorkList = 512;
+// Up to four items of one expert (g.w: its gate and up, or its matrix).
+struct __align__(16) MmaWorkEntry {
+  MmaGroupEntry g;    // item: place in the list
+  float* dst[4];      // scatter: destination row of each item, how many of its elements there are, its weight
+  int room[4];
+  float weight[4];
+};
+struct MmaWorkLaunch {
+  const unsigned char* tiled;  // (filled in)
+  const float* x;              // [items][in_dim]
+  const uint32_t* experts;     // [items], or nullptr: all 0
+  const uint32_t* pos;         // scatter: destination row of each item; nullptr: out[items][rows] = gelu(gate) * up
+  const float* weight;
+  float* out;
+  unsigned long long dst_len;
+  int* status;                 // 601: expert outside the matrix, 602: destination outside out (skipped)
+  int items, active, mats, rows, in_dim;  // experts, matrices of each (gate and up: 2), rows of each of them
+};
+// Two launches (entries and activations; products) with the caller's scratch, which is in use until they are through.
+// *taken: false where this is not a list for it (nothing is launched then).
+int gguf_mma_launch_work(const goph_gguf_matrix* m, const MmaWorkLaunch& g, unsigned char* scratch, size_t bytes, cudaStream_t stream, bool* taken);
+
 // Reads the device status word (0 = every wait completed); synchronises the copy stream.
 int mlx_mma_status(int device);
 void mlx_mma_status_clear(int device);

@@ -1653,6 +1653,8 @@ QBufs* qgemm_scratch(int device, cudaStream_t stream) {
   return &b;
 }
 
+QScratch qgemm_scratch_area(QBufs* b) { return QScratch{b->xb, b->xb_bytes, &b->enqueue}; }
+
 void qgemm_weights(int device, int change) {
   StreamAreas& s = stream_areas(device);
   std::lock_guard<std::mutex> lock(s.mu);

@@ -2,6 +2,8 @@
 // cores, for every weight format and both device layouts; implemented in qgemm.cu.
 #pragma once
 
+#include <mutex>
+
 #include "goph_internal.cuh"
 
 namespace goph {
@@ -37,6 +39,14 @@ bool qgemm_wants(int fmt, bool tiled, bool x_bf16, long out_dim, int in_dim, int
 // there is none, the call is the business of the kernels for few rows, which need none.
 struct QBufs;
 QBufs* qgemm_scratch(int device, cudaStream_t stream);
+
+// The area itself, for other launches that prepare activations; enqueue is to be held from the first of them to the last.
+struct QScratch {
+  unsigned char* bytes;
+  size_t size;
+  std::mutex* enqueue;
+};
+QScratch qgemm_scratch_area(QBufs* b);
 
 // A weight handle of any format was made (+1) or is being freed (-1).
 void qgemm_weights(int device, int change);

@@ -6,7 +6,7 @@ list, every item checked against the single-expert product."""
 import numpy as np
 import pytest
 
-from gpu_util import F, TOL, out_with_canary, read_and_check_canary
+from gpu_util import CANARY, F, TOL, out_with_canary, read_and_check_canary
 from oracle import binding as orc
 
 pytestmark = pytest.mark.gpu
@@ -195,4 +195,51 @@ def test_work_calls_reject_malformed_arguments(gpu, pkg):
         gpu.GemvQ8_0ScatterByWork(out, x, we, we, out, 1, 3, m)          # 128 rows do not divide into 3 experts
     gpu.GateUpGELUQ4KByWorkToBuffer(out, x, we, 0, 64, 1, m)             # an empty work list is a no-op, as in the reference
     for t in (m, x, out, we):
+        t.Free()
+
+
+# The grouped tensor-core form (tensor-core layouts, lists of up to 512 items on streams with scratch): entries of two and
+# four items, experts with more items than one, either side of the blocks of 256 list words and of the longest list, one expert with all.
+@pytest.mark.parametrize("qtype", [Q4_K, Q8_0])
+@pytest.mark.parametrize("items,active", [(128, 160), (129, 7), (128, 1), (257, 128), (512, 40), (513, 40)])
+def test_grouped_work_lists(gpu, pkg, qtype, items, active):
+    """Against the streaming layout's kernels on the same blocks: exact integer dot products against f32 ones in another order,
+    2^-23 times the square root of 512 terms on either side, and the gate's part through an exponential: 2e-5 of the largest.  An expert and a
+    destination outside the matrix are skipped, the rest of their list is not."""
+    inter, hidden, tokens = 128, 512, 9        # lists from 8 Mi and 6 Mi weights on
+    g = pkg.synth.rng("grouped", items, active)
+    raw_gu, raw_dn = make(pkg, qtype, ("ggu", active), active * 2 * inter, hidden), make(pkg, qtype, ("gdn", active), active * hidden, inter * 2)
+    ids = g.integers(0, active, items).astype(np.uint32)
+    ids[items // 2], ids[-1] = active, 0xFFFFFFFF
+    pos = g.integers(0, tokens, items).astype(np.uint32)
+    pos[1] = tokens                                   # behind dst
+    wt = g.uniform(0.1, 0.5, items).astype(F)
+    x, h = pkg.synth.activations(("gx", items), items * hidden, bf16=False), pkg.synth.activations(("gh", items), items * inter * 2, bf16=False)
+    bufs = [gpu.from_numpy(a) for a in (x, ids, h, pos, wt)]
+    got = []
+    for layout in (1, 2):
+        gpu.SetOption("gguf_layout", layout)
+        try:
+            gu, dn = gpu.UploadGGUFMatrix(qtype, raw_gu, hidden, active * 2 * inter), gpu.UploadGGUFMatrix(qtype, raw_dn, inter * 2, active * hidden)
+        finally:
+            gpu.SetOption("gguf_layout", 0)
+        out, dst = out_with_canary(gpu, items * inter), out_with_canary(gpu, tokens * hidden)
+        dst.Upload(np.concatenate([np.zeros(tokens * hidden, dtype=F), np.full(64, CANARY, dtype=F)]))
+        before = gpu.LaunchCount()
+        gpu.GateUpGELUQ4KByWorkToBuffer(out, bufs[0], bufs[1], items, inter, active, gu)
+        gpu.GemvQ8_0ScatterByWork(gpu.wrap(dst.Ptr, tokens * hidden * 4), bufs[2], bufs[1], bufs[3], bufs[4], items, active, dn)
+        grouped = layout == 2 and items <= 512
+        assert gpu.LaunchCount() - before == (4 if grouped else 2)
+        gpu.Sync()
+        assert gpu.KernelStatus() in (601, 602)
+        gpu.KernelStatusClear()
+        got.append((read_and_check_canary(out, items * inter).reshape(items, inter), read_and_check_canary(dst, tokens * hidden).reshape(tokens, hidden)))
+        for t in (gu, dn, out, dst):
+            t.Free()
+    for act, _ in got:
+        assert np.all(act[items // 2] == CANARY) and np.all(act[-1] == CANARY)
+    keep = np.delete(np.arange(items), [items // 2, items - 1])
+    for a, b in ((got[0][0][keep], got[1][0][keep]), (got[0][1], got[1][1])):
+        assert np.max(np.abs(a - b)) <= 2e-5 * np.max(np.abs(a)) and np.max(np.abs(a)) > 0
+    for t in bufs:
         t.Free()
