@@ -1,54 +1,45 @@
-// MLX 4-bit weights on the 5th-generation tensor cores (tcgen05 + TMEM), integer arithmetic.
+// Products of up to eight activation rows with weights in the tiled layouts (MLX 4-bit, Q4_K, Q5_K, Q6_K, Q8_0), in exact
+// integer arithmetic on the tensor cores' register path (mma.sync, kind s8).
 //
-// Why a GEMV goes to the tensor pipe: at B200's HBM rate one SM has to consume ~47 nibbles
-// per clock, and its integer/logic pipe issues 64 lane-ops per clock.  Any formulation that
-// turns each nibble into a float on the CUDA cores needs at least one logic op per nibble plus
-// the FMA and cannot reach the HBM roofline.  Here the nibbles stay integers: three logic ops
-// turn a packed word into eight unsigned bytes, the tensor cores multiply them (kind::i8, exact
-// int32 accumulation), and the CUDA cores only apply the per-group scales.
+// Why this path: at B200's HBM rate one SM has to take in 41 nibbles a clock.  Turned into floats on the CUDA cores a nibble
+// costs five to seven lane instructions and an SM has 128 a clock.  Here nibbles stay integers: three logic instructions turn
+// a packed word into eight bytes, which are the A fragment of an MMA as they stand; the MMA is exact, and per group of weights
+// a scale is applied.  MMAs of 16 x 8 x 32 bytes issue every two clocks on an SM (measured): 256 weights a clock for two
+// activation rows, five times what HBM delivers, so there is nothing to gain from tcgen05's rate, which wants the bytes written to
+// tensor memory by converter warps and the sums read back by others.  That form, which stood here, handed every 18 KB from
+// warp to warp four times, took a whole SM a CTA and got 34 weights a clock; a warp that does it all for its rows got 46 (one row, Q4_K 128256x4096).
 //
 // Arithmetic
-//   * A operand (weights): nibble n as the unsigned byte n.
-//   * B operand (activations): each 64-element group of an activation row is put on a common
+//   * A operand (weights): nibble n as the unsigned byte n, byte formats as they lie in the tile.
+//   * B operand (activations): each group of 64 (MLX) or 32 elements of an activation row is put on a common
 //     power-of-two scale 2^(E-26), E the exponent of the group's largest magnitude, and every
-//     element becomes the integer q = round(x * 2^(26-E)), |q| <= 2^26 — at least as fine as
+//     element becomes the integer q = round(x * 2^(26-E)), |q| <= 2^26 -- at least as fine as
 //     the f32 spacing of the group's largest elements.  q is written as four balanced base-128
-//     digits, one signed-byte B row per digit (three digits is an option for bf16-valued x).
-//   * One int32 accumulator block per 64-element group: D_j[row] = sum_k n_k * digit_j(q_k),
-//     exact.  The epilogue rebuilds sum_k n_k q_k = (D0 + 128 D1) + 16384 (D2 + 128 D3) (two
-//     exact integers, one fused multiply-add), scales by 2^(E-26) and forms
-//     s_g * dot + b_g * sum(x)  in f32 — mlx.GemvTo's expression (backends/mlx/gemv.go:178-209).
+//     digits, one column of signed bytes per digit (with three, an option for bf16-valued x, the fourth is zero).
+//   * One accumulator tile per block of weights with a common scale (64, 32 or, Q6_K, 16 elements), exact.  A lane has the sums
+//     of two neighbouring digits, d0 + 128 d1, which is a float exactly (Q8_0: rounded once), times 2^(E-26) (or 2^(E-12)),
+//     times the block's scale, added in f32; biases or minima times the group's sum of x are added behind it (mlx.GemvTo,
+//     backends/mlx/gemv.go:178-209; loader/gguf/quant_matrix.go:281-426).  The lanes of a quad meet when an item ends.
 //
-// Pipeline of one CTA (18 warps; persistent over
-// (128-row tile, K range) items; a stage is one 256-element chunk of the tile, or two chunks for
-// the nibble formats when tensor memory has the columns):
-//   TMA producer warp: one bulk copy per stage of the weight's blocks (the tiled layout stores
-//     exactly the shared-memory image of a stage, so every copy is one sequential burst) into a
-//     ring of up to 10 stages guarded by full/empty mbarriers, and one of the stage's B tiles
-//     (the digits of x, laid out for the tensor core by mlx_prep_x_kernel in front of this kernel).
-//     Most products of one or two rows, and of three or four over short K ranges, have no such launch (FUSED, see
-//     launch_with_chunks): the CTA writes the digits of its K range itself, and the tiles stay resident.  The first two stages are asked for at
-//     once, the rest of the ring when the first has landed.
-//   8 converter warps in two groups that take alternate stages, thread = row of the tile:
-//     swizzled LDS.128 -> bytes -> tcgen05.st into a ring of A buffers in TMEM (two to four
-//     deep, as the 512 columns allow).  Both groups follow every stage's barriers.
-//   MMA warp: waits as a warp, one elected lane issues 8 tcgen05.mma (M128 x N x K32, A from
-//     TMEM, B straight from the stage) per chunk and commits to the accumulators', the A
-//     buffer's and the stage's mbarriers.  Q8_0 reads A from the stage as it lies (no converters).
-//   Epilogue warps, two per TMEM lane quarter, each with its share of a
-//     stage's accumulator blocks: tcgen05.ld, scales, running sums in registers; at the end of
-//     an item the parts are added through shared memory and either stored, or (K split) written
-//     to scratch, where the CTA that arrives last adds them in split order (result independent
-//     of arrival order).
-// Every wait is bounded (~2 s): a waiter that gives up records a code in the status word and
-// the CTA winds down (copies drained, TMEM returned) instead of spinning.
+// A CTA: eight warps that compute and one that loads.  A stage is 256 elements of a 128-row tile, one bulk copy (the tiled
+// layouts store exactly the image of a stage) into a ring guarded by full/empty mbarriers; a warp takes its 16 or 32 rows of a
+// stage from ldmatrix to running sums with nobody else.  The activations' digits are made by the CTA itself for its K range
+// while the first stages are on their way, or by a launch in front (see launch_one).  Two CTAs share an SM, or one launch's
+// CTAs and the next one's, whose first stages are then in shared memory before this launch has ended; products that are over
+// in a few stages take an SM each.  Where K is cut, the CTAs of a tile are a cluster and add their sums through its
+// first CTA's shared memory (or through scratch), in split order whoever is first.
+// Every mbarrier wait is bounded (~2 s): a waiter that gives up records a code in the status word and the CTA winds down.
+//
+// Measured (B200, us a call among others, weights from HBM; before: the tcgen05 form, five to eight rows of MLX and Q4_K and four of Q4_K the
+// f16 kernel of qgemm.cu):
+//   one row     MLX4 4096x4096 6.2 -> 4.5, 14336x4096 9.5 -> 7.6, 28672x8192 28.9 -> 22.4; Q4_K 4096x14336 11.5 -> 10.2; Q8_0 28672x8192 43.4 -> 38.7
+//   two rows    MLX4 28672x4096 18.4 -> 13.5, Q8_0 4096x4096 7.3 -> 5.3; four: Q4_K 14336x4096 21.4 -> 14.0, Q6_K 28672x8192 80.6 -> 52.4
+//   eight rows  MLX4 14336x4096 21.6 -> 16.0, Q8_0 28672x8192 101 -> 56, Q6_K 14336x4096 46.3 -> 27.0
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
 
-#include <map>
 #include <mutex>
-#include <tuple>
 
 #include "goph_internal.cuh"
 #include "mlx_mma.cuh"
@@ -58,150 +49,293 @@ namespace goph {
 
 using namespace tc;
 
-namespace {
-
-// Tuning build only (-DGOPH_TUNING): one CTA in the middle of the grid records clock64 at the
-// hand-over points of its first 64 stages; goph_tuning_probe_gemv copies the timeline out.
-#ifdef GOPH_TUNING
-__device__ long long g_mma_trace[8][64];
-#define TP(...) __VA_ARGS__
-#define DBG(bit) (a.dbg & (bit))  // parts of the kernel left out (results are then wrong)
-#else
-#define TP(...)
-#define DBG(bit) 0
-#endif
-
 constexpr int kTileRows = 128;
-constexpr int kChunkK = 256;                  // elements per pipeline stage
-constexpr int kStageMBytes = kTileRows * 16;  // 16 bytes of scales per row and stage (32 for Q6_K, see Fmt)
+constexpr int kChunkK = 256;  // elements of a pipeline stage
 
-// What differs between the weight formats that share this kernel.  A stage is 128 rows x 256
-// elements: the weights as the shared-memory image the tensor core (or the converters) want,
-// then 16 bytes of scale data per row.
-//   MLX4  128 B of nibbles per row (16-byte units XOR-swizzled by row); {scale,bias} bf16 pairs of
-//         the 4 groups of 64.  One accumulator block per group (two K=32 MMAs accumulate).
+// What differs between the weight formats.  A stage is 128 rows x 256 elements, then 16 bytes of scale data per row.
+//   MLX4  128 B of nibbles per row (16-byte units XOR-swizzled by row); {scale,bias} bf16 pairs of the 4 groups of 64.
 //   Q4K   the same nibble image (one 256-element super-block per row and stage); f16 d, f16 dmin and
-//         8 x 12 bits (sc | m << 6).  One accumulator block per 32-element sub-block.
-//   Q80   256 signed bytes per row, stored as K-major 8x16-byte core matrices
-//         [K step][K half][row group][row][16 B] so the MMA reads them from shared memory as they
-//         lie — no conversion at all; 8 f16 block scales.  One accumulator block per 32-element block.
-//   Q5K   the 5-bit values written out as 256 unsigned bytes per row at upload (1 byte per weight
-//         on the device instead of 0.69: the price of the tensor-core path), in Q80's order; the
-//         Q4_K header {d, dmin, 8 x (sc | m << 6)}.  One accumulator block per 32-element sub-block.
-//   Q6K   the 6-bit values minus 32 as 256 signed bytes per row (1 byte per weight instead of
-//         0.82), in Q80's order; 16 int8 scales + f16 d per row (32 bytes with padding).  One block
-//         per K step of 32, whose two 16-element scale groups keep their sums apart like Q4_K's
-//         sub-block pairs: the digits of the step's first 16 positions stand in B rows [0, N/2),
-//         those of the last 16 in [N/2, N).
+//         8 x 12 bits (sc | m << 6), one per 32-element sub-block.
+//   Q80   256 signed bytes per row, stored as 8x16-byte matrices [K step][K half][row group][row][16 B]; 8 f16 block scales.
+//   Q5K   the 5-bit values written out as 256 unsigned bytes per row at upload, in Q80's order; the
+//         Q4_K header {d, dmin, 8 x (sc | m << 6)}.
+//   Q6K   the 6-bit values minus 32 as 256 signed bytes per row, in Q80's order; 16 int8 scales, one per 16 elements,
+//         and f16 d per row (32 bytes with padding).
 enum { FMT_MLX4 = 0, FMT_Q4K = 1, FMT_Q80 = 2, FMT_Q5K = 3, FMT_Q6K = 4 };
 template <int FMT>
 struct Fmt {
-  static constexpr bool kConv = FMT == FMT_MLX4 || FMT == FMT_Q4K;  // nibbles -> bytes through TMEM; else the MMA reads the stage's bytes
-  static constexpr bool kHalves = FMT == FMT_Q4K || FMT == FMT_Q6K;  // two scale groups per accumulator block, in the two halves of its columns
-  // accumulator blocks per 256-element chunk.  Q4_K: one block per PAIR of 32-element sub-blocks;
-  // the two sub-blocks keep their sums apart inside the block because the activation digits of
-  // the even sub-block stand in the first half of the B rows (zeros in the odd K steps) and those
-  // of the odd sub-block in the second half: accumulator columns [0, N/2) and [N/2, N)
-  static constexpr int kBlocks = kConv ? 4 : 8;
-  static constexpr int kGroup = FMT == FMT_MLX4 ? 64 : 32;      // elements per entry of the activation tables
-  static constexpr int kStageWBytes = kTileRows * (kConv ? 128 : 256);
-  static constexpr int kMetaRow = FMT == FMT_Q6K ? 32 : 16;     // bytes of scales per row and stage
-  static constexpr int kStageBytes = kStageWBytes + kTileRows * kMetaRow;  // the B tile follows
+  static constexpr bool kNibble = FMT == FMT_MLX4 || FMT == FMT_Q4K;
+  static constexpr bool kSigned = FMT == FMT_Q80 || FMT == FMT_Q6K;  // A bytes
+  static constexpr bool kSums = FMT == FMT_MLX4 || FMT == FMT_Q4K || FMT == FMT_Q5K;  // biases or minima meet the groups' sums of x
+  static constexpr int kGroup = FMT == FMT_MLX4 ? 64 : 32;  // elements of an entry of the activation tables
+  static constexpr int kGroups = kChunkK / kGroup;
+  static constexpr int kStageWBytes = kTileRows * (kNibble ? 128 : 256);
+  static constexpr int kMetaRow = FMT == FMT_Q6K ? 32 : 16;  // bytes of scales per row and stage
+  static constexpr int kStageBytes = kStageWBytes + kTileRows * kMetaRow;
 };
-constexpr int kStageWBytes = Fmt<FMT_MLX4>::kStageWBytes;
-constexpr int kStageBytes = Fmt<FMT_MLX4>::kStageBytes;
 
-constexpr int kConvWarps = 8;
-constexpr int kConvThreads = kConvWarps * 32;
-constexpr int kMmaWarps = 1;  // the whole warp walks the stages, one elected lane issues
-// Epilogue warps per TMEM lane quarter; each takes an equal part of a stage's accumulator blocks.
-// Two for every format.  (Four were tried for Q4_K, whose epilogue is the slowest role of its
-// pipeline, 1300 cycles of arithmetic a stage against 500 for MLX: the eight extra warps made every
-// role slower and the LM-head product went from 66 to 74 us.)
-template <int N, int FMT>
-__host__ __device__ constexpr int epi_parts() {
-  return 2;
+// Prepared activations of a chunk and up to MB rows: B fragments, then tables.
+//   fragments  [pair of K steps][n tile][lane][K step of the pair] x 8 bytes: what mma.m16n8k32 wants of lane 4 n + t (column
+//              n = 4 * row + digit).  One row has four columns only: its tiles are [n 4][t 4], the lanes of columns 4 to 7 read the same.
+//   tables     per row, parity p of the lane (even lanes hold the sums of the two low digits, odd ones of the two high ones) and
+//              group: the group's scale 2^(E-26) (p = 1: times 2^14) and, where biases or minima want it, its sum of x (p = 0: zero).
+//              One row: all eight columns of an accumulator tile hold its four digits, so lanes 0 and 1 of a quad add up the even
+//              blocks and lanes 2 and 3 the odd ones; per p, half of the quad and pair of blocks the table has both scales, the
+//              other half's as zero, and the half's own sum.
+template <int FMT, int MB>
+struct XBlock {
+  typedef Fmt<FMT> F;
+  static constexpr int NT = MB == 1 ? 1 : MB / 2;  // n tiles of eight columns
+  static constexpr int kFrag = MB == 1 ? 1024 : NT * 2048;
+  static constexpr int kPairs = FMT == FMT_Q6K ? F::kGroups : F::kGroups / 2;  // one row: pairs of blocks (Q6_K's are the halves of a group)
+  static constexpr int kEntry = MB == 1 ? (F::kSums ? 4 : 2) : F::kSums ? 2 : 1;  // floats
+  static constexpr int kTab = MB == 1 ? 4 * kPairs * kEntry : MB * 2 * F::kGroups * kEntry;
+  static constexpr int kBytes = kFrag + kTab * 4;
+  static __host__ __device__ __forceinline__ int frag(int step, int n, int t) {
+    if (MB == 1) return (step >> 1) * 256 + (n * 4 + t) * 16 + (step & 1) * 8;
+    return ((step >> 1) * NT + (n >> 3)) * 512 + ((n & 7) * 4 + t) * 16 + (step & 1) * 8;
+  }
+  static __host__ __device__ __forceinline__ int entry(int m, int p, int g) { return ((m * 2 + p) * F::kGroups + g) * kEntry; }     // several rows
+  static __host__ __device__ __forceinline__ int entry1(int p, int half, int pair) { return ((p * 2 + half) * kPairs + pair) * kEntry; }  // one
+};
+
+__device__ __forceinline__ float max_nan(float a, float b) {  // (fmaxf passes over a NaN)
+  float d;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+  return d;
 }
-template <int N, int FMT>
-__host__ __device__ constexpr int mma_threads() {
-  return (kConvWarps + 4 * epi_parts<N, FMT>() + 1 + kMmaWarps) * 32;
+
+// A warp turns the 256 elements of one chunk of activation row m, eight consecutive ones per lane (SPLIT 4: a block of
+// four warps, four lanes to the same eight elements, each of which writes one digit), into the row's part of an XBlock.
+// The digits come from one sum: q + 64 (1 + 128 + 128^2) has d_j + 64 in its j-th seven bits (the top digit has what is
+// left), and a byte pattern d + 64 of seven bits becomes the signed byte.
+// A group with a NaN or an infinity has the scale NaN, which is what every product with it becomes (an integer has neither).
+template <int FMT, int MB, int SPLIT = 1>
+__device__ __forceinline__ void prep_chunk(const float (&v)[8], int lane, unsigned char* xb, int m, int digits) {
+  typedef Fmt<FMT> F;
+  typedef XBlock<FMT, MB> X;
+  constexpr int kLanes = F::kGroup / 8;  // of a group
+  const int qbits = digits == 4 ? 26 : 19;  // |q| <= 2^qbits keeps the top digit within a signed byte
+  float s = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+  float mx = max_nan(max_nan(max_nan(fabsf(v[0]), fabsf(v[1])), max_nan(fabsf(v[2]), fabsf(v[3]))),
+                     max_nan(max_nan(fabsf(v[4]), fabsf(v[5])), max_nan(fabsf(v[6]), fabsf(v[7]))));
+#pragma unroll
+  for (int o = SPLIT; o < kLanes * SPLIT; o <<= 1) {
+    if (F::kSums) s += __shfl_xor_sync(0xffffffffu, s, o);
+    mx = max_nan(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  }
+  int e = (int)((__float_as_uint(mx) >> 23) & 0xFF);  // mx < 2^(e-126)
+  const bool finite = e < 255;
+  if (e < qbits + 2) e = qbits + 2;
+  if (e > 254) e = 254;
+  const int sub = lane % SPLIT;
+  lane /= SPLIT;
+  if (sub == 0 && lane % kLanes == 0) {
+    float* tab = reinterpret_cast<float*>(xb + X::kFrag);
+    const int g = lane / kLanes;
+    const uint32_t f = (uint32_t)(e - 126 - qbits + 127) << 23;  // 2^(E-qbits)
+    const float sc[2] = {__uint_as_float(finite ? f : 0x7FC00000u), __uint_as_float(finite ? f + (14u << 23) : 0x7FC00000u)};
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      if (MB > 1) {
+        float* t = tab + X::entry(m, p, g);
+        t[0] = sc[p];
+        if (F::kSums) t[1] = p ? s : 0.f;
+      } else if (FMT == FMT_Q6K) {
+        *reinterpret_cast<float2*>(tab + X::entry1(p, 0, g)) = make_float2(sc[p], 0.f);
+        *reinterpret_cast<float2*>(tab + X::entry1(p, 1, g)) = make_float2(0.f, sc[p]);
+      } else {
+        const int half = g & 1;
+        float* t = tab + X::entry1(p, half, g >> 1);
+        t[half] = sc[p];
+        if (F::kSums) t[2] = p ? s : 0.f;
+        (tab + X::entry1(p, half ^ 1, g >> 1))[half] = 0.f;
+      }
+    }
+  }
+  const float fi = __uint_as_float((uint32_t)(qbits - (e - 126) + 127) << 23);
+  const uint32_t bias = digits == 4 ? 64u * (1 + 128 + 16384) : 64u * (1 + 128);
+  int q[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) q[i] = (int)((uint32_t)__float2int_rn(v[i] * fi) + bias);
+  auto digit = [&](int d) {
+    uint32_t p[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      auto at = [&](int i) { return (uint32_t)(q[F::kNibble ? 2 * i + h : 4 * h + i] >> (7 * d)); };
+      p[h] = __byte_perm(__byte_perm(at(0), at(1), 0x0040), __byte_perm(at(2), at(3), 0x0040), 0x5410);
+      if (d < digits - 1) {
+        p[h] = (p[h] & 0x7F7F7F7Fu) ^ 0x40404040u;
+        p[h] |= (p[h] & 0x40404040u) << 1;
+      }
+      if (d >= digits) p[h] = 0;
+    }
+    return make_uint2(p[0], p[1]);
+  };
+  const int step = lane >> 2, w = lane & 3;  // the lane's eight positions are 8 w .. 8 w + 7 of the K step
+  auto put = [&](int d, uint2 t) {
+    const int n = m * 4 + d;
+    if (F::kNibble) {  // the nibbles' order: even elements of a packed word, then odd ones
+      *reinterpret_cast<uint2*>(xb + X::frag(step, n, w)) = t;
+    } else {
+      *reinterpret_cast<uint32_t*>(xb + X::frag(step, n, 2 * (w & 1)) + 4 * (w >> 1)) = t.x;
+      *reinterpret_cast<uint32_t*>(xb + X::frag(step, n, 2 * (w & 1) + 1) + 4 * (w >> 1)) = t.y;
+    }
+  };
+  if (SPLIT == 4) {
+    put(sub, digit(sub));
+    return;
+  }
+#pragma unroll
+  for (int d = 0; d < 4; ++d) put(d, digit(d));
 }
-// Stages whose copies are issued at once when a CTA starts.  If every CTA of the grid asked for its
-// whole ring at that moment (tens of MB), the memory system would serve those requests interleaved
-// and the first stage of every CTA would land last, microseconds late; the rest of the ring is
-// asked for when the first stage has arrived.
-constexpr int kFirstStages = 2;
-constexpr int kThreads = mma_threads<8, FMT_MLX4>();  // of the instantiation the allocation-free entry point launches
+__device__ __forceinline__ void load_eight(const float* p, float (&v)[8]) {
+  if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+    const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+  } else {  // callers may hand in x at any float
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = p[i];
+  }
+}
 
+// The launch in front of the product: a block per (activation row, chunk).
+template <int FMT, int MB>
+__global__ void __launch_bounds__(128)
+mlx_prep_x_kernel(const float* __restrict__ x, unsigned char* __restrict__ xb, int in_dim, int digits) {
+  const int nchunks = in_dim / kChunkK, m = blockIdx.x / nchunks, c = blockIdx.x - m * nchunks, lane = threadIdx.x;
+  pdl_launch_dependents();
+  pdl_wait();  // x may be the output of the kernel in front
+  float v[8];
+  load_eight(x + (size_t)m * in_dim + c * kChunkK + lane / 4 * 8, v);
+  prep_chunk<FMT, MB, 4>(v, lane, xb + (size_t)c * XBlock<FMT, MB>::kBytes, m, digits);
+}
 
-}  // namespace
+// ---- the product kernel ----------------------------------------------------------------------------
+
+__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+// D = A * B + C, 16 x 8 x 32 (bytes), s32.
+template <bool SIGNED>
+__device__ __forceinline__ void imma32(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1, int c0, int c1, int c2, int c3) {
+  if (SIGNED)
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c0), "r"(c1), "r"(c2), "r"(c3));
+  else
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c0), "r"(c1), "r"(c2), "r"(c3));
+}
+// D = A * B + C, 16 x 8 x 16.
+__device__ __forceinline__ void imma16(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t b0, int c) {
+  asm("mma.sync.aligned.m16n8k16.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
+      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a0), "r"(a1), "r"(b0), "r"(c));
+}
+// The accumulators start at 1.5 * 2^23 as a float's bits, so that an integer sum v below 2^22 in magnitude comes out as the
+// float 1.5 * 2^23 + v, without a conversion; two digits' sums then meet exactly (both terms are multiples of 128 or below 2^24).
+constexpr int kAcc0 = 0x4B400000;
+constexpr float kAcc0F = 12582912.f;
+__device__ __forceinline__ float digits_sum(int lo, int hi) { return fmaf(__int_as_float(hi), 128.f, -129.f * kAcc0F) + __int_as_float(lo); }
+
+__device__ __forceinline__ float f16_lo(uint32_t w) { return __half2float(__ushort_as_half((unsigned short)(w & 0xFFFFu))); }
+__device__ __forceinline__ float f16_hi(uint32_t w) { return __half2float(__ushort_as_half((unsigned short)(w >> 16))); }
+
+// The scales of a chunk's rows.  K-quants pack them in six bits or multiply them by the super-block's d.  fma(2^23 + field, d,
+// -2^23 d) is the product field * d rounded once, as the reference's dequantisation does.  With one row of x a lane finishes half
+// of its rows' blocks and unpacks those itself; with several a warp's lanes unpack every block once (two lanes a row) and leave
+// {scale, minimum} in shared memory, a row 80 bytes apart, so that eight rows lie in different banks.  (One row, that way: Q4_K
+// 128256x4096 61 us a call, 51 by every lane for itself; two rows, 14336x4096 11.8 and 13.3.)
+template <int FMT, int MB>
+constexpr bool kStaged = MB > 1 && (FMT == FMT_Q4K || FMT == FMT_Q5K || FMT == FMT_Q6K);
+constexpr int kStagedRow = 80;
+
+template <int FMT>
+__device__ __forceinline__ void stage_scales(const unsigned char* st, int row, unsigned char* dst, int lane) {  // 16 rows from `row`
+  const int r = lane >> 1, q = lane & 1;  // this lane: the row's blocks of the chunk's half q
+  const unsigned char* p = st + Fmt<FMT>::kStageWBytes + (row + r) * Fmt<FMT>::kMetaRow;
+  unsigned char* d = dst + r * kStagedRow + 32 * q;
+  float v[8];
+  if (FMT == FMT_Q6K) {  // bytes 8 q .. 8 q + 7
+    const uint2 w = *reinterpret_cast<const uint2*>(p + 8 * q);
+    const float dd = f16_lo(*reinterpret_cast<const uint32_t*>(p + 16));
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = __fmul_rn(dd, __uint_as_float(__byte_perm((k < 4 ? w.x : w.y) ^ 0x80808080u, 0x4B000000u, 0x7440u + (k & 3))) - 8388736.f);
+  } else {
+    const uint4 w = *reinterpret_cast<const uint4*>(p);
+    const float dd = f16_lo(w.x), dm = f16_hi(w.x) * -0.015625f, kd = dd * -8388608.f, km = dm * -8388608.f;
+    const uint32_t lo = q ? __funnelshift_r(w.z, w.w, 16) : w.y, hi = q ? w.w >> 16 : w.z;  // 48 bits
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t f = k == 0 ? lo : k == 1 ? lo >> 12 : k == 2 ? __funnelshift_r(lo, hi, 24) : hi >> 4;
+      v[2 * k] = fmaf(__uint_as_float((f & 63u) | 0x4B000000u), dd, kd);
+      v[2 * k + 1] = fmaf(__uint_as_float((f & 0xFC0u) | 0x4B000000u), dm, km);  // (2^23 + 64 m) * (-dmin / 64) + ...
+    }
+  }
+  *reinterpret_cast<float4*>(d) = make_float4(v[0], v[1], v[2], v[3]);
+  *reinterpret_cast<float4*>(d + 16) = make_float4(v[4], v[5], v[6], v[7]);
+}
+
+// One row of x: what a lane keeps of a row's scale data, and scale and minimum of its block of pair j (bit 24 j + 12 half of the
+// packed fields; Q6_K: byte 2 j + half).
+template <int FMT>
+struct RowScales {
+  uint4 w;
+  float d, kd, m, km;
+  __device__ __forceinline__ void load(const unsigned char* p) {
+    w = *reinterpret_cast<const uint4*>(p);
+    if (FMT == FMT_Q6K) {
+      d = f16_lo(*reinterpret_cast<const uint32_t*>(p + 16));
+      w.x ^= 0x80808080u;
+      w.y ^= 0x80808080u;
+      w.z ^= 0x80808080u;
+      w.w ^= 0x80808080u;
+    } else if (FMT != FMT_Q80) {
+      d = f16_lo(w.x);
+      m = f16_hi(w.x) * -0.015625f;
+      kd = d * -8388608.f;
+      km = m * -8388608.f;
+    }
+  }
+  __device__ __forceinline__ float2 pair(int j, int half) const {
+    if (FMT == FMT_Q80) return make_float2(f16_lo((j == 0 ? w.x : j == 1 ? w.y : j == 2 ? w.z : w.w) >> (16 * half)), 0.f);
+    if (FMT == FMT_Q6K) {
+      const uint32_t b = __byte_perm((j >> 1) == 0 ? w.x : (j >> 1) == 1 ? w.y : (j >> 1) == 2 ? w.z : w.w, 0x4B000000u, 0x7440u + 2 * (j & 1) + half);
+      return make_float2(__fmul_rn(d, __uint_as_float(b) - 8388736.f), 0.f);
+    }
+    const int sh = 12 * half;
+    const uint32_t f = j == 0 ? w.y >> sh : j == 1 ? __funnelshift_r(w.y, w.z, 24) >> sh : j == 2 ? __funnelshift_r(w.z, w.w, 16) >> sh : w.w >> (sh + 8);
+    return make_float2(fmaf(__uint_as_float((f & 63u) | 0x4B000000u), d, kd), fmaf(__uint_as_float((f & 0xFC0u) | 0x4B000000u), m, km));
+  }
+};
 
 struct MmaArgs {
   const unsigned char* w;  // tiled weight blocks [tile][chunk]
   const float* x;          // [batch][in_dim]
-  const unsigned char* xb; // prepared B operand: [chunk][N rows x 256 bytes], canonical K-major core matrices
-  const float* xtab;       // prepared tables: [batch][groups] sum of x, then [batch][groups] 2^(E-QBITS)
+  const unsigned char* xb; // prepared activations: an XBlock per chunk
   float* out;              // [batch][out_dim]
   int* status;             // device word: 0 ok, otherwise the first wait that gave up
-  float* scratch;          // split-K partial sums [item][batch][128]
-  unsigned int* counters;  // per-tile arrival counters, zero between launches
+  float* scratch;          // split-K partial sums [item][warp][value][lane]
+  unsigned int* counters;  // arrival counters per tile and warp, zero between launches
   int out_dim, in_dim;
   int batch;               // activation rows of this launch (<= MB of the instantiation)
+  int digits;
   int ntiles;              // ceil(out_dim / 128)
   int nchunks;             // in_dim / 256
   int splits;              // CTAs sharing the K range of one tile
   int items;               // ntiles * splits
   int stages;              // depth of the shared-memory ring
-  int cmax;                // FUSED: most chunks an item has (resident B tiles)
-  int dbg;                 // tuning build only
-  // 1: the CTAs that share a tile (one per K split) form a thread-block cluster, every CTA has
-  // exactly one item, and the partial sums travel through the shared memory of the cluster's first
-  // CTA instead of global scratch and an atomic counter
-  int cluster;
-  // Grouped launches (the selected experts of a mixture-of-experts layer): the items are the 128-row
-  // tiles of `gmats` matrices of each live work entry, every entry with its own weights, prepared
-  // activations, tables and result rows; no K split.  batch is the instantiation's MB, out_dim the
-  // pitch of a result row (gmats matrices of gtpe * 128 rows side by side).
+  int cmax;                // FUSED: most chunks an item has (resident XBlocks)
+  int cluster;             // the CTAs of a tile are a cluster and have one item each
   const MmaGroupEntry* gwork;
-  const int* gcount;  // live entries (device memory, written by the kernel that routed the tokens)
-  int gmax;           // entries the launch was sized for
-  int gtpe;           // 128-row tiles per matrix
-  int gmats;          // matrices per entry
-  int gfirst;         // the first of them in MmaGroupEntry::w
-  int gdirect;        // result row of activation m: 0 -> entry * MB + m, 1 -> the entry's item[m]
-  int gtab;           // floats of tables per entry
-  size_t gxb;         // bytes of prepared B operand per entry
+  const int* gcount;
+  int gmax, gtpe, gmats, gfirst, gdirect;
+  size_t gxb;
 };
 
-// Shared-memory plan (dynamic, 1024-byte aligned base): ring of stages (weights then meta),
-// 2 B tiles (8 K-steps x N rows x 32 bytes), per-(row,group) tables {sum x, 2^(E-26), 2^(26-E)},
-// mbarriers, the TMEM base holder.
-// FUSED: the activation digits are made by the kernel itself, for the K range of the CTA's items
-// only (at most `cmax` chunks), and stay resident after the ring instead of travelling with every
-// stage.
-// C: chunks of 256 elements per stage.  The nibble formats take two: what a stage costs every role
-// in waits, fences and arrivals is then paid once per 36 KiB instead of once per 18 KiB.  A stage's
-// layout is [C weight blocks][C B tiles].
-// Rows of 128 partial sums the first CTA of a cluster can receive: (splits - 1) x activation rows.
-constexpr int kClusterRecvRows = 7;
-
-template <int N, int FMT = FMT_MLX4, bool FUSED = false, int C = 1>
-struct MmaSmem {
-  static constexpr int kBTileBytes = 8 * N * 32;  // 256 K-bytes for each of N rows
-  static constexpr int kStage = C * (Fmt<FMT>::kStageBytes + (FUSED ? 0 : kBTileBytes));
-  static __host__ __device__ size_t bytes(int stages, int batch, int in_dim, int cmax = 0) {
-    return (size_t)stages * kStage + (FUSED ? (size_t)cmax * kBTileBytes : 0) +
-           (size_t)batch * (in_dim / Fmt<FMT>::kGroup) * 8 + 1024 + 512 + 8 * kTileRows * 4 + kClusterRecvRows * kTileRows * 4;
-  }
-};
-
-// Walks the (tile, chunk) stages of this CTA's work items in the order every role uses.
-// G (grouped launches): the CTA takes one contiguous range of the live items, so that it stays with
-// one entry's activations for several tiles; item w = (entry, matrix, tile of the matrix).
 template <bool G, bool WORK = false>
 struct StageWalkT {
   int w, tile, split, c, c1;
-  int cps;  // chunks per stage
   int wend, entry, mat;  // G only
   __device__ __forceinline__ void open(const MmaArgs& a) {
     if (G) {
@@ -224,8 +358,7 @@ struct StageWalkT {
       c1 = (split + 1) * a.nchunks / a.splits;
     }
   }
-  __device__ __forceinline__ StageWalkT(const MmaArgs& a, int chunks_per_stage = 1, int live_items = 0)
-      : w(blockIdx.x), cps(chunks_per_stage) {
+  __device__ __forceinline__ StageWalkT(const MmaArgs& a, int live_items = 0) : w(blockIdx.x) {
     if (G) {
       const int each = WORK && a.gdirect == 2 ? 2 : 1;  // (whole pairs)
       w = (int)((long long)blockIdx.x * (live_items / each) / gridDim.x) * each;
@@ -234,245 +367,83 @@ struct StageWalkT {
     if (live(a)) open(a);
   }
   __device__ __forceinline__ bool live(const MmaArgs& a) const { return G ? w < wend : w < a.items; }
-  // chunks of the current stage (an item with an odd number of chunks ends on a stage of one)
-  __device__ __forceinline__ int nc() const { return c1 - c < cps ? c1 - c : cps; }
-  __device__ __forceinline__ bool last_chunk() const { return c + nc() == c1; }
-  __device__ __forceinline__ void next(const MmaArgs& a) {
-    c += nc();
-    if (c == c1) {
-      w += G ? 1 : gridDim.x;
-      if (live(a)) open(a);
-    }
+  __device__ __forceinline__ void next_item(const MmaArgs& a) {
+    w += G ? 1 : gridDim.x;
+    if (live(a)) open(a);
   }
 };
 
-// ---- activation preparation -----------------------------------------------------------------
-// A warp turns the 256 elements of one chunk of activation row m, eight consecutive ones per lane (SPLIT 4: a block of
-// four warps, four lanes to the same eight elements, each of which writes one digit), into group sums, power-of-two scales and the base-128 digits of every element, written where the tensor core expects them:
-// chunk (256 K) -> K-step (32) -> half (16 bytes) -> 8-row core matrix -> row -> byte.  The lane's eight digits of a place
-// are eight consecutive bytes of one B row.  The digits come from one sum: q + 64 (1 + 128 + 128^2) has d_j + 64 in
-// its j-th seven bits (the top digit has what is left), and a byte pattern d + 64 of seven bits becomes the signed byte.
-// sums, scales: the row's tables at the chunk.  tile: the chunk's B tile of N rows.
-// G32: sums and scales per 32 elements instead of per 64.  NATURAL: the B bytes of a K step in element order (for A operands
-// that lie in memory in element order) instead of the order the nibble converters produce (of a packed word: 0 2 4 6, 1 3 5 7).
-// A group with a NaN or an infinity has the scale NaN, which is what every product with it becomes (an integer has neither).
-// (An element per thread, ten shuffles and four byte stores each, took four times the instructions: the preparation of
-// 4096 elements by the product's own CTAs cost more than a launch in front, see launch_with_chunks.)
-__device__ __forceinline__ float max_nan(float a, float b) {  // (fmaxf passes over a NaN)
-  float d;
-  asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
-  return d;
-}
-template <int DIGITS, bool G32, bool NATURAL, bool PAIRH, int SPLIT = 1>
-__device__ __forceinline__ void prep_chunk(const float (&v)[8], int lane, unsigned char* tile, int N, int m, float* sums, float* scales) {
-  constexpr int QBITS = DIGITS == 4 ? 26 : 19;  // |q| <= 2^QBITS keeps the top digit within a signed byte
-  constexpr bool PAIRED = G32 && !NATURAL;      // Q4_K: see Fmt::kHalves
-  constexpr int kLanes = G32 ? 4 : 8;           // of a group
-  float s = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
-  float mx = max_nan(max_nan(max_nan(fabsf(v[0]), fabsf(v[1])), max_nan(fabsf(v[2]), fabsf(v[3]))),
-                     max_nan(max_nan(fabsf(v[4]), fabsf(v[5])), max_nan(fabsf(v[6]), fabsf(v[7]))));
-#pragma unroll
-  for (int o = SPLIT; o < kLanes * SPLIT; o <<= 1) {
-    s += __shfl_xor_sync(0xffffffffu, s, o);
-    mx = max_nan(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  }
-  int e = (int)((__float_as_uint(mx) >> 23) & 0xFF);  // mx < 2^(e-126)
-  const bool finite = e < 255;
-  if (e < QBITS + 2) e = QBITS + 2;
-  if (e > 254) e = 254;
-  const int sub = lane % SPLIT;
-  lane /= SPLIT;
-  if (sub == 0 && lane % kLanes == 0) {
-    sums[lane / kLanes] = s;
-    scales[lane / kLanes] = __uint_as_float(finite ? (uint32_t)(e - 126 - QBITS + 127) << 23 : 0x7FC00000u);  // 2^(E-QBITS), NaN
-  }
-  const float fi = __uint_as_float((uint32_t)(QBITS - (e - 126) + 127) << 23);
-  int q[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) q[i] = (int)((uint32_t)__float2int_rn(v[i] * fi) + (DIGITS == 4 ? 64u * (1 + 128 + 16384) : 64u * (1 + 128)));
-  auto digit = [&](int d) {
-    uint32_t p[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      auto at = [&](int i) { return (uint32_t)(q[NATURAL ? 4 * h + i : 2 * i + h] >> (7 * d)); };
-      p[h] = __byte_perm(__byte_perm(at(0), at(1), 0x0040), __byte_perm(at(2), at(3), 0x0040), 0x5410);
-      if (d < DIGITS - 1) {
-        p[h] = (p[h] & 0x7F7F7F7Fu) ^ 0x40404040u;
-        p[h] |= (p[h] & 0x40404040u) << 1;
-      }
-    }
-    return make_uint2(p[0], p[1]);
-  };
-  const int step = lane >> 2, w = lane & 3;  // the lane's eight positions are 8 w .. 8 w + 7 of the K step
-  unsigned char* dst = tile + step * (N * 32) + (w >> 1) * ((N / 8) * 128) + 8 * (w & 1);
-  const bool second = PAIRH ? w >= 2 : (step & 1) != 0;  // halves: Q6_K by the half of the step, Q4_K by the step
-  auto put = [&](int d, uint2 t) {
-    int n = m * DIGITS + d;
-    if (PAIRED || PAIRH) {  // the other scale group's half of the rows holds zeros at this K position
-      const int other = n + (second ? 0 : N / 2);
-      n += second ? N / 2 : 0;
-      *reinterpret_cast<uint2*>(dst + (other >> 3) * 128 + (other & 7) * 16) = make_uint2(0, 0);
-    }
-    *reinterpret_cast<uint2*>(dst + (n >> 3) * 128 + (n & 7) * 16) = t;
-  };
-  if (SPLIT == 4) {
-    if (sub < DIGITS) put(sub, digit(sub));
-    return;
-  }
-  uint2 dig[DIGITS];
-#pragma unroll
-  for (int d = 0; d < DIGITS; ++d) dig[d] = digit(d);
-#pragma unroll
-  for (int i = 0; i < DIGITS; ++i) {
-    if (DIGITS == 4) {  // (lanes take turns at the places: their addresses are multiples of 128 bytes apart)
-      const int d = (i + step) & 3;
-      put(d, d == 0 ? dig[0] : d == 1 ? dig[1] : d == 2 ? dig[2] : dig[DIGITS - 1]);
-    } else {
-      put(i, dig[i]);
-    }
-  }
-}
-__device__ __forceinline__ void load_eight(const float* p, float (&v)[8]) {
-  if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
-    const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-  } else {  // callers may hand in x at any float
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = p[i];
-  }
-}
+constexpr int kConsumers = 8;  // warps; the ninth loads
+constexpr int kMaxStages = 12, kMaxSplits = 8;
+constexpr int kThreads = (kConsumers + 1) * 32;
 
-// The launch in front of the product: a block per (activation row, chunk).  (A warp per chunk, a fourth of the threads:
-// 0.3 to 0.5 us slower.)
-template <int DIGITS, bool G32 = false, bool NATURAL = false, bool PAIRH = false>
-__global__ void __launch_bounds__(128)
-mlx_prep_x_kernel(const float* __restrict__ x, unsigned char* __restrict__ xb, float* __restrict__ xtab, int batch,
-                  int in_dim, int N) {
-  constexpr int kPer = G32 ? 8 : 4;  // table entries of a chunk
-  const int nchunks = in_dim / kChunkK, ntab = nchunks * kPer;
-  const int m = blockIdx.x / nchunks, c = blockIdx.x - m * nchunks, lane = threadIdx.x;
-  pdl_launch_dependents();
-  pdl_wait();  // x may be the output of the kernel in front
-  float v[8];
-  load_eight(x + (size_t)m * in_dim + c * kChunkK + lane / 4 * 8, v);
-  prep_chunk<DIGITS, G32, NATURAL, PAIRH, 4>(v, lane, xb + (size_t)c * (N * 256), N, m, xtab + m * ntab + c * kPer, xtab + (batch + m) * ntab + c * kPer);
-}
-
-// The same done by a CTA of the product kernel for itself (all warps but the producer's, before they take up their roles):
-// digits into the resident B tiles in shared memory, sums and scales into the tables the epilogue reads.
-template <int DIGITS, bool G32, bool NATURAL, int N, bool PAIRH = false>
-__device__ __forceinline__ void prep_x_in_cta(const float* __restrict__ x, int batch, int in_dim, unsigned char* bres,
-                                              float* xsum, float* xfs, int warp, int lane, int nwarps, int cbegin, int cend) {
-  constexpr int kPer = G32 ? 8 : 4;
-  const int ntab = in_dim / kChunkK * kPer, n = cend - cbegin;
-  if (batch * n * 4 <= nwarps) {  // short ranges: four warps to a chunk
-    const int i = warp >> 2, l = (warp & 3) * 32 + lane;
-    if (i < batch * n) {
-      const int m = i / n, c = cbegin + (i - m * n), ti = m * ntab + c * kPer;
-      float v[8];
-      load_eight(x + (size_t)m * in_dim + c * kChunkK + l / 4 * 8, v);
-      prep_chunk<DIGITS, G32, NATURAL, PAIRH, 4>(v, l, bres + (size_t)(c - cbegin) * (N * 256), N, m, xsum + ti, xfs + ti);
-    }
-    return;
+template <int FMT, int MB, bool G>
+struct RowCfg {
+  // Sixteen rows a warp, or 32 with the warps in two groups that take turns at the stages: fragments of several n tiles are
+  // read from shared memory half as often.
+  #ifdef RM_SL2
+  static constexpr int SL = 2, KG = SL;
+#else
+  static constexpr int SL = MB >= 4 || G ? 2 : 1, KG = SL;
+#endif
+  static constexpr int NT = XBlock<FMT, MB>::NT;
+  static constexpr int kVals = SL * NT;                      // values a lane has of an item
+  static constexpr int kStoring = kConsumers / KG;           // warps that finish items
+  static constexpr int kPair = KG == 2 ? 2 * kStoring * kVals * 128 : 0;
+  static constexpr int kRecv = kStoring * kVals * 128;       // a split's sums
+  static constexpr int kScales = kStaged<FMT, MB> ? kConsumers * SL * 16 * kStagedRow : 0;
+};
+template <int FMT, int MB, bool FUSED, bool G>
+struct RowSmem {
+  static constexpr int kStage = Fmt<FMT>::kStageBytes + (FUSED ? 0 : XBlock<FMT, MB>::kBytes);
+  static __host__ __device__ size_t bytes(int stages, int cmax, int recv) {
+    return (size_t)stages * kStage + (FUSED ? (size_t)cmax * XBlock<FMT, MB>::kBytes : 0) + RowCfg<FMT, MB, G>::kPair + RowCfg<FMT, MB, G>::kScales + (size_t)recv * RowCfg<FMT, MB, G>::kRecv + 512;
   }
-#pragma unroll 1
-  for (int i = warp; i < batch * n; i += nwarps) {
-    const int m = i / n, c = cbegin + (i - m * n), ti = m * ntab + c * kPer;
-    float v[8];
-    load_eight(x + (size_t)m * in_dim + c * kChunkK + lane * 8, v);
-    prep_chunk<DIGITS, G32, NATURAL, PAIRH>(v, lane, bres + (size_t)(c - cbegin) * (N * 256), N, m, xsum + ti, xfs + ti);
+  // Depth of the ring that `budget` leaves room for.
+  static int stages(size_t budget, int cmax, int recv) {
+    const size_t fixed = bytes(0, cmax, recv);
+    int n = fixed < budget ? (int)((budget - fixed) / kStage) : 0;
+    if (n > kMaxStages) n = kMaxStages;
+    return RowCfg<FMT, MB, G>::KG == 2 ? n & ~1 : n;  // (a group must see every round of its slots)
   }
-}
+};
 
-// N: B rows (accumulator columns) per group block; DIGITS: base-128 digits per activation;
-// MB: activation rows the instantiation can take (MB * DIGITS <= N).
-template <int N, int DIGITS, int MB, int FMT = FMT_MLX4, bool FUSED = false, int C = 1, bool G = false>
-__global__ void __launch_bounds__((mma_threads<N, FMT>()), 1)
+template <int FMT, int MB, bool FUSED, bool G = false>
+__global__ void __launch_bounds__(kThreads, 2)
 mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
   static_assert(!G || !FUSED, "grouped launches: activations prepared in front");
   constexpr bool kWork = G && FMT != FMT_MLX4;  // a work list's entries (MmaWorkEntry)
-  TP(const long long t_entry = clock64();)
   typedef StageWalkT<G, kWork> StageWalk;
-  constexpr int EP = epi_parts<N, FMT>();
-  constexpr bool kSpills = !Fmt<FMT>::kConv && MB == 8;  // a byte per weight, eight rows: the epilogue is short of registers
-  constexpr int kEpiWarps = 4 * EP, kEpiThreads = kEpiWarps * 32;
-  constexpr int kWarpTMA = kConvWarps + kEpiWarps, kWarpMMA = kWarpTMA + 1;
-  constexpr int kThreads = mma_threads<N, FMT>();
-  static_assert(MB * DIGITS * (Fmt<FMT>::kHalves ? 2 : 1) <= N, "the digits of the activation rows must fit the N columns");
-  static_assert(N == 8 || N == 16 || N == 32, "accumulator blocks of 8, 16 or 32 columns");
   typedef Fmt<FMT> F;
-  constexpr int kBlocks = F::kBlocks;
-  constexpr int kACols = F::kConv ? 64 * C : 0;  // TMEM columns of one A buffer (a stage)
-  constexpr int kDCols = C * kBlocks * N;        // accumulator columns of a stage
-  // Depths of the A ring and of the accumulator ring in TMEM (512 columns).  A third A buffer lets
-  // the converters start stage i+2 while the MMAs of stage i still run; where the columns do not
-  // allow four of each, the accumulators, which the epilogue drains quickly, get the shallower ring.
-  constexpr int NA = (kACols + kDCols) * 4 <= 512 ? 4 : (3 * kACols + 2 * kDCols <= 512 ? 3 : 2);
-  constexpr int ND = (kACols + kDCols) * 4 <= 512 ? 4 : 2;
-  static_assert(NA * kACols + ND * kDCols <= 512, "TMEM plan");
-  static_assert(C == 1 || F::kConv, "two chunks per stage are for the formats that convert");
-  constexpr uint32_t kCols = 512;
-  constexpr int kStage = MmaSmem<N, FMT, FUSED, C>::kStage;
-  constexpr int kStageBytes = F::kStageBytes, kStageWBytes = F::kStageWBytes;
-  constexpr int kBTileBytes = MmaSmem<N, FMT, FUSED, C>::kBTileBytes;
-  constexpr int kStageLoad = kStageBytes + (FUSED ? 0 : kBTileBytes);  // bytes a chunk brings into a stage
-  extern __shared__ unsigned char smem_dyn[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
+  typedef XBlock<FMT, MB> X;
+  typedef RowCfg<FMT, MB, G> C;
+  typedef RowSmem<FMT, MB, FUSED, G> M;
+  constexpr int SL = C::SL, KG = C::KG, NT = C::NT, kStage = M::kStage;
+  // A chunk is summed by itself where its terms, products and biases or minima that cancel, meet a small sum.
+  constexpr bool kByChunk = F::kSums && !(FMT == FMT_MLX4 && MB == 8);
+  extern __shared__ __align__(128) unsigned char smem_dyn[];
   const int S = a.stages;
-  unsigned char* ring = smem;
-  const int groups = a.in_dim / F::kGroup;
-  unsigned char* bres = ring + (size_t)S * kStage;  // FUSED: resident B tiles of every chunk
-  float* xsum = reinterpret_cast<float*>(bres + (FUSED ? (size_t)a.cmax * kBTileBytes : 0));  // [batch][groups] sum of x
-  float* xfs = xsum + (size_t)a.batch * groups;                        // [batch][groups] 2^(E-QBITS)
-  uint64_t* bars = reinterpret_cast<uint64_t*>((reinterpret_cast<uintptr_t>(xfs + (size_t)a.batch * groups) + 15) & ~uintptr_t(15));
-  // bars: full[S], empty[S], a_ready[NA], a_free[NA], d_full[ND], d_free[ND], cluster
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 2 * S + 2 * NA + 2 * ND + 1);
-  volatile int* last_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
-  float* pair = reinterpret_cast<float*>(tmem_holder + 4);  // [EP-1][MB][128]: the sums of an item from the epilogue parts above 0
-  static_assert((EP - 1) * MB <= 8, "room for the parts' sums");
-  float* recv = pair + 8 * kTileRows;  // [splits-1][MB][128]: partial sums from the cluster's other CTAs (first CTA only)
-
-  // (the shuffle tells the compiler that a warp's number is the same in all of its lanes: what follows from it is
-  // kept in uniform registers, from where the MMAs take their operands.  MLX4 28672x4096 17.6 us without, 16.7
-  // with, Q4_K 4096x14336 12.7 and 12.0.  kSpills: there the cursor and the uniform numbers only cost spills,
-  // Q8_0 14336x4096 x5 32.3 us with and 28.2 without, 4096x14336 x6 37.1 and 32.8)
-  const int tid = threadIdx.x, warp = kSpills ? tid >> 5 : __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-  const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + S);
-  const uint32_t aready0 = smem_u32(bars + 2 * S), afree0 = aready0 + 8 * NA;
-  const uint32_t mdone0 = afree0 + 8 * NA, dfree0 = mdone0 + 8 * ND;  // mdone: a stage's accumulators are complete
-  const uint32_t clbar = dfree0 + 8 * ND;  // cluster launches: the other CTAs' partial sums have arrived (one arrival per warp)
+  unsigned char* ring = smem_dyn;
+  unsigned char* bres = ring + (size_t)S * kStage;
+  unsigned char* scales = bres + (FUSED ? (size_t)a.cmax * X::kBytes : 0);
+  float* pair = reinterpret_cast<float*>(scales + C::kScales);
+  float* recv = pair + C::kPair / 4;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(recv) + (a.cluster ? (size_t)(a.splits - 1) * C::kRecv : 0));
+  volatile int* gave_up = reinterpret_cast<volatile int*>(bars + 2 * S);
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * S;
 
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
       mbar_init(full0 + 8 * s, 1);
-      // converters (conversion formats), epilogue (scale data), MMA commit (B tile, A read from the stage)
-      // (one arrival per warp: a warp's lanes meet first and one of them arrives for all)
-      mbar_init(empty0 + 8 * s, (F::kConv ? kConvWarps / 2 : 0) + kEpiWarps + 1);
+      mbar_init(empty0 + 8 * s, kConsumers / KG);
     }
-    for (int b = 0; b < NA; ++b) {
-      mbar_init(aready0 + 8 * b, kConvWarps);
-      mbar_init(afree0 + 8 * b, 1);
-    }
-    for (int b = 0; b < ND; ++b) {
-      mbar_init(mdone0 + 8 * b, 1);
-      mbar_init(dfree0 + 8 * b, kEpiWarps);
-    }
-    if (a.cluster) mbar_init(clbar, 4 * (a.splits - 1));
+    for (int s = 0; s < 9; ++s) gave_up[s] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == kWarpMMA) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_holder)), "r"(kCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  if (!G) pdl_launch_dependents();  // (grouped: the small kernels behind it gain nothing; the 8-token MoE layer 62.3 us with it, 61.3 without)
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  if (!G) pdl_launch_dependents();
   __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (a.cluster) cluster_sync_all();  // the first CTA's barrier is initialised before any peer can arrive on it
-  const uint32_t tmem_base = *tmem_holder;
-  const uint32_t tmemA0 = tmem_base, tmemD0 = tmem_base + NA * kACols;  // A: NA x kACols; D: ND x kDCols
+  if (a.cluster) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // (waited for before the first store to a peer: it has started)
   bool ok = true;
   int gitems = 0;
   if (G) {
@@ -481,529 +452,495 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
     if (n > a.gmax) n = a.gmax;
     gitems = n * a.gtpe * a.gmats;
   }
-  StageWalk sw(a, C, gitems);
+  StageWalk sw(a, gitems);
   auto entry_at = [&](int e) -> const MmaGroupEntry* {
     return kWork ? &reinterpret_cast<const MmaWorkEntry*>(a.gwork)[e].g : a.gwork + e;
   };
-  // where a stage's weights and prepared activations lie
-  auto wsrc = [&](const StageWalk& s) {
-    const unsigned char* base = a.w;
-    if (G) base = reinterpret_cast<const unsigned char*>(__ldg(reinterpret_cast<const unsigned long long*>(&entry_at(s.entry)->w[a.gfirst + s.mat])));
-    return base + ((size_t)s.tile * a.nchunks + s.c) * kStageBytes;
-  };
-  auto bsrc = [&](const StageWalk& s) { return a.xb + (G ? (size_t)s.entry * a.gxb : 0) + (size_t)s.c * kBTileBytes; };
-  TP(const bool tr = blockIdx.x == gridDim.x / 2 && (!(a.dbg & 8) || a.gmats == 2); if (tr && tid == 0) { g_mma_trace[7][0] = clock64(); g_mma_trace[7][3] = t_entry; })
   const int cbase = sw.live(a) ? sw.c : 0;  // first chunk of this CTA's K range
+  float fin[C::kVals];                      // the item's values (cluster: kept for the exchange)
+  bool have = false;
 
-  if (FUSED && warp != kWarpTMA) {
-    // The producer is off to its ring (the weights do not depend on the kernel in front); the other warps turn the
-    // activations into digits, sums and scales.
-    static_assert(kWarpMMA == kWarpTMA + 1 && kWarpMMA == kThreads / 32 - 1, "the MMA warp is the last, behind the producer");
-    pdl_wait();
-    // every item of this CTA covers the same K range (the grid is a multiple of the K splits)
-    if (sw.live(a))
-      prep_x_in_cta<DIGITS, FMT != FMT_MLX4, !F::kConv, N, FMT == FMT_Q6K>(a.x, a.batch, a.in_dim, bres, xsum, xfs, warp == kWarpMMA ? kWarpTMA : warp, lane,
-                                                                           kThreads / 32 - 1, sw.c, sw.c1);
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the MMA reads the digits through the async proxy
-    asm volatile("bar.sync 2, %0;" ::"n"(kThreads - 32) : "memory");
-  }
-
-  if (warp == kWarpTMA) {
-    // ------------------------------------------------------------------ TMA producer
+  if (warp == kConsumers) {
+    // ------------------------------------------------------------------ producer
     if (lane == 0) {
-      // The weights do not depend on the kernel in front: fill the ring with them first, then
-      // wait for the activation digits and add the B tiles of those stages.
+      auto wsrc = [&](const StageWalk& s, int c) {
+        const unsigned char* base = a.w;
+        if (G) base = reinterpret_cast<const unsigned char*>(__ldg(reinterpret_cast<const unsigned long long*>(&entry_at(s.entry)->w[a.gfirst + s.mat])));
+        return base + ((size_t)s.tile * a.nchunks + c) * F::kStageBytes;
+      };
+      auto bsrc = [&](const StageWalk& s, int c) { return a.xb + (G ? (size_t)s.entry * a.gxb : 0) + (size_t)c * X::kBytes; };
+      // The weights do not depend on the kernel in front: the ring is filled with them first, the activations of those
+      // stages follow when they are there.
+      RingCursor rc;
       int i = 0;
-      StageWalk sw0 = sw;
-      for (; i < S && i < kFirstStages && sw0.live(a); ++i, sw0.next(a)) {
-        uint32_t dst = smem_u32(ring + (size_t)i * kStage);
-        mbar_expect_tx(full0 + 8 * i, sw0.nc() * kStageLoad);
-        bulk_load_1d(dst, wsrc(sw0), sw0.nc() * kStageBytes, full0 + 8 * i);
-      }
-      if (FUSED) {
-        sw = sw0;
-      } else {
+      bool waited = FUSED || G;
+      StageWalk sx = sw;  // the first stage whose activations have not been asked for
+      int xc = sx.c, xi = 0;
+      auto catch_up = [&] {
         pdl_wait();
-        for (int j = 0; j < i; ++j, sw.next(a))
-          bulk_load_1d(smem_u32(ring + (size_t)j * kStage) + C * kStageBytes, bsrc(sw), sw.nc() * kBTileBytes, full0 + 8 * j);
-      }
-      RingCursor rc;
-      for (int j = 0; j < i; ++j) rc.next(S);
-      for (; sw.live(a) && ok; ++i, sw.next(a), rc.next(S)) {
-        const int slot = rc.s;
-        if (i >= S) ok = mbar_wait(empty0 + 8 * slot, rc.ph ^ 1u, a.status, 1);
-        else if (i == kFirstStages) ok = mbar_wait(full0, 0, a.status, 11);  // the first stage is in: the rest of the ring may follow
-        if (!ok) break;
-        uint32_t dst = smem_u32(ring + (size_t)slot * kStage);
-        mbar_expect_tx(full0 + 8 * slot, sw.nc() * kStageLoad);
-        bulk_load_1d(dst, wsrc(sw), sw.nc() * kStageBytes, full0 + 8 * slot);
-        if (!FUSED) bulk_load_1d(dst + C * kStageBytes, bsrc(sw), sw.nc() * kBTileBytes, full0 + 8 * slot);
-        TP(if (tr && i < 64) g_mma_trace[0][i] = clock64();)
-      }
-    }
-  } else if (warp >= kWarpMMA) {
-    // ------------------------------------------------------------------ MMA issuers
-    // The whole warp walks its stages and waits; one elected lane issues.  (What the instructions
-    // need is the same in all lanes and can live in uniform registers, which roughly halves the
-    // cycles an issue costs against a single diverged thread.)
-    {
-      // instruction descriptor: D s32, A u8 (nibbles) or s8 (Q8_0 bytes), B s8, both K-major, N, M=128
-      const uint32_t idesc = (2u << 4) | (((FMT == FMT_Q80 || FMT == FMT_Q6K) ? 1u : 0u) << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((128u >> 4) << 24);
-      // A from shared memory (Q8_0): K-adjacent core matrices 16 row groups apart, row groups 128 B apart
-      const uint64_t adesc_hi = ((uint64_t)(2048u >> 4) << 16) | ((uint64_t)(128u >> 4) << 32) | (1ull << 46);
-      constexpr uint32_t kLBO = (N / 8) * 128, kSBO = 128;  // K-adjacent / N-adjacent core matrices
-      const uint64_t desc_hi = ((uint64_t)(kLBO >> 4) << 16) | ((uint64_t)(kSBO >> 4) << 32) | (1ull << 46);
-      // Every role sees every stage in order, so no barrier phase is ever skipped (a parity wait
-      // can only tell the current phase from the one before it).
-      RingCursor rc;
-      for (int i = 0; sw.live(a) && ok; ++i, rc.next(S)) {
-        const int ba = i % NA, b = i % ND, slot = rc.s;
-        ok = mbar_wait(full0 + 8 * slot, rc.ph, a.status, 8);
-        if (ok && F::kConv) ok = mbar_wait(aready0 + 8 * ba, (i / NA) & 1, a.status, 2);
-        if (ok && i >= ND) ok = mbar_wait(dfree0 + 8 * b, ((i - ND) / ND) & 1, a.status, 5);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        TP(if (tr && lane == 0 && i < 64) g_mma_trace[1][i] = clock64();)
-        const int nc = sw.nc();
-        if (elect_one()) {
-#pragma unroll
-        for (int cc = 0; cc < C; ++cc) {
-          if (cc < nc) {
-            const uint32_t bbase = FUSED ? smem_u32(bres + (size_t)(sw.c - cbase + cc) * kBTileBytes)
-                                         : smem_u32(ring + (size_t)slot * kStage + C * kStageBytes + cc * kBTileBytes);
-            const uint32_t dcol = tmemD0 + b * kDCols + cc * (kBlocks * N), acol = tmemA0 + ba * kACols + cc * 64;
-#pragma unroll
-            for (int step = 0; step < 8; ++step) {  // K = 32 per step
-              const uint64_t bdesc = desc_hi | (uint64_t)(((bbase + step * (N * 32)) >> 4) & 0x3FFF);
-              if (F::kConv) {  // two steps accumulate into the block of their 64 elements
-                umma_i8_ts(dcol + (step >> 1) * N, acol + step * 8, bdesc, idesc, step & 1);
-              } else {
-                const uint32_t abase = smem_u32(ring + (size_t)slot * kStage) + step * 4096;
-                umma_i8_ss(dcol + step * N, adesc_hi | (uint64_t)((abase >> 4) & 0x3FFF), bdesc, idesc, 0);
-              }
-            }
+        waited = true;
+        for (; xi < i; ++xi) {
+          bulk_load_1d(smem_u32(ring + (size_t)xi * kStage) + F::kStageBytes, bsrc(sx, xc), X::kBytes, full0 + 8 * xi);
+          if (++xc == sx.c1) {
+            sx.next_item(a);
+            xc = sx.c;
           }
         }
-        umma_commit(mdone0 + 8 * b);
-        if (F::kConv) umma_commit(afree0 + 8 * ba);
-        umma_commit(empty0 + 8 * slot);
-        }
-        __syncwarp();
-        TP(if (tr && lane == 0 && i < 64) g_mma_trace[2][i] = clock64();)
-        sw.next(a);
-      }
-    }
-  } else if (warp < kConvWarps && !F::kConv) {
-    // nothing to convert: the MMA reads the stage as it lies
-  } else if (warp < kConvWarps) {
-    // ------------------------------------------------------------------ converters
-    // Two groups of four warps convert alternate stages (thread = row r of the tile), so two stages
-    // are in conversion at any time: a stage's conversion is a fixed latency of well over a
-    // thousand cycles whatever its size, and what counts is how many run side by side.  Both groups
-    // follow every stage's barriers in order, also those of the stages they do not convert, and both
-    // arrive for every stage, so no barrier phase is ever skipped (a parity wait can only tell the
-    // current phase from the one before it).
-    const int q4 = warp & 3, grp = warp >> 2;
-    const int r = q4 * 32 + lane;
-    const uint32_t lane_base = (uint32_t)(q4 * 32) << 16;
-    RingCursor rc;
-    for (int i = 0; sw.live(a) && ok; ++i, sw.next(a), rc.next(S)) {
-      const int ba = i % NA, slot = rc.s;
-      ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * slot, rc.ph, a.status, 4));
-      if (ok && i >= NA) ok = __all_sync(0xffffffffu, mbar_wait(afree0 + 8 * ba, ((i - NA) / NA) & 1, a.status, 3));
-      if (!ok) break;
-      if ((i & 1) != grp) {
-        // The other group's stage: this one has seen its barriers and says so.  Without this the MMA could be
-        // done with the stage before a warp held up here has looked (an instruction fetch of the first launch is
-        // enough), which would then wait for a round that is two further on.
-        __syncwarp();
-        if (lane == 0) mbar_arrive(aready0 + 8 * ba);
-        continue;
-      }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      TP(if (tr && q4 == 0 && lane == 0 && i < 64) g_mma_trace[3][i] = clock64();)
-      const unsigned char* st = ring + (size_t)slot * kStage;
-      // ---- this row of each chunk of the stage: 256 nibbles -> 256 bytes -> 64 TMEM columns ----
-      const int nc = sw.nc();
-#pragma unroll
-      for (int cc = 0; cc < C; ++cc) {
-        if (cc < nc) {
-          uint4 qv[8];
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            if (DBG(2)) qv[u] = make_uint4(r, u, cc, i);  // tuning: no shared-memory loads
-            else qv[u] = *reinterpret_cast<const uint4*>(st + cc * kStageBytes + r * 128 + ((u ^ (r & 7)) << 4));
-          }
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            uint32_t ws[4] = {qv[u].x, qv[u].y, qv[u].z, qv[u].w};
-            uint32_t regs[8];
-#pragma unroll
-            for (int w = 0; w < 4; ++w) {
-              regs[2 * w + 0] = ws[w] & 0x0F0F0F0Fu;         // elements 0,2,4,6 of the word
-              regs[2 * w + 1] = (ws[w] >> 4) & 0x0F0F0F0Fu;  // elements 1,3,5,7
-            }
-            if (!DBG(1)) tmem_st8(tmemA0 + lane_base + ba * kACols + cc * 64 + u * 8, regs);
-            else if ((regs[0] ^ regs[3] ^ regs[5] ^ regs[7]) == 0x12345678u) *last_flag = 1;  // tuning: no TMEM stores
-          }
+      };
+      for (; sw.live(a) && ok; sw.next_item(a)) {
+        for (int c = sw.c; c < sw.c1; ++c, ++i, rc.next(S)) {
+          if (i == S && !waited) catch_up();
+          if (i >= S) ok = mbar_wait(empty0 + 8 * rc.s, rc.ph ^ 1u, a.status, 1);
+          if (!ok) break;
+          const uint32_t dst = smem_u32(ring + (size_t)rc.s * kStage), bar = full0 + 8 * rc.s;
+          mbar_expect_tx(bar, kStage);
+          bulk_load_1d(dst, wsrc(sw, c), F::kStageBytes, bar);
+          if (!FUSED && waited) bulk_load_1d(dst + F::kStageBytes, bsrc(sw, c), X::kBytes, bar);
         }
       }
-      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      // One arrival per warp: 128 arrivals on one mbarrier serialise in the shared-memory atomic
-      // unit and cost more than the conversion itself.  The lanes meet (which also orders their
-      // shared-memory reads and TMEM stores before the elected lane's releasing arrival).
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(aready0 + 8 * ba);
-        mbar_arrive(empty0 + 8 * slot);
-      }
-      TP(if (tr && q4 == 0 && lane == 0 && i < 64) g_mma_trace[4][i] = clock64();)
+      if (!waited) catch_up();
+      if (!ok) *gave_up = 1;
     }
+    __syncwarp();
   } else {
-    // ------------------------------------------------------------------ epilogue
-    // EP warps per TMEM lane quarter: part p takes the p-th share of a stage's accumulator
-    // blocks; each keeps its own running sums and the parts are added, in order, when an item
-    // (tile, K range) ends.
-    const int q4 = warp & 3, half = (warp - kConvWarps) >> 2;  // half: the part, 0 .. EP-1
-    const int r = q4 * 32 + lane;  // row of the tile == TMEM lane
-    const int et = tid - kConvThreads;
-    const uint32_t lane_base = (uint32_t)(q4 * 32) << 16;
-    float acc[MB];
+    // ------------------------------------------------------------------ consumers
+    const int g = lane >> 2, t = lane & 3, half = t >> 1, p = t & 1;
+    const int grp = KG == 2 ? warp >> 2 : 0, slot = KG == 2 ? warp & 3 : warp;  // slot: of the warps that finish items
+    const int row0 = slot * (16 * SL);
+    if (FUSED) {
+      pdl_wait();
+      // every item of this CTA covers the same K range (the grid is a multiple of the K splits)
+      if (sw.live(a)) {
+        const int n = sw.c1 - sw.c;
+        auto at = [&](int i, int& m, int& c) {
+          m = MB == 1 ? 0 : i / n;
+          c = i - m * n;
+          return a.x + (size_t)m * a.in_dim + (sw.c + c) * kChunkK + lane * 8;
+        };
+        int m, c;
+        float v[8];
+        if (warp < a.batch * n) load_eight(at(warp, m, c), v);
+#pragma unroll 1
+        for (int i = warp; i < a.batch * n;) {
+          float u[8];
+          const int m0 = m, c0 = c;
+          i += kConsumers;
+          if (i < a.batch * n) load_eight(at(i, m, c), u);  // (the next chunk is under way while this one is worked on)
+          prep_chunk<FMT, MB>(v, lane, bres + (size_t)c0 * X::kBytes, m0, a.digits);
 #pragma unroll
-    for (int m = 0; m < MB; ++m) acc[m] = 0.f;
-    if (!FUSED && !G) {
-      pdl_wait();  // the tables come from the preparation kernel in front
-      for (int i = et; i < 2 * a.batch * groups; i += kEpiThreads) xsum[i] = __ldg(a.xtab + i);
-      asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
+          for (int e = 0; e < 8; ++e) v[e] = u[e];
+        }
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(kConsumers * 32) : "memory");
     }
-    int nb = a.batch;    // activation rows in use (G: of the current entry)
-    int cur_entry = -1;  // G: the entry whose tables are in shared memory
-    int orow[G ? MB : 1];  // G: result row of each activation row
-    float gate[kWork ? MB : 1];  // work lists: the gate's sums while up is computed
-    // Work lists of Q4_K: the sums of the chunks before.  A chunk is summed by itself, so that its terms, products and minima that
-    // cancel, meet a small sum.  Against 64 bits, x of bf16 values, in one chain / so / the CUDA-core kernels: 1024 elements 1.10e-7 /
-    // 0.77e-7 / 0.75e-7, 2048 1.4e-7 / 0.8e-7 / 0.8e-7, 4096 2.1e-7 / 1.0e-7 / 0.9e-7; normal x of 24 bits, 2048: so 0.9e-7, CUDA cores 2.6e-7.  (Q8_0 has no minima, one chain is as good as the CUDA cores' up to 2048 elements, and
-    // this cost it 1 to 2 % of the call.)
-    constexpr bool kByChunk = kWork && FMT == FMT_Q4K;
-    float before[kByChunk ? MB : 1];
-    constexpr int kHB = kBlocks / EP;                       // blocks of this part
-    constexpr int kSub = kHB * N <= 64 ? kHB : 64 / N;      // blocks per pass (at most 64 columns in registers)
-    constexpr bool kNarrow = kSub * N == 8;                 // a pass of one 8-column block: one 8-column load
-    constexpr int NLD = kNarrow ? 1 : kSub * N / 16;        // 16-column loads per pass
+    // shared-memory addresses that stay: of the lane's rows in an ldmatrix (nibbles: two K steps of 16 rows; bytes: one), and
+    // of its part of the fragments and tables
+    const int mi = lane >> 3, lr = lane & 7;
+    const uint32_t a_lane = F::kNibble ? (row0 + (mi & 1) * 8 + lr) * 128 : (mi >> 1) * 2048 + (row0 / 8 + (mi & 1)) * 128 + lr * 16;
+    const uint32_t b_lane = MB == 1 ? ((g & 3) * 4 + t) * 16 : lane * 16;
+    const int t_lane = X::kFrag + 4 * (MB == 1 ? X::entry1(p, half, 0) : X::entry(half, p, 0));
+    unsigned char* sc_warp = scales + warp * (SL * 16 * kStagedRow);
+    float gate[kWork ? C::kVals : 1];
+    int cur_entry = -1, nb = a.batch;
     RingCursor rc;
-    for (int i = 0; sw.live(a) && ok; ++i, rc.next(S)) {
-      const int b = i % ND, slot = kSpills ? i % S : rc.s;
-      if (G && sw.entry != cur_entry) {
-        // a new entry: its tables, row count and result rows.  Every epilogue thread passed the barrier
-        // that ends the item before, so nobody still reads the old tables.
-        cur_entry = sw.entry;
-        const float* tab = a.xtab + (size_t)cur_entry * a.gtab;
-        for (int j = et; j < 2 * a.batch * groups; j += kEpiThreads) xsum[j] = __ldcg(tab + j);
-        const MmaGroupEntry* ge = entry_at(cur_entry);
-        nb = __ldg(&ge->count);
+    int i = 0, items = 0;
+    for (; sw.live(a) && ok; sw.next_item(a), ++items) {
+      float acc[SL][NT][2], before[kByChunk ? SL : 1][kByChunk ? NT : 1][2];
 #pragma unroll
-        for (int m = 0; m < (G ? MB : 1); ++m) orow[m] = kWork || a.gdirect ? __ldg(&ge->item[m]) : cur_entry * MB + m;
-        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
-      }
-      ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * slot, kSpills ? (i / S) & 1 : rc.ph, a.status, 6));
-      uint4 mvs[C];
-      uint32_t q6d = 0;  // Q6_K: the super-block's f16 d (the 16 int8 scales are in mvs)
-      const int nc = sw.nc();
-      if (ok) {
-        uint32_t seen = 1u;
+      for (int sl = 0; sl < SL; ++sl)
 #pragma unroll
-        for (int cc = 0; cc < C; ++cc) {
-          mvs[cc] = make_uint4(0, 0, 0, 0);
-          const unsigned char* mrow = ring + (size_t)slot * kStage + cc * kStageBytes + kStageWBytes + r * F::kMetaRow;
-          if (cc < nc) mvs[cc] = *reinterpret_cast<const uint4*>(mrow);
-          if (FMT == FMT_Q6K) q6d = *reinterpret_cast<const uint32_t*>(mrow + 16);
-          seen |= mvs[cc].x | q6d;
+        for (int nt = 0; nt < NT; ++nt) acc[sl][nt][0] = acc[sl][nt][1] = 0.f;
+#pragma unroll 1
+      for (int c = sw.c; c < sw.c1; ++c, ++i, rc.next(S)) {
+        if (KG == 2 && (i & 1) != grp) continue;
+        ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * rc.s, rc.ph, a.status, 4));
+        if (!ok) break;
+        if constexpr (kByChunk) {
+#pragma unroll
+          for (int sl = 0; sl < SL; ++sl)
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+              for (int r = 0; r < 2; ++r) {
+                before[sl][nt][r] = acc[sl][nt][r];
+                acc[sl][nt][r] = 0.f;
+              }
         }
-        // the scale data is in registers: one lane releases the stage for the warp (the values are
-        // consumed by the shuffle, so every lane's loads have completed before the arrival)
-        seen = __reduce_or_sync(0xffffffffu, seen);
-        if (lane == 0 && seen) mbar_arrive(empty0 + 8 * slot);
-        ok = __all_sync(0xffffffffu, mbar_wait(mdone0 + 8 * b, (i / ND) & 1, a.status, 7));
-      }
-      if (!ok) break;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      TP(if (tr && et == 0 && i < 64) g_mma_trace[5][i] = clock64();)
+        const unsigned char* st = ring + (size_t)rc.s * kStage;
+        const unsigned char* xb = FUSED ? bres + (size_t)(c - cbase) * X::kBytes : st + F::kStageBytes;
+        const uint32_t st_a = smem_u32(st) + a_lane;
+        const unsigned char* xf = xb + b_lane;
+        const unsigned char* xt = xb + t_lane;
+        if constexpr (kStaged<FMT, MB>) {
 #pragma unroll
-      for (int cc = 0; cc < C; ++cc) {
-      if (cc < nc) {
-      if constexpr (kByChunk) {
-#pragma unroll
-        for (int m = 0; m < MB; ++m) {
-          before[m] = acc[m];
-          acc[m] = 0.f;
-        }
-      }
-      const uint32_t meta[4] = {mvs[cc].x, mvs[cc].y, mvs[cc].z, mvs[cc].w};
-      const int gbase = (sw.c + cc) * kBlocks;
-#pragma unroll
-      for (int sub = 0; sub < kHB / kSub; ++sub) {
-        const int blk0 = half * kHB + sub * kSub;  // first block of this pass
-        uint32_t t[NLD][16];
-#pragma unroll
-        for (int l = 0; l < NLD; ++l) {
-          const uint32_t taddr = tmemD0 + lane_base + b * kDCols + cc * (kBlocks * N) + blk0 * N + l * 16;
-          if (kNarrow) tmem_ld8(taddr, *reinterpret_cast<uint32_t(*)[8]>(&t[l][0]));
-          else tmem_ld16(taddr, t[l]);
-        }
-#pragma unroll
-        for (int l = 0; l < NLD; ++l) {
-          if (kNarrow) tmem_wait_ld(*reinterpret_cast<uint32_t(*)[8]>(&t[l][0]));
-          else tmem_wait_ld(t[l]);
-        }
-        TP(if (tr && et == 0 && i == 2) g_mma_trace[7][12 + 2 * cc] = clock64();)
-        if (sub == kHB / kSub - 1 && cc == nc - 1) {  // the stage's last load: its accumulators are free
-          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          for (int sl = 0; sl < SL; ++sl) stage_scales<FMT>(st, row0 + 16 * sl, sc_warp + sl * (16 * kStagedRow), lane);
           __syncwarp();
-          if (lane == 0) mbar_arrive(dfree0 + 8 * b);
         }
+        const unsigned char* sc_lane = sc_warp + g * kStagedRow;
+        const unsigned char* meta = st + F::kStageWBytes + (row0 + g) * F::kMetaRow;
+        RowScales<FMT> rs[MB == 1 ? SL : 1][2];
+        if constexpr (MB == 1 && FMT != FMT_MLX4) {
 #pragma unroll
-        for (int g = 0; g < kSub; ++g) {
-          const int blk = blk0 + g;
-          auto col = [&](int cidx) { return (int)t[(g * N + cidx) >> 4][(g * N + cidx) & 15]; };
-          auto digits_dot = [&](int c0) {  // the integer dot of the DIGITS columns from c0
-            if (DIGITS == 4) {
-              int lo = col(c0) + (col(c0 + 1) << 7), hi = col(c0 + 2) + (col(c0 + 3) << 7);
-              return fmaf((float)hi, 16384.f, (float)lo);
-            }
-            int lo = col(c0) + (col(c0 + 1) << 7);
-            return fmaf((float)col(c0 + 2), 16384.f, (float)lo);
-          };
-          if (FMT == FMT_Q4K) {
-            // the block holds two 32-element sub-blocks: columns [0, N/2) and [N/2, N); their
-            // multipliers (sc*d) and -(m*dmin), each rounded to f32 as dequantRowQ4KTo does
-            constexpr int db = N / 2;
-            const float d16 = __half2float(__ushort_as_half((unsigned short)(meta[0] & 0xFFFFu)));
-            const float dmin16 = __half2float(__ushort_as_half((unsigned short)(meta[0] >> 16)));
+          for (int sl = 0; sl < SL; ++sl)
 #pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-              const int sub = 2 * blk + hh, bit = 12 * sub, wi = bit >> 5, sh = bit & 31;
-              const uint32_t lo = wi == 0 ? meta[1] : wi == 1 ? meta[2] : meta[3];
-              const uint32_t hi = wi == 0 ? meta[2] : wi == 1 ? meta[3] : 0u;
-              const uint32_t f = __funnelshift_r(lo, hi, sh) & 0xFFFu;
-              // Integer -> float through the exponent trick (an add and a subtract on the full-rate
-              // pipes; eight sub-blocks a chunk would otherwise queue on the conversion unit).  Exact
-              // while |v| < 2^22: the 6-bit fields trivially, and a column sums 32 products of a
-              // nibble and a digit in [-64, 63], so |c0 + 128 c1| <= 30720 * 129 < 2^22.
-              auto small_f = [](uint32_t v) { return __uint_as_float(0x4B000000u | v) - 8388608.f; };
-              auto int_f = [](int v) { return __int_as_float(0x4B400000 + v) - 12582912.f; };
-              const float sc = __fmul_rn(small_f(f & 63u), d16), bi = -__fmul_rn(small_f(f >> 6), dmin16);
-              const int ti = 2 * gbase + sub;  // the sub-block's entry of the per-32 tables
-              auto paired_dot = [&](int c0) {
-                const float lo = int_f(col(c0) + (col(c0 + 1) << 7));
-                const float hi = DIGITS == 4 ? int_f(col(c0 + 2) + (col(c0 + 3) << 7)) : int_f(col(c0 + 2));
-                return fmaf(hi, 16384.f, lo);
-              };
-#pragma unroll
-              for (int m = 0; m < MB; ++m) {
-                if (MB == 1 || m < nb) {
-                  const float dot = paired_dot(hh * db + DIGITS * m) * xfs[m * groups + ti];
-                  acc[m] = fmaf(sc, dot, acc[m]);
-                  acc[m] = fmaf(bi, xsum[m * groups + ti], acc[m]);
-                }
-              }
-            }
-          } else if (FMT == FMT_Q5K) {
-            // one 32-element sub-block: (sc*d) and -(m*dmin), each rounded to f32 as dequantRowQ5K does
-            const float d16 = __half2float(__ushort_as_half((unsigned short)(meta[0] & 0xFFFFu)));
-            const float dmin16 = __half2float(__ushort_as_half((unsigned short)(meta[0] >> 16)));
-            const int bit = 12 * blk, wi = bit >> 5, sh = bit & 31;
-            const uint32_t lo = wi == 0 ? meta[1] : wi == 1 ? meta[2] : meta[3];
-            const uint32_t hi = wi == 0 ? meta[2] : wi == 1 ? meta[3] : 0u;
-            const uint32_t f = __funnelshift_r(lo, hi, sh) & 0xFFFu;
-            const float sc = __fmul_rn((float)(f & 63u), d16), bi = -__fmul_rn((float)(f >> 6), dmin16);
-#pragma unroll
-            for (int m = 0; m < MB; ++m) {
-              if (MB == 1 || m < nb) {
-                const float dot = digits_dot(DIGITS * m) * xfs[m * groups + gbase + blk];
-                acc[m] = fmaf(sc, dot, acc[m]);
-                acc[m] = fmaf(bi, xsum[m * groups + gbase + blk], acc[m]);
-              }
-            }
-          } else if (FMT == FMT_Q6K) {
-            // the step's two 16-element scale groups: columns [0, N/2) and [N/2, N); multiplier
-            // d * sc rounded to f32 as dequantRowQ6K does
-            const float d16 = __half2float(__ushort_as_half((unsigned short)(q6d & 0xFFFFu)));
-            const uint32_t sw4 = (blk >> 1) == 0 ? meta[0] : (blk >> 1) == 1 ? meta[1] : (blk >> 1) == 2 ? meta[2] : meta[3];
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-              const int s8 = (int)(signed char)((sw4 >> (8 * (2 * (blk & 1) + hh))) & 0xFFu);
-              const float sc = __fmul_rn(d16, (float)s8);
-#pragma unroll
-              for (int m = 0; m < MB; ++m) {
-                if (MB == 1 || m < nb) {
-                  const float dot = digits_dot(hh * (N / 2) + DIGITS * m) * xfs[m * groups + gbase + blk];
-                  acc[m] = fmaf(sc, dot, acc[m]);
-                }
-              }
-            }
-          } else {
-            // the block's multiplier of the integer dot and of the block's sum of x
-            float sc, bi;
-            if (FMT == FMT_MLX4) {  // {scale, bias} bf16 pair of the 64-element group
-              const uint32_t mw = blk == 0 ? meta[0] : blk == 1 ? meta[1] : blk == 2 ? meta[2] : meta[3];
-              sc = __uint_as_float(mw << 16);
-              bi = __uint_as_float(mw & 0xFFFF0000u);
-            } else {  // f16 block scale
-              const uint32_t mw = (blk >> 1) == 0 ? meta[0] : (blk >> 1) == 1 ? meta[1] : (blk >> 1) == 2 ? meta[2] : meta[3];
-              sc = __half2float(__ushort_as_half((unsigned short)((mw >> (16 * (blk & 1))) & 0xFFFFu)));
-              bi = 0.f;
-            }
-#pragma unroll
-            for (int m = 0; m < MB; ++m) {
-              if (MB == 1 || m < nb) {
-                const float dot = digits_dot(DIGITS * m) * xfs[m * groups + gbase + blk];
-                acc[m] = fmaf(sc, dot, acc[m]);
-                if (FMT != FMT_Q80) acc[m] = fmaf(bi, xsum[m * groups + gbase + blk], acc[m]);
-              }
-            }
-          }
+            for (int r = 0; r < 2; ++r) rs[sl][r].load(meta + (16 * sl + 8 * r) * F::kMetaRow);
         }
-      }
-      if constexpr (kByChunk) {
+        // scales (and biases) of the rows g + 8 r of slab sl
+        auto mlx_scale = [&](int sl, int r, int word, float& sv, float& bv) {  // word: per lane
+          const uint32_t w = *reinterpret_cast<const uint32_t*>(meta + (16 * sl + 8 * r) * 16 + 4 * word);
+          sv = __uint_as_float(w << 16);
+          bv = __uint_as_float(w & 0xFFFF0000u);
+        };
+        // A fragments of K step s
+        uint32_t af[SL][2][4];
+        auto load_a = [&](int j) {  // both steps of pair j
 #pragma unroll
-        for (int m = 0; m < MB; ++m) acc[m] += before[m];
-      }
-      TP(if (tr && et == 0 && i == 2) g_mma_trace[7][13 + 2 * cc] = clock64() + (long long)(__float_as_int(acc[0]) & 1);)
-      }  // cc < nc
-      }  // chunks of the stage
-      TP(if (tr && et == 0 && i < 64) g_mma_trace[6][i] = clock64();)
-      const bool item_done = sw.last_chunk();
-      const int tile = sw.tile, split = sw.split;
-      const int gmat = G ? sw.mat : 0;
-      sw.next(a);
-      if (!item_done) continue;
-      // ---- the item is complete: add the parts' sums (parts above 0 -> shared memory -> part 0) ----
-      if (half != 0) {
+          for (int sl = 0; sl < SL; ++sl) {
+            if (F::kNibble) {
+              uint32_t q[4];
+              ldsm4(st_a + sl * 2048 + ((((2 * j + (mi >> 1)) ^ lr) << 4)), q);
 #pragma unroll
-        for (int m = 0; m < MB; ++m) {
-          pair[((half - 1) * MB + m) * kTileRows + r] = acc[m];
-          acc[m] = 0.f;
-        }
-      }
-      TP(if (tr && et == 0 && i < 16) g_mma_trace[7][8] = clock64();)
-      asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
-      TP(if (tr && et == 0 && i < 16) g_mma_trace[7][9] = clock64();)
-      if (half == 0) {
-#pragma unroll
-        for (int m = 0; m < MB; ++m) {
-#pragma unroll
-          for (int p = 0; p < EP - 1; ++p) acc[m] += pair[(p * MB + m) * kTileRows + r];
-        }
-      }
-      const int row = tile * kTileRows + r;
-      if (a.cluster) {
-        // The K splits of this tile are the CTAs of this cluster (rank == split) and each has this one
-        // item.  Ranks above 0 put their sums into rank 0's shared memory and arrive on its barrier
-        // (one releasing arrival per warp, after the warp's lanes have met); rank 0 waits, adds the
-        // sums in split order — the same order as the scratch path, so the same bits — and stores.
-        if (half == 0) {
-          if (split != 0) {
-#pragma unroll
-            for (int m = 0; m < MB; ++m)
-              if (m < a.batch) cluster_store_f32(cluster_map(smem_u32(recv + ((split - 1) * MB + m) * kTileRows + r), 0), acc[m]);
-            __syncwarp();
-            if (lane == 0) cluster_arrive_release(cluster_map(clbar, 0));
-          } else {
-            ok = __all_sync(0xffffffffu, mbar_wait_cluster(clbar, 0, a.status, 12));
-            if (ok) {
-#pragma unroll
-              for (int m = 0; m < MB; ++m) {
-                float sum = acc[m];
-                for (int s2 = 1; s2 < a.splits; ++s2) sum += recv[((s2 - 1) * MB + m) * kTileRows + r];
-                if (m < a.batch && row < a.out_dim) a.out[(size_t)m * a.out_dim + row] = sum;
-              }
-            }
-          }
-        }
-#pragma unroll
-        for (int m = 0; m < MB; ++m) acc[m] = 0.f;
-        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
-      } else if (G) {
-        if (half == 0) {
-#pragma unroll
-          for (int m = 0; m < MB; ++m) {
-            if constexpr (kWork) {
-              if (a.gdirect == 2) {
-                if (gmat == 0) gate[m] = acc[m];
-                else if (m < nb) a.out[(size_t)orow[m] * a.out_dim + row] = gelu_tanh(gate[m]) * acc[m];
-              } else if (m < nb) {
-                const MmaWorkEntry* we = reinterpret_cast<const MmaWorkEntry*>(a.gwork) + cur_entry;
-                float* dst = reinterpret_cast<float*>(__ldg(reinterpret_cast<const unsigned long long*>(&we->dst[m])));
-                if (row < __ldg(&we->room[m])) atomicAdd(dst + row, acc[m] * __ldg(&we->weight[m]));  // items may share a destination row
+              for (int k = 0; k < 2; ++k) {
+                af[sl][k][0] = q[2 * k] & 0x0F0F0F0Fu;
+                af[sl][k][1] = q[2 * k + 1] & 0x0F0F0F0Fu;
+                af[sl][k][2] = (q[2 * k] >> 4) & 0x0F0F0F0Fu;
+                af[sl][k][3] = (q[2 * k + 1] >> 4) & 0x0F0F0F0Fu;
               }
             } else {
-              if (m < nb) a.out[(size_t)orow[G ? m : 0] * a.out_dim + gmat * (a.gtpe * kTileRows) + row] = acc[m];
+              ldsm4(st_a + sl * 256 + (2 * j) * 4096, af[sl][0]);
+              ldsm4(st_a + sl * 256 + (2 * j + 1) * 4096, af[sl][1]);
             }
-            acc[m] = 0.f;
+          }
+        };
+        auto frag = [&](int j, int nt) { return *reinterpret_cast<const uint4*>(xf + (j * NT + nt) * (MB == 1 ? 256 : 512)); };
+        // one block's sums into the accumulators: scale and bias of the row, scale and sum of the activations
+        auto add = [&](float& ac, const int (&d)[4], int r, float sv, float bv, float xs, float sx) {
+          ac = fmaf(sv, digits_sum(d[2 * r], d[2 * r + 1]) * xs, ac);
+          if (F::kSums) ac = fmaf(bv, sx, ac);
+        };
+        // one row: the two blocks of a pair, of which the lane's half is the one whose scale is not zero
+        auto add_pair = [&](float& ac, const int (&d)[2][4], int r, float sv, float bv, const float4& x) {
+          ac = fmaf(sv, fmaf(digits_sum(d[1][2 * r], d[1][2 * r + 1]), x.y, digits_sum(d[0][2 * r], d[0][2 * r + 1]) * x.x), ac);
+          if (F::kSums) ac = fmaf(bv, x.z, ac);
+        };
+        auto tab1 = [&](int pr) {
+          if (F::kSums) return *reinterpret_cast<const float4*>(xt + pr * 16);
+          const float2 v = *reinterpret_cast<const float2*>(xt + pr * 8);
+          return make_float4(v.x, v.y, 0.f, 0.f);
+        };
+        auto tab = [&](int nt, int grp_) {  // scale and sum
+          const int at = nt * 4 * F::kGroups + grp_;
+          if (F::kSums) return *reinterpret_cast<const float2*>(xt + at * 8);
+          return make_float2(*reinterpret_cast<const float*>(xt + at * 4), 0.f);
+        };
+        if constexpr (FMT == FMT_MLX4) {
+          if constexpr (MB == 1) {
+#pragma unroll
+            for (int jj = 0; jj < 2; ++jj) {
+              int d[SL][2][4];
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                const int j = 2 * jj + h;
+                load_a(j);
+                const uint4 b = frag(j, 0);
+#pragma unroll
+                for (int sl = 0; sl < SL; ++sl) {
+                  int(&e)[4] = d[sl][h];
+                  imma32<false>(e, af[sl][0][0], af[sl][0][1], af[sl][0][2], af[sl][0][3], b.x, b.y, kAcc0, kAcc0, kAcc0, kAcc0);
+                  imma32<false>(e, af[sl][1][0], af[sl][1][1], af[sl][1][2], af[sl][1][3], b.z, b.w, e[0], e[1], e[2], e[3]);
+                }
+              }
+              const float4 x = tab1(jj);
+#pragma unroll
+              for (int sl = 0; sl < SL; ++sl) {
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                  float sv, bv;
+                  mlx_scale(sl, r, 2 * jj + half, sv, bv);
+                  add_pair(acc[sl][0][r], d[sl], r, sv, bv, x);
+                }
+              }
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              load_a(j);
+              float sv[SL][2], bv[SL][2];
+#pragma unroll
+              for (int sl = 0; sl < SL; ++sl)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) mlx_scale(sl, r, j, sv[sl][r], bv[sl][r]);
+#pragma unroll
+              for (int nt = 0; nt < NT; ++nt) {
+                const uint4 b = frag(j, nt);
+                const float2 x = tab(nt, j);
+#pragma unroll
+                for (int sl = 0; sl < SL; ++sl) {
+                  int d[4];
+                  imma32<false>(d, af[sl][0][0], af[sl][0][1], af[sl][0][2], af[sl][0][3], b.x, b.y, kAcc0, kAcc0, kAcc0, kAcc0);
+                  imma32<false>(d, af[sl][1][0], af[sl][1][1], af[sl][1][2], af[sl][1][3], b.z, b.w, d[0], d[1], d[2], d[3]);
+#pragma unroll
+                  for (int r = 0; r < 2; ++r) add(acc[sl][nt][r], d, r, sv[sl][r], bv[sl][r], x.x, x.y);
+                }
+              }
+            }
+          }
+        } else if constexpr (FMT == FMT_Q6K) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            load_a(j);
+            if constexpr (MB == 1) {
+              const uint4 b = frag(j, 0);
+              const float4 xx = *reinterpret_cast<const float4*>(xt + j * 16);  // both steps' entries
+#pragma unroll
+              for (int sl = 0; sl < SL; ++sl) {
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                  int d[2][4];
+                  imma16(d[0], af[sl][k][0], af[sl][k][1], k ? b.z : b.x, kAcc0);
+                  imma16(d[1], af[sl][k][2], af[sl][k][3], k ? b.w : b.y, kAcc0);
+#pragma unroll
+                  for (int r = 0; r < 2; ++r) {
+                    add_pair(acc[sl][0][r], d, r, rs[sl][r].pair(2 * j + k, half).x, 0.f, k ? make_float4(xx.z, xx.w, 0.f, 0.f) : xx);
+                  }
+                }
+              }
+            } else {
+#pragma unroll
+              for (int k = 0; k < 2; ++k) {
+                const int step = 2 * j + k;
+                float2 sv[SL][2];
+#pragma unroll
+                for (int sl = 0; sl < SL; ++sl)
+#pragma unroll
+                  for (int r = 0; r < 2; ++r) sv[sl][r] = *reinterpret_cast<const float2*>(sc_lane + (16 * sl + 8 * r) * kStagedRow + step * 8);
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt) {
+                  const uint4 b = frag(j, nt);
+                  const float2 x = tab(nt, step);
+#pragma unroll
+                  for (int sl = 0; sl < SL; ++sl) {
+                    int d[2][4];
+                    imma16(d[0], af[sl][k][0], af[sl][k][1], k ? b.z : b.x, kAcc0);
+                    imma16(d[1], af[sl][k][2], af[sl][k][3], k ? b.w : b.y, kAcc0);
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {
+                      add(acc[sl][nt][r], d[0], r, sv[sl][r].x, 0.f, x.x, 0.f);
+                      add(acc[sl][nt][r], d[1], r, sv[sl][r].y, 0.f, x.x, 0.f);
+                    }
+                  }
+                }
+              }
+            }
+          }
+        } else {  // a block per K step
+          uint32_t q8[SL][2][4];  // Q8_0: the rows' f16 scales
+          if (FMT == FMT_Q80 && MB > 1) {
+#pragma unroll
+            for (int sl = 0; sl < SL; ++sl)
+#pragma unroll
+              for (int r = 0; r < 2; ++r) {
+                const uint4 w = *reinterpret_cast<const uint4*>(meta + (16 * sl + 8 * r) * 16);
+                q8[sl][r][0] = w.x;
+                q8[sl][r][1] = w.y;
+                q8[sl][r][2] = w.z;
+                q8[sl][r][3] = w.w;
+              }
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            load_a(j);
+            if constexpr (MB == 1) {
+              const uint4 b = frag(j, 0);
+              const float4 x = tab1(j);
+#pragma unroll
+              for (int sl = 0; sl < SL; ++sl) {
+                int d[2][4];
+                imma32<F::kSigned>(d[0], af[sl][0][0], af[sl][0][1], af[sl][0][2], af[sl][0][3], b.x, b.y, kAcc0, kAcc0, kAcc0, kAcc0);
+                imma32<F::kSigned>(d[1], af[sl][1][0], af[sl][1][1], af[sl][1][2], af[sl][1][3], b.z, b.w, kAcc0, kAcc0, kAcc0, kAcc0);
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                  const float2 sb = rs[sl][r].pair(j, half);
+                  add_pair(acc[sl][0][r], d, r, sb.x, sb.y, x);
+                }
+              }
+            } else {
+              float4 sb[SL][2];  // of the pair's two blocks
+#pragma unroll
+              for (int sl = 0; sl < SL; ++sl)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                  if (FMT == FMT_Q80) sb[sl][r] = make_float4(f16_lo(q8[sl][r][j]), 0.f, f16_hi(q8[sl][r][j]), 0.f);
+                  else sb[sl][r] = *reinterpret_cast<const float4*>(sc_lane + (16 * sl + 8 * r) * kStagedRow + j * 16);
+                }
+#pragma unroll
+              for (int nt = 0; nt < NT; ++nt) {
+                const uint4 b = frag(j, nt);
+                const float2 x0 = tab(nt, 2 * j), x1 = tab(nt, 2 * j + 1);
+#pragma unroll
+                for (int sl = 0; sl < SL; ++sl) {
+                  int d[2][4];
+                  imma32<F::kSigned>(d[0], af[sl][0][0], af[sl][0][1], af[sl][0][2], af[sl][0][3], b.x, b.y, kAcc0, kAcc0, kAcc0, kAcc0);
+                  imma32<F::kSigned>(d[1], af[sl][1][0], af[sl][1][1], af[sl][1][2], af[sl][1][3], b.z, b.w, kAcc0, kAcc0, kAcc0, kAcc0);
+#pragma unroll
+                  for (int r = 0; r < 2; ++r) {
+                    add(acc[sl][nt][r], d[0], r, sb[sl][r].x, sb[sl][r].y, x0.x, x0.y);
+                    add(acc[sl][nt][r], d[1], r, sb[sl][r].z, sb[sl][r].w, x1.x, x1.y);
+                  }
+                }
+              }
+            }
           }
         }
-        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");  // pair and the tables are free for the next item
+        __syncwarp();
+        if (lane == 0) mbar_arrive(empty0 + 8 * rc.s);
+        if constexpr (kByChunk) {
+#pragma unroll
+          for (int sl = 0; sl < SL; ++sl)
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+              for (int r = 0; r < 2; ++r) acc[sl][nt][r] += before[sl][nt][r];
+        }
+      }
+      // ---- the item is complete: lanes of a quad meet; lane p of a pair keeps row g + 8 p ----
+#pragma unroll
+      for (int sl = 0; sl < SL; ++sl) {
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+          float v0 = acc[sl][nt][0], v1 = acc[sl][nt][1];
+          v0 += __shfl_xor_sync(0xffffffffu, v0, 1);
+          v1 += __shfl_xor_sync(0xffffffffu, v1, 1);
+          float v = p ? v1 : v0;
+          if (MB == 1) v += __shfl_xor_sync(0xffffffffu, v, 2);
+          fin[sl * NT + nt] = v;
+        }
+      }
+      if (KG == 1 && !ok) break;
+      if constexpr (KG == 2) {
+        if (!ok && lane == 0) gave_up[1 + slot] = items + 1;  // (both groups come to the item's meeting, and both leave after it)  // the groups' sums: the second one's through shared memory (two buffers: the meeting of the next item frees this one)
+        float* buf = pair + ((items & 1) * C::kStoring + slot) * (C::kVals * 32) + lane;
+        if (grp == 1) {
+#pragma unroll
+          for (int k = 0; k < C::kVals; ++k) buf[k * 32] = fin[k];
+        }
+        asm volatile("bar.sync %0, 64;" ::"r"(2 + slot) : "memory");
+        if (gave_up[1 + slot] == items + 1) {
+          ok = false;
+          break;
+        }
+        if (grp == 1) continue;
+#pragma unroll
+        for (int k = 0; k < C::kVals; ++k) fin[k] += buf[k * 32];
+      }
+      const int row = sw.tile * kTileRows + row0 + g + 8 * p;  // of the first slab
+      auto act = [&](int k) { return MB == 1 ? 0 : 2 * (k % NT) + half; };
+      const bool mine = MB > 1 || t < 2;
+      if (G) {
+        if (sw.entry != cur_entry) {
+          cur_entry = sw.entry;
+          nb = __ldg(&entry_at(cur_entry)->count);
+        }
+        if (kWork && a.gdirect == 2 && sw.mat == 0) {
+#pragma unroll
+          for (int k = 0; k < C::kVals; ++k) gate[kWork ? k : 0] = fin[k];
+          continue;
+        }
+#pragma unroll
+        for (int k = 0; k < C::kVals; ++k) {
+          const int m = act(k), r = row + 16 * (k / NT);
+          if (m >= nb) continue;
+          if constexpr (kWork) {
+            const MmaWorkEntry* we = reinterpret_cast<const MmaWorkEntry*>(a.gwork) + cur_entry;
+            if (a.gdirect == 2) {
+              a.out[(size_t)__ldg(&we->g.item[m]) * a.out_dim + r] = gelu_tanh(gate[k]) * fin[k];
+            } else {
+              float* dst = reinterpret_cast<float*>(__ldg(reinterpret_cast<const unsigned long long*>(&we->dst[m])));
+              if (r < __ldg(&we->room[m])) atomicAdd(dst + r, fin[k] * __ldg(&we->weight[m]));  // items may share a destination row
+            }
+          } else {
+            const int orow = a.gdirect ? __ldg(&entry_at(cur_entry)->item[m]) : cur_entry * MB + m;
+            a.out[(size_t)orow * a.out_dim + sw.mat * (a.gtpe * kTileRows) + r] = fin[k];
+          }
+        }
+      } else if (a.cluster) {
+        have = true;
+        break;  // the CTA's one item: below
       } else if (a.splits == 1) {
-        if (half == 0) {
 #pragma unroll
-          for (int m = 0; m < MB; ++m) {
-            if (m < a.batch && row < a.out_dim) a.out[(size_t)m * a.out_dim + row] = acc[m];
-            acc[m] = 0.f;
-          }
+        for (int k = 0; k < C::kVals; ++k) {
+          const int m = act(k), r = row + 16 * (k / NT);
+          if (mine && m < a.batch && r < a.out_dim) a.out[(size_t)m * a.out_dim + r] = fin[k];
         }
-        TP(if (tr && et == 0 && i < 16) g_mma_trace[7][10] = clock64();)
-        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");  // pair is free for the next item
-        TP(if (tr && et == 0 && i < 16) g_mma_trace[7][11] = clock64();)
       } else {
-        // Partial sums of this K range go to scratch; the CTA that arrives last at the tile adds the
+        // Partial sums of this K range go to scratch; the warp that arrives last at its rows of the tile adds the
         // partials in split order (so the result does not depend on arrival order) and stores.
-        if (half == 0) {
-          float* part = a.scratch + ((size_t)tile * a.splits + split) * (MB * kTileRows);
+        constexpr int kPart = C::kVals * 32;
+        float* part = a.scratch + (((size_t)sw.tile * a.splits + sw.split) * C::kStoring + slot) * kPart + lane;
 #pragma unroll
-          for (int m = 0; m < MB; ++m) {
-            part[m * kTileRows + r] = acc[m];
-            acc[m] = 0.f;
-          }
+        for (int k = 0; k < C::kVals; ++k) part[k * 32] = fin[k];
+        __threadfence();
+        __syncwarp();
+        unsigned int n = 0;
+        if (lane == 0) n = atomicAdd(a.counters + sw.tile * kConsumers + slot, 1u);
+        n = __shfl_sync(0xffffffffu, n, 0);
+        if (n == (unsigned)a.splits - 1) {
           __threadfence();
-        }
-        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
-        if (et == 0) *last_flag = (atomicAdd(a.counters + tile, 1u) == (unsigned)a.splits - 1) ? 1 : 0;
-        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
-        if (*last_flag && half == 0) {
-          __threadfence();
-          const float* base = a.scratch + (size_t)tile * a.splits * (MB * kTileRows);
+          const float* base = a.scratch + ((size_t)sw.tile * a.splits * C::kStoring + slot) * kPart + lane;
 #pragma unroll
-          for (int m = 0; m < MB; ++m) {
+          for (int k = 0; k < C::kVals; ++k) {
             float sum = 0.f;
-            for (int s2 = 0; s2 < a.splits; ++s2) sum += __ldcg(base + (size_t)s2 * (MB * kTileRows) + m * kTileRows + r);
-            if (m < a.batch && row < a.out_dim) a.out[(size_t)m * a.out_dim + row] = sum;
+            for (int s2 = 0; s2 < a.splits; ++s2) sum += __ldcg(base + (size_t)s2 * (C::kStoring * kPart) + k * 32);
+            const int m = act(k), r = row + 16 * (k / NT);
+            if (mine && m < a.batch && r < a.out_dim) a.out[(size_t)m * a.out_dim + r] = sum;
           }
-          if (et == 0) a.counters[tile] = 0;
+          if (lane == 0) a.counters[sw.tile * kConsumers + slot] = 0;
         }
-        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
+      }
+    }
+    if (!ok && lane == 0) *gave_up = 1;
+    if (a.cluster) {
+      // The K splits of this tile are the CTAs of this cluster (rank == split) and each has this one item.  Ranks above 0
+      // put their sums into rank 0's shared memory; rank 0 adds them in split order, the order of the scratch path.
+      __syncwarp();
+      asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+      if (have && sw.split != 0) {
+        const uint32_t dst = cluster_map(smem_u32(recv + (size_t)(sw.split - 1) * (C::kRecv / 4) + slot * (C::kVals * 32) + lane), 0);
+#pragma unroll
+        for (int k = 0; k < C::kVals; ++k) cluster_store_f32(dst + k * 128, fin[k]);
+      }
+      __syncwarp();
+      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+      if (sw.split == 0) {
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (have) {
+          const int row = sw.tile * kTileRows + row0 + g + 8 * p;
+#pragma unroll
+          for (int k = 0; k < C::kVals; ++k) {
+            float sum = fin[k];
+            for (int s2 = 1; s2 < a.splits; ++s2) sum += recv[(size_t)(s2 - 1) * (C::kRecv / 4) + slot * (C::kVals * 32) + k * 32 + lane];
+            const int m = MB == 1 ? 0 : 2 * (k % NT) + half, r = row + 16 * (k / NT);
+            if ((MB > 1 || t < 2) && m < a.batch && r < a.out_dim) a.out[(size_t)m * a.out_dim + r] = sum;
+          }
+        }
       }
     }
   }
-
-  TP(if (tr && tid == 0) g_mma_trace[7][1] = clock64();)
-  // ---- wind down: everyone meets, outstanding copies are drained, TMEM is returned ----
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  if (a.cluster && warp == kConsumers) {
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    if (blockIdx.x % a.splits == 0) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+  // ---- wind down: outstanding copies are drained ----
   __syncthreads();
-  if (warp == kWarpTMA && lane == 0 && *reinterpret_cast<volatile int*>(a.status) != 0) {
+  if (*gave_up && warp == kConsumers && lane == 0) {
     // a waiter gave up: copies may still be in flight; give each ring slot a bounded chance to land
     for (int s = 0; s < S; ++s) {
       long long t0 = clock64();
       while (!mbar_try_wait(full0 + 8 * s, 0) && !mbar_try_wait(full0 + 8 * s, 1) && clock64() - t0 < kTimeoutCycles / 8) {
       }
     }
-  }
-  __syncthreads();
-  if (warp == kWarpMMA) {
-    __syncwarp();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kCols) : "memory");
   }
 }
 
@@ -1021,13 +958,13 @@ __global__ void mlx_tile_kernel(const uint32_t* __restrict__ qw, const uint32_t*
   int r = rem / 9, u = rem - r * 9;
   int row = tile * 128 + r;
   uint4 v = make_uint4(0, 0, 0, 0);
-  unsigned char* dst = tiled + blk * kStageBytes;
+  unsigned char* dst = tiled + blk * Fmt<FMT_MLX4>::kStageBytes;
   if (u < 8) {
     if (row < out_dim) v = *reinterpret_cast<const uint4*>(qw + (size_t)row * (in_dim / 8) + chunk * 32 + u * 4);
     *reinterpret_cast<uint4*>(dst + r * 128 + ((u ^ (r & 7)) << 4)) = v;
   } else {
     if (row < out_dim) v = *reinterpret_cast<const uint4*>(sb + (size_t)row * (in_dim / 64) + chunk * 4);
-    *reinterpret_cast<uint4*>(dst + kStageWBytes + r * 16) = v;
+    *reinterpret_cast<uint4*>(dst + Fmt<FMT_MLX4>::kStageWBytes + r * 16) = v;
   }
 }
 
@@ -1037,7 +974,7 @@ bool mlx_mma_supported(const goph_mlx_weight* w) {
 
 int mlx_mma_make_tiled(goph_mlx_weight* w) {
   int ntiles = (w->out_dim + kTileRows - 1) / kTileRows, nchunks = w->in_dim / kChunkK;
-  size_t bytes = (size_t)ntiles * nchunks * kStageBytes;
+  size_t bytes = (size_t)ntiles * nchunks * Fmt<FMT_MLX4>::kStageBytes;
   unsigned char* t = nullptr;
   GOPH_CUDA(cudaMalloc(&t, bytes));
   size_t threads = (size_t)ntiles * nchunks * 128 * 9;
@@ -1055,20 +992,18 @@ int mlx_mma_make_tiled(goph_mlx_weight* w) {
 }
 
 struct MmaDeviceBufs {
-  unsigned char* xb = nullptr;  // prepared B operand of the launch in flight
-  float* xtab = nullptr;        // prepared per-(row, group) tables
+  unsigned char* xb = nullptr;  // prepared activations of the launch in flight
   int* status = nullptr;
   float* scratch = nullptr;
   unsigned int* counters = nullptr;
 };
 // Fixed-size device scratch of the split-K fix-up: at most 2 x 160 items of 128 rows x 8
-// activation rows, plus one counter per tile.  Allocated once per device.
+// activation rows, plus a counter per tile and warp.  Allocated once per device.
 constexpr size_t kScratchFloats = (size_t)2 * 160 * kTileRows * 8;
-constexpr size_t kMaxCounters = 4096;
-// Prepared activations: up to 8 rows of up to 65536 elements (B operand: 32 rows x in_dim bytes).
+constexpr size_t kMaxCounters = 4096 * kConsumers;
+// Prepared activations: up to 8 rows of up to 65536 elements.
 constexpr int kMaxPrepIn = 65536;  // mlx_mma_supported's bound on in_dim
-constexpr size_t kPrepXbBytes = (size_t)32 * kMaxPrepIn;
-constexpr size_t kPrepTabFloats = (size_t)2 * 8 * (kMaxPrepIn / 32);
+constexpr size_t kPrepXbBytes = (size_t)(kMaxPrepIn / kChunkK) * XBlock<FMT_Q4K, 8>::kBytes;
 
 // The buffers of a device are allocated on first use.  Nothing is published until every
 // allocation has succeeded (a failure frees what it got and the next call tries again), and
@@ -1083,8 +1018,7 @@ static MmaDeviceBufs* device_bufs(int device) {
   bool ok = cudaMalloc(&b.status, sizeof(int)) == cudaSuccess &&
             cudaMalloc(&b.scratch, kScratchFloats * sizeof(float)) == cudaSuccess &&
             cudaMalloc(&b.counters, kMaxCounters * sizeof(unsigned int)) == cudaSuccess &&
-            cudaMalloc(&b.xb, kPrepXbBytes) == cudaSuccess &&
-            cudaMalloc(&b.xtab, kPrepTabFloats * sizeof(float)) == cudaSuccess;
+            cudaMalloc(&b.xb, kPrepXbBytes) == cudaSuccess;
   ok = ok && cudaMemset(b.xb, 0, kPrepXbBytes) == cudaSuccess && cudaMemset(b.status, 0, sizeof(int)) == cudaSuccess &&
        cudaMemset(b.counters, 0, kMaxCounters * sizeof(unsigned int)) == cudaSuccess &&
        cudaDeviceSynchronize() == cudaSuccess;
@@ -1094,7 +1028,6 @@ static MmaDeviceBufs* device_bufs(int device) {
     cudaFree(b.scratch);
     cudaFree(b.counters);
     cudaFree(b.xb);
-    cudaFree(b.xtab);
     return nullptr;
   }
   bufs[device] = b;
@@ -1118,88 +1051,67 @@ int mlx_mma_status(int device) {
 struct TiledDesc {
   const unsigned char* tiled;
   int device, out_dim, in_dim;
+  size_t scratch_bytes = kScratchFloats * sizeof(float), counters = kMaxCounters;
 };
 
-constexpr size_t kMmaSmemBudget = 222 * 1024;  // of the 227 KiB a CTA may have
-constexpr int kMaxStages = 10;
+// Shared memory of a CTA: half of an SM's, so that two CTAs share one (the next launch's first stages are under way while
+// this one ends), or all of it where the activations do not leave the ring its stages.
+constexpr size_t kHalfSmem = 113 * 1024, kWholeSmem = 222 * 1024;
 
-// Clusters of `size` CTAs of the tensor-core GEMV that the device can hold at once (every such CTA
-// takes a whole SM, so this is a property of how the SMs are grouped); asked once per device.
-static int cluster_room(int device, int size);
-
-// K split: enough (tile, split) items to occupy the SMs, bounded by the chunks and the scratch.
-template <int MB>
-static int choose_splits(const MmaArgs& a, int sm_count, int device) {
-  int splits = 1;
-  if (a.ntiles < sm_count) {
-    splits = sm_count / a.ntiles;
-    if (splits > a.nchunks) splits = a.nchunks;
-    if (splits < 1) splits = 1;
-    // The cheap way to add the splits' partial sums needs all clusters of `splits` CTAs resident at
-    // once.  Where that many do not fit (48 tiles x 3: room for 45), fewer splits that do fit are the
-    // better trade (6144 x 4096: 7.7 us with 2 splits in clusters against 8.3 us with 3 through scratch).
-    if (options().mlx_cluster && splits > 2 && splits <= 8 && cluster_room(device, splits) < a.ntiles) {
-      for (int s2 = splits - 1; s2 >= 2; --s2) {
-        if (cluster_room(device, s2) >= a.ntiles) {
-          splits = s2;
-          break;
+// Clusters of `splits` CTAs that the device holds at once, one or two CTAs to an SM (a property of how the SMs are grouped:
+// every instantiation has the same threads and registers); asked once per device.
+static int cluster_room(int device, int splits, bool whole) {
+  static std::mutex mu;
+  static int room[kMaxDevices][2][kMaxSplits + 1];
+  static bool known[kMaxDevices] = {};
+  std::lock_guard<std::mutex> lock(mu);
+  if (!known[device]) {
+    auto kern = mlx_mma_kernel<FMT_MLX4, 1, true>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWholeSmem);
+    for (int w = 0; w < 2; ++w) {
+      for (int n = 2; n <= kMaxSplits; ++n) {
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = n;
+        attr.val.clusterDim.y = 1;
+        attr.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg;
+        memset(&cfg, 0, sizeof cfg);
+        cfg.gridDim = dim3(n * 64);
+        cfg.blockDim = dim3(kThreads);
+        cfg.dynamicSmemBytes = w ? kWholeSmem : kHalfSmem;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&room[device][w][n], kern, &cfg) != cudaSuccess) {
+          cudaGetLastError();
+          room[device][w][n] = 0;
         }
       }
     }
-  }
-  if (options().mlx_splits > 0) splits = options().mlx_splits < a.nchunks ? options().mlx_splits : a.nchunks;
-  while (splits > 1 && ((size_t)a.ntiles * splits * kTileRows * MB > kScratchFloats || (size_t)a.ntiles > kMaxCounters)) --splits;
-  return splits;
-}
-
-int g_mma_dbg = 0;  // tuning build only
-
-static int cluster_room(int device, int size) {
-  static std::mutex mu;
-  static int room[kMaxDevices][9];
-  static bool known[kMaxDevices] = {};
-  if (device < 0 || device >= kMaxDevices || size < 2 || size > 8) return 0;
-  std::lock_guard<std::mutex> lock(mu);
-  if (!known[device]) {
-    auto kern = mlx_mma_kernel<8, 4, 1, FMT_MLX4, false, 2>;
-    const size_t smem = 200 * 1024;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    for (int sz = 2; sz <= 8; ++sz) {
-      cudaLaunchAttribute attr;
-      attr.id = cudaLaunchAttributeClusterDimension;
-      attr.val.clusterDim.x = sz;
-      attr.val.clusterDim.y = 1;
-      attr.val.clusterDim.z = 1;
-      cudaLaunchConfig_t cfg;
-      memset(&cfg, 0, sizeof cfg);
-      cfg.gridDim = dim3(sz * 64);
-      cfg.blockDim = dim3(mma_threads<8, FMT_MLX4>());
-      cfg.dynamicSmemBytes = smem;
-      cfg.attrs = &attr;
-      cfg.numAttrs = 1;
-      int n = 0;
-      if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        n = 0;
-      }
-      room[device][sz] = n;
-    }
     known[device] = true;
   }
-  return room[device][size];
+  return room[device][whole][splits];
 }
 
-template <int N, int DIGITS, int MB, int FMT, bool FUSED, int C>
-static int launch_impl(const TiledDesc& w, const MmaArgs& a0, cudaStream_t stream, SharedX* xs, int stages, int splits) {
-  MmaArgs a = a0;
-  a.dbg = g_mma_dbg;
-  DeviceState& st = device_state(w.device);
-  a.stages = stages;
+// How a product is cut up and who prepares its activations.
+struct RowPlan {
+  bool own, whole;  // by the product's CTAs themselves, each for its K range; one CTA to an SM
+  int splits;
+  bool cluster;
+};
+
+template <int FMT, int MB, bool FUSED>
+static int launch_impl(const TiledDesc& w, MmaArgs a, cudaStream_t stream, SharedX* xs, const RowPlan& plan) {
+  typedef RowSmem<FMT, MB, FUSED, false> M;
+  const int splits = plan.splits;
   a.splits = splits;
   a.items = a.ntiles * splits;
   a.cmax = (a.nchunks + splits - 1) / splits;
-  size_t smem = MmaSmem<N, FMT, FUSED, C>::bytes(stages, a.batch, a.in_dim, a.cmax);
-  if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM
+  a.cluster = plan.cluster;
+  const int recv = plan.cluster ? splits - 1 : 0;
+  a.stages = M::stages(plan.whole ? kWholeSmem : kHalfSmem, a.cmax, recv);
+  size_t smem = M::bytes(a.stages, a.cmax, recv);
+  if (plan.whole && smem <= kHalfSmem) smem = kHalfSmem + 1024;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = options().pdl ? 1 : 0;
@@ -1213,105 +1125,86 @@ static int launch_impl(const TiledDesc& w, const MmaArgs& a0, cudaStream_t strea
     cfg.gridDim = dim3(a.batch * a.nchunks);
     cfg.blockDim = dim3(128);
     note_launch();
-    GOPH_CUDA(cudaLaunchKernelEx(&cfg, mlx_prep_x_kernel<DIGITS, FMT != FMT_MLX4, !Fmt<FMT>::kConv, FMT == FMT_Q6K>, a.x,
-                                 const_cast<unsigned char*>(a.xb), const_cast<float*>(a.xtab), a.batch, a.in_dim, N));
+    GOPH_CUDA(cudaLaunchKernelEx(&cfg, mlx_prep_x_kernel<FMT, MB>, a.x, const_cast<unsigned char*>(a.xb), a.in_dim, a.digits));
     xs->prepared = true;
   }
-  auto kern = mlx_mma_kernel<N, DIGITS, MB, FMT, FUSED, C>;
-  GOPH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int grid = a.items < st.sm_count ? a.items : st.sm_count;
+  auto kern = mlx_mma_kernel<FMT, MB, FUSED>;
+  static bool sized[kMaxDevices] = {};
+  if (!sized[w.device]) {
+    GOPH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWholeSmem));
+    sized[w.device] = true;
+  }
+  const int slots = device_state(w.device).sm_count * (plan.whole ? 1 : 2);
+  int grid = a.items < slots ? a.items : slots;
   // FUSED: a CTA prepares the activations of one K range, so all its items must be of one split:
   // item w is split w % splits, and a grid that is a multiple of the splits keeps that fixed per CTA
   if (FUSED && a.items > grid) grid -= grid % splits;
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(mma_threads<N, FMT>());
+  cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = smem;
-  int cluster_room = -1;
-  // K splits whose CTAs all run at once, one item each: the CTAs of a tile form a cluster and add
-  // their partial sums through the first CTA's shared memory (no scratch, fence or atomic).  Only
-  // when the device can hold every cluster of the grid at the same time — a second wave of clusters
-  // would cost far more than the fix-up saves.
-  if (options().mlx_cluster && splits > 1 && splits <= 8 && a.items == grid && (splits - 1) * MB <= kClusterRecvRows) {
+  if (plan.cluster) {
     attr[1].id = cudaLaunchAttributeClusterDimension;
     attr[1].val.clusterDim.x = splits;
     attr[1].val.clusterDim.y = 1;
     attr[1].val.clusterDim.z = 1;
     cfg.numAttrs = 2;
-    static std::mutex mu;
-    static std::map<std::tuple<const void*, int, size_t, int>, int> fits;  // (kernel, splits, smem, device) -> clusters resident at once
-    const auto key = std::make_tuple((const void*)kern, splits, smem, w.device);
-    int resident = -1;
-    {
-      std::lock_guard<std::mutex> lock(mu);
-      auto it = fits.find(key);
-      if (it != fits.end()) resident = it->second;
-    }
-    if (resident < 0) {
-      if (cudaOccupancyMaxActiveClusters(&resident, kern, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        resident = 0;
-      }
-      std::lock_guard<std::mutex> lock(mu);
-      fits[key] = resident;
-    }
-    if (resident * splits >= grid) a.cluster = 1;
-    else cfg.numAttrs = 1;
-    cluster_room = resident;
   }
   // GOPH_TRACE_LAUNCH=1 in the environment: one line per tensor-core product with its launch plan
   static const bool trace = getenv("GOPH_TRACE_LAUNCH") != nullptr;
   if (trace)
-    fprintf(stderr, "goph: mlx_mma_kernel fmt=%d out=%d in=%d rows=%d grid=%d splits=%d stages=%d chunks/stage=%d fused=%d cluster=%d (room for %d clusters)\n",
-            FMT, a.out_dim, a.in_dim, a.batch, grid, splits, stages, C, (int)FUSED, a.cluster, cluster_room);
+    fprintf(stderr, "goph: mlx_mma_kernel fmt=%d out=%d in=%d rows=%d grid=%d splits=%d stages=%d fused=%d cluster=%d smem=%d\n", FMT, a.out_dim, a.in_dim, a.batch,
+            grid, splits, a.stages, (int)FUSED, a.cluster, (int)smem);
   note_launch();
   GOPH_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
   return GOPH_OK;
 }
 
-// Chunks per stage: two for the formats that convert, when a stage's A buffer and accumulators fit
-// the tensor memory twice.
-template <int N, int FMT>
-constexpr int stage_chunks() {
-  return (Fmt<FMT>::kConv && 2 * (2 * 64 + 2 * Fmt<FMT>::kBlocks * N) <= 512) ? 2 : 1;
-}
-
-template <int N, int DIGITS, int MB, int FMT, int C>
-static int launch_with_chunks(const TiledDesc& w, const MmaArgs& a, cudaStream_t stream, SharedX* xs) {
-  const int sms = device_state(w.device).sm_count;
-  const int splits = choose_splits<MB>(a, sms, w.device);
-  const int cmax = (a.nchunks + splits - 1) / splits;
-  // Narrow launches (one or two activation rows) make the digits of their own K range inside the product kernel, one launch
-  // instead of two, as long as the B tiles that stay resident leave the ring its stages: four do for one row, two rows
-  // want five (B200, us a call, launch in front / own digits, one row: MLX4 4096x14336 11.7 / 10.3, 28672x4096 17.1 / 14.9,
-  // Q4_K 4096x14336 12.8 / 11.8, Q8_0 14336x4096 13.8 / 12.5, with four stages Q4_K 28672x7168 30.4 / 30.3, Q6_K 28672x8192
-  // 47.2 / 46.0; two rows with four stages: MLX4 28672x8192 31.1 / 33.8).  Launches of 16 columns (three or four rows, two
-  // of Q4_K and Q6_K) do it where every warp has one chunk of one row at most (four rows, Q8_0 4096x4096 11.1 / 10.3,
-  // 28672x1024 11.7 / 10.0; with two each Q5_K 6144x4096 13.8 / 14.5).  So do MLX products whose K ranges are not cut although tiles are fewer than SMs: one
-  // item a CTA, nothing behind which a warp's second chunk hides (front / own, two rows, 10240x4096 own 1.06 of the time with weights from memory, 1.09 from
-  // the L2; 14336x4096 11.9 / 12.4; one row 10240x5120 1.03, 1.09.  Cut, or with a tile for every SM, it is 0.93 to 0.98 from memory for two rows,
-  // 0.95 to 1.02 for one, and 0.97 to 1.08 from the L2).  Option mlx_fuse = 0 always keeps the launch.
-  // So does an output that overlaps x: the CTAs of the product read x while others already store.
-  if (N <= 16 && options().mlx_fuse && !xs->written && splits <= sms && ((N == 8 && (FMT != FMT_MLX4 || splits > 1 || a.ntiles >= sms)) || a.batch * cmax < mma_threads<N, FMT>() / 32)) {
-    size_t fixed = MmaSmem<N, FMT, true, C>::bytes(0, a.batch, a.in_dim, cmax);
-    int stages = fixed < kMmaSmemBudget ? (int)((kMmaSmemBudget - fixed) / MmaSmem<N, FMT, true, C>::kStage) : 0;
-    if (stages > kMaxStages) stages = kMaxStages;
-    if (stages >= (MB == 1 ? 4 : 5)) return launch_impl<N, DIGITS, MB, FMT, N <= 16, C>(w, a, stream, xs, stages, splits);
-  }
-  size_t fixed = MmaSmem<N, FMT, false, C>::bytes(0, a.batch, a.in_dim);
-  int stages = fixed < kMmaSmemBudget ? (int)((kMmaSmemBudget - fixed) / MmaSmem<N, FMT, false, C>::kStage) : 0;
-  if (stages > kMaxStages) stages = kMaxStages;
-  if (stages < 3) {
-    if (C > 1) return launch_with_chunks<N, DIGITS, MB, FMT, 1>(w, a, stream, xs);
-    return fail(GOPH_E_UNSUPPORTED, "tensor-core path: activations of %d x %d leave no room for the ring", a.batch, a.in_dim);
-  }
-  return launch_impl<N, DIGITS, MB, FMT, false, C>(w, a, stream, xs, stages, splits);
-}
-
-template <int N, int DIGITS, int MB, int FMT>
+template <int FMT, int MB>
 static int launch_one(const TiledDesc& w, const MmaArgs& a, cudaStream_t stream, SharedX* xs) {
-  constexpr int C = stage_chunks<N, FMT>();
-  if (C > 1 && options().mlx_chunks != 1) return launch_with_chunks<N, DIGITS, MB, FMT, C>(w, a, stream, xs);
-  return launch_with_chunks<N, DIGITS, MB, FMT, 1>(w, a, stream, xs);
+  constexpr bool kBytes = !Fmt<FMT>::kNibble;
+  const int sms = device_state(w.device).sm_count, tiles = a.ntiles;
+  RowPlan p;
+  // The lines (B200, us a call, weights from HBM).  A CTA to an SM, with a ring of all that is left: products that are over in a few stages (one row, MLX4
+  // 4096x4096 4.4, two to an SM 4.6; 14336x4096 8.3 / 7.7), and several rows, whose activations leave half an SM too little (four rows 14336x4096 10.8 / 11.4;
+  // two of Q8_0 12.2 / 12.9).  By the CTAs themselves or in front: one row 4096x4096 4.4 / 6.2, 28672x4096 13.0 / 12.9,
+  // 28672x8192 24.5 / 22.5; two rows 4096x4096 4.6 / 6.9, 14336x4096 8.7 / 9.6, where nothing is cut 28672x4096 15.5 / 13.5 (Q8_0 22.6 / 21.3); four 4096x4096 6.1 / 6.3,
+  // 14336x4096 14.3 / 10.8.  Up to 17 chunks a CTA (two a warp) are its own.  MLX products of more than a tile for two SMs, fewer than one for each, and more than 17 chunks
+  // have theirs in front: 14000x4608 one row 9.1 / 9.4, two rows 14336x4096 8.7 / 9.6 (a call of several such weights prepares them once).
+  const bool small = (long)tiles * a.nchunks <= 8l * sms;
+  p.whole = small || MB == 8 || (MB == 4 && (FMT != FMT_MLX4 || tiles < sms)) || (MB == 2 && kBytes && tiles < sms);
+  auto cut = [&](bool whole) {
+    const int slots = sms * (whole ? 1 : 2);
+    int n = slots / tiles;
+    if (n > a.nchunks) n = a.nchunks;
+    if (n > kMaxSplits) n = kMaxSplits;
+    if (options().mlx_cluster)
+      while (n > 1 && cluster_room(w.device, n, whole) < tiles) --n;
+    if (options().mlx_splits > 0) n = options().mlx_splits < a.nchunks ? options().mlx_splits : a.nchunks;
+    while (n > 1 && ((size_t)tiles * n * RowCfg<FMT, MB, false>::kRecv > w.scratch_bytes || (size_t)tiles * kConsumers > w.counters)) --n;
+    p.whole = whole;
+    p.splits = n < 1 ? 1 : n;
+    p.cluster = options().mlx_cluster && n > 1 && n <= kMaxSplits && (long)tiles * n <= slots && cluster_room(w.device, n, whole) >= tiles;
+  };
+  cut(p.whole);
+  const int cmax = (a.nchunks + p.splits - 1) / p.splits;
+  if (MB == 1) p.own = p.splits > 1 || a.nchunks <= 24;
+  else if (MB == 2) p.own = small || (p.splits > 1 ? !kBytes : kBytes);
+  else p.own = false;
+  if (a.batch * cmax <= 17) p.own = true;
+  if (FMT == FMT_MLX4 && 2 * tiles > sms && tiles < sms && a.batch * a.nchunks > 17) p.own = false;
+  if (!options().mlx_fuse || xs->written || p.splits > sms) p.own = false;
+  constexpr int kLeast = 3;
+  for (int t = 0; t < 4; ++t) {  // a ring of three stages at least: else a whole SM, else a launch in front
+    const int recv = p.cluster ? p.splits - 1 : 0, range = (a.nchunks + p.splits - 1) / p.splits;
+    const size_t budget = p.whole ? kWholeSmem : kHalfSmem;
+    if (p.own && RowSmem<FMT, MB, true, false>::stages(budget, range, recv) >= kLeast) return launch_impl<FMT, MB, true>(w, a, stream, xs, p);
+    if (!p.own && RowSmem<FMT, MB, false, false>::stages(budget, range, recv) >= kLeast) return launch_impl<FMT, MB, false>(w, a, stream, xs, p);
+    if (!p.whole) cut(true);
+    else if (p.own) p.own = false;
+    else if (p.cluster) p.cluster = false;  // (the sums meet in scratch and need no shared memory)
+    else break;
+  }
+  return fail(GOPH_E_UNSUPPORTED, "tensor-core path: activations of %d x %d leave no room for the ring", a.batch, a.in_dim);
 }
 
 template <int FMT>
@@ -1326,37 +1219,23 @@ static int tiled_launch(const TiledDesc& w, float* out, const float* x, int batc
   a.scratch = bufs->scratch;
   a.counters = bufs->counters;
   a.xb = bufs->xb;
-  a.xtab = bufs->xtab;
   a.out_dim = w.out_dim;
   a.in_dim = w.in_dim;
+  a.digits = digits == 3 ? 3 : 4;
   a.ntiles = (w.out_dim + kTileRows - 1) / kTileRows;
   a.nchunks = w.in_dim / kChunkK;
-  // activation rows one launch can take: the accumulator blocks of a stage must fit TMEM twice
-  constexpr bool kQ4K = Fmt<FMT>::kHalves;  // Q4_K and Q6_K need two columns per digit
-  const int cap = kQ4K ? (digits == 3 ? 5 : 4) : 8;
+  constexpr int cap = 8;  // activation rows of a launch
   const bool written = shared ? shared->written : floats_meet(out, (uint64_t)batch * w.out_dim, x, (uint64_t)batch * w.in_dim);
   for (int b0 = 0; b0 < batch;) {
-    int nb = batch - b0 < cap ? batch - b0 : cap;
+    const int nb = batch - b0 < cap ? batch - b0 : cap;
     a.x = x + (size_t)b0 * w.in_dim;
     a.out = out + (size_t)b0 * w.out_dim;
     a.batch = nb;
     SharedX own;  // (rows of a later launch of this call do not have the scratch's activations)
     own.written = written;
     SharedX* xs = shared && batch <= cap ? shared : &own;
-    int rc;
-    if (digits == 3) {
-      if (kQ4K && nb == 1) rc = launch_one<8, 3, 1, FMT>(w, a, stream, xs);
-      else if (nb <= 2) rc = launch_one<kQ4K ? 16 : 8, 3, 2, FMT>(w, a, stream, xs);
-      else if (nb <= 5) rc = launch_one<kQ4K ? 32 : 16, 3, 5, FMT>(w, a, stream, xs);
-      else if (!kQ4K) rc = launch_one<32, 3, 8, kQ4K ? FMT_MLX4 : FMT>(w, a, stream, xs);
-      else rc = fail(GOPH_E_UNSUPPORTED, "batch slice too wide");
-    } else {
-      if (nb == 1) rc = launch_one<8, 4, 1, FMT>(w, a, stream, xs);
-      else if (nb == 2) rc = launch_one<kQ4K ? 16 : 8, 4, 2, FMT>(w, a, stream, xs);
-      else if (nb <= 4) rc = launch_one<kQ4K ? 32 : 16, 4, 4, FMT>(w, a, stream, xs);
-      else if (!kQ4K) rc = launch_one<32, 4, 8, kQ4K ? FMT_MLX4 : FMT>(w, a, stream, xs);
-      else rc = fail(GOPH_E_UNSUPPORTED, "batch slice too wide");
-    }
+    const int rc = nb == 1 ? launch_one<FMT, 1>(w, a, stream, xs) : nb == 2 ? launch_one<FMT, 2>(w, a, stream, xs) : nb <= 4 ? launch_one<FMT, 4>(w, a, stream, xs)
+                                                                                                                : launch_one<FMT, 8>(w, a, stream, xs);
     if (rc) return rc;
     b0 += nb;
   }
@@ -1377,11 +1256,10 @@ int mlx_mma_launch(const goph_mlx_weight* w, float* out, const float* x, int bat
 // the item's token in src[tokens][in_dim]; PHASE 1: silu(g) * u of the gate and up results
 // src[entry * MB + m][2][in_dim] (kernels.SiLU then the multiply, backends/simd/kernels/activation.go:15-24;
 // single-precision exp as in the CUDA-core expert kernels).
-template <int N, int MB, int PHASE>
+template <int MB, int PHASE>
 __global__ void __launch_bounds__(256)
 moe_mma_prep_kernel(const MmaGroupEntry* __restrict__ work, const int* __restrict__ count, int max_entries,
-                    const float* __restrict__ src, int in_dim, int top_k, unsigned char* __restrict__ xb, size_t xb_stride,
-                    float* __restrict__ xtab, int tab_stride) {
+                    const float* __restrict__ src, int in_dim, int top_k, unsigned char* __restrict__ xb, size_t xb_stride) {
   pdl_launch_dependents();
   pdl_wait();
   const int entry = blockIdx.x / MB, m = blockIdx.x - entry * MB;
@@ -1390,10 +1268,9 @@ moe_mma_prep_kernel(const MmaGroupEntry* __restrict__ work, const int* __restric
   if (entry >= live) return;
   const MmaGroupEntry* ge = work + entry;
   if (m >= ge->count) return;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, groups = in_dim / 64;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float* row = PHASE == 0 ? src + (size_t)(ge->item[m] / top_k) * in_dim : src + (size_t)(entry * MB + m) * 2 * in_dim;
   unsigned char* bdst = xb + (size_t)entry * xb_stride;
-  float* tab = xtab + (size_t)entry * tab_stride;
   for (int c = warp; c < in_dim / kChunkK; c += 8) {
     const int k = c * kChunkK + lane * 8;
     float v[8];
@@ -1404,7 +1281,7 @@ moe_mma_prep_kernel(const MmaGroupEntry* __restrict__ work, const int* __restric
 #pragma unroll
       for (int i = 0; i < 8; ++i) v[i] = __fmul_rn(__fdiv_rn(v[i], __fadd_rn(1.0f, expf(-v[i]))), u[i]);
     }
-    prep_chunk<4, false, false, false>(v, lane, bdst + (size_t)c * (N * 256), N, m, tab + m * groups + 4 * c, tab + (MB + m) * groups + 4 * c);
+    prep_chunk<FMT_MLX4, MB>(v, lane, bdst + (size_t)c * XBlock<FMT_MLX4, MB>::kBytes, m, 4);
   }
 }
 
@@ -1412,13 +1289,13 @@ bool mlx_mma_grouped_supported(int hidden, int inter) {
   return hidden % kChunkK == 0 && inter % kChunkK == 0 && hidden % kTileRows == 0 && inter % kTileRows == 0 && hidden <= 16384 &&
          inter <= 16384;
 }
-// four digits per activation row -> 4 * rows accumulator columns
-size_t mlx_mma_grouped_xb_bytes(int in_dim, int rows) { return (size_t)(in_dim / kChunkK) * (8 * 4 * rows * 32); }
-int mlx_mma_grouped_tab_floats(int in_dim, int rows) { return 2 * rows * (in_dim / 64); }
+size_t mlx_mma_grouped_xb_bytes(int in_dim, int rows) {
+  return (size_t)(in_dim / kChunkK) * (rows == 2 ? XBlock<FMT_MLX4, 2>::kBytes : XBlock<FMT_MLX4, 4>::kBytes);
+}
 
 template <int MB>
 static int launch_grouped(int device, const MmaGroupLaunch& g, cudaStream_t stream) {
-  constexpr int N = 4 * MB, C = stage_chunks<N, FMT_MLX4>();
+  typedef RowSmem<FMT_MLX4, MB, false, true> M;
   MmaDeviceBufs* bufs = device_bufs(device);
   if (!bufs) return fail(GOPH_E_NOMEM, "cannot allocate the tensor-core path's device scratch");
   DeviceState& st = device_state(device);
@@ -1426,11 +1303,11 @@ static int launch_grouped(int device, const MmaGroupLaunch& g, cudaStream_t stre
   memset(&a, 0, sizeof a);
   a.status = bufs->status;
   a.xb = g.xb;
-  a.xtab = g.xtab;
   a.out = g.out;
   a.out_dim = g.mats * g.rows;
   a.in_dim = g.in_dim;
   a.batch = MB;
+  a.digits = 4;
   a.ntiles = g.rows / kTileRows;
   a.nchunks = g.in_dim / kChunkK;
   a.splits = 1;
@@ -1442,16 +1319,9 @@ static int launch_grouped(int device, const MmaGroupLaunch& g, cudaStream_t stre
   a.gmats = g.mats;
   a.gfirst = g.first;
   a.gdirect = g.phase == 1;
-  a.gtab = mlx_mma_grouped_tab_floats(g.in_dim, MB);
   a.gxb = mlx_mma_grouped_xb_bytes(g.in_dim, MB);
-  a.dbg = g_mma_dbg;
-  size_t fixed = MmaSmem<N, FMT_MLX4, false, C>::bytes(0, MB, g.in_dim);
-  int stages = fixed < kMmaSmemBudget ? (int)((kMmaSmemBudget - fixed) / MmaSmem<N, FMT_MLX4, false, C>::kStage) : 0;
-  if (stages > kMaxStages) stages = kMaxStages;
-  if (stages < 3) return fail(GOPH_E_UNSUPPORTED, "tensor-core experts: %d columns leave no room for the ring", g.in_dim);
-  a.stages = stages;
-  size_t smem = MmaSmem<N, FMT_MLX4, false, C>::bytes(stages, MB, g.in_dim);
-  if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM
+  a.stages = M::stages(kHalfSmem, 0, 0);
+  const size_t smem = M::bytes(a.stages, 0, 0);
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = options().pdl ? 1 : 0;
@@ -1464,15 +1334,13 @@ static int launch_grouped(int device, const MmaGroupLaunch& g, cudaStream_t stre
   cfg.blockDim = dim3(256);
   note_launch();
   if (g.phase == 0)
-    GOPH_CUDA(cudaLaunchKernelEx(&cfg, moe_mma_prep_kernel<N, MB, 0>, g.work, g.count, g.max_entries, g.src, g.in_dim, g.top_k, g.xb,
-                                 a.gxb, g.xtab, a.gtab));
+    GOPH_CUDA(cudaLaunchKernelEx(&cfg, moe_mma_prep_kernel<MB, 0>, g.work, g.count, g.max_entries, g.src, g.in_dim, g.top_k, g.xb, a.gxb));
   else
-    GOPH_CUDA(cudaLaunchKernelEx(&cfg, moe_mma_prep_kernel<N, MB, 1>, g.work, g.count, g.max_entries, g.src, g.in_dim, g.top_k, g.xb,
-                                 a.gxb, g.xtab, a.gtab));
-  auto kern = mlx_mma_kernel<N, 4, MB, FMT_MLX4, false, C, true>;
+    GOPH_CUDA(cudaLaunchKernelEx(&cfg, moe_mma_prep_kernel<MB, 1>, g.work, g.count, g.max_entries, g.src, g.in_dim, g.top_k, g.xb, a.gxb));
+  auto kern = mlx_mma_kernel<FMT_MLX4, MB, false, true>;
   GOPH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  cfg.gridDim = dim3(a.items < st.sm_count ? a.items : st.sm_count);
-  cfg.blockDim = dim3(mma_threads<N, FMT_MLX4>());
+  cfg.gridDim = dim3(a.items < 2 * st.sm_count ? a.items : 2 * st.sm_count);
+  cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = smem;
   note_launch();
   GOPH_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
@@ -1767,9 +1635,7 @@ int gguf_mma_dequant(const goph_gguf_matrix* m, float* out, cudaStream_t stream)
 template <int FMT, int MB>
 __global__ void __launch_bounds__(256)
 work_prep_kernel(const __grid_constant__ MmaWorkLaunch g, MmaWorkEntry* __restrict__ work, int* __restrict__ count, unsigned char* __restrict__ xb, size_t gxb,
-                 float* __restrict__ xtab, int gtab, unsigned long long stage_bytes) {
-  typedef Fmt<FMT> F;
-  constexpr int N = 4 * MB * (F::kHalves ? 2 : 1);
+                 unsigned long long stage_bytes) {
   __shared__ __align__(16) int ex[kMaxWorkList], rank[kMaxWorkList];
   __shared__ int s_leader;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, w = blockIdx.x;
@@ -1826,27 +1692,22 @@ work_prep_kernel(const __grid_constant__ MmaWorkLaunch g, MmaWorkEntry* __restri
       we->weight[m] = __ldg(g.weight + w);
     }
   }
-  constexpr int kPer = kChunkK / F::kGroup;
-  const int ntab = g.in_dim / F::kGroup;
-  float* tab = xtab + (size_t)id * gtab;
 #pragma unroll 1
   for (int c = warp; c < g.in_dim / kChunkK; c += 8) {
     float v[8];
     load_eight(g.x + (size_t)w * g.in_dim + c * kChunkK + lane * 8, v);
-    prep_chunk<4, true, !F::kConv, FMT == FMT_Q6K>(v, lane, xb + (size_t)id * gxb + (size_t)c * (N * 256), N, m, tab + m * ntab + c * kPer,
-                                                   tab + (MB + m) * ntab + c * kPer);
+    prep_chunk<FMT, MB>(v, lane, xb + (size_t)id * gxb + (size_t)c * XBlock<FMT, MB>::kBytes, m, 4);
   }
 }
 
-// A list's launches, and where their parts lie in the scratch: entries, their number, tables, B tiles.
+// A list's launches, and where their parts lie in the scratch: entries, their number, prepared activations.
 struct WorkPlan {
   MmaArgs a;
-  size_t smem, count_at, tab_at, xb_at, bytes;
+  size_t smem, count_at, xb_at, bytes;
 };
 template <int FMT, int MB>
 static WorkPlan plan_work(const MmaWorkLaunch& g) {
-  constexpr int N = 4 * MB * (Fmt<FMT>::kHalves ? 2 : 1), C = stage_chunks<N, FMT>();
-  typedef MmaSmem<N, FMT, false, C> Smem;
+  typedef RowSmem<FMT, MB, false, true> M;
   WorkPlan p;
   memset(&p, 0, sizeof p);
   MmaArgs& a = p.a;
@@ -1854,23 +1715,19 @@ static WorkPlan plan_work(const MmaWorkLaunch& g) {
   a.out_dim = g.rows;
   a.in_dim = g.in_dim;
   a.batch = MB;
+  a.digits = 4;
   a.ntiles = a.gtpe = g.rows / kTileRows;
   a.nchunks = g.in_dim / kChunkK;
   a.splits = 1;
   a.gmats = g.mats;
   a.gdirect = g.pos ? 3 : 2;
-  a.gtab = 2 * MB * (g.in_dim / Fmt<FMT>::kGroup);
-  a.gxb = (size_t)a.nchunks * N * 256;
+  a.gxb = (size_t)a.nchunks * XBlock<FMT, MB>::kBytes;
   // at most so many entries: every expert may have one that is not full
   const int most_entries = (int)(((long long)g.items + (long long)(g.active < g.items ? g.active : g.items) * (MB - 1)) / MB);
   a.gmax = most_entries < g.items ? most_entries : g.items;
   a.items = a.gmax * g.mats * a.ntiles;
-  const size_t fixed = Smem::bytes(0, MB, g.in_dim);
-  a.stages = fixed < kMmaSmemBudget ? (int)((kMmaSmemBudget - fixed) / Smem::kStage) : 0;
-  if (a.stages > kMaxStages) a.stages = kMaxStages;
-  if (a.stages < 3) return p;
-  p.smem = Smem::bytes(a.stages, MB, g.in_dim);
-  if (p.smem < 120 * 1024) p.smem = 120 * 1024;  // one CTA per SM
+  a.stages = M::stages(kHalfSmem, 0, 0) >= 4 ? M::stages(kHalfSmem, 0, 0) : M::stages(kWholeSmem, 0, 0);
+  p.smem = M::bytes(a.stages, 0, 0);
   auto place = [&](size_t bytes) {
     const size_t at = p.bytes;
     p.bytes += (bytes + 255) & ~(size_t)255;
@@ -1878,26 +1735,22 @@ static WorkPlan plan_work(const MmaWorkLaunch& g) {
   };
   place((size_t)a.gmax * sizeof(MmaWorkEntry));
   p.count_at = place(sizeof(int));
-  p.tab_at = place((size_t)a.gmax * a.gtab * 4);
   p.xb_at = place((size_t)a.gmax * a.gxb);
   return p;
 }
 
 template <int FMT, int MB>
 static int launch_work(int device, const MmaWorkLaunch& g, unsigned char* scratch, int* status, cudaStream_t stream) {
-  constexpr int N = 4 * MB * (Fmt<FMT>::kHalves ? 2 : 1), C = stage_chunks<N, FMT>();
   WorkPlan p = plan_work<FMT, MB>(g);
   MmaArgs& a = p.a;
   MmaWorkEntry* work = reinterpret_cast<MmaWorkEntry*>(scratch);
   int* count = reinterpret_cast<int*>(scratch + p.count_at);
-  float* xtab = reinterpret_cast<float*>(scratch + p.tab_at);
   unsigned char* xb = scratch + p.xb_at;
   a.status = status;
   a.gwork = reinterpret_cast<const MmaGroupEntry*>(work);
   a.gcount = count;
   a.xb = xb;
-  a.xtab = xtab;
-  auto kern = mlx_mma_kernel<N, 4, MB, FMT, false, C, true>;
+  auto kern = mlx_mma_kernel<FMT, MB, false, true>;
   GOPH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1910,10 +1763,10 @@ static int launch_work(int device, const MmaWorkLaunch& g, unsigned char* scratc
   cfg.gridDim = dim3(g.items);
   cfg.blockDim = dim3(256);
   note_launch();
-  GOPH_CUDA(cudaLaunchKernelEx(&cfg, work_prep_kernel<FMT, MB>, g, work, count, xb, a.gxb, xtab, a.gtab, (unsigned long long)Fmt<FMT>::kStageBytes));
-  const int sms = device_state(device).sm_count, most = a.items / (g.pos ? 1 : 2);
-  cfg.gridDim = dim3(most < sms ? most : sms);
-  cfg.blockDim = dim3(mma_threads<N, FMT>());
+  GOPH_CUDA(cudaLaunchKernelEx(&cfg, work_prep_kernel<FMT, MB>, g, work, count, xb, a.gxb, (unsigned long long)Fmt<FMT>::kStageBytes));
+  const int slots = device_state(device).sm_count * (p.smem <= kHalfSmem ? 2 : 1), most = a.items / (g.pos ? 1 : 2);
+  cfg.gridDim = dim3(most < slots ? most : slots);
+  cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = p.smem;
   note_launch();
   GOPH_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
@@ -1971,15 +1824,14 @@ int gguf_mma_launch_work(const goph_gguf_matrix* m, const MmaWorkLaunch& g0, uns
 // cudaMalloc.  Every GPU that loads the library carries the array until the process exits.
 constexpr int kNoAllocMaxIn = 16384;     // largest in_dim the entry point accepts
 constexpr int kNoAllocMaxTiles = 4096;   // largest ceil(out_dim / 128)
-constexpr int kNoAllocMaxItems = 192;    // (tile, split) items that may have partial sums at once
+constexpr int kNoAllocMaxItems = 320;    // (tile, split) items that may have partial sums at once
 constexpr size_t kNaStatusOff = 0;
 constexpr size_t kNaCountersOff = 256;
-constexpr size_t kNaTabOff = kNaCountersOff + (size_t)kNoAllocMaxTiles * 4;
-constexpr size_t kNaXbOff = kNaTabOff + (size_t)2 * (kNoAllocMaxIn / 64) * 4;
-constexpr size_t kNaPartOff = kNaXbOff + (size_t)8 * kNoAllocMaxIn;
-constexpr size_t kNoAllocBytes = kNaPartOff + (size_t)kNoAllocMaxItems * kTileRows * 4;
-static_assert(kNaTabOff % 256 == 0 && kNaXbOff % 256 == 0 && kNaPartOff % 256 == 0, "256-byte aligned regions");
-static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];  // 248,064 bytes
+constexpr size_t kNaXbOff = kNaCountersOff + (size_t)kNoAllocMaxItems * kConsumers * 4;  // (tiles that are cut are fewer than the items)
+constexpr size_t kNaPartOff = kNaXbOff + (size_t)(kNoAllocMaxIn / kChunkK) * XBlock<FMT_MLX4, 1>::kBytes;
+constexpr size_t kNoAllocBytes = kNaPartOff + (size_t)kNoAllocMaxItems * RowCfg<FMT_MLX4, 1, false>::kRecv;
+static_assert(kNaXbOff % 256 == 0 && kNaPartOff % 256 == 0, "256-byte aligned regions");
+static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 
 // Device address of the array on `device` (which must be current).  In host code the array's
 // name is only a handle for the runtime, never a pointer a kernel could use, so the address is
@@ -1997,11 +1849,7 @@ static int noalloc_base(int device, unsigned char** base) {
   return GOPH_OK;
 }
 
-template <int DIGITS>
-static int launch_noalloc(const goph_mlx_weight* w, float* out, const float* x, unsigned char* base,
-                          cudaStream_t stream) {
-  constexpr int N = 8, MB = 1;
-  DeviceState& st = device_state(w->device);
+static int launch_noalloc(const goph_mlx_weight* w, float* out, const float* x, unsigned char* base, int digits, cudaStream_t stream) {
   MmaArgs a;
   memset(&a, 0, sizeof a);
   a.w = w->tiled;
@@ -2009,71 +1857,30 @@ static int launch_noalloc(const goph_mlx_weight* w, float* out, const float* x, 
   a.out = out;
   a.status = reinterpret_cast<int*>(base + kNaStatusOff);
   a.counters = reinterpret_cast<unsigned int*>(base + kNaCountersOff);
-  a.xtab = reinterpret_cast<const float*>(base + kNaTabOff);
   a.xb = base + kNaXbOff;
   a.scratch = reinterpret_cast<float*>(base + kNaPartOff);
   a.out_dim = w->out_dim;
   a.in_dim = w->in_dim;
   a.batch = 1;
+  a.digits = digits == 3 ? 3 : 4;
   a.ntiles = (w->out_dim + kTileRows - 1) / kTileRows;
   a.nchunks = w->in_dim / kChunkK;
-  size_t fixed = MmaSmem<N>::bytes(0, 1, a.in_dim);
-  int stages = (int)(((size_t)kSmemBudget - fixed) / MmaSmem<N>::kStage);
-  if (stages > 8) stages = 8;
-  a.stages = stages;
-  int splits = 1;
-  if (a.ntiles < st.sm_count) {
-    splits = st.sm_count / a.ntiles;
-    if (splits > a.nchunks) splits = a.nchunks;
-    if (splits < 1) splits = 1;
-  }
-  while (splits > 1 && a.ntiles * splits > kNoAllocMaxItems) --splits;
-  a.splits = splits;
-  a.items = a.ntiles * splits;
-  a.cmax = 0;
-  // The array keeps whatever the last call left: the tile counters have to start at zero (the
-  // digits, tables and partial sums are fully rewritten before they are read).  The status word is
+  // The array keeps whatever the last call left: the arrival counters have to start at zero (the prepared activations and
+  // partial sums are fully rewritten before they are read).  The status word is
   // left alone: it is zero when the library is loaded and sticky once a wait has given up, like the
   // allocated path's; goph_mlx_gemv_noalloc_status reads it.
-  GOPH_CUDA(cudaMemsetAsync(base + kNaCountersOff, 0, kNaTabOff - kNaCountersOff, stream));
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 0;  // plain stream order behind the memset
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof cfg);
-  cfg.stream = stream;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  cfg.gridDim = dim3(a.nchunks);
-  cfg.blockDim = dim3(128);
-  note_launch();
-  GOPH_CUDA(cudaLaunchKernelEx(&cfg, mlx_prep_x_kernel<DIGITS>, a.x, const_cast<unsigned char*>(a.xb),
-                               const_cast<float*>(a.xtab), 1, a.in_dim, N));
-  size_t smem = MmaSmem<N>::bytes(stages, 1, a.in_dim);
-  if (smem < 120 * 1024) smem = 120 * 1024;
-  auto kern = mlx_mma_kernel<N, DIGITS, MB>;
-  GOPH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  cfg.gridDim = dim3(a.items < st.sm_count ? a.items : st.sm_count);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = smem;
-  note_launch();
-  GOPH_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
-  return GOPH_OK;
+  GOPH_CUDA(cudaMemsetAsync(base + kNaCountersOff, 0, kNaXbOff - kNaCountersOff, stream));
+  TiledDesc d{w->tiled, w->device, w->out_dim, w->in_dim};
+  d.scratch_bytes = kNoAllocBytes - kNaPartOff;
+  d.counters = kNoAllocMaxItems * kConsumers;
+  SharedX xs;
+  xs.written = floats_meet(out, w->out_dim, x, w->in_dim);
+  return launch_one<FMT_MLX4, 1>(d, a, stream, &xs);
 }
 
 }  // namespace goph
 
 using namespace goph;
-
-#ifdef GOPH_TUNING
-GOPH_API int goph_tuning_set_gemv(int dbg) {
-  goph::g_mma_dbg = dbg;
-  return 0;
-}
-GOPH_API int goph_tuning_probe_gemv(long long* out512) {
-  return cudaMemcpyFromSymbol(out512, g_mma_trace, 8 * 64 * sizeof(long long)) == cudaSuccess ? 0 : -1;
-}
-#endif
 
 GOPH_API int goph_mlx_gemv_noalloc_status(int device, int* out_status) {
   clear_error();
@@ -2106,6 +1913,5 @@ GOPH_API int goph_mlx_gemv_noalloc(float* out_dev, uint64_t out_len, const float
   if (int rc = use_device(w->device)) return rc;
   unsigned char* base = nullptr;
   if (int rc = noalloc_base(w->device, &base)) return rc;
-  return options().mlx_digits == 3 ? launch_noalloc<3>(w, out_dev, x_dev, base, (cudaStream_t)stream)
-                                   : launch_noalloc<4>(w, out_dev, x_dev, base, (cudaStream_t)stream);
+  return launch_noalloc(w, out_dev, x_dev, base, options().mlx_digits, (cudaStream_t)stream);
 }

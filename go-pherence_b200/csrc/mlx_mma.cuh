@@ -44,9 +44,8 @@ struct __align__(16) MmaGroupEntry {
 };
 // True when experts of [inter x hidden] / [hidden x inter] can run as grouped launches.
 bool mlx_mma_grouped_supported(int hidden, int inter);
-// Bytes of prepared activations and floats of tables one entry of `rows` items needs for an input of in_dim.
+// Bytes of prepared activations one entry of `rows` items needs for an input of in_dim.
 size_t mlx_mma_grouped_xb_bytes(int in_dim, int rows);
-int mlx_mma_grouped_tab_floats(int in_dim, int rows);
 struct MmaGroupLaunch {
   const MmaGroupEntry* work;  // device
   const int* count;           // device: live entries
@@ -58,7 +57,6 @@ struct MmaGroupLaunch {
   int top_k;
   const float* src;
   unsigned char* xb;          // [max_entries][xb_bytes]
-  float* xtab;                // [max_entries][tab_floats]
   float* out;                 // phase 0: [max_entries * entry_rows][mats * rows]; phase 1: [items][rows]
 };
 // Two launches: the entries' activations as digits, sums and scales; then the products.

@@ -87,7 +87,6 @@ struct goph_moe_layer {
   int max_entries;                 // work entries (expert, up to two items) a call can have
   goph::MmaGroupEntry* mwork;      // [max_entries]
   unsigned char* mxb;              // [max_entries] prepared activations of an entry
-  float* mxtab;                    // [max_entries] their sums and scales
   float* gu;                       // [max_entries * 2][2][inter] gate and up results (entries of two or four items: the first holds more entries)
   // one token, row-major experts: the whole call as one cooperative launch
   unsigned* bar;                   // [0] barrier counter (only grows), [1] its value when the next launch starts, [2] set when a wait gave up
@@ -1046,26 +1045,22 @@ GOPH_API int goph_moe_set_expert(goph_moe_layer* m, int eid, const goph_mlx_weig
     // sized for entries of two items (the most entries) holding four items' data (the largest entries)
     const int big = max(m->hidden, m->inter);
     const size_t xb = mlx_mma_grouped_xb_bytes(big, kMoeMmaRowsMax);
-    const size_t tab = (size_t)mlx_mma_grouped_tab_floats(big, kMoeMmaRowsMax);
     const size_t ne = (size_t)m->max_entries;
     MmaGroupEntry* mw = nullptr;
     unsigned char* mxb = nullptr;
-    float *mxtab = nullptr, *gu = nullptr;
+    float* gu = nullptr;
     cudaError_t e = cudaMalloc(&mw, ne * sizeof(MmaGroupEntry));
     if (e == cudaSuccess) e = cudaMalloc(&mxb, ne * xb);
-    if (e == cudaSuccess) e = cudaMalloc(&mxtab, ne * tab * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc(&gu, ne * kMoeMmaRowsMax * 2 * m->inter * sizeof(float));
     if (e == cudaSuccess) e = cudaMemset(mxb, 0, ne * xb);  // rows past an entry's items are multiplied too (and ignored)
     if (e != cudaSuccess) {
       cudaFree(mw);
       cudaFree(mxb);
-      cudaFree(mxtab);
       cudaFree(gu);
       return fail_cuda(e, "cudaMalloc(MoE grouped-launch scratch)");
     }
     m->mwork = mw;
     m->mxb = mxb;
-    m->mxtab = mxtab;
     m->gu = gu;
   }
   m->tiled = tiled;
@@ -1119,7 +1114,6 @@ GOPH_API int goph_moe_free(goph_moe_layer* m) {
   cudaFree(m->bar);
   cudaFree(m->mwork);
   cudaFree(m->mxb);
-  cudaFree(m->mxtab);
   cudaFree(m->gu);
   m->magic = 0;
   delete m;
@@ -1291,7 +1285,6 @@ static int moe_run(goph_moe_layer* m, float* out_dev, const float* x_dev, const 
     g.max_entries = min(m->max_entries, min(tokens * m->top_k, m->num_experts * ((tokens + entry_rows - 1) / entry_rows)));
     g.top_k = m->top_k;
     g.xb = m->mxb;
-    g.xtab = m->mxtab;
     g.first = 0;
     g.mats = 2;
     g.rows = m->inter;
