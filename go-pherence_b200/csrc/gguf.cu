@@ -359,14 +359,14 @@ static int q_format(int qtype) {
 }
 
 // The several-row tensor-core product (qgemm.cu) reads both layouts.
-// rows: its scratch in the streaming layout.
+// rows: the scratch of a matrix whose products need no order.
 static bool qgemm_takes(const goph_gguf_matrix* m, const void* x, int batch, cudaStream_t stream, QBufs** rows) {
   return m->in_dim <= 65536 && (m->tiled || m->qmaps.ok) && (uintptr_t)x % 16 == 0 && qgemm_wants(q_format(m->qtype), m->tiled != nullptr, false, m->out_dim, m->in_dim, batch) &&
-         (m->tiled || (*rows = qgemm_scratch(m->device, stream)));
+         ((m->tiled && !m->unordered) || (*rows = qgemm_scratch(m->device, stream)));
 }
 
 static QWeight q_weight(const goph_gguf_matrix* m) {
-  return QWeight{q_format(m->qtype), m->tiled != nullptr, m->tiled ? m->tiled : m->data, m->d16, nullptr, nullptr, m->device, m->out_dim, m->in_dim, &m->qmaps};
+  return QWeight{q_format(m->qtype), m->tiled != nullptr, m->tiled ? m->tiled : m->data, m->d16, nullptr, nullptr, m->device, m->out_dim, m->in_dim, &m->qmaps, m->unordered};
 }
 
 static long gguf_row_bytes(int qtype, int in_dim) {
@@ -455,11 +455,14 @@ GOPH_API int goph_gguf_upload(int device, int qtype, const uint8_t* raw, uint64_
   UP(cudaGetLastError());
   UP(cudaDeviceSynchronize());
 #undef UP
-  // Large matrices go to the tensor-core layout (the CUDA-core kernels are instruction-bound on
-  // this part); small ones stay in the streaming layout, whose launch is leaner.
-  const bool big = (uint64_t)in_dim * (uint64_t)out_dim >= (8ull << 20);
-  if (gguf_mma_supported(qtype, in_dim) && (options().gguf_layout == 2 || (options().gguf_layout == 0 && big))) {
+  // The tensor-core layout for all but the smallest (rows are padded to tiles of 128; B200, us a call, streaming layout / this one:
+  // 1024x1024 one row 3.0 / 2.9 for every type, eight 5.3 to 5.7 / 5.2 to 6.3, 2048x2048 Q4_K 3.7 / 3.4 and 8.7 / 6.4).
+  const uint64_t size = (uint64_t)in_dim * (uint64_t)out_dim;
+  const bool big = size >= (8ull << 20) && in_dim % 256 == 0, tile = big || (size >= (qtype == GOPH_GGUF_Q6_K ? 1536ull << 10 : 512ull << 10) && out_dim >= 256);
+  if (gguf_mma_supported(qtype, in_dim) && (options().gguf_layout == 2 || (options().gguf_layout == 0 && tile))) {
     if (int rc = gguf_mma_make_tiled(h)) return bail(rc);
+    h->unordered = options().gguf_layout == 0 && !big;
+    if (!mlx_mma_ready(device)) return bail(fail(GOPH_E_NOMEM, "cannot allocate the tensor-core path's device scratch"));
     cudaFree(h->data);
     cudaFree(h->d16);
     h->data = nullptr;

@@ -405,7 +405,7 @@ bool launch_stream_work(const goph_gguf_matrix* m, const float* x, const WorkArg
   a.in_dim = m->in_dim;
   a.units = q4 ? m->in_dim / 32 : m->in_dim / 16;
   a.iters = (a.units + 31) / 32;
-  a.row_bytes = tiled ? m->in_dim / 256 : (q4 ? m->in_dim / 256 * 144 : m->in_dim);
+  a.row_bytes = tiled ? (m->in_dim + 255) / 256 : (q4 ? m->in_dim / 256 * 144 : m->in_dim);
   a.x_aligned = 1;
   const size_t smem = q4 ? stream_smem_bytes<Q4KFmt>(kWorkM, a.iters) : stream_smem_bytes<Q80Fmt>(kWorkM, a.iters);
   if (smem > (size_t)kSmemBudget) return false;
@@ -460,7 +460,7 @@ WorkView view_of(const goph_gguf_matrix* m) {
   v.qtype = m->qtype;
   v.in_dim = m->in_dim;
   v.out_dim = m->out_dim;
-  v.nchunks = m->in_dim / 256;
+  v.nchunks = (m->in_dim + 255) / 256;
   return v;
 }
 

@@ -55,7 +55,7 @@ struct Options {
   int mlx_layout = 0;  // layout chosen at upload: 0 by size, 1 always row-major, 2 tiled whenever the shape allows
   int mlx_splits = 0;  // K splits on the tensor-core path (0 = by shape)
   int mlx_fuse = 1;    // 1: narrow tensor-core launches make the activation digits of their own K range themselves (one launch)
-  int mlx_chunks = 0;  // 1: one 256-element chunk per pipeline stage of the tensor-core GEMV; 0: two where the format allows
+  int mlx_chunks = 0;  // without effect
   int moe_fused = 1;   // MoE call of one token with row-major experts: 1 one cooperative launch, 0 the five launches of any token count
   int moe_rows = 0;    // tiled MoE experts: items per work entry (2 or 4); 0 = by the number of tokens
   int mlx_cluster = 1; // 1: K splits that run in one wave exchange their partial sums inside a thread-block cluster; 0: always through global scratch
@@ -134,6 +134,7 @@ struct goph_gguf_matrix {
   uint8_t* data;   // Q4_K, Q5_K: blocks; Q8_0: biased int8 plane; Q6_K: low-nibble plane
   uint16_t* d16;   // Q8_0: f16 scales; Q6_K: two-bit highs, int8 scales and f16 d, one plane after another
   uint8_t* tiled;  // tensor-core layout (data and d16 are then null): one stage per 128 rows x 256 elements
+  bool unordered;  // tiled by size alone and small, or with rows that end inside a stage: products need no order between streams
   uint64_t bytes;
   goph::QMaps qmaps;  // streaming layout
 };

@@ -40,6 +40,7 @@
 #include <string.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "goph_internal.cuh"
 #include "mlx_mma.cuh"
@@ -110,84 +111,101 @@ __device__ __forceinline__ float max_nan(float a, float b) {  // (fmaxf passes o
 // The digits come from one sum: q + 64 (1 + 128 + 128^2) has d_j + 64 in its j-th seven bits (the top digit has what is
 // left), and a byte pattern d + 64 of seven bits becomes the signed byte.
 // A group with a NaN or an infinity has the scale NaN, which is what every product with it becomes (an integer has neither).
-template <int FMT, int MB, int SPLIT = 1>
-__device__ __forceinline__ void prep_chunk(const float (&v)[8], int lane, unsigned char* xb, int m, int digits) {
+// R: chunks at once, each with its own values, place and row (their chains of shuffles interleave).
+template <int FMT, int MB, int SPLIT = 1, int R = 1>
+__device__ __forceinline__ void prep_chunks(const float (&v)[R][8], int lane, unsigned char* const (&xb)[R], const int (&m)[R], int digits) {
   typedef Fmt<FMT> F;
   typedef XBlock<FMT, MB> X;
   constexpr int kLanes = F::kGroup / 8;  // of a group
   const int qbits = digits == 4 ? 26 : 19;  // |q| <= 2^qbits keeps the top digit within a signed byte
-  float s = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
-  float mx = max_nan(max_nan(max_nan(fabsf(v[0]), fabsf(v[1])), max_nan(fabsf(v[2]), fabsf(v[3]))),
-                     max_nan(max_nan(fabsf(v[4]), fabsf(v[5])), max_nan(fabsf(v[6]), fabsf(v[7]))));
+  float s[R], mx[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    s[r] = ((v[r][0] + v[r][1]) + (v[r][2] + v[r][3])) + ((v[r][4] + v[r][5]) + (v[r][6] + v[r][7]));
+    mx[r] = max_nan(max_nan(max_nan(fabsf(v[r][0]), fabsf(v[r][1])), max_nan(fabsf(v[r][2]), fabsf(v[r][3]))),
+                    max_nan(max_nan(fabsf(v[r][4]), fabsf(v[r][5])), max_nan(fabsf(v[r][6]), fabsf(v[r][7]))));
+  }
 #pragma unroll
   for (int o = SPLIT; o < kLanes * SPLIT; o <<= 1) {
-    if (F::kSums) s += __shfl_xor_sync(0xffffffffu, s, o);
-    mx = max_nan(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (F::kSums) s[r] += __shfl_xor_sync(0xffffffffu, s[r], o);
+      mx[r] = max_nan(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], o));
+    }
   }
-  int e = (int)((__float_as_uint(mx) >> 23) & 0xFF);  // mx < 2^(e-126)
-  const bool finite = e < 255;
-  if (e < qbits + 2) e = qbits + 2;
-  if (e > 254) e = 254;
   const int sub = lane % SPLIT;
   lane /= SPLIT;
-  if (sub == 0 && lane % kLanes == 0) {
-    float* tab = reinterpret_cast<float*>(xb + X::kFrag);
-    const int g = lane / kLanes;
-    const uint32_t f = (uint32_t)(e - 126 - qbits + 127) << 23;  // 2^(E-qbits)
-    const float sc[2] = {__uint_as_float(finite ? f : 0x7FC00000u), __uint_as_float(finite ? f + (14u << 23) : 0x7FC00000u)};
 #pragma unroll
-    for (int p = 0; p < 2; ++p) {
-      if (MB > 1) {
-        float* t = tab + X::entry(m, p, g);
-        t[0] = sc[p];
-        if (F::kSums) t[1] = p ? s : 0.f;
-      } else if (FMT == FMT_Q6K) {
-        *reinterpret_cast<float2*>(tab + X::entry1(p, 0, g)) = make_float2(sc[p], 0.f);
-        *reinterpret_cast<float2*>(tab + X::entry1(p, 1, g)) = make_float2(0.f, sc[p]);
+  for (int r = 0; r < R; ++r) {
+    int e = (int)((__float_as_uint(mx[r]) >> 23) & 0xFF);  // mx < 2^(e-126)
+    const bool finite = e < 255;
+    if (e < qbits + 2) e = qbits + 2;
+    if (e > 254) e = 254;
+    if (sub == 0 && lane % kLanes == 0) {
+      float* tab = reinterpret_cast<float*>(xb[r] + X::kFrag);
+      const int g = lane / kLanes;
+      const uint32_t f = (uint32_t)(e - 126 - qbits + 127) << 23;  // 2^(E-qbits)
+      const float sc[2] = {__uint_as_float(finite ? f : 0x7FC00000u), __uint_as_float(finite ? f + (14u << 23) : 0x7FC00000u)};
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        if (MB > 1) {
+          float* t = tab + X::entry(m[r], p, g);
+          t[0] = sc[p];
+          if (F::kSums) t[1] = p ? s[r] : 0.f;
+        } else if (FMT == FMT_Q6K) {
+          *reinterpret_cast<float2*>(tab + X::entry1(p, 0, g)) = make_float2(sc[p], 0.f);
+          *reinterpret_cast<float2*>(tab + X::entry1(p, 1, g)) = make_float2(0.f, sc[p]);
+        } else {
+          const int half = g & 1;
+          float* t = tab + X::entry1(p, half, g >> 1);
+          t[half] = sc[p];
+          if (F::kSums) t[2] = p ? s[r] : 0.f;
+          (tab + X::entry1(p, half ^ 1, g >> 1))[half] = 0.f;
+        }
+      }
+    }
+    const float fi = __uint_as_float((uint32_t)(qbits - (e - 126) + 127) << 23);
+    const uint32_t bias = digits == 4 ? 64u * (1 + 128 + 16384) : 64u * (1 + 128);
+    int q[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) q[i] = (int)((uint32_t)__float2int_rn(v[r][i] * fi) + bias);
+    auto digit = [&](int d) {
+      uint32_t p[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        auto at = [&](int i) { return (uint32_t)(q[F::kNibble ? 2 * i + h : 4 * h + i] >> (7 * d)); };
+        p[h] = __byte_perm(__byte_perm(at(0), at(1), 0x0040), __byte_perm(at(2), at(3), 0x0040), 0x5410);
+        if (d < digits - 1) {
+          p[h] = (p[h] & 0x7F7F7F7Fu) ^ 0x40404040u;
+          p[h] |= (p[h] & 0x40404040u) << 1;
+        }
+        if (d >= digits) p[h] = 0;
+      }
+      return make_uint2(p[0], p[1]);
+    };
+    const int step = lane >> 2, w = lane & 3;  // the lane's eight positions are 8 w .. 8 w + 7 of the K step
+    auto put = [&](int d, uint2 t) {
+      const int n = m[r] * 4 + d;
+      if (F::kNibble) {  // the nibbles' order: even elements of a packed word, then odd ones
+        *reinterpret_cast<uint2*>(xb[r] + X::frag(step, n, w)) = t;
       } else {
-        const int half = g & 1;
-        float* t = tab + X::entry1(p, half, g >> 1);
-        t[half] = sc[p];
-        if (F::kSums) t[2] = p ? s : 0.f;
-        (tab + X::entry1(p, half ^ 1, g >> 1))[half] = 0.f;
+        *reinterpret_cast<uint32_t*>(xb[r] + X::frag(step, n, 2 * (w & 1)) + 4 * (w >> 1)) = t.x;
+        *reinterpret_cast<uint32_t*>(xb[r] + X::frag(step, n, 2 * (w & 1) + 1) + 4 * (w >> 1)) = t.y;
       }
-    }
-  }
-  const float fi = __uint_as_float((uint32_t)(qbits - (e - 126) + 127) << 23);
-  const uint32_t bias = digits == 4 ? 64u * (1 + 128 + 16384) : 64u * (1 + 128);
-  int q[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) q[i] = (int)((uint32_t)__float2int_rn(v[i] * fi) + bias);
-  auto digit = [&](int d) {
-    uint32_t p[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      auto at = [&](int i) { return (uint32_t)(q[F::kNibble ? 2 * i + h : 4 * h + i] >> (7 * d)); };
-      p[h] = __byte_perm(__byte_perm(at(0), at(1), 0x0040), __byte_perm(at(2), at(3), 0x0040), 0x5410);
-      if (d < digits - 1) {
-        p[h] = (p[h] & 0x7F7F7F7Fu) ^ 0x40404040u;
-        p[h] |= (p[h] & 0x40404040u) << 1;
-      }
-      if (d >= digits) p[h] = 0;
-    }
-    return make_uint2(p[0], p[1]);
-  };
-  const int step = lane >> 2, w = lane & 3;  // the lane's eight positions are 8 w .. 8 w + 7 of the K step
-  auto put = [&](int d, uint2 t) {
-    const int n = m * 4 + d;
-    if (F::kNibble) {  // the nibbles' order: even elements of a packed word, then odd ones
-      *reinterpret_cast<uint2*>(xb + X::frag(step, n, w)) = t;
+    };
+    if (SPLIT == 4) {
+      put(sub, digit(sub));
     } else {
-      *reinterpret_cast<uint32_t*>(xb + X::frag(step, n, 2 * (w & 1)) + 4 * (w >> 1)) = t.x;
-      *reinterpret_cast<uint32_t*>(xb + X::frag(step, n, 2 * (w & 1) + 1) + 4 * (w >> 1)) = t.y;
-    }
-  };
-  if (SPLIT == 4) {
-    put(sub, digit(sub));
-    return;
-  }
 #pragma unroll
-  for (int d = 0; d < 4; ++d) put(d, digit(d));
+      for (int d = 0; d < 4; ++d) put(d, digit(d));
+    }
+  }
+}
+template <int FMT, int MB, int SPLIT = 1>
+__device__ __forceinline__ void prep_chunk(const float (&v)[8], int lane, unsigned char* xb, int m, int digits) {
+  unsigned char* const xbs[1] = {xb};
+  const int ms[1] = {m};
+  prep_chunks<FMT, MB, SPLIT, 1>(reinterpret_cast<const float(&)[1][8]>(v), lane, xbs, ms, digits);
 }
 __device__ __forceinline__ void load_eight(const float* p, float (&v)[8]) {
   if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
@@ -204,11 +222,12 @@ __device__ __forceinline__ void load_eight(const float* p, float (&v)[8]) {
 template <int FMT, int MB>
 __global__ void __launch_bounds__(128)
 mlx_prep_x_kernel(const float* __restrict__ x, unsigned char* __restrict__ xb, int in_dim, int digits) {
-  const int nchunks = in_dim / kChunkK, m = blockIdx.x / nchunks, c = blockIdx.x - m * nchunks, lane = threadIdx.x;
+  const int nchunks = (in_dim + kChunkK - 1) / kChunkK, m = blockIdx.x / nchunks, c = blockIdx.x - m * nchunks, lane = threadIdx.x;
   pdl_launch_dependents();
   pdl_wait();  // x may be the output of the kernel in front
-  float v[8];
-  load_eight(x + (size_t)m * in_dim + c * kChunkK + lane / 4 * 8, v);
+  float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // (past the row)
+  const int k = c * kChunkK + lane / 4 * 8;
+  if (k < in_dim) load_eight(x + (size_t)m * in_dim + k, v);
   prep_chunk<FMT, MB, 4>(v, lane, xb + (size_t)c * XBlock<FMT, MB>::kBytes, m, digits);
 }
 
@@ -309,19 +328,28 @@ struct RowScales {
   }
 };
 
+// One weight of a launch.
+struct RowSeg {
+  const unsigned char* w;  // tiled: weight blocks [tile][chunk]
+  const uint32_t* sb;      // row-major MLX: the {scale, bias} table
+  float* out;              // [batch][out_dim]
+  int out_dim, tile0;      // first of its tiles among the launch's
+};
+constexpr int kMaxRowSeg = 4;
+
 struct MmaArgs {
-  const unsigned char* w;  // tiled weight blocks [tile][chunk]
+  RowSeg seg[kMaxRowSeg];
+  int nseg;
   const float* x;          // [batch][in_dim]
   const unsigned char* xb; // prepared activations: an XBlock per chunk
-  float* out;              // [batch][out_dim]
   int* status;             // device word: 0 ok, otherwise the first wait that gave up
   float* scratch;          // split-K partial sums [item][warp][value][lane]
   unsigned int* counters;  // arrival counters per tile and warp, zero between launches
-  int out_dim, in_dim;
+  int in_dim;
   int batch;               // activation rows of this launch (<= MB of the instantiation)
   int digits;
-  int ntiles;              // ceil(out_dim / 128)
-  int nchunks;             // in_dim / 256
+  int ntiles;              // tiles of 128 rows, of all weights
+  int nchunks;             // ceil(in_dim / 256)
   int splits;              // CTAs sharing the K range of one tile
   int items;               // ntiles * splits
   int stages;              // depth of the shared-memory ring
@@ -332,6 +360,22 @@ struct MmaArgs {
   int gmax, gtpe, gmats, gfirst, gdirect;
   size_t gxb;
 };
+
+// Row-major MLX weights: their tiles come as boxes of 128 rows, 128 bytes of nibbles (whose 128-byte swizzle is the tiled image's) and
+// 16 bytes of the table; zeros past the edges.  A table whose rows are no whole 16-byte units comes by cp.async.
+struct RowMaps {
+  CUtensorMap map[kMaxRowSeg][2];
+  int meta_tma;
+};
+struct NoMaps {};
+template <bool TILED>
+using MapArgs = std::conditional_t<TILED, NoMaps, RowMaps>;
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, int bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
 
 template <bool G, bool WORK = false>
 struct StageWalkT {
@@ -374,7 +418,7 @@ struct StageWalkT {
 };
 
 constexpr int kConsumers = 8;  // warps; the ninth loads
-constexpr int kMaxStages = 12, kMaxSplits = 8;
+constexpr int kMaxStages = 12, kMaxSplits = 16;
 constexpr int kThreads = (kConsumers + 1) * 32;
 
 template <int FMT, int MB, bool G>
@@ -393,11 +437,12 @@ struct RowCfg {
   static constexpr int kRecv = kStoring * kVals * 128;       // a split's sums
   static constexpr int kScales = kStaged<FMT, MB> ? kConsumers * SL * 16 * kStagedRow : 0;
 };
-template <int FMT, int MB, bool FUSED, bool G>
+template <int FMT, int MB, bool FUSED, bool G, bool TILED = true>
 struct RowSmem {
   static constexpr int kStage = Fmt<FMT>::kStageBytes + (FUSED ? 0 : XBlock<FMT, MB>::kBytes);
   static __host__ __device__ size_t bytes(int stages, int cmax, int recv) {
-    return (size_t)stages * kStage + (FUSED ? (size_t)cmax * XBlock<FMT, MB>::kBytes : 0) + RowCfg<FMT, MB, G>::kPair + RowCfg<FMT, MB, G>::kScales + (size_t)recv * RowCfg<FMT, MB, G>::kRecv + 512;
+    return (size_t)stages * kStage + (FUSED ? (size_t)cmax * XBlock<FMT, MB>::kBytes : 0) + RowCfg<FMT, MB, G>::kPair + RowCfg<FMT, MB, G>::kScales + (size_t)recv * RowCfg<FMT, MB, G>::kRecv + 512 +
+           (TILED ? 0 : 1024);  // (boxes with a swizzle start on multiples of 1024 bytes)
   }
   // Depth of the ring that `budget` leaves room for.
   static int stages(size_t budget, int cmax, int recv) {
@@ -408,22 +453,23 @@ struct RowSmem {
   }
 };
 
-template <int FMT, int MB, bool FUSED, bool G = false>
+template <int FMT, int MB, bool FUSED, bool G = false, bool TILED = true>
 __global__ void __launch_bounds__(kThreads, 2)
-mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
+mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArgs<TILED> maps) {
   static_assert(!G || !FUSED, "grouped launches: activations prepared in front");
+  static_assert(TILED || (FMT == FMT_MLX4 && FUSED), "row-major: MLX, activations by the CTAs themselves");
   constexpr bool kWork = G && FMT != FMT_MLX4;  // a work list's entries (MmaWorkEntry)
   typedef StageWalkT<G, kWork> StageWalk;
   typedef Fmt<FMT> F;
   typedef XBlock<FMT, MB> X;
   typedef RowCfg<FMT, MB, G> C;
-  typedef RowSmem<FMT, MB, FUSED, G> M;
+  typedef RowSmem<FMT, MB, FUSED, G, TILED> M;
   constexpr int SL = C::SL, KG = C::KG, NT = C::NT, kStage = M::kStage;
   // A chunk is summed by itself where its terms, products and biases or minima that cancel, meet a small sum.
   constexpr bool kByChunk = F::kSums && !(FMT == FMT_MLX4 && MB == 8);
   extern __shared__ __align__(128) unsigned char smem_dyn[];
   const int S = a.stages;
-  unsigned char* ring = smem_dyn;
+  unsigned char* ring = TILED ? smem_dyn : reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
   unsigned char* bres = ring + (size_t)S * kStage;
   unsigned char* scales = bres + (FUSED ? (size_t)a.cmax * X::kBytes : 0);
   float* pair = reinterpret_cast<float*>(scales + C::kScales);
@@ -435,7 +481,9 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
 
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
-      mbar_init(full0 + 8 * s, 1);
+      int arrivals = 1;
+      if constexpr (!TILED) arrivals += maps.meta_tma ? 0 : 32;
+      mbar_init(full0 + 8 * s, arrivals);
       mbar_init(empty0 + 8 * s, kConsumers / KG);
     }
     for (int s = 0; s < 9; ++s) gave_up[s] = 0;
@@ -457,16 +505,58 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
     return kWork ? &reinterpret_cast<const MmaWorkEntry*>(a.gwork)[e].g : a.gwork + e;
   };
   const int cbase = sw.live(a) ? sw.c : 0;  // first chunk of this CTA's K range
+  auto seg_of = [&](int tile) {
+    int k = 0;
+#pragma unroll
+    for (int j = 1; j < kMaxRowSeg; ++j)
+      if (j < a.nseg && tile >= a.seg[j].tile0) k = j;
+    return k;
+  };
   float fin[C::kVals];                      // the item's values (cluster: kept for the exchange)
   bool have = false;
 
   if (warp == kConsumers) {
     // ------------------------------------------------------------------ producer
-    if (lane == 0) {
+    if constexpr (!TILED) {
+      RingCursor rc;
+      int i = 0;
+      for (; sw.live(a) && ok; sw.next_item(a)) {
+        const int k = seg_of(sw.tile), row0 = (sw.tile - a.seg[k].tile0) * kTileRows;
+        for (int c = sw.c; c < sw.c1; ++c, ++i, rc.next(S)) {
+          if (i >= S) ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8 * rc.s, rc.ph ^ 1u, a.status, 1));
+          if (!ok) break;
+          const uint32_t dst = smem_u32(ring + (size_t)rc.s * kStage), meta = dst + F::kStageWBytes, bar = full0 + 8 * rc.s;
+          if (lane == 0) {
+            mbar_expect_tx(bar, F::kStageWBytes + (maps.meta_tma ? kTileRows * 16 : 0));
+            tma_load_2d(dst, &maps.map[k][0], c * 128, row0, bar);
+            if (maps.meta_tma) tma_load_2d(meta, &maps.map[k][1], c * 16, row0, bar);
+          }
+          __syncwarp();
+          if (!maps.meta_tma) {
+            const int groups = a.in_dim / 64;
+            const uint32_t* sb = a.seg[k].sb;
+            for (int j = lane; j < 4 * kTileRows; j += 32) {
+              const int r = j >> 2, g = j & 3;
+              const bool in = row0 + r < a.seg[k].out_dim && c * 4 + g < groups;
+              cp_async4(meta + r * 16 + g * 4, in ? sb + (size_t)(row0 + r) * groups + c * 4 + g : sb, in ? 4 : 0);
+            }
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+          }
+        }
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      if (!ok && lane == 0) *gave_up = 1;
+    } else if (lane == 0) {
       auto wsrc = [&](const StageWalk& s, int c) {
-        const unsigned char* base = a.w;
+        const unsigned char* base;
+        int tile = s.tile;
+        if (!G) {
+          const int k = seg_of(tile);
+          base = a.seg[k].w;
+          tile -= a.seg[k].tile0;
+        }
         if (G) base = reinterpret_cast<const unsigned char*>(__ldg(reinterpret_cast<const unsigned long long*>(&entry_at(s.entry)->w[a.gfirst + s.mat])));
-        return base + ((size_t)s.tile * a.nchunks + c) * F::kStageBytes;
+        return base + ((size_t)tile * a.nchunks + c) * F::kStageBytes;
       };
       auto bsrc = [&](const StageWalk& s, int c) { return a.xb + (G ? (size_t)s.entry * a.gxb : 0) + (size_t)c * X::kBytes; };
       // The weights do not depend on the kernel in front: the ring is filled with them first, the activations of those
@@ -512,23 +602,38 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
       // every item of this CTA covers the same K range (the grid is a multiple of the K splits)
       if (sw.live(a)) {
         const int n = sw.c1 - sw.c;
-        auto at = [&](int i, int& m, int& c) {
-          m = MB == 1 ? 0 : i / n;
-          c = i - m * n;
-          return a.x + (size_t)m * a.in_dim + (sw.c + c) * kChunkK + lane * 8;
-        };
-        int m, c;
-        float v[8];
-        if (warp < a.batch * n) load_eight(at(warp, m, c), v);
-#pragma unroll 1
-        for (int i = warp; i < a.batch * n;) {
-          float u[8];
-          const int m0 = m, c0 = c;
-          i += kConsumers;
-          if (i < a.batch * n) load_eight(at(i, m, c), u);  // (the next chunk is under way while this one is worked on)
-          prep_chunk<FMT, MB>(v, lane, bres + (size_t)c0 * X::kBytes, m0, a.digits);
+        // (two of a warp's chunks at once, and the next two are under way)
+        auto load = [&](int i, float (&v)[8]) {
+          if (i >= a.batch * n) return;
+          const int m = MB == 1 ? 0 : i / n, k = (sw.c + i - m * n) * kChunkK + lane * 8;
+          if (k < a.in_dim) {
+            load_eight(a.x + (size_t)m * a.in_dim + k, v);
+          } else {  // (past the row, which ends with a lane's eight)
 #pragma unroll
-          for (int e = 0; e < 8; ++e) v[e] = u[e];
+            for (int e = 0; e < 8; ++e) v[e] = 0.f;
+          }
+        };
+        float v[2][8] = {};
+        load(warp, v[0]);
+        load(warp + kConsumers, v[1]);
+#pragma unroll 1
+        for (int i = warp; i < a.batch * n; i += 2 * kConsumers) {
+          float u[2][8] = {};
+          load(i + 2 * kConsumers, u[0]);
+          load(i + 3 * kConsumers, u[1]);
+          const int i1 = i + kConsumers, m0 = MB == 1 ? 0 : i / n, m1 = MB == 1 ? 0 : i1 / n;
+          if (i1 < a.batch * n) {
+            unsigned char* const at[2] = {bres + (size_t)(i - m0 * n) * X::kBytes, bres + (size_t)(i1 - m1 * n) * X::kBytes};
+            const int ms[2] = {m0, m1};
+            prep_chunks<FMT, MB, 1, 2>(v, lane, at, ms, a.digits);
+          } else {
+            prep_chunk<FMT, MB>(v[0], lane, bres + (size_t)(i - m0 * n) * X::kBytes, m0, a.digits);
+          }
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            v[0][e] = u[0][e];
+            v[1][e] = u[1][e];
+          }
         }
       }
       asm volatile("bar.sync 1, %0;" ::"n"(kConsumers * 32) : "memory");
@@ -833,7 +938,10 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
 #pragma unroll
         for (int k = 0; k < C::kVals; ++k) fin[k] += buf[k * 32];
       }
-      const int row = sw.tile * kTileRows + row0 + g + 8 * p;  // of the first slab
+      const int sg = G ? 0 : seg_of(sw.tile);
+      const int row = (sw.tile - (G ? 0 : a.seg[sg].tile0)) * kTileRows + row0 + g + 8 * p;  // of the first slab
+      float* const out = a.seg[sg].out;
+      const int out_dim = a.seg[sg].out_dim;
       auto act = [&](int k) { return MB == 1 ? 0 : 2 * (k % NT) + half; };
       const bool mine = MB > 1 || t < 2;
       if (G) {
@@ -853,14 +961,14 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
           if constexpr (kWork) {
             const MmaWorkEntry* we = reinterpret_cast<const MmaWorkEntry*>(a.gwork) + cur_entry;
             if (a.gdirect == 2) {
-              a.out[(size_t)__ldg(&we->g.item[m]) * a.out_dim + r] = gelu_tanh(gate[k]) * fin[k];
+              out[(size_t)__ldg(&we->g.item[m]) * out_dim + r] = gelu_tanh(gate[k]) * fin[k];
             } else {
               float* dst = reinterpret_cast<float*>(__ldg(reinterpret_cast<const unsigned long long*>(&we->dst[m])));
               if (r < __ldg(&we->room[m])) atomicAdd(dst + r, fin[k] * __ldg(&we->weight[m]));  // items may share a destination row
             }
           } else {
             const int orow = a.gdirect ? __ldg(&entry_at(cur_entry)->item[m]) : cur_entry * MB + m;
-            a.out[(size_t)orow * a.out_dim + sw.mat * (a.gtpe * kTileRows) + r] = fin[k];
+            out[(size_t)orow * out_dim + sw.mat * (a.gtpe * kTileRows) + r] = fin[k];
           }
         }
       } else if (a.cluster) {
@@ -870,7 +978,7 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
 #pragma unroll
         for (int k = 0; k < C::kVals; ++k) {
           const int m = act(k), r = row + 16 * (k / NT);
-          if (mine && m < a.batch && r < a.out_dim) a.out[(size_t)m * a.out_dim + r] = fin[k];
+          if (mine && m < a.batch && r < out_dim) out[(size_t)m * out_dim + r] = fin[k];
         }
       } else {
         // Partial sums of this K range go to scratch; the warp that arrives last at its rows of the tile adds the
@@ -892,7 +1000,7 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
             float sum = 0.f;
             for (int s2 = 0; s2 < a.splits; ++s2) sum += __ldcg(base + (size_t)s2 * (C::kStoring * kPart) + k * 32);
             const int m = act(k), r = row + 16 * (k / NT);
-            if (mine && m < a.batch && r < a.out_dim) a.out[(size_t)m * a.out_dim + r] = sum;
+            if (mine && m < a.batch && r < out_dim) out[(size_t)m * out_dim + r] = sum;
           }
           if (lane == 0) a.counters[sw.tile * kConsumers + slot] = 0;
         }
@@ -914,13 +1022,15 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a) {
       if (sw.split == 0) {
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         if (have) {
-          const int row = sw.tile * kTileRows + row0 + g + 8 * p;
+          const int sg = seg_of(sw.tile), row = (sw.tile - a.seg[sg].tile0) * kTileRows + row0 + g + 8 * p;
+          float* const out = a.seg[sg].out;
+          const int out_dim = a.seg[sg].out_dim;
 #pragma unroll
           for (int k = 0; k < C::kVals; ++k) {
             float sum = fin[k];
             for (int s2 = 1; s2 < a.splits; ++s2) sum += recv[(size_t)(s2 - 1) * (C::kRecv / 4) + slot * (C::kVals * 32) + k * 32 + lane];
             const int m = MB == 1 ? 0 : 2 * (k % NT) + half, r = row + 16 * (k / NT);
-            if ((MB > 1 || t < 2) && m < a.batch && r < a.out_dim) a.out[(size_t)m * a.out_dim + r] = sum;
+            if ((MB > 1 || t < 2) && m < a.batch && r < out_dim) out[(size_t)m * out_dim + r] = sum;
           }
         }
       }
@@ -1048,9 +1158,12 @@ int mlx_mma_status(int device) {
 }
 
 // A matrix in one of the tiled layouts, as the launch code sees it.
-struct TiledDesc {
-  const unsigned char* tiled;
-  int device, out_dim, in_dim;
+// Weights of one launch that share x, as the launch code sees them.
+struct RowWeights {
+  int device, in_dim, n;
+  RowSeg seg[kMaxRowSeg];              // tile0 filled in
+  const QMaps* maps[kMaxRowSeg] = {};  // row-major MLX
+  bool unordered = false;              // callers need no order between such products: no scratch of the device's
   size_t scratch_bytes = kScratchFloats * sizeof(float), counters = kMaxCounters;
 };
 
@@ -1068,6 +1181,7 @@ static int cluster_room(int device, int splits, bool whole) {
   if (!known[device]) {
     auto kern = mlx_mma_kernel<FMT_MLX4, 1, true>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWholeSmem);
+    cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     for (int w = 0; w < 2; ++w) {
       for (int n = 2; n <= kMaxSplits; ++n) {
         cudaLaunchAttribute attr;
@@ -1100,9 +1214,9 @@ struct RowPlan {
   bool cluster;
 };
 
-template <int FMT, int MB, bool FUSED>
-static int launch_impl(const TiledDesc& w, MmaArgs a, cudaStream_t stream, SharedX* xs, const RowPlan& plan) {
-  typedef RowSmem<FMT, MB, FUSED, false> M;
+template <int FMT, int MB, bool FUSED, bool TILED>
+static int launch_impl(const RowWeights& w, MmaArgs a, cudaStream_t stream, SharedX* xs, const RowPlan& plan) {
+  typedef RowSmem<FMT, MB, FUSED, false, TILED> M;
   const int splits = plan.splits;
   a.splits = splits;
   a.items = a.ntiles * splits;
@@ -1128,10 +1242,11 @@ static int launch_impl(const TiledDesc& w, MmaArgs a, cudaStream_t stream, Share
     GOPH_CUDA(cudaLaunchKernelEx(&cfg, mlx_prep_x_kernel<FMT, MB>, a.x, const_cast<unsigned char*>(a.xb), a.in_dim, a.digits));
     xs->prepared = true;
   }
-  auto kern = mlx_mma_kernel<FMT, MB, FUSED>;
+  auto kern = mlx_mma_kernel<FMT, MB, FUSED, false, TILED>;
   static bool sized[kMaxDevices] = {};
   if (!sized[w.device]) {
     GOPH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWholeSmem));
+    GOPH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     sized[w.device] = true;
   }
   const int slots = device_state(w.device).sm_count * (plan.whole ? 1 : 2);
@@ -1152,17 +1267,29 @@ static int launch_impl(const TiledDesc& w, MmaArgs a, cudaStream_t stream, Share
   // GOPH_TRACE_LAUNCH=1 in the environment: one line per tensor-core product with its launch plan
   static const bool trace = getenv("GOPH_TRACE_LAUNCH") != nullptr;
   if (trace)
-    fprintf(stderr, "goph: mlx_mma_kernel fmt=%d out=%d in=%d rows=%d grid=%d splits=%d stages=%d fused=%d cluster=%d smem=%d\n", FMT, a.out_dim, a.in_dim, a.batch,
-            grid, splits, a.stages, (int)FUSED, a.cluster, (int)smem);
+    fprintf(stderr, "goph: mlx_mma_kernel fmt=%d tiled=%d weights=%d out=%d in=%d rows=%d grid=%d splits=%d stages=%d fused=%d cluster=%d smem=%d\n", FMT, (int)TILED, a.nseg,
+            a.seg[0].out_dim, a.in_dim, a.batch, grid, splits, a.stages, (int)FUSED, a.cluster, (int)smem);
   note_launch();
-  GOPH_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
+  if constexpr (TILED) {
+    GOPH_CUDA(cudaLaunchKernelEx(&cfg, kern, a, NoMaps()));
+  } else {
+    RowMaps maps;
+    for (int i = 0; i < w.n; ++i) memcpy(maps.map[i], w.maps[i]->map, sizeof maps.map[i]);
+    maps.meta_tma = w.in_dim % kChunkK == 0;
+    GOPH_CUDA(cudaLaunchKernelEx(&cfg, kern, a, maps));
+  }
   return GOPH_OK;
 }
 
-template <int FMT, int MB>
-static int launch_one(const TiledDesc& w, const MmaArgs& a, cudaStream_t stream, SharedX* xs) {
+// 0: done; 1: the activations of so many rows do not fit (nothing launched); else an error.
+constexpr int kDoesNotFit = 1 << 20;
+template <int FMT, int MB, bool TILED>
+static int launch_one(const RowWeights& w, const MmaArgs& a, cudaStream_t stream, SharedX* xs) {
   constexpr bool kBytes = !Fmt<FMT>::kNibble;
+  typedef RowSmem<FMT, MB, true, false, TILED> Own;
+  typedef RowSmem<FMT, MB, false, false> Front;
   const int sms = device_state(w.device).sm_count, tiles = a.ntiles;
+  const bool alone = w.unordered || !TILED;  // no scratch: activations by the CTAs, sums inside clusters
   RowPlan p;
   // The lines (B200, us a call, weights from HBM).  A CTA to an SM, with a ring of all that is left: products that are over in a few stages (one row, MLX4
   // 4096x4096 4.4, two to an SM 4.6; 14336x4096 8.3 / 7.7), and several rows, whose activations leave half an SM too little (four rows 14336x4096 10.8 / 11.4;
@@ -1174,16 +1301,20 @@ static int launch_one(const TiledDesc& w, const MmaArgs& a, cudaStream_t stream,
   p.whole = small || MB == 8 || (MB == 4 && (FMT != FMT_MLX4 || tiles < sms)) || (MB == 2 && kBytes && tiles < sms);
   auto cut = [&](bool whole) {
     const int slots = sms * (whole ? 1 : 2);
+    const int most = 1 + 28 * 1024 / RowCfg<FMT, MB, false>::kRecv;  // (of the others' sums that the first CTA of a cluster has room for)
     int n = slots / tiles;
     if (n > a.nchunks) n = a.nchunks;
     if (n > kMaxSplits) n = kMaxSplits;
-    if (options().mlx_cluster)
+    if (n > most) n = most;
+    if (n > 8 && 16 * tiles > slots) n = 8;  // (larger clusters where eight CTAs a tile leave more than half of the places empty: 256x16384 5.7 / 4.5; 4096x14336 8.4 / 9.2)
+    const bool clusters = options().mlx_cluster || alone;
+    if (clusters)
       while (n > 1 && cluster_room(w.device, n, whole) < tiles) --n;
-    if (options().mlx_splits > 0) n = options().mlx_splits < a.nchunks ? options().mlx_splits : a.nchunks;
+    if (options().mlx_splits > 0 && !alone) n = options().mlx_splits < a.nchunks ? options().mlx_splits : a.nchunks;
     while (n > 1 && ((size_t)tiles * n * RowCfg<FMT, MB, false>::kRecv > w.scratch_bytes || (size_t)tiles * kConsumers > w.counters)) --n;
     p.whole = whole;
     p.splits = n < 1 ? 1 : n;
-    p.cluster = options().mlx_cluster && n > 1 && n <= kMaxSplits && (long)tiles * n <= slots && cluster_room(w.device, n, whole) >= tiles;
+    p.cluster = clusters && n > 1 && n <= most && n <= kMaxSplits && (long)tiles * n <= slots && cluster_room(w.device, n, whole) >= tiles;
   };
   cut(p.whole);
   const int cmax = (a.nchunks + p.splits - 1) / p.splits;
@@ -1193,51 +1324,71 @@ static int launch_one(const TiledDesc& w, const MmaArgs& a, cudaStream_t stream,
   if (a.batch * cmax <= 17) p.own = true;
   if (FMT == FMT_MLX4 && 2 * tiles > sms && tiles < sms && a.batch * a.nchunks > 17) p.own = false;
   if (!options().mlx_fuse || xs->written || p.splits > sms) p.own = false;
-  constexpr int kLeast = 3;
-  for (int t = 0; t < 4; ++t) {  // a ring of three stages at least: else a whole SM, else a launch in front
-    const int recv = p.cluster ? p.splits - 1 : 0, range = (a.nchunks + p.splits - 1) / p.splits;
+  if (alone) p.own = true;
+  // a ring of three stages at least (of two where groups of warps take turns): else a whole SM, else a launch in front
+  for (int t = 0; t < 5; ++t) {
+    const int recv = p.cluster ? p.splits - 1 : 0, range = (a.nchunks + p.splits - 1) / p.splits, least = RowCfg<FMT, MB, false>::KG == 2 && p.whole ? 2 : 3;
     const size_t budget = p.whole ? kWholeSmem : kHalfSmem;
-    if (p.own && RowSmem<FMT, MB, true, false>::stages(budget, range, recv) >= kLeast) return launch_impl<FMT, MB, true>(w, a, stream, xs, p);
-    if (!p.own && RowSmem<FMT, MB, false, false>::stages(budget, range, recv) >= kLeast) return launch_impl<FMT, MB, false>(w, a, stream, xs, p);
+    if (p.own && Own::stages(budget, range, recv) >= least) return launch_impl<FMT, MB, true, TILED>(w, a, stream, xs, p);
+    if constexpr (TILED)
+      if (!p.own && Front::stages(budget, range, recv) >= least) return launch_impl<FMT, MB, false, true>(w, a, stream, xs, p);
     if (!p.whole) cut(true);
+    else if (alone) break;
     else if (p.own) p.own = false;
     else if (p.cluster) p.cluster = false;  // (the sums meet in scratch and need no shared memory)
     else break;
   }
-  return fail(GOPH_E_UNSUPPORTED, "tensor-core path: activations of %d x %d leave no room for the ring", a.batch, a.in_dim);
+  return kDoesNotFit;
 }
 
-template <int FMT>
-static int tiled_launch(const TiledDesc& w, float* out, const float* x, int batch, int digits, cudaStream_t stream,
-                        SharedX* shared) {
-  MmaDeviceBufs* bufs = device_bufs(w.device);
+// The next rows of a call: as many as fit a launch.  Their number, or minus the error.
+template <int FMT, bool TILED>
+static int rows_slice(const RowWeights& w0, MmaArgs a, cudaStream_t stream, SharedX* xs, int* taken = nullptr) {
+  RowWeights w = w0;
+  a.in_dim = w.in_dim;
+  a.nchunks = (w.in_dim + kChunkK - 1) / kChunkK;
+  a.nseg = w.n;
+  a.ntiles = 0;
+  for (int i = 0; i < w.n; ++i) {
+    a.seg[i] = w.seg[i];
+    a.seg[i].tile0 = a.ntiles;
+    a.ntiles += (w.seg[i].out_dim + kTileRows - 1) / kTileRows;
+  }
+  for (int nb = a.batch < 8 ? a.batch : 8; nb > 0; nb = nb > 4 ? 4 : nb > 2 ? 2 : nb - 1) {
+    a.batch = nb;
+    const int rc = nb == 1 ? launch_one<FMT, 1, TILED>(w, a, stream, xs) : nb == 2 ? launch_one<FMT, 2, TILED>(w, a, stream, xs)
+                 : nb <= 4 ? launch_one<FMT, 4, TILED>(w, a, stream, xs) : launch_one<FMT, 8, TILED>(w, a, stream, xs);
+    if (rc == kDoesNotFit) continue;
+    if (taken) *taken = nb;
+    return rc;
+  }
+  return fail(GOPH_E_UNSUPPORTED, "tensor-core path: activations of %d elements leave no room for the ring", w.in_dim);
+}
+
+template <int FMT, bool TILED>
+static int rows_launch(const RowWeights& w0, const float* x, int batch, int digits, cudaStream_t stream, SharedX* shared) {
+  MmaDeviceBufs* bufs = device_bufs(w0.device);
   if (!bufs) return fail(GOPH_E_NOMEM, "cannot allocate the tensor-core path's device scratch");
+  RowWeights w = w0;
   MmaArgs a;
   memset(&a, 0, sizeof a);
-  a.w = w.tiled;
   a.status = bufs->status;
   a.scratch = bufs->scratch;
   a.counters = bufs->counters;
   a.xb = bufs->xb;
-  a.out_dim = w.out_dim;
-  a.in_dim = w.in_dim;
   a.digits = digits == 3 ? 3 : 4;
-  a.ntiles = (w.out_dim + kTileRows - 1) / kTileRows;
-  a.nchunks = w.in_dim / kChunkK;
-  constexpr int cap = 8;  // activation rows of a launch
-  const bool written = shared ? shared->written : floats_meet(out, (uint64_t)batch * w.out_dim, x, (uint64_t)batch * w.in_dim);
+  bool written = shared && shared->written;
+  if (!shared)
+    for (int i = 0; i < w.n; ++i) written = written || floats_meet(w.seg[i].out, (uint64_t)batch * w.seg[i].out_dim, x, (uint64_t)batch * w.in_dim);
   for (int b0 = 0; b0 < batch;) {
-    const int nb = batch - b0 < cap ? batch - b0 : cap;
     a.x = x + (size_t)b0 * w.in_dim;
-    a.out = out + (size_t)b0 * w.out_dim;
-    a.batch = nb;
+    for (int i = 0; i < w.n; ++i) w.seg[i].out = w0.seg[i].out + (size_t)b0 * w.seg[i].out_dim;
+    a.batch = batch - b0;
     SharedX own;  // (rows of a later launch of this call do not have the scratch's activations)
     own.written = written;
-    SharedX* xs = shared && batch <= cap ? shared : &own;
-    const int rc = nb == 1 ? launch_one<FMT, 1>(w, a, stream, xs) : nb == 2 ? launch_one<FMT, 2>(w, a, stream, xs) : nb <= 4 ? launch_one<FMT, 4>(w, a, stream, xs)
-                                                                                                                : launch_one<FMT, 8>(w, a, stream, xs);
-    if (rc) return rc;
-    b0 += nb;
+    int taken = 0;
+    if (int rc = rows_slice<FMT, TILED>(w, a, stream, shared && batch <= 8 ? shared : &own, &taken)) return rc;
+    b0 += taken;
   }
   return GOPH_OK;
 }
@@ -1245,8 +1396,30 @@ static int tiled_launch(const TiledDesc& w, float* out, const float* x, int batc
 int mlx_mma_launch(const goph_mlx_weight* w, float* out, const float* x, int batch, int digits, cudaStream_t stream,
                    SharedX* shared) {
   if (!w->tiled) return fail(GOPH_E_UNSUPPORTED, "weight is not in the tiled layout");
-  TiledDesc d{w->tiled, w->device, w->out_dim, w->in_dim};
-  return tiled_launch<FMT_MLX4>(d, out, x, batch, digits, stream, shared);
+  RowWeights d;
+  d.device = w->device;
+  d.in_dim = w->in_dim;
+  d.n = 1;
+  d.seg[0] = RowSeg{w->tiled, nullptr, out, w->out_dim, 0};
+  return rows_launch<FMT_MLX4, true>(d, x, batch, digits, stream, shared);
+}
+
+bool mlx_mma_ready(int device) { return device_bufs(device) != nullptr; }
+
+int mlx_mma_launch_rows(int n, const goph_mlx_weight* const* ws, float* const* outs, const float* x, int batch, int digits, cudaStream_t stream) {
+  for (int i0 = 0; i0 < n; i0 += kMaxRowSeg) {
+    RowWeights d;
+    d.device = ws[0]->device;
+    d.in_dim = ws[0]->in_dim;
+    d.n = n - i0 < kMaxRowSeg ? n - i0 : kMaxRowSeg;
+    for (int i = 0; i < d.n; ++i) {
+      const goph_mlx_weight* w = ws[i0 + i];
+      d.seg[i] = RowSeg{nullptr, static_cast<const uint32_t*>(w->sb), outs[i0 + i], w->out_dim, 0};
+      d.maps[i] = &w->qmaps;
+    }
+    if (int rc = rows_launch<FMT_MLX4, false>(d, x, batch, digits, stream, nullptr)) return rc;
+  }
+  return GOPH_OK;
 }
 
 // ---- grouped launches (mixture-of-experts) -----------------------------------------------------
@@ -1303,8 +1476,9 @@ static int launch_grouped(int device, const MmaGroupLaunch& g, cudaStream_t stre
   memset(&a, 0, sizeof a);
   a.status = bufs->status;
   a.xb = g.xb;
-  a.out = g.out;
-  a.out_dim = g.mats * g.rows;
+  a.nseg = 1;
+  a.seg[0].out = g.out;
+  a.seg[0].out_dim = g.mats * g.rows;
   a.in_dim = g.in_dim;
   a.batch = MB;
   a.digits = 4;
@@ -1343,7 +1517,7 @@ static int launch_grouped(int device, const MmaGroupLaunch& g, cudaStream_t stre
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = smem;
   note_launch();
-  GOPH_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
+  GOPH_CUDA(cudaLaunchKernelEx(&cfg, kern, a, NoMaps()));
   return GOPH_OK;
 }
 
@@ -1391,7 +1565,8 @@ __global__ void q80_tile_kernel(const unsigned char* __restrict__ plane, const u
   int row = tile * 128 + r;
   unsigned char* dst = tiled + stg * Fmt<FMT_Q80>::kStageBytes;
   uint4 v = make_uint4(0, 0, 0, 0);
-  if (row < out_dim) {
+  const bool in = row < out_dim && chunk * 256 + step * 32 < in_dim;  // (rows may end inside a chunk, at a block)
+  if (in) {
     v = *reinterpret_cast<const uint4*>(plane + (size_t)row * in_dim + chunk * 256 + step * 32 + half * 16);
     v.x ^= 0x80808080u;
     v.y ^= 0x80808080u;
@@ -1400,7 +1575,7 @@ __global__ void q80_tile_kernel(const unsigned char* __restrict__ plane, const u
   }
   *reinterpret_cast<uint4*>(dst + step * 4096 + half * 2048 + (r >> 3) * 128 + (r & 7) * 16) = v;
   if (half == 0) {
-    uint16_t d = row < out_dim ? d16[(size_t)row * (in_dim / 32) + chunk * 8 + step] : (uint16_t)0;
+    uint16_t d = in ? d16[(size_t)row * (in_dim / 32) + chunk * 8 + step] : (uint16_t)0;
     *reinterpret_cast<uint16_t*>(dst + Fmt<FMT_Q80>::kStageWBytes + r * 16 + step * 2) = d;
   }
 }
@@ -1554,11 +1729,11 @@ __global__ void q6k_dequant_tiled_kernel(const unsigned char* __restrict__ tiled
 
 bool gguf_mma_supported(int qtype, int in_dim) {
   return (qtype == GOPH_GGUF_Q4_K || qtype == GOPH_GGUF_Q8_0 || qtype == GOPH_GGUF_Q5_K || qtype == GOPH_GGUF_Q6_K) &&
-         in_dim % kChunkK == 0 && in_dim <= kMaxPrepIn;
+         (in_dim % kChunkK == 0 || (qtype == GOPH_GGUF_Q8_0 && in_dim % 32 == 0)) && in_dim <= kMaxPrepIn;
 }
 
 int gguf_mma_make_tiled(goph_gguf_matrix* m) {
-  const int ntiles = (m->out_dim + kTileRows - 1) / kTileRows, nchunks = m->in_dim / kChunkK;
+  const int ntiles = (m->out_dim + kTileRows - 1) / kTileRows, nchunks = (m->in_dim + kChunkK - 1) / kChunkK;
   const bool q4 = m->qtype == GOPH_GGUF_Q4_K;
   const size_t stage = q4 ? Fmt<FMT_Q4K>::kStageBytes
                           : m->qtype == GOPH_GGUF_Q5_K ? Fmt<FMT_Q5K>::kStageBytes
@@ -1598,15 +1773,20 @@ int gguf_mma_make_tiled(goph_gguf_matrix* m) {
 int gguf_mma_launch(const goph_gguf_matrix* m, float* out, const float* x, int batch, int digits, cudaStream_t stream,
                     SharedX* shared) {
   if (!m->tiled) return fail(GOPH_E_UNSUPPORTED, "matrix is not in the tiled layout");
-  TiledDesc d{m->tiled, m->device, m->out_dim, m->in_dim};
-  if (m->qtype == GOPH_GGUF_Q4_K) return tiled_launch<FMT_Q4K>(d, out, x, batch, digits, stream, shared);
-  if (m->qtype == GOPH_GGUF_Q5_K) return tiled_launch<FMT_Q5K>(d, out, x, batch, digits, stream, shared);
-  if (m->qtype == GOPH_GGUF_Q6_K) return tiled_launch<FMT_Q6K>(d, out, x, batch, digits, stream, shared);
-  return tiled_launch<FMT_Q80>(d, out, x, batch, digits, stream, shared);
+  RowWeights d;
+  d.device = m->device;
+  d.in_dim = m->in_dim;
+  d.n = 1;
+  d.seg[0] = RowSeg{m->tiled, nullptr, out, m->out_dim, 0};
+  d.unordered = m->unordered;
+  if (m->qtype == GOPH_GGUF_Q4_K) return rows_launch<FMT_Q4K, true>(d, x, batch, digits, stream, shared);
+  if (m->qtype == GOPH_GGUF_Q5_K) return rows_launch<FMT_Q5K, true>(d, x, batch, digits, stream, shared);
+  if (m->qtype == GOPH_GGUF_Q6_K) return rows_launch<FMT_Q6K, true>(d, x, batch, digits, stream, shared);
+  return rows_launch<FMT_Q80, true>(d, x, batch, digits, stream, shared);
 }
 
 int gguf_mma_dequant(const goph_gguf_matrix* m, float* out, cudaStream_t stream) {
-  const int nchunks = m->in_dim / kChunkK;
+  const int nchunks = (m->in_dim + kChunkK - 1) / kChunkK;
   if (m->qtype == GOPH_GGUF_Q4_K) {
     size_t units = (size_t)m->out_dim * (m->in_dim / 32);
     q4k_dequant_tiled_kernel<<<(unsigned)((units + 255) / 256), 256, 0, stream>>>(m->tiled, out, m->out_dim, m->in_dim, nchunks);
@@ -1711,8 +1891,9 @@ static WorkPlan plan_work(const MmaWorkLaunch& g) {
   WorkPlan p;
   memset(&p, 0, sizeof p);
   MmaArgs& a = p.a;
-  a.out = g.out;
-  a.out_dim = g.rows;
+  a.nseg = 1;
+  a.seg[0].out = g.out;
+  a.seg[0].out_dim = g.rows;
   a.in_dim = g.in_dim;
   a.batch = MB;
   a.digits = 4;
@@ -1769,7 +1950,7 @@ static int launch_work(int device, const MmaWorkLaunch& g, unsigned char* scratc
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = p.smem;
   note_launch();
-  GOPH_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
+  GOPH_CUDA(cudaLaunchKernelEx(&cfg, kern, a, NoMaps()));
   return GOPH_OK;
 }
 
@@ -1852,30 +2033,28 @@ static int noalloc_base(int device, unsigned char** base) {
 static int launch_noalloc(const goph_mlx_weight* w, float* out, const float* x, unsigned char* base, int digits, cudaStream_t stream) {
   MmaArgs a;
   memset(&a, 0, sizeof a);
-  a.w = w->tiled;
   a.x = x;
-  a.out = out;
   a.status = reinterpret_cast<int*>(base + kNaStatusOff);
   a.counters = reinterpret_cast<unsigned int*>(base + kNaCountersOff);
   a.xb = base + kNaXbOff;
   a.scratch = reinterpret_cast<float*>(base + kNaPartOff);
-  a.out_dim = w->out_dim;
-  a.in_dim = w->in_dim;
   a.batch = 1;
   a.digits = digits == 3 ? 3 : 4;
-  a.ntiles = (w->out_dim + kTileRows - 1) / kTileRows;
-  a.nchunks = w->in_dim / kChunkK;
   // The array keeps whatever the last call left: the arrival counters have to start at zero (the prepared activations and
   // partial sums are fully rewritten before they are read).  The status word is
   // left alone: it is zero when the library is loaded and sticky once a wait has given up, like the
   // allocated path's; goph_mlx_gemv_noalloc_status reads it.
   GOPH_CUDA(cudaMemsetAsync(base + kNaCountersOff, 0, kNaXbOff - kNaCountersOff, stream));
-  TiledDesc d{w->tiled, w->device, w->out_dim, w->in_dim};
+  RowWeights d;
+  d.device = w->device;
+  d.in_dim = w->in_dim;
+  d.n = 1;
+  d.seg[0] = RowSeg{w->tiled, nullptr, out, w->out_dim, 0};
   d.scratch_bytes = kNoAllocBytes - kNaPartOff;
   d.counters = kNoAllocMaxItems * kConsumers;
   SharedX xs;
   xs.written = floats_meet(out, w->out_dim, x, w->in_dim);
-  return launch_one<FMT_MLX4, 1>(d, a, stream, &xs);
+  return rows_slice<FMT_MLX4, true>(d, a, stream, &xs);
 }
 
 }  // namespace goph

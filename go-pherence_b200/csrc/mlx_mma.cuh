@@ -31,6 +31,13 @@ struct SharedX {
 int mlx_mma_launch(const goph_mlx_weight* w, float* out, const float* x, int batch, int digits, cudaStream_t stream,
                    SharedX* shared = nullptr);
 
+// The same for n row-major weights of one device and in_dim that share x, in one launch for up to four of them: groups of 64, bf16 tables, tensor maps
+// (mlx_mma_rows_ok).  No scratch: callers need no order between such calls.
+inline bool mlx_mma_rows_ok(const goph_mlx_weight* w) { return !w->tiled && w->group_size == 64 && w->sb_bf16 && w->qmaps.ok && w->in_dim <= 65536; }
+int mlx_mma_launch_rows(int n, const goph_mlx_weight* const* ws, float* const* outs, const float* x, int batch, int digits, cudaStream_t stream);
+// Allocates the device's scratch (uploads do, so that no product of a weight that may be used under capture has to).
+bool mlx_mma_ready(int device);
+
 // ---- grouped launches: the selected experts of a mixture-of-experts layer --------------------
 // One work entry = one expert (tiled matrices of equal shapes) and up to `rows` (2 or 4, the same
 // for every entry of a call) of the (token, slot) items that chose it; an expert chosen by more

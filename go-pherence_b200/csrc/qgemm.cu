@@ -1535,7 +1535,7 @@ bool qgemm_wants(int fmt, bool tiled, bool x_bf16, long out_dim, int in_dim, int
   }
   if (weights > 1) {  // (MLX) by their mean size: 2048, 1024 and 1024 rows of 1024 at 16 rows 21.4 / 20.2, at 20 28.2 / 22.3;
     const long mean = size / weights;  // 2048, 512, 512 of 2048 at 9 21.6 / 22.6, at 12 24.9 / 22.7; twice 2048x2048 at 8 18.1 / 16.4;
-    return batch > (mean < Mi ? 24 : mean < 2 * Mi ? 16 : mean < 3 * Mi ? 10 : mean < 5 * Mi ? 8 : 4);  // twice 2000x4096 at 4 18.1 / 19.1, at 5 30.2 / 19.1
+    return batch > (mean < Mi ? 24 : mean < 2 * Mi ? 16 : mean < 3 * Mi ? 10 : size <= 12 * Mi ? 8 : 4);
   }
   // Above 8 Mi weights this layout is the exception (widths that no tile takes, NaN codes, the layout options).
   // in_dim above 8192: of x the CUDA-core kernels' shared memory holds four rows (Q8_0, FP8) for one CTA an SM only, or two.
@@ -1555,9 +1555,9 @@ bool qgemm_wants(int fmt, bool tiled, bool x_bf16, long out_dim, int in_dim, int
       const bool two = wide_x || (size >= 8 * Mi && (in_dim >= 6144 || (in_dim >= 2048 ? size < 48 * Mi : many)));
       return batch > (2 * size < 5 * Mi ? 8 : two ? 2 : 4);
     }
-    case Q_Q4K: case Q_MLX4: case Q_MLX4F:
-      // MLX 1024x1024 8 rows 5.4 / 7.2, 9 rows 9.5 / 7.2; 1536x4096 2 rows 7.7 / 9.1, 3 rows 12.6 / 9.1; 8192x2112 13.6 / 11.7, 22.0 / 11.7; 28672x1088
-      // 4 rows 31 / 14.2; Q4_K 1536x4096 2 rows 7.7 / 9.4, 3 rows 12.2 / 9.4
+    case Q_MLX4: case Q_MLX4F: return batch > (size <= 5 * Mi ? 8 : 4);  // 8 rows 2048x2048 6.9 / 8.6, 512x8192 9.9 / 11.3, 5722x1280 11.9 / 8.8, 8192x2112 12.0 / 11.8
+    case Q_Q4K:
+      // 1536x4096 2 rows 7.7 / 9.4, 3 rows 12.2 / 9.4
       return batch > (small ? 8 : (long_rows || (size >= 8 * Mi && in_dim > 1024)) && size <= 64 * Mi ? 2 : 4);
     default:     // FP8 1024x1024 8 rows 5.3 / 7.0, 9 rows 7.1 / 7.0; 2048x2048 4 rows 5.7 / 8.2, 5 rows 9.4 / 8.1; 4096x4160 2 rows 11.4 / 10.1; 512x14336
                  // 2 rows 12.7 / 13.4, 3 rows 22.7 / 13.4; 8192x8256 2 rows 36.2 / 15.8
@@ -1614,7 +1614,7 @@ int qgemm(int n, const QWeight* w, float* const* out, const void* x, bool x_bf16
   bool any[2] = {};
   for (int i = 0; i < n; ++i) {
     if (w[i].in_dim > kMaxIn) return fail(GOPH_E_UNSUPPORTED, "several-row products: in_dim=%d is above %d", w[i].in_dim, kMaxIn);
-    any[w[i].tiled] = true;
+    any[w[i].tiled && !w[i].unordered] = true;
   }
   // the device's area for tiled weights, the stream's for the others; both are held to the call's last launch
   QBufs* bufs[2] = {any[0] ? rows : nullptr, any[1] ? q_bufs(w[0].device) : nullptr};
@@ -1626,7 +1626,7 @@ int qgemm(int n, const QWeight* w, float* const* out, const void* x, bool x_bf16
     held[t] = std::unique_lock<std::mutex>(bufs[t]->enqueue);
   }
   for (int i = 0; i < n; ++i)
-    if (int rc = run_one(w[i], out[i], x, x_bf16, batch, bufs[w[i].tiled], &prep[w[i].tiled], stream)) return rc;
+    if (int rc = run_one(w[i], out[i], x, x_bf16, batch, bufs[w[i].tiled && !w[i].unordered], &prep[w[i].tiled && !w[i].unordered], stream)) return rc;
   return GOPH_OK;
 }
 

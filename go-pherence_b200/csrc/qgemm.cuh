@@ -24,6 +24,7 @@ struct QWeight {
   const float* bias;   // FP8: [out_dim] or nullptr
   int device, out_dim, in_dim;
   const QMaps* maps;
+  bool unordered = false;  // tiled: the scratch is the stream's all the same
 };
 
 // The tensor maps of a weight in its row-major or streaming layout (w and aux as in QWeight).  maps->ok is false where there
@@ -35,7 +36,7 @@ void qgemm_maps(int fmt, const void* w, const void* aux, int out_dim, int in_dim
 // share a launch there count together, out_dim being the sum of theirs.
 bool qgemm_wants(int fmt, bool tiled, bool x_bf16, long out_dim, int in_dim, int batch, int weights = 1);
 
-// Layouts other than the tiled ones: the scratch of a call on this stream (see the definition), which qgemm wants; if
+// Layouts other than the tiled ones, and small tiled matrices: the scratch of a call on this stream (see the definition), which qgemm wants; if
 // there is none, the call is the business of the kernels for few rows, which need none.
 struct QBufs;
 QBufs* qgemm_scratch(int device, cudaStream_t stream);
@@ -54,7 +55,7 @@ void qgemm_weights(int device, int change);
 
 // out[i] [batch][out_dim] = x [batch][in_dim] . W[i]^T for n weights of one device and in_dim, x f32 or bf16 bit
 // patterns, 16-byte aligned, prepared once for weights of the same format and kind of layout.  rows: qgemm_scratch's
-// answer where a weight is not tiled.
+// answer where a weight is not tiled or is unordered.
 int qgemm(int n, const QWeight* w, float* const* out, const void* x, bool x_bf16, int batch, QBufs* rows, cudaStream_t stream);
 
 int qgemm_status(int device);

@@ -26,7 +26,8 @@
  *     on one device whose kernels could overlap on the GPU — different streams with no ordering
  *     between them — must be ordered by the caller (one stream, or events), whatever handles
  *     they use.  The reference launches everything on one stream, which satisfies this.
- *     Products of weights in the other layouts need no such order and may be captured at any time:
+ *     Products of weights in the other layouts, and of GGUF matrices that are in the tensor-core layout by their size alone
+ *     (gguf_layout 0) and have fewer than 8 Mi weights or rows that are no multiple of 256, need no such order and may be captured at any time:
  *     those of several rows keep an area per stream (28 MB, for up to eight streams of a device,
  *     until its last weight is freed) and use the kernels that need none where they have no area
  *     (under capture, on further streams, without memory), whose sums are grouped differently.
@@ -120,9 +121,7 @@ int goph_sm_count(int device);
  *                 over short K ranges, make the activation digits of their own K range inside the
  *                 product kernel (one launch per product);
  *                 0: a separate preparation kernel in front of every product
- *   "mlx_chunks"  256-element chunks per pipeline stage of the tensor-core GEMV: 0 (default) two for
- *                 the nibble formats where tensor memory has the columns (up to 4 activation rows
- *                 for MLX 4-bit, 2 for Q4_K), 1 always one
+ *   "mlx_chunks"  accepted, without effect (a stage of the few-row kernel is one 256-element chunk)
  *   "mlx_splits"  CTAs that share the K range of one 128-row tile (0 = chosen by shape); with several
  *                 rows of an item of the last wave, up to 8, where the device holds that many clusters
  *   "mlx_cluster" 1 (default): K splits that all run at once are launched as thread-block clusters and
