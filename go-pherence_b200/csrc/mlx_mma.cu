@@ -58,46 +58,53 @@ constexpr int kChunkK = 256;  // elements of a pipeline stage
 //   Q4K   the same nibble image (one 256-element super-block per row and stage); f16 d, f16 dmin and
 //         8 x 12 bits (sc | m << 6), one per 32-element sub-block.
 //   Q80   256 signed bytes per row, stored as 8x16-byte matrices [K step][K half][row group][row][16 B]; 8 f16 block scales.
-//   Q5K   the 5-bit values written out as 256 unsigned bytes per row at upload, in Q80's order; the
-//         Q4_K header {d, dmin, 8 x (sc | m << 6)}.
-//   Q6K   the 6-bit values minus 32 as 256 signed bytes per row, in Q80's order; 16 int8 scales, one per 16 elements,
-//         and f16 d per row (32 bytes with padding).
+//   Q5K   the nibble image, in which word t of a unit (32 elements) holds elements 4 t .. 4 t + 3 in the low nibbles of its bytes and
+//         16 + 4 t .. in the high ones; then the fifth bits: [4 units][row][word t], byte b of which has, from bit 0, those of unit 0 low and
+//         high, unit 1 low, ... of byte b; the Q4_K header {d, dmin, 8 x (sc | m << 6)}.
+//   Q6K   the same image; two bits beside every nibble: [2 units][row][word t], byte b: unit 0 low, high, unit 1 low, high (the A byte
+//         is nibble and bits at its top, the highest one inverted: 4 (q - 32), signed); 16 int8 scales per row, one per 16
+//         elements; then f16 d [row].
+//   (Both are as large as in the file.  Written out to bytes, 1.06 and 1.13 a weight, they were bound by HBM at 1.5 and 1.4 times the time.)
 enum { FMT_MLX4 = 0, FMT_Q4K = 1, FMT_Q80 = 2, FMT_Q5K = 3, FMT_Q6K = 4 };
 template <int FMT>
 struct Fmt {
-  static constexpr bool kNibble = FMT == FMT_MLX4 || FMT == FMT_Q4K;
+  static constexpr bool kNibble = FMT != FMT_Q80;                     // a nibble image
+  static constexpr bool kWords = FMT == FMT_MLX4 || FMT == FMT_Q4K;   // whose words hold eight consecutive elements
   static constexpr bool kSigned = FMT == FMT_Q80 || FMT == FMT_Q6K;  // A bytes
   static constexpr bool kSums = FMT == FMT_MLX4 || FMT == FMT_Q4K || FMT == FMT_Q5K;  // biases or minima meet the groups' sums of x
   static constexpr int kGroup = FMT == FMT_MLX4 ? 64 : 32;  // elements of an entry of the activation tables
   static constexpr int kGroups = kChunkK / kGroup;
-  static constexpr int kStageWBytes = kTileRows * (kNibble ? 128 : 256);
-  static constexpr int kMetaRow = FMT == FMT_Q6K ? 32 : 16;  // bytes of scales per row and stage
-  static constexpr int kStageBytes = kStageWBytes + kTileRows * kMetaRow;
+  static constexpr int kHigh = FMT == FMT_Q5K ? 4096 : FMT == FMT_Q6K ? 8192 : 0;  // bits beside the nibbles
+  static constexpr int kHighOff = kTileRows * 128;
+  static constexpr int kStageWBytes = kTileRows * (kNibble ? 128 : 256) + kHigh;
+  static constexpr int kMetaRow = 16;                                               // bytes of scales per row and stage
+  static constexpr int kDOff = kStageWBytes + kTileRows * kMetaRow;                 // Q6_K: d
+  static constexpr int kStageBytes = kDOff + (FMT == FMT_Q6K ? kTileRows * 2 : 0);
 };
 
 // Prepared activations of a chunk and up to MB rows: B fragments, then tables.
 //   fragments  [pair of K steps][n tile][lane][K step of the pair] x 8 bytes: what mma.m16n8k32 wants of lane 4 n + t (column
-//              n = 4 * row + digit).  One row has four columns only: its tiles are [n 4][t 4], the lanes of columns 4 to 7 read the same.
+//              n = 4 * row + digit).  One row would leave columns 4 to 7 idle: blocks of weights with a scale of their own go in pairs,
+//              the digits of the first one's elements stand in columns 0 to 3, of the second one's in 4 to 7, zeros elsewhere, so
+//              that one accumulator tile holds both sums (MLX: groups, Q6_K: the halves of a K step, others: K steps).
 //   tables     per row, parity p of the lane (even lanes hold the sums of the two low digits, odd ones of the two high ones) and
 //              group: the group's scale 2^(E-26) (p = 1: times 2^14) and, where biases or minima want it, its sum of x (p = 0: zero).
-//              One row: all eight columns of an accumulator tile hold its four digits, so lanes 0 and 1 of a quad add up the even
-//              blocks and lanes 2 and 3 the odd ones; per p, half of the quad and pair of blocks the table has both scales, the
-//              other half's as zero, and the half's own sum.
+//              One row: per p, half of the quad (lanes 0 and 1 finish the pairs' first blocks) and pair (Q6_K: per p and group).
 template <int FMT, int MB>
 struct XBlock {
   typedef Fmt<FMT> F;
   static constexpr int NT = MB == 1 ? 1 : MB / 2;  // n tiles of eight columns
-  static constexpr int kFrag = MB == 1 ? 1024 : NT * 2048;
-  static constexpr int kPairs = FMT == FMT_Q6K ? F::kGroups : F::kGroups / 2;  // one row: pairs of blocks (Q6_K's are the halves of a group)
-  static constexpr int kEntry = MB == 1 ? (F::kSums ? 4 : 2) : F::kSums ? 2 : 1;  // floats
-  static constexpr int kTab = MB == 1 ? 4 * kPairs * kEntry : MB * 2 * F::kGroups * kEntry;
+  static constexpr int kFrag = NT * 2048;
+  static constexpr int kEntry = F::kSums ? 2 : 1;  // floats
+  static constexpr int kTab = MB * 2 * F::kGroups * kEntry;
   static constexpr int kBytes = kFrag + kTab * 4;
   static __host__ __device__ __forceinline__ int frag(int step, int n, int t) {
-    if (MB == 1) return (step >> 1) * 256 + (n * 4 + t) * 16 + (step & 1) * 8;
     return ((step >> 1) * NT + (n >> 3)) * 512 + ((n & 7) * 4 + t) * 16 + (step & 1) * 8;
   }
-  static __host__ __device__ __forceinline__ int entry(int m, int p, int g) { return ((m * 2 + p) * F::kGroups + g) * kEntry; }     // several rows
-  static __host__ __device__ __forceinline__ int entry1(int p, int half, int pair) { return ((p * 2 + half) * kPairs + pair) * kEntry; }  // one
+  static __host__ __device__ __forceinline__ int entry(int m, int p, int g) {
+    if (MB == 1 && FMT != FMT_Q6K) return ((p * 2 + (g & 1)) * (F::kGroups / 2) + (g >> 1)) * kEntry;
+    return ((m * 2 + p) * F::kGroups + g) * kEntry;
+  }
 };
 
 __device__ __forceinline__ float max_nan(float a, float b) {  // (fmaxf passes over a NaN)
@@ -148,20 +155,9 @@ __device__ __forceinline__ void prep_chunks(const float (&v)[R][8], int lane, un
       const float sc[2] = {__uint_as_float(finite ? f : 0x7FC00000u), __uint_as_float(finite ? f + (14u << 23) : 0x7FC00000u)};
 #pragma unroll
       for (int p = 0; p < 2; ++p) {
-        if (MB > 1) {
-          float* t = tab + X::entry(m[r], p, g);
-          t[0] = sc[p];
-          if (F::kSums) t[1] = p ? s[r] : 0.f;
-        } else if (FMT == FMT_Q6K) {
-          *reinterpret_cast<float2*>(tab + X::entry1(p, 0, g)) = make_float2(sc[p], 0.f);
-          *reinterpret_cast<float2*>(tab + X::entry1(p, 1, g)) = make_float2(0.f, sc[p]);
-        } else {
-          const int half = g & 1;
-          float* t = tab + X::entry1(p, half, g >> 1);
-          t[half] = sc[p];
-          if (F::kSums) t[2] = p ? s[r] : 0.f;
-          (tab + X::entry1(p, half ^ 1, g >> 1))[half] = 0.f;
-        }
+        float* t = tab + X::entry(m[r], p, g);
+        t[0] = sc[p];
+        if (F::kSums) t[1] = p ? s[r] : 0.f;
       }
     }
     const float fi = __uint_as_float((uint32_t)(qbits - (e - 126) + 127) << 23);
@@ -173,7 +169,7 @@ __device__ __forceinline__ void prep_chunks(const float (&v)[R][8], int lane, un
       uint32_t p[2];
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        auto at = [&](int i) { return (uint32_t)(q[F::kNibble ? 2 * i + h : 4 * h + i] >> (7 * d)); };
+        auto at = [&](int i) { return (uint32_t)(q[F::kWords ? 2 * i + h : 4 * h + i] >> (7 * d)); };
         p[h] = __byte_perm(__byte_perm(at(0), at(1), 0x0040), __byte_perm(at(2), at(3), 0x0040), 0x5410);
         if (d < digits - 1) {
           p[h] = (p[h] & 0x7F7F7F7Fu) ^ 0x40404040u;
@@ -184,13 +180,21 @@ __device__ __forceinline__ void prep_chunks(const float (&v)[R][8], int lane, un
       return make_uint2(p[0], p[1]);
     };
     const int step = lane >> 2, w = lane & 3;  // the lane's eight positions are 8 w .. 8 w + 7 of the K step
-    auto put = [&](int d, uint2 t) {
-      const int n = m[r] * 4 + d;
-      if (F::kNibble) {  // the nibbles' order: even elements of a packed word, then odd ones
+    auto put_at = [&](int n, uint2 t) {
+      if (F::kWords) {  // the nibbles' order: even elements of a packed word, then odd ones
         *reinterpret_cast<uint2*>(xb[r] + X::frag(step, n, w)) = t;
       } else {
         *reinterpret_cast<uint32_t*>(xb[r] + X::frag(step, n, 2 * (w & 1)) + 4 * (w >> 1)) = t.x;
         *reinterpret_cast<uint32_t*>(xb[r] + X::frag(step, n, 2 * (w & 1) + 1) + 4 * (w >> 1)) = t.y;
+      }
+    };
+    const int half = FMT == FMT_MLX4 ? (step >> 1) & 1 : FMT == FMT_Q6K ? w >> 1 : step & 1;
+    auto put = [&](int d, uint2 t) {
+      if (MB > 1) {
+        put_at(m[r] * 4 + d, t);
+      } else {
+        put_at(half * 4 + d, t);
+        put_at((half ^ 1) * 4 + d, make_uint2(0, 0));
       }
     };
     if (SPLIT == 4) {
@@ -277,7 +281,7 @@ __device__ __forceinline__ void stage_scales(const unsigned char* st, int row, u
   float v[8];
   if (FMT == FMT_Q6K) {  // bytes 8 q .. 8 q + 7
     const uint2 w = *reinterpret_cast<const uint2*>(p + 8 * q);
-    const float dd = f16_lo(*reinterpret_cast<const uint32_t*>(p + 16));
+    const float dd = 0.25f * __half2float(*reinterpret_cast<const __half*>(st + Fmt<FMT>::kDOff + (row + r) * 2));  // (the bytes are 4 (q - 32))
 #pragma unroll
     for (int k = 0; k < 8; ++k) v[k] = __fmul_rn(dd, __uint_as_float(__byte_perm((k < 4 ? w.x : w.y) ^ 0x80808080u, 0x4B000000u, 0x7440u + (k & 3))) - 8388736.f);
   } else {
@@ -301,10 +305,10 @@ template <int FMT>
 struct RowScales {
   uint4 w;
   float d, kd, m, km;
-  __device__ __forceinline__ void load(const unsigned char* p) {
-    w = *reinterpret_cast<const uint4*>(p);
+  __device__ __forceinline__ void load(const unsigned char* st, int row) {
+    w = *reinterpret_cast<const uint4*>(st + Fmt<FMT>::kStageWBytes + row * Fmt<FMT>::kMetaRow);
     if (FMT == FMT_Q6K) {
-      d = f16_lo(*reinterpret_cast<const uint32_t*>(p + 16));
+      d = 0.25f * __half2float(*reinterpret_cast<const __half*>(st + Fmt<FMT>::kDOff + row * 2));
       w.x ^= 0x80808080u;
       w.y ^= 0x80808080u;
       w.z ^= 0x80808080u;
@@ -602,9 +606,7 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
       // every item of this CTA covers the same K range (the grid is a multiple of the K splits)
       if (sw.live(a)) {
         const int n = sw.c1 - sw.c;
-        // (two of a warp's chunks at once, and the next two are under way)
         auto load = [&](int i, float (&v)[8]) {
-          if (i >= a.batch * n) return;
           const int m = MB == 1 ? 0 : i / n, k = (sw.c + i - m * n) * kChunkK + lane * 8;
           if (k < a.in_dim) {
             load_eight(a.x + (size_t)m * a.in_dim + k, v);
@@ -613,27 +615,16 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
             for (int e = 0; e < 8; ++e) v[e] = 0.f;
           }
         };
-        float v[2][8] = {};
-        load(warp, v[0]);
-        load(warp + kConsumers, v[1]);
+        float v[8];
+        if (warp < a.batch * n) load(warp, v);
 #pragma unroll 1
-        for (int i = warp; i < a.batch * n; i += 2 * kConsumers) {
-          float u[2][8] = {};
-          load(i + 2 * kConsumers, u[0]);
-          load(i + 3 * kConsumers, u[1]);
-          const int i1 = i + kConsumers, m0 = MB == 1 ? 0 : i / n, m1 = MB == 1 ? 0 : i1 / n;
-          if (i1 < a.batch * n) {
-            unsigned char* const at[2] = {bres + (size_t)(i - m0 * n) * X::kBytes, bres + (size_t)(i1 - m1 * n) * X::kBytes};
-            const int ms[2] = {m0, m1};
-            prep_chunks<FMT, MB, 1, 2>(v, lane, at, ms, a.digits);
-          } else {
-            prep_chunk<FMT, MB>(v[0], lane, bres + (size_t)(i - m0 * n) * X::kBytes, m0, a.digits);
-          }
+        for (int i = warp; i < a.batch * n; i += kConsumers) {
+          float u[8] = {};
+          if (i + kConsumers < a.batch * n) load(i + kConsumers, u);  // (the next chunk is under way while this one is worked on)
+          const int m = MB == 1 ? 0 : i / n;
+          prep_chunk<FMT, MB>(v, lane, bres + (size_t)(i - m * n) * X::kBytes, m, a.digits);
 #pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            v[0][e] = u[0][e];
-            v[1][e] = u[1][e];
-          }
+          for (int e = 0; e < 8; ++e) v[e] = u[e];
         }
       }
       asm volatile("bar.sync 1, %0;" ::"n"(kConsumers * 32) : "memory");
@@ -642,8 +633,8 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
     // of its part of the fragments and tables
     const int mi = lane >> 3, lr = lane & 7;
     const uint32_t a_lane = F::kNibble ? (row0 + (mi & 1) * 8 + lr) * 128 : (mi >> 1) * 2048 + (row0 / 8 + (mi & 1)) * 128 + lr * 16;
-    const uint32_t b_lane = MB == 1 ? ((g & 3) * 4 + t) * 16 : lane * 16;
-    const int t_lane = X::kFrag + 4 * (MB == 1 ? X::entry1(p, half, 0) : X::entry(half, p, 0));
+    const uint32_t b_lane = lane * 16;
+    const int t_lane = X::kFrag + 4 * (MB > 1 ? X::entry(half, p, 0) : X::entry(0, p, FMT == FMT_Q6K ? 0 : half));
     unsigned char* sc_warp = scales + warp * (SL * 16 * kStagedRow);
     float gate[kWork ? C::kVals : 1];
     int cur_entry = -1, nb = a.batch;
@@ -688,7 +679,7 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
 #pragma unroll
           for (int sl = 0; sl < SL; ++sl)
 #pragma unroll
-            for (int r = 0; r < 2; ++r) rs[sl][r].load(meta + (16 * sl + 8 * r) * F::kMetaRow);
+            for (int r = 0; r < 2; ++r) rs[sl][r].load(st, row0 + 16 * sl + 8 * r + g);
         }
         // scales (and biases) of the rows g + 8 r of slab sl
         auto mlx_scale = [&](int sl, int r, int word, float& sv, float& bv) {  // word: per lane
@@ -697,13 +688,33 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
           bv = __uint_as_float(w & 0xFFFF0000u);
         };
         // A fragments of K step s
-        uint32_t af[SL][2][4];
+        uint32_t af[SL][2][4], high[FMT == FMT_Q5K || FMT == FMT_Q6K ? SL : 1][4];
         auto load_a = [&](int j) {  // both steps of pair j
 #pragma unroll
           for (int sl = 0; sl < SL; ++sl) {
             if (F::kNibble) {
               uint32_t q[4];
               ldsm4(st_a + sl * 2048 + ((((2 * j + (mi >> 1)) ^ lr) << 4)), q);
+              if (FMT == FMT_Q5K || FMT == FMT_Q6K) {  // bits [block][row]: two blocks of rows g and g + 8 a load
+                if (FMT == FMT_Q6K ? j % 2 == 0 : j == 0) ldsm4(smem_u32(st) + F::kHighOff + (j + (mi >> 1)) * 2048 + (row0 + 16 * sl + (mi & 1) * 8 + lr) * 16, high[sl]);
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+#pragma unroll
+                  for (int r = 0; r < 2; ++r) {
+                    const uint32_t w = q[2 * k + r], hb = high[sl][2 * (FMT == FMT_Q6K ? j % 2 : j / 2) + r];
+                    auto at = [&](int left) { return left > 0 ? hb << left : hb >> -left; };
+                    if (FMT == FMT_Q6K) {
+                      af[sl][k][r] = ((w << 2) & 0x3C3C3C3Cu) | ((at(6 - 4 * k) & 0xC0C0C0C0u) ^ 0x80808080u);
+                      af[sl][k][2 + r] = ((w >> 2) & 0x3C3C3C3Cu) | ((at(4 - 4 * k) & 0xC0C0C0C0u) ^ 0x80808080u);
+                    } else {
+                      const int f = 2 * (2 * (j % 2) + k);
+                      af[sl][k][r] = (w & 0x0F0F0F0Fu) | (at(4 - f) & 0x10101010u);
+                      af[sl][k][2 + r] = ((w >> 4) & 0x0F0F0F0Fu) | (at(3 - f) & 0x10101010u);
+                    }
+                  }
+                }
+                continue;
+              }
 #pragma unroll
               for (int k = 0; k < 2; ++k) {
                 af[sl][k][0] = q[2 * k] & 0x0F0F0F0Fu;
@@ -717,21 +728,15 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
             }
           }
         };
-        auto frag = [&](int j, int nt) { return *reinterpret_cast<const uint4*>(xf + (j * NT + nt) * (MB == 1 ? 256 : 512)); };
+        auto frag = [&](int j, int nt) { return *reinterpret_cast<const uint4*>(xf + (j * NT + nt) * 512); };
         // one block's sums into the accumulators: scale and bias of the row, scale and sum of the activations
         auto add = [&](float& ac, const int (&d)[4], int r, float sv, float bv, float xs, float sx) {
           ac = fmaf(sv, digits_sum(d[2 * r], d[2 * r + 1]) * xs, ac);
           if (F::kSums) ac = fmaf(bv, sx, ac);
         };
-        // one row: the two blocks of a pair, of which the lane's half is the one whose scale is not zero
-        auto add_pair = [&](float& ac, const int (&d)[2][4], int r, float sv, float bv, const float4& x) {
-          ac = fmaf(sv, fmaf(digits_sum(d[1][2 * r], d[1][2 * r + 1]), x.y, digits_sum(d[0][2 * r], d[0][2 * r + 1]) * x.x), ac);
-          if (F::kSums) ac = fmaf(bv, x.z, ac);
-        };
-        auto tab1 = [&](int pr) {
-          if (F::kSums) return *reinterpret_cast<const float4*>(xt + pr * 16);
-          const float2 v = *reinterpret_cast<const float2*>(xt + pr * 8);
-          return make_float4(v.x, v.y, 0.f, 0.f);
+        auto tab1 = [&](int pr) {  // one row: of pair pr
+          if (F::kSums) return *reinterpret_cast<const float2*>(xt + pr * 8);
+          return make_float2(*reinterpret_cast<const float*>(xt + pr * 4), 0.f);
         };
         auto tab = [&](int nt, int grp_) {  // scale and sum
           const int at = nt * 4 * F::kGroups + grp_;
@@ -742,7 +747,7 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
           if constexpr (MB == 1) {
 #pragma unroll
             for (int jj = 0; jj < 2; ++jj) {
-              int d[SL][2][4];
+              int d[SL][4];
 #pragma unroll
               for (int h = 0; h < 2; ++h) {
                 const int j = 2 * jj + h;
@@ -750,19 +755,20 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
                 const uint4 b = frag(j, 0);
 #pragma unroll
                 for (int sl = 0; sl < SL; ++sl) {
-                  int(&e)[4] = d[sl][h];
-                  imma32<false>(e, af[sl][0][0], af[sl][0][1], af[sl][0][2], af[sl][0][3], b.x, b.y, kAcc0, kAcc0, kAcc0, kAcc0);
+                  int(&e)[4] = d[sl];
+                  if (h == 0) imma32<false>(e, af[sl][0][0], af[sl][0][1], af[sl][0][2], af[sl][0][3], b.x, b.y, kAcc0, kAcc0, kAcc0, kAcc0);
+                  else imma32<false>(e, af[sl][0][0], af[sl][0][1], af[sl][0][2], af[sl][0][3], b.x, b.y, e[0], e[1], e[2], e[3]);
                   imma32<false>(e, af[sl][1][0], af[sl][1][1], af[sl][1][2], af[sl][1][3], b.z, b.w, e[0], e[1], e[2], e[3]);
                 }
               }
-              const float4 x = tab1(jj);
+              const float2 x = tab1(jj);
 #pragma unroll
               for (int sl = 0; sl < SL; ++sl) {
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
                   float sv, bv;
                   mlx_scale(sl, r, 2 * jj + half, sv, bv);
-                  add_pair(acc[sl][0][r], d[sl], r, sv, bv, x);
+                  add(acc[sl][0][r], d[sl], r, sv, bv, x.x, x.y);
                 }
               }
             }
@@ -796,18 +802,15 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
             load_a(j);
             if constexpr (MB == 1) {
               const uint4 b = frag(j, 0);
-              const float4 xx = *reinterpret_cast<const float4*>(xt + j * 16);  // both steps' entries
+              const float2 xx = *reinterpret_cast<const float2*>(xt + j * 8);  // both steps' scales
 #pragma unroll
               for (int sl = 0; sl < SL; ++sl) {
 #pragma unroll
                 for (int k = 0; k < 2; ++k) {
-                  int d[2][4];
-                  imma16(d[0], af[sl][k][0], af[sl][k][1], k ? b.z : b.x, kAcc0);
-                  imma16(d[1], af[sl][k][2], af[sl][k][3], k ? b.w : b.y, kAcc0);
+                  int d[4];
+                  imma32<true>(d, af[sl][k][0], af[sl][k][1], af[sl][k][2], af[sl][k][3], k ? b.z : b.x, k ? b.w : b.y, kAcc0, kAcc0, kAcc0, kAcc0);
 #pragma unroll
-                  for (int r = 0; r < 2; ++r) {
-                    add_pair(acc[sl][0][r], d, r, rs[sl][r].pair(2 * j + k, half).x, 0.f, k ? make_float4(xx.z, xx.w, 0.f, 0.f) : xx);
-                  }
+                  for (int r = 0; r < 2; ++r) add(acc[sl][0][r], d, r, rs[sl][r].pair(2 * j + k, half).x, 0.f, k ? xx.y : xx.x, 0.f);
                 }
               }
             } else {
@@ -857,16 +860,16 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
             load_a(j);
             if constexpr (MB == 1) {
               const uint4 b = frag(j, 0);
-              const float4 x = tab1(j);
+              const float2 x = tab1(j);
 #pragma unroll
               for (int sl = 0; sl < SL; ++sl) {
-                int d[2][4];
-                imma32<F::kSigned>(d[0], af[sl][0][0], af[sl][0][1], af[sl][0][2], af[sl][0][3], b.x, b.y, kAcc0, kAcc0, kAcc0, kAcc0);
-                imma32<F::kSigned>(d[1], af[sl][1][0], af[sl][1][1], af[sl][1][2], af[sl][1][3], b.z, b.w, kAcc0, kAcc0, kAcc0, kAcc0);
+                int d[4];
+                imma32<F::kSigned>(d, af[sl][0][0], af[sl][0][1], af[sl][0][2], af[sl][0][3], b.x, b.y, kAcc0, kAcc0, kAcc0, kAcc0);
+                imma32<F::kSigned>(d, af[sl][1][0], af[sl][1][1], af[sl][1][2], af[sl][1][3], b.z, b.w, d[0], d[1], d[2], d[3]);
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
                   const float2 sb = rs[sl][r].pair(j, half);
-                  add_pair(acc[sl][0][r], d, r, sb.x, sb.y, x);
+                  add(acc[sl][0][r], d, r, sb.x, sb.y, x.x, x.y);
                 }
               }
             } else {
@@ -1308,6 +1311,7 @@ static int launch_one(const RowWeights& w, const MmaArgs& a, cudaStream_t stream
     if (n > most) n = most;
     if (n > 8 && 16 * tiles > slots) n = 8;  // (larger clusters where eight CTAs a tile leave more than half of the places empty: 256x16384 5.7 / 4.5; 4096x14336 8.4 / 9.2)
     const bool clusters = options().mlx_cluster || alone;
+    if (!whole && n == 8 && 40 * tiles > 4 * slots) n = 7;  // (eights pack badly where they would have to fill the device: 4096x14336 9.2 / 8.3)
     if (clusters)
       while (n > 1 && cluster_room(w.device, n, whole) < tiles) --n;
     if (options().mlx_splits > 0 && !alone) n = options().mlx_splits < a.nchunks ? options().mlx_splits : a.nchunks;
@@ -1620,78 +1624,78 @@ __global__ void q80_dequant_tiled_kernel(const unsigned char* __restrict__ tiled
   out[i] = __fmul_rn(__half2float(__ushort_as_half(d)), (float)q);
 }
 
+// Where element k of a stage's row r lies in the nibble image of Q5_K and Q6_K: byte, and whether in the high nibble; the bits beside it.
+__device__ __forceinline__ int kq_byte(int r, int k) { return r * 128 + (((k >> 5) ^ (r & 7)) << 4) + (k & 15); }
+__device__ __forceinline__ bool kq_upper(int k) { return (k & 16) != 0; }
+__device__ __forceinline__ int q5k_bit_byte(int r, int k) { return Fmt<FMT_Q5K>::kHighOff + (k >> 7) * 2048 + r * 16 + (k & 15); }
+__device__ __forceinline__ int q5k_bit(int k) { return 2 * ((k >> 5) & 3) + ((k >> 4) & 1); }
+__device__ __forceinline__ int q6k_bits_byte(int r, int k) { return Fmt<FMT_Q6K>::kHighOff + (k >> 6) * 2048 + r * 16 + (k & 15); }
+__device__ __forceinline__ int q6k_bits(int k) { return 4 * ((k >> 5) & 1) + 2 * ((k >> 4) & 1); }
+
 // Q5_K super-blocks in the streaming layout {16-byte header, 8 x 16 bytes of nibbles, 8 x 4 bytes of
-// fifth bits} -> stages of unsigned bytes in Q80's order + the header; one thread per 16-byte unit.
+// fifth bits} -> stages; a thread per byte of nibbles (two elements), of bits (eight) and per header.
 __global__ void q5k_tile_kernel(const unsigned char* __restrict__ blocks, unsigned char* __restrict__ tiled, int out_dim,
                                 int ntiles, int nchunks) {
   size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr int kPer = 128 + 32 + 1;
   size_t nstages = (size_t)ntiles * nchunks;
-  if (idx >= nstages * (128 * 17)) return;
-  size_t stg = idx / (128 * 17);
-  int rem = (int)(idx - stg * (128 * 17));
+  if (idx >= nstages * (128 * kPer)) return;
+  size_t stg = idx / (128 * kPer);
+  int rem = (int)(idx - stg * (128 * kPer));
   int tile = (int)(stg / nchunks), chunk = (int)(stg - (size_t)tile * nchunks);
-  int r = rem / 17, hb = rem - r * 17, row = tile * 128 + r;
+  int r = rem / kPer, i = rem - r * kPer, row = tile * 128 + r;
   unsigned char* dst = tiled + stg * Fmt<FMT_Q5K>::kStageBytes;
   const unsigned char* src = blocks + ((size_t)row * nchunks + chunk) * 176;
-  uint4 v = make_uint4(0, 0, 0, 0);
-  if (hb == 16) {
-    if (row < out_dim) v = *reinterpret_cast<const uint4*>(src);
+  const bool in = row < out_dim;
+  auto nib = [&](int k) { return (uint32_t)(src[16 + (k >> 1)] >> (4 * (k & 1))) & 0xFu; };
+  auto fifth = [&](int k) { return (uint32_t)(src[144 + (k >> 3)] >> (k & 7)) & 1u; };
+  if (i < 128) {
+    const int k = (i >> 4) * 32 + (i & 15);  // and k + 16
+    dst[kq_byte(r, k)] = in ? (unsigned char)(nib(k) | (nib(k + 16) << 4)) : 0;
+  } else if (i < 160) {
+    const int k = (i - 128) / 16 * 128 + (i & 15);  // of units 0 to 3 of the block, low and high
+    uint32_t b = 0;
+    for (int f = 0; f < 8 && in; ++f) b |= fifth(k + (f >> 1) * 32 + (f & 1) * 16) << f;
+    dst[q5k_bit_byte(r, k)] = (unsigned char)b;
+  } else {
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (in) v = *reinterpret_cast<const uint4*>(src);
     *reinterpret_cast<uint4*>(dst + Fmt<FMT_Q5K>::kStageWBytes + r * 16) = v;
-    return;
   }
-  const int step = hb >> 1, half = hb & 1;
-  if (row < out_dim) {
-    const uint2 q = *reinterpret_cast<const uint2*>(src + 16 + 16 * step + 8 * half);  // 16 nibbles
-    const uint32_t fifth = *reinterpret_cast<const uint32_t*>(src + 144 + 4 * step) >> (16 * half);
-    uint32_t out[4] = {0, 0, 0, 0};
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const uint32_t nib = ((j < 8 ? q.x : q.y) >> (4 * (j & 7))) & 0xFu;
-      out[j >> 2] |= (nib | (((fifth >> j) & 1u) << 4)) << (8 * (j & 3));
-    }
-    v = make_uint4(out[0], out[1], out[2], out[3]);
-  }
-  *reinterpret_cast<uint4*>(dst + step * 4096 + half * 2048 + (r >> 3) * 128 + (r & 7) * 16) = v;
 }
 
-// Q6_K planes (low nibbles, two-bit highs, int8 scales, f16 d) -> stages of signed bytes (value - 32)
-// in Q80's order + {16 scales, d, padding} per row; one thread per 16-byte unit.
+// Q6_K planes (low nibbles, two-bit highs, int8 scales, f16 d) -> stages; a thread per byte of nibbles (two elements), of bits (four) and
+// per row's scales.
 __global__ void q6k_tile_kernel(const unsigned char* __restrict__ lo, const unsigned char* __restrict__ hi,
                                 const signed char* __restrict__ sc, const uint16_t* __restrict__ dd,
                                 unsigned char* __restrict__ tiled, int out_dim, int in_dim, int ntiles, int nchunks) {
   size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr int kPer = 128 + 64 + 1;
   size_t nstages = (size_t)ntiles * nchunks;
-  if (idx >= nstages * (128 * 18)) return;
-  size_t stg = idx / (128 * 18);
-  int rem = (int)(idx - stg * (128 * 18));
+  if (idx >= nstages * (128 * kPer)) return;
+  size_t stg = idx / (128 * kPer);
+  int rem = (int)(idx - stg * (128 * kPer));
   int tile = (int)(stg / nchunks), chunk = (int)(stg - (size_t)tile * nchunks);
-  int r = rem / 18, hb = rem - r * 18, row = tile * 128 + r;
+  int r = rem / kPer, i = rem - r * kPer, row = tile * 128 + r;
   unsigned char* dst = tiled + stg * Fmt<FMT_Q6K>::kStageBytes;
-  uint4 v = make_uint4(0, 0, 0, 0);
-  if (hb == 16) {
-    if (row < out_dim) v = *reinterpret_cast<const uint4*>(sc + (size_t)row * (in_dim / 16) + chunk * 16);
-    *reinterpret_cast<uint4*>(dst + Fmt<FMT_Q6K>::kStageWBytes + r * 32) = v;
-    return;
+  const bool in = row < out_dim;
+  const unsigned char *l = lo + (size_t)row * (in_dim / 2) + chunk * 128, *h = hi + (size_t)row * (in_dim / 4) + chunk * 64;
+  auto nib = [&](int k) { return (uint32_t)(l[k >> 1] >> (4 * (k & 1))) & 0xFu; };
+  auto two = [&](int k) { return (uint32_t)(h[k >> 2] >> (2 * (k & 3))) & 3u; };
+  if (i < 128) {
+    const int k = (i >> 4) * 32 + (i & 15);
+    dst[kq_byte(r, k)] = in ? (unsigned char)(nib(k) | (nib(k + 16) << 4)) : 0;
+  } else if (i < 192) {
+    const int k = (i - 128) / 16 * 64 + (i & 15);
+    uint32_t b = 0;
+    for (int f = 0; f < 4 && in; ++f) b |= two(k + (f >> 1) * 32 + (f & 1) * 16) << (2 * f);
+    dst[q6k_bits_byte(r, k)] = (unsigned char)b;
+  } else {
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (in) v = *reinterpret_cast<const uint4*>(sc + (size_t)row * (in_dim / 16) + chunk * 16);
+    *reinterpret_cast<uint4*>(dst + Fmt<FMT_Q6K>::kStageWBytes + r * 16) = v;
+    *reinterpret_cast<uint16_t*>(dst + Fmt<FMT_Q6K>::kDOff + r * 2) = in ? dd[(size_t)row * nchunks + chunk] : (uint16_t)0;
   }
-  if (hb == 17) {
-    if (row < out_dim) v.x = dd[(size_t)row * nchunks + chunk];
-    *reinterpret_cast<uint4*>(dst + Fmt<FMT_Q6K>::kStageWBytes + r * 32 + 16) = v;
-    return;
-  }
-  const int step = hb >> 1, half = hb & 1;
-  if (row < out_dim) {
-    const size_t col = (size_t)chunk * 256 + step * 32 + half * 16;  // 16 elements: two words of nibbles, one of highs
-    const uint2 wl = *reinterpret_cast<const uint2*>(lo + (size_t)row * (in_dim / 2) + col / 2);
-    const uint32_t wh = *reinterpret_cast<const uint32_t*>(hi + (size_t)row * (in_dim / 4) + col / 4);
-    uint32_t out[4] = {0, 0, 0, 0};
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const int q = (int)((((j < 8 ? wl.x : wl.y) >> (4 * (j & 7))) & 0xFu) | (((wh >> (2 * j)) & 3u) << 4)) - 32;
-      out[j >> 2] |= (uint32_t)(q & 0xFF) << (8 * (j & 3));
-    }
-    v = make_uint4(out[0], out[1], out[2], out[3]);
-  }
-  *reinterpret_cast<uint4*>(dst + step * 4096 + half * 2048 + (r >> 3) * 128 + (r & 7) * 16) = v;
 }
 
 // dequantRowQ5K / dequantRowQ6K from the tiled layouts (loader/gguf/quant_matrix.go:331-426), the
@@ -1701,7 +1705,7 @@ __global__ void q5k_dequant_tiled_kernel(const unsigned char* __restrict__ tiled
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (size_t)out_dim * in_dim) return;
   int row = (int)(i / in_dim), col = (int)(i - (size_t)row * in_dim);
-  int chunk = col >> 8, k = col & 255, step = k >> 5, half = (k >> 4) & 1, r = row & 127;
+  int chunk = col >> 8, k = col & 255, step = k >> 5, r = row & 127;
   const unsigned char* stg = tiled + ((size_t)(row >> 7) * nchunks + chunk) * Fmt<FMT_Q5K>::kStageBytes;
   const uint4 h = *reinterpret_cast<const uint4*>(stg + Fmt<FMT_Q5K>::kStageWBytes + r * 16);
   const int bit = 12 * step, wi = bit >> 5, sh = bit & 31;
@@ -1709,7 +1713,7 @@ __global__ void q5k_dequant_tiled_kernel(const unsigned char* __restrict__ tiled
   const uint32_t f = __funnelshift_r(lo, hi, sh) & 0xFFFu;
   const float sd = __fmul_rn((float)(f & 63u), __half2float(__ushort_as_half((unsigned short)(h.x & 0xFFFFu))));
   const float md = __fmul_rn((float)(f >> 6), __half2float(__ushort_as_half((unsigned short)(h.x >> 16))));
-  const unsigned char q = stg[step * 4096 + half * 2048 + (r >> 3) * 128 + (r & 7) * 16 + (k & 15)];
+  const uint32_t q = ((stg[kq_byte(r, k)] >> (kq_upper(k) ? 4 : 0)) & 0xFu) | (((stg[q5k_bit_byte(r, k)] >> q5k_bit(k)) & 1u) << 4);
   out[i] = __fsub_rn(__fmul_rn(sd, (float)q), md);
 }
 
@@ -1718,13 +1722,12 @@ __global__ void q6k_dequant_tiled_kernel(const unsigned char* __restrict__ tiled
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (size_t)out_dim * in_dim) return;
   int row = (int)(i / in_dim), col = (int)(i - (size_t)row * in_dim);
-  int chunk = col >> 8, k = col & 255, step = k >> 5, half = (k >> 4) & 1, r = row & 127;
+  int chunk = col >> 8, k = col & 255, r = row & 127;
   const unsigned char* stg = tiled + ((size_t)(row >> 7) * nchunks + chunk) * Fmt<FMT_Q6K>::kStageBytes;
-  const unsigned char* mrow = stg + Fmt<FMT_Q6K>::kStageWBytes + r * 32;
-  const float d = __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short*>(mrow + 16)));
-  const signed char sc = (signed char)mrow[k >> 4];
-  const signed char q = (signed char)stg[step * 4096 + half * 2048 + (r >> 3) * 128 + (r & 7) * 16 + (k & 15)];
-  out[i] = __fmul_rn(__fmul_rn(d, (float)sc), (float)q);
+  const float d = __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short*>(stg + Fmt<FMT_Q6K>::kDOff + r * 2)));
+  const signed char sc = (signed char)stg[Fmt<FMT_Q6K>::kStageWBytes + r * 16 + (k >> 4)];
+  const uint32_t low = (stg[kq_byte(r, k)] >> (kq_upper(k) ? 4 : 0)) & 0xFu, two = (stg[q6k_bits_byte(r, k)] >> q6k_bits(k)) & 3u;
+  out[i] = __fmul_rn(__fmul_rn(d, (float)sc), (float)((int)(low | (two << 4)) - 32));
 }
 
 bool gguf_mma_supported(int qtype, int in_dim) {
@@ -1735,23 +1738,23 @@ bool gguf_mma_supported(int qtype, int in_dim) {
 int gguf_mma_make_tiled(goph_gguf_matrix* m) {
   const int ntiles = (m->out_dim + kTileRows - 1) / kTileRows, nchunks = (m->in_dim + kChunkK - 1) / kChunkK;
   const bool q4 = m->qtype == GOPH_GGUF_Q4_K;
-  const size_t stage = q4 ? Fmt<FMT_Q4K>::kStageBytes
-                          : m->qtype == GOPH_GGUF_Q5_K ? Fmt<FMT_Q5K>::kStageBytes
-                          : m->qtype == GOPH_GGUF_Q6_K ? Fmt<FMT_Q6K>::kStageBytes : Fmt<FMT_Q80>::kStageBytes;
-  const size_t bytes = (size_t)ntiles * nchunks * stage;
+  // Bytes of a row and stage.  Q5_K and Q6_K lie in the front of theirs (176 and 210): the sizes are those that programs budget
+  // with (goph_gguf_resident_bytes), from when these formats were written out to bytes.
+  const size_t row = q4 ? 144 : m->qtype == GOPH_GGUF_Q6_K ? 288 : 272;
+  const size_t bytes = (size_t)ntiles * nchunks * kTileRows * row;
   unsigned char* t = nullptr;
   GOPH_CUDA(cudaMalloc(&t, bytes));
   if (q4) {
     size_t threads = (size_t)ntiles * nchunks * 128 * 9;
     q4k_tile_kernel<<<(unsigned)((threads + 255) / 256), 256>>>(m->data, t, m->out_dim, ntiles, nchunks);
   } else if (m->qtype == GOPH_GGUF_Q5_K) {
-    size_t threads = (size_t)ntiles * nchunks * 128 * 17;
+    size_t threads = (size_t)ntiles * nchunks * 128 * 161;
     q5k_tile_kernel<<<(unsigned)((threads + 255) / 256), 256>>>(m->data, t, m->out_dim, ntiles, nchunks);
   } else if (m->qtype == GOPH_GGUF_Q6_K) {
     // planes behind one another: low nibbles in data; highs, int8 scales, f16 d in d16's buffer
     const size_t n = (size_t)m->out_dim * m->in_dim;
     const unsigned char* hi = reinterpret_cast<const unsigned char*>(m->d16);
-    size_t threads = (size_t)ntiles * nchunks * 128 * 18;
+    size_t threads = (size_t)ntiles * nchunks * 128 * 193;
     q6k_tile_kernel<<<(unsigned)((threads + 255) / 256), 256>>>(m->data, hi, reinterpret_cast<const signed char*>(hi + n / 4),
                                                                 reinterpret_cast<const uint16_t*>(hi + n / 4 + n / 16), t, m->out_dim,
                                                                 m->in_dim, ntiles, nchunks);

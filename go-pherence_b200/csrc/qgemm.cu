@@ -108,15 +108,17 @@ struct QF {
   // (metadata beside them: kMeta bytes a row; Q6_K of the streaming layout: 16 of scales a row, then 4 with d a row)
   static constexpr bool kMLX = F == Q_MLX4 || F == Q_MLX4F;
   static constexpr bool kNibble = kMLX || F == Q_Q4K || (!TILED && (F == Q_Q5K || F == Q_Q6K));
-  static constexpr int kHigh = kNibble && F == Q_Q5K ? 4096 : kNibble && F == Q_Q6K ? 8192 : 0;  // bits above the nibble, [16-byte unit][row]
+  // Q5_K, Q6_K tiled: a nibble image in another order, and the bits above the nibbles beside it (mlx_mma.cu, Fmt)
+  static constexpr bool kPacked = TILED && (F == Q_Q5K || F == Q_Q6K);
+  static constexpr int kHigh = !kNibble && !kPacked ? 0 : F == Q_Q5K ? 4096 : F == Q_Q6K ? 8192 : 0;  // bits above the nibble, [16-byte unit][row]
   static constexpr int kHighOff = kTileRows * 128;
-  static constexpr int kWBytes = (kNibble ? kTileRows * 128 : kTileRows * 256) + kHigh;
-  static constexpr int kMeta = F == Q_FP8 ? 0 : F == Q_Q6K || (F == Q_Q80 && !TILED) ? 32 : 16;  // metadata bytes of a row
+  static constexpr int kWBytes = (kNibble || kPacked ? kTileRows * 128 : kTileRows * 256) + kHigh;
+  static constexpr int kMeta = F == Q_FP8 ? 0 : (F == Q_Q6K || F == Q_Q80) && !TILED ? 32 : 16;  // metadata bytes of a row
   static constexpr int kAux = F == Q_MLX4 ? 1 : F == Q_Q4K || F == Q_Q5K || F == Q_MLX4F ? 2 : 0;  // K16 steps of the affine term per chunk
   static constexpr bool kLong = F == Q_FP8 || F == Q_MLX4F;  // accumulator blocks of many chunks: nothing is scaled in between
   static constexpr bool kChunk = F == Q_Q4K || F == Q_Q5K;    // a block per pipe and chunk
   static constexpr int kBlk = F == Q_MLX4 ? 64 : F == Q_Q80 ? 32 : F == Q_Q6K ? 16 : 128;  // elements of a block, for the others
-  static constexpr int kSlot = kWBytes + kTileRows * kMeta;
+  static constexpr int kSlot = kWBytes + kTileRows * kMeta + (kPacked && F == Q_Q6K ? kTileRows * 2 : 0);  // (d behind the scales)
   static constexpr float kUnit = F == Q_MLX4 ? 16777216.f : F == Q_MLX4F ? 1.f / 1024.f : F == Q_Q4K || F == Q_Q5K ? 16384.f : 1.f;  // A holds the weights (the nibbles, the scale times the nibble) / kUnit
   // order of the elements inside a K16 step: 0 natural; 1 the nibble order (0 4 1 5 2 6 3 7 of each
   // packed word); 2 the same with the odd elements' activations scaled by 1/16
@@ -524,6 +526,37 @@ __device__ __forceinline__ void convert_unit(const unsigned char* st, int r, int
         tmem_st8(abuf + (2 * u + s2) * 8, regs);
       }
     }
+  } else if (T::kPacked) {
+    uint4 qv[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) qv[u] = *reinterpret_cast<const uint4*>(st + r * 128 + (((u0 + u) ^ (r & 7)) << 4));
+    const uint4 hv = *reinterpret_cast<const uint4*>(st + T::kHighOff + (F == Q_Q6K ? 2 * hh + kq : hh) * 2048 + r * 16);
+    const uint32_t hs[4] = {hv.x, hv.y, hv.z, hv.w};
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const uint32_t ws[4] = {qv[u].x, qv[u].y, qv[u].z, qv[u].w};
+      uint32_t m0 = 0;
+      if (F == Q_Q5K) m0 = kq_scale2(kq_field(head, u0 + u));
+#pragma unroll
+      for (int s2 = 0; s2 < 2; ++s2) {  // the unit's first 16 elements are the low nibbles, the others the high ones
+        uint32_t regs[8];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const int f = (F == Q_Q6K ? 2 * u : 4 * kq + 2 * u) + s2;  // the field in the bits' bytes
+          uint32_t w = (s2 ? ws[t] >> 4 : ws[t]) & 0x0F0F0F0Fu;
+          if (F == Q_Q6K) {
+            w |= (f < 2 ? hs[t] << (4 - 2 * f) : hs[t] >> (2 * f - 4)) & 0x30303030u;
+            regs[2 * t] = sub2(__byte_perm(w, 0x64646464u, 0x4140), 0x64206420u);  // (1024 + q) - 1056
+            regs[2 * t + 1] = sub2(__byte_perm(w, 0x64646464u, 0x4342), 0x64206420u);
+          } else {
+            w |= (f < 4 ? hs[t] << (4 - f) : hs[t] >> (f - 4)) & 0x10101010u;
+            regs[2 * t] = mul2(__byte_perm(w, 0u, 0x4140), m0);
+            regs[2 * t + 1] = mul2(__byte_perm(w, 0u, 0x4342), m0);
+          }
+        }
+        tmem_st8(abuf + (2 * u + s2) * 8, regs);
+      }
+    }
   } else {
     uint4 qv[4];
 #pragma unroll
@@ -532,8 +565,6 @@ __device__ __forceinline__ void convert_unit(const unsigned char* st, int r, int
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const uint32_t ws[4] = {qv[u].x, qv[u].y, qv[u].z, qv[u].w};
-      uint32_t m0 = 0;
-      if (F == Q_Q5K) m0 = kq_scale2(kq_field(head, u0 + (u >> 1)));
       uint32_t regs[8];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
@@ -541,9 +572,6 @@ __device__ __forceinline__ void convert_unit(const unsigned char* st, int r, int
         if (F == Q_FP8) {
           asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(regs[2 * k]) : "h"((unsigned short)(w & 0xFFFFu)));
           asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(regs[2 * k + 1]) : "h"((unsigned short)(w >> 16)));
-        } else if (F == Q_Q5K) {
-          regs[2 * k] = mul2(__byte_perm(w, 0u, 0x4140), m0);
-          regs[2 * k + 1] = mul2(__byte_perm(w, 0u, 0x4342), m0);
         } else {
           if (TILED) w ^= 0x80808080u;  // signed bytes; the streaming layout keeps q + 128
           regs[2 * k] = sub2(__byte_perm(w, 0x64646464u, 0x4140), 0x64806480u);  // (1024 + 128 + q) - 1152
@@ -1027,10 +1055,11 @@ qg_kernel(const __grid_constant__ QArgs a, const __grid_constant__ QMapArgs<TILE
           for (int ci = 0; ci < chunks && ok; ++ci) {
             ok = __all_sync(0xffffffffu, mbar_wait(wfull + 8 * wc.s, wc.ph, a.status, 811));
             if (!ok) break;
-            const unsigned char* mrow = wring + wc.s * T::kSlot + T::kWBytes + r * (F == Q_Q6K && !TILED ? 16 : T::kMeta);
+            const unsigned char* mrow = wring + wc.s * T::kSlot + T::kWBytes + r * (F == Q_Q6K ? 16 : T::kMeta);
             uint4 mv = *reinterpret_cast<const uint4*>(mrow);
             uint32_t m4 = 0;  // Q6_K: d; streaming Q8_0: the fifth pair of scales
-            if (F == Q_Q6K || (F == Q_Q80 && !TILED)) m4 = *reinterpret_cast<const uint32_t*>(F == Q_Q6K && !TILED ? mrow + 2048 - r * 12 : mrow + 16);
+            if (F == Q_Q6K && TILED) m4 = *reinterpret_cast<const unsigned short*>(mrow + 2048 - r * 14);
+            else if (F == Q_Q6K || (F == Q_Q80 && !TILED)) m4 = *reinterpret_cast<const uint32_t*>(F == Q_Q6K ? mrow + 2048 - r * 12 : mrow + 16);
             // the metadata is in registers (the reduction consumes it): the slot is free for the next load
             if (__reduce_or_sync(0xffffffffu, mv.x | mv.y | mv.z | mv.w | m4 | 1u) && lane == 0) mbar_arrive(wempty + 8 * wc.s);
             wc.next(SW);
@@ -1307,7 +1336,8 @@ struct Plan {
   int TT, grid, nfull, ntail, splits;
 };
 
-// The plan with the smallest estimate, in cycles of the busiest SM.  A chunk of an item takes the
+// The plan with the smallest estimate, in cycles of the busiest SM (packed formats are counted as a byte a weight, the
+// conversion of their bits being what a chunk waits for).  A chunk of an item takes the
 // largest of the tensor pipe's time (half a cycle per column and K16 step), the converters' (300
 // cycles a tile) and what the L2 can hand to one SM (45 bytes a cycle); sharing the last items costs two
 // meetings of the cluster and the exchange.  max_chunks: longest K range of an item.  The option mlx_splits asks
@@ -1438,7 +1468,7 @@ int run_rows(const QWeight& w, float* out, const void* x, int batch, QBufs* bufs
     a.nblocks = (rows + NB - 1) / NB;
     a.pmax = pmax;
     const int n = rows >= NB ? NB : (rows + 15) & ~15;  // columns of the first (widest) block
-    if (!choose_plan(w.device, a.ntiles, nchunks, a.nblocks, n, T::kMLX ? 1 : pmax, T::kSlot, NB, NB == 128 ? 32 : 1 << 20, &p))
+    if (!choose_plan(w.device, a.ntiles, nchunks, a.nblocks, n, T::kMLX ? 1 : pmax, T::kPacked ? kTileRows * 288 : T::kSlot, NB, NB == 128 ? 32 : 1 << 20, &p))
       return fail(GOPH_E_UNSUPPORTED, "several-row products: the device holds no CTA of this kernel");
     a.nfull = p.nfull;
     a.ntail = p.ntail;

@@ -101,9 +101,9 @@ int goph_sm_count(int device);
  *                 rows (from 3 to 25, by size) the tensor-core kernel of several rows as well.
  *                 0 (default): tiled for matrices of 8 Mi weights or more, row-major below; 1: always
  *                 row-major; 2: tiled whenever the shape allows
- *   "gguf_layout" the same choice for goph_gguf_upload (Q4_K, Q5_K, Q6_K, Q8_0; in_dim a multiple of 256;
- *                 Q5_K and Q6_K take 1.06 / 1.13 bytes per weight in the tensor-core layout):
- *                 0 (default) tensor-core layout from 8 Mi weights, 1 always the streaming layout,
+ *   "gguf_layout" the same choice for goph_gguf_upload (Q4_K, Q5_K, Q6_K: in_dim a multiple of 256, Q8_0: of 32;
+ *                 Q5_K and Q6_K keep 1.06 / 1.13 bytes per weight in the tensor-core layout, and read 0.69 / 0.82 of them):
+ *                 0 (default) tensor-core layout from 0.5 Mi weights and 256 rows (Q6_K 1.5 Mi), 1 always the streaming layout,
  *                 2 tensor-core layout whenever the shape allows.  "mlx_digits" (few rows) and
  *                 "mlx_splits" apply to these products as well
  *   "fp8_layout"  the same choice for goph_fp8_upload (in_dim a multiple of 256, no NaN codes in the
