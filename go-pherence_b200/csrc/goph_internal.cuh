@@ -119,6 +119,7 @@ struct goph_mlx_weight {
   void* sb;             // [out_dim][groups]
   uint8_t* tiled;       // tiled layout or nullptr
   uint64_t bytes;
+  void* sb_rows;        // row-major, groups % 4 != 0: a copy of the table whose rows are whole 16-byte units (boxes of it are copied)
   goph::QMaps qmaps;    // row-major
 };
 

@@ -1472,6 +1472,7 @@ static int mlx_upload_common(int device, const uint32_t* weight, const float* sc
     if (rc) {
       cudaFree(h->qweight);
       cudaFree(h->sb);
+      cudaFree(h->sb_rows);
       cudaFree(h->tiled);
       delete h;
     }
@@ -1517,7 +1518,18 @@ static int mlx_upload_common(int device, const uint32_t* weight, const float* sc
     h->qweight = nullptr;
     h->sb = nullptr;
   } else if (gs == 64 && h->sb_bf16) {
-    qgemm_maps(Q_MLX4, h->qweight, h->sb, out_dim, in_dim, &h->qmaps);
+    const void* table = h->sb;
+    if (in_dim % 256) {
+      const size_t pitch = (size_t)(in_dim + 255) / 256 * 16;
+      if (cudaMalloc(&h->sb_rows, pitch * out_dim) != cudaSuccess) return cleanup(fail_cuda(cudaGetLastError(), "cudaMalloc(table rows)"));
+      if (cudaMemset(h->sb_rows, 0, pitch * out_dim) != cudaSuccess ||
+          cudaMemcpy2D(h->sb_rows, pitch, h->sb, (size_t)in_dim / 16, (size_t)in_dim / 16, out_dim, cudaMemcpyDeviceToDevice) != cudaSuccess ||
+          cudaDeviceSynchronize() != cudaSuccess)
+        return cleanup(fail_cuda(cudaGetLastError(), "copying table rows"));
+      h->bytes += pitch * out_dim;
+      table = h->sb_rows;
+    }
+    qgemm_maps(Q_MLX4, h->qweight, table, out_dim, in_dim, &h->qmaps);
     if (!mlx_mma_ready(device)) return cleanup(fail(GOPH_E_NOMEM, "cannot allocate the tensor-core path's device scratch"));
   }
   qgemm_weights(device, 1);
@@ -1576,6 +1588,7 @@ GOPH_API int goph_mlx_free(goph_mlx_weight* w) {
   cudaFree(w->qweight);
   cudaFree(w->sb);
   cudaFree(w->tiled);
+  cudaFree(w->sb_rows);
   qgemm_weights(w->device, -1);
   w->magic = 0;
   delete w;

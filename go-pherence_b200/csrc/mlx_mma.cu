@@ -335,7 +335,6 @@ struct RowScales {
 // One weight of a launch.
 struct RowSeg {
   const unsigned char* w;  // tiled: weight blocks [tile][chunk]
-  const uint32_t* sb;      // row-major MLX: the {scale, bias} table
   float* out;              // [batch][out_dim]
   int out_dim, tile0;      // first of its tiles among the launch's
 };
@@ -366,10 +365,9 @@ struct MmaArgs {
 };
 
 // Row-major MLX weights: their tiles come as boxes of 128 rows, 128 bytes of nibbles (whose 128-byte swizzle is the tiled image's) and
-// 16 bytes of the table; zeros past the edges.  A table whose rows are no whole 16-byte units comes by cp.async.
+// 16 bytes of the table; zeros past the edges.
 struct RowMaps {
   CUtensorMap map[kMaxRowSeg][2];
-  int meta_tma;
 };
 struct NoMaps {};
 template <bool TILED>
@@ -377,10 +375,6 @@ using MapArgs = std::conditional_t<TILED, NoMaps, RowMaps>;
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, int bytes) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-}
-
 template <bool G, bool WORK = false>
 struct StageWalkT {
   int w, tile, split, c, c1;
@@ -485,9 +479,7 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
 
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
-      int arrivals = 1;
-      if constexpr (!TILED) arrivals += maps.meta_tma ? 0 : 32;
-      mbar_init(full0 + 8 * s, arrivals);
+      mbar_init(full0 + 8 * s, 1);
       mbar_init(empty0 + 8 * s, kConsumers / KG);
     }
     for (int s = 0; s < 9; ++s) gave_up[s] = 0;
@@ -522,34 +514,22 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
   if (warp == kConsumers) {
     // ------------------------------------------------------------------ producer
     if constexpr (!TILED) {
-      RingCursor rc;
-      int i = 0;
-      for (; sw.live(a) && ok; sw.next_item(a)) {
-        const int k = seg_of(sw.tile), row0 = (sw.tile - a.seg[k].tile0) * kTileRows;
-        for (int c = sw.c; c < sw.c1; ++c, ++i, rc.next(S)) {
-          if (i >= S) ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8 * rc.s, rc.ph ^ 1u, a.status, 1));
-          if (!ok) break;
-          const uint32_t dst = smem_u32(ring + (size_t)rc.s * kStage), meta = dst + F::kStageWBytes, bar = full0 + 8 * rc.s;
-          if (lane == 0) {
-            mbar_expect_tx(bar, F::kStageWBytes + (maps.meta_tma ? kTileRows * 16 : 0));
+      if (lane == 0) {
+        RingCursor rc;
+        int i = 0;
+        for (; sw.live(a) && ok; sw.next_item(a)) {
+          const int k = seg_of(sw.tile), row0 = (sw.tile - a.seg[k].tile0) * kTileRows;
+          for (int c = sw.c; c < sw.c1; ++c, ++i, rc.next(S)) {
+            if (i >= S) ok = mbar_wait(empty0 + 8 * rc.s, rc.ph ^ 1u, a.status, 1);
+            if (!ok) break;
+            const uint32_t dst = smem_u32(ring + (size_t)rc.s * kStage), bar = full0 + 8 * rc.s;
+            mbar_expect_tx(bar, F::kStageBytes);
             tma_load_2d(dst, &maps.map[k][0], c * 128, row0, bar);
-            if (maps.meta_tma) tma_load_2d(meta, &maps.map[k][1], c * 16, row0, bar);
-          }
-          __syncwarp();
-          if (!maps.meta_tma) {
-            const int groups = a.in_dim / 64;
-            const uint32_t* sb = a.seg[k].sb;
-            for (int j = lane; j < 4 * kTileRows; j += 32) {
-              const int r = j >> 2, g = j & 3;
-              const bool in = row0 + r < a.seg[k].out_dim && c * 4 + g < groups;
-              cp_async4(meta + r * 16 + g * 4, in ? sb + (size_t)(row0 + r) * groups + c * 4 + g : sb, in ? 4 : 0);
-            }
-            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+            tma_load_2d(dst + F::kStageWBytes, &maps.map[k][1], c * 16, row0, bar);
           }
         }
+        if (!ok) *gave_up = 1;
       }
-      asm volatile("cp.async.wait_all;" ::: "memory");
-      if (!ok && lane == 0) *gave_up = 1;
     } else if (lane == 0) {
       auto wsrc = [&](const StageWalk& s, int c) {
         const unsigned char* base;
@@ -1278,7 +1258,6 @@ static int launch_impl(const RowWeights& w, MmaArgs a, cudaStream_t stream, Shar
   } else {
     RowMaps maps;
     for (int i = 0; i < w.n; ++i) memcpy(maps.map[i], w.maps[i]->map, sizeof maps.map[i]);
-    maps.meta_tma = w.in_dim % kChunkK == 0;
     GOPH_CUDA(cudaLaunchKernelEx(&cfg, kern, a, maps));
   }
   return GOPH_OK;
@@ -1404,7 +1383,7 @@ int mlx_mma_launch(const goph_mlx_weight* w, float* out, const float* x, int bat
   d.device = w->device;
   d.in_dim = w->in_dim;
   d.n = 1;
-  d.seg[0] = RowSeg{w->tiled, nullptr, out, w->out_dim, 0};
+  d.seg[0] = RowSeg{w->tiled, out, w->out_dim, 0};
   return rows_launch<FMT_MLX4, true>(d, x, batch, digits, stream, shared);
 }
 
@@ -1418,7 +1397,7 @@ int mlx_mma_launch_rows(int n, const goph_mlx_weight* const* ws, float* const* o
     d.n = n - i0 < kMaxRowSeg ? n - i0 : kMaxRowSeg;
     for (int i = 0; i < d.n; ++i) {
       const goph_mlx_weight* w = ws[i0 + i];
-      d.seg[i] = RowSeg{nullptr, static_cast<const uint32_t*>(w->sb), outs[i0 + i], w->out_dim, 0};
+      d.seg[i] = RowSeg{nullptr, outs[i0 + i], w->out_dim, 0};
       d.maps[i] = &w->qmaps;
     }
     if (int rc = rows_launch<FMT_MLX4, false>(d, x, batch, digits, stream, nullptr)) return rc;
@@ -1780,7 +1759,7 @@ int gguf_mma_launch(const goph_gguf_matrix* m, float* out, const float* x, int b
   d.device = m->device;
   d.in_dim = m->in_dim;
   d.n = 1;
-  d.seg[0] = RowSeg{m->tiled, nullptr, out, m->out_dim, 0};
+  d.seg[0] = RowSeg{m->tiled, out, m->out_dim, 0};
   d.unordered = m->unordered;
   if (m->qtype == GOPH_GGUF_Q4_K) return rows_launch<FMT_Q4K, true>(d, x, batch, digits, stream, shared);
   if (m->qtype == GOPH_GGUF_Q5_K) return rows_launch<FMT_Q5K, true>(d, x, batch, digits, stream, shared);
@@ -2052,7 +2031,7 @@ static int launch_noalloc(const goph_mlx_weight* w, float* out, const float* x, 
   d.device = w->device;
   d.in_dim = w->in_dim;
   d.n = 1;
-  d.seg[0] = RowSeg{w->tiled, nullptr, out, w->out_dim, 0};
+  d.seg[0] = RowSeg{w->tiled, out, w->out_dim, 0};
   d.scratch_bytes = kNoAllocBytes - kNaPartOff;
   d.counters = kNoAllocMaxItems * kConsumers;
   SharedX xs;

@@ -150,7 +150,6 @@ struct QArgs {
 // layouts' kernels registers: Q6_K 21504x1536 x256 129 us without, 136 with.)
 struct QRowMaps {
   CUtensorMap map[3];
-  int meta_tma;  // MLX: the table's rows are whole 16-byte units
 };
 struct QNoMaps {};
 template <bool TILED>
@@ -372,12 +371,12 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
 // The row-major and streaming layouts: one chunk of one tile into a slot, by a warp.  Weights come as boxes of 128 rows x
 // 128 bytes, whose 128-byte swizzle is the row image's (16-byte unit u of row r at r * 128 + ((u ^ (r & 7)) << 4)), what
 // stands between or beside them as boxes of 128 rows x 16 bytes; every x is a multiple of 16.  Only the f16 scales of
-// Q6_K and Q8_0 and an MLX table whose rows are no whole 16-byte units come by cp.async.  (One warp's cp.async of
+// Q6_K and Q8_0 come by cp.async (an MLX table whose rows are no whole 16-byte units is copied once, at upload; by cp.async 5018x15424 x8 33.0 us, so 24.1, 3000x4160 x30 15.5 and 13.3).  (One warp's cp.async of
 // everything, 44 to 72 a chunk with their addresses, set the pace: B200, us a call, Q5_K 489x9728 x93 39.6 -> 22.7, Q8_0
 // 11376x1504 x42 28.5 -> 23.3, Q6_K 1024x1792 x29 21.4 -> 11.2, FP8 2816x3136 x5 12.3 -> 9.4, MLX4 5722x1280 x99 16.1 -> 12.8.)
 template <int F>
 __device__ __forceinline__ bool rows_cp(const QRowMaps& t) {  // whether a chunk has a part for cp.async
-  return F == Q_Q6K || F == Q_Q80 || (QF<F, false>::kMLX && !t.meta_tma);
+  return F == Q_Q6K || F == Q_Q80;
 }
 template <int F>
 __device__ __forceinline__ void load_rows(const QArgs& a, const QRowMaps& t, uint32_t slot, uint32_t bar, int tile, int c, int lane) {
@@ -385,11 +384,11 @@ __device__ __forceinline__ void load_rows(const QArgs& a, const QRowMaps& t, uin
   const int row0 = tile * kTileRows;
   const uint32_t meta = slot + T::kWBytes;
   if (lane == 0) {
-    constexpr uint32_t kBytes = T::kWBytes + (F == Q_Q80 || F == Q_FP8 || T::kMLX ? 0 : 2048);
-    mbar_expect_tx(bar, kBytes + (T::kMLX && t.meta_tma ? 2048 : 0));
+    constexpr uint32_t kBytes = T::kWBytes + (F == Q_Q80 || F == Q_FP8 ? 0 : 2048);
+    mbar_expect_tx(bar, kBytes);
     if (T::kMLX) {
       tma_load_2d(slot, &t.map[0], c * 128, row0, bar);
-      if (t.meta_tma) tma_load_2d(meta, &t.map[1], c * 16, row0, bar);
+      tma_load_2d(meta, &t.map[1], c * 16, row0, bar);
     } else if (F == Q_Q4K || F == Q_Q5K) {  // super-blocks {16-byte header, nibbles, Q5_K: fifth bits}
       const int x = c * (F == Q_Q4K ? 144 : 176);
       tma_load_2d(slot, &t.map[0], x + 16, row0, bar);
@@ -409,17 +408,7 @@ __device__ __forceinline__ void load_rows(const QArgs& a, const QRowMaps& t, uin
     }
   }
   __syncwarp();
-  if (T::kMLX) {
-    if (!t.meta_tma) {
-      const int G = a.in_dim / 64;
-      const uint32_t* sb = static_cast<const uint32_t*>(a.aux);
-      for (int i = lane; i < 512; i += 32) {
-        const int r = i >> 2, g = i & 3;
-        const bool ok = row0 + r < a.out_dim && c * 4 + g < G;
-        cp_async4(meta + r * 16 + g * 4, ok ? sb + (size_t)(row0 + r) * G + c * 4 + g : sb, ok ? 4 : 0);
-      }
-    }
-  } else if (F == Q_Q6K) {  // the f16 d, in its aligned pair (the last one of an odd count stands alone)
+  if (F == Q_Q6K) {  // the f16 d, in its aligned pair (the last one of an odd count stands alone)
     const unsigned char* dd = static_cast<const unsigned char*>(a.aux) + (size_t)a.out_dim * a.in_dim / 4 + (size_t)a.out_dim * a.in_dim / 16;
     const size_t total = (size_t)a.out_dim * a.nchunks;
     for (int r = lane; r < 128; r += 32) {
@@ -1447,7 +1436,6 @@ int run_rows(const QWeight& w, float* out, const void* x, int batch, QBufs* bufs
     QMapArgs<TILED> maps;
     if constexpr (!TILED) {
       memcpy(maps.map, w.maps->map, sizeof maps.map);
-      maps.meta_tma = w.in_dim % kChunkK == 0;
     }
     a.w = static_cast<const unsigned char*>(w.w);
     a.aux = w.aux;
@@ -1622,7 +1610,7 @@ void qgemm_maps(int fmt, const void* w, const void* aux, int out_dim, int in_dim
   memset(maps, 0, sizeof *maps);
   switch (fmt) {
     case Q_MLX4: case Q_MLX4F:
-      ok = encode_map(&maps->map[0], w, in / 2, rows, in / 2, 128) && (in % 256 != 0 || encode_map(&maps->map[1], aux, in / 16, rows, in / 16, 16));
+      ok = encode_map(&maps->map[0], w, in / 2, rows, in / 2, 128) && encode_map(&maps->map[1], aux, (in + 255) / 256 * 16, rows, (in + 255) / 256 * 16, 16);
       break;
     case Q_Q4K: case Q_Q5K: {
       const uint64_t row = chunks * (fmt == Q_Q4K ? 144 : 176);

@@ -29,6 +29,7 @@ struct QWeight {
 
 // The tensor maps of a weight in its row-major or streaming layout (w and aux as in QWeight).  maps->ok is false where there
 // are none (no such driver call, rows that are no whole 16-byte units): such a weight is not for this kernel.
+// MLX: aux has rows of whole 16-byte units (in_dim / 64 entries, rounded up to four).
 void qgemm_maps(int fmt, const void* w, const void* aux, int out_dim, int in_dim, QMaps* maps);
 
 // Whether `batch` activation rows of such a weight go to this kernel; the others are the business of the kernels
