@@ -13,6 +13,7 @@
 #include "stream_gemv.cuh"
 #include "qgemm.cuh"
 #include "fp8_mma.cuh"
+#include "mlx_mma.cuh"
 
 namespace goph {
 
@@ -193,6 +194,7 @@ GOPH_API int goph_fp8_upload(int device, const uint8_t* weight, uint64_t weight_
     }
   }
   if (!h->tiled) qgemm_maps(Q_FP8, h->weight, nullptr, out_dim, in_dim, &h->qmaps);
+  if (!mlx_mma_ready(device)) return bail(fail(GOPH_E_NOMEM, "cannot allocate the tensor-core path's device scratch"));
   qgemm_weights(device, 1);
   *out = h;
   return bail(GOPH_OK);
@@ -245,11 +247,21 @@ GOPH_API int goph_fp8_gemm(float* out_dev, uint64_t out_len, const float* x_dev,
                 (unsigned long long)need_x, (unsigned long long)out_len, (unsigned long long)need_o);
   if (int rc = use_device(w->device)) return rc;
   cudaStream_t s = (cudaStream_t)stream;
-  // Several rows: qgemm.cu.  Few rows: in the tensor-core layout the kernel that feeds the e4m3 bytes to the
-  // MMA as they lie (fp8_mma.cu), in the row-major layout the CUDA-core kernels below.
+  // Several rows: qgemm.cu.  Few rows: the kernels that feed the e4m3 bytes to the MMA as they lie (mlx_mma.cu, fp8_mma.cu), in the row-major
+  // layout also the CUDA-core kernels below.
   QBufs* rows;
   if (qgemm_takes(w, x_dev, false, batch, s, &rows)) return fp8_qgemm(w, out_dev, x_dev, false, batch, rows, s);
-  if (w->tiled) return tc_gemm_fp8(w, out_dev, x_dev, false, batch, s);
+  if (w->tiled && (uintptr_t)x_dev % 16) return fail(GOPH_E_INVALID, "x must be 16-byte aligned");
+  // One and two rows (mlx_mma.cu), B200, us a call, before / so: one row 4096x4096 13.5 / 5.9, 8192x28672 47.3 / 40.9, two rows 14336x4096 19.6 / 15.0; three and
+  // four pay for a tile of columns each: 4096x4096 13.8 / 10.1, 14336x4096 19.5 / 22.2.  Row-major: 2048x2048 3.9 / 4.4, 2816x3136 6.1 / 5.1, 512x8192 9.8 / 4.8;
+  // two rows 4.5 / 5.5, 7.4 / 6.3, 10.7 / 6.6.
+  const long size = (long)w->out_dim * w->in_dim;
+  if (w->tiled) {
+    if (batch <= 2 || (size <= 20l << 20 && w->in_dim <= 8192)) return fp8_mma_launch_rows(w, out_dev, x_dev, batch, s);
+    return tc_gemm_fp8(w, out_dev, x_dev, false, batch, s);
+  }
+  if (batch <= 2 && w->qmaps.ok && w->in_dim <= 65536 && options().fp8_rows == 0 && (w->in_dim > 4096 || size >= 6l << 20))
+    return fp8_mma_launch_rows(w, out_dev, x_dev, batch, s);
   if (!w->tiled && w->in_dim % 16 != 0) {
     note_launch();
     fp8_gemv_ragged_kernel<<<(w->out_dim + kGWarps - 1) / kGWarps, kGThreads, 0, s>>>(

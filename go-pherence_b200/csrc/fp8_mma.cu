@@ -697,7 +697,7 @@ __global__ void fp8_dequant_tiled_kernel(const unsigned char* __restrict__ tiled
 
 }  // namespace
 
-// f32 activations: six pieces (an f32 exactly), up to 4 rows; bf16 activations: two pieces, up to 16 rows.
+// f32 activations: six pieces (an f32 exactly), three and four rows (one and two: mlx_mma.cu); bf16 activations: two pieces, up to 16 rows.
 int tc_gemm_fp8(const goph_fp8_linear* w, float* out, const void* x, bool x_bf16, int batch, cudaStream_t stream) {
   if (!w->tiled) return fail(GOPH_E_UNSUPPORTED, "FP8 linear is not in the tensor-core layout");
   if (w->in_dim % kChunkK != 0 || w->in_dim > kMaxIn)
@@ -716,8 +716,7 @@ int tc_gemm_fp8(const goph_fp8_linear* w, float* out, const void* x, bool x_bf16
       else rc = launch_pass<32, 2, 16, true>(w, op, xp, nb = left < 16 ? left : 16, bufs, stream);
     } else {
       // six pieces hold an f32 exactly
-      if (left <= 2) rc = launch_pass<16, 6, 2, false>(w, op, xp, nb = left, bufs, stream);
-      else rc = launch_pass<32, 6, 4, false>(w, op, xp, nb = left < 4 ? left : 4, bufs, stream);
+      rc = launch_pass<32, 6, 4, false>(w, op, xp, nb = left < 4 ? left : 4, bufs, stream);
     }
     if (rc) return rc;
     b0 += nb;

@@ -1,5 +1,5 @@
-// Products of up to eight activation rows with weights in the tiled layouts (MLX 4-bit, Q4_K, Q5_K, Q6_K, Q8_0), in exact
-// integer arithmetic on the tensor cores' register path (mma.sync, kind s8).
+// Products of up to eight activation rows (FP8: four) with weights in the tiled layouts and row-major MLX and FP8 ones, in exact
+// integer arithmetic (FP8: e4m3 pieces, f32) on the tensor cores' register path (mma.sync).
 //
 // Why this path: at B200's HBM rate one SM has to take in 41 nibbles a clock.  Turned into floats on the CUDA cores a nibble
 // costs five to seven lane instructions and an SM has 128 a clock.  Here nibbles stay integers: three logic instructions turn
@@ -64,20 +64,22 @@ constexpr int kChunkK = 256;  // elements of a pipeline stage
 //   Q6K   the same image; two bits beside every nibble: [2 units][row][word t], byte b: unit 0 low, high, unit 1 low, high (the A byte
 //         is nibble and bits at its top, the highest one inverted: 4 (q - 32), signed); 16 int8 scales per row, one per 16
 //         elements; then f16 d [row].
-//   (Both are as large as in the file.  Written out to bytes, 1.06 and 1.13 a weight, they were bound by HBM at 1.5 and 1.4 times the time.)
-enum { FMT_MLX4 = 0, FMT_Q4K = 1, FMT_Q80 = 2, FMT_Q5K = 3, FMT_Q6K = 4 };
+//   FP8   256 e4m3 bytes per row, in Q80's order; no scales (one per row, applied at the end).  Row-major: two images of 128 rows x 128
+//         bytes, 16-byte units XOR-swizzled by row.
+//   (Q5K and Q6K are as large as in the file.  Written out to bytes, 1.06 and 1.13 a weight, they were bound by HBM at 1.5 and 1.4 times the time.)
+enum { FMT_MLX4 = 0, FMT_Q4K = 1, FMT_Q80 = 2, FMT_Q5K = 3, FMT_Q6K = 4, FMT_FP8 = 5 };
 template <int FMT>
 struct Fmt {
-  static constexpr bool kNibble = FMT != FMT_Q80;                     // a nibble image
+  static constexpr bool kNibble = FMT != FMT_Q80 && FMT != FMT_FP8;   // a nibble image
   static constexpr bool kWords = FMT == FMT_MLX4 || FMT == FMT_Q4K;   // whose words hold eight consecutive elements
   static constexpr bool kSigned = FMT == FMT_Q80 || FMT == FMT_Q6K;  // A bytes
   static constexpr bool kSums = FMT == FMT_MLX4 || FMT == FMT_Q4K || FMT == FMT_Q5K;  // biases or minima meet the groups' sums of x
-  static constexpr int kGroup = FMT == FMT_MLX4 ? 64 : 32;  // elements of an entry of the activation tables
+  static constexpr int kGroup = FMT == FMT_FP8 ? 256 : FMT == FMT_MLX4 ? 64 : 32;  // elements of an entry of the activation tables
   static constexpr int kGroups = kChunkK / kGroup;
   static constexpr int kHigh = FMT == FMT_Q5K ? 4096 : FMT == FMT_Q6K ? 8192 : 0;  // bits beside the nibbles
   static constexpr int kHighOff = kTileRows * 128;
   static constexpr int kStageWBytes = kTileRows * (kNibble ? 128 : 256) + kHigh;
-  static constexpr int kMetaRow = 16;                                               // bytes of scales per row and stage
+  static constexpr int kMetaRow = FMT == FMT_FP8 ? 0 : 16;                          // bytes of scales per row and stage
   static constexpr int kDOff = kStageWBytes + kTileRows * kMetaRow;                 // Q6_K: d
   static constexpr int kStageBytes = kDOff + (FMT == FMT_Q6K ? kTileRows * 2 : 0);
 };
@@ -93,10 +95,11 @@ struct Fmt {
 template <int FMT, int MB>
 struct XBlock {
   typedef Fmt<FMT> F;
-  static constexpr int NT = MB == 1 ? 1 : MB / 2;  // n tiles of eight columns
+  static constexpr bool kRowTile = FMT == FMT_FP8;  // a tile of columns per activation row, which has six pieces
+  static constexpr int NT = kRowTile ? MB : MB == 1 ? 1 : MB / 2;  // n tiles of eight columns
   static constexpr int kFrag = NT * 2048;
   static constexpr int kEntry = F::kSums ? 2 : 1;  // floats
-  static constexpr int kTab = MB * 2 * F::kGroups * kEntry;
+  static constexpr int kTab = FMT == FMT_FP8 ? MB * 4 : MB * 2 * F::kGroups * kEntry;
   static constexpr int kBytes = kFrag + kTab * 4;
   static __host__ __device__ __forceinline__ int frag(int step, int n, int t) {
     return ((step >> 1) * NT + (n >> 3)) * 512 + ((n & 7) * 4 + t) * 16 + (step & 1) * 8;
@@ -107,6 +110,8 @@ struct XBlock {
   }
 };
 
+__device__ __forceinline__ float f16_lo(uint32_t w) { return __half2float(__ushort_as_half((unsigned short)(w & 0xFFFFu))); }
+__device__ __forceinline__ float f16_hi(uint32_t w) { return __half2float(__ushort_as_half((unsigned short)(w >> 16))); }
 __device__ __forceinline__ float max_nan(float a, float b) {  // (fmaxf passes over a NaN)
   float d;
   asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
@@ -205,8 +210,56 @@ __device__ __forceinline__ void prep_chunks(const float (&v)[R][8], int lane, un
     }
   }
 }
+// FP8: the chunk is scaled by a power of two so that its largest magnitude lies in [128, 256) and every element written as six e4m3
+// values, each the rounding of what those before it left (exact in f32), the remainder times 2^8 after every second one: an f32
+// exactly, down to 2^-32 of the chunk's largest element.  Column p of the row's tile holds piece p; the table has, per lane of a quad, the scale of
+// its two columns.
+template <int MB>
+__device__ __forceinline__ void prep_fp8(const float (&v)[8], int lane, unsigned char* xb, int m) {
+  typedef XBlock<FMT_FP8, MB> X;
+  float mx = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) mx = max_nan(mx, fabsf(v[i]));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = max_nan(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  int e = (int)((__float_as_uint(mx) >> 23) & 0xFF) - 127;
+  const bool finite = e < 128;
+  if (e < -110) e = -110;
+  if (e > 127) e = 127;
+  const float s = __uint_as_float((uint32_t)(7 - e + 127) << 23);
+  if (lane < 3) reinterpret_cast<float*>(xb + X::kFrag)[m * 4 + lane] = finite ? __uint_as_float((uint32_t)(e - 7 - 8 * lane + 127) << 23) : __uint_as_float(0x7FC00000u);
+  float r[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) r[i] = v[i] * s;
+  const int step = lane >> 2, w = lane & 3;
+#pragma unroll
+  for (int p = 0; p < 6; ++p) {
+    uint32_t h[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      unsigned short b;
+      asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(b) : "f"(r[2 * i + 1]), "f"(r[2 * i]));
+      uint32_t f;
+      asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(f) : "h"(b));
+      r[2 * i] -= f16_lo(f);
+      r[2 * i + 1] -= f16_hi(f);
+      h[i] = b;
+    }
+    if (p & 1) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) r[i] *= 256.f;
+    }
+    const int n = m * 8 + p;
+    *reinterpret_cast<uint32_t*>(xb + X::frag(step, n, 2 * (w & 1)) + 4 * (w >> 1)) = h[0] | (h[1] << 16);
+    *reinterpret_cast<uint32_t*>(xb + X::frag(step, n, 2 * (w & 1) + 1) + 4 * (w >> 1)) = h[2] | (h[3] << 16);
+  }
+}
 template <int FMT, int MB, int SPLIT = 1>
 __device__ __forceinline__ void prep_chunk(const float (&v)[8], int lane, unsigned char* xb, int m, int digits) {
+  if constexpr (FMT == FMT_FP8) {
+    prep_fp8<MB>(v, lane, xb, m);
+    return;
+  }
   unsigned char* const xbs[1] = {xb};
   const int ms[1] = {m};
   prep_chunks<FMT, MB, SPLIT, 1>(reinterpret_cast<const float(&)[1][8]>(v), lane, xbs, ms, digits);
@@ -230,6 +283,12 @@ mlx_prep_x_kernel(const float* __restrict__ x, unsigned char* __restrict__ xb, i
   pdl_launch_dependents();
   pdl_wait();  // x may be the output of the kernel in front
   float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // (past the row)
+  if constexpr (FMT == FMT_FP8) {  // (a block of one warp)
+    const int k = c * kChunkK + lane * 8;
+    if (k < in_dim) load_eight(x + (size_t)m * in_dim + k, v);
+    prep_fp8<MB>(v, lane, xb + (size_t)c * XBlock<FMT, MB>::kBytes, m);
+    return;
+  }
   const int k = c * kChunkK + lane / 4 * 8;
   if (k < in_dim) load_eight(x + (size_t)m * in_dim + k, v);
   prep_chunk<FMT, MB, 4>(v, lane, xb + (size_t)c * XBlock<FMT, MB>::kBytes, m, digits);
@@ -255,14 +314,17 @@ __device__ __forceinline__ void imma16(int (&d)[4], uint32_t a0, uint32_t a1, ui
   asm("mma.sync.aligned.m16n8k16.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
       : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a0), "r"(a1), "r"(b0), "r"(c));
 }
+// D = A * B + D, 16 x 8 x 32, e4m3, f32 (an MMA's error is that of f32: 3e-7 of its largest term at most, measured).
+__device__ __forceinline__ void qmma32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k32.row.col.f32.e4m3.e4m3.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
 // The accumulators start at 1.5 * 2^23 as a float's bits, so that an integer sum v below 2^22 in magnitude comes out as the
 // float 1.5 * 2^23 + v, without a conversion; two digits' sums then meet exactly (both terms are multiples of 128 or below 2^24).
 constexpr int kAcc0 = 0x4B400000;
 constexpr float kAcc0F = 12582912.f;
 __device__ __forceinline__ float digits_sum(int lo, int hi) { return fmaf(__int_as_float(hi), 128.f, -129.f * kAcc0F) + __int_as_float(lo); }
 
-__device__ __forceinline__ float f16_lo(uint32_t w) { return __half2float(__ushort_as_half((unsigned short)(w & 0xFFFFu))); }
-__device__ __forceinline__ float f16_hi(uint32_t w) { return __half2float(__ushort_as_half((unsigned short)(w >> 16))); }
 
 // The scales of a chunk's rows.  K-quants pack them in six bits or multiply them by the super-block's d.  fma(2^23 + field, d,
 // -2^23 d) is the product field * d rounded once, as the reference's dequantisation does.  With one row of x a lane finishes half
@@ -337,6 +399,7 @@ struct RowSeg {
   const unsigned char* w;  // tiled: weight blocks [tile][chunk]
   float* out;              // [batch][out_dim]
   int out_dim, tile0;      // first of its tiles among the launch's
+  const float *scale, *bias;  // FP8: [out_dim]; [out_dim] or nullptr
 };
 constexpr int kMaxRowSeg = 4;
 
@@ -364,8 +427,8 @@ struct MmaArgs {
   size_t gxb;
 };
 
-// Row-major MLX weights: their tiles come as boxes of 128 rows, 128 bytes of nibbles (whose 128-byte swizzle is the tiled image's) and
-// 16 bytes of the table; zeros past the edges.
+// Row-major weights: their tiles come as boxes of 128 rows, 128 bytes of nibbles (whose 128-byte swizzle is the tiled image's) and
+// 16 bytes of the table, or twice 128 bytes (FP8); zeros past the edges.
 struct RowMaps {
   CUtensorMap map[kMaxRowSeg][2];
 };
@@ -426,7 +489,7 @@ struct RowCfg {
   #ifdef RM_SL2
   static constexpr int SL = 2, KG = SL;
 #else
-  static constexpr int SL = MB >= 4 || G ? 2 : 1, KG = SL;
+  static constexpr int SL = (FMT != FMT_FP8 && MB >= 4) || G ? 2 : 1, KG = SL;  // (FP8: a tile of sums for every activation row is registers enough)
 #endif
   static constexpr int NT = XBlock<FMT, MB>::NT;
   static constexpr int kVals = SL * NT;                      // values a lane has of an item
@@ -455,7 +518,7 @@ template <int FMT, int MB, bool FUSED, bool G = false, bool TILED = true>
 __global__ void __launch_bounds__(kThreads, 2)
 mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArgs<TILED> maps) {
   static_assert(!G || !FUSED, "grouped launches: activations prepared in front");
-  static_assert(TILED || (FMT == FMT_MLX4 && FUSED), "row-major: MLX, activations by the CTAs themselves");
+  static_assert(TILED || ((FMT == FMT_MLX4 || FMT == FMT_FP8) && FUSED), "row-major: MLX and FP8, activations by the CTAs themselves");
   constexpr bool kWork = G && FMT != FMT_MLX4;  // a work list's entries (MmaWorkEntry)
   typedef StageWalkT<G, kWork> StageWalk;
   typedef Fmt<FMT> F;
@@ -501,6 +564,11 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
     return kWork ? &reinterpret_cast<const MmaWorkEntry*>(a.gwork)[e].g : a.gwork + e;
   };
   const int cbase = sw.live(a) ? sw.c : 0;  // first chunk of this CTA's K range
+  auto finish = [&](int k, int r, float v) {
+    if (FMT != FMT_FP8) return v;
+    const float* bias = a.seg[k].bias;
+    return fmaf(v, __ldg(a.seg[k].scale + r), bias ? __ldg(bias + r) : 0.f);
+  };
   auto seg_of = [&](int tile) {
     int k = 0;
 #pragma unroll
@@ -524,8 +592,13 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
             if (!ok) break;
             const uint32_t dst = smem_u32(ring + (size_t)rc.s * kStage), bar = full0 + 8 * rc.s;
             mbar_expect_tx(bar, F::kStageBytes);
-            tma_load_2d(dst, &maps.map[k][0], c * 128, row0, bar);
-            tma_load_2d(dst + F::kStageWBytes, &maps.map[k][1], c * 16, row0, bar);
+            if (FMT == FMT_FP8) {
+              tma_load_2d(dst, &maps.map[k][0], c * 256, row0, bar);
+              tma_load_2d(dst + 16384, &maps.map[k][0], c * 256 + 128, row0, bar);
+            } else {
+              tma_load_2d(dst, &maps.map[k][0], c * 128, row0, bar);
+              tma_load_2d(dst + F::kStageWBytes, &maps.map[k][1], c * 16, row0, bar);
+            }
           }
         }
         if (!ok) *gave_up = 1;
@@ -612,9 +685,9 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
     // shared-memory addresses that stay: of the lane's rows in an ldmatrix (nibbles: two K steps of 16 rows; bytes: one), and
     // of its part of the fragments and tables
     const int mi = lane >> 3, lr = lane & 7;
-    const uint32_t a_lane = F::kNibble ? (row0 + (mi & 1) * 8 + lr) * 128 : (mi >> 1) * 2048 + (row0 / 8 + (mi & 1)) * 128 + lr * 16;
+    const uint32_t a_lane = F::kNibble || !TILED ? (row0 + (mi & 1) * 8 + lr) * 128 : (mi >> 1) * 2048 + (row0 / 8 + (mi & 1)) * 128 + lr * 16;
     const uint32_t b_lane = lane * 16;
-    const int t_lane = X::kFrag + 4 * (MB > 1 ? X::entry(half, p, 0) : X::entry(0, p, FMT == FMT_Q6K ? 0 : half));
+    const int t_lane = X::kFrag + 4 * (FMT == FMT_FP8 ? t : MB > 1 ? X::entry(half, p, 0) : X::entry(0, p, FMT == FMT_Q6K ? 0 : half));
     unsigned char* sc_warp = scales + warp * (SL * 16 * kStagedRow);
     float gate[kWork ? C::kVals : 1];
     int cur_entry = -1, nb = a.batch;
@@ -626,6 +699,7 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
       for (int sl = 0; sl < SL; ++sl)
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) acc[sl][nt][0] = acc[sl][nt][1] = 0.f;
+      float lost[FMT == FMT_FP8 ? SL : 1][FMT == FMT_FP8 ? NT : 1][2] = {};
 #pragma unroll 1
       for (int c = sw.c; c < sw.c1; ++c, ++i, rc.next(S)) {
         if (KG == 2 && (i & 1) != grp) continue;
@@ -702,9 +776,12 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
                 af[sl][k][2] = (q[2 * k] >> 4) & 0x0F0F0F0Fu;
                 af[sl][k][3] = (q[2 * k + 1] >> 4) & 0x0F0F0F0Fu;
               }
-            } else {
+            } else if (TILED) {
               ldsm4(st_a + sl * 256 + (2 * j) * 4096, af[sl][0]);
               ldsm4(st_a + sl * 256 + (2 * j + 1) * 4096, af[sl][1]);
+            } else {
+#pragma unroll
+              for (int k = 0; k < 2; ++k) ldsm4(st_a + sl * 2048 + (j >> 1) * 16384 + (((2 * ((2 * j + k) & 3) + (mi >> 1)) ^ lr) << 4), af[sl][k]);
             }
           }
         };
@@ -723,7 +800,44 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
           if (F::kSums) return *reinterpret_cast<const float2*>(xt + at * 8);
           return make_float2(*reinterpret_cast<const float*>(xt + at * 4), 0.f);
         };
-        if constexpr (FMT == FMT_MLX4) {
+        if constexpr (FMT == FMT_FP8) {
+          // A sum of 128 elements leaves the tensor core, which cuts f32 sums off, before it gets long, and is added with what the sums before
+          // it lost (2-norm of the error against 64 bits, 4096 elements, normal x / of bf16 values: 256 elements in one chain 7.6e-8 / 6.9e-8,
+          // so 7.3e-8 / 6.3e-8; the kernel that kept whole rows in tensor memory 6.8e-8 / 7.0e-8; 8192 elements 7.5e-8 / 7.0e-8 and 7.8e-8 / 7.8e-8).
+#pragma unroll
+          for (int hh = 0; hh < 2; ++hh) {
+            float d[SL][NT][4];
+#pragma unroll
+            for (int sl = 0; sl < SL; ++sl)
+#pragma unroll
+              for (int nt = 0; nt < NT; ++nt) d[sl][nt][0] = d[sl][nt][1] = d[sl][nt][2] = d[sl][nt][3] = 0.f;
+#pragma unroll
+            for (int j = 2 * hh; j < 2 * hh + 2; ++j) {
+              load_a(j);
+#pragma unroll
+              for (int nt = 0; nt < NT; ++nt) {
+                const uint4 b = frag(j, nt);
+#pragma unroll
+                for (int sl = 0; sl < SL; ++sl) {
+                  qmma32(d[sl][nt], af[sl][0], b.x, b.y);
+                  qmma32(d[sl][nt], af[sl][1], b.z, b.w);
+                }
+              }
+            }
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+              const float xs = *reinterpret_cast<const float*>(xt + nt * 16);
+#pragma unroll
+              for (int sl = 0; sl < SL; ++sl)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                  const float y = fmaf(d[sl][nt][2 * r] + d[sl][nt][2 * r + 1], xs, -lost[sl][nt][r]), sum = acc[sl][nt][r] + y;
+                  lost[sl][nt][r] = (sum - acc[sl][nt][r]) - y;
+                  acc[sl][nt][r] = sum;
+                }
+            }
+          }
+        } else if constexpr (FMT == FMT_MLX4) {
           if constexpr (MB == 1) {
 #pragma unroll
             for (int jj = 0; jj < 2; ++jj) {
@@ -897,10 +1011,15 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
           float v0 = acc[sl][nt][0], v1 = acc[sl][nt][1];
+          if (X::kRowTile) {  // the small pieces meet first, and lanes 0 and 1 have the sum: one rounding of its size
+            if (t == 3) v0 = v1 = 0.f;  // (columns without a piece)
+            v0 += __shfl_xor_sync(0xffffffffu, v0, 3);
+            v1 += __shfl_xor_sync(0xffffffffu, v1, 3);
+          }
           v0 += __shfl_xor_sync(0xffffffffu, v0, 1);
           v1 += __shfl_xor_sync(0xffffffffu, v1, 1);
           float v = p ? v1 : v0;
-          if (MB == 1) v += __shfl_xor_sync(0xffffffffu, v, 2);
+          if (MB == 1 && !X::kRowTile) v += __shfl_xor_sync(0xffffffffu, v, 2);
           fin[sl * NT + nt] = v;
         }
       }
@@ -925,8 +1044,8 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
       const int row = (sw.tile - (G ? 0 : a.seg[sg].tile0)) * kTileRows + row0 + g + 8 * p;  // of the first slab
       float* const out = a.seg[sg].out;
       const int out_dim = a.seg[sg].out_dim;
-      auto act = [&](int k) { return MB == 1 ? 0 : 2 * (k % NT) + half; };
-      const bool mine = MB > 1 || t < 2;
+      auto act = [&](int k) { return MB == 1 ? 0 : X::kRowTile ? k % NT : 2 * (k % NT) + half; };
+      const bool mine = t < 2 || (MB > 1 && !X::kRowTile);
       if (G) {
         if (sw.entry != cur_entry) {
           cur_entry = sw.entry;
@@ -961,7 +1080,7 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
 #pragma unroll
         for (int k = 0; k < C::kVals; ++k) {
           const int m = act(k), r = row + 16 * (k / NT);
-          if (mine && m < a.batch && r < out_dim) out[(size_t)m * out_dim + r] = fin[k];
+          if (mine && m < a.batch && r < out_dim) out[(size_t)m * out_dim + r] = finish(sg, r, fin[k]);
         }
       } else {
         // Partial sums of this K range go to scratch; the warp that arrives last at its rows of the tile adds the
@@ -983,7 +1102,7 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
             float sum = 0.f;
             for (int s2 = 0; s2 < a.splits; ++s2) sum += __ldcg(base + (size_t)s2 * (C::kStoring * kPart) + k * 32);
             const int m = act(k), r = row + 16 * (k / NT);
-            if (mine && m < a.batch && r < out_dim) out[(size_t)m * out_dim + r] = sum;
+            if (mine && m < a.batch && r < out_dim) out[(size_t)m * out_dim + r] = finish(sg, r, sum);
           }
           if (lane == 0) a.counters[sw.tile * kConsumers + slot] = 0;
         }
@@ -1012,8 +1131,8 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
           for (int k = 0; k < C::kVals; ++k) {
             float sum = fin[k];
             for (int s2 = 1; s2 < a.splits; ++s2) sum += recv[(size_t)(s2 - 1) * (C::kRecv / 4) + slot * (C::kVals * 32) + k * 32 + lane];
-            const int m = MB == 1 ? 0 : 2 * (k % NT) + half, r = row + 16 * (k / NT);
-            if ((MB > 1 || t < 2) && m < a.batch && r < out_dim) out[(size_t)m * out_dim + r] = sum;
+            const int m = MB == 1 ? 0 : X::kRowTile ? k % NT : 2 * (k % NT) + half, r = row + 16 * (k / NT);
+            if ((t < 2 || (MB > 1 && !X::kRowTile)) && m < a.batch && r < out_dim) out[(size_t)m * out_dim + r] = finish(sg, r, sum);
           }
         }
       }
@@ -1097,6 +1216,7 @@ constexpr size_t kMaxCounters = 4096 * kConsumers;
 // Prepared activations: up to 8 rows of up to 65536 elements.
 constexpr int kMaxPrepIn = 65536;  // mlx_mma_supported's bound on in_dim
 constexpr size_t kPrepXbBytes = (size_t)(kMaxPrepIn / kChunkK) * XBlock<FMT_Q4K, 8>::kBytes;
+static_assert(XBlock<FMT_FP8, 4>::kBytes <= XBlock<FMT_Q4K, 8>::kBytes, "the widest activations");
 
 // The buffers of a device are allocated on first use.  Nothing is published until every
 // allocation has succeeded (a failure frees what it got and the next call tries again), and
@@ -1220,7 +1340,7 @@ static int launch_impl(const RowWeights& w, MmaArgs a, cudaStream_t stream, Shar
   if (!FUSED && !xs->prepared) {
     // activations -> digits, sums and scales, once per launch
     cfg.gridDim = dim3(a.batch * a.nchunks);
-    cfg.blockDim = dim3(128);
+    cfg.blockDim = dim3(FMT == FMT_FP8 ? 32 : 128);
     note_launch();
     GOPH_CUDA(cudaLaunchKernelEx(&cfg, mlx_prep_x_kernel<FMT, MB>, a.x, const_cast<unsigned char*>(a.xb), a.in_dim, a.digits));
     xs->prepared = true;
@@ -1337,10 +1457,11 @@ static int rows_slice(const RowWeights& w0, MmaArgs a, cudaStream_t stream, Shar
     a.seg[i].tile0 = a.ntiles;
     a.ntiles += (w.seg[i].out_dim + kTileRows - 1) / kTileRows;
   }
-  for (int nb = a.batch < 8 ? a.batch : 8; nb > 0; nb = nb > 4 ? 4 : nb > 2 ? 2 : nb - 1) {
+  constexpr int kMost = FMT == FMT_FP8 ? 4 : 8;
+  for (int nb = a.batch < kMost ? a.batch : kMost; nb > 0; nb = nb > 4 ? 4 : nb > 2 ? 2 : nb - 1) {
     a.batch = nb;
     const int rc = nb == 1 ? launch_one<FMT, 1, TILED>(w, a, stream, xs) : nb == 2 ? launch_one<FMT, 2, TILED>(w, a, stream, xs)
-                 : nb <= 4 ? launch_one<FMT, 4, TILED>(w, a, stream, xs) : launch_one<FMT, 8, TILED>(w, a, stream, xs);
+                 : nb <= 4 ? launch_one<FMT, 4, TILED>(w, a, stream, xs) : launch_one<FMT, kMost, TILED>(w, a, stream, xs);
     if (rc == kDoesNotFit) continue;
     if (taken) *taken = nb;
     return rc;
@@ -1385,6 +1506,16 @@ int mlx_mma_launch(const goph_mlx_weight* w, float* out, const float* x, int bat
   d.n = 1;
   d.seg[0] = RowSeg{w->tiled, out, w->out_dim, 0};
   return rows_launch<FMT_MLX4, true>(d, x, batch, digits, stream, shared);
+}
+
+int fp8_mma_launch_rows(const goph_fp8_linear* w, float* out, const float* x, int batch, cudaStream_t stream) {
+  RowWeights d;
+  d.device = w->device;
+  d.in_dim = w->in_dim;
+  d.n = 1;
+  d.seg[0] = RowSeg{w->tiled, out, w->out_dim, 0, w->scale, w->bias};
+  d.maps[0] = &w->qmaps;
+  return w->tiled ? rows_launch<FMT_FP8, true>(d, x, batch, 4, stream, nullptr) : rows_launch<FMT_FP8, false>(d, x, batch, 4, stream, nullptr);
 }
 
 bool mlx_mma_ready(int device) { return device_bufs(device) != nullptr; }

@@ -35,6 +35,8 @@ int mlx_mma_launch(const goph_mlx_weight* w, float* out, const float* x, int bat
 // (mlx_mma_rows_ok).  No scratch: callers need no order between such calls.
 inline bool mlx_mma_rows_ok(const goph_mlx_weight* w) { return !w->tiled && w->group_size == 64 && w->sb_bf16 && w->qmaps.ok && w->in_dim <= 65536; }
 int mlx_mma_launch_rows(int n, const goph_mlx_weight* const* ws, float* const* outs, const float* x, int batch, int digits, cudaStream_t stream);
+// FP8 linears of either layout (row-major: with tensor maps), f32 activations; row-major: no scratch.
+int fp8_mma_launch_rows(const goph_fp8_linear* w, float* out, const float* x, int batch, cudaStream_t stream);
 // Allocates the device's scratch (uploads do, so that no product of a weight that may be used under capture has to).
 bool mlx_mma_ready(int device);
 
