@@ -1327,18 +1327,18 @@ struct Plan {
 
 // The plan with the smallest estimate, in cycles of the busiest SM (packed formats are counted as a byte a weight, the
 // conversion of their bits being what a chunk waits for).  A chunk of an item takes the
-// largest of the tensor pipe's time (half a cycle per column and K16 step), the converters' (300
-// cycles a tile) and what the L2 can hand to one SM (45 bytes a cycle); sharing the last items costs two
+// largest of the tensor pipe's time (half a cycle per column and K16 step), the converters' and the
+// hand-overs' (tile_cycles) and what the L2 can hand to one SM (45 bytes a cycle); sharing the last items costs two
 // meetings of the cluster and the exchange.  max_chunks: longest K range of an item.  The option mlx_splits asks
 // for a number of CTAs per shared item, as far as there is a plan with that many.
-bool choose_plan(int device, int ntiles, int nchunks, int nblocks, int n, int pieces, int wbytes, int NB, int max_chunks, Plan* best) {
+bool choose_plan(int device, int ntiles, int nchunks, int nblocks, int n, int pieces, int wbytes, double tile_cycles, int NB, int max_chunks, Plan* best) {
   double best_cost = -1;
   int want = options().mlx_splits < kMaxSplits ? options().mlx_splits : kMaxSplits;
   if (want > nchunks) want = nchunks;
   for (int TT = NB == 128 ? 2 : 1; TT <= 2; ++TT) {
     if (TT == 2 && ntiles < 2) break;
     const int items = (ntiles + TT - 1) / TT * nblocks;
-    const double mma = TT * 8.0 * pieces * n, conv = 300.0 * TT, mem = (TT * (double)wbytes + pieces * n * 512.0) / 45;
+    const double mma = TT * 8.0 * pieces * n, conv = tile_cycles * TT, mem = (TT * (double)wbytes + pieces * n * 512.0) / 45;
     const double chunk = mma > conv ? (mma > mem ? mma : mem) : (conv > mem ? conv : mem);
     for (int S = 1; S <= kMaxSplits && S <= nchunks; ++S) {
       if (S > 1 && !options().mlx_cluster) break;
@@ -1357,6 +1357,21 @@ bool choose_plan(int device, int ntiles, int nchunks, int nblocks, int n, int pi
     }
   }
   return best_cost >= 0;
+}
+
+// What a chunk of one tile costs where its conversion and the hand-overs of its accumulator blocks set the pace (28672x4096, 16 and 64 rows).  With
+// 300 for every format the plan took two tiles an item, and fewer items than SMs, where one was better (B200, us a call): Q8_0 6000x2048 x200 43.4 ->
+// 36.5, 12000x1024 x30 14.6 -> 12.8, Q6_K 20000x1024 x64 39.1 -> 29.7, Q4_K 4096x14336 x20 28.7 -> 26.1, Q5_K 20000x1536 x12 19.5 -> 17.1.  Full blocks of
+// columns of Q4_K and Q5_K keep it: there the B tiles, which two tiles of an item share, count for more than the estimate has (Q4_K 14336x4096 x64 29.7, with
+// one tile 35.6; Q4_K 3584x18944 x11 28.0 and 30.4).  MLX with foldable scales and FP8 close a block in 16 chunks and wait for the L2 or the tensor cores.
+template <int F>
+double tile_cycles(int n) {
+  const double more = (n - 16) / 48.0;  // of 64 columns
+  if (F == Q_Q80) return 3100 + 1500 * more;
+  if (F == Q_Q6K) return 5500 + 2100 * more;
+  if (F == Q_Q4K && n > 16 && n < 64) return 1700 + 800 * more;
+  if (F == Q_Q5K && n < 64) return 2000 + 1000 * more;
+  return 300;
 }
 
 template <int F, bool TILED, int TT, int NB>
@@ -1424,7 +1439,7 @@ int run_rows(const QWeight& w, float* out, const void* x, int batch, QBufs* bufs
     Plan p;
     if (NB == 128) {
       const int rows = batch - b0 < kMaxRows ? batch - b0 : kMaxRows;
-      if (!choose_plan(w.device, (w.out_dim + kTileRows - 1) / kTileRows, nchunks, (rows + 127) / 128, rows < 128 ? (rows + 15) & ~15 : 128, 1, T::kSlot, NB, 32, &p))
+      if (!choose_plan(w.device, (w.out_dim + kTileRows - 1) / kTileRows, nchunks, (rows + 127) / 128, rows < 128 ? (rows + 15) & ~15 : 128, 1, T::kSlot, 300, NB, 32, &p))
         NB = 64;
     }
     const size_t block_bytes = (size_t)NB * nchunks * kChunkK * 2 * pmax;
@@ -1456,7 +1471,7 @@ int run_rows(const QWeight& w, float* out, const void* x, int batch, QBufs* bufs
     a.nblocks = (rows + NB - 1) / NB;
     a.pmax = pmax;
     const int n = rows >= NB ? NB : (rows + 15) & ~15;  // columns of the first (widest) block
-    if (!choose_plan(w.device, a.ntiles, nchunks, a.nblocks, n, T::kMLX ? 1 : pmax, T::kPacked ? kTileRows * 288 : T::kSlot, NB, NB == 128 ? 32 : 1 << 20, &p))
+    if (!choose_plan(w.device, a.ntiles, nchunks, a.nblocks, n, T::kMLX ? 1 : pmax, T::kPacked ? kTileRows * 288 : T::kSlot, tile_cycles<F>(n), NB, NB == 128 ? 32 : 1 << 20, &p))
       return fail(GOPH_E_UNSUPPORTED, "several-row products: the device holds no CTA of this kernel");
     a.nfull = p.nfull;
     a.ntail = p.ntail;
