@@ -1,0 +1,146 @@
+"""GPU parity at the edges of the few-row products (one to eight activation rows: exact integer or e4m3 MMAs, tiles of 128 rows,
+stages of 256 elements, K ranges cut over clusters of up to sixteen), against the oracle's dequantised weights in double precision."""
+import numpy as np
+import pytest
+
+from gpu_util import F, out_with_canary, read_and_check_canary
+from test_gpu_rows import make
+
+pytestmark = pytest.mark.gpu
+
+# (out_dim, in_dim): one tile and stage; a row and a stage more; rows cut eight- and sixteenfold; a tile for every SM and one more
+SHAPES = ((128, 256), (129, 512), (640, 2816), (200, 16384), (19072, 512))
+# rows that end inside a stage
+RAGGED = {"mlx": ((1, 64), (130, 320), (640, 2112), (200, 12352)), "q8_0": ((1, 32), (129, 288), (640, 2080)), "fp8": ((1, 16), (129, 272), (640, 2064), (300, 8208))}
+
+
+def _norm_err(got, want):
+    return np.linalg.norm(got - want) / np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("fmt,tiled", [("mlx", True), ("mlx_wide", True), ("mlx", False), ("mlx_wide", False), ("q4_k", True), ("q5_k", True), ("q6_k", True),
+                                       ("q8_0", True), ("fp8", True), ("fp8", False)])
+def test_few_rows(gpu, pkg, fmt, tiled):
+    """The 2-norm of the error over that of the result.  An element of x is held to 2^-27 of its group's (FP8: exactly, to 2^-32 of its chunk's) largest, dot products of
+    a group are exact, and f32 sums of at most 512 terms (16384 elements, 32 a group) add 2^-24 of a partial sum each: 3e-7 for sums that
+    grow like a walk, three times that where minima and biases cancel most of the products.  Without the lowest digit it were 1.6e-6."""
+    kind = fmt.split("_w")[0]
+    shapes = (() if not tiled and kind == "q8_0" else SHAPES) + (RAGGED.get(kind, ()) if not tiled or kind == "q8_0" else ())
+    for out_dim, in_dim in shapes:
+        h, run, W, bias = make(gpu, pkg, fmt, tiled, out_dim, in_dim)
+        W = np.asarray(W, dtype=np.float64).reshape(out_dim, in_dim)
+        ok = ~np.isnan(W).any(1)
+        for rows in (1, 2, 3, 4, 5, 8):
+            x = pkg.synth.activations(("few", rows, in_dim), rows * in_dim, bf16=False).reshape(rows, in_dim)
+            x[rows // 2] *= F(2.0 ** 40)  # every row has its own scale
+            if rows > 2:
+                x[0] = 0
+            xo, out = gpu.from_numpy(x.reshape(-1)), out_with_canary(gpu, rows * out_dim)
+            run(out, xo, rows)
+            gpu.Sync()
+            got = read_and_check_canary(out, rows * out_dim).reshape(rows, out_dim).astype(np.float64)
+            want = x.astype(np.float64) @ W.T + (0 if bias is None else bias)
+            assert np.isnan(got[:, ~ok]).all() and not np.isnan(got[:, ok]).any()
+            bound = 3e-6 if kind in ("fp8", "mlx") and rows > 4 else 1e-6  # (the several-row kernel: f32 sums of 4096 elements in tensor memory, 1.5e-6 measured)
+            for m in range(rows):
+                # (a matrix of one row has a single output, which may cancel to nothing: against its terms)
+                size = np.linalg.norm(want[m, ok]) if ok.sum() > 100 else np.linalg.norm(np.abs(x[m].astype(np.float64)) @ np.abs(W[ok]).T)
+                assert np.linalg.norm(got[m, ok] - want[m, ok]) <= bound * size, (out_dim, in_dim, rows, m)
+            xo.Free(); out.Free()
+        h.Free()
+    assert gpu.KernelStatus() == 0
+
+
+@pytest.mark.parametrize("fmt,tiled", [("mlx", False), ("fp8", True), ("fp8", False)])
+def test_a_row_that_is_not_finite_is_nan(gpu, pkg, fmt, tiled):
+    """As the tiled integer products: the row is NaN throughout, and no other row knows of it.  (Row-major FP8 widths from 4096 on.)"""
+    out_dim, in_dim = 200, 4352
+    h, run, W, _ = make(gpu, pkg, fmt, tiled, out_dim, in_dim)
+    ok = ~np.isnan(np.asarray(W).reshape(out_dim, in_dim)).any(1)
+    x = pkg.synth.activations(("odd", fmt), 2 * in_dim, bf16=False).reshape(2, in_dim)
+    got = []
+    for k, bad in ((0, 1.0), (0, np.nan), (517, np.inf), (in_dim - 1, -np.inf)):
+        y = x.copy()
+        y[1, k] = bad
+        xo, out = gpu.from_numpy(y.reshape(-1)), out_with_canary(gpu, 2 * out_dim)
+        run(out, xo, 2)
+        gpu.Sync()
+        got.append(read_and_check_canary(out, 2 * out_dim).reshape(2, out_dim).copy())
+        xo.Free(); out.Free()
+    assert np.isfinite(got[0][:, ok]).all()
+    for g in got[1:]:
+        assert np.isnan(g[1]).all() and np.array_equal(g[0, ok].view(np.uint32), got[0][0, ok].view(np.uint32))
+    h.Free()
+
+
+@pytest.mark.parametrize("rows", [2, 4, 8])
+def test_row_major_weights_of_one_call_share_a_launch(gpu, pkg, rows):
+    """Up to four weights a launch, the bits of separate calls; tiles of several weights in one K cut (short, long and ragged rows)."""
+    for in_dim in (512, 2112, 9216):
+        hs = [make(gpu, pkg, fmt, False, o, in_dim)[0] for fmt, o in (("mlx", 300), ("mlx_wide", 1), ("mlx", 128), ("mlx", 129), ("mlx", 64))]
+        x = gpu.from_numpy(pkg.synth.activations(("share", in_dim), rows * in_dim, bf16=False))
+        one, both = ([out_with_canary(gpu, rows * h.OutDim) for h in hs] for _ in range(2))
+        for h, o in zip(hs, one):
+            gpu.GemmMLX(o, x, h, rows)
+        before = gpu.LaunchCount()
+        gpu.GemmMLXMulti(both, x, hs, rows)
+        assert gpu.LaunchCount() - before == 2
+        gpu.Sync()
+        for h, a, b in zip(hs, one, both):
+            # (how K is cut, and with it the order of the sums, follows the number of tiles of a launch)
+            u, v = (read_and_check_canary(t, rows * h.OutDim).astype(np.float64) for t in (a, b))
+            assert np.linalg.norm(u - v) <= 5e-7 * np.linalg.norm(u)
+        for t in hs + [x] + one + both:
+            t.Free()
+    assert gpu.KernelStatus() == 0
+
+
+@pytest.mark.parametrize("qtype,gen,in_dim", [("Q4_K", "q4k_matrix", 2048), ("Q6_K", "q6k_matrix", 4096), ("Q8_0", "q8_0_matrix", 2080)])
+def test_small_gguf_matrices_need_no_order(gpu, pkg, qtype, gen, in_dim):
+    """Matrices that are tiled by their size alone: streams without an order between them, and graphs beside each other, give the
+    bits of calls one after another.  Inputs of very different sizes: rows that two calls mix up are off by orders of magnitude."""
+    import torch
+    from oracle import binding as orc
+    out_dim, n = 512, 10
+    m = gpu.UploadGGUFMatrix(getattr(orc, qtype), getattr(pkg.synth, gen)("free", out_dim, in_dim), in_dim, out_dim)
+    for rows in (1, 3, 8, 13):
+        xs = [gpu.from_numpy(pkg.synth.activations(("free", i), rows * in_dim, bf16=False) * F(2.0 ** (7 * (i % 8) - 24))) for i in range(n)]
+        want, outs = ([out_with_canary(gpu, rows * out_dim) for _ in range(n)] for _ in range(2))
+        for x, o in zip(xs, want):
+            m.ProjectBatchToBuffer(o, x, rows)
+        gpu.Sync()
+        want = [read_and_check_canary(o, rows * out_dim).astype(np.float64) for o in want]
+
+        def check():
+            gpu.Sync()
+            torch.cuda.synchronize()
+            for a, o in zip(want, outs):
+                b = read_and_check_canary(o, rows * out_dim).astype(np.float64)
+                # (13 rows: the several-row kernel where a stream has scratch, passes of eight where it has none)
+                assert np.linalg.norm(a - b) <= (0 if rows <= 8 else 1e-6) * np.linalg.norm(a)
+
+        streams = [torch.cuda.Stream() for _ in range(n)]
+        for _ in range(5):
+            for s, x, o in zip(streams, xs, outs):
+                m.ProjectBatchToBuffer(o, x, rows, s)
+        check()
+        graphs, capture = [], torch.cuda.Stream()
+        for x, o in zip(xs, outs):
+            o.Zero()
+            g = torch.cuda.CUDAGraph()
+            gpu.Sync()
+            with torch.cuda.graph(g, stream=capture):
+                m.ProjectBatchToBuffer(o, x, rows, capture)
+            graphs.append(g)
+        gpu.Sync()
+        for o in outs:
+            o.Upload(np.full(rows * out_dim + 64, 123.0, dtype=F))
+        for s, g in zip(streams, graphs):
+            with torch.cuda.stream(s):
+                g.replay()
+        check()
+        del graphs
+        for t in xs + outs:
+            t.Free()
+    m.Free()
+    assert gpu.KernelStatus() == 0
