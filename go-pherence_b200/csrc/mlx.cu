@@ -1162,15 +1162,15 @@ static int mlx_row_products(int n, float* const* outs, const goph_mlx_weight* co
                             cudaStream_t stream) {
   const goph_mlx_weight* w0 = ws[0];
   // Several rows go to the integer tensor-core kernel, which reads the same buffers; a row alone does where the one-pass kernel of
-  // short rows does not take it (long rows) or is bound by its instructions (B200, us a call, CUDA cores / tensor cores: one row 2048x2048 2.8 / 3.2,
-  // 512x8192 4.6 / 3.9, 256x16384 10.0 / 5.7; two 1024x1024 3.4 / 3.0, 2048x2048 5.0 / 3.3; four 1024x1024 3.6 / 3.6, 2048x2048 7.5 / 4.0).
+  // short rows does not take it (long rows) or is bound by its instructions (B200, us a call, CUDA cores / tensor cores: one row 2048x2048 2.8 / 3.2, 1024x4096 3.6 / 3.7,
+  // 1024x6144 4.7 / 4.1, 2560x2560 5.8 / 3.7, 768x8192 5.5 / 3.9, 256x16384 10.0 / 4.5; two 1024x1024 3.4 / 3.0, 2048x2048 5.0 / 3.3; four 1024x1024 3.6 / 3.6, 2048x2048 7.5 / 4.0).
   bool tensor = options().mlx_rows == 0;
   long weights = 0;
   for (int i = 0; i < n; ++i) {
     tensor = tensor && mlx_mma_rows_ok(ws[i]);
     weights += (long)ws[i]->out_dim * w0->in_dim;
   }
-  if (tensor && (batch > 1 || w0->in_dim > 8192 || weights >= 8l << 20)) return mlx_mma_launch_rows(n, ws, outs, x, batch, options().mlx_digits, stream);
+  if (tensor && (batch > 1 || w0->in_dim > 4096 || weights > 6l << 20)) return mlx_mma_launch_rows(n, ws, outs, x, batch, options().mlx_digits, stream);
   bool uniform = true;
   for (int i = 0; i < n; ++i)
     uniform = uniform && fast_path_ok(ws[i]) && ws[i]->sb_bf16 == w0->sb_bf16;

@@ -1348,8 +1348,11 @@ bool choose_plan(int device, int ntiles, int nchunks, int nblocks, int n, int pi
       const int nfull = items / grid * grid, ntail = items - nfull;
       if (ntail > clusters || (S > 1 && ntail == 0)) continue;  // the shared items are the last thing a cluster does
       if ((nfull && nchunks > max_chunks) || (ntail && (nchunks + S - 1) / S > max_chunks)) continue;
-      const double cost = (nfull / grid * (nchunks * chunk + 1500.0)) + (ntail ? (nchunks + S - 1) / S * chunk + 1500.0 : 0) + (S > 1 ? 1500.0 + TT * n * 8.0 : 0) +
-                          (want && S != want ? 1e12 : 0);
+      double cost = (nfull / grid * (nchunks * chunk + 1500.0)) + (ntail ? (nchunks + S - 1) / S * chunk + 1500.0 : 0) + (S > 1 ? 1500.0 + TT * n * 8.0 : 0) +
+                    (want && S != want ? 1e12 : 0);
+      // Clusters of three and more that the device only just holds do not start all at once behind another kernel (Q8_0 3250x14080 x29: 26 clusters
+      // of five 46.7 us, of four 33.1).
+      if (S > 2 && (nfull ? grid / S : ntail) == clusters) cost *= 1.35;
       if (best_cost < 0 || cost < best_cost) {
         best_cost = cost;
         *best = Plan{TT, nfull ? grid : ntail * S, nfull, ntail, S};
@@ -1361,16 +1364,14 @@ bool choose_plan(int device, int ntiles, int nchunks, int nblocks, int n, int pi
 
 // What a chunk of one tile costs where its conversion and the hand-overs of its accumulator blocks set the pace (28672x4096, 16 and 64 rows).  With
 // 300 for every format the plan took two tiles an item, and fewer items than SMs, where one was better (B200, us a call): Q8_0 6000x2048 x200 43.4 ->
-// 36.5, 12000x1024 x30 14.6 -> 12.8, Q6_K 20000x1024 x64 39.1 -> 29.7, Q4_K 4096x14336 x20 28.7 -> 26.1, Q5_K 20000x1536 x12 19.5 -> 17.1.  Full blocks of
-// columns of Q4_K and Q5_K keep it: there the B tiles, which two tiles of an item share, count for more than the estimate has (Q4_K 14336x4096 x64 29.7, with
-// one tile 35.6; Q4_K 3584x18944 x11 28.0 and 30.4).  MLX with foldable scales and FP8 close a block in 16 chunks and wait for the L2 or the tensor cores.
+// 36.5, 12000x1024 x30 14.6 -> 12.8, 1500x12288 x100 40.5 -> 37.4, Q6_K 20000x1024 x64 39.1 -> 29.7, 2000x8192 x40 39.9 -> 31.4.  The others keep it: what
+// two tiles of an item share, the B tiles, counts for more than the estimate has (Q4_K 14336x4096 x64 29.7, with one tile 35.6, 3584x18944 x11 28.0
+// and 30.4; Q5_K 28.0 and 32.1); MLX with foldable scales and FP8 close a block in 16 chunks and wait for the L2 or the tensor cores.
 template <int F>
 double tile_cycles(int n) {
   const double more = (n - 16) / 48.0;  // of 64 columns
   if (F == Q_Q80) return 3100 + 1500 * more;
   if (F == Q_Q6K) return 5500 + 2100 * more;
-  if (F == Q_Q4K && n > 16 && n < 64) return 1700 + 800 * more;
-  if (F == Q_Q5K && n < 64) return 2000 + 1000 * more;
   return 300;
 }
 
