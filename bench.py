@@ -655,7 +655,7 @@ def run_ours(args):
                     "ms_per_step": round(ms_e2e / timed_steps, 4)},
             "gpu_launches": wl.launches_per_step * timed_steps,
             "roofline": {"bound": "hbm",
-                         "kernel": ("mlx_mma_kernel (tcgen05 GEMV): %d launches per step, %s; its duration is the step's CUDA-event time"
+                         "kernel": ("mlx_mma_kernel (integer tensor-core GEMV): %d launches per step, %s; its duration is the step's CUDA-event time"
                                     % (n_products, "all that there is in it" if others == 0 else "beside %d others, whose time counts as its own" % others)),
                          "achieved": round(achieved, 1), "peak": hbm_peak, "unit": "GB/s",
                          "frac": round(achieved / hbm_peak, 4), "peak_kind": peak_kind,

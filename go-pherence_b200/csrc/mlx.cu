@@ -1508,8 +1508,8 @@ static int mlx_upload_common(int device, const uint32_t* weight, const float* sc
   UP(cudaDeviceSynchronize());
 #undef UP
   h->bytes = want_w * 4 + want_s * (h->sb_bf16 ? 4 : 8);
-  // Tiled layout + tensor-core kernel for matrices large enough to amortise that kernel's fixed
-  // cost (TMEM set-up, activation preparation, pipeline fill); small ones stay row-major.
+  // Tiled layout for large matrices; small ones stay row-major, the layout that product lists, fused preparations and
+  // single-token experts read (the tensor-core kernels read either).
   const bool big = (uint64_t)out_dim * (uint64_t)in_dim >= (8u << 20);
   if (mlx_mma_supported(h) && (options().mlx_layout == 2 || (options().mlx_layout == 0 && big))) {
     if (int rc = mlx_mma_make_tiled(h)) return cleanup(rc);

@@ -1,4 +1,4 @@
-// Tensor-core (tcgen05) path for MLX 4-bit weights; implemented in mlx_mma.cu.
+// Tensor-core products of few activation rows (MLX, GGUF, FP8); implemented in mlx_mma.cu.
 #pragma once
 
 #include "goph_internal.cuh"
@@ -101,7 +101,7 @@ int gguf_mma_launch_work(const goph_gguf_matrix* m, const MmaWorkLaunch& g, unsi
 int mlx_mma_status(int device);
 void mlx_mma_status_clear(int device);
 
-// GGUF Q4_K / Q8_0 on the same kernel.  make_tiled builds m->tiled from the matrix's device
+// GGUF matrices on the same kernel.  make_tiled builds m->tiled from the matrix's device
 // buffers (which the caller then frees); dequant reproduces dequantRowQ4KTo / dequantRowQ8_0To.
 bool gguf_mma_supported(int qtype, int in_dim);
 int gguf_mma_make_tiled(goph_gguf_matrix* m);

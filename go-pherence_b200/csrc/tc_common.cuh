@@ -136,36 +136,6 @@ __device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[16]) {
                : "memory");
 }
 
-// D[tmem] (+)= A[tmem] * B[smem descriptor], 8-bit integers, int32 accumulate; one thread issues.
-__device__ __forceinline__ void umma_i8_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                           uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
-      : "memory");
-}
-// The same with A read from shared memory through a descriptor.
-__device__ __forceinline__ void umma_i8_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                           uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
-      : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem descriptor], bf16 operands, f32 accumulate (kind::f16).
-__device__ __forceinline__ void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                             uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
-      : "memory");
-}
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
@@ -177,13 +147,6 @@ __device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[8]) {
                : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
                :
                : "memory");
-}
-// One lane waits for the whole warp (32 lanes polling the same barrier only crowd the shared-memory
-// pipeline); the shuffle hands the outcome to the others and orders their later accesses behind it.
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, int* status, int code, int lane) {
-  int ok = 1;
-  if (lane == 0) ok = mbar_wait(bar, parity, status, code) ? 1 : 0;
-  return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 // One arrival for the whole warp: the lanes meet (which orders their shared-memory reads and, with
 // the tcgen05 fence each lane has executed, their TMEM accesses before the releasing arrival).

@@ -96,9 +96,9 @@ int goph_sm_count(int device);
  *   "pdl"         1 (default) launches kernels with programmatic stream serialization so a kernel's
  *                 prologue and weight prefetch overlap the tail of the kernel in front; 0 plain launches
  *   "mlx_layout"  device layout chosen by goph_mlx_upload.  The tiled layout feeds the tensor-core
- *                 (tcgen05) kernel and needs group size 64, in_dim a multiple of 256 and bf16-valued
- *                 scales and biases; the row-major layout feeds the CUDA-core kernels, and with several
- *                 rows (from 3 to 25, by size) the tensor-core kernel of several rows as well.
+ *                 kernels and needs group size 64, in_dim a multiple of 256 and bf16-valued
+ *                 scales and biases; the row-major layout feeds the CUDA-core kernels (one row, other groups and
+ *                 tables) and, with two rows and more, or one of a long or large matrix, the tensor-core kernels as well.
  *                 0 (default): tiled for matrices of 8 Mi weights or more, row-major below; 1: always
  *                 row-major; 2: tiled whenever the shape allows
  *   "gguf_layout" the same choice for goph_gguf_upload (Q4_K, Q5_K, Q6_K: in_dim a multiple of 256, Q8_0: of 32;
@@ -109,12 +109,13 @@ int goph_sm_count(int device);
  *   "fp8_layout"  the same choice for goph_fp8_upload (in_dim a multiple of 256, no NaN codes in the
  *                 weight).  In the tensor-core layout up to 4 f32 or 16 bf16 rows run with the e4m3
  *                 bytes read by the MMA as they lie (f32 activations as six e4m3 pieces, exact, bf16
- *                 activations as two); the row-major layout is served by the CUDA-core kernels.
+ *                 activations as two); the row-major layout is served by the same kernel (one and two rows of long or
+ *                 large matrices) and the CUDA-core kernels.  Where e4m3 pieces are used a NaN or an infinity makes all outputs of its activation row NaN
  *                 More rows of either layout run on the kernel of several rows, the bytes turned into
  *                 f16 (exact), f32 activations as up to three f16 pieces, bf16 ones as one
  *   "fp8_convert" accepted, without effect (it chose between two kernels for larger bf16 batches)
  *   "mlx_digits"  signed base-128 digits each activation is written in on the tensor-core path,
- *                 relative to the largest magnitude of its 64-element group: 4 (default, 27 bits)
+ *                 (few rows of MLX and GGUF weights) relative to the largest magnitude of its 64- or 32-element group: 4 (default, 27 bits)
  *                 or 3 (20 bits; enough for bf16-valued activations).  A NaN or an infinity makes all
  *                 outputs of its activation row NaN
  *   "mlx_fuse"    1 (default): tensor-core launches of one or two activation rows, and of three or four
