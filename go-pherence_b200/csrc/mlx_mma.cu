@@ -486,11 +486,7 @@ template <int FMT, int MB, bool G>
 struct RowCfg {
   // Sixteen rows a warp, or 32 with the warps in two groups that take turns at the stages: fragments of several n tiles are
   // read from shared memory half as often.
-  #ifdef RM_SL2
-  static constexpr int SL = 2, KG = SL;
-#else
   static constexpr int SL = (FMT != FMT_FP8 && MB >= 4) || G ? 2 : 1, KG = SL;  // (FP8: a tile of sums for every activation row is registers enough)
-#endif
   static constexpr int NT = XBlock<FMT, MB>::NT;
   static constexpr int kVals = SL * NT;                      // values a lane has of an item
   static constexpr int kStoring = kConsumers / KG;           // warps that finish items
@@ -699,7 +695,7 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
       for (int sl = 0; sl < SL; ++sl)
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) acc[sl][nt][0] = acc[sl][nt][1] = 0.f;
-      float lost[FMT == FMT_FP8 ? SL : 1][FMT == FMT_FP8 ? NT : 1][2] = {};
+      float low[FMT == FMT_FP8 ? SL : 1][FMT == FMT_FP8 ? NT : 1][2] = {};
 #pragma unroll 1
       for (int c = sw.c; c < sw.c1; ++c, ++i, rc.next(S)) {
         if (KG == 2 && (i & 1) != grp) continue;
@@ -801,9 +797,10 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
           return make_float2(*reinterpret_cast<const float*>(xt + at * 4), 0.f);
         };
         if constexpr (FMT == FMT_FP8) {
-          // A sum of 128 elements leaves the tensor core, which cuts f32 sums off, before it gets long, and is added with what the sums before
-          // it lost (2-norm of the error against 64 bits, 4096 elements, normal x / of bf16 values: 256 elements in one chain 7.6e-8 / 6.9e-8,
-          // so 7.3e-8 / 6.3e-8; the kernel that kept whole rows in tensor memory 6.8e-8 / 7.0e-8; 8192 elements 7.5e-8 / 7.0e-8 and 7.8e-8 / 7.8e-8).
+          // A sum of 128 elements leaves the tensor core, which cuts f32 sums off, before it gets long.  The lane's larger piece is added in one
+          // rounding; what that loses goes, with the smaller piece, into a second sum (2-norm of the error against 64 bits, 4096 elements, normal x /
+          // of bf16 values: 6.2e-8 / 5.9e-8; both pieces added before they meet the sum 7.3e-8 / 6.3e-8, and with 256 elements in one chain 7.6e-8 /
+          // 6.9e-8; the kernel that kept whole rows in tensor memory 6.8e-8 / 7.0e-8; 8192 elements 6.0e-8 / 6.3e-8, and 7.8e-8 / 7.8e-8).
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh) {
             float d[SL][NT][4];
@@ -831,8 +828,8 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
               for (int sl = 0; sl < SL; ++sl)
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
-                  const float y = fmaf(d[sl][nt][2 * r] + d[sl][nt][2 * r + 1], xs, -lost[sl][nt][r]), sum = acc[sl][nt][r] + y;
-                  lost[sl][nt][r] = (sum - acc[sl][nt][r]) - y;
+                  const float sum = fmaf(d[sl][nt][2 * r], xs, acc[sl][nt][r]), rest = fmaf(d[sl][nt][2 * r + 1], xs, low[sl][nt][r]);
+                  low[sl][nt][r] = rest + fmaf(d[sl][nt][2 * r], xs, acc[sl][nt][r] - sum);
                   acc[sl][nt][r] = sum;
                 }
             }
@@ -1011,13 +1008,24 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
           float v0 = acc[sl][nt][0], v1 = acc[sl][nt][1];
-          if (X::kRowTile) {  // the small pieces meet first, and lanes 0 and 1 have the sum: one rounding of its size
-            if (t == 3) v0 = v1 = 0.f;  // (columns without a piece)
-            v0 += __shfl_xor_sync(0xffffffffu, v0, 3);
-            v1 += __shfl_xor_sync(0xffffffffu, v1, 3);
+          if constexpr (X::kRowTile) {  // all but lane 0's sum meet first, and lanes 0 and 1 have the total: one rounding of its size
+            float l0 = low[sl][nt][0], l1 = low[sl][nt][1];
+            if (t != 0) {
+              l0 = t == 3 ? 0.f : l0 + v0;  // (3: columns without a piece)
+              l1 = t == 3 ? 0.f : l1 + v1;
+            }
+            l0 += __shfl_xor_sync(0xffffffffu, l0, 3);
+            l1 += __shfl_xor_sync(0xffffffffu, l1, 3);
+            l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
+            l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
+            v0 = __shfl_sync(0xffffffffu, v0, lane & ~3);
+            v1 = __shfl_sync(0xffffffffu, v1, lane & ~3);
+            if (!isinf(v0)) v0 += l0;  // (an infinite sum has lost no number)
+            if (!isinf(v1)) v1 += l1;
+          } else {
+            v0 += __shfl_xor_sync(0xffffffffu, v0, 1);
+            v1 += __shfl_xor_sync(0xffffffffu, v1, 1);
           }
-          v0 += __shfl_xor_sync(0xffffffffu, v0, 1);
-          v1 += __shfl_xor_sync(0xffffffffu, v1, 1);
           float v = p ? v1 : v0;
           if (MB == 1 && !X::kRowTile) v += __shfl_xor_sync(0xffffffffu, v, 2);
           fin[sl * NT + nt] = v;

@@ -219,7 +219,7 @@ int goph_mlx_gemm_multi(int n, float* const* outs_dev, const goph_mlx_weight* co
  * a serving loop whose memory budget is fully committed to KV and expert pools, a thread that must
  * not take the allocator's device-wide synchronisation in the middle of a decode step, or code that
  * is already capturing its stream.  The kernel's scratch (health word, tile counters, prepared
- * activation digits, split-K partial sums) lives in a 242 KiB array that is part of the library
+ * activation digits, split-K partial sums) lives in a 462 KiB array that is part of the library
  * image on every GPU that loads it.
  * Limits: in_dim <= 16384, out_dim <= 524288, batch 1, tiled layout only (group size 64, in_dim a
  * multiple of 256, bf16-valued scales/biases, uploaded with "mlx_layout" 0 or 2) — anything else
