@@ -210,10 +210,13 @@ __device__ __forceinline__ void prep_chunks(const float (&v)[R][8], int lane, un
     }
   }
 }
+// 2^(field - 127), field > -23: below 1 a subnormal float, which is a power of two exactly as well.
+__device__ __forceinline__ float pow2_biased(int field) { return __uint_as_float(field > 0 ? (uint32_t)field << 23 : 1u << (22 + field)); }
 // FP8: the chunk is scaled by a power of two so that its largest magnitude lies in [128, 256) and every element written as six e4m3
 // values, each the rounding of what those before it left (exact in f32), the remainder times 2^8 after every second one: an f32
 // exactly, down to 2^-32 of the chunk's largest element.  Column p of the row's tile holds piece p; the table has, per lane of a quad, the scale of
-// its two columns.
+// its two columns.  (Chunks below 2^-120 are scaled as if they had an element of that size, which leaves their elements exact down to the
+// smallest subnormal; the scales of their last pieces, down to 2^-143, are subnormal themselves.)
 template <int MB>
 __device__ __forceinline__ void prep_fp8(const float (&v)[8], int lane, unsigned char* xb, int m) {
   typedef XBlock<FMT_FP8, MB> X;
@@ -224,10 +227,10 @@ __device__ __forceinline__ void prep_fp8(const float (&v)[8], int lane, unsigned
   for (int o = 16; o > 0; o >>= 1) mx = max_nan(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   int e = (int)((__float_as_uint(mx) >> 23) & 0xFF) - 127;
   const bool finite = e < 128;
-  if (e < -110) e = -110;
+  if (e < -120) e = -120;
   if (e > 127) e = 127;
   const float s = __uint_as_float((uint32_t)(7 - e + 127) << 23);
-  if (lane < 3) reinterpret_cast<float*>(xb + X::kFrag)[m * 4 + lane] = finite ? __uint_as_float((uint32_t)(e - 7 - 8 * lane + 127) << 23) : __uint_as_float(0x7FC00000u);
+  if (lane < 3) reinterpret_cast<float*>(xb + X::kFrag)[m * 4 + lane] = finite ? pow2_biased(e - 7 - 8 * lane + 127) : __uint_as_float(0x7FC00000u);
   float r[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) r[i] = v[i] * s;

@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 from gpu_util import F, out_with_canary, read_and_check_canary
+from oracle import binding as orc
 from test_gpu_rows import make
 
 pytestmark = pytest.mark.gpu
@@ -143,4 +144,35 @@ def test_small_gguf_matrices_need_no_order(gpu, pkg, qtype, gen, in_dim):
         for t in xs + outs:
             t.Free()
     m.Free()
+    assert gpu.KernelStatus() == 0
+
+
+@pytest.mark.parametrize("tiled", [True, False])
+def test_tiny_fp8_activations(gpu, pkg, tiled):
+    """Rows, and single chunks of 256 elements beside ordinary ones, down to the subnormal floats: the e4m3 pieces and their scales stay exact.  Every output
+    is off by f32 sums (2^-24 of a partial sum each, as above), and by half a subnormal (2^-150) for every sum of a piece and 128 elements
+    and where the weight's scale meets them: at most 400 for 33 chunks of six pieces."""
+    out_dim, in_dim = 300, 4352 if tiled else 8208
+    w, s, _ = pkg.synth.fp8_linear("tiny", out_dim, in_dim)
+    gpu.SetOption("fp8_layout", 2 if tiled else 1)
+    try:
+        h = gpu.UploadFP8E4M3Linear(w, s, None, out_dim, in_dim)
+    finally:
+        gpu.SetOption("fp8_layout", 0)
+    W = np.asarray(orc.fp8_dequant(w, s, out_dim, in_dim), dtype=np.float64).reshape(out_dim, in_dim)
+    for rows in (1, 2, 3):
+        for exponent in (-100, -104, -106, -109, -112, -119, -122, -127, -136, -146):
+            for chunk in (False, True):
+                x = pkg.synth.activations(("tiny", rows, exponent), rows * in_dim, bf16=False).reshape(rows, in_dim)
+                part = x[-1, 256:512] if chunk else x[-1]
+                part[...] = (part.astype(np.float64) * 2.0 ** exponent).astype(F)
+                xo, out = gpu.from_numpy(x.reshape(-1)), out_with_canary(gpu, rows * out_dim)
+                gpu.GemmFP8E4M3Buffer(out, xo, rows, h)
+                gpu.Sync()
+                got = read_and_check_canary(out, rows * out_dim).reshape(rows, out_dim).astype(np.float64)
+                want = x.astype(np.float64) @ W.T
+                bound = 1e-6 * np.linalg.norm(want, axis=1) + np.sqrt(out_dim) * 2.0 ** -150 * (1 + 400 * np.abs(s).max())
+                assert np.isfinite(got).all() and (np.linalg.norm(got - want, axis=1) <= bound).all(), (rows, exponent, chunk)
+                xo.Free(); out.Free()
+    h.Free()
     assert gpu.KernelStatus() == 0
