@@ -118,10 +118,13 @@ __device__ __forceinline__ float max_nan(float a, float b) {  // (fmaxf passes o
   return d;
 }
 
+// 2^(field - 127), field > -23: below 1 a subnormal float, which is a power of two exactly as well.
+__device__ __forceinline__ float pow2_biased(int field) { return __uint_as_float(field > 0 ? (uint32_t)field << 23 : 1u << (22 + field)); }
 // A warp turns the 256 elements of one chunk of activation row m, eight consecutive ones per lane (SPLIT 4: a block of
 // four warps, four lanes to the same eight elements, each of which writes one digit), into the row's part of an XBlock.
 // The digits come from one sum: q + 64 (1 + 128 + 128^2) has d_j + 64 in its j-th seven bits (the top digit has what is
 // left), and a byte pattern d + 64 of seven bits becomes the signed byte.
+// The smallest unit is 2^-149: activations keep their bits down to the subnormal floats (their groups' scales are subnormal then).
 // A group with a NaN or an infinity has the scale NaN, which is what every product with it becomes (an integer has neither).
 // R: chunks at once, each with its own values, place and row (their chains of shuffles interleave).
 template <int FMT, int MB, int SPLIT = 1, int R = 1>
@@ -150,14 +153,14 @@ __device__ __forceinline__ void prep_chunks(const float (&v)[R][8], int lane, un
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     int e = (int)((__float_as_uint(mx[r]) >> 23) & 0xFF);  // mx < 2^(e-126)
-    const bool finite = e < 255;
-    if (e < qbits + 2) e = qbits + 2;
+    const bool finite = e < 255, tiny = e < qbits;  // (whose elements want a factor above 2^127)
+    if (e < qbits - 23) e = qbits - 23;             // units of 2^-149, as fine as floats get
     if (e > 254) e = 254;
     if (sub == 0 && lane % kLanes == 0) {
       float* tab = reinterpret_cast<float*>(xb[r] + X::kFrag);
       const int g = lane / kLanes;
-      const uint32_t f = (uint32_t)(e - 126 - qbits + 127) << 23;  // 2^(E-qbits)
-      const float sc[2] = {__uint_as_float(finite ? f : 0x7FC00000u), __uint_as_float(finite ? f + (14u << 23) : 0x7FC00000u)};
+      const int f = e - 126 - qbits + 127;  // 2^(E-qbits)
+      const float sc[2] = {finite ? pow2_biased(f) : __uint_as_float(0x7FC00000u), finite ? pow2_biased(f + 14) : __uint_as_float(0x7FC00000u)};
 #pragma unroll
       for (int p = 0; p < 2; ++p) {
         float* t = tab + X::entry(m[r], p, g);
@@ -165,11 +168,18 @@ __device__ __forceinline__ void prep_chunks(const float (&v)[R][8], int lane, un
         if (F::kSums) t[1] = p ? s[r] : 0.f;
       }
     }
-    const float fi = __uint_as_float((uint32_t)(qbits - (e - 126) + 127) << 23);
+    const float fi = __uint_as_float((uint32_t)(qbits - (e - 126) + 127 - (tiny ? 64 : 0)) << 23);
     const uint32_t bias = digits == 4 ? 64u * (1 + 128 + 16384) : 64u * (1 + 128);
+    float y[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) y[i] = v[r][i];
+    if (tiny) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) y[i] *= 18446744073709551616.f;  // 2^64: exact
+    }
     int q[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) q[i] = (int)((uint32_t)__float2int_rn(v[r][i] * fi) + bias);
+    for (int i = 0; i < 8; ++i) q[i] = (int)((uint32_t)__float2int_rn(y[i] * fi) + bias);
     auto digit = [&](int d) {
       uint32_t p[2];
 #pragma unroll
@@ -210,8 +220,6 @@ __device__ __forceinline__ void prep_chunks(const float (&v)[R][8], int lane, un
     }
   }
 }
-// 2^(field - 127), field > -23: below 1 a subnormal float, which is a power of two exactly as well.
-__device__ __forceinline__ float pow2_biased(int field) { return __uint_as_float(field > 0 ? (uint32_t)field << 23 : 1u << (22 + field)); }
 // FP8: the chunk is scaled by a power of two so that its largest magnitude lies in [128, 256) and every element written as six e4m3
 // values, each the rounding of what those before it left (exact in f32), the remainder times 2^8 after every second one: an f32
 // exactly, down to 2^-32 of the chunk's largest element.  Column p of the row's tile holds piece p; the table has, per lane of a quad, the scale of

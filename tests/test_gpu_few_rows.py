@@ -176,3 +176,28 @@ def test_tiny_fp8_activations(gpu, pkg, tiled):
                 xo.Free(); out.Free()
     h.Free()
     assert gpu.KernelStatus() == 0
+
+
+@pytest.mark.parametrize("fmt,tiled", [("mlx", True), ("mlx", False), ("q4_k", True), ("q5_k", True), ("q6_k", True), ("q8_0", True)])
+def test_tiny_activations(gpu, pkg, fmt, tiled):
+    """The same for the integer formats: a digit's unit goes down to 2^-149.  Roundings to a subnormal: two (scale and minimum or bias) for every block of 16 elements
+    or more in each of the two pairs of digits, 2^-150 each."""
+    out_dim, in_dim = 300, 2048
+    h, run, W, _ = make(gpu, pkg, fmt, tiled, out_dim, in_dim)
+    W = np.asarray(W, dtype=np.float64).reshape(out_dim, in_dim)
+    for rows in (1, 2, 4, 8):
+        for exponent in (-96, -99, -104, -112, -121, -124, -127, -136, -146):
+            for chunk in (False, True):
+                x = pkg.synth.activations(("tiny", rows, exponent), rows * in_dim, bf16=False).reshape(rows, in_dim)
+                part = x[-1, 256:512] if chunk else x[-1]
+                part[...] = (part.astype(np.float64) * 2.0 ** exponent).astype(F)
+                xo, out = gpu.from_numpy(x.reshape(-1)), out_with_canary(gpu, rows * out_dim)
+                run(out, xo, rows)
+                gpu.Sync()
+                got = read_and_check_canary(out, rows * out_dim).reshape(rows, out_dim).astype(np.float64)
+                want = x.astype(np.float64) @ W.T
+                bound = 1e-6 * np.linalg.norm(want, axis=1) + np.sqrt(out_dim) * 2.0 ** -150 * (4 * in_dim / 16)
+                assert (np.linalg.norm(got - want, axis=1) <= bound).all(), (rows, exponent, chunk)
+                xo.Free(); out.Free()
+    h.Free()
+    assert gpu.KernelStatus() == 0
