@@ -1372,7 +1372,7 @@ static int launch_impl(const RowWeights& w, MmaArgs a, cudaStream_t stream, Shar
     sized[w.device] = true;
   }
   const int slots = device_state(w.device).sm_count * (plan.whole ? 1 : 2);
-  int grid = a.items < slots ? a.items : slots;
+  int grid = plan.cluster || a.items < slots ? a.items : slots;  // (a CTA of a cluster has one item)
   // FUSED: a CTA prepares the activations of one K range, so all its items must be of one split:
   // item w is split w % splits, and a grid that is a multiple of the splits keeps that fixed per CTA
   if (FUSED && a.items > grid) grid -= grid % splits;
@@ -1420,9 +1420,9 @@ static int launch_one(const RowWeights& w, const MmaArgs& a, cudaStream_t stream
   // have theirs in front: 14000x4608 one row 9.1 / 9.4, two rows 14336x4096 8.7 / 9.6 (a call of several such weights prepares them once).
   const bool small = (long)tiles * a.nchunks <= 8l * sms;
   p.whole = small || MB == 8 || (MB == 4 && (FMT != FMT_MLX4 || tiles < sms)) || (MB == 2 && kBytes && tiles < sms);
+  const int most = 1 + 28 * 1024 / RowCfg<FMT, MB, false>::kRecv;  // (of the others' sums that the first CTA of a cluster has room for)
   auto cut = [&](bool whole) {
     const int slots = sms * (whole ? 1 : 2);
-    const int most = 1 + 28 * 1024 / RowCfg<FMT, MB, false>::kRecv;  // (of the others' sums that the first CTA of a cluster has room for)
     int n = slots / tiles;
     if (n > a.nchunks) n = a.nchunks;
     if (n > kMaxSplits) n = kMaxSplits;
@@ -1454,11 +1454,30 @@ static int launch_one(const RowWeights& w, const MmaArgs& a, cudaStream_t stream
     if (p.own && Own::stages(budget, range, recv) >= least) return launch_impl<FMT, MB, true, TILED>(w, a, stream, xs, p);
     if constexpr (TILED)
       if (!p.own && Front::stages(budget, range, recv) >= least) return launch_impl<FMT, MB, false, true>(w, a, stream, xs, p);
-    if (!p.whole) cut(true);
-    else if (alone) break;
-    else if (p.own) p.own = false;
-    else if (p.cluster) p.cluster = false;  // (the sums meet in scratch and need no shared memory)
-    else break;
+    if (!p.whole) {
+      cut(true);
+    } else if (alone) {
+      // K ranges short enough for a CTA's activations, in more clusters than the device holds at once: they run in waves (9473 rows and
+      // more of 14593 elements and more).  The cut whose waves take the fewest chunks, a start of four chunks for each.  B200, us a call, one row, CUDA cores / so:
+      // Q8_0 9600x14624 63.5 / 41.0, FP8 9600x15696 53.2 / 46.0, MLX 9600x20800 67.6 / 44.0.
+      long best = 0;
+      for (int n = p.splits + 1; n <= kMaxSplits && n <= most && n <= a.nchunks; ++n) {
+        const int room = cluster_room(w.device, n, true), range = (a.nchunks + n - 1) / n;
+        if (room == 0 || Own::stages(kWholeSmem, range, n - 1) < least) continue;
+        const long cost = (long)((tiles + room - 1) / room) * (range + 4);
+        if (best && cost >= best) continue;
+        best = cost;
+        p.splits = n;
+      }
+      if (!best) break;
+      p.cluster = true;
+    } else if (p.own) {
+      p.own = false;
+    } else if (p.cluster) {
+      p.cluster = false;  // (the sums meet in scratch and need no shared memory)
+    } else {
+      break;
+    }
   }
   return kDoesNotFit;
 }

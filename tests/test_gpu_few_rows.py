@@ -201,3 +201,59 @@ def test_tiny_activations(gpu, pkg, fmt, tiled):
                 xo.Free(); out.Free()
     h.Free()
     assert gpu.KernelStatus() == 0
+
+
+@pytest.mark.parametrize("fmt,widths,rows", [("q8_0", (14624, 29216), (1, 3, 8, 12)), ("fp8", (15680, 31264), (1, 2)), ("mlx", (20800, 40992), (1, 2, 4))])
+def test_rows_too_wide_for_one_cta(gpu, pkg, fmt, widths, rows):
+    """Products without scratch whose K range is cut for no other reason than that its activations fill a CTA's shared memory: 75 tiles of rows too many for one
+    piece, 74 for two.  Rows repeat every 96th one, which keeps the reference small; the bits of equal rows are equal."""
+    for out_dim, in_dim in zip((9600, 9472), widths):
+        part = 96
+        n = -(-out_dim // part)
+        if fmt == "mlx":
+            in_dim = in_dim // 64 * 64
+            w, s, b = (np.asarray(t) for t in pkg.synth.mlx_weight("wide", part, in_dim))
+            W = orc.mlx_dequant(w, s, b, part, in_dim, 64)
+            w, s, b = (np.tile(t.reshape(part, -1), (n, 1))[:out_dim].reshape(-1) for t in (w, s, b))
+            hs = [gpu.UploadMLXWeight(w, s, b, in_dim, out_dim, 64, True)]
+            half = out_dim // 2
+            hs += [gpu.UploadMLXWeight(w[:half * in_dim // 8], s[:half * in_dim // 64], b[:half * in_dim // 64], in_dim, half, 64, True) for _ in range(2)]
+
+            def run(o, x, m):
+                gpu.GemmMLX(o, x, hs[0], m)
+                outs = [out_with_canary(gpu, m * half) for _ in range(2)]
+                gpu.GemmMLXMulti(outs, x, hs[1:], m)  # (their tiles count together)
+                gpu.Sync()
+                both = [read_and_check_canary(t, m * half).reshape(m, half) for t in outs]
+                assert np.array_equal(both[0], both[1])
+                assert np.linalg.norm(both[0] - o.Download()[:m * out_dim].reshape(m, out_dim)[:, :half]) <= 1e-6 * np.linalg.norm(both[0])
+                for t in outs:
+                    t.Free()
+        elif fmt == "fp8":
+            in_dim = in_dim // 16 * 16
+            w, s, _ = pkg.synth.fp8_linear("wide", part, in_dim)
+            W = orc.fp8_dequant(w, s, part, in_dim)
+            w, s = np.tile(w.reshape(part, -1), (n, 1))[:out_dim].reshape(-1), np.tile(s, n)[:out_dim]
+            gpu.SetOption("fp8_layout", 1)
+            hs = [gpu.UploadFP8E4M3Linear(w, s, None, out_dim, in_dim)]
+            gpu.SetOption("fp8_layout", 0)
+            run = lambda o, x, m: gpu.GemmFP8E4M3Buffer(o, x, m, hs[0])
+        else:
+            raw = np.asarray(pkg.synth.q8_0_matrix("wide", part, in_dim))
+            W = orc.gguf_dequant(raw, orc.Q8_0, in_dim, part)
+            hs = [gpu.UploadGGUFMatrix(orc.Q8_0, np.tile(raw.reshape(part, -1), (n, 1))[:out_dim].reshape(-1), in_dim, out_dim)]
+            run = lambda o, x, m: hs[0].ProjectBatchToBuffer(o, x, m)
+        W = np.asarray(W, dtype=np.float64).reshape(part, in_dim)
+        for m in rows:
+            x = pkg.synth.activations(("wide", m, in_dim), m * in_dim, bf16=False).reshape(m, in_dim)
+            xo, out = gpu.from_numpy(x.reshape(-1)), out_with_canary(gpu, m * out_dim)
+            run(out, xo, m)
+            gpu.Sync()
+            got = read_and_check_canary(out, m * out_dim).reshape(m, out_dim)
+            assert np.array_equal(got, np.tile(got[:, :part], (1, n))[:, :out_dim])
+            want = x.astype(np.float64) @ W.T
+            assert np.linalg.norm(got[:, :part] - want) <= 1e-6 * np.linalg.norm(want)
+            xo.Free(); out.Free()
+        for h in hs:
+            h.Free()
+    assert gpu.KernelStatus() == 0
