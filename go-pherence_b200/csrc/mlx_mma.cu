@@ -1285,7 +1285,7 @@ struct RowWeights {
   int device, in_dim, n;
   RowSeg seg[kMaxRowSeg];              // tile0 filled in
   const QMaps* maps[kMaxRowSeg] = {};  // row-major MLX
-  bool unordered = false;              // callers need no order between such products: no scratch of the device's
+  bool unordered = false;              // callers need no order between such products: no scratch of the device's (unless an output meets x)
   size_t scratch_bytes = kScratchFloats * sizeof(float), counters = kMaxCounters;
 };
 
@@ -1410,7 +1410,8 @@ static int launch_one(const RowWeights& w, const MmaArgs& a, cudaStream_t stream
   typedef RowSmem<FMT, MB, true, false, TILED> Own;
   typedef RowSmem<FMT, MB, false, false> Front;
   const int sms = device_state(w.device).sm_count, tiles = a.ntiles;
-  const bool alone = w.unordered || !TILED;  // no scratch: activations by the CTAs, sums inside clusters
+  // No scratch: activations by the CTAs, sums inside clusters.  (An output that meets x has x prepared in front all the same, in the device's scratch.)
+  const bool alone = (w.unordered && !xs->written) || !TILED;
   RowPlan p;
   // The lines (B200, us a call, weights from HBM).  A CTA to an SM, with a ring of all that is left: products that are over in a few stages (one row, MLX4
   // 4096x4096 4.4, two to an SM 4.6; 14336x4096 8.3 / 7.7), and several rows, whose activations leave half an SM too little (four rows 14336x4096 10.8 / 11.4;

@@ -36,7 +36,8 @@
  *     there is none the CUDA-core kernels.
  *   - Matrices are row-major; x is [batch, in_dim], out is [batch, out_dim], both f32.
  *   - Outputs do not overlap x, with one exception: few rows (those that "mlx_fuse" below names) of MLX and
- *     GGUF weights in the tensor-core layouts, one or several weights a call, where x is prepared before the first product.
+ *     GGUF weights in the tensor-core layouts, one or several weights a call, where x is prepared before the first product
+ *     (in the device's scratch: such calls are ordered by the caller, of GGUF matrices that need no order otherwise as well).
  */
 #ifndef GOPH_B200_H
 #define GOPH_B200_H

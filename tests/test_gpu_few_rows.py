@@ -257,3 +257,35 @@ def test_rows_too_wide_for_one_cta(gpu, pkg, fmt, widths, rows):
         for h in hs:
             h.Free()
     assert gpu.KernelStatus() == 0
+
+
+@pytest.mark.parametrize("fmt,n", [("q4_k", 2048), ("q5_k", 1024), ("q6_k", 2048), ("q8_0", 2048), ("q8_0", 2080), ("q8_0", 4128)])
+@pytest.mark.parametrize("rows", [1, 2])
+def test_outputs_of_small_gguf_matrices_that_overlap_x(gpu, pkg, fmt, n, rows):
+    """An output in the place of x, or across its edge, of matrices that are tiled by their size alone and otherwise use no scratch: x is
+    prepared in front, and the bits are those of buffers apart."""
+    from test_gpu_rows import GGUF
+    qtype, gen = GGUF[fmt]
+    raw = getattr(pkg.synth, gen)("over", n, n)
+    h, other_h = (gpu.UploadGGUFMatrix(qtype, raw, n, n) for _ in range(2))
+    x = pkg.synth.activations(("over", rows), rows * n, bf16=False)
+    xo, want = gpu.from_numpy(x), out_with_canary(gpu, rows * n)
+    h.ProjectBatchToBuffer(want, xo, rows)
+    gpu.Sync()
+    want = read_and_check_canary(want, rows * n)
+    buf, other = gpu.Malloc(2 * rows * n), gpu.Malloc(rows * n)
+    for out_at, x_at in ((0, 0), (0, rows * n // 2), (rows * n - 4, 0)):
+        for _ in range(20):
+            out, xb = gpu.wrap(buf.Ptr + 4 * out_at, 4 * rows * n), gpu.wrap(buf.Ptr + 4 * x_at, 4 * rows * n)
+            xb.Upload(x)
+            h.ProjectBatchToBuffer(out, xb, rows)
+            gpu.Sync()
+            assert np.array_equal(out.Download().view(np.uint32), want.view(np.uint32))
+            xb.Upload(x)
+            gpu.ProjectQ4PairToBuffers(out, other, xb, rows, h, other_h)
+            gpu.Sync()
+            assert np.array_equal(out.Download().view(np.uint32), want.view(np.uint32))
+            assert np.array_equal(other.Download().view(np.uint32), want.view(np.uint32))
+    for t in (h, other_h, xo, buf, other):
+        t.Free()
+    assert gpu.KernelStatus() == 0
