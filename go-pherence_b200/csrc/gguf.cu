@@ -461,7 +461,7 @@ GOPH_API int goph_gguf_upload(int device, int qtype, const uint8_t* raw, uint64_
   const bool big = size >= (8ull << 20) && in_dim % 256 == 0, tile = big || (size >= (qtype == GOPH_GGUF_Q6_K ? 1536ull << 10 : 512ull << 10) && out_dim >= 256);
   if (gguf_mma_supported(qtype, in_dim) && (options().gguf_layout == 2 || (options().gguf_layout == 0 && tile))) {
     if (int rc = gguf_mma_make_tiled(h)) return bail(rc);
-    h->unordered = options().gguf_layout == 0 && !big;
+    h->unordered = in_dim % 256 != 0 || (options().gguf_layout == 0 && !big);
     if (!mlx_mma_ready(device)) return bail(fail(GOPH_E_NOMEM, "cannot allocate the tensor-core path's device scratch"));
     cudaFree(h->data);
     cudaFree(h->d16);

@@ -26,8 +26,8 @@
  *     on one device whose kernels could overlap on the GPU — different streams with no ordering
  *     between them — must be ordered by the caller (one stream, or events), whatever handles
  *     they use.  The reference launches everything on one stream, which satisfies this.
- *     Products of weights in the other layouts, and of GGUF matrices that are in the tensor-core layout by their size alone
- *     (gguf_layout 0) and have fewer than 8 Mi weights or rows that are no multiple of 256, need no such order and may be captured at any time:
+ *     Products of weights in the other layouts, of GGUF matrices that are in the tensor-core layout by their size alone
+ *     (gguf_layout 0) and have fewer than 8 Mi weights, and of those whose rows are no multiple of 256, need no such order and may be captured at any time:
  *     those of several rows keep an area per stream (28 MB, for up to eight streams of a device,
  *     until its last weight is freed) and use the kernels that need none where they have no area
  *     (under capture, on further streams, without memory), whose sums are grouped differently.

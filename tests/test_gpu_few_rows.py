@@ -289,3 +289,34 @@ def test_outputs_of_small_gguf_matrices_that_overlap_x(gpu, pkg, fmt, n, rows):
     for t in (h, other_h, xo, buf, other):
         t.Free()
     assert gpu.KernelStatus() == 0
+
+
+def test_ragged_gguf_rows_need_no_order_in_any_layout(gpu, pkg):
+    """Q8_0 rows that end inside a stage, with the tensor-core layout asked for: launches on streams without an order between them give the bits of calls
+    one after another (eight rows of values of very different sizes, so that activations of two calls do not mix unseen)."""
+    import torch
+    out_dim, in_dim, rows, n = 512, 4128, 8, 10
+    gpu.SetOption("gguf_layout", 2)
+    try:
+        m = gpu.UploadGGUFMatrix(orc.Q8_0, pkg.synth.q8_0_matrix("free", out_dim, in_dim), in_dim, out_dim)
+    finally:
+        gpu.SetOption("gguf_layout", 0)
+    xs = [gpu.from_numpy(pkg.synth.activations(("free", i), rows * in_dim, bf16=False) * F(2.0 ** (7 * (i % 8) - 24))) for i in range(n)]
+    want, outs = ([out_with_canary(gpu, rows * out_dim) for _ in range(n)] for _ in range(2))
+    before = gpu.LaunchCount()
+    for x, o in zip(xs, want):
+        m.ProjectBatchToBuffer(o, x, rows)
+    assert gpu.LaunchCount() - before == n  # nothing is prepared in front, in scratch that they share
+    gpu.Sync()
+    streams = [torch.cuda.Stream() for _ in range(n)]
+    for _ in range(5):
+        for s, x, o in zip(streams, xs, outs):
+            m.ProjectBatchToBuffer(o, x, rows, s)
+    gpu.Sync()
+    torch.cuda.synchronize()
+    for a, b in zip(want, outs):
+        a, b = (read_and_check_canary(t, rows * out_dim) for t in (a, b))
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+    for t in [m] + xs + want + outs:
+        t.Free()
+    assert gpu.KernelStatus() == 0
