@@ -1569,7 +1569,8 @@ bool qgemm_wants(int fmt, bool tiled, bool x_bf16, long out_dim, int in_dim, int
   }
   if (weights > 1) {  // (MLX) by their mean size: 2048, 1024 and 1024 rows of 1024 at 16 rows 21.4 / 20.2, at 20 28.2 / 22.3;
     const long mean = size / weights;  // 2048, 512, 512 of 2048 at 9 21.6 / 22.6, at 12 24.9 / 22.7; twice 2048x2048 at 8 18.1 / 16.4;
-    return batch > (mean < Mi ? 24 : mean < 2 * Mi ? 16 : mean < 3 * Mi ? 10 : size <= 12 * Mi ? 8 : 4);
+    // four of 1024x4096 at 8 19.4 / 38.7 (and 1.6e-7 / 7.7e-7 off)
+    return batch > (mean < Mi ? 24 : mean < 2 * Mi ? 16 : mean < 3 * Mi ? 10 : mean < 5 * Mi || size <= 12 * Mi ? 8 : 4);
   }
   // Above 8 Mi weights this layout is the exception (widths that no tile takes, NaN codes, the layout options).
   // in_dim above 8192: of x the CUDA-core kernels' shared memory holds four rows (Q8_0, FP8) for one CTA an SM only, or two.

@@ -320,3 +320,27 @@ def test_ragged_gguf_rows_need_no_order_in_any_layout(gpu, pkg):
     for t in [m] + xs + want + outs:
         t.Free()
     assert gpu.KernelStatus() == 0
+
+
+# The 2-norm of the error over that of the result, x normal.  Products and biases are each five times the sum that they cancel to; their f32 sums, a term for each
+# of 64 groups, added by 16 chunks, are off by 2^-25 of at most 64 partial sums that grow like a walk: 4e-7 (1.6e-7 measured).  The several-row kernel's sums in
+# tensor memory are off by 7.7e-7.
+@pytest.mark.parametrize("rows", [5, 8])
+def test_several_mlx_weights_of_a_call_keep_exact_sums(gpu, pkg, rows):
+    in_dim, out_dim = 4096, 1024
+    hs, Ws = [], []
+    for k in range(4):
+        w, sc, b = pkg.synth.mlx_weight(("lines", k), out_dim, in_dim)
+        hs.append(gpu.UploadMLXWeight(w, sc, b, in_dim, out_dim, 64, True))
+        Ws.append(np.asarray(orc.mlx_dequant(w, sc, b, out_dim, in_dim, 64), dtype=np.float64).reshape(out_dim, in_dim))
+    x = pkg.synth.activations(("lines", rows), rows * in_dim, bf16=False)
+    xo, outs = gpu.from_numpy(x), [out_with_canary(gpu, rows * out_dim) for _ in hs]
+    gpu.GemmMLXMulti(outs, xo, hs, rows)
+    gpu.Sync()
+    for W, out in zip(Ws, outs):
+        got = read_and_check_canary(out, rows * out_dim).reshape(rows, out_dim).astype(np.float64)
+        err = _norm_err(got, x.reshape(rows, in_dim).astype(np.float64) @ W.T)
+        assert err <= 4e-7, err
+    for t in hs + [xo] + outs:
+        t.Free()
+    assert gpu.KernelStatus() == 0
