@@ -360,9 +360,13 @@ static int q_format(int qtype) {
 
 // The several-row tensor-core product (qgemm.cu) reads both layouts.
 // rows: the scratch of a matrix whose products need no order.
+// Small tiled matrices: past both layouts' lines only.  The streaming one's say how long f32 sums in registers are preferred to coarser ones in tensor memory;
+// here the rows up to there go in passes of eight (errors against 64 bits, and B200, us a call, several-row kernel / so: Q6_K 2048x2048 x16 1.2e-7 / 0.9e-7, 11.5 / 16.0;
+// 1024x1792 x24 1.2e-7 / 0.9e-7, 10.0 / 22.1; Q5_K 640x1024 x10 4.6e-7 / 1.0e-7, 7.3 / 9.8; 10000x512 x8 4.9e-7 / 0.8e-7, 8.2 / 5.8; Q4_K 10000x256 x8 4.7e-7 / 0.8e-7, 7.6 / 4.2).
 static bool qgemm_takes(const goph_gguf_matrix* m, const void* x, int batch, cudaStream_t stream, QBufs** rows) {
-  return m->in_dim <= 65536 && (m->tiled || m->qmaps.ok) && (uintptr_t)x % 16 == 0 && qgemm_wants(q_format(m->qtype), m->tiled != nullptr, false, m->out_dim, m->in_dim, batch) &&
-         ((m->tiled && !m->unordered) || (*rows = qgemm_scratch(m->device, stream)));
+  const int fmt = q_format(m->qtype);
+  return m->in_dim <= 65536 && (m->tiled || m->qmaps.ok) && (uintptr_t)x % 16 == 0 && qgemm_wants(fmt, m->tiled != nullptr, false, m->out_dim, m->in_dim, batch) &&
+         (!m->unordered || qgemm_wants(fmt, false, false, m->out_dim, m->in_dim, batch)) && ((m->tiled && !m->unordered) || (*rows = qgemm_scratch(m->device, stream)));
 }
 
 static QWeight q_weight(const goph_gguf_matrix* m) {

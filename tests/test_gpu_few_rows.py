@@ -344,3 +344,29 @@ def test_several_mlx_weights_of_a_call_keep_exact_sums(gpu, pkg, rows):
     for t in hs + [xo] + outs:
         t.Free()
     assert gpu.KernelStatus() == 0
+
+
+@pytest.mark.parametrize("fmt,out_dim,in_dim,rows", [("q4_k", 10000, 256, 8), ("q5_k", 10000, 512, 5), ("q5_k", 640, 1024, 10), ("q6_k", 1024, 2048, 16), ("q6_k", 640, 2560, 24),
+                                                     ("q6_k", 1536, 4096, 12)])
+def test_small_gguf_matrices_keep_exact_sums(gpu, pkg, fmt, out_dim, in_dim, rows):
+    """Sums of a block's products are exact here, f32 sums of at most 4096 / 16 of them off by 2^-25 of partial sums that grow like a walk: 1.2e-7 for the longest, by 16 chunks where
+    minima cancel them (1.0e-7 measured).  The several-row kernel: 4.2e-7 to 5.1e-7 with minima, 1.2e-7 to 1.4e-7 for Q6_K.  Rows of further passes have the bits of calls by themselves."""
+    from test_gpu_rows import GGUF
+    qtype, gen = GGUF[fmt]
+    raw = getattr(pkg.synth, gen)("exact", out_dim, in_dim)
+    h = gpu.UploadGGUFMatrix(qtype, raw, in_dim, out_dim)
+    W = np.asarray(orc.gguf_dequant(raw, qtype, in_dim, out_dim), dtype=np.float64).reshape(out_dim, in_dim)
+    x = pkg.synth.activations(("exact", rows), rows * in_dim, bf16=False).reshape(rows, in_dim)
+    xo, out = gpu.from_numpy(x.reshape(-1)), out_with_canary(gpu, rows * out_dim)
+    h.ProjectBatchToBuffer(out, xo, rows)
+    gpu.Sync()
+    got = read_and_check_canary(out, rows * out_dim).reshape(rows, out_dim)
+    assert _norm_err(got.astype(np.float64), x.astype(np.float64) @ W.T) <= 1.2e-7
+    last = (rows - 1) // 8 * 8
+    xl, one = gpu.from_numpy(x[last:].reshape(-1)), out_with_canary(gpu, (rows - last) * out_dim)
+    h.ProjectBatchToBuffer(one, xl, rows - last)
+    gpu.Sync()
+    assert np.array_equal(got[last:].view(np.uint32), read_and_check_canary(one, (rows - last) * out_dim).reshape(-1, out_dim).view(np.uint32))
+    for t in (h, xo, out, xl, one):
+        t.Free()
+    assert gpu.KernelStatus() == 0
