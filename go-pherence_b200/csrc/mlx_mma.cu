@@ -521,8 +521,12 @@ struct RowSmem {
   }
 };
 
+// Formats without minima, three rows and more: launches have an SM to a CTA always (launch_one), which leaves registers for two sums of every value.
+template <int FMT, int MB, bool G>
+constexpr bool kAlone = (FMT == FMT_Q80 || FMT == FMT_Q6K) && MB >= 4 && !G;
+
 template <int FMT, int MB, bool FUSED, bool G = false, bool TILED = true>
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kThreads, kAlone<FMT, MB, G> ? 1 : 2)
 mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArgs<TILED> maps) {
   static_assert(!G || !FUSED, "grouped launches: activations prepared in front");
   static_assert(TILED || ((FMT == FMT_MLX4 || FMT == FMT_FP8) && FUSED), "row-major: MLX and FP8, activations by the CTAs themselves");
@@ -533,8 +537,10 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
   typedef RowCfg<FMT, MB, G> C;
   typedef RowSmem<FMT, MB, FUSED, G, TILED> M;
   constexpr int SL = C::SL, KG = C::KG, NT = C::NT, kStage = M::kStage;
-  // A chunk is summed by itself where its terms, products and biases or minima that cancel, meet a small sum.
-  constexpr bool kByChunk = F::kSums && !(FMT == FMT_MLX4 && MB == 8);
+  // A chunk is summed by itself: its terms, products and biases or minima that cancel, meet a small sum, and without minima the lane's sum has a sixteenth or an
+  // eighth of the terms (errors against 64 bits, as one sum / so: Q6_K 28672x8192 two rows 4.0e-7 / 1.3e-7, 4096x4096 1.5e-7 / 1.0e-7, Q8_0 2.9e-7 / 1.1e-7; the kernels
+  // that these came from: 2.9e-7, 1.2e-7 and 2.1e-7).
+  constexpr bool kByChunk = FMT != FMT_FP8 && !(FMT == FMT_MLX4 && MB == 8) && !(FMT == FMT_Q80 && G);
   extern __shared__ __align__(128) unsigned char smem_dyn[];
   const int S = a.stages;
   unsigned char* ring = TILED ? smem_dyn : reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));

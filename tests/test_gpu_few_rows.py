@@ -370,3 +370,28 @@ def test_small_gguf_matrices_keep_exact_sums(gpu, pkg, fmt, out_dim, in_dim, row
     for t in (h, xo, out, xl, one):
         t.Free()
     assert gpu.KernelStatus() == 0
+
+
+@pytest.mark.parametrize("fmt,out_dim,in_dim", [("q8_0", 19072, 4096), ("q6_k", 19072, 4096), ("q8_0", 1000, 30720), ("q6_k", 1000, 30720)])
+def test_sums_of_many_blocks(gpu, pkg, fmt, out_dim, in_dim):
+    """Long K ranges, with a tile for every SM and with few tiles.  Sums of a chunk of 256 elements meet a sum of at most 16 chunks (120 of them cut into eight
+    ranges and more): 2^-25 of 16 partial sums of a chunk and of 16 of chunks, that grow like walks, 1.2e-7 for both digits' sums (1.0e-7 measured; one sum of all
+    blocks 1.5e-7 to 2.1e-7).  Rows repeat every 100th one."""
+    from test_gpu_rows import GGUF
+    qtype, gen = GGUF[fmt]
+    part = 100
+    raw = np.asarray(getattr(pkg.synth, gen)("many", part, in_dim))
+    W = np.asarray(orc.gguf_dequant(raw, qtype, in_dim, part), dtype=np.float64).reshape(part, in_dim)
+    h = gpu.UploadGGUFMatrix(qtype, np.tile(raw.reshape(part, -1), (-(-out_dim // part), 1))[:out_dim].reshape(-1), in_dim, out_dim)
+    for rows in (1, 2, 4, 8):
+        x = pkg.synth.activations(("many", rows), rows * in_dim, bf16=False).reshape(rows, in_dim)
+        xo, out = gpu.from_numpy(x.reshape(-1)), out_with_canary(gpu, rows * out_dim)
+        h.ProjectBatchToBuffer(out, xo, rows)
+        gpu.Sync()
+        got = read_and_check_canary(out, rows * out_dim).reshape(rows, out_dim)
+        err = _norm_err(got[:, :part].astype(np.float64), x.astype(np.float64) @ W.T)
+        assert err <= 1.3e-7, (rows, err)
+        assert np.array_equal(got, np.tile(got[:, :part], (1, -(-out_dim // part)))[:, :out_dim])
+        xo.Free(); out.Free()
+    h.Free()
+    assert gpu.KernelStatus() == 0
