@@ -407,7 +407,7 @@ struct RowScales {
 
 // One weight of a launch.
 struct RowSeg {
-  const unsigned char* w;  // tiled: weight blocks [tile][chunk]
+  const unsigned char* w;  // weight blocks [tile][chunk]; row-major FP8: the bytes (row-major MLX: by its tensor maps only)
   float* out;              // [batch][out_dim]
   int out_dim, tile0;      // first of its tiles among the launch's
   const float *scale, *bias;  // FP8: [out_dim]; [out_dim] or nullptr
@@ -432,11 +432,61 @@ struct MmaArgs {
   int stages;              // depth of the shared-memory ring
   int cmax;                // FUSED: most chunks an item has (resident XBlocks)
   int cluster;             // the CTAs of a tile are a cluster and have one item each
+  int plain;               // outputs of an activation row with a NaN or an infinity are those of f32 products (see plain_product); else all NaN
   const MmaGroupEntry* gwork;
   const int* gcount;
   int gmax, gtpe, gmats, gfirst, gdirect;
   size_t gxb;
 };
+
+// Where element k of a stage's row r lies in the nibble image of Q5_K and Q6_K: byte, and whether in the high nibble; the bits beside it.
+__device__ __forceinline__ int kq_byte(int r, int k) { return r * 128 + (((k >> 5) ^ (r & 7)) << 4) + (k & 15); }
+__device__ __forceinline__ bool kq_upper(int k) { return (k & 16) != 0; }
+__device__ __forceinline__ int q5k_bit_byte(int r, int k) { return Fmt<FMT_Q5K>::kHighOff + (k >> 7) * 2048 + r * 16 + (k & 15); }
+__device__ __forceinline__ int q5k_bit(int k) { return 2 * ((k >> 5) & 3) + ((k >> 4) & 1); }
+__device__ __forceinline__ int q6k_bits_byte(int r, int k) { return Fmt<FMT_Q6K>::kHighOff + (k >> 6) * 2048 + r * 16 + (k & 15); }
+__device__ __forceinline__ int q6k_bits(int k) { return 4 * ((k >> 5) & 1) + 2 * ((k >> 4) & 1); }
+
+// Weight k of a stage's row r, rounded as the reference's dequantisation does (loader/gguf/quant_matrix.go:138-158, :378-426).
+template <int FMT>
+__device__ __forceinline__ float tiled_weight(const unsigned char* stg, int r, int k) {
+  if (FMT == FMT_Q80) {
+    const signed char q = (signed char)stg[(k >> 5) * 4096 + ((k >> 4) & 1) * 2048 + (r >> 3) * 128 + (r & 7) * 16 + (k & 15)];
+    return __fmul_rn(__half2float(*reinterpret_cast<const __half*>(stg + Fmt<FMT_Q80>::kStageWBytes + r * 16 + (k >> 5) * 2)), (float)q);
+  }
+  const float d = __half2float(*reinterpret_cast<const __half*>(stg + Fmt<FMT_Q6K>::kDOff + r * 2));
+  const signed char sc = (signed char)stg[Fmt<FMT_Q6K>::kStageWBytes + r * 16 + (k >> 4)];
+  const uint32_t low = (stg[kq_byte(r, k)] >> (kq_upper(k) ? 4 : 0)) & 0xFu, two = (stg[q6k_bits_byte(r, k)] >> q6k_bits(k)) & 3u;
+  return __fmul_rn(__fmul_rn(d, (float)sc), (float)((int)(low | (two << 4)) - 32));
+}
+
+// A row with an infinity: its digits are NaN, and so is what the tensor cores give.  Formats without minima have an answer all the same, an infinity of the weight's
+// sign (NaN where two meet or the weight is zero), and the kernels for other numbers of rows give it.  Launches that share a weight with those look at their NaN
+// outputs again: if the activation row is not finite, the lane takes the f32 products of its weight row one after another.  (A NaN code of an FP8 weight costs the scan
+// of the activations only.)
+__device__ __forceinline__ bool row_is_finite(const float* x, int n, int lane) {  // by a warp
+  bool ok = true;
+  for (int k = lane; k < n; k += 32) ok = ok && (__float_as_uint(x[k]) & 0x7F800000u) != 0x7F800000u;
+  return __all_sync(0xffffffffu, ok);
+}
+template <int FMT, bool TILED>
+__device__ float plain_product(const unsigned char* w, const float* x, int row, int in_dim, int nchunks) {
+  float acc = 0.f;
+  if (FMT == FMT_FP8) {
+    for (int k = 0; k < in_dim; ++k) {
+      uint32_t f;
+      asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(f) : "h"((unsigned short)w[(size_t)row * in_dim + k]));
+      acc = fmaf(f16_lo(f), x[k], acc);
+    }
+    return acc;
+  }
+  const int r = row & (kTileRows - 1);
+  for (int c = 0; c < nchunks; ++c) {
+    const unsigned char* st = w + ((size_t)(row / kTileRows) * nchunks + c) * Fmt<FMT>::kStageBytes;
+    for (int k = 0; k < kChunkK && c * kChunkK + k < in_dim; ++k) acc = fmaf(tiled_weight<FMT>(st, r, k), x[c * kChunkK + k], acc);
+  }
+  return acc;
+}
 
 // Row-major weights: their tiles come as boxes of 128 rows, 128 bytes of nibbles (whose 128-byte swizzle is the tiled image's) and
 // 16 bytes of the table, or twice 128 bytes (FP8); zeros past the edges.
@@ -505,6 +555,33 @@ struct RowCfg {
   static constexpr int kRecv = kStoring * kVals * 128;       // a split's sums
   static constexpr int kScales = kStaged<FMT, MB> ? kConsumers * SL * 16 * kStagedRow : 0;
 };
+// A warp's outputs of a tile, of which some are NaN (see plain_product); row: of the lane's first output.  Once behind all stores, expected not to run: inside the loop
+// over the values, or as a function of its own, it cost the ends of short products 0.3 to 0.6 us (B200, Q8_0 2048x3072 x8 6.4 before, 7.1 and 6.6; so 6.45).
+template <int FMT, int MB, bool TILED, int VALS>
+__device__ __forceinline__ void store_again(const MmaArgs& a, int sg, int row, int lane) {
+  typedef XBlock<FMT, MB> X;
+  constexpr int kHalves = MB > 1 && !X::kRowTile ? 2 : 1;  // activation rows that a warp has values of at a time
+  const int t = lane & 3;
+  const RowSeg& w = a.seg[sg];
+  for (int k = 0; k < VALS; ++k) {
+    const int r = row + 16 * (k / X::NT), m0 = MB == 1 ? 0 : kHalves * (k % X::NT), m = m0 + (kHalves == 2 ? t >> 1 : 0);
+    float* const out = w.out + (size_t)m * w.out_dim + r;
+    const bool odd = (t < 2 || kHalves == 2) && m < a.batch && r < w.out_dim && isnan(*out);
+    if (!__any_sync(0xffffffffu, odd)) continue;
+    bool finite = true;
+    for (int h = 0; h < kHalves; ++h) {
+      if (m0 + h >= a.batch) continue;
+      const bool f = row_is_finite(a.x + (size_t)(m0 + h) * a.in_dim, a.in_dim, lane);
+      if (m0 + h == m) finite = f;
+    }
+    if (odd && !finite) {
+      const float v = plain_product<FMT, TILED>(w.w, a.x + (size_t)m * a.in_dim, r, a.in_dim, a.nchunks);
+      *out = FMT == FMT_FP8 ? fmaf(v, w.scale[r], w.bias ? w.bias[r] : 0.f) : v;
+    }
+    __syncwarp();
+  }
+}
+
 template <int FMT, int MB, bool FUSED, bool G, bool TILED = true>
 struct RowSmem {
   static constexpr int kStage = Fmt<FMT>::kStageBytes + (FUSED ? 0 : XBlock<FMT, MB>::kBytes);
@@ -701,6 +778,24 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
     const uint32_t a_lane = F::kNibble || !TILED ? (row0 + (mi & 1) * 8 + lr) * 128 : (mi >> 1) * 2048 + (row0 / 8 + (mi & 1)) * 128 + lr * 16;
     const uint32_t b_lane = lane * 16;
     const int t_lane = X::kFrag + 4 * (FMT == FMT_FP8 ? t : MB > 1 ? X::entry(half, p, 0) : X::entry(0, p, FMT == FMT_Q6K ? 0 : half));
+    const bool mine = t < 2 || (MB > 1 && !X::kRowTile);
+    auto act = [&](int k) { return MB == 1 ? 0 : X::kRowTile ? k % NT : 2 * (k % NT) + half; };
+    constexpr bool kPlain = !G && (TILED ? FMT == FMT_Q80 || FMT == FMT_Q6K : FMT == FMT_FP8);
+    auto store = [&](int tile, auto&& value) {  // the warp's values of a tile, by the warp as one
+      const int sg = seg_of(tile), row = (tile - a.seg[sg].tile0) * kTileRows + row0 + g + 8 * p, out_dim = a.seg[sg].out_dim;
+      float* const out = a.seg[sg].out;
+      bool odd = false;
+#pragma unroll
+      for (int k = 0; k < C::kVals; ++k) {
+        const int m = act(k), r = row + 16 * (k / NT);
+        const float v = value(k);
+        odd = odd || isnan(v);
+        if (mine && m < a.batch && r < out_dim) out[(size_t)m * out_dim + r] = finish(sg, r, v);
+      }
+      if constexpr (kPlain) {
+        if (__builtin_expect(__any_sync(0xffffffffu, odd && a.plain), 0)) store_again<FMT, MB, TILED, C::kVals>(a, sg, row, lane);
+      }
+    };
     unsigned char* sc_warp = scales + warp * (SL * 16 * kStagedRow);
     float gate[kWork ? C::kVals : 1];
     int cur_entry = -1, nb = a.batch;
@@ -1065,13 +1160,9 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
 #pragma unroll
         for (int k = 0; k < C::kVals; ++k) fin[k] += buf[k * 32];
       }
-      const int sg = G ? 0 : seg_of(sw.tile);
-      const int row = (sw.tile - (G ? 0 : a.seg[sg].tile0)) * kTileRows + row0 + g + 8 * p;  // of the first slab
-      float* const out = a.seg[sg].out;
-      const int out_dim = a.seg[sg].out_dim;
-      auto act = [&](int k) { return MB == 1 ? 0 : X::kRowTile ? k % NT : 2 * (k % NT) + half; };
-      const bool mine = t < 2 || (MB > 1 && !X::kRowTile);
       if (G) {
+        const int row = sw.tile * kTileRows + row0 + g + 8 * p, out_dim = a.seg[0].out_dim;  // of the first slab
+        float* const out = a.seg[0].out;
         if (sw.entry != cur_entry) {
           cur_entry = sw.entry;
           nb = __ldg(&entry_at(cur_entry)->count);
@@ -1102,11 +1193,7 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
         have = true;
         break;  // the CTA's one item: below
       } else if (a.splits == 1) {
-#pragma unroll
-        for (int k = 0; k < C::kVals; ++k) {
-          const int m = act(k), r = row + 16 * (k / NT);
-          if (mine && m < a.batch && r < out_dim) out[(size_t)m * out_dim + r] = finish(sg, r, fin[k]);
-        }
+        store(sw.tile, [&](int k) { return fin[k]; });
       } else {
         // Partial sums of this K range go to scratch; the warp that arrives last at its rows of the tile adds the
         // partials in split order (so the result does not depend on arrival order) and stores.
@@ -1122,13 +1209,11 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
         if (n == (unsigned)a.splits - 1) {
           __threadfence();
           const float* base = a.scratch + ((size_t)sw.tile * a.splits * C::kStoring + slot) * kPart + lane;
-#pragma unroll
-          for (int k = 0; k < C::kVals; ++k) {
+          store(sw.tile, [&](int k) {
             float sum = 0.f;
             for (int s2 = 0; s2 < a.splits; ++s2) sum += __ldcg(base + (size_t)s2 * (C::kStoring * kPart) + k * 32);
-            const int m = act(k), r = row + 16 * (k / NT);
-            if (mine && m < a.batch && r < out_dim) out[(size_t)m * out_dim + r] = finish(sg, r, sum);
-          }
+            return sum;
+          });
           if (lane == 0) a.counters[sw.tile * kConsumers + slot] = 0;
         }
       }
@@ -1149,16 +1234,11 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
       if (sw.split == 0) {
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         if (have) {
-          const int sg = seg_of(sw.tile), row = (sw.tile - a.seg[sg].tile0) * kTileRows + row0 + g + 8 * p;
-          float* const out = a.seg[sg].out;
-          const int out_dim = a.seg[sg].out_dim;
-#pragma unroll
-          for (int k = 0; k < C::kVals; ++k) {
+          store(sw.tile, [&](int k) {
             float sum = fin[k];
             for (int s2 = 1; s2 < a.splits; ++s2) sum += recv[(size_t)(s2 - 1) * (C::kRecv / 4) + slot * (C::kVals * 32) + k * 32 + lane];
-            const int m = MB == 1 ? 0 : X::kRowTile ? k % NT : 2 * (k % NT) + half, r = row + 16 * (k / NT);
-            if ((t < 2 || (MB > 1 && !X::kRowTile)) && m < a.batch && r < out_dim) out[(size_t)m * out_dim + r] = finish(sg, r, sum);
-          }
+            return sum;
+          });
         }
       }
     }
@@ -1529,6 +1609,7 @@ static int rows_launch(const RowWeights& w0, const float* x, int batch, int digi
   bool written = shared && shared->written;
   if (!shared)
     for (int i = 0; i < w.n; ++i) written = written || floats_meet(w.seg[i].out, (uint64_t)batch * w.seg[i].out_dim, x, (uint64_t)batch * w.in_dim);
+  a.plain = !written && (FMT == FMT_FP8 || w.unordered || batch > 4);
   for (int b0 = 0; b0 < batch;) {
     a.x = x + (size_t)b0 * w.in_dim;
     for (int i = 0; i < w.n; ++i) w.seg[i].out = w0.seg[i].out + (size_t)b0 * w.seg[i].out_dim;
@@ -1558,7 +1639,7 @@ int fp8_mma_launch_rows(const goph_fp8_linear* w, float* out, const float* x, in
   d.device = w->device;
   d.in_dim = w->in_dim;
   d.n = 1;
-  d.seg[0] = RowSeg{w->tiled, out, w->out_dim, 0, w->scale, w->bias};
+  d.seg[0] = RowSeg{w->tiled ? w->tiled : w->weight, out, w->out_dim, 0, w->scale, w->bias};
   d.maps[0] = &w->qmaps;
   return w->tiled ? rows_launch<FMT_FP8, true>(d, x, batch, 4, stream, nullptr) : rows_launch<FMT_FP8, false>(d, x, batch, 4, stream, nullptr);
 }
@@ -1772,20 +1853,9 @@ __global__ void q80_dequant_tiled_kernel(const unsigned char* __restrict__ tiled
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (size_t)out_dim * in_dim) return;
   int row = (int)(i / in_dim), col = (int)(i - (size_t)row * in_dim);
-  int chunk = col >> 8, k = col & 255, step = k >> 5, half = (k >> 4) & 1, r = row & 127;
-  const unsigned char* stg = tiled + ((size_t)(row >> 7) * nchunks + chunk) * Fmt<FMT_Q80>::kStageBytes;
-  signed char q = (signed char)stg[step * 4096 + half * 2048 + (r >> 3) * 128 + (r & 7) * 16 + (k & 15)];
-  uint16_t d = *reinterpret_cast<const uint16_t*>(stg + Fmt<FMT_Q80>::kStageWBytes + r * 16 + step * 2);
-  out[i] = __fmul_rn(__half2float(__ushort_as_half(d)), (float)q);
+  const int chunk = col >> 8;
+  out[i] = tiled_weight<FMT_Q80>(tiled + ((size_t)(row >> 7) * nchunks + chunk) * Fmt<FMT_Q80>::kStageBytes, row & 127, col & 255);
 }
-
-// Where element k of a stage's row r lies in the nibble image of Q5_K and Q6_K: byte, and whether in the high nibble; the bits beside it.
-__device__ __forceinline__ int kq_byte(int r, int k) { return r * 128 + (((k >> 5) ^ (r & 7)) << 4) + (k & 15); }
-__device__ __forceinline__ bool kq_upper(int k) { return (k & 16) != 0; }
-__device__ __forceinline__ int q5k_bit_byte(int r, int k) { return Fmt<FMT_Q5K>::kHighOff + (k >> 7) * 2048 + r * 16 + (k & 15); }
-__device__ __forceinline__ int q5k_bit(int k) { return 2 * ((k >> 5) & 3) + ((k >> 4) & 1); }
-__device__ __forceinline__ int q6k_bits_byte(int r, int k) { return Fmt<FMT_Q6K>::kHighOff + (k >> 6) * 2048 + r * 16 + (k & 15); }
-__device__ __forceinline__ int q6k_bits(int k) { return 4 * ((k >> 5) & 1) + 2 * ((k >> 4) & 1); }
 
 // Q5_K super-blocks in the streaming layout {16-byte header, 8 x 16 bytes of nibbles, 8 x 4 bytes of
 // fifth bits} -> stages; a thread per byte of nibbles (two elements), of bits (eight) and per header.
@@ -1877,12 +1947,8 @@ __global__ void q6k_dequant_tiled_kernel(const unsigned char* __restrict__ tiled
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (size_t)out_dim * in_dim) return;
   int row = (int)(i / in_dim), col = (int)(i - (size_t)row * in_dim);
-  int chunk = col >> 8, k = col & 255, r = row & 127;
-  const unsigned char* stg = tiled + ((size_t)(row >> 7) * nchunks + chunk) * Fmt<FMT_Q6K>::kStageBytes;
-  const float d = __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short*>(stg + Fmt<FMT_Q6K>::kDOff + r * 2)));
-  const signed char sc = (signed char)stg[Fmt<FMT_Q6K>::kStageWBytes + r * 16 + (k >> 4)];
-  const uint32_t low = (stg[kq_byte(r, k)] >> (kq_upper(k) ? 4 : 0)) & 0xFu, two = (stg[q6k_bits_byte(r, k)] >> q6k_bits(k)) & 3u;
-  out[i] = __fmul_rn(__fmul_rn(d, (float)sc), (float)((int)(low | (two << 4)) - 32));
+  const int chunk = col >> 8;
+  out[i] = tiled_weight<FMT_Q6K>(tiled + ((size_t)(row >> 7) * nchunks + chunk) * Fmt<FMT_Q6K>::kStageBytes, row & 127, col & 255);
 }
 
 bool gguf_mma_supported(int qtype, int in_dim) {

@@ -111,14 +111,16 @@ int goph_sm_count(int device);
  *                 weight).  In the tensor-core layout up to 4 f32 or 16 bf16 rows run with the e4m3
  *                 bytes read by the MMA as they lie (f32 activations as six e4m3 pieces, exact, bf16
  *                 activations as two); the row-major layout is served by the same kernel (one and two rows of long or
- *                 large matrices) and the CUDA-core kernels.  Where e4m3 pieces are used a NaN or an infinity makes all outputs of its activation row NaN
+ *                 large matrices) and the CUDA-core kernels.  In the tensor-core layout, where e4m3 pieces are used, a NaN or an infinity makes
+ *                 all outputs of its activation row NaN
  *                 More rows of either layout run on the kernel of several rows, the bytes turned into
  *                 f16 (exact), f32 activations as up to three f16 pieces, bf16 ones as one
  *   "fp8_convert" accepted, without effect (it chose between two kernels for larger bf16 batches)
  *   "mlx_digits"  signed base-128 digits each activation is written in on the tensor-core path,
  *                 (few rows of MLX and GGUF weights) relative to the largest magnitude of its 64- or 32-element group: 4 (default, 27 bits)
  *                 or 3 (20 bits; enough for bf16-valued activations).  A NaN or an infinity makes all
- *                 outputs of its activation row NaN
+ *                 outputs of its activation row NaN, but those of Q6_K and Q8_0 with more than four rows or in small or
+ *                 ragged matrices (tiled by their size alone) are what the dequantised weights give: infinities by the weight's sign
  *   "mlx_fuse"    1 (default): tensor-core launches of one or two activation rows, and of three or four
  *                 over short K ranges, make the activation digits of their own K range inside the
  *                 product kernel (one launch per product);

@@ -52,9 +52,9 @@ def test_few_rows(gpu, pkg, fmt, tiled):
     assert gpu.KernelStatus() == 0
 
 
-@pytest.mark.parametrize("fmt,tiled", [("mlx", False), ("fp8", True), ("fp8", False)])
+@pytest.mark.parametrize("fmt,tiled", [("mlx", False), ("fp8", True)])
 def test_a_row_that_is_not_finite_is_nan(gpu, pkg, fmt, tiled):
-    """As the tiled integer products: the row is NaN throughout, and no other row knows of it.  (Row-major FP8 widths from 4096 on.)"""
+    """As the tiled integer products: the row is NaN throughout, and no other row knows of it.  (Row-major FP8: test_an_infinity_in_few_rows.)"""
     out_dim, in_dim = 200, 4352
     h, run, W, _ = make(gpu, pkg, fmt, tiled, out_dim, in_dim)
     ok = ~np.isnan(np.asarray(W).reshape(out_dim, in_dim)).any(1)
@@ -393,5 +393,54 @@ def test_sums_of_many_blocks(gpu, pkg, fmt, out_dim, in_dim):
         assert err <= 1.3e-7, (rows, err)
         assert np.array_equal(got, np.tile(got[:, :part], (1, -(-out_dim // part)))[:, :out_dim])
         xo.Free(); out.Free()
+    h.Free()
+    assert gpu.KernelStatus() == 0
+
+
+@pytest.mark.parametrize("fmt,layout,out_dim,in_dim,rows", [
+    ("fp8", 1, 300, 8208, (1, 2)), ("fp8", 1, 2560, 2560, (1, 2)), ("q6_k", 0, 1024, 2048, (1, 2, 4, 8, 10)), ("q6_k", 0, 300, 8192, (1, 2, 5)), ("q6_k", 2, 300, 2048, (5, 8)),
+    ("q8_0", 0, 640, 2080, (1, 2, 4, 8)), ("q8_0", 2, 300, 2048, (5, 8)), ("q8_0", 2, 19000, 768, (5, 8))])
+@pytest.mark.parametrize("cluster", [1, 0])
+def test_an_infinity_in_few_rows(gpu, pkg, fmt, layout, out_dim, in_dim, rows, cluster):
+    """Weights without a minimum whose other numbers of rows run on kernels of f32 or f16 products: +-inf by the weight's sign, NaN where two infinities meet, the weight
+    is zero or a NaN code, as there; the other rows keep their bits.  Outputs of one CTA a tile, of clusters, and of sums that meet in scratch."""
+    from test_gpu_rows import GGUF
+    option = "fp8_layout" if fmt == "fp8" else "gguf_layout"
+    gpu.SetOption(option, layout)
+    try:
+        if fmt == "fp8":
+            w, s, b = pkg.synth.fp8_linear("inf", out_dim, in_dim, bias=True)
+            w[(out_dim - 1) * in_dim + 7] = 0x7F
+            h = gpu.UploadFP8E4M3Linear(w, s, b, out_dim, in_dim)
+            W, run = orc.fp8_dequant(w, s, out_dim, in_dim), lambda o, x, n: gpu.GemmFP8E4M3Buffer(o, x, n, h)
+        else:
+            raw = getattr(pkg.synth, GGUF[fmt][1])("inf", out_dim, in_dim)
+            h = gpu.UploadGGUFMatrix(GGUF[fmt][0], raw, in_dim, out_dim)
+            W, run = orc.gguf_dequant(raw, GGUF[fmt][0], in_dim, out_dim), lambda o, x, n: h.ProjectBatchToBuffer(o, x, n)
+    finally:
+        gpu.SetOption(option, 0)
+    W = np.asarray(W, dtype=np.float64).reshape(out_dim, in_dim)
+    gpu.SetOption("mlx_cluster", cluster)
+    try:
+        for m in rows:
+            x = pkg.synth.activations(("inf", m), m * in_dim, bf16=False).reshape(m, in_dim)
+            got = []
+            for bad in ({}, {100: np.inf}, {700: -np.inf, 701: F(1e30)}, {5: np.inf, in_dim - 3: np.inf}, {64: np.nan}):
+                y = x.copy()
+                for k, v in bad.items():
+                    y[m // 2, k] = v
+                xo, out = gpu.from_numpy(y.reshape(-1)), out_with_canary(gpu, m * out_dim)
+                run(out, xo, m)
+                gpu.Sync()
+                got.append(read_and_check_canary(out, m * out_dim).reshape(m, out_dim))
+                if bad:
+                    with np.errstate(invalid="ignore"):
+                        want = (y[m // 2].astype(np.float64) * W).sum(-1).astype(F)
+                    assert np.array_equal(got[-1][m // 2], want, equal_nan=True), (m, bad)
+                    others = [r for r in range(m) if r != m // 2]
+                    assert np.array_equal(got[-1][others].view(np.uint32), got[0][others].view(np.uint32))
+                xo.Free(); out.Free()
+    finally:
+        gpu.SetOption("mlx_cluster", 1)
     h.Free()
     assert gpu.KernelStatus() == 0
