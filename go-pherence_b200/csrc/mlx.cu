@@ -1157,14 +1157,14 @@ static QWeight q_weight(const goph_mlx_weight* w) {
   return QWeight{w->foldable ? Q_MLX4F : Q_MLX4, w->tiled != nullptr, w->tiled ? (const void*)w->tiled : w->qweight, w->sb, nullptr, nullptr, w->device, w->out_dim, w->in_dim, &w->qmaps};
 }
 
-// Row-major weights sharing x on the CUDA cores.
+// Row-major weights sharing x, those that the several-row kernel does not take.
 static int mlx_row_products(int n, float* const* outs, const goph_mlx_weight* const* ws, const float* x, int batch,
                             cudaStream_t stream) {
   const goph_mlx_weight* w0 = ws[0];
   // Several rows go to the integer tensor-core kernel, which reads the same buffers; a row alone does where the one-pass kernel of
   // short rows does not take it (long rows) or is bound by its instructions (B200, us a call, CUDA cores / tensor cores: one row 2048x2048 2.8 / 3.2, 1024x4096 3.6 / 3.7,
   // 1024x6144 4.7 / 4.1, 2560x2560 5.8 / 3.7, 768x8192 5.5 / 3.9, 256x16384 10.0 / 4.5; two 1024x1024 3.4 / 3.0, 2048x2048 5.0 / 3.3; four 1024x1024 3.6 / 3.6, 2048x2048 7.5 / 4.0).
-  bool tensor = options().mlx_rows == 0;
+  bool tensor = options().mlx_rows == 0 && options().mlx_unpack == UNPACK_EXACT && options().mlx_ctas_per_sm == 0;  // (options of the CUDA-core kernels ask for them)
   long weights = 0;
   for (int i = 0; i < n; ++i) {
     tensor = tensor && mlx_mma_rows_ok(ws[i]);

@@ -444,3 +444,32 @@ def test_an_infinity_in_few_rows(gpu, pkg, fmt, layout, out_dim, in_dim, rows, c
         gpu.SetOption("mlx_cluster", 1)
     h.Free()
     assert gpu.KernelStatus() == 0
+
+
+@pytest.mark.parametrize("option,value", [("mlx_unpack", 1), ("mlx_unpack", 2), ("mlx_ctas_per_sm", 1)])
+@pytest.mark.parametrize("rows", [1, 3])
+def test_options_of_the_cuda_core_kernels_reach_them(gpu, pkg, option, value, rows):
+    """Row-major weights that go to the tensor cores by default: an option of the streaming kernel has it run, as "mlx_rows" does (rows of a warp change no sum)."""
+    out_dim, in_dim = 1000, 8192
+    h, run, _, _ = make(gpu, pkg, "mlx", False, out_dim, in_dim)
+    x = gpu.from_numpy(pkg.synth.activations(("opt", rows), rows * in_dim, bf16=False))
+
+    def product(**opts):
+        for k, v in opts.items():
+            gpu.SetOption(k, v)
+        try:
+            out = out_with_canary(gpu, rows * out_dim)
+            run(out, x, rows)
+            gpu.Sync()
+            got = read_and_check_canary(out, rows * out_dim).view(np.uint32).copy()
+            out.Free()
+            return got
+        finally:
+            for k in opts:
+                gpu.SetOption(k, 0)
+
+    plain, asked = product(), product(**{option: value})
+    assert np.array_equal(asked, product(**{option: value, "mlx_rows": 1}))
+    assert not np.array_equal(asked, plain)
+    for t in (h, x):
+        t.Free()
