@@ -1959,10 +1959,8 @@ bool gguf_mma_supported(int qtype, int in_dim) {
 int gguf_mma_make_tiled(goph_gguf_matrix* m) {
   const int ntiles = (m->out_dim + kTileRows - 1) / kTileRows, nchunks = (m->in_dim + kChunkK - 1) / kChunkK;
   const bool q4 = m->qtype == GOPH_GGUF_Q4_K;
-  // Bytes of a row and stage.  Q5_K and Q6_K lie in the front of theirs (176 and 210): the sizes are those that programs budget
-  // with (goph_gguf_resident_bytes), from when these formats were written out to bytes.
-  const size_t row = q4 ? 144 : m->qtype == GOPH_GGUF_Q6_K ? 288 : 272;
-  const size_t bytes = (size_t)ntiles * nchunks * kTileRows * row;
+  const size_t stage = q4 ? Fmt<FMT_Q4K>::kStageBytes : m->qtype == GOPH_GGUF_Q5_K ? Fmt<FMT_Q5K>::kStageBytes : m->qtype == GOPH_GGUF_Q6_K ? Fmt<FMT_Q6K>::kStageBytes : Fmt<FMT_Q80>::kStageBytes;
+  const size_t bytes = (size_t)ntiles * nchunks * stage;
   unsigned char* t = nullptr;
   GOPH_CUDA(cudaMalloc(&t, bytes));
   if (q4) {

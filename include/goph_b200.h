@@ -59,9 +59,8 @@ enum {
 };
 
 /* GGUF tensor type ids accepted by goph_gguf_upload (loader/gguf/gguf.go:51-56).  Q5_K and Q6_K
-   (176- and 210-byte super-blocks of 256 elements; loader/gguf/quant_matrix.go:331-426) go through
-   the CUDA-core streaming kernel at file size, or, for large matrices ("gguf_layout"), to the
-   tensor-core kernel with their values written out as one byte per weight. */
+   (176- and 210-byte super-blocks of 256 elements; loader/gguf/quant_matrix.go:331-426) are kept at
+   file size in either layout ("gguf_layout"). */
 enum { GOPH_GGUF_Q8_0 = 8, GOPH_GGUF_Q4_K = 12, GOPH_GGUF_Q5_K = 13, GOPH_GGUF_Q6_K = 14 };
 
 typedef struct goph_mlx_weight goph_mlx_weight;   /* nvidia.GPUMLXWeight      (runtime/mlx.go:21-32)   */
@@ -103,7 +102,7 @@ int goph_sm_count(int device);
  *                 0 (default): tiled for matrices of 8 Mi weights or more, row-major below; 1: always
  *                 row-major; 2: tiled whenever the shape allows
  *   "gguf_layout" the same choice for goph_gguf_upload (Q4_K, Q5_K, Q6_K: in_dim a multiple of 256, Q8_0: of 32;
- *                 Q5_K and Q6_K keep 1.06 / 1.13 bytes per weight in the tensor-core layout, and read 0.69 / 0.82 of them):
+ *                 the tensor-core layout has the file's bytes per weight, rows padded to 128 and Q8_0's to 256 elements):
  *                 0 (default) tensor-core layout from 0.5 Mi weights and 256 rows (Q6_K 1.5 Mi), 1 always the streaming layout,
  *                 2 tensor-core layout whenever the shape allows.  "mlx_digits" (few rows) and
  *                 "mlx_splits" apply to these products as well
