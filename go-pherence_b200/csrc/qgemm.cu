@@ -1350,9 +1350,10 @@ bool choose_plan(int device, int ntiles, int nchunks, int nblocks, int n, int pi
       if ((nfull && nchunks > max_chunks) || (ntail && (nchunks + S - 1) / S > max_chunks)) continue;
       double cost = (nfull / grid * (nchunks * chunk + 1500.0)) + (ntail ? (nchunks + S - 1) / S * chunk + 1500.0 : 0) + (S > 1 ? 1500.0 + TT * n * 8.0 : 0) +
                     (want && S != want ? 1e12 : 0);
-      // Clusters of three and more that the device only just holds do not start all at once behind another kernel (Q8_0 3250x14080 x29: 26 clusters
-      // of five 46.7 us, of four 33.1).
-      if (S > 2 && (nfull ? grid / S : ntail) == clusters) cost *= 1.35;
+      // Clusters of three, five or seven that the device only just holds do not start all at once behind another kernel, and one that starts late is late for all
+      // its items (B200, us a call: Q8_0 3250x14080 x29, 26 clusters of five 46.7, of four 33.1; Q4_K 28672x8192 x256, 45 of three 432, of two 289).  Those of four and six do: Q4_K
+      // 19072x8192 x9, 132 whole items and 17 shared by six 49.8, two tiles an item by one CTA each 62.1; 10000x4096 x200 by four 58.3, by two 65.8.
+      if (S > 2 && S % 2 && (nfull ? grid / S : ntail) == clusters) cost *= 1.35;
       if (best_cost < 0 || cost < best_cost) {
         best_cost = cost;
         *best = Plan{TT, nfull ? grid : ntail * S, nfull, ntail, S};

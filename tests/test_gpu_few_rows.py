@@ -473,3 +473,22 @@ def test_options_of_the_cuda_core_kernels_reach_them(gpu, pkg, option, value, ro
     assert not np.array_equal(asked, plain)
     for t in (h, x):
         t.Free()
+
+
+def test_a_tile_more_than_sms_shares_the_last_round(gpu, pkg):
+    """149 tiles of 8192 elements with eight rows, on the several-row kernel: the items behind the first round are shared by clusters, whose shorter sums in tensor memory
+    keep the error at 5e-7 (a CTA with two tiles and the whole range: 8.4e-7).  Rows repeat every 100th one; bound halfway between."""
+    part, out_dim, in_dim, rows = 100, 149 * 128, 8192, 8
+    raw = np.asarray(pkg.synth.q4k_matrix("more", part, in_dim))
+    W = np.asarray(orc.gguf_dequant(raw, orc.Q4_K, in_dim, part), dtype=np.float64).reshape(part, in_dim)
+    h = gpu.UploadGGUFMatrix(orc.Q4_K, np.tile(raw.reshape(part, -1), (-(-out_dim // part), 1))[:out_dim].reshape(-1), in_dim, out_dim)
+    x = pkg.synth.activations("more", rows * in_dim, bf16=False).reshape(rows, in_dim)
+    xo, out = gpu.from_numpy(x.reshape(-1)), out_with_canary(gpu, rows * out_dim)
+    h.ProjectBatchToBuffer(out, xo, rows)
+    gpu.Sync()
+    got = read_and_check_canary(out, rows * out_dim).reshape(rows, out_dim).astype(np.float64)
+    err = np.linalg.norm(got - np.tile(x.astype(np.float64) @ W.T, (1, -(-out_dim // part)))[:, :out_dim]) / np.linalg.norm(got)
+    assert err <= 6.7e-7, err
+    for t in (h, xo, out):
+        t.Free()
+    assert gpu.KernelStatus() == 0
