@@ -52,9 +52,9 @@ def test_few_rows(gpu, pkg, fmt, tiled):
     assert gpu.KernelStatus() == 0
 
 
-@pytest.mark.parametrize("fmt,tiled", [("mlx", False), ("fp8", True)])
+@pytest.mark.parametrize("fmt,tiled", [("mlx", False), ("fp8", True), ("fp8", False)])
 def test_a_row_that_is_not_finite_is_nan(gpu, pkg, fmt, tiled):
-    """As the tiled integer products: the row is NaN throughout, and no other row knows of it.  (Row-major FP8: test_an_infinity_in_few_rows.)"""
+    """As the tiled integer products: the row is NaN throughout, and no other row knows of it.  (Row-major FP8 widths from 4096 on.)"""
     out_dim, in_dim = 200, 4352
     h, run, W, _ = make(gpu, pkg, fmt, tiled, out_dim, in_dim)
     ok = ~np.isnan(np.asarray(W).reshape(out_dim, in_dim)).any(1)

@@ -189,9 +189,26 @@ def test_tiled_dequant_bit_exact(gpu, pkg, tiled_layout, qtype, out_dim, in_dim)
     raw = make(pkg, qtype, "deq-t", out_dim, in_dim)
     m = gpu.UploadGGUFMatrix(qtype, raw, in_dim, out_dim)
     padded = (out_dim + 127) // 128 * 128
-    # bytes per row and 256 elements, rows padded to the 128-row tile: the file's
-    per_chunk = {Q8_0: 272, Q4_K: 144, Q5_K: 176, Q6_K: 210}[qtype]
+    # bytes per row and 256 elements, rows padded to the 128-row tile: the file's for Q8_0 and Q4_K; Q5_K and
+    # Q6_K are written out as one byte per weight (+ 16 / 32 bytes of scales) for the tensor cores
+    per_chunk = {Q8_0: 272, Q4_K: 144, Q5_K: 272, Q6_K: 288}[qtype]
     assert m.ResidentBytes() == padded * (in_dim // 256) * per_chunk
+    out = out_with_canary(gpu, out_dim * in_dim)
+    m.Dequant(out)
+    gpu.Sync()
+    got = read_and_check_canary(out, out_dim * in_dim)
+    want = orc.gguf_dequant(raw, qtype, in_dim, out_dim, nthreads=8).reshape(-1)
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+    m.Free(); out.Free()
+
+
+@pytest.mark.parametrize("qtype,per_chunk", [(Q5_K, 176), (Q6_K, 210)])
+@pytest.mark.parametrize("out_dim,in_dim", [(128, 256), (64, 4096), (300, 512), (259, 2816)])
+def test_tiles_of_packed_bits_are_as_large_as_the_file(gpu, pkg, tiled_layout, qtype, per_chunk, out_dim, in_dim):
+    """Rows padded to the 128-row tile; the dequantisation bit for bit."""
+    raw = make(pkg, qtype, "deq-t", out_dim, in_dim)
+    m = gpu.UploadGGUFMatrix(qtype, raw, in_dim, out_dim)
+    assert m.ResidentBytes() == (out_dim + 127) // 128 * 128 * (in_dim // 256) * per_chunk
     out = out_with_canary(gpu, out_dim * in_dim)
     m.Dequant(out)
     gpu.Sync()
