@@ -555,8 +555,7 @@ struct RowCfg {
   static constexpr int kRecv = kStoring * kVals * 128;       // a split's sums
   static constexpr int kScales = kStaged<FMT, MB> ? kConsumers * SL * 16 * kStagedRow : 0;
 };
-// A warp's outputs of a tile, of which some are NaN (see plain_product); row: of the lane's first output.  Once behind all stores, expected not to run: inside the loop
-// over the values, or as a function of its own, it cost the ends of short products 0.3 to 0.6 us (B200, Q8_0 2048x3072 x8 6.4 before, 7.1 and 6.6; so 6.45).
+// A warp's outputs of a tile, of which some are NaN (see plain_product); row: of the lane's first output.  Called once, where the kernel ends.
 template <int FMT, int MB, bool TILED, int VALS>
 __device__ __forceinline__ void store_again(const MmaArgs& a, int sg, int row, int lane) {
   typedef XBlock<FMT, MB> X;
@@ -668,6 +667,8 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
   };
   float fin[C::kVals];                      // the item's values (cluster: kept for the exchange)
   bool have = false;
+  constexpr bool kPlain = !G && (TILED ? FMT == FMT_Q80 || FMT == FMT_Q6K : FMT == FMT_FP8);
+  uint32_t odd = 0;  // items of which this lane has stored a NaN (bit 31: or a later one; where K is cut and sums meet in scratch a CTA has at most 10)
 
   if (warp == kConsumers) {
     // ------------------------------------------------------------------ producer
@@ -780,21 +781,20 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
     const int t_lane = X::kFrag + 4 * (FMT == FMT_FP8 ? t : MB > 1 ? X::entry(half, p, 0) : X::entry(0, p, FMT == FMT_Q6K ? 0 : half));
     const bool mine = t < 2 || (MB > 1 && !X::kRowTile);
     auto act = [&](int k) { return MB == 1 ? 0 : X::kRowTile ? k % NT : 2 * (k % NT) + half; };
-    constexpr bool kPlain = !G && (TILED ? FMT == FMT_Q80 || FMT == FMT_Q6K : FMT == FMT_FP8);
-    auto store = [&](int tile, auto&& value) {  // the warp's values of a tile, by the warp as one
+    auto store = [&](int tile, int item, auto&& value) {  // the warp's values of a tile, by the warp as one
       const int sg = seg_of(tile), row = (tile - a.seg[sg].tile0) * kTileRows + row0 + g + 8 * p, out_dim = a.seg[sg].out_dim;
       float* const out = a.seg[sg].out;
-      bool odd = false;
+      bool nan = false;
 #pragma unroll
       for (int k = 0; k < C::kVals; ++k) {
         const int m = act(k), r = row + 16 * (k / NT);
         const float v = value(k);
-        odd = odd || isnan(v);
-        if (mine && m < a.batch && r < out_dim) out[(size_t)m * out_dim + r] = finish(sg, r, v);
+        if (mine && m < a.batch && r < out_dim) {  // (of rows past the batch the digits are whatever was there)
+          nan = nan || isnan(v);
+          out[(size_t)m * out_dim + r] = finish(sg, r, v);
+        }
       }
-      if constexpr (kPlain) {
-        if (__builtin_expect(__any_sync(0xffffffffu, odd && a.plain), 0)) store_again<FMT, MB, TILED, C::kVals>(a, sg, row, lane);
-      }
+      if (kPlain && nan) odd |= 1u << (item < 31 ? item : 31);
     };
     unsigned char* sc_warp = scales + warp * (SL * 16 * kStagedRow);
     float gate[kWork ? C::kVals : 1];
@@ -1193,7 +1193,7 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
         have = true;
         break;  // the CTA's one item: below
       } else if (a.splits == 1) {
-        store(sw.tile, [&](int k) { return fin[k]; });
+        store(sw.tile, items, [&](int k) { return fin[k]; });
       } else {
         // Partial sums of this K range go to scratch; the warp that arrives last at its rows of the tile adds the
         // partials in split order (so the result does not depend on arrival order) and stores.
@@ -1209,7 +1209,7 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
         if (n == (unsigned)a.splits - 1) {
           __threadfence();
           const float* base = a.scratch + ((size_t)sw.tile * a.splits * C::kStoring + slot) * kPart + lane;
-          store(sw.tile, [&](int k) {
+          store(sw.tile, items, [&](int k) {
             float sum = 0.f;
             for (int s2 = 0; s2 < a.splits; ++s2) sum += __ldcg(base + (size_t)s2 * (C::kStoring * kPart) + k * 32);
             return sum;
@@ -1234,7 +1234,7 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
       if (sw.split == 0) {
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         if (have) {
-          store(sw.tile, [&](int k) {
+          store(sw.tile, 0, [&](int k) {
             float sum = fin[k];
             for (int s2 = 1; s2 < a.splits; ++s2) sum += recv[(size_t)(s2 - 1) * (C::kRecv / 4) + slot * (C::kVals * 32) + k * 32 + lane];
             return sum;
@@ -1251,6 +1251,16 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
   }
   // ---- wind down: outstanding copies are drained ----
   __syncthreads();
+  if constexpr (kPlain) {
+    if (__builtin_expect(__any_sync(0xffffffffu, odd != 0 && a.plain), 0)) {
+      StageWalk again(a);
+      for (int item = 0; again.live(a); again.next_item(a), ++item) {
+        if (!__any_sync(0xffffffffu, (odd >> (item < 31 ? item : 31)) & 1u)) continue;
+        const int sg = seg_of(again.tile), slot = C::KG == 2 ? warp & 3 : warp;
+        store_again<FMT, MB, TILED, C::kVals>(a, sg, (again.tile - a.seg[sg].tile0) * kTileRows + slot * (16 * SL) + (lane >> 2) + 8 * (lane & 1), lane);
+      }
+    }
+  }
   if (*gave_up && warp == kConsumers && lane == 0) {
     // a waiter gave up: copies may still be in flight; give each ring slot a bounded chance to land
     for (int s = 0; s < S; ++s) {
