@@ -1157,7 +1157,7 @@ static QWeight q_weight(const goph_mlx_weight* w) {
   return QWeight{w->foldable ? Q_MLX4F : Q_MLX4, w->tiled != nullptr, w->tiled ? (const void*)w->tiled : w->qweight, w->sb, nullptr, nullptr, w->device, w->out_dim, w->in_dim, &w->qmaps};
 }
 
-// Row-major weights sharing x, those that the several-row kernel does not take.
+// Row-major weights sharing x, those that the several-row kernel does not take: the integer tensor-core kernel, or the CUDA-core ones.
 static int mlx_row_products(int n, float* const* outs, const goph_mlx_weight* const* ws, const float* x, int batch,
                             cudaStream_t stream) {
   const goph_mlx_weight* w0 = ws[0];

@@ -32,9 +32,9 @@
 //
 // Measured (B200, us a call among others, weights from HBM; before: the tcgen05 form, five to eight rows of MLX and Q4_K and four of Q4_K the
 // f16 kernel of qgemm.cu):
-//   one row     MLX4 4096x4096 6.2 -> 4.5, 14336x4096 9.5 -> 7.6, 28672x8192 28.9 -> 22.4; Q4_K 4096x14336 11.5 -> 10.2; Q8_0 28672x8192 43.4 -> 38.7
-//   two rows    MLX4 28672x4096 18.4 -> 13.5, Q8_0 4096x4096 7.3 -> 5.3; four: Q4_K 14336x4096 21.4 -> 14.0, Q6_K 28672x8192 80.6 -> 52.4
-//   eight rows  MLX4 14336x4096 21.6 -> 16.0, Q8_0 28672x8192 101 -> 56, Q6_K 14336x4096 46.3 -> 27.0
+//   one row     MLX4 4096x4096 5.9 -> 4.8, 14336x4096 9.3 -> 7.1, 28672x8192 28.9 -> 23.3; Q4_K 4096x14336 11.1 -> 9.3; Q8_0 28672x8192 43.5 -> 39.7
+//   two rows    MLX4 28672x4096 17.8 -> 12.7, Q8_0 4096x4096 7.1 -> 5.4; four: Q4_K 14336x4096 20.9 -> 13.7, Q6_K 28672x8192 80.3 -> 62.1
+//   eight rows  MLX4 14336x4096 20.9 -> 15.6, Q8_0 28672x8192 101 -> 54, Q6_K 14336x4096 46.4 -> 27.2
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
@@ -1145,7 +1145,8 @@ mlx_mma_kernel(const __grid_constant__ MmaArgs a, const __grid_constant__ MapArg
       }
       if (KG == 1 && !ok) break;
       if constexpr (KG == 2) {
-        if (!ok && lane == 0) gave_up[1 + slot] = items + 1;  // (both groups come to the item's meeting, and both leave after it)  // the groups' sums: the second one's through shared memory (two buffers: the meeting of the next item frees this one)
+        if (!ok && lane == 0) gave_up[1 + slot] = items + 1;  // (both groups come to the item's meeting, and both leave after it)
+        // the groups' sums: the second one's through shared memory (two buffers: the meeting of the next item frees this one)
         float* buf = pair + ((items & 1) * C::kStoring + slot) * (C::kVals * 32) + lane;
         if (grp == 1) {
 #pragma unroll
@@ -1375,12 +1376,11 @@ int mlx_mma_status(int device) {
   return v;
 }
 
-// A matrix in one of the tiled layouts, as the launch code sees it.
 // Weights of one launch that share x, as the launch code sees them.
 struct RowWeights {
   int device, in_dim, n;
   RowSeg seg[kMaxRowSeg];              // tile0 filled in
-  const QMaps* maps[kMaxRowSeg] = {};  // row-major MLX
+  const QMaps* maps[kMaxRowSeg] = {};  // row-major
   bool unordered = false;              // callers need no order between such products: no scratch of the device's (unless an output meets x)
   size_t scratch_bytes = kScratchFloats * sizeof(float), counters = kMaxCounters;
 };
@@ -1526,7 +1526,7 @@ static int launch_one(const RowWeights& w, const MmaArgs& a, cudaStream_t stream
     if (n > most) n = most;
     if (n > 8 && 16 * tiles > slots) n = 8;  // (larger clusters where eight CTAs a tile leave more than half of the places empty: 256x16384 5.7 / 4.5; 4096x14336 8.4 / 9.2)
     const bool clusters = options().mlx_cluster || alone;
-    if (!whole && n == 8 && 40 * tiles > 4 * slots) n = 7;  // (eights pack badly where they would have to fill the device: 4096x14336 9.2 / 8.3)
+    if (!whole && n == 8 && 40 * tiles > 4 * slots) n = 7;  // (eights pack badly where they would have to fill the device, 30 tiles to 37: MLX4 4096x14336 9.2 / 8.3)
     if (clusters)
       while (n > 1 && cluster_room(w.device, n, whole) < tiles) --n;
     if (options().mlx_splits > 0 && !alone) n = options().mlx_splits < a.nchunks ? options().mlx_splits : a.nchunks;
@@ -2186,8 +2186,8 @@ static int launch_work(int device, const MmaWorkLaunch& g, unsigned char* scratc
   return GOPH_OK;
 }
 
-// Entries of two items; of four for Q8_0 (whose kernel spills 44 bytes a thread) where experts have three and more on average.  (Q4_K with four takes accumulator blocks of
-// 32 columns and one chunk a stage: 1.2 us an entry against 0.55.)
+// Entries of two items; of four for Q8_0 (whose kernel spills 84 bytes a thread) where experts have three and more on average.  (Q4_K, whose scales want registers
+// beside a chunk's own sums, spills more: entries of four and eight items were 7 to 30 % slower, as were those of eight for Q8_0.)
 static bool wide_entries(const MmaWorkLaunch& g) { return g.items >= 3 * g.active; }
 
 size_t gguf_mma_work_bytes(const goph_gguf_matrix* m, const MmaWorkLaunch& g) {

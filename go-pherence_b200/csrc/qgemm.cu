@@ -1545,7 +1545,9 @@ int run_one(const QWeight& w, float* out, const void* x, bool x_bf16, int batch,
 // The lines lie where this kernel's time and the few-row kernels' met (B200, us a call: few-row / this).
 // Tiled layouts: the few-row kernel takes 8 rows a launch, and its time grows with the rows; it is bound by its instructions from
 // four rows on, sooner where scales are packed.  Q6_K and Q8_0, with a block per 16 or 32 elements here too, gain later.
-// Other layouts: the CUDA-core kernels' time grows with the rows and the weights (four rows a pass, eight in two), this
+// Other layouts: MLX rows up to the line are on the integer tensor cores too.  GGUF matrices have these layouts only below 0.5 Mi weights (Q6_K 1.5 Mi) or 256
+// rows, or by option; the lines beyond are for the option, and hold small tiled matrices on exact sums (gguf.cu).  The CUDA-core
+// kernels' time grows with the rows and the weights (four rows a pass, eight in two), this
 // one's hardly, but two launches and the start cost it 7 to 9 us (Q6_K, a block per 16 elements, 9 to 19).  For Q8_0
 // the lines are where the times meet.  Elsewhere this kernel's f32 sums in tensor memory are
 // a little coarser than those of the CUDA cores (against 64 bits, 4096 elements a row: Q4_K 4.6e-7 / 2.9e-7, Q5_K 4.5e-7 /
@@ -1559,11 +1561,11 @@ bool qgemm_wants(int fmt, bool tiled, bool x_bf16, long out_dim, int in_dim, int
   if (tiled) {
     switch (fmt) {
       case Q_FP8: return batch > 4;  // 4096x14336 4 rows 17.4 / 19.7, 5 rows 34.1 / 19.8
-      // 18944 rows: a tile for every SM.  MLX 8 rows 4096x4096 8.5 / 10.7, 14336x4096 16.0 / 21.4, 18688x4096 16.5 / 25.1, 19072x4096 26.7 / 26.4, 28672x8192 50.9 / 47.1
+      // 18944 rows: a tile for each of 148 SMs.  MLX 8 rows 4096x4096 8.5 / 10.7, 14336x4096 16.0 / 21.4, 18688x4096 16.5 / 25.1, 19072x4096 26.7 / 26.4, 28672x8192 50.9 / 47.1
       case Q_MLX4: case Q_MLX4F: return batch > (out_dim <= 18944 ? 8 : 4);
       // 9472: two.  Q4_K 4 rows 14336x4096 14.0 / 21.3; 8 rows 4096x4096 10.1 / 11.6, 4096x14336 21.2 / 24.4, 8192x8192 23.6 / 22.9, 14336x4096 21.6 / 21.3
       case Q_Q4K: case Q_Q5K: return batch > (out_dim <= 9472 && size < 64 * Mi ? 8 : 4);
-      // 4096x4096 10 rows 17.1 / 19.2, 12 rows 19.9 / 19.3; 14336x4096 12 rows 43.5 / 53.7, 16 rows 53.1 / 53.7
+      // 4096x4096 10 rows 18.2 / 19.2, 12 rows 19.9 / 19.3; 14336x4096 12 rows 46.8 / 53.6, 16 rows 53.1 / 53.7
       case Q_Q6K: return batch > (size <= 16 * Mi ? 10 : 12);
       default: return batch > (size <= 16 * Mi ? 8 : 12);  // Q8_0 4096x4096 9 rows 14.1 / 13.8; 14336x4096 12 rows 29.1 / 33.5, 16 rows 34.8 / 33.6
     }
